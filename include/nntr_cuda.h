@@ -109,8 +109,8 @@ int nntr_cuda_dequantize_weight_dev(int qtype, const void *w, float *y, int64_t 
 size_t nntr_cuda_gemm_workspace_bytes(int qtype, unsigned M, unsigned N, unsigned K);
 
 /** Which kernels serve Q4_K GEMMs with M > 1 (process-wide):
- *   EXACT       integer dot products on the CUDA cores with the reference's exact
- *               floating-point chain: C equals the CPU result bit for bit;
+ *   EXACT       integer dot products with the reference's exact floating-point
+ *               chain: C equals the CPU result bit for bit;
  *   TENSOR      tcgen05 int8 tensor-core kernel (needs N % 128 == 0): exact
  *               integer sums, one rounding more per super-block in the fp32
  *               combination (measured 1e-6 from the CPU result);
@@ -161,7 +161,7 @@ int nntr_cuda_gemm_q6_K_dev(unsigned M, unsigned N, unsigned K, const float *A, 
  *  device-wide stall of a cudaMalloc. Same arguments as
  *  nntr_cuda_gemm_q4_K_dev minus the workspace: the quantized activations go to
  *  an array compiled into the library (NNTR_CUDA_NOALLOC_SCRATCH_BYTES per GPU,
- *  held from load to exit). It always runs the bit-exact CUDA-core kernels, so
+ *  held from load to exit). It always runs the bit-exact kernels, so
  *  its result equals that of nntr_cuda_gemm_q4_K_dev under
  *  NNTR_CUDA_GEMM_PATH_EXACT (and the CPU result) bit for bit; from about 32
  *  rows up the regular entry point's tensor-core paths are many times faster.

@@ -269,9 +269,9 @@ __global__ void host_done_kernel(unsigned long long *word, unsigned long long va
 
 /* --------------------------------------------------------- GEMM dispatch */
 static std::atomic<int> g_gemm_path{NNTR_CUDA_GEMM_PATH_AUTO};
-constexpr unsigned TENSOR_PATH_MIN_M = 32; // below this the dp4a kernels win (a 128-row activation tile is mostly padding)
+constexpr unsigned TENSOR_PATH_MIN_M = 32; // below this the exact kernels win (a 128-row activation tile is mostly padding)
 
-/* 0: exact CUDA-core kernels, 1: integer tensor path (kind::i8), 2: fp16 tensor path (kind::f16) */
+/* 0: exact kernels, 1: integer tensor path (kind::i8), 2: fp16 tensor path (kind::f16) */
 static int pick_gemm_kernel(int qtype, unsigned M, unsigned N, unsigned K) {
   const int path = g_gemm_path.load(std::memory_order_relaxed);
   if (path == NNTR_CUDA_GEMM_PATH_EXACT)
@@ -296,10 +296,10 @@ static size_t workspace_bytes(int qtype, unsigned M, unsigned N, unsigned K) {
   if (M <= 1)
     return 0;
   if (qtype == NNTR_Q4_0) {
-    const size_t rows0 = (size_t)M * (K / 32) * sizeof(BlockQ80);
+    const size_t rows0 = gemm_mma_workspace_bytes(qtype, M, K);
     return umma_f16_supported(qtype, M, N, K) ? std::max(rows0, umma_f16_workspace_bytes(M, K)) : rows0;
   }
-  const size_t rows = (size_t)M * (K / 256) * sizeof(BlockQ8K);
+  const size_t rows = (size_t)(qtype == NNTR_Q4_K ? (M + 7) / 8 * 8 : M) * (K / 256) * sizeof(BlockQ8K); // Q4_K: tiles of 8 rows
   // large enough for every path the setting may select at call time
   size_t need = rows;
   if (umma_supported(qtype, M, N, K))
@@ -346,27 +346,11 @@ static int gemm_dev(int qtype, unsigned M, unsigned N, unsigned K, const float *
   default:
     break;
   }
-  const unsigned M4 = (M / 4) * 4;
-  if (qtype == NNTR_Q4_0) {
-    rc = launch_quantize_q8_0(A, K, ws, M, K, st);
-  } else if (qtype == NNTR_Q6_K) {
-    rc = launch_quantize_q8_K(A, K, ws, M, K, 0, st); // ggml_interface_omp.cpp:545-551: row quantizer for all rows
-  } else {
-    rc = M4 ? launch_quantize_q8_K(A, K, ws, M4, K, 1, st) : NNTR_CUDA_OK;
-    if (!rc && M4 < M)
-      rc = launch_quantize_q8_K(A + (size_t)M4 * K, K, static_cast<uint8_t *>(ws) + (size_t)M4 * (K / 256) * sizeof(BlockQ8K),
-                                M - M4, K, 0, st);
-  }
-  if (rc)
+  if (qtype != NNTR_Q6_K)
+    return launch_gemm_mma(qtype, M, M / 4 * 4, N, K, A, B, C, ldc, ws, ws_bytes, st);
+  if ((rc = launch_quantize_q8_K(A, K, ws, M, K, 0, st))) // ggml_interface_omp.cpp:545-551: row quantizer for all rows
     return rc;
-  switch (qtype) {
-  case NNTR_Q4_K:
-    return launch_gemm_q4_K(M, N, K, ws, B, C, ldc, st);
-  case NNTR_Q4_0:
-    return launch_gemm_q4_0(M, N, K, ws, B, C, ldc, st);
-  default:
-    return launch_gemm_q6_K(M, N, K, ws, B, C, ldc, st);
-  }
+  return launch_gemm_q6_K(M, N, K, ws, B, C, ldc, st);
 }
 
 static int gemm_host(int qtype, unsigned M, unsigned N, unsigned K, const float *A, const void *B, float *C,
@@ -541,6 +525,8 @@ int nntr_cuda_device_status(void) {
     return rc;
   if (!v && (rc = read_attn_status(&v)))
     return rc;
+  if (!v && (rc = read_mma_status(&v)))
+    return rc;
   if (v)
     return set_error(v, "a device kernel gave up on a bounded wait (status %d)", v);
   if ((rc = read_embed_status(&v, false)))
@@ -557,7 +543,7 @@ int clear_device_status_words() {
   int rc;
   if ((rc = clear_device_status()) || (rc = clear_umma_status()) || (rc = clear_q6_status()) ||
       (rc = clear_moe_status()) || (rc = clear_q40_status()) || (rc = clear_f16_status()) || (rc = clear_resident_status()) ||
-      (rc = clear_attn_status()))
+      (rc = clear_attn_status()) || (rc = clear_mma_status()))
     return rc;
   return NNTR_CUDA_OK;
 }

@@ -323,11 +323,12 @@ int launch_gemv_q4_0_batched(unsigned N, unsigned K, const float *x, const void 
 int launch_gemv_q4_0_batched_publish(unsigned N, unsigned K, const float *x, unsigned n_problems, GemvBatch batch,
                                      GemvExchange ex, cudaStream_t st);
 int read_q40_status(int *out);
-/* M > 1 with activations already quantized to plain Q8 rows in `qa` */
-int launch_gemm_q4_K(unsigned M, unsigned N, unsigned K, const void *qa, const void *B, float *C, unsigned ldc,
-                     cudaStream_t st);
-int launch_gemm_q4_0(unsigned M, unsigned N, unsigned K, const void *qa, const void *B, float *C, unsigned ldc,
-                     cudaStream_t st);
+/* bit-exact GEMM of Q4_K / Q4_0 weights (gemm_mma.cu): quantizes the fp32 activations itself, into ws */
+int read_mma_status(int *out);
+int clear_mma_status();
+size_t gemm_mma_workspace_bytes(int qtype, unsigned M, unsigned K);
+int launch_gemm_mma(int qtype, unsigned M, unsigned M4, unsigned N, unsigned K, const float *A, const void *B, float *C,
+                    unsigned ldc, void *ws, size_t ws_bytes, cudaStream_t st);
 /* tensor-core path (gemm_umma.cu): quantizes the fp32 activations itself, into ws */
 bool umma_supported(int qtype, unsigned M, unsigned N, unsigned K);
 size_t umma_workspace_bytes(unsigned M, unsigned K);
@@ -344,10 +345,17 @@ int read_f16_status(int *out);
 int measure_int8_peak(double *tops_out, double *clk_per_mma_out);
 int launch_gemm_q6_K(unsigned M, unsigned N, unsigned K, const void *qa, const void *B, float *C, unsigned ldc,
                      cudaStream_t st);
-/* per-expert grouped GEMM of the MoE prefill (gemm_dp4a.cu) */
-int launch_gemm_grouped(int qtype, unsigned N, unsigned K, const void *qa, float *C, unsigned ldc,
+/* per-expert grouped GEMM of the MoE prefill (gemm_mma.cu): (token, expert) pairs sorted by expert, position p of the
+ * order being pair perm[p]; expert e has the positions off[e] .. off[e+1], the tiles tile_off[e] .. of tile_rows rows each
+ * and the activation tiles act_off[e] .. of 8 rows each (rows: perm[p] / a_div of x); output row perm[p] * c_mul (+ 1 for
+ * w_table1). */
+int grouped_tile_rows(unsigned pairs, unsigned n_experts);
+int launch_act_tiles_grouped(int qtype, const float *x, unsigned rows, unsigned K, void *act, const int *perm, const int *idx,
+                             const int *off, const int *act_off, int a_div, cudaStream_t st);
+int launch_gemm_grouped(int qtype, unsigned N, unsigned K, const void *act, float *C, unsigned ldc,
                         const void *const *w_table0, const void *const *w_table1, const int *off, const int *tile_off,
-                        const int *perm, int n_experts, int a_div, int c_mul, unsigned max_tiles, cudaStream_t st);
+                        const int *act_off, const int *perm, int n_experts, int c_mul, int tile_rows, unsigned pairs,
+                        cudaStream_t st);
 /* operators between the matmuls (glue.cu, dequantize.cu) */
 int launch_rms_norm(const float *x, const float *residual, float *sum_out, const float *gamma, float *y, long long rows,
                     int width, float eps, unsigned flags, cudaStream_t st);

@@ -87,16 +87,17 @@ extern "C" int nntr_cuda_gemm_q4_K_noalloc_dev(unsigned M, unsigned N, unsigned 
   if (rc)
     return rc;
   cudaStream_t st = static_cast<cudaStream_t>(stream);
-  /* same split as the regular entry point (ggml_interface_omp.cpp:433-461): rows
-   * below 4*floor(M/4) take the 4-row quantizer's sign rule, the rest the row
-   * quantizer's; M == 1 is all "rest" */
-  const unsigned M4 = (M == 1) ? 0 : (M / 4) * 4;
-  if (M4)
-    rc = launch_quantize_q8_K(A, K, scratch, M4, K, 1, st);
-  if (!rc && M4 < M)
-    rc = launch_quantize_q8_K(A + (size_t)M4 * K, K, static_cast<unsigned char *>(scratch) + (size_t)M4 * row_bytes,
-                              M - M4, K, 0, st);
-  if (rc)
-    return rc;
-  return launch_gemm_q4_K(M, N, K, scratch, B, C, ldc, st);
+  /* The kernels of the regular entry point's exact path, over as many rows at a time as the scratch holds: their tiles of
+   * 8 rows take 288 of the 292 bytes per row and super-block that the limit above counts. Rows below 4*floor(M/4) take the
+   * GEMM chain, the others the GEMV's, as in one call over all rows (ggml_interface_omp.cpp:433-461). */
+  const size_t tile = gemm_mma_workspace_bytes(NNTR_Q4_K, 8, K);
+  const unsigned step = tile <= (size_t)NNTR_CUDA_NOALLOC_SCRATCH_BYTES ? (unsigned)(NNTR_CUDA_NOALLOC_SCRATCH_BYTES / tile) * 8 : M;
+  for (unsigned m = 0; m < M; m += step) {
+    const unsigned rows = M - m < step ? M - m : step, M4 = M / 4 * 4;
+    rc = launch_gemm_mma(NNTR_Q4_K, rows, M4 <= m ? 0 : M4 - m < rows ? M4 - m : rows, N, K, A + (size_t)m * K, B,
+                         C + (size_t)m * ldc, ldc, scratch, NNTR_CUDA_NOALLOC_SCRATCH_BYTES, st);
+    if (rc)
+      return rc;
+  }
+  return NNTR_CUDA_OK;
 }

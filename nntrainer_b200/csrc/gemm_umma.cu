@@ -16,7 +16,7 @@
  * The integers I and J are exact; the floating-point combination uses one
  * rounding more per super-block than the reference's chain, so results agree
  * with the reference within the path's tolerance (max-rel 2e-3), not bit for
- * bit. The dp4a kernels of gemm_dp4a.cu remain the bit-exact path.
+ * bit. The warp-MMA kernels of gemm_mma.cu remain the bit-exact path.
  *
  * How. sc is a 6-bit number, q a 4-bit one: q*sc does not fit a byte. The
  * scale is split, sc = 16*(sc >> 4) + (sc & 15), which gives two unsigned

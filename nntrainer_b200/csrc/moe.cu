@@ -30,6 +30,7 @@
  */
 #include <algorithm>
 
+#include "act_tiles.cuh"
 #include "common.cuh"
 #include "moe_combine.cuh"
 #include "swiglu.cuh"
@@ -46,7 +47,6 @@ struct MoeEp {
 };
 
 constexpr unsigned GROUPED_MIN_TOKENS = 8; // from here on the pairs are sorted by expert and run as per-expert GEMMs
-constexpr int GROUPED_MT = 4;              // rows per tile of the grouped GEMM (MT of gemm_dp4a.cu)
 constexpr int MOE_COUNTER_TOKENS = 4096;   // arrival counters kept at the start of the scratch for up to this many tokens
 constexpr int ROUTER_WARPS = 8;
 constexpr int ROUTER_SLICES = 32; // CTAs per token
@@ -304,34 +304,104 @@ moe_router_kernel(const float *__restrict__ x, const float *__restrict__ wr, con
 }
 
 /* Sorts the (token, expert) pairs of a batch by expert: off[e] = first position of expert e's pairs in perm, tile_off[e]
- * = first tile of GROUPED_MT rows of expert e, perm = pair indices grouped by expert (order inside an expert is
+ * = first tile of tile_rows rows of expert e, act_off[e] = its first activation tile of 8 rows, perm = pair indices grouped by expert (order inside an expert is
  * arbitrary: every row of the grouped GEMM is computed on its own). One CTA; the pair list of a prefill is a few
- * thousand entries. */
-__global__ void moe_permute_kernel(const int *__restrict__ idx, int P, int E, int *__restrict__ off,
-                                   int *__restrict__ tile_off, int *__restrict__ perm) {
-  __shared__ int cnt[256], cur[256];
+ * thousand entries. E <= 256 = one expert per lane of the first eight warps, so the two prefix sums are warp scans. */
+__global__ void __launch_bounds__(1024) moe_permute_kernel(const int *__restrict__ idx, int P, int E, int tile_rows,
+                                                          int *__restrict__ off, int *__restrict__ tile_off,
+                                                          int *__restrict__ act_off, int *__restrict__ perm) {
+  __shared__ int cnt[256], cur[256], sums[3][8];
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  if (tid < 256)
+    cnt[tid] = 0;
+  pdl_launch_dependents();
   pdl_wait(); // idx comes from the router launched just before
-  for (int e = threadIdx.x; e < E; e += blockDim.x)
-    cnt[e] = 0;
   __syncthreads();
-  for (int p = threadIdx.x; p < P; p += blockDim.x)
+  for (int p = tid; p < P; p += blockDim.x)
     atomicAdd(&cnt[idx[p]], 1);
   __syncthreads();
-  if (threadIdx.x == 0) {
-    int o = 0, t = 0;
-    for (int e = 0; e < E; ++e) {
-      off[e] = o;
-      tile_off[e] = t;
-      cur[e] = o;
-      o += cnt[e];
-      t += (cnt[e] + GROUPED_MT - 1) / GROUPED_MT;
+  int c = 0, n[3] = {}, s[3] = {}; // pairs, tiles, activation tiles: of this expert, up to and including it
+  if (tid < 256) {
+    c = tid < E ? cnt[tid] : 0;
+    n[0] = c;
+    n[1] = (c + tile_rows - 1) / tile_rows;
+    n[2] = (c + 7) / 8;
+#pragma unroll
+    for (int k = 0; k < 3; ++k) {
+      s[k] = n[k];
+      for (int d = 1; d < 32; d <<= 1) {
+        const int v = __shfl_up_sync(FULL, s[k], d);
+        if (lane >= d)
+          s[k] += v;
+      }
+      if (lane == 31)
+        sums[k][warp] = s[k];
     }
-    off[E] = o;
-    tile_off[E] = t;
   }
   __syncthreads();
-  for (int p = threadIdx.x; p < P; p += blockDim.x)
+  if (tid < 256) {
+#pragma unroll
+    for (int k = 0; k < 3; ++k)
+      for (int w = 0; w < warp; ++w)
+        s[k] += sums[k][w];
+    if (tid < E) {
+      off[tid] = cur[tid] = s[0] - n[0];
+      tile_off[tid] = s[1] - n[1];
+      act_off[tid] = s[2] - n[2];
+    }
+    if (tid == E - 1) {
+      off[E] = s[0];
+      tile_off[E] = s[1];
+    }
+  }
+  __syncthreads();
+  for (int p = tid; p < P; p += blockDim.x)
     perm[atomicAdd(&cur[idx[p]], 1)] = p;
+}
+
+/* The activation between the grouped GEMMs, quantized for the second one: position p of the sorted pairs, unit b of 256
+ * of the intermediate width; one warp each. Same element functions as moe_act_kernel. */
+template <int QT>
+__global__ void __launch_bounds__(256)
+moe_act_tiles_kernel(const float *__restrict__ gu, uint8_t *__restrict__ act, const int *__restrict__ perm,
+                     const int *__restrict__ idx, const int *__restrict__ off, const int *__restrict__ act_off,
+                     const float *const *__restrict__ gate_b, const float *const *__restrict__ up_b, int kind, float alpha, int I, int nb, int P) {
+  pdl_launch_dependents();
+  pdl_wait();
+  const int lane = threadIdx.x & 31;
+  const long w = (long)blockIdx.x * 8 + (threadIdx.x >> 5);
+  if (w >= (long)P * nb)
+    return;
+  const int pos = (int)(w / nb), b = (int)(w - (long)pos * nb), pair = perm[pos], e = idx[pair];
+  const int i = pos - off[e];
+  const int c0 = b * QK_K + lane * 8;
+  float v[8];
+  if (c0 < I) { // I % 8 == 0; blocks past I are zeros
+    const float4 *gp = reinterpret_cast<const float4 *>(gu + (size_t)(2 * pair) * I + c0);
+    const float4 *up = reinterpret_cast<const float4 *>(gu + (size_t)(2 * pair + 1) * I + c0);
+    const float4 g0 = gp[0], g1 = gp[1], u0 = up[0], u1 = up[1];
+    const float g[8] = {g0.x, g0.y, g0.z, g0.w, g1.x, g1.y, g1.z, g1.w},
+                u[8] = {u0.x, u0.y, u0.z, u0.w, u1.x, u1.y, u1.z, u1.w};
+    if (kind == 0) {
+#pragma unroll
+      for (int k = 0; k < 8; ++k)
+        v[k] = swish_mul_elem(g[k], u[k]);
+    } else {
+#pragma unroll
+      for (int k = 0; k < 8; ++k)
+        v[k] = swiglu_elem(__fadd_rn(g[k], gate_b[e][c0 + k]), __fadd_rn(__fadd_rn(u[k], up_b[e][c0 + k]), 1.f), true, alpha);
+    }
+  } else {
+#pragma unroll
+    for (int k = 0; k < 8; ++k)
+      v[k] = 0.f;
+  }
+  uint8_t *unit = act_unit<QT>(act, act_off[e] + (i >> 3), 8, nb, b);
+  const float4 v0 = make_float4(v[0], v[1], v[2], v[3]), v1 = make_float4(v[4], v[5], v[6], v[7]);
+  if constexpr (QT == NNTR_Q4_K)
+    put_q8K(unit, 8, i & 7, q8K_quantize_warp(v0, v1, lane, 0), lane);
+  else
+    put_q80(unit, 8, i & 7, q80_quantize_warp(v0, v1), lane);
 }
 
 /* a[p][i] from the gate / up GEMV outputs gu[2p][i], gu[2p+1][i] */
@@ -468,7 +538,7 @@ static cudaError_t launch_pdl(void (*kernel)(KArgs...), unsigned grid, unsigned 
 }
 
 struct MoeWs {
-  size_t idx, ord, w, gu_tab, dn_tab, rpart, rcount, gu, act, dn, off, tile_off, perm, qx, qact, total;
+  size_t idx, ord, w, gu_tab, dn_tab, rpart, rcount, gu, act, dn, off, tile_off, act_off, perm, qx, qact, total;
 };
 
 static MoeWs moe_ws(unsigned T, unsigned H, unsigned I, unsigned topk, unsigned E = 256) {
@@ -503,14 +573,15 @@ static MoeWs moe_ws(unsigned T, unsigned H, unsigned I, unsigned topk, unsigned 
   o = align_up(o + (E + 1) * 4, 256);
   s.tile_off = o;
   o = align_up(o + (E + 1) * 4, 256);
+  s.act_off = o;
+  o = align_up(o + E * 4, 256);
   s.perm = o;
   o = align_up(o + P * 4, 256);
-  const size_t rowH = std::max((size_t)(H / 32) * 34, (size_t)((H + 255) / 256) * 292);
-  const size_t rowI = std::max((size_t)(I / 32) * 34, (size_t)((I + 255) / 256) * 292);
+  const size_t act_rows = std::min(8 * P, P + 8 * E); // every expert's rows fill tiles of 8 of their own
   s.qx = o;
-  o = align_up(o + (T >= GROUPED_MIN_TOKENS ? (size_t)T * rowH : 0), 256);
+  o = align_up(o + (T >= GROUPED_MIN_TOKENS ? gemm_mma_workspace_bytes(NNTR_Q4_K, (unsigned)act_rows, H) : 0), 256);
   s.qact = o;
-  o = align_up(o + (T >= GROUPED_MIN_TOKENS ? P * rowI : 0), 256);
+  o = align_up(o + (T >= GROUPED_MIN_TOKENS ? gemm_mma_workspace_bytes(NNTR_Q4_K, (unsigned)act_rows, I) : 0), 256);
   s.total = o;
   return s;
 }
@@ -602,30 +673,28 @@ static int moe_forward(const nntr_moe_desc *d, const nntr_moe_ep *epd, unsigned 
   }
 
   if (!epd && tokens >= GROUPED_MIN_TOKENS) {
-    /* prefill: sort the pairs by expert, quantize every token's activation once, one grouped GEMM for gate and up,
-     * activation, quantize the activations, one grouped GEMM for down, combine. Same bits as the per-pair GEMVs. */
+    /* prefill: sort the pairs by expert, quantize every pair's activation into the tiles of its expert, one grouped GEMM
+     * for gate and up, activation and its quantization, one grouped GEMM for down, combine. Same bits as the per-pair
+     * GEMVs. */
     int *off = reinterpret_cast<int *>(ws + s.off), *tile_off = reinterpret_cast<int *>(ws + s.tile_off),
-        *perm = reinterpret_cast<int *>(ws + s.perm);
-    NNTR_CHECK_CUDA(launch_pdl(moe_permute_kernel, 1u, 1024u, st, idx, (int)P, (int)E, off, tile_off, perm));
+        *act_off = reinterpret_cast<int *>(ws + s.act_off), *perm = reinterpret_cast<int *>(ws + s.perm);
+    const int tile_rows = grouped_tile_rows(P, E);
+    NNTR_CHECK_CUDA(launch_pdl(moe_permute_kernel, 1u, 1024u, st, idx, (int)P, (int)E, tile_rows, off, tile_off, act_off,
+                               perm));
     count_launch();
-    const unsigned max_tiles = P / GROUPED_MT + E; // sum over experts of ceil(count / MT) <= P / MT + E
-    int rc2 = d->qtype == NNTR_Q4_K ? launch_quantize_q8_K(x, H, ws + s.qx, tokens, H, 0, st)
-                                    : launch_quantize_q8_0(x, H, ws + s.qx, tokens, H, st);
+    int rc2 = launch_act_tiles_grouped(d->qtype, x, P, H, ws + s.qx, perm, idx, off, act_off, (int)K, st);
     if (rc2)
       return rc2;
-    if ((rc2 = launch_gemm_grouped(d->qtype, I, H, ws + s.qx, gu, I, d->gate_w, d->up_w, off, tile_off, perm, (int)E,
-                                   (int)K, 2, max_tiles, st)))
+    if ((rc2 = launch_gemm_grouped(d->qtype, I, H, ws + s.qx, gu, I, d->gate_w, d->up_w, off, tile_off, act_off, perm, (int)E, 2,
+                                   tile_rows, P, st)))
       return rc2;
-    const long n_act2 = (long)P * I;
-    NNTR_CHECK_CUDA(launch_pdl(moe_act_kernel, (unsigned)((n_act2 + 255) / 256), 256, st, gu, act, idx, d->gate_b,
-                               d->up_b, d->kind, d->alpha, (int)I, n_act2, 0, (int)E));
+    const int nbI = (int)((I + 255) / 256);
+    NNTR_CHECK_CUDA(launch_pdl(d->qtype == NNTR_Q4_K ? moe_act_tiles_kernel<NNTR_Q4_K> : moe_act_tiles_kernel<NNTR_Q4_0>,
+                               (unsigned)(((long)P * nbI + 7) / 8), 256, st, gu, ws + s.qact, perm, idx, off, act_off,
+                               d->gate_b, d->up_b, d->kind, d->alpha, (int)I, nbI, (int)P));
     count_launch();
-    rc2 = d->qtype == NNTR_Q4_K ? launch_quantize_q8_K(act, I, ws + s.qact, P, I, 0, st)
-                                : launch_quantize_q8_0(act, I, ws + s.qact, P, I, st);
-    if (rc2)
-      return rc2;
-    if ((rc2 = launch_gemm_grouped(d->qtype, H, I, ws + s.qact, dn, H, d->down_w, nullptr, off, tile_off, perm, (int)E,
-                                   1, 1, max_tiles, st)))
+    if ((rc2 = launch_gemm_grouped(d->qtype, H, I, ws + s.qact, dn, H, d->down_w, nullptr, off, tile_off, act_off, perm, (int)E, 1,
+                                   tile_rows, P, st)))
       return rc2;
     const long n_out2 = (long)tokens * H;
     const cudaError_t e2 = launch_pdl(moe_combine_kernel, (unsigned)((n_out2 + 255) / 256), 256, st, dn, idx, ord, w,

@@ -1,0 +1,68 @@
+"""The integer warp-MMA GEMM (exact path of Q4_K and Q4_0 with more than one row) where its tiles end: rows and weight rows
+around multiples of 8, 16 and 32, units of 256 that do not divide by the eight warps of the K split, a short last unit of
+Q4_0, and the largest magnitudes a chain can meet. Every result must equal the checker's bit for bit, so no tolerance."""
+import numpy as np
+import pytest
+
+torch = pytest.importorskip("torch")
+pytestmark = pytest.mark.gpu
+
+from oracle import oracle as O  # noqa: E402
+
+
+@pytest.fixture(scope="module")
+def be():
+    if not torch.cuda.is_available():
+        pytest.skip("no CUDA device")
+    from nntrainer_b200 import backend, build
+    build.build()
+    backend.init(0)
+    yield backend
+    backend.set_gemm_path("auto")
+
+
+def exact(be, q, A, B, N):
+    M, K = A.shape
+    C = torch.full((M, N + 8), float("nan"), device="cuda")
+    be.set_gemm_path("exact")
+    getattr(be, f"gemm_{q}")(M, N, K, torch.from_numpy(A).cuda(), K, torch.from_numpy(B).cuda(), N, C, N + 8)
+    be.device_status()
+    got = C.cpu().numpy()
+    assert np.isnan(got[:, N:]).all()
+    return got[:, :N]
+
+
+# the first shapes run the K split, the wide ones (from about 1200 tiles of 16 rows) the kernel in which a warp owns its rows
+SHAPES = [(2, 8, 256), (7, 24, 2304), (8, 136, 2560), (9, 16, 4352), (17, 40, 768), (33, 24, 512), (3, 19000, 512),
+          (16, 19000, 256), (37, 19000, 768)]
+
+
+@pytest.mark.parametrize("M,N,K", SHAPES)
+@pytest.mark.parametrize("q,gen", [("q4_K", O.random_q4_Kx8), ("q4_0", O.random_q4_0x8)])
+def test_tile_edges(be, port, q, gen, M, N, K):
+    if q == "q4_0":
+        K += 96  # a last unit of three 32-blocks
+    rng = np.random.default_rng(M * 1000 + N + K)
+    A = rng.standard_normal((M, K)).astype(np.float32)
+    A[1, :256] = 0.0
+    A[0, :256] = np.where(np.arange(256) % 2 == 0, -2.5, 2.5)  # -amax first: the two quantizers' sign rules part
+    B = gen(rng, N, K)
+    want = port.gemm(q, A, B, N)
+    assert np.array_equal(exact(be, q, A, B, N).view(np.uint32), want.view(np.uint32))
+
+
+@pytest.mark.parametrize("M", [4, 6])
+def test_largest_sums(be, port, M):
+    """All nibbles 15, all scales and mins 63, activations all +-amax: sums of a super-block beyond 2^24, where the
+    one-step chain (the last M % 4 rows) rounds them once."""
+    N, K = 16, 512
+    block = np.zeros(1152, dtype=np.uint8)
+    block[:32] = np.full(16, 0x2000 + 7, dtype=np.uint16).view(np.uint8)  # d, dmin: small odd fp16 values
+    block[32:128] = 0xff
+    block[128:] = 0xff
+    B = np.tile(block, N // 8 * (K // 256))
+    A = np.full((M, K), 3.0, dtype=np.float32)
+    A[:, 5] = 2.99  # 126 or 127 steps: odd sums
+    A[M - 1, 256:] *= -1
+    want = port.gemm("q4_K", A, B, N)
+    assert np.array_equal(exact(be, "q4_K", A, B, N).view(np.uint32), want.view(np.uint32))
