@@ -299,7 +299,8 @@ static size_t workspace_bytes(int qtype, unsigned M, unsigned N, unsigned K) {
     const size_t rows0 = gemm_mma_workspace_bytes(qtype, M, K);
     return umma_f16_supported(qtype, M, N, K) ? std::max(rows0, umma_f16_workspace_bytes(M, K)) : rows0;
   }
-  const size_t rows = (size_t)(qtype == NNTR_Q4_K ? (M + 7) / 8 * 8 : M) * (K / 256) * sizeof(BlockQ8K); // Q4_K: tiles of 8 rows
+  const size_t rows = qtype == NNTR_Q6_K ? gemm_mma_q6_K_workspace_bytes(M, K)
+                                         : (size_t)((M + 7) / 8 * 8) * (K / 256) * sizeof(BlockQ8K); // tiles of 8 rows
   // large enough for every path the setting may select at call time
   size_t need = rows;
   if (umma_supported(qtype, M, N, K))
@@ -348,9 +349,7 @@ static int gemm_dev(int qtype, unsigned M, unsigned N, unsigned K, const float *
   }
   if (qtype != NNTR_Q6_K)
     return launch_gemm_mma(qtype, M, M / 4 * 4, N, K, A, B, C, ldc, ws, ws_bytes, st);
-  if ((rc = launch_quantize_q8_K(A, K, ws, M, K, 0, st))) // ggml_interface_omp.cpp:545-551: row quantizer for all rows
-    return rc;
-  return launch_gemm_q6_K(M, N, K, ws, B, C, ldc, st);
+  return launch_gemm_mma_q6_K(M, N, K, A, B, C, ldc, ws, st);
 }
 
 static int gemm_host(int qtype, unsigned M, unsigned N, unsigned K, const float *A, const void *B, float *C,
@@ -527,6 +526,8 @@ int nntr_cuda_device_status(void) {
     return rc;
   if (!v && (rc = read_mma_status(&v)))
     return rc;
+  if (!v && (rc = read_q6m_status(&v)))
+    return rc;
   if (v)
     return set_error(v, "a device kernel gave up on a bounded wait (status %d)", v);
   if ((rc = read_embed_status(&v, false)))
@@ -543,7 +544,7 @@ int clear_device_status_words() {
   int rc;
   if ((rc = clear_device_status()) || (rc = clear_umma_status()) || (rc = clear_q6_status()) ||
       (rc = clear_moe_status()) || (rc = clear_q40_status()) || (rc = clear_f16_status()) || (rc = clear_resident_status()) ||
-      (rc = clear_attn_status()) || (rc = clear_mma_status()))
+      (rc = clear_attn_status()) || (rc = clear_mma_status()) || (rc = clear_q6m_status()))
     return rc;
   return NNTR_CUDA_OK;
 }

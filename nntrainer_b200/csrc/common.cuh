@@ -343,8 +343,12 @@ int launch_gemm_f16(int qtype, unsigned M, unsigned N, unsigned K, const float *
 int read_f16_status(int *out);
 /* dense int8 tensor-core rate of the current device, measured (umma_peak.cu) */
 int measure_int8_peak(double *tops_out, double *clk_per_mma_out);
-int launch_gemm_q6_K(unsigned M, unsigned N, unsigned K, const void *qa, const void *B, float *C, unsigned ldc,
-                     cudaStream_t st);
+/* bit-exact GEMM of Q6_K weights (gemm_mma_q6k.cu): quantizes the fp32 activations itself, into ws */
+int read_q6m_status(int *out);
+int clear_q6m_status();
+size_t gemm_mma_q6_K_workspace_bytes(unsigned M, unsigned K);
+int launch_gemm_mma_q6_K(unsigned M, unsigned N, unsigned K, const float *A, const void *B, float *C, unsigned ldc, void *ws,
+                         cudaStream_t st);
 /* per-expert grouped GEMM of the MoE prefill (gemm_mma.cu): (token, expert) pairs sorted by expert, position p of the
  * order being pair perm[p]; expert e has the positions off[e] .. off[e+1], the tiles tile_off[e] .. of tile_rows rows each
  * and the activation tiles act_off[e] .. of 8 rows each (rows: perm[p] / a_div of x); output row perm[p] * c_mul (+ 1 for

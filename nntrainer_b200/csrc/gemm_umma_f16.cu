@@ -13,7 +13,7 @@
  * in half precision, a as fp16(d_a * q8)) and the products are summed in fp32 by
  * the tensor core. Measured against the reference chain on random-byte weights:
  * max-rel 3.5e-4 (bar 2e-3). This is the fast prefill path; the integer-exact
- * tensor path (gemm_umma.cu) and the bit-exact path (gemm_mma.cu, gemm_dp4a.cu)
+ * tensor path (gemm_umma.cu) and the bit-exact path (gemm_mma.cu, gemm_mma_q6k.cu)
  * stay selectable. Q4_0 weights (nntr_gemm_q4_0_8x8_q8_0, nntr_ggml_impl.cpp:650-3259) take the same route:
  * w = (q4 - 8) * d as one half-precision multiply, a = fp16(fp32(d_a) * q8) with the Q8_0 quantizer, a stage of 64
  * being two 32-weight blocks; their 32-element block scale would force an integer kernel to leave the tensor pipe at

@@ -1,8 +1,7 @@
 // SPDX-License-Identifier: Apache-2.0
 /**
- * @file  gemm_dp4a.cu
- * @brief Kernels on CUDA cores (dp4a): the decode GEMV of Q4_0 for shapes the streaming kernel does not take, and the
- *        bit-exact GEMM / GEMV of Q6_K.
+ * @file  gemv_dp4a.cu
+ * @brief Decode GEMVs on CUDA cores (dp4a) of Q4_0 and Q6_K, for the shapes that the streaming kernels do not take.
  *
  * They reproduce the reference's per-output float chains exactly:
  *   Q4_0  one fused multiply-add per 32-block (nntr_ggml_impl.cpp:9751-9753).
@@ -10,13 +9,9 @@
  *         lane l), fused multiply-add per super-block, fixed pairwise final sum
  *         (nntr_vec_dot_q6_K_q8_K, :8600-8696; nntr_ggml_impl_utils.h:59-65).
  *
- * Work split: one warp per (group of 8 output rows, tile of MT activation
- * rows); it walks K in units of 256 weights, keeps the unit's weights in
- * registers across the MT activation rows, and runs the chains in the lanes
- * 0-7 (one per output row). Lane (r = lane%8, c = lane/8) computes the integer
- * sums of quarter c of the unit for row r. Activations are plain block_q8_K
- * rows in global memory (M > 1, written by the quantizer kernel) or
- * quantized by the CTA itself into shared memory (M == 1).
+ * Work split: one warp per group of 8 output rows; it walks K in units of 256 weights and runs the chains in the lanes
+ * 0-7 (one per output row). Lane (r = lane%8, c = lane/8) computes the integer sums of quarter c of the unit for row r.
+ * The CTA quantizes the activation into shared memory first.
  */
 #include <cstdlib>
 
@@ -25,7 +20,6 @@
 namespace nntr {
 
 constexpr int DP_WARPS = 8; // warps per CTA
-constexpr int MT = 4;       // activation rows per warp pass
 
 __device__ __forceinline__ uint32_t ld_u32_a2(const uint8_t *p) { // 2-byte aligned 32-bit load
   const uint16_t *h = reinterpret_cast<const uint16_t *>(p);
@@ -137,48 +131,34 @@ gemv_q4_0_dp4a_kernel(const float *__restrict__ x, const BlockQ40x8 *__restrict_
 }
 
 /* ------------------------------------------------------------------ Q6_K */
-/* Activations: plain block_q8_K rows. When x_f32 != nullptr (M == 1) the CTA
- * first quantizes x into shared memory. Rows of W are plain block_q6_K rows
+/* The CTA first quantizes x into shared memory (plain block_q8_K layout). Rows of W are plain block_q6_K rows
  * (210-byte blocks, 2-byte aligned). */
 __global__ void __launch_bounds__(DP_WARPS * 32)
-gemm_q6_K_dp4a_kernel(const float *__restrict__ x_f32, const uint8_t *__restrict__ qa_g,
-                      const uint8_t *__restrict__ W, float *__restrict__ C, int ldc, int M, int N, int nb) {
+gemv_q6_K_dp4a_kernel(const float *__restrict__ x, const uint8_t *__restrict__ W, float *__restrict__ y, int N, int nb) {
   extern __shared__ __align__(16) uint8_t dp_smem[];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const uint8_t *qa = qa_g;
-  if (x_f32) {
-    for (int b = warp; b < nb; b += DP_WARPS) {
-      const float *src = x_f32 + b * QK_K + lane * 8;
-      const Q8KLane q = q8K_quantize_warp(*reinterpret_cast<const float4 *>(src),
-                                          *reinterpret_cast<const float4 *>(src + 4), lane, 0);
-      BlockQ8K *out = reinterpret_cast<BlockQ8K *>(dp_smem) + b;
-      uint32_t *qs = reinterpret_cast<uint32_t *>(out->qs);
-      qs[lane * 2] = q.w0;
-      qs[lane * 2 + 1] = q.w1;
-      const int s16 = q.sum8 + __shfl_xor_sync(FULL, q.sum8, 1);
-      if (!(lane & 1))
-        out->bsums[lane >> 1] = (int16_t)s16;
-      if (lane == 0)
-        out->d = q.d;
-    }
-    __syncthreads();
-    qa = dp_smem;
+  for (int b = warp; b < nb; b += DP_WARPS) {
+    const float *src = x + b * QK_K + lane * 8;
+    const Q8KLane q = q8K_quantize_warp(*reinterpret_cast<const float4 *>(src), *reinterpret_cast<const float4 *>(src + 4),
+                                        lane, 0);
+    BlockQ8K *out = reinterpret_cast<BlockQ8K *>(dp_smem) + b;
+    uint32_t *qs = reinterpret_cast<uint32_t *>(out->qs);
+    qs[lane * 2] = q.w0;
+    qs[lane * 2 + 1] = q.w1;
+    if (lane == 0)
+      out->d = q.d;
   }
+  __syncthreads();
   const int r = lane & 7, c = lane >> 3;
-  const int n_groups = (N + 7) / 8;
-  const int m_tiles = (M + MT - 1) / MT;
-  const long task = (long)blockIdx.x * DP_WARPS + warp;
-  if (task >= (long)n_groups * m_tiles)
+  const int g = (int)blockIdx.x * DP_WARPS + warp;
+  if (g * 8 >= N)
     return;
-  const int g = (int)(task / m_tiles), m0 = (int)(task % m_tiles) * MT;
   const int n = g * 8 + r;
   const bool row_ok = n < N;
-  float acc[MT][8];
+  float acc[8];
 #pragma unroll
-  for (int i = 0; i < MT; ++i)
-#pragma unroll
-    for (int l = 0; l < 8; ++l)
-      acc[i][l] = 0.f;
+  for (int l = 0; l < 8; ++l)
+    acc[l] = 0.f;
   for (int b = 0; b < nb; ++b) {
     const uint8_t *blk = W + ((size_t)(row_ok ? n : 0) * nb + b) * sizeof(BlockQ6K);
     // the lane's two 32-element chunks: ch = 2c, 2c+1; chunk ch = (half h = ch/4, quarter w = ch%4)
@@ -199,49 +179,36 @@ gemm_q6_K_dp4a_kernel(const float *__restrict__ x_f32, const uint8_t *__restrict
       sc[s][1] = scp[1];
     }
     const float dw = half_bits_to_float(*reinterpret_cast<const uint16_t *>(blk + 208));
+    const uint8_t *a = dp_smem + (size_t)b * sizeof(BlockQ8K);
+    int part[8];
 #pragma unroll
-    for (int i = 0; i < MT; ++i) {
-      const int m = m0 + i;
-      if (m >= M)
-        break;
-      const uint8_t *a = qa + ((size_t)m * nb + b) * sizeof(BlockQ8K);
-      int part[8];
+    for (int l = 0; l < 8; ++l)
+      part[l] = 0;
 #pragma unroll
-      for (int l = 0; l < 8; ++l)
-        part[l] = 0;
+    for (int s = 0; s < 2; ++s) {
+      const uint32_t *aw = reinterpret_cast<const uint32_t *>(a + 4 + 32 * (2 * c + s));
 #pragma unroll
-      for (int s = 0; s < 2; ++s) {
-        const uint32_t *aw = reinterpret_cast<const uint32_t *>(a + 4 + 32 * (2 * c + s));
-#pragma unroll
-        for (int l = 0; l < 8; ++l) {
-          const uint32_t av = aw[l];
-          const int dot = dp4a_us_(v[s][l], av, 0) - 32 * __dp4a(0x01010101, (int)av, 0);
-          part[l] += sc[s][l >> 2] * dot;
-        }
-      }
-#pragma unroll
-      for (int l = 0; l < 8; ++l) { // sum over the four quarters of the super-block
-        part[l] += __shfl_xor_sync(FULL, part[l], 8);
-        part[l] += __shfl_xor_sync(FULL, part[l], 16);
-      }
-      if (lane < 8) {
-        const float d = __fmul_rn(*reinterpret_cast<const float *>(a), dw);
-#pragma unroll
-        for (int l = 0; l < 8; ++l)
-          acc[i][l] = __fmaf_rn(d, (float)part[l], acc[i][l]);
+      for (int l = 0; l < 8; ++l) {
+        const uint32_t av = aw[l];
+        const int dot = dp4a_us_(v[s][l], av, 0) - 32 * __dp4a(0x01010101, (int)av, 0);
+        part[l] += sc[s][l >> 2] * dot;
       }
     }
-  }
-  if (lane < 8 && row_ok) {
 #pragma unroll
-    for (int i = 0; i < MT; ++i)
-      if (m0 + i < M) {
-        const float *a = acc[i];
-        const float s = __fadd_rn(__fadd_rn(__fadd_rn(a[4], a[0]), __fadd_rn(a[6], a[2])),
-                                  __fadd_rn(__fadd_rn(a[5], a[1]), __fadd_rn(a[7], a[3])));
-        C[(size_t)(m0 + i) * ldc + n] = s;
-      }
+    for (int l = 0; l < 8; ++l) { // sum over the four quarters of the super-block
+      part[l] += __shfl_xor_sync(FULL, part[l], 8);
+      part[l] += __shfl_xor_sync(FULL, part[l], 16);
+    }
+    if (lane < 8) {
+      const float d = __fmul_rn(*reinterpret_cast<const float *>(a), dw);
+#pragma unroll
+      for (int l = 0; l < 8; ++l)
+        acc[l] = __fmaf_rn(d, (float)part[l], acc[l]);
+    }
   }
+  if (lane < 8 && row_ok)
+    y[n] = __fadd_rn(__fadd_rn(__fadd_rn(acc[4], acc[0]), __fadd_rn(acc[6], acc[2])),
+                     __fadd_rn(__fadd_rn(acc[5], acc[1]), __fadd_rn(acc[7], acc[3])));
 }
 
 /* ---------------------------------------------------------------- launchers */
@@ -251,19 +218,6 @@ static int set_smem_attr(const void *fn, size_t bytes) {
   if (bytes > 48 * 1024)
     NNTR_CHECK_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes));
   return NNTR_CUDA_OK;
-}
-
-int launch_gemm_q6_K(unsigned M, unsigned N, unsigned K, const void *qa, const void *B, float *C, unsigned ldc,
-                     cudaStream_t st) {
-  const int nb = (int)(K / QK_K);
-  const long tasks = (long)((N + 7) / 8) * ((M + MT - 1) / MT);
-  if (tasks == 0)
-    return NNTR_CUDA_OK;
-  gemm_q6_K_dp4a_kernel<<<grid_for(tasks), DP_WARPS * 32, 0, st>>>(nullptr, static_cast<const uint8_t *>(qa),
-                                                                   static_cast<const uint8_t *>(B), C, (int)ldc, (int)M,
-                                                                   (int)N, nb);
-  count_launch();
-  return check_cuda(cudaGetLastError(), "gemm_q6_K launch");
 }
 
 int launch_gemv_q4_0(unsigned N, unsigned K, const float *x, const void *B, float *y, unsigned flags, cudaStream_t st) {
@@ -312,11 +266,11 @@ int launch_gemv_q6_K(unsigned N, unsigned K, const float *x, const void *B, floa
   const size_t smem = (size_t)(K / QK_K) * sizeof(BlockQ8K) + 16;
   if (smem > 200 * 1024)
     return set_error(NNTR_CUDA_ERR_UNSUPPORTED, "gemv_q6_K: K=%u too large", K);
-  int rc = set_smem_attr(reinterpret_cast<const void *>(gemm_q6_K_dp4a_kernel), smem);
+  int rc = set_smem_attr(reinterpret_cast<const void *>(gemv_q6_K_dp4a_kernel), smem);
   if (rc)
     return rc;
-  gemm_q6_K_dp4a_kernel<<<grid_for((N + 7) / 8), DP_WARPS * 32, smem, st>>>(x, nullptr, static_cast<const uint8_t *>(B),
-                                                                           y, (int)N, 1, (int)N, (int)(K / QK_K));
+  gemv_q6_K_dp4a_kernel<<<grid_for((N + 7) / 8), DP_WARPS * 32, smem, st>>>(x, static_cast<const uint8_t *>(B), y, (int)N,
+                                                                           (int)(K / QK_K));
   count_launch();
   return check_cuda(cudaGetLastError(), "gemv_q6_K launch");
 }

@@ -36,7 +36,7 @@
  * not by HBM. Algorithmic bytes per launch: N * nb * 210 (weights) + 4K (x) +
  * 4N (y). Rows beyond the last whole stage form one short stage for the last
  * CTA when their byte size is a multiple of 16; otherwise they are left to the
- * caller (the dp4a kernel of gemm_dp4a.cu takes them).
+ * caller (the dp4a kernel of gemv_dp4a.cu takes them).
  */
 #include "common.cuh"
 #include "pipeline.cuh"

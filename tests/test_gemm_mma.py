@@ -1,4 +1,4 @@
-"""The integer warp-MMA GEMM (exact path of Q4_K and Q4_0 with more than one row) where its tiles end: rows and weight rows
+"""The warp-MMA GEMMs (exact path with more than one row) where its tiles end: rows and weight rows
 around multiples of 8, 16 and 32, units of 256 that do not divide by the eight warps of the K split, a short last unit of
 Q4_0, and the largest magnitudes a chain can meet. Every result must equal the checker's bit for bit, so no tolerance."""
 import numpy as np
@@ -49,6 +49,29 @@ def test_tile_edges(be, port, q, gen, M, N, K):
     B = gen(rng, N, K)
     want = port.gemm(q, A, B, N)
     assert np.array_equal(exact(be, q, A, B, N).view(np.uint32), want.view(np.uint32))
+
+
+@pytest.mark.parametrize("M,N,K", [(2, 1, 256), (7, 17, 768), (8, 130, 2560), (9, 33, 512), (31, 4097, 2304)])
+def test_tile_edges_q6_K(be, port, M, N, K):
+    """Rows of 210-byte blocks at every alignment (odd and even blocks per row), N that ends inside a tile of 16."""
+    rng = np.random.default_rng(M + N + K)
+    A = rng.standard_normal((M, K)).astype(np.float32)
+    A[1, :256] = 0.0
+    B = O.random_q6_K(rng, N, K)
+    assert np.array_equal(exact(be, "q6_K", A, B, N).view(np.uint32), port.gemm("q6_K", A, B, N).view(np.uint32))
+
+
+def test_largest_sums_q6_K(be, port):
+    """Every 6-bit value -32, every scale -128: the integers of the chain reach 32 * 32 * 128 * 127, just under 2^24."""
+    N, K = 5, 512
+    block = np.zeros(210, dtype=np.uint8)
+    block[192:208] = 0x80
+    block[208:] = np.full(1, 0x2000 + 7, dtype=np.uint16).view(np.uint8)
+    B = np.tile(block, N * (K // 256))
+    A = np.full((3, K), 3.0, dtype=np.float32)
+    A[:, 5] = 2.99
+    A[2, 256:] *= -1
+    assert np.array_equal(exact(be, "q6_K", A, B, N).view(np.uint32), port.gemm("q6_K", A, B, N).view(np.uint32))
 
 
 @pytest.mark.parametrize("M", [4, 6])
