@@ -23,6 +23,9 @@
  *
  * Cache layout as the reference's: [row][kv head][head_dim] fp16, one row per position.
  */
+#include <atomic>
+#include <cstring>
+
 #include <cuda.h>
 
 #include "common.cuh"
@@ -72,6 +75,47 @@ __device__ __forceinline__ void rope_head(const float *__restrict__ src, const f
     st[kk + half] = __fadd_rn(__fmul_rn(a0, s), __fmul_rn(a1, c));
   }
   __syncwarp();
+}
+
+/* The same for heads of 32 * NE dimensions (64, 128): a lane's NE elements lane + 32 k are both what it adds up for the norm
+ * and whole rotary pairs, so everything stays in registers and all loads are issued at once. */
+template <int NE>
+__device__ __forceinline__ void rope_head_regs(const float *__restrict__ src, const float *__restrict__ gamma, float eps,
+                                               const float *__restrict__ ct, const float *__restrict__ sn, int lane, float *st) {
+  float x[NE], gm[NE], c[NE / 2], sv[NE / 2];
+#pragma unroll
+  for (int k = 0; k < NE; ++k)
+    x[k] = src[lane + 32 * k];
+#pragma unroll
+  for (int k = 0; k < NE / 2; ++k) {
+    c[k] = ct[lane + 32 * k];
+    sv[k] = sn[lane + 32 * k];
+  }
+  if (gamma) {
+#pragma unroll
+    for (int k = 0; k < NE; ++k)
+      gm[k] = gamma[lane + 32 * k];
+    float acc = 0.f;
+#pragma unroll
+    for (int k = 0; k < NE; ++k)
+      acc = __fmaf_rn(x[k], x[k], acc);
+    float t = __fadd_rn(acc, __shfl_down_sync(FULL, acc, 4));
+    t = __fadd_rn(t, __shfl_down_sync(FULL, t, 1));
+    t = __fadd_rn(t, __shfl_down_sync(FULL, t, 2));
+    const float h0 = __shfl_sync(FULL, t, 0), h1 = __shfl_sync(FULL, t, 8), h2 = __shfl_sync(FULL, t, 16),
+                h3 = __shfl_sync(FULL, t, 24);
+    const float sumsq = __fadd_rn(__fadd_rn(__fadd_rn(h0, h1), h2), h3);
+    const float scale = __fdiv_rn(1.0f, __fsqrt_rn(__fadd_rn(__fdiv_rn(sumsq, (float)(32 * NE)), eps)));
+#pragma unroll
+    for (int k = 0; k < NE; ++k)
+      x[k] = __fmul_rn(__fmul_rn(x[k], scale), gm[k]);
+  }
+#pragma unroll
+  for (int k = 0; k < NE / 2; ++k) {
+    const float a0 = x[k], a1 = x[k + NE / 2];
+    st[lane + 32 * k] = __fsub_rn(__fmul_rn(a0, c[k]), __fmul_rn(a1, sv[k]));
+    st[lane + 32 * (k + NE / 2)] = __fadd_rn(__fmul_rn(a0, sv[k]), __fmul_rn(a1, c[k]));
+  }
 }
 
 /* One warp per head (query heads, then key heads, then value heads). Optional per-head RMS norm first
@@ -124,7 +168,7 @@ __global__ void rope_cache_append_kernel(float *__restrict__ q, const float *__r
 constexpr int SCORE_WARPS = 4;
 __global__ void attn_scores_kernel(const float *__restrict__ q, const uint16_t *__restrict__ kcache,
                                    float *__restrict__ scores, const unsigned *__restrict__ pos_dev, unsigned pos,
-                                   int hq, int hkv, int hd, unsigned window, unsigned head_stride) {
+                                   int hq, int hkv, int hd, unsigned window) {
   extern __shared__ __align__(16) uint8_t smem_raw[];
   pdl_launch_dependents(); // the next kernel may start its own prologue; it waits before it reads
   pdl_wait();
@@ -167,91 +211,7 @@ __global__ void attn_scores_kernel(const float *__restrict__ q, const uint16_t *
     s = __fadd_rn(s, __shfl_down_sync(FULL, s, 2));
     if (l == 0 && t0 + j < row_cnt) {
       const float sum = __fadd_rn(0.0f, s);
-      // head_stride != 0: head-major [head][head_stride] (what the fused softmax + values kernel reads, one head per
-      // CTA, contiguously); else the reference's [row][head]
-      const size_t at = head_stride ? (size_t)(n * gqa + g) * head_stride + t0 + j : (size_t)(t0 + j) * hq + n * gqa + g;
-      scores[at] = (float)((double)sum / norm);
-    }
-  }
-}
-
-/* The rotary launch folded into the scores launch (short windows, head-major scores for attn_softmax_values_kernel):
- * every CTA normalises and rotates the raw query heads of its group for itself (four warps, a few hundred operations:
- * far cheaper than a launch and a trip through memory); the one warp whose four cache rows include the token's own row
- * computes the new key row, stores it to the cache AND uses it, and converts the token's value row into the cache.
- * q_rot, when not null, receives the rotated query heads (written by the CTAs of the first row tile). Same bits as
- * rope_cache_append_kernel + attn_scores_kernel. */
-__global__ void attn_rope_scores_kernel(const float *__restrict__ q, const float *__restrict__ k,
-                                        const float *__restrict__ v, const float *__restrict__ q_gamma,
-                                        const float *__restrict__ k_gamma, float eps, uint16_t *__restrict__ kcache,
-                                        uint16_t *__restrict__ vcache, const float *__restrict__ cos_tab,
-                                        const float *__restrict__ sin_tab, float *__restrict__ q_rot,
-                                        float *__restrict__ scores, const unsigned *__restrict__ pos_dev, unsigned pos,
-                                        int hq, int hkv, int hd, unsigned window, unsigned head_stride) {
-  extern __shared__ __align__(16) uint8_t smem_raw[];
-  pdl_launch_dependents();
-  pdl_wait();
-  const unsigned p = pos_dev ? *pos_dev : pos;
-  const unsigned num_rows = p + 1;
-  const unsigned start_row = num_rows < window ? 0u : num_rows - window;
-  const unsigned row_cnt = num_rows < window ? num_rows : window;
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int n = blockIdx.y;
-  const int gqa = hq / hkv;
-  if (blockIdx.x * SCORE_WARPS * 4 >= row_cnt)
-    return;
-  float *qs = reinterpret_cast<float *>(smem_raw);                                    // [gqa][hd]
-  uint16_t *kall = reinterpret_cast<uint16_t *>(smem_raw + (size_t)gqa * hd * 4);     // [16][hd]
-  float *ktmp = reinterpret_cast<float *>(smem_raw + (size_t)gqa * hd * 4 + (size_t)SCORE_WARPS * 4 * hd * 2) +
-                (size_t)warp * hd;                                                     // [SCORE_WARPS][hd]
-  const float *ct = cos_tab + (size_t)p * hd, *sn = sin_tab + (size_t)p * hd;
-  for (int g = warp; g < gqa; g += SCORE_WARPS) {
-    rope_head(q + (size_t)(n * gqa + g) * hd, q_gamma, eps, ct, sn, hd, lane, qs + (size_t)g * hd);
-    if (q_rot && blockIdx.x == 0)
-      for (int e = lane; e < hd; e += 32)
-        q_rot[(size_t)(n * gqa + g) * hd + e] = qs[(size_t)g * hd + e];
-  }
-  const unsigned t0 = (blockIdx.x * SCORE_WARPS + warp) * 4;
-  uint16_t *ks = kall + (size_t)warp * 4 * hd;
-  const int chunks_per_row = hd / 8;
-  const unsigned own = p - start_row; // the token's own row, window-relative (the last one)
-  for (int c = lane; c < 4 * chunks_per_row; c += 32) {
-    const int r = c / chunks_per_row, cc = c - r * chunks_per_row;
-    uint4 vv = make_uint4(0, 0, 0, 0);
-    if (t0 + r < row_cnt && t0 + r != own)
-      vv = *reinterpret_cast<const uint4 *>(kcache + ((size_t)(start_row + t0 + r) * hkv + n) * hd + cc * 8);
-    *reinterpret_cast<uint4 *>(ks + (size_t)r * hd + cc * 8) = vv;
-  }
-  if (own >= t0 && own < t0 + 4) { // this warp appends the token's key and value rows of kv head n
-    __syncwarp();
-    rope_head(k + (size_t)n * hd, k_gamma, eps, ct, sn, hd, lane, ktmp);
-    uint16_t *krow = kcache + ((size_t)p * hkv + n) * hd, *vrow = vcache + ((size_t)p * hkv + n) * hd;
-    for (int e = lane; e < hd; e += 32) {
-      const uint16_t kb = float_to_half_bits_rn(ktmp[e]);
-      krow[e] = kb;
-      ks[(size_t)(own - t0) * hd + e] = kb;
-      vrow[e] = float_to_half_bits_rn(v[(size_t)n * hd + e]);
-    }
-  }
-  __syncthreads();
-  if (t0 >= row_cnt)
-    return;
-  const int j = lane >> 3, l = lane & 7;
-  const uint16_t *kr = ks + (size_t)j * hd;
-  const double norm = sqrt((double)(float)hd);
-  for (int g = 0; g < gqa; ++g) {
-    const float *qh = qs + (size_t)g * hd;
-    float acc = 0.f;
-#pragma unroll 8
-    for (int i = 0; i < hd; i += 8)
-      acc = __fmaf_rn(qh[i + l], half_bits_to_float(kr[i + l]), acc);
-    float s = __fadd_rn(acc, __shfl_down_sync(FULL, acc, 4));
-    s = __fadd_rn(s, __shfl_down_sync(FULL, s, 1));
-    s = __fadd_rn(s, __shfl_down_sync(FULL, s, 2));
-    if (l == 0 && t0 + j < row_cnt) {
-      const float sum = __fadd_rn(0.0f, s);
-      const size_t at = head_stride ? (size_t)(n * gqa + g) * head_stride + t0 + j : (size_t)(t0 + j) * hq + n * gqa + g;
-      scores[at] = (float)((double)sum / norm);
+      scores[(size_t)(t0 + j) * hq + n * gqa + g] = (float)((double)sum / norm);
     }
   }
 }
@@ -457,143 +417,504 @@ __global__ void attn_values_kernel(const float *__restrict__ probs, const uint16
     out[(size_t)(n * gqa + h) * hd + d0 + lane] = acc;
 }
 
-/* Softmax and values in one launch, for windows of at most SV_MAX_ROWS rows. One CTA per query head, warp w = head
- * dimensions 32 w .. 32 w + 31. The scores arrive head-major, so the CTA reads its head's row contiguously. All warps
- * share the softmax (maximum, exponentials, the division), thread 0 adds the exponentials in ascending row order (the
- * reference's order), and meanwhile the first value tiles are on their way; then every thread runs its row-ordered
- * multiply-add chain over tiles of SVT rows of the kv head's values (the heads of a group read the same tiles from
- * L2). Same arithmetic and order as attn_softmax_kernel + attn_values_kernel. */
-constexpr unsigned SV_MAX_ROWS = 2048;
-constexpr int SVT = 128;  // rows per value tile
-constexpr int SVBUF = 3;  // tiles in the ring
-__device__ int g_attn_status = 0; // raised when a bounded wait for a value tile runs out
-__global__ void attn_softmax_values_kernel(const __grid_constant__ CUtensorMap vmap, const float *__restrict__ scores,
-                                           float *__restrict__ out, const float *__restrict__ sink,
-                                           const unsigned *__restrict__ pos_dev, unsigned pos, int hq, int hkv, int hd,
-                                           unsigned window, unsigned cap_rows) {
-  extern __shared__ __align__(128) uint8_t svsm[]; // the value tiles are TMA destinations: 128-byte aligned
-  __shared__ float red[8];
+/* ------------------------------------------------- the whole step in one launch */
+
+/* One cluster of CTAs per kv head (and up to eight of its query heads); everything a token's attention does for those heads
+ * stays inside it.
+ *   scores   every CTA normalises and rotates the group's query heads for itself (a few hundred operations per head) and
+ *            dots them against its share of the cache rows: key tiles by tiled TMA copies (128-byte swizzle, so that
+ *            thread = row reads its 16-byte pieces without bank conflicts), eight partial sums per (row, head) in the
+ *            thread. A score goes straight into the shared memory of the CTA(s) that own the head. The token's own row
+ *            comes from the inputs, rounded to fp16 as the cache holds it: the CTA that scores it patches it into its
+ *            tile and appends it to the caches.
+ *   softmax  a CTA owns one head (or 64 of its dimensions): maximum, exponentials and division by all threads, the sum in
+ *            ascending row order by one warp (ordered_sum).
+ *   values   a thread per dimension runs the row-ordered chain over value tiles that a producer warp keeps ahead of it
+ *            (tiled TMA copies, started before the scores).
+ * The chains are serial at four clocks per row; they bound the kernel for long contexts, launch and exchange latencies do
+ * for short ones: 64 / 8 heads of 64 at 4096 rows 48 us (four launches before: 120), 32 / 8 heads of 128 at 512 rows 11 us (two
+ * launches before: 15.7), at 128 rows of a window 7 us (10.8). Ring positions are counted, not divided: an integer division in a loop that one thread runs costs more than
+ * a tile's copy. */
+constexpr int AC_THREADS = 256;
+constexpr int AC_WARPS = AC_THREADS / 32;
+constexpr int AC_TILE = 128; // cache rows per tile of keys or values
+constexpr int AC_KBUF_MAX = 4;
+constexpr int AC_VBUF_MAX = 6;
+constexpr unsigned AC_MAX_ROWS = 16384; // rows of one head kept as floats in shared memory
+constexpr uint32_t AC_POLLS = 1u << 22;
+__device__ int g_attn_status = 0; // raised when a bounded wait for a tile runs out
+
+struct AttnStep {
+  const float *q, *k, *v, *q_gamma, *k_gamma;
+  float eps;
+  uint16_t *kcache, *vcache;
+  const float *cos_tab, *sin_tab;
+  float *q_rot, *q_inplace, *out;
+  const float *sink;
+  const unsigned *pos_dev;
+  unsigned pos, window, cap_rows;
+  int hq, hkv, hd;
+  int groups; // clusters per kv head: more than eight query heads per kv head are split over several
+  int rope;   // 0: q is rotated already and the token's rows are in the caches
+  int k_bufs, v_bufs;
+  int k_box, v_box; // rows a copy brings: a tile, fewer where one short tile is all there is
+};
+
+__device__ __forceinline__ void tma_tile(uint32_t dst, const CUtensorMap *map, int x, int y, uint32_t bar) {
+  asm volatile("cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];" ::"r"(dst),
+               "l"(reinterpret_cast<uint64_t>(map)), "r"(x), "r"(y), "r"(bar)
+               : "memory");
+}
+__device__ __forceinline__ uint32_t cluster_rank() {
+  uint32_t r;
+  asm("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
+  return r;
+}
+__device__ __forceinline__ uint32_t cluster_size() {
+  uint32_t r;
+  asm("mov.u32 %0, %%cluster_nctarank;" : "=r"(r));
+  return r;
+}
+/** store to the same shared-memory address of another CTA of the cluster */
+__device__ __forceinline__ void st_cluster(uint32_t addr, uint32_t rank, float v) {
+  uint32_t remote;
+  asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(remote) : "r"(addr), "r"(rank));
+  asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(remote), "f"(v) : "memory");
+}
+__device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory"); }
+__device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
+
+struct AcLayout {
+  uint32_t ktile, vtile, e, q, total; // offsets; the tiles are 1024-byte aligned
+};
+__host__ __device__ inline AcLayout ac_layout(int gqa, int hd, int dims, int k_bufs, int v_bufs, unsigned cap_rows) {
+  AcLayout L;
+  uint32_t o = 0;
+  L.ktile = o;
+  o += (uint32_t)k_bufs * (uint32_t)((hd + 63) / 64) * AC_TILE * 128;
+  L.vtile = o;
+  o += (uint32_t)v_bufs * AC_TILE * dims * 2;
+  L.e = o; // scores, exponentials, probabilities of whole tiles; a spare block so that the sum may read ahead
+  o += (cap_rows + AC_TILE - 1) / AC_TILE * AC_TILE * 4 + 1024;
+  L.q = o; // rotated query heads, then the new key head
+  o += (uint32_t)(gqa + 1) * hd * 4;
+  L.total = o + 1024;
+  return L;
+}
+
+/** Scores (not yet divided) of one thread's key row against the H query heads at qs: ascending groups of eight elements. */
+template <int H, int HD>
+__device__ __forceinline__ void dot_rows(const uint8_t *tile, int row, const float *qs, int hd, float (&sum)[H]) {
+  float acc[H][8];
+#pragma unroll
+  for (int h = 0; h < H; ++h)
+#pragma unroll
+    for (int l = 0; l < 8; ++l)
+      acc[h][l] = 0.f;
+#pragma unroll 8
+  for (int c = 0; c < (HD ? HD : hd) / 8; ++c) {
+    const uint4 w = *reinterpret_cast<const uint4 *>(tile + (c >> 3) * (AC_TILE * 128) + row * 128 + (((c & 7) ^ (row & 7)) << 4));
+    const uint32_t ws[4] = {w.x, w.y, w.z, w.w};
+    float kv[8];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const float2 f = __half22float2(*reinterpret_cast<const __half2 *>(&ws[i]));
+      kv[2 * i] = f.x;
+      kv[2 * i + 1] = f.y;
+    }
+#pragma unroll
+    for (int h = 0; h < H; ++h) {
+      const float4 a = *reinterpret_cast<const float4 *>(qs + h * hd + 8 * c),
+                   b = *reinterpret_cast<const float4 *>(qs + h * hd + 8 * c + 4);
+      const float qv[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
+#pragma unroll
+      for (int l = 0; l < 8; ++l)
+        acc[h][l] = __fmaf_rn(qv[l], kv[l], acc[h][l]);
+    }
+  }
+#pragma unroll
+  for (int h = 0; h < H; ++h)
+    sum[h] = __fadd_rn(__fadd_rn(__fadd_rn(acc[h][0], acc[h][4]), __fadd_rn(acc[h][1], acc[h][5])),
+                       __fadd_rn(__fadd_rn(acc[h][2], acc[h][6]), __fadd_rn(acc[h][3], acc[h][7])));
+}
+
+/** s + e[lo] + e[lo + 1] + ... + e[hi - 1], one rounded addition after the other; lo and hi multiples of 8, e may be read up
+ *  to hi + 63. */
+__device__ __forceinline__ float serial_sum(const float *e, unsigned lo, unsigned hi, float s) {
+  const float4 *e4 = reinterpret_cast<const float4 *>(e);
+  // thirty-two rows are added while the next thirty-two are on their way
+  float4 ev[2][8];
+#pragma unroll
+  for (int u = 0; u < 8; ++u)
+    ev[0][u] = e4[lo / 4 + u];
+  unsigned r = lo;
+  auto add32 = [&](float4(&cur)[8], float4(&nxt)[8]) {
+#pragma unroll
+    for (int u = 0; u < 8; ++u)
+      nxt[u] = e4[r / 4 + 8 + u];
+#pragma unroll
+    for (int u = 0; u < 8; ++u) {
+      s = __fadd_rn(s, cur[u].x);
+      s = __fadd_rn(s, cur[u].y);
+      s = __fadd_rn(s, cur[u].z);
+      s = __fadd_rn(s, cur[u].w);
+    }
+    r += 32;
+  };
+  for (; r + 64 <= hi;) {
+    add32(ev[0], ev[1]);
+    add32(ev[1], ev[0]);
+  }
+  if (r + 32 <= hi)
+    add32(ev[0], ev[1]);
+  for (; r < hi; r += 4) {
+    const float4 v = e4[r / 4];
+    s = __fadd_rn(s, v.x);
+    s = __fadd_rn(s, v.y);
+    s = __fadd_rn(s, v.z);
+    s = __fadd_rn(s, v.w);
+  }
+  return s;
+}
+
+/* The ordered sum of cnt values e >= 0 (cnt a multiple of 8) by one warp, with the bits of the serial chain. While the running sum s stays inside one
+ * power of two [2^k, 2^(k+1)) it is an integer multiple S of u = 2^(k-23), and adding e rounds e / u to an integer: to the
+ * nearest, and only for an exact half does the choice depend on S. So the integers of 256 rows are added in any order, eight rows
+ * per lane, and S + their sum is the serial result as long as it stays below 2^24 and no half occurred. Where one of the two
+ * happens, the lanes in front of the first such lane are taken, that lane's eight rows are added serially, and the next 256
+ * rows start behind them. That takes about 250 clocks per 256 rows or interruption against 1050 for the serial chain, and
+ * interruptions are few (a power of two is passed log2(rows) times; a half has probability e / s per row, so the first rows
+ * are added serially) -- after AC_SUM_STOPS of them the rest is added serially. */
+constexpr unsigned AC_SUM_SERIAL = 64;    // rows at the start
+constexpr unsigned AC_SUM_PARALLEL = 768; // below this many rows the serial chain is as fast
+constexpr int AC_SUM_STOPS = 40;
+__device__ __forceinline__ float ordered_sum(const float *e, unsigned cnt, float s, int lane) {
+  if (cnt < AC_SUM_PARALLEL)
+    return serial_sum(e, 0, cnt, s);
+  s = serial_sum(e, 0, AC_SUM_SERIAL, s);
+  unsigned r = AC_SUM_SERIAL;
+  int stops = 0;
+  while (r + 256 <= cnt && stops < AC_SUM_STOPS) {
+    const uint32_t ex = __float_as_uint(s) >> 23;
+    if (ex < 32) // too small for u to be a normal number
+      break;
+    const float inv_u = __uint_as_float((277u - ex) << 23), u = __uint_as_float((ex - 23u) << 23); // u = 2^(k - 23), k = ex - 127
+    const int S = (int)(s * inv_u);                         // in [2^23, 2^24)
+    const float4 a = *reinterpret_cast<const float4 *>(e + r + 8 * lane), b = *reinterpret_cast<const float4 *>(e + r + 8 * lane + 4);
+    const float v[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
+    int sum = 0;
+    bool half = false;
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+      const float x = fminf(v[i] * inv_u, 16777216.f); // exact, or far below one half
+      const int n = __float2int_rn(x);
+      half |= fabsf(x - (float)n) == 0.5f;
+      sum += n;
+    }
+    sum = min(sum, 1 << 24);
+    const int total = (int)__reduce_add_sync(FULL, (unsigned)sum);
+    if (S + total < (1 << 24) && !__any_sync(FULL, half)) {
+      s = (float)(S + total) * u;
+      r += 256;
+      continue;
+    }
+    int incl = sum;
+#pragma unroll
+    for (int d = 1; d < 32; d <<= 1) {
+      const int o = __shfl_up_sync(FULL, incl, d);
+      if (lane >= d)
+        incl += o;
+    }
+    const int stop = __ffs(__ballot_sync(FULL, half || S + incl >= (1 << 24))) - 1;
+    const int before = __shfl_sync(FULL, incl - sum, stop);
+    s = (float)(S + before) * u;
+    r += 8 * stop;
+#pragma unroll
+    for (int i = 0; i < 8; ++i)
+      s = __fadd_rn(s, e[r + i]);
+    r += 8;
+    ++stops;
+  }
+  return serial_sum(e, r, cnt, s);
+}
+
+template <int HD, int DIMS> // head_dim (0: a.hd), dimensions a CTA owns
+__global__ void __launch_bounds__(AC_THREADS, 1)
+attn_cluster_kernel(const __grid_constant__ CUtensorMap kmap, const __grid_constant__ CUtensorMap vmap,
+                    const __grid_constant__ AttnStep a) {
+  extern __shared__ uint8_t ac_raw[];
+  __shared__ __align__(8) unsigned long long kbar[AC_KBUF_MAX], vfull[AC_VBUF_MAX], vempty[AC_VBUF_MAX];
+  __shared__ float red[AC_WARPS];
   __shared__ float s_bcast;
-  __shared__ __align__(8) unsigned long long tile_bar[SVBUF];
   __shared__ int abort_word;
   volatile int *abort_flag = &abort_word;
-  if (threadIdx.x == 0) {
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int gqa = a.hq / a.hkv / a.groups, hd = HD ? HD : a.hd, per_head = (hd + DIMS - 1) / DIMS, items = gqa * per_head;
+  const uint32_t rank = cluster_rank(), csize = cluster_size();
+  const int cluster = (int)(blockIdx.x / csize), n = cluster / a.groups, h0 = cluster * gqa; // kv head, first query head
+  uint8_t *base = reinterpret_cast<uint8_t *>((reinterpret_cast<uintptr_t>(ac_raw) + 1023) & ~(uintptr_t)1023);
+  const AcLayout L = ac_layout(gqa, hd, DIMS, a.k_bufs, a.v_bufs, a.cap_rows);
+  uint8_t *ktile = base + L.ktile, *vtile = base + L.vtile;
+  float *e = reinterpret_cast<float *>(base + L.e), *qs = reinterpret_cast<float *>(base + L.q), *kown = qs + gqa * hd;
+  const int k_halves = (hd + 63) / 64;
+  const uint32_t kbytes = (uint32_t)k_halves * AC_TILE * 128, vbytes = AC_TILE * DIMS * 2; // of a buffer
+  const uint32_t ksm = smem_u32(ktile), vsm = smem_u32(vtile), esm = smem_u32(e);
+  const uint32_t kbar0 = smem_u32(kbar), vfull0 = smem_u32(vfull), vempty0 = smem_u32(vempty);
+  if (tid == 0) {
     abort_word = 0;
-    for (int i = 0; i < SVBUF; ++i)
-      mbar_init(smem_u32(&tile_bar[i]), 1);
+    for (int i = 0; i < a.k_bufs; ++i)
+      mbar_init(kbar0 + 8 * i, 1);
+    for (int i = 0; i < a.v_bufs; ++i) {
+      mbar_init(vfull0 + 8 * i, 1);
+      mbar_init(vempty0 + 8 * i, DIMS / 32);
+    }
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   __syncthreads();
+  cluster_arrive(); // "this CTA has started": waited for before the first store into another one
   pdl_launch_dependents();
   pdl_wait();
-  const unsigned row_num = pos_dev ? *pos_dev : pos;
-  const unsigned first = row_num < window ? 0u : row_num + 1 - window;
-  unsigned cnt = row_num + 1 - first;
-  if (cnt > cap_rows)
-    cnt = cap_rows; // the launch was sized for cap_rows (the scores kernel before it computed no more either)
-  const int gqa = hq / hkv;
-  const int c = blockIdx.x, n = c / gqa;
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nthreads = blockDim.x, nwarps = nthreads >> 5;
-  const int d = threadIdx.x;
-  // shared memory: probabilities [stride] f32 | ring of SVBUF value tiles [SVT][hd] f16
-  const unsigned p_stride = (cap_rows + 3u) & ~3u;
-  float *e = reinterpret_cast<float *>(svsm);
-  uint8_t *vring = svsm + (((size_t)p_stride * 4 + 127) & ~(size_t)127); // TMA destination: 128-byte aligned
-  const size_t vbytes = (size_t)SVT * hd * 2;
-  const uint32_t vbase = (uint32_t)__cvta_generic_to_shared(vring);
-  // One tiled TMA copy per tile: a box of SVT cache rows x head_dim values of kv head n out of the [row][kv head x
-  // head_dim] cache (rows of a head are 2 x hkv x head_dim bytes apart, so plain bulk copies would be one per row, and
-  // an SM accepts those far too slowly: measured 16 GB/s). The box's first coordinate, n * head_dim elements, is a
-  // multiple of 8 elements = 16 bytes. Rows of the box past the end of the cache arrive as zeros and are not used.
-  auto issue = [&](unsigned tile, int buf) {
-    if (threadIdx.x == 0) {
-      const uint32_t vdst = vbase + buf * (uint32_t)vbytes, bar = smem_u32(&tile_bar[buf]);
-      mbar_expect_tx(bar, (uint32_t)vbytes);
-      asm volatile("cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];"
-                   ::"r"(vdst), "l"(reinterpret_cast<uint64_t>(&vmap)), "r"(n * hd), "r"((int)(first + tile * SVT)), "r"(bar)
-                   : "memory");
-    }
+  const unsigned p = a.pos_dev ? *a.pos_dev : a.pos;
+  const unsigned first = p + 1 < a.window ? 0u : p + 1 - a.window;
+  unsigned cnt = p + 1 - first;
+  if (cnt > a.cap_rows)
+    cnt = a.cap_rows; // the launch was sized for cap_rows
+  const unsigned cached = a.rope ? cnt - 1 : cnt; // rows whose values are read from the cache
+  const unsigned share = (cnt + csize - 1) / csize, r_lo = min(rank * share, cnt), r_hi = min((rank + 1) * share, cnt);
+  const int item_head = (int)rank / per_head, item_d0 = ((int)rank % per_head) * DIMS;
+  const bool has_item = (int)rank < items, has_own = a.rope && r_lo < cnt && r_hi == cnt;
+  const bool append = has_own && cluster % a.groups == 0; // one cluster per kv head appends the token's rows
+  const unsigned k_tiles = (r_hi - r_lo + AC_TILE - 1) / AC_TILE, v_tiles = (cached + AC_TILE - 1) / AC_TILE;
+  auto issue_k = [&](unsigned t, int buf) {
+    const uint32_t bar = kbar0 + 8 * buf;
+    mbar_expect_tx(bar, (uint32_t)(k_halves * a.k_box) * 128);
+    for (int h = 0; h < k_halves; ++h)
+      tma_tile(ksm + buf * kbytes + h * (AC_TILE * 128), &kmap, n * hd + 64 * h, (int)(first + r_lo + t * AC_TILE), bar);
   };
-  const unsigned n_tiles = (cnt + SVT - 1) / SVT;
-  for (int t = 0; t < SVBUF - 1; ++t)
-    if ((unsigned)t < n_tiles)
-      issue(t, t);
-  // ---- softmax of head c by the whole CTA (attn_softmax_kernel's steps)
-  {
-    const float *sr = scores + (size_t)c * p_stride; // head-major, stride = the launch's row bound rounded up to 4
-    float mx = -INFINITY;
-    for (unsigned r = threadIdx.x; r < cnt; r += nthreads) {
-      const float v = sr[r];
-      e[r] = v;
-      mx = fmaxf(mx, v);
-    }
+  auto issue_v = [&](unsigned t, int buf) {
+    const uint32_t bar = vfull0 + 8 * buf;
+    mbar_expect_tx(bar, (uint32_t)a.v_box * DIMS * 2);
+    tma_tile(vsm + buf * vbytes, &vmap, n * hd + item_d0, (int)(first + t * AC_TILE), bar);
+  };
+  if (tid == 0)
+    for (unsigned t = 0; t < (unsigned)a.k_bufs && t < k_tiles; ++t)
+      issue_k(t, (int)t);
+  if (tid == AC_THREADS - 32 && has_item)
+    for (unsigned t = 0; t < (unsigned)a.v_bufs && t < v_tiles; ++t)
+      issue_v(t, (int)t);
+  /* ---- query heads; the CTA that scores the token's own row also makes its key */
+  const float *ct = a.cos_tab + (size_t)p * hd, *sn = a.sin_tab + (size_t)p * hd;
+  for (int g = warp; g < gqa + has_own; g += AC_WARPS) {
+    const float *src = g < gqa ? a.q + (size_t)(h0 + g) * hd : a.k + (size_t)n * hd;
+    const float *gamma = g < gqa ? a.q_gamma : a.k_gamma;
+    if (!a.rope)
+      for (int i = lane; i < hd; i += 32)
+        qs[g * hd + i] = src[i];
+    else if constexpr (HD != 0)
+      rope_head_regs<HD / 32>(src, gamma, a.eps, ct, sn, lane, qs + g * hd);
+    else
+      rope_head(src, gamma, a.eps, ct, sn, hd, lane, qs + g * hd);
+  }
+  if (append && warp == AC_WARPS - 1)
+    for (int i = lane; i < hd; i += 32)
+      a.vcache[((size_t)p * a.hkv + n) * hd + i] = float_to_half_bits_rn(a.v[(size_t)n * hd + i]);
+  __syncthreads();
+  if (a.q_rot && rank == 0)
+    for (int i = tid; i < gqa * hd; i += AC_THREADS)
+      a.q_rot[(size_t)h0 * hd + i] = qs[i];
+  cluster_wait();
+  /* ---- scores */
+  const double norm = sqrt((double)(float)hd);
+  auto put = [&](unsigned t, int g, float sum) {
+    const float v = HD == 64 ? __fmul_rn(__fadd_rn(0.0f, sum), 0.125f) // sqrt(64): the same quotient
+                             : (float)((double)__fadd_rn(0.0f, sum) / norm);
+#pragma unroll 2
+    for (int i = 0; i < per_head; ++i)
+      st_cluster(esm + 4 * t, (uint32_t)(g * per_head + i), v);
+  };
+  bool ok = true;
+  int kbuf = 0;
+  uint32_t kpar = 0;
+  for (unsigned t = 0; t < k_tiles; ++t) {
+    ok = ok && mbar_wait_bounded(kbar0 + 8 * kbuf, kpar, abort_flag, &g_attn_status, AC_POLLS, 1024);
+    uint8_t *tile = ktile + kbuf * kbytes;
+    const unsigned t0 = r_lo + t * AC_TILE, rows = min(r_hi - t0, (unsigned)AC_TILE);
+    if (has_own && t + 1 == k_tiles) { // the token's own row, as the cache will hold it, over what the copy found there
+      const int row = (int)rows - 1;
+      for (int c = tid; c < hd / 8; c += AC_THREADS) {
+        const float *src = kown + 8 * c;
+        uint32_t w[4];
 #pragma unroll
-    for (int o = 16; o; o >>= 1)
-      mx = fmaxf(mx, __shfl_xor_sync(FULL, mx, o));
+        for (int i = 0; i < 4; ++i)
+          w[i] = (uint32_t)float_to_half_bits_rn(src[2 * i]) | ((uint32_t)float_to_half_bits_rn(src[2 * i + 1]) << 16);
+        const uint4 v = make_uint4(w[0], w[1], w[2], w[3]);
+        *reinterpret_cast<uint4 *>(tile + (c >> 3) * (AC_TILE * 128) + row * 128 + (((c & 7) ^ (row & 7)) << 4)) = v;
+        if (append)
+          *reinterpret_cast<uint4 *>(a.kcache + ((size_t)p * a.hkv + n) * hd + 8 * c) = v;
+      }
+      __syncthreads();
+    }
+    if (ok) { // a unit of work: 32 rows and one or two heads
+      const int lg = rows <= 32 ? 0 : rows <= 64 ? 1 : 2, mask = (1 << lg) - 1;
+      if (gqa % 2 == 0 && ((gqa / 2) << lg) >= AC_WARPS) { // two heads at a time: a key row is converted once for both
+        for (int u = warp; u < (gqa / 2) << lg; u += AC_WARPS) {
+          const int row = (u & mask) * 32 + lane, g = 2 * (u >> lg);
+          float s[2];
+          dot_rows<2, HD>(tile, row, qs + g * hd, hd, s);
+          if (row < (int)rows) {
+            put(t0 + row, g, s[0]);
+            put(t0 + row, g + 1, s[1]);
+          }
+        }
+      } else {
+        for (int u = warp; u < gqa << lg; u += AC_WARPS) {
+          const int row = (u & mask) * 32 + lane, g = u >> lg;
+          float s[1];
+          dot_rows<1, HD>(tile, row, qs + g * hd, hd, s);
+          if (row < (int)rows)
+            put(t0 + row, g, s[0]);
+        }
+      }
+    }
+    if (t + a.k_bufs < k_tiles) {
+      __syncthreads(); // the tile's readers are done
+      if (tid == 0)
+        issue_k(t + a.k_bufs, kbuf);
+    }
+    if (++kbuf == a.k_bufs) {
+      kbuf = 0;
+      kpar ^= 1;
+    }
+  }
+  cluster_arrive();
+  cluster_wait(); // every score of this CTA's head is here
+  if (a.q_inplace && rank == 0) // every CTA of the cluster has read the raw heads
+    for (int i = tid; i < gqa * hd; i += AC_THREADS)
+      a.q_inplace[(size_t)h0 * hd + i] = qs[i];
+  if (!has_item)
+    return;
+  /* ---- softmax of head item_head (attn_softmax_kernel's steps) */
+  const int head = h0 + item_head;
+  float mx = -INFINITY;
+  for (unsigned r = tid; r < cnt; r += AC_THREADS)
+    mx = fmaxf(mx, e[r]);
+#pragma unroll
+  for (int o = 16; o; o >>= 1)
+    mx = fmaxf(mx, __shfl_xor_sync(FULL, mx, o));
+  if (lane == 0)
+    red[warp] = mx;
+  __syncthreads();
+  mx = red[0];
+#pragma unroll
+  for (int w = 1; w < AC_WARPS; ++w)
+    mx = fmaxf(mx, red[w]);
+  if (a.sink)
+    mx = fmaxf(mx, a.sink[head]);
+  const unsigned cnt32 = (cnt + 31) & ~31u; // zeros behind the last row: adding them changes nothing
+  for (unsigned r = tid; r < cnt32; r += AC_THREADS)
+    e[r] = r < cnt ? exp256_lane(__fsub_rn(e[r], mx)) : 0.f;
+  __syncthreads();
+  if (warp == 0) {
+    const float sum = ordered_sum(e, cnt32, a.sink ? exp256_lane(__fsub_rn(a.sink[head], mx)) : 0.0f, lane);
     if (lane == 0)
-      red[warp] = mx;
-    __syncthreads();
-    mx = red[0];
-    for (int w = 1; w < nwarps; ++w)
-      mx = fmaxf(mx, red[w]);
-    if (sink)
-      mx = fmaxf(mx, sink[c]);
-    for (unsigned r = threadIdx.x; r < cnt; r += nthreads)
-      e[r] = exp256_lane(__fsub_rn(e[r], mx)); // each thread rewrites the elements it stored itself
-    __syncthreads();
-    if (threadIdx.x == 0) {
-      float sum = sink ? exp256_lane(__fsub_rn(sink[c], mx)) : 0.0f;
-      unsigned r = 0;
-      for (; r + 16 <= cnt; r += 16) { // loads issued together, adds in order
-        float ev[16];
-#pragma unroll
-        for (int u = 0; u < 16; ++u)
-          ev[u] = e[r + u];
-#pragma unroll
-        for (int u = 0; u < 16; ++u)
-          sum = __fadd_rn(sum, ev[u]);
-      }
-      for (; r < cnt; ++r)
-        sum = __fadd_rn(sum, e[r]);
       s_bcast = sum;
-    }
-    __syncthreads();
-    const float sum = s_bcast;
-    for (unsigned r = threadIdx.x; r < cnt; r += nthreads)
-      e[r] = __fdiv_rn(e[r], sum);
-    __syncthreads(); // the chain below reads every thread's probabilities
   }
-  // ---- values
-  float acc = 0.f;
-  for (unsigned t = 0; t < n_tiles; ++t) {
-    const int buf = t % SVBUF;
-    if (t + SVBUF - 1 < n_tiles)
-      issue(t + SVBUF - 1, (t + SVBUF - 1) % SVBUF); // the buffer tile t - 1 used: everyone left it at the barrier below
-    if (!mbar_wait_bounded(smem_u32(&tile_bar[buf]), (t / SVBUF) & 1, abort_flag, &g_attn_status, 1u << 22, 1024))
-      break;
-    const uint16_t *vt = reinterpret_cast<const uint16_t *>(vring + buf * vbytes);
-    const float *pt = e + t * SVT;
-    const unsigned rows = cnt - t * SVT < (unsigned)SVT ? cnt - t * SVT : (unsigned)SVT;
-    if (d < hd) {
-      unsigned j = 0;
-      for (; j + 8 <= rows; j += 8) {
-        const float4 pa = *reinterpret_cast<const float4 *>(pt + j), pb = *reinterpret_cast<const float4 *>(pt + j + 4);
-        const float a[8] = {pa.x, pa.y, pa.z, pa.w, pb.x, pb.y, pb.z, pb.w};
-        float b[8];
-#pragma unroll
-        for (int u = 0; u < 8; ++u)
-          b[u] = half_bits_to_float(vt[(j + u) * hd + d]);
-#pragma unroll
-        for (int u = 0; u < 8; ++u)
-          acc = __fmaf_rn(a[u], b[u], acc);
+  __syncthreads();
+  const float sum = s_bcast;
+  for (unsigned r = tid; r < cnt; r += AC_THREADS)
+    e[r] = __fdiv_rn(e[r], sum);
+  __syncthreads();
+  /* ---- values */
+  if (warp == AC_WARPS - 1) { // keeps the ring of value tiles full
+    if (lane == 0) {
+      int buf = 0;
+      uint32_t par = 0;
+      for (unsigned t = a.v_bufs; t < v_tiles; ++t) {
+        if (!mbar_wait_bounded(vempty0 + 8 * buf, par, abort_flag, &g_attn_status, AC_POLLS, 1024))
+          break;
+        issue_v(t, buf);
+        if (++buf == a.v_bufs) {
+          buf = 0;
+          par ^= 1;
+        }
       }
-      for (; j < rows; ++j)
-        acc = __fmaf_rn(pt[j], half_bits_to_float(vt[j * hd + d]), acc);
     }
-    __syncthreads(); // done with this buffer before a later tile is copied into it
+    __syncwarp();
+  } else if (warp < DIMS / 32) {
+    const int d = item_d0 + tid;
+    float acc = 0.f;
+    // Sixteen rows in the chain while the next sixteen -- of the next tile at a tile's end -- are on their way: 4.3 clocks per
+    // row (the chain alone: 4.1; loads issued by the compiler's own schedule: 8 to 12).
+    float pr[2][16];
+    uint16_t vb[2][16];
+    auto load = [&](const uint16_t *vt, const float *pt, float(&pp)[16], uint16_t(&vv)[16]) {
+#pragma unroll
+      for (int u = 0; u < 4; ++u) {
+        const float4 f = *reinterpret_cast<const float4 *>(pt + 4 * u);
+        pp[4 * u] = f.x, pp[4 * u + 1] = f.y, pp[4 * u + 2] = f.z, pp[4 * u + 3] = f.w;
+      }
+#pragma unroll
+      for (int u = 0; u < 16; ++u)
+        vv[u] = vt[u * DIMS];
+    };
+    int buf = 0;
+    uint32_t par = 0;
+    const uint16_t *vt = reinterpret_cast<const uint16_t *>(vtile) + tid;
+    if (v_tiles) {
+      ok = mbar_wait_bounded(vfull0, 0, abort_flag, &g_attn_status, AC_POLLS, 1024) && ok;
+      load(vt, e, pr[0], vb[0]); // reads past the last row stay in shared memory and are not used
+    }
+    for (unsigned t = 0; t < v_tiles; ++t) {
+      const float *pt = e + t * AC_TILE;
+      const unsigned rows = min(cached - t * AC_TILE, (unsigned)AC_TILE);
+      int nbuf = buf + 1;
+      uint32_t npar = par;
+      if (nbuf == a.v_bufs) {
+        nbuf = 0;
+        npar ^= 1;
+      }
+      const uint16_t *nvt = reinterpret_cast<const uint16_t *>(vtile + nbuf * vbytes) + tid;
+      if (rows == AC_TILE) {
+#pragma unroll
+        for (int j = 0; j < AC_TILE; j += 16) {
+          const int k = (j / 16) & 1;
+          if (j + 16 < AC_TILE) {
+            load(vt + (j + 16) * DIMS, pt + j + 16, pr[k ^ 1], vb[k ^ 1]);
+          } else if (t + 1 < v_tiles) {
+            ok = mbar_wait_bounded(vfull0 + 8 * nbuf, npar, abort_flag, &g_attn_status, AC_POLLS, 1024) && ok;
+            load(nvt, pt + AC_TILE, pr[k ^ 1], vb[k ^ 1]);
+          }
+#pragma unroll
+          for (int u = 0; u < 16; ++u)
+            acc = __fmaf_rn(pr[k][u], half_bits_to_float(vb[k][u]), acc);
+        }
+      } else { // the last tile
+        unsigned j = 0;
+        for (; j + 16 <= rows; j += 16) {
+          load(vt + j * DIMS, pt + j, pr[0], vb[0]);
+#pragma unroll
+          for (int u = 0; u < 16; ++u)
+            acc = __fmaf_rn(pr[0][u], half_bits_to_float(vb[0][u]), acc);
+        }
+        for (; j < rows; ++j)
+          acc = __fmaf_rn(pt[j], half_bits_to_float(vt[j * DIMS]), acc);
+      }
+      __syncwarp();
+      if (lane == 0)
+        mbar_arrive(vempty0 + 8 * buf);
+      buf = nbuf;
+      par = npar;
+      vt = nvt;
+    }
+    if (d < hd && ok) {
+      if (a.rope)
+        acc = __fmaf_rn(e[cnt - 1], half_bits_to_float(float_to_half_bits_rn(a.v[(size_t)n * hd + d])), acc);
+      a.out[(size_t)head * hd + d] = acc;
+    }
   }
-  if (d < hd && !*abort_flag)
-    out[(size_t)c * hd + d] = acc;
+  if (*abort_flag) // give the copies in flight time to land in this CTA's shared memory
+    for (int i = 0; i < 1000; ++i)
+      __nanosleep(1000);
 }
 
 int read_attn_status(int *out) {
@@ -609,33 +930,56 @@ int clear_attn_status() {
 
 /* ---------------------------------------------------------------- launchers */
 
-/* The driver's tensor-map encoder, looked up through the runtime (the library does not link against the driver). */
-static int encode_value_map(CUtensorMap *map, const uint16_t *vcache, unsigned rows, unsigned hkv, unsigned hd) {
+/* Tensor map over a cache [rows][hkv * hd] fp16 with boxes of box_rows x box_dims values (swizzled: 64 values = 128
+ * bytes). The driver's encoder is looked up through the runtime (the library does not link against the driver). A map depends
+ * on its arguments alone; every thread keeps the last ones it made, because a decode loop comes back with the same. */
+static int encode_cache_map(CUtensorMap *map, const uint16_t *cache, unsigned rows, unsigned hkv, unsigned hd, unsigned box_dims,
+                            unsigned box_rows, bool swizzle) {
   typedef CUresult (*EncodeTiled)(CUtensorMap *, CUtensorMapDataType, cuuint32_t, void *, const cuuint64_t *,
                                   const cuuint64_t *, const cuuint32_t *, const cuuint32_t *, CUtensorMapInterleave,
                                   CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
-  static EncodeTiled encode = nullptr;
-  if (!encode) {
+  static std::atomic<EncodeTiled> encode{nullptr};
+  EncodeTiled enc = encode.load(std::memory_order_acquire);
+  if (!enc) {
     void *fn = nullptr;
     cudaDriverEntryPointQueryResult found;
     NNTR_CHECK_CUDA(cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &fn, cudaEnableDefault, &found));
     if (!fn || found != cudaDriverEntryPointSuccess)
       return set_error(NNTR_CUDA_ERR_UNSUPPORTED, "attention: the driver has no cuTensorMapEncodeTiled");
-    encode = reinterpret_cast<EncodeTiled>(fn);
+    enc = reinterpret_cast<EncodeTiled>(fn);
+    encode.store(enc, std::memory_order_release);
+  }
+  struct Key { // compared as bytes: no padding
+    const uint16_t *cache;
+    unsigned rows, hkv, hd, box_dims, box_rows, swizzle; // never all zero: an empty entry matches nothing
+  };
+  struct Entry {
+    Key key;
+    CUtensorMap map;
+  };
+  constexpr unsigned SLOTS = 64; // 12 KB per thread
+  static thread_local Entry slots[SLOTS] = {};
+  const Key key = {cache, rows, hkv, hd, box_dims, box_rows, swizzle};
+  Entry &slot = slots[((uint32_t)(reinterpret_cast<uintptr_t>(cache) >> 12) * 2654435761u >> 26) ^ (swizzle ? 1u : 0u)];
+  if (memcmp(&slot.key, &key, sizeof key) == 0) {
+    *map = slot.map;
+    return NNTR_CUDA_OK;
   }
   const cuuint64_t dims[2] = {(cuuint64_t)hkv * hd, rows};
   const cuuint64_t strides[1] = {(cuuint64_t)hkv * hd * 2}; // bytes between rows: a multiple of 16 (head_dim % 8 == 0)
-  const cuuint32_t box[2] = {hd, (cuuint32_t)SVT};
+  const cuuint32_t box[2] = {box_dims, box_rows};
   const cuuint32_t estr[2] = {1, 1};
-  const CUresult r = encode(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, const_cast<uint16_t *>(vcache), dims, strides, box, estr,
-                            CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
-                            CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-  if (r != CUDA_SUCCESS)
+  const CUresult r = enc(&slot.map, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, const_cast<uint16_t *>(cache), dims, strides, box, estr,
+                         CU_TENSOR_MAP_INTERLEAVE_NONE, swizzle ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_NONE,
+                         CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  if (r != CUDA_SUCCESS) {
+    slot.key = Key{};
     return set_error(NNTR_CUDA_ERR_CUDA, "attention: cuTensorMapEncodeTiled failed (%d)", (int)r);
+  }
+  slot.key = key;
+  *map = slot.map;
   return NNTR_CUDA_OK;
 }
-
-
 
 static int check_attn(const nntr_attn_desc *a) {
   if (!a || a->n_heads_q == 0 || a->n_heads_kv == 0 || a->head_dim == 0)
@@ -692,6 +1036,73 @@ size_t attention_workspace_bytes(const nntr_attn_desc *a, unsigned max_rows) {
   return ((rows + 3) & ~(size_t)3) * a->n_heads_q * sizeof(float); // head-major rows are padded to four elements
 }
 
+/* The cluster launch, or *taken = false where it does not apply: heads of more than 128 dimensions, more rows than shared
+ * memory keeps, or NNTR_CUDA_ATTN_SEPARATE. */
+static int launch_attn_cluster(AttnStep a, unsigned bound, unsigned rows, unsigned flags, cudaStream_t st, bool *taken) {
+  const int hd = a.hd;
+  *taken = false;
+  if ((flags & NNTR_CUDA_ATTN_SEPARATE) || hd > 128 || rows > AC_MAX_ROWS)
+    return NNTR_CUDA_OK;
+  int gqa = a.hq / a.hkv;
+  a.groups = 1;
+  while (gqa % a.groups || gqa / a.groups > 8) // at most 16 query heads in all (check_attn)
+    ++a.groups;
+  gqa /= a.groups;
+  // a CTA owns 64 dimensions of a head where eight CTAs are enough for that, else the whole head
+  const int dims = hd <= 64 || gqa * 2 <= 8 ? 64 : 128;
+  const int items = gqa * ((hd + dims - 1) / dims);
+  // eight CTAs per cluster while that leaves no cluster waiting for SMs -- 16 clusters of eight run in two waves (11.1 us for a
+  // window of 50 rows, clusters of four 8), because a cluster lies inside one part of the chip --, at least as many as items
+  const unsigned clusters = (unsigned)(a.hkv * a.groups);
+  unsigned csize = clusters > 12 && items <= 4 ? 4 : 8;
+  while (csize > 1 && clusters * csize > 144u && (int)(csize / 2) >= items)
+    csize /= 2;
+  // buffers for what the launch can need, no more: the next kernel's CTAs want room beside this one's
+  a.cap_rows = rows;
+  const unsigned k_tiles = ((rows + csize - 1) / csize + AC_TILE - 1) / AC_TILE, v_tiles = (rows + AC_TILE - 1) / AC_TILE;
+  const unsigned k_max = hd <= 64 ? 4u : 2u;
+  a.k_bufs = (int)(k_tiles < k_max ? k_tiles : k_max);
+  a.v_bufs = (int)(v_tiles < (unsigned)AC_VBUF_MAX ? v_tiles : (unsigned)AC_VBUF_MAX);
+  const auto box = [](unsigned n) { return n <= 32 ? 32 : n <= 64 ? 64 : AC_TILE; };
+  a.k_box = box((rows + csize - 1) / csize);
+  a.v_box = box(rows);
+  AcLayout L = ac_layout(gqa, hd, dims, a.k_bufs, a.v_bufs, rows);
+  while (L.total > 200u * 1024u && a.v_bufs > 2)
+    L = ac_layout(gqa, hd, dims, a.k_bufs, --a.v_bufs, rows);
+  const auto kernel = hd == 128  ? (dims == 64 ? attn_cluster_kernel<128, 64> : attn_cluster_kernel<128, 128>)
+                      : hd == 64 ? attn_cluster_kernel<64, 64>
+                                 : (dims == 64 ? attn_cluster_kernel<0, 64> : attn_cluster_kernel<0, 128>);
+  static std::atomic<uint32_t> attr_done[64];
+  int dev = 0;
+  NNTR_CHECK_CUDA(cudaGetDevice(&dev));
+  const uint32_t bit = 1u << (hd == 128 ? (dims == 64 ? 0 : 1) : hd == 64 ? 2 : (dims == 64 ? 3 : 4));
+  if (!(attr_done[dev & 63].load(std::memory_order_acquire) & bit)) {
+    NNTR_CHECK_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
+    attr_done[dev & 63].fetch_or(bit, std::memory_order_release);
+  }
+  CUtensorMap kmap, vmap;
+  int rc = encode_cache_map(&kmap, a.kcache, bound, (unsigned)a.hkv, (unsigned)hd, 64, (unsigned)a.k_box, true);
+  if (rc || (rc = encode_cache_map(&vmap, a.vcache, bound, (unsigned)a.hkv, (unsigned)hd, (unsigned)dims, (unsigned)a.v_box, false)))
+    return rc;
+  cudaLaunchConfig_t cfg = {};
+  cudaLaunchAttribute attr[2];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = csize;
+  attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+  attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[1].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = (flags & NNTR_CUDA_GEMV_PDL) ? 2 : 1;
+  cfg.stream = st;
+  cfg.gridDim = dim3(clusters * csize);
+  cfg.blockDim = dim3(AC_THREADS);
+  cfg.dynamicSmemBytes = L.total;
+  const cudaError_t e = cudaLaunchKernelEx(&cfg, kernel, kmap, vmap, a);
+  count_launch();
+  *taken = true;
+  return check_cuda(e, "attention launch");
+}
+
 int launch_attention_decode(const nntr_attn_desc *a, unsigned pos, const unsigned *pos_dev, unsigned max_rows,
                             const float *q, const uint16_t *kcache, const uint16_t *vcache, float *out, void *ws,
                             size_t ws_bytes, unsigned flags, cudaStream_t st) {
@@ -714,43 +1125,23 @@ int launch_attention_decode(const nntr_attn_desc *a, unsigned pos, const unsigne
     return set_error(NNTR_CUDA_ERR_INVALID, "attention_decode: q, caches and workspace must be 16-byte aligned");
   float *scores = static_cast<float *>(ws);
   const int hq = (int)a->n_heads_q, hkv = (int)a->n_heads_kv, hd = (int)a->head_dim;
+  AttnStep s = {};
+  s.q = q, s.kcache = const_cast<uint16_t *>(kcache), s.vcache = const_cast<uint16_t *>(vcache);
+  s.out = out, s.sink = a->sink, s.pos_dev = pos_dev, s.pos = pos, s.window = a->window;
+  s.hq = hq, s.hkv = hkv, s.hd = hd;
+  bool taken;
+  if ((rc = launch_attn_cluster(s, bound, rows, flags, st, &taken)) || taken)
+    return rc;
   cudaLaunchConfig_t cfg = {};
   cudaLaunchAttribute attr[1];
   pdl_cfg(cfg, attr, flags, st);
   cfg.gridDim = dim3((rows + SCORE_WARPS * 4 - 1) / (SCORE_WARPS * 4), (unsigned)hkv);
   cfg.blockDim = dim3(32 * SCORE_WARPS);
   cfg.dynamicSmemBytes = (size_t)(hq / hkv) * hd * sizeof(float) + (size_t)SCORE_WARPS * 4 * hd * sizeof(uint16_t);
-  // short windows: the softmax runs in front of the values, in the same launch, on scores stored head-major
-  // (NNTR_CUDA_ATTN_SEPARATE keeps the three kernels)
-  const unsigned sv_stride = (rows + 3u) & ~3u;
-  const int sv_threads = 32 * ((hd + 31) / 32);
-  const size_t sv_smem = (((size_t)sv_stride * sizeof(float) + 127) & ~(size_t)127) + (size_t)SVBUF * SVT * hd * 2;
-  const bool fused = !(flags & NNTR_CUDA_ATTN_SEPARATE) && rows <= SV_MAX_ROWS && sv_threads <= 256 && sv_smem <= 200u * 1024u;
-  cudaError_t e = cudaLaunchKernelEx(&cfg, attn_scores_kernel, q, kcache, scores, pos_dev, pos, hq, hkv, hd, a->window,
-                                     fused ? sv_stride : 0u);
+  cudaError_t e = cudaLaunchKernelEx(&cfg, attn_scores_kernel, q, kcache, scores, pos_dev, pos, hq, hkv, hd, a->window);
   count_launch();
   if ((rc = check_cuda(e, "attention scores launch")))
     return rc;
-  if (fused) {
-    static bool attr_done[64] = {};
-    int dev = 0;
-    NNTR_CHECK_CUDA(cudaGetDevice(&dev));
-    if (!attr_done[dev & 63]) {
-      NNTR_CHECK_CUDA(cudaFuncSetAttribute(attn_softmax_values_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
-      attr_done[dev & 63] = true;
-    }
-    // tensor map of the value cache as seen by this call: [bound rows][hkv * hd] fp16, boxes of SVT rows x hd values
-    CUtensorMap vmap;
-    if ((rc = encode_value_map(&vmap, vcache, bound, (unsigned)hkv, (unsigned)hd)))
-      return rc;
-    cfg.gridDim = dim3((unsigned)hq);
-    cfg.blockDim = dim3((unsigned)sv_threads);
-    cfg.dynamicSmemBytes = sv_smem;
-    e = cudaLaunchKernelEx(&cfg, attn_softmax_values_kernel, vmap, static_cast<const float *>(scores), out, a->sink,
-                           pos_dev, pos, hq, hkv, hd, a->window, rows);
-    count_launch();
-    return check_cuda(e, "attention softmax + values launch");
-  }
   cfg.gridDim = dim3((unsigned)hq);
   cfg.blockDim = dim3(SOFTMAX_THREADS);
   const unsigned cap_rows = rows < 11264u ? rows : 11264u; // 44 KB of shared memory at most; later rows stay in global
@@ -768,9 +1159,10 @@ int launch_attention_decode(const nntr_attn_desc *a, unsigned pos, const unsigne
   return check_cuda(e, "attention values launch");
 }
 
-/* One token's whole attention step: per-head norms (gammas may be null) + rotary + cache append + scores, then
- * softmax + values -- two launches for windows of up to SV_MAX_ROWS rows; otherwise (or with NNTR_CUDA_ATTN_SEPARATE)
- * the rotary launch followed by launch_attention_decode, which rotates q in place. */
+/* One token's whole attention step: per-head norms (gammas may be null) + rotary + cache append + scores + softmax +
+ * values -- one launch where launch_attn_cluster applies, else the rotary launch followed by launch_attention_decode, which
+ * rotates q in place. For windows beyond ATTN_INPLACE_ROWS q is rotated in place either way, as the interface says. */
+constexpr unsigned ATTN_INPLACE_ROWS = 2048;
 int launch_attention_step(const nntr_attn_desc *a, unsigned pos, const unsigned *pos_dev, unsigned max_rows, float *q,
                           const float *k, const float *v, const float *q_gamma, const float *k_gamma, float eps,
                           uint16_t *kcache, uint16_t *vcache, const float *cos_tab, const float *sin_tab, float *q_rot,
@@ -787,55 +1179,27 @@ int launch_attention_step(const nntr_attn_desc *a, unsigned pos, const unsigned 
     return set_error(NNTR_CUDA_ERR_INVALID, "attention_step: position %u beyond the %u rows allowed", pos, max_rows);
   const unsigned rows = bound < a->window ? bound : a->window;
   const int hq = (int)a->n_heads_q, hkv = (int)a->n_heads_kv, hd = (int)a->head_dim;
-  const unsigned sv_stride = (rows + 3u) & ~3u;
-  const int sv_threads = 32 * ((hd + 31) / 32);
-  const size_t sv_smem = (((size_t)sv_stride * sizeof(float) + 127) & ~(size_t)127) + (size_t)SVBUF * SVT * hd * 2;
-  const bool fused = !(flags & NNTR_CUDA_ATTN_SEPARATE) && rows <= SV_MAX_ROWS && sv_threads <= 256 && sv_smem <= 200u * 1024u;
-  if (!fused) {
-    if ((rc = launch_rope_cache_append(a, pos, pos_dev, q, k, v, q_gamma, k_gamma, eps, kcache, vcache, cos_tab, sin_tab, flags,
-                                       st)))
-      return rc;
-    if (q_rot)
-      NNTR_CHECK_CUDA(cudaMemcpyAsync(q_rot, q, (size_t)hq * hd * sizeof(float), cudaMemcpyDeviceToDevice, st));
-    return launch_attention_decode(a, pos, pos_dev, max_rows, q, kcache, vcache, out, ws, ws_bytes, flags, st);
-  }
-  const size_t ws_need = (size_t)sv_stride * a->n_heads_q * sizeof(float);
-  if (ws_bytes < ws_need)
-    return set_error(NNTR_CUDA_ERR_INVALID, "attention_step: workspace of %zu bytes needed, %zu given", ws_need, ws_bytes);
   if ((reinterpret_cast<uintptr_t>(kcache) & 15) || (reinterpret_cast<uintptr_t>(vcache) & 15) ||
       (reinterpret_cast<uintptr_t>(ws) & 15))
     return set_error(NNTR_CUDA_ERR_INVALID, "attention_step: caches and workspace must be 16-byte aligned");
-  float *scores = static_cast<float *>(ws);
-  cudaLaunchConfig_t cfg = {};
-  cudaLaunchAttribute attr[1];
-  pdl_cfg(cfg, attr, flags, st);
-  cfg.gridDim = dim3((rows + SCORE_WARPS * 4 - 1) / (SCORE_WARPS * 4), (unsigned)hkv);
-  cfg.blockDim = dim3(32 * SCORE_WARPS);
-  cfg.dynamicSmemBytes = (size_t)(hq / hkv) * hd * sizeof(float) + (size_t)SCORE_WARPS * 4 * hd * sizeof(uint16_t) +
-                         (size_t)SCORE_WARPS * hd * sizeof(float);
-  cudaError_t e = cudaLaunchKernelEx(&cfg, attn_rope_scores_kernel, static_cast<const float *>(q), k, v, q_gamma, k_gamma, eps,
-                                     kcache, vcache, cos_tab, sin_tab, q_rot, scores, pos_dev, pos, hq, hkv, hd, a->window,
-                                     sv_stride);
-  count_launch();
-  if ((rc = check_cuda(e, "attention rotary + scores launch")))
+  const size_t ws_need = (((size_t)rows + 3) & ~(size_t)3) * a->n_heads_q * sizeof(float);
+  if (ws_bytes < ws_need)
+    return set_error(NNTR_CUDA_ERR_INVALID, "attention_step: workspace of %zu bytes needed, %zu given", ws_need, ws_bytes);
+  AttnStep s = {};
+  s.q = q, s.k = k, s.v = v, s.q_gamma = q_gamma, s.k_gamma = k_gamma, s.eps = eps;
+  s.kcache = kcache, s.vcache = vcache, s.cos_tab = cos_tab, s.sin_tab = sin_tab;
+  s.q_rot = q_rot, s.q_inplace = rows > ATTN_INPLACE_ROWS ? q : nullptr, s.out = out, s.sink = a->sink;
+  s.pos_dev = pos_dev, s.pos = pos, s.window = a->window;
+  s.hq = hq, s.hkv = hkv, s.hd = hd, s.rope = 1;
+  bool taken;
+  if ((rc = launch_attn_cluster(s, bound, rows, flags, st, &taken)) || taken)
     return rc;
-  static bool attr_done[64] = {};
-  int dev = 0;
-  NNTR_CHECK_CUDA(cudaGetDevice(&dev));
-  if (!attr_done[dev & 63]) {
-    NNTR_CHECK_CUDA(cudaFuncSetAttribute(attn_softmax_values_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
-    attr_done[dev & 63] = true;
-  }
-  CUtensorMap vmap;
-  if ((rc = encode_value_map(&vmap, vcache, bound, (unsigned)hkv, (unsigned)hd)))
+  if ((rc = launch_rope_cache_append(a, pos, pos_dev, q, k, v, q_gamma, k_gamma, eps, kcache, vcache, cos_tab, sin_tab, flags,
+                                     st)))
     return rc;
-  cfg.gridDim = dim3((unsigned)hq);
-  cfg.blockDim = dim3((unsigned)sv_threads);
-  cfg.dynamicSmemBytes = sv_smem;
-  e = cudaLaunchKernelEx(&cfg, attn_softmax_values_kernel, vmap, static_cast<const float *>(scores), out, a->sink, pos_dev, pos,
-                         hq, hkv, hd, a->window, rows);
-  count_launch();
-  return check_cuda(e, "attention softmax + values launch");
+  if (q_rot)
+    NNTR_CHECK_CUDA(cudaMemcpyAsync(q_rot, q, (size_t)hq * hd * sizeof(float), cudaMemcpyDeviceToDevice, st));
+  return launch_attention_decode(a, pos, pos_dev, max_rows, q, kcache, vcache, out, ws, ws_bytes, flags, st);
 }
 
 } // namespace nntr

@@ -139,10 +139,10 @@ class Qwen3Decoder:
         a CUDA graph and replayed for every later token.
 
         Launches per layer without ``fuse``: (residual add +) RMS norm; q | k | v projections (one batched launch);
-        per-head norms + rotary + cache append + scores; softmax + values; attention_out; residual add + RMS norm;
-        ffn_up | ffn_gate (one batched launch); SwiGLU; ffn_down -- ten. With ``fuse`` the two norms run in the
-        prologues of the projections behind them and the SwiGLU in the epilogue of the up | gate launch -- seven. Every fusion keeps the bits of the
-        separate operators."""
+        attention with its per-head norms, rotary work and cache append; attention_out; residual add + RMS norm;
+        ffn_up | ffn_gate (one batched launch); SwiGLU; ffn_down -- nine. With ``fuse`` the two norms run in the
+        prologues of the projections behind them and the SwiGLU in the epilogue of the up | gate launch -- five (attention
+        takes more launches beyond 16384 rows). Every fusion keeps the bits of the separate operators."""
         c, b, pdl = self.cfg, self.b, self.pdl
         q_dim, kv_dim = c.n_heads * c.head_dim, c.n_kv_heads * c.head_dim
         be.embedding(c.embedding_dtype, self._P(self.ptr["embedding0"]), token_f, c.vocab, c.hidden,
@@ -153,7 +153,7 @@ class Qwen3Decoder:
             p = f"layer{i}_"
             qk_norm = (self._P(self.ptr[p + "q_norm"]), self._P(self.ptr[p + "k_norm"]), c.norm_eps)
             if fuse:
-                # 7 launches: (add +) norm + q|k|v; rotary + scores; softmax + values; o; add + norm + up|gate + SwiGLU; down
+                # 5 launches: (add +) norm + q|k|v; attention; o; add + norm + up|gate + SwiGLU; down
                 g_att, g_ffn = self._P(self.ptr[p + "attention_norm"]), self._P(self.ptr[p + "ffn_norm"])
                 if i == 0:
                     be.gemv_add_norm(c.fc_dtype, q_dim + 2 * kv_dim, c.hidden, x, None, None, g_att, c.norm_eps,
@@ -179,7 +179,7 @@ class Qwen3Decoder:
                 self._gemv(p + "wv", b["n"], b["v"])
                 self._gemv(p + "wk", b["n"], b["k"])
                 self._gemv(p + "wq", b["n"], b["q"])
-            # k_norm and q_norm (per-head RMS norms) run inside the rotary / cache-append launch
+            # k_norm and q_norm (per-head RMS norms) run inside the attention launch
             self.attn[i].step(b["q"], b["k"], b["v"], pos, pos_dev=pos_dev, out=b["a"], pdl=pdl, qk_norm=qk_norm)
             self._gemv(p + "attention_out", b["a"], b["o"])
             be.add_rms_norm(x, b["o"], self._P(self.ptr[p + "ffn_norm"]), c.norm_eps, sum_out=b["h"], out=b["n"], pdl=pdl)

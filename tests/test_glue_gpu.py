@@ -339,3 +339,27 @@ def test_single_projection_with_the_add_and_norm_in_its_prologue(be, port, N, K,
         if with_residual:
             assert same_bits(sum_out.cpu().numpy(), s)
     be.device_status()
+
+
+@pytest.mark.parametrize("rows", [1, 31, 33, 129, 767, 769, 1000, 2049])
+@pytest.mark.parametrize("hq,hkv,hd", [(32, 8, 128), (32, 4, 128), (16, 2, 64), (16, 1, 64), (8, 2, 72), (8, 1, 32)])
+def test_attention_in_one_launch_equals_the_separate_launches(be, hq, hkv, hd, rows):
+    """The one-launch step against rotary, scores, softmax and values in launches of their own, where the clusters' tiles,
+    boxes and shares end and where the ordered sum changes its form. Scores from nearly equal to far apart, because the
+    sum's fast form stops at rounding halves and powers of two. Equal bits, caches included."""
+    for spread in (0.02, 1.0, 8.0):
+        g = torch.Generator(device="cuda").manual_seed(rows + hq)
+        r = lambda *n: torch.randn(*n, generator=g, device="cuda")  # noqa: E731
+        sink = r(hq) if hd == 64 else None
+        kc, vc = r(rows, hkv, hd).half(), r(rows, hkv, hd).half()
+        q, k, v, norm = r(hq * hd) * spread, r(hkv * hd), r(hkv * hd), (1 + 0.1 * r(hd), 1 + 0.1 * r(hd), 1e-6)
+        got = []
+        for separate in (False, True):
+            a = be.Attention(hq, hkv, hd, rows, sink=sink)
+            a.kcache.copy_(kc)
+            a.vcache.copy_(vc)
+            out = a.step(q.clone(), k, v, rows - 1, qk_norm=None if spread == 0.02 else norm, separate=separate)
+            got.append((out, a.kcache, a.vcache))
+        be.device_status()
+        for x, y in zip(*got):
+            assert torch.equal(x.view(torch.uint8), y.view(torch.uint8))
