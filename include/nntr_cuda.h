@@ -181,6 +181,12 @@ int nntr_cuda_gemm_q4_K_noalloc_dev(unsigned M, unsigned N, unsigned K, const fl
 int nntr_cuda_gemv_dev(int qtype, unsigned N, unsigned K, const float *x, const void *B, float *y, unsigned flags,
                        void *stream);
 
+/** M decode GEMVs of one weight: C[m][0..N) = W A[m] for m < M with the bits of M calls with M == 1 (a GEMM's rows go through
+ *  the reference's four-row chain, a decode step's do not): what a prompt needs whose caches must equal those of decoding it
+ *  token by token. ldc = row stride of C; workspace as for nntr_cuda_gemm_*_dev. */
+int nntr_cuda_gemv_rows_dev(int qtype, unsigned M, unsigned N, unsigned K, const float *A, const void *B, float *C,
+                            unsigned ldc, void *workspace, size_t workspace_bytes, void *stream);
+
 /** Several decode GEMVs that share one activation in one launch: y[p][0..N) = W_p x for p < n_problems, with
  *  w_table a DEVICE array of n_problems device pointers to Q4_K weights of N rows x K each (e.g. the q, k and v
  *  projections of a layer cut into equal row slices, or the two halves of a gated FFN). Each output equals the
@@ -308,6 +314,14 @@ int nntr_cuda_attention_step_dev(const nntr_attn_desc *a, unsigned pos, const un
                                  const float *k, const float *v, const float *q_gamma, const float *k_gamma, float eps,
                                  void *kcache, void *vcache, const float *cos_tab, const float *sin_tab, float *q_rot,
                                  float *out, void *workspace, size_t workspace_bytes, unsigned flags, void *stream);
+
+/** nntr_cuda_attention_step_dev for `tokens` consecutive tokens from position pos on, in two launches: token i's heads are at
+ *  q, k, v + i * ld, its result goes to out + i * ld_out; q is rotated in place; all rows are appended to the caches. Same
+ *  bits as that many steps. Heads of up to 128 dimensions, windows of up to 16384 rows. */
+int nntr_cuda_attention_rows_dev(const nntr_attn_desc *a, unsigned pos, unsigned tokens, float *q, const float *k,
+                                 const float *v, size_t ld, const float *q_gamma, const float *k_gamma, float eps,
+                                 void *kcache, void *vcache, const float *cos_tab, const float *sin_tab, float *out,
+                                 size_t ld_out, unsigned flags, void *stream);
 
 /* ------------------------------------------------------- .bin weight files */
 

@@ -199,6 +199,18 @@ def gemv(qtype: str, N: int, K: int, x, B, y, pdl: bool = False):
     return y
 
 
+def gemv_rows(qtype: str, M: int, N: int, K: int, A, B, C, ldc: int, workspace=None):
+    """C[m] = W A[m] for every row with the bits of M decode calls (gemv); device tensors."""
+    torch = _torch()
+    need = gemm_workspace_bytes(qtype, M, N, K)
+    if need and (workspace is None or workspace.numel() < need):
+        workspace = torch.empty(need, dtype=torch.uint8, device="cuda")
+    check(lib().nntr_cuda_gemv_rows_dev(QTYPE[qtype], M, N, K, A.data_ptr(), B.data_ptr(), C.data_ptr(), ldc,
+                                        workspace.data_ptr() if workspace is not None else None,
+                                        workspace.numel() if workspace is not None else 0, _stream()))
+    return C
+
+
 def gemv_batched(qtype: str, N: int, K: int, x, w_table, n_problems: int, y, pdl: bool = False):
     """n_problems decode GEMVs sharing the activation x in one launch; w_table is a device int64 tensor of weight
     addresses (N rows x K each), y is [n_problems, N]."""
@@ -522,6 +534,18 @@ class Attention:
             self.kcache.data_ptr(), self.vcache.data_ptr(), self.cos.data_ptr(), self.sin.data_ptr(),
             q_rot.data_ptr() if q_rot is not None else None, out.data_ptr(), self.ws.data_ptr(), self.ws.numel(),
             _flags(pdl) | (capi.ATTN_SEPARATE if separate else 0), _stream()))
+        return out
+
+
+    def rows(self, q, k, v, ld: int, pos: int, tokens: int, out, ld_out: int, qk_norm=None, pdl: bool = False):
+        """``step`` for ``tokens`` consecutive tokens from ``pos`` on: token i's heads at element i * ld of q, k and v (q is
+        rotated in place), its result at element i * ld_out of out."""
+        qg, kg, eps = qk_norm if qk_norm is not None else (None, None, 0.0)
+        check(lib().nntr_cuda_attention_rows_dev(
+            self._C.byref(self.desc), pos, tokens, q.data_ptr(), k.data_ptr(), v.data_ptr(), ld,
+            qg.data_ptr() if qg is not None else None, kg.data_ptr() if kg is not None else None, eps,
+            self.kcache.data_ptr(), self.vcache.data_ptr(), self.cos.data_ptr(), self.sin.data_ptr(), out.data_ptr(), ld_out,
+            _flags(pdl), _stream()))
         return out
 
 

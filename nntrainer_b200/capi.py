@@ -55,6 +55,8 @@ SIGNATURES = {
     "nntr_cuda_attention_decode_dev": (_i, [_vp, _u, _vp, _u, _vp, _vp, _vp, _vp, _vp, _sz, _u, _vp]),
     "nntr_cuda_attention_step_dev": (_i, [_vp, _u, _vp, _u, _vp, _vp, _vp, _vp, _vp, C.c_float, _vp, _vp, _vp, _vp, _vp, _vp,
                                           _vp, _sz, _u, _vp]),
+    "nntr_cuda_attention_rows_dev": (_i, [_vp, _u, _u, _vp, _vp, _vp, _sz, _vp, _vp, C.c_float, _vp, _vp, _vp, _vp, _vp, _sz,
+                                          _u, _vp]),
     "nntr_cuda_bin_layout": (_i, [_vp, _sz, _vp, _vp, _vp]),
     "nntr_cuda_bin_load": (_i, [C.c_char_p, _vp, _sz, _i, _i, _vp, _vp]),
     "nntr_cuda_quantize_q8_K_dev": (_i, [_vp, _i64, _vp, _i64, _i64, _i, _vp]),
@@ -69,6 +71,7 @@ SIGNATURES = {
     "nntr_cuda_gemm_q6_K_dev": (_i, _GEMM_DEV),
     "nntr_cuda_gemm_q4_K_noalloc_dev": (_i, [_u, _u, _u, _vp, _u, _vp, _u, _vp, _u, _vp]),
     "nntr_cuda_gemv_dev": (_i, [_i, _u, _u, _vp, _vp, _vp, _u, _vp]),
+    "nntr_cuda_gemv_rows_dev": (_i, [_i, _u, _u, _u, _vp, _vp, _vp, _u, _vp, _sz, _vp]),
     "nntr_cuda_gemv_batched_dev": (_i, [_i, _u, _u, _vp, _vp, _u, _vp, _u, _vp]),
     "nntr_cuda_gemv_add_norm_dev": (_i, [_i, _u, _u, _vp, _vp, _vp, _vp, C.c_float, _vp, _vp, _u, _vp]),
     "nntr_cuda_gated_ffn_in_dev": (_i, [_i, _u, _u, _vp, _vp, _vp, _vp, C.c_float, _vp, _vp, _vp, _u, _vp]),

@@ -128,11 +128,15 @@ __global__ void rope_cache_append_kernel(float *__restrict__ q, const float *__r
                                          const float *__restrict__ q_gamma, const float *__restrict__ k_gamma, float eps,
                                          uint16_t *__restrict__ kcache, uint16_t *__restrict__ vcache,
                                          const float *__restrict__ cos_tab, const float *__restrict__ sin_tab,
-                                         const unsigned *__restrict__ pos_dev, unsigned pos, int hq, int hkv, int hd) {
+                                         const unsigned *__restrict__ pos_dev, unsigned pos, int hq, int hkv, int hd,
+                                         long long ld) {
   extern __shared__ __align__(16) float rsm[]; // [ROPE_WARPS][hd]
   pdl_launch_dependents(); // the next kernel may start its own prologue (weight prefetch); it waits before it reads
   pdl_wait();
-  const unsigned p = pos_dev ? *pos_dev : pos;
+  const unsigned p = (pos_dev ? *pos_dev : pos) + blockIdx.y; // consecutive tokens, ld elements apart
+  q += blockIdx.y * ld;
+  k += blockIdx.y * ld;
+  v += blockIdx.y * ld;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int head = blockIdx.x * ROPE_WARPS + warp;
   if (head >= hq + 2 * hkv)
@@ -457,6 +461,8 @@ struct AttnStep {
   int groups; // clusters per kv head: more than eight query heads per kv head are split over several
   int rope;   // 0: q is rotated already and the token's rows are in the caches
   int k_bufs, v_bufs;
+  unsigned tokens;   // consecutive tokens (blockIdx.y), q_ld and out_ld elements apart; their rows are in the caches
+  long long q_ld, out_ld;
   int k_box, v_box; // rows a copy brings: a tile, fewer where one short tile is all there is
 };
 
@@ -674,7 +680,9 @@ attn_cluster_kernel(const __grid_constant__ CUtensorMap kmap, const __grid_const
   cluster_arrive(); // "this CTA has started": waited for before the first store into another one
   pdl_launch_dependents();
   pdl_wait();
-  const unsigned p = a.pos_dev ? *a.pos_dev : a.pos;
+  const unsigned p = (a.pos_dev ? *a.pos_dev : a.pos) + blockIdx.y;
+  const float *q_in = a.q + (long long)blockIdx.y * a.q_ld;
+  float *out = a.out + (long long)blockIdx.y * a.out_ld;
   const unsigned first = p + 1 < a.window ? 0u : p + 1 - a.window;
   unsigned cnt = p + 1 - first;
   if (cnt > a.cap_rows)
@@ -705,7 +713,7 @@ attn_cluster_kernel(const __grid_constant__ CUtensorMap kmap, const __grid_const
   /* ---- query heads; the CTA that scores the token's own row also makes its key */
   const float *ct = a.cos_tab + (size_t)p * hd, *sn = a.sin_tab + (size_t)p * hd;
   for (int g = warp; g < gqa + has_own; g += AC_WARPS) {
-    const float *src = g < gqa ? a.q + (size_t)(h0 + g) * hd : a.k + (size_t)n * hd;
+    const float *src = g < gqa ? q_in + (size_t)(h0 + g) * hd : a.k + (size_t)n * hd;
     const float *gamma = g < gqa ? a.q_gamma : a.k_gamma;
     if (!a.rope)
       for (int i = lane; i < hd; i += 32)
@@ -909,7 +917,7 @@ attn_cluster_kernel(const __grid_constant__ CUtensorMap kmap, const __grid_const
     if (d < hd && ok) {
       if (a.rope)
         acc = __fmaf_rn(e[cnt - 1], half_bits_to_float(float_to_half_bits_rn(a.v[(size_t)n * hd + d])), acc);
-      a.out[(size_t)head * hd + d] = acc;
+      out[(size_t)head * hd + d] = acc;
     }
   }
   if (*abort_flag) // give the copies in flight time to land in this CTA's shared memory
@@ -1006,10 +1014,10 @@ static void pdl_cfg(cudaLaunchConfig_t &cfg, cudaLaunchAttribute *attr, unsigned
   cfg.numAttrs = (flags & NNTR_CUDA_GEMV_PDL) ? 1 : 0;
 }
 
-int launch_rope_cache_append(const nntr_attn_desc *a, unsigned pos, const unsigned *pos_dev, float *q, const float *k,
-                             const float *v, const float *q_gamma, const float *k_gamma, float eps, uint16_t *kcache,
-                             uint16_t *vcache, const float *cos_tab, const float *sin_tab, unsigned flags,
-                             cudaStream_t st) {
+static int launch_rope_rows(const nntr_attn_desc *a, unsigned pos, const unsigned *pos_dev, unsigned tokens, size_t ld, float *q,
+                            const float *k, const float *v, const float *q_gamma, const float *k_gamma, float eps,
+                            uint16_t *kcache, uint16_t *vcache, const float *cos_tab, const float *sin_tab, unsigned flags,
+                            cudaStream_t st) {
   int rc = check_attn(a);
   if (rc)
     return rc;
@@ -1019,14 +1027,21 @@ int launch_rope_cache_append(const nntr_attn_desc *a, unsigned pos, const unsign
   cudaLaunchConfig_t cfg = {};
   cudaLaunchAttribute attr[1];
   pdl_cfg(cfg, attr, flags, st);
-  cfg.gridDim = dim3((unsigned)((heads + ROPE_WARPS - 1) / ROPE_WARPS));
+  cfg.gridDim = dim3((unsigned)((heads + ROPE_WARPS - 1) / ROPE_WARPS), tokens);
   cfg.blockDim = dim3(32 * ROPE_WARPS);
   cfg.dynamicSmemBytes = (size_t)ROPE_WARPS * a->head_dim * sizeof(float);
   cudaError_t e = cudaLaunchKernelEx(&cfg, rope_cache_append_kernel, q, k, v, q_gamma, k_gamma, eps, kcache, vcache,
                                      cos_tab, sin_tab, pos_dev, pos, (int)a->n_heads_q, (int)a->n_heads_kv,
-                                     (int)a->head_dim);
+                                     (int)a->head_dim, (long long)ld);
   count_launch();
   return check_cuda(e, "rope_cache_append launch");
+}
+
+int launch_rope_cache_append(const nntr_attn_desc *a, unsigned pos, const unsigned *pos_dev, float *q, const float *k,
+                             const float *v, const float *q_gamma, const float *k_gamma, float eps, uint16_t *kcache,
+                             uint16_t *vcache, const float *cos_tab, const float *sin_tab, unsigned flags,
+                             cudaStream_t st) {
+  return launch_rope_rows(a, pos, pos_dev, 1, 0, q, k, v, q_gamma, k_gamma, eps, kcache, vcache, cos_tab, sin_tab, flags, st);
 }
 
 size_t attention_workspace_bytes(const nntr_attn_desc *a, unsigned max_rows) {
@@ -1048,14 +1063,16 @@ static int launch_attn_cluster(AttnStep a, unsigned bound, unsigned rows, unsign
   while (gqa % a.groups || gqa / a.groups > 8) // at most 16 query heads in all (check_attn)
     ++a.groups;
   gqa /= a.groups;
-  // a CTA owns 64 dimensions of a head where eight CTAs are enough for that, else the whole head
-  const int dims = hd <= 64 || gqa * 2 <= 8 ? 64 : 128;
+  // a CTA owns 64 dimensions of a head where eight CTAs are enough for that, else -- and for many tokens, which fill the
+  // machine anyway -- the whole head
+  const bool many = a.tokens > 1;
+  const int dims = hd <= 64 || (gqa * 2 <= 8 && !many) ? 64 : 128;
   const int items = gqa * ((hd + dims - 1) / dims);
   // eight CTAs per cluster while that leaves no cluster waiting for SMs -- 16 clusters of eight run in two waves (11.1 us for a
   // window of 50 rows, clusters of four 8), because a cluster lies inside one part of the chip --, at least as many as items
   const unsigned clusters = (unsigned)(a.hkv * a.groups);
   unsigned csize = clusters > 12 && items <= 4 ? 4 : 8;
-  while (csize > 1 && clusters * csize > 144u && (int)(csize / 2) >= items)
+  while (csize > 1 && (many || clusters * csize > 144u) && (int)(csize / 2) >= items)
     csize /= 2;
   // buffers for what the launch can need, no more: the next kernel's CTAs want room beside this one's
   a.cap_rows = rows;
@@ -1094,7 +1111,7 @@ static int launch_attn_cluster(AttnStep a, unsigned bound, unsigned rows, unsign
   cfg.attrs = attr;
   cfg.numAttrs = (flags & NNTR_CUDA_GEMV_PDL) ? 2 : 1;
   cfg.stream = st;
-  cfg.gridDim = dim3(clusters * csize);
+  cfg.gridDim = dim3(clusters * csize, a.tokens);
   cfg.blockDim = dim3(AC_THREADS);
   cfg.dynamicSmemBytes = L.total;
   const cudaError_t e = cudaLaunchKernelEx(&cfg, kernel, kmap, vmap, a);
@@ -1128,7 +1145,7 @@ int launch_attention_decode(const nntr_attn_desc *a, unsigned pos, const unsigne
   AttnStep s = {};
   s.q = q, s.kcache = const_cast<uint16_t *>(kcache), s.vcache = const_cast<uint16_t *>(vcache);
   s.out = out, s.sink = a->sink, s.pos_dev = pos_dev, s.pos = pos, s.window = a->window;
-  s.hq = hq, s.hkv = hkv, s.hd = hd;
+  s.hq = hq, s.hkv = hkv, s.hd = hd, s.tokens = 1;
   bool taken;
   if ((rc = launch_attn_cluster(s, bound, rows, flags, st, &taken)) || taken)
     return rc;
@@ -1190,7 +1207,7 @@ int launch_attention_step(const nntr_attn_desc *a, unsigned pos, const unsigned 
   s.kcache = kcache, s.vcache = vcache, s.cos_tab = cos_tab, s.sin_tab = sin_tab;
   s.q_rot = q_rot, s.q_inplace = rows > ATTN_INPLACE_ROWS ? q : nullptr, s.out = out, s.sink = a->sink;
   s.pos_dev = pos_dev, s.pos = pos, s.window = a->window;
-  s.hq = hq, s.hkv = hkv, s.hd = hd, s.rope = 1;
+  s.hq = hq, s.hkv = hkv, s.hd = hd, s.rope = 1, s.tokens = 1;
   bool taken;
   if ((rc = launch_attn_cluster(s, bound, rows, flags, st, &taken)) || taken)
     return rc;
@@ -1200,6 +1217,38 @@ int launch_attention_step(const nntr_attn_desc *a, unsigned pos, const unsigned 
   if (q_rot)
     NNTR_CHECK_CUDA(cudaMemcpyAsync(q_rot, q, (size_t)hq * hd * sizeof(float), cudaMemcpyDeviceToDevice, st));
   return launch_attention_decode(a, pos, pos_dev, max_rows, q, kcache, vcache, out, ws, ws_bytes, flags, st);
+}
+
+/* Consecutive tokens of a prompt: every token's rotary work and cache rows in one launch, every token's attention -- over its own
+ * row and the rows before it -- in a second one. The same kernels as a decode step's, so the same bits as that many steps. */
+int launch_attention_rows(const nntr_attn_desc *a, unsigned pos, unsigned tokens, float *q, const float *k, const float *v,
+                          size_t ld, const float *q_gamma, const float *k_gamma, float eps, uint16_t *kcache, uint16_t *vcache,
+                          const float *cos_tab, const float *sin_tab, float *out, size_t ld_out, unsigned flags,
+                          cudaStream_t st) {
+  int rc = check_attn(a);
+  if (rc)
+    return rc;
+  if (!q || !k || !v || !kcache || !vcache || !cos_tab || !sin_tab || !out)
+    return set_error(NNTR_CUDA_ERR_INVALID, "attention_rows: null pointer");
+  if ((q_gamma == nullptr) != (k_gamma == nullptr))
+    return set_error(NNTR_CUDA_ERR_INVALID, "attention_rows: q_gamma and k_gamma come together or not at all");
+  if ((reinterpret_cast<uintptr_t>(kcache) & 15) || (reinterpret_cast<uintptr_t>(vcache) & 15))
+    return set_error(NNTR_CUDA_ERR_INVALID, "attention_rows: caches must be 16-byte aligned");
+  if (tokens == 0)
+    return NNTR_CUDA_OK;
+  const unsigned bound = pos + tokens, rows = bound < a->window ? bound : a->window;
+  if (tokens > 65535 || a->head_dim > 128 || rows > AC_MAX_ROWS)
+    return set_error(NNTR_CUDA_ERR_UNSUPPORTED, "attention_rows: heads of at most 128 dimensions, windows of at most %u rows",
+                     AC_MAX_ROWS);
+  if ((rc = launch_rope_rows(a, pos, nullptr, tokens, ld, q, k, v, q_gamma, k_gamma, eps, kcache, vcache, cos_tab, sin_tab, flags,
+                             st)))
+    return rc;
+  AttnStep s = {};
+  s.q = q, s.kcache = kcache, s.vcache = vcache, s.out = out, s.sink = a->sink, s.pos = pos, s.window = a->window;
+  s.hq = (int)a->n_heads_q, s.hkv = (int)a->n_heads_kv, s.hd = (int)a->head_dim;
+  s.tokens = tokens, s.q_ld = (long long)ld, s.out_ld = (long long)ld_out;
+  bool taken;
+  return launch_attn_cluster(s, bound, rows, flags & ~NNTR_CUDA_ATTN_SEPARATE, st, &taken);
 }
 
 } // namespace nntr

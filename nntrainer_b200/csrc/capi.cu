@@ -640,6 +640,15 @@ int nntr_cuda_attention_step_dev(const nntr_attn_desc *a, unsigned pos, const un
                                static_cast<cudaStream_t>(stream));
 }
 
+int nntr_cuda_attention_rows_dev(const nntr_attn_desc *a, unsigned pos, unsigned tokens, float *q, const float *k,
+                                 const float *v, size_t ld, const float *q_gamma, const float *k_gamma, float eps,
+                                 void *kcache, void *vcache, const float *cos_tab, const float *sin_tab, float *out,
+                                 size_t ld_out, unsigned flags, void *stream) {
+  return launch_attention_rows(a, pos, tokens, q, k, v, ld, q_gamma, k_gamma, eps, static_cast<uint16_t *>(kcache),
+                               static_cast<uint16_t *>(vcache), cos_tab, sin_tab, out, ld_out, flags,
+                               static_cast<cudaStream_t>(stream));
+}
+
 int nntr_cuda_bin_layout(const nntr_bin_tensor *t, size_t n, size_t *data_offset, size_t *bytes, size_t *total) {
   return bin_layout(t, n, data_offset, bytes, total);
 }
@@ -708,6 +717,28 @@ int nntr_cuda_gemv_dev(int qtype, unsigned N, unsigned K, const float *x, const 
   default:
     return launch_gemv_q6_K(N, K, x, B, y, flags, st);
   }
+}
+
+int nntr_cuda_gemv_rows_dev(int qtype, unsigned M, unsigned N, unsigned K, const float *A, const void *B, float *C,
+                            unsigned ldc, void *ws, size_t ws_bytes, void *stream) {
+  int rc = check_weight_shape(qtype, N, K);
+  if (rc)
+    return rc;
+  if (M == 0 || N == 0)
+    return NNTR_CUDA_OK;
+  if (!A || !B || !C)
+    return set_error(NNTR_CUDA_ERR_INVALID, "gemv_rows: null pointer");
+  cudaStream_t st = static_cast<cudaStream_t>(stream);
+  if (M == 1)
+    return nntr_cuda_gemv_dev(qtype, N, K, A, B, C, 0, stream);
+  if (ldc < N)
+    return set_error(NNTR_CUDA_ERR_INVALID, "gemv_rows: ldc (%u) < N (%u)", ldc, N);
+  const size_t need = workspace_bytes(qtype, M, N, K);
+  if (!ws || ws_bytes < need)
+    return set_error(NNTR_CUDA_ERR_INVALID, "gemv_rows: workspace of %zu bytes needed, %zu given", need, ws_bytes);
+  if (qtype == NNTR_Q6_K) // one chain for all rows anyway
+    return launch_gemm_mma_q6_K(M, N, K, A, B, C, ldc, ws, st);
+  return launch_gemm_mma(qtype, M, 0, N, K, A, B, C, ldc, ws, ws_bytes, st); // no row takes the four-row chain
 }
 
 int nntr_cuda_gemv_batched_dev(int qtype, unsigned N, unsigned K, const float *x, const void *const *w_table,

@@ -548,6 +548,8 @@ __global__ void __launch_bounds__(ROWS_WARPS * 32, NT == 4 ? 3 : 4) gemm_mma_row
           q4k_unit<n, CHAIN_ONE, true>(acc, accm, sc, w0, w1, act, 8, 0, g, t, lane);
         else if (TH8 && tl.pos + tl.rows <= a.M4)
           q4k_unit<n, CHAIN_FOUR, true>(acc, accm, sc, w0, w1, act, 8, 0, g, t, lane);
+        else if (TH8 && tl.pos >= a.M4)
+          q4k_unit<n, CHAIN_ONE, true>(acc, accm, sc, w0, w1, act, 8, 0, g, t, lane);
         else // the last tile, with up to three rows of the one-step chain
           q4k_unit<n, CHAIN_MIXED, TH8>(acc, accm, sc, w0, w1, act, th, a.M4 - tl.pos, g, t, lane);
       });

@@ -217,21 +217,77 @@ class Qwen3Decoder:
         torch.cuda.current_stream().wait_stream(s)
         return g
 
+    # Prompt tokens per batched pass: enough rows for the matrix kernels to read every weight once or a few times, few enough
+    # for buffers of a few tens of megabytes.
+    PROMPT_ROWS = 256
+
+    def _prompt(self, ids, pos: int):
+        """Fills the caches with the rows of the tokens ``ids`` from position ``pos`` on, all of them through each layer
+        together. Every row runs the decode kernels' float chains (gemv_rows, Attention.rows, row norms), so the caches equal
+        those of decoding the tokens one by one bit for bit. The last layer needs its keys and values only."""
+        torch, c, pdl = self.torch, self.cfg, self.pdl
+        T, q_dim, kv_dim = len(ids), c.n_heads * c.head_dim, c.n_kv_heads * c.head_dim
+        ld = q_dim + 2 * kv_dim
+        f = lambda n: torch.empty((T, n), dtype=torch.float32, device=self.dev)  # noqa: E731
+        x, h, n, qkv, a, o, d = (f(k) for k in (c.hidden, c.hidden, c.hidden, ld, q_dim, c.hidden, c.hidden))
+        up, gate = f(c.inter), f(c.inter)
+        need = max(be.gemm_workspace_bytes(c.fc_dtype, T, N, K) for N, K in (
+            (ld, c.hidden), (q_dim, c.hidden), (kv_dim, c.hidden), (c.hidden, q_dim), (c.inter, c.hidden), (c.hidden, c.inter)))
+        ws = torch.empty(max(need, 16), dtype=torch.uint8, device=self.dev)
+        be.embedding(c.embedding_dtype, self._P(self.ptr["embedding0"]),
+                     torch.tensor([float(t) for t in ids], dtype=torch.float32).to(self.dev), c.vocab, c.hidden, out=x, pdl=pdl)
+
+        def rows(name, src, dst, ldc):
+            dtype, N, K = self._shape[name]
+            be.gemv_rows(dtype, T, N, K, src, self._P(self.ptr[name]), dst, ldc, ws)
+
+        q, k, v = qkv, qkv[:, q_dim:], qkv[:, q_dim + kv_dim:]
+        for i in range(c.n_layers):
+            p = f"layer{i}_"
+            qk_norm = (self._P(self.ptr[p + "q_norm"]), self._P(self.ptr[p + "k_norm"]), c.norm_eps)
+            if i == 0:
+                self._norm(x, p + "attention_norm", n)
+            else:
+                be.add_rms_norm(h, d, self._P(self.ptr[p + "attention_norm"]), c.norm_eps, sum_out=x, out=n, pdl=pdl)
+            if self._qkv_packed:
+                be.gemv_rows(c.fc_dtype, T, ld, c.hidden, n, self._qkv_packed[i], qkv, ld, ws)
+            else:
+                rows(p + "wq", n, q, ld)
+                rows(p + "wk", n, k, ld)
+                rows(p + "wv", n, v, ld)
+            self.attn[i].rows(q, k, v, ld, pos, T, a, q_dim, qk_norm=qk_norm, pdl=pdl)
+            if i + 1 == c.n_layers:
+                return
+            rows(p + "attention_out", a, o, c.hidden)
+            be.add_rms_norm(x, o, self._P(self.ptr[p + "ffn_norm"]), c.norm_eps, sum_out=h, out=n, pdl=pdl)
+            rows(p + "ffn_up", n, up, c.inter)
+            rows(p + "ffn_gate", n, gate, c.inter)
+            be.swiglu(up, gate, out=up, pdl=pdl)
+            rows(p + "ffn_down", up, d, c.hidden)
+
     def generate(self, prompt_ids, n_new: int):
-        """Feeds the prompt one token at a time, then ``n_new`` greedy tokens; returns them as a Python list."""
-        torch = self.torch
+        """Feeds the prompt, then ``n_new`` greedy tokens; returns them as a Python list. All of the prompt but its last token
+        goes through the layers in batched passes (where their kernels apply: heads of up to 128 dimensions, hidden rows of
+        up to 11264, up to 16384 positions), with the results of feeding it token by token; the token ids stay on the device until
+        the end."""
+        torch, c = self.torch, self.cfg
+        prompt_ids = list(prompt_ids)
         tok = torch.empty(1, dtype=torch.float32, device=self.dev)
-        out, pos = [], 0
-        for t in prompt_ids:
+        out = torch.empty(n_new + 1, dtype=torch.int32, device=self.dev)
+        pos = 0
+        if len(prompt_ids) > 3 and c.head_dim <= 128 and c.hidden <= 11264 and c.max_seq <= 16384:
+            while pos < len(prompt_ids) - 1:
+                n = min(self.PROMPT_ROWS, len(prompt_ids) - 1 - pos)
+                self._prompt(prompt_ids[pos:pos + n], pos)
+                pos += n
+        for t in prompt_ids[pos:]:
             tok.fill_(float(t))
-            nxt, nxt_f = self.step(tok, pos)
+            self.step(tok, pos, out_idx=out[:1], out_idx_f=tok)
             pos += 1
-        for _ in range(n_new):
-            out.append(int(nxt.item()))
-            tok.copy_(nxt_f)
-            nxt, nxt_f = self.step(tok, pos)
+        for i in range(n_new):
+            self.step(tok, pos, out_idx=out[i + 1:i + 2], out_idx_f=tok)
             pos += 1
-        return out
+        return out[:n_new].tolist()
 
     def close(self):
         self.w.close()

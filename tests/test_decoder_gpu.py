@@ -79,3 +79,35 @@ def test_sliding_window_shorter_than_the_context(be):
     got, want, gl, cl, _ = _run(be, cfg, prompt=[1, 2, 3], n_new=40, seed=1)
     assert got == want
     assert np.array_equal(gl.view(np.uint32), cl.view(np.uint32))
+
+
+@pytest.mark.parametrize("window,fc,P", [(None, "q4_K", 2), (None, "q4_K", 9), (16, "q4_K", 40), (None, "q6_K", 33),
+                                         (None, "q4_K", 300)])
+def test_batched_prompt_equals_token_by_token(be, window, fc, P):
+    """The prompt's batched pass against feeding the prompt through step(): tokens, final logits and both caches of every
+    layer, equal bits -- a prompt too short to be batched, ragged tiles of eight rows, a window shorter than the prompt,
+    separate q, k and v projections (Q6_K), and more tokens than one pass takes."""
+    cfg = DecoderConfig(n_layers=3, hidden=512, n_heads=8, n_kv_heads=2, head_dim=64, inter=768, vocab=1024, max_seq=P + 8,
+                        sliding_window=window, fc_dtype=fc)
+    w = synthetic_weights(cfg, 3)
+    rng = np.random.default_rng(P)
+    prompt = [int(t) for t in rng.integers(0, cfg.vocab, P)]
+    with tempfile.TemporaryDirectory() as td:
+        path = os.path.join(td, "model.bin")
+        write_bin(path, cfg, w)
+        got, want = Qwen3Decoder(cfg, path), Qwen3Decoder(cfg, path)
+    tokens = got.generate(prompt, 4)
+    ref, tok = [], torch.empty(1, device="cuda")
+    for pos in range(P + 4):
+        tok.fill_(float(prompt[pos] if pos < P else ref[-1]))
+        nxt, _ = want.step(tok, pos)
+        if pos >= P - 1 and len(ref) < 4:
+            ref.append(int(nxt.item()))
+    be.device_status()
+    assert tokens == ref
+    assert torch.equal(got.b["logits"].view(torch.int32), want.b["logits"].view(torch.int32))
+    for a, b in zip(got.attn, want.attn):
+        assert torch.equal(a.kcache.view(torch.int16), b.kcache.view(torch.int16))
+        assert torch.equal(a.vcache.view(torch.int16), b.vcache.view(torch.int16))
+    got.close()
+    want.close()
