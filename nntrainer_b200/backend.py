@@ -39,7 +39,13 @@ def launch_count() -> int:
 
 
 def _stream() -> int:
-    return int(_torch().cuda.current_stream().cuda_stream)
+    """torch's current stream on the current device. Asked of torch's C layer: building a Stream object for it costs more than
+    the launch it is for."""
+    C = _torch()._C
+    try:
+        return C._cuda_getCurrentRawStream(C._cuda_getDevice())
+    except (AttributeError, RuntimeError):  # another torch, or CUDA not initialised yet
+        return int(_torch().cuda.current_stream().cuda_stream)
 
 
 def _np_ptr(a: np.ndarray) -> int:
@@ -74,14 +80,22 @@ def _gemm(qtype: str, M: int, N: int, K: int, A, lda: int, B, ldb: int, C, ldc: 
     torch = _torch()
     if not (A.is_cuda and B.is_cuda and C.is_cuda):
         raise ValueError("device path needs CUDA tensors for A, B and C")
+    fn = getattr(L, _GEMM_DEV[qtype])
+    if M == 1:  # a decode step: no workspace, and short enough for the call itself to count
+        rc = fn(1, N, K, A.data_ptr(), lda, B.data_ptr(), ldb, C.data_ptr(), ldc, None, 0, _stream())
+        if rc:
+            check(rc)
+        return C
     need = int(L.nntr_cuda_gemm_workspace_bytes(QTYPE[qtype], M, N, K))
     if need and (workspace is None or workspace.numel() * workspace.element_size() < need):
         workspace = torch.empty(need, dtype=torch.uint8, device=A.device)
     ws_ptr = workspace.data_ptr() if workspace is not None else 0
     ws_len = workspace.numel() * workspace.element_size() if workspace is not None else 0
-    fn = getattr(L, f"nntr_cuda_gemm_{qtype}_dev")
     check(fn(M, N, K, A.data_ptr(), lda, B.data_ptr(), ldb, C.data_ptr(), ldc, ws_ptr, ws_len, _stream()))
     return C
+
+
+_GEMM_DEV = {q: f"nntr_cuda_gemm_{q}_dev" for q in ("q4_0", "q4_K", "q6_K")}
 
 
 class _HostBlock:
@@ -342,11 +356,15 @@ class MoeLayer:
                                  ptr(self._tabs[0]), ptr(self._tabs[1]), ptr(self._tabs[2]), ptr(self._tabs[3]),
                                  ptr(self._tabs[4]), ptr(self._tabs[5]), alpha)
         self._ws = None
+        self._ws_need = {}
         self._C = C
+        self._desc_ref = C.byref(self.desc)
 
     def _workspace(self, tokens):
         torch = _torch()
-        need = int(lib().nntr_cuda_moe_workspace_bytes(self._C.byref(self.desc), tokens))
+        need = self._ws_need.get(tokens)
+        if need is None:
+            need = self._ws_need[tokens] = int(lib().nntr_cuda_moe_workspace_bytes(self._desc_ref, tokens))
         if self._ws is None or self._ws.numel() < need:
             self._ws = torch.zeros(need, dtype=torch.uint8, device=self._keep[0].device)  # zero-filled before first use
         return self._ws
@@ -356,8 +374,9 @@ class MoeLayer:
         T = x.shape[0]
         y = torch.empty((T, self.H), dtype=torch.float32, device=x.device)
         ws = self._workspace(T)
-        check(lib().nntr_cuda_moe_forward_dev(self._C.byref(self.desc), T, x.data_ptr(), y.data_ptr(), ws.data_ptr(),
-                                              ws.numel(), _stream()))
+        rc = lib().nntr_cuda_moe_forward_dev(self._desc_ref, T, x.data_ptr(), y.data_ptr(), ws.data_ptr(), ws.numel(), _stream())
+        if rc:
+            check(rc)
         return y
 
     def enable_expert_parallel(self, max_tokens: int, layers_per_epoch: int = 1, group=None, share_with=None):

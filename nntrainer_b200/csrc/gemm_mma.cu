@@ -287,17 +287,17 @@ template <int NT> __device__ __forceinline__ bool find_tile(Tile &tl, const MmaA
     tl.rows = min(8 * NT, a.M - tl.pos);
     return true;
   }
-  // the expert whose tiles of 8 * NT rows hold this one
-  if (tile >= a.tile_off[a.n_experts])
-    return false;
-  int lo = 0, hi = a.n_experts;
-  while (hi - lo > 1) {
-    const int mid = (lo + hi) >> 1;
-    if (a.tile_off[mid] <= tile)
-      lo = mid;
-    else
-      hi = mid;
+  // the expert whose tiles of 8 * NT rows hold this one: the last one that starts at or before it. All offsets are loaded at
+  // once (one round trip; a binary search is a chain of five to eight, a third of a small CTA's life).
+  const int lane = threadIdx.x & 31, end = a.tile_off[a.n_experts];
+  int lo = -1;
+#pragma unroll
+  for (int i = 0; i < 8; ++i) { // at most 256 experts
+    const int x = 32 * i + lane;
+    lo += __popc(__ballot_sync(FULL, x < a.n_experts && a.tile_off[x < a.n_experts ? x : 0] <= tile));
   }
+  if (tile >= end)
+    return false;
   const int k = tile - a.tile_off[lo], first = k * 8 * NT;
   tl.W = (tl.z ? a.w_table[1] : a.w_table[0])[lo];
   tl.pos = a.off[lo] + first;

@@ -51,6 +51,7 @@ constexpr int MOE_COUNTER_TOKENS = 4096;   // arrival counters kept at the start
 constexpr int ROUTER_WARPS = 8;
 constexpr int ROUTER_SLICES = 32; // CTAs per token
 constexpr int MAX_E_PER_LANE = 8; // up to 256 experts
+constexpr unsigned ROUTER_ROWS_MIN_TOKENS = 48; // below, a CTA row per token has the weight in L2 anyway and more CTAs
 constexpr int ROUTER_PRE = 8;     // rows of a warp's slice fetched before the dependency wait
 
 /* std::partial_sort(idx, idx + k, idx + n, [&](a, b) { return v[a] > v[b]; }) on idx = 0..n-1, as the GNU C++ library
@@ -101,16 +102,157 @@ __device__ void partial_sort_desc(const float *v, int n, int k, int *out) {
     out[i] = h[i];
 }
 
+/* What a routed token leaves behind, and the scratch of the partial logits. */
+struct RouterOut {
+  const float *bias;
+  int topk;
+  const void *const *gate_w, *const *up_w, *const *down_w;
+  int *idx, *ord;
+  float *w;
+  const void **gu_table, **dn_table;
+  float *rpart;     // [token][slice][E]
+  unsigned *rcount; // arrivals per token (or group of tokens)
+};
+
+/* One warp: logits, softmax and top-k of token t from its partial sums. area: E + 32 floats of shared memory. PER: experts per
+ * lane at most (4: up to 128 experts). */
+template <int PER>
+__device__ __forceinline__ void router_finish(const RouterOut &o, int t, int E, int lane, float *area) {
+  const int per = (E + 31) / 32, topk = o.topk;
+  const float *rpart = o.rpart, *bias = o.bias;
+  const void *const *gate_w = o.gate_w, *const *up_w = o.up_w, *const *down_w = o.down_w;
+  int *idx_out = o.idx, *ord_out = o.ord;
+  float *w_out = o.w;
+  const void **gu_table = o.gu_table, **dn_table = o.dn_table;
+  float p[PER];
+  float mx = -INFINITY;
+#pragma unroll
+  for (int i = 0; i < PER; ++i)
+    p[i] = 0.f;
+  constexpr int FLY = 64 / PER; // partial sums of that many slices are on their way at a time, added in order
+#pragma unroll
+  for (int w0 = 0; w0 < ROUTER_SLICES; w0 += FLY) {
+    float v[FLY][PER];
+#pragma unroll
+    for (int w = 0; w < FLY; ++w)
+#pragma unroll
+      for (int i = 0; i < PER; ++i)
+        v[w][i] = __ldcg(rpart + ((size_t)t * ROUTER_SLICES + w0 + w) * E + min(lane + 32 * i, E - 1));
+#pragma unroll
+    for (int w = 0; w < FLY; ++w)
+#pragma unroll
+      for (int i = 0; i < PER; ++i)
+        p[i] += v[w][i];
+  }
+#pragma unroll
+  for (int i = 0; i < PER; ++i) {
+    const int e = lane + 32 * i;
+    if (i < per && e < E) {
+      p[i] += bias ? bias[e] : 0.f;
+      mx = fmaxf(mx, p[i]);
+    } else {
+      p[i] = -INFINITY;
+    }
+  }
+  for (int o = 16; o; o >>= 1)
+    mx = fmaxf(mx, __shfl_xor_sync(FULL, mx, o));
+  float sum = 0.f;
+#pragma unroll
+  for (int i = 0; i < PER; ++i) {
+    const int e = lane + 32 * i;
+    if (i < per && e < E) {
+      p[i] = (float)exp((double)__fsub_rn(p[i], mx)); // exp_util<float>: the double exponential, rounded to float
+      sum += p[i];
+    } else {
+      p[i] = -1.f; // never selected: probabilities are >= 0
+    }
+  }
+  for (int o = 16; o; o >>= 1)
+    sum += __shfl_xor_sync(FULL, sum, o);
+#pragma unroll
+  for (int i = 0; i < PER; ++i)
+    if (p[i] >= 0.f)
+      p[i] = __fdiv_rn(p[i], sum);
+  // top-k in the order Tensor::topK returns it: std::partial_sort over the expert indices with the comparator
+  // "probability greater" (nntrainer/tensor/float_tensor.cpp:1155-1160). With distinct values that is plain descending
+  // order: k (+1) rounds of a warp arg-max. Among EQUAL probabilities the library's order comes from its heap moves,
+  // so when a tie touches the selection (two equal values among the k + 1 greatest) one lane reruns the selection
+  // with the library's own procedure.
+  float *pv = area; // the probabilities, expert-indexed
+  __syncwarp();
+#pragma unroll
+  for (int i = 0; i < PER; ++i) {
+    const int e = lane + 32 * i;
+    if (i < per && e < E)
+      pv[e] = p[i];
+  }
+  int *sel = reinterpret_cast<int *>(area + E); // [topk]
+  float prev = -1.f;
+  bool tie = false;
+  const int rounds = topk < E ? topk + 1 : topk;
+  for (int k = 0; k < rounds; ++k) {
+    float bv = -1.f;
+    int be = 0x7fffffff;
+#pragma unroll
+    for (int i = 0; i < PER; ++i) {
+      const int e = lane + 32 * i;
+      if (p[i] > bv) { // ascending e within the lane: the first maximum wins
+        bv = p[i];
+        be = e;
+      }
+    }
+    for (int o = 16; o; o >>= 1) {
+      const float ov = __shfl_xor_sync(FULL, bv, o);
+      const int oe = __shfl_xor_sync(FULL, be, o);
+      if (ov > bv || (ov == bv && oe < be)) {
+        bv = ov;
+        be = oe;
+      }
+    }
+    if ((be & 31) == lane) { // the owner retires the winner
+#pragma unroll
+      for (int i = 0; i < PER; ++i)
+        if (i == (be >> 5))
+          p[i] = -1.f;
+    }
+    tie = tie || (k > 0 && bv == prev);
+    prev = bv;
+    if (k < topk && lane == 0)
+      sel[k] = be;
+  }
+  __syncwarp();
+  if (tie && lane == 0)
+    partial_sort_desc(pv, E, topk, sel);
+  __syncwarp();
+  float vsel = 0.f;
+  int esel = 0;
+  float ksum = 0.f;
+  for (int k = 0; k < topk; ++k)
+    ksum += pv[sel[k]]; // same sequential sum in every lane
+  if (lane < topk) {
+    esel = sel[lane];
+    vsel = pv[esel];
+  }
+  if (lane < topk) {
+    const int pr = t * topk + lane;
+    idx_out[pr] = esel;
+    w_out[pr] = __fdiv_rn(vsel, ksum);
+    gu_table[2 * pr] = gate_w[esel];
+    gu_table[2 * pr + 1] = up_w[esel];
+    dn_table[pr] = down_w[esel];
+    // the combine adds a token's experts in ascending index: slot of the k-th smallest, for its use
+    int rank = 0;
+    for (int j = 0; j < topk; ++j)
+      rank += sel[j] < esel;
+    ord_out[t * topk + rank] = lane;
+  }
+}
+
 /* ROUTER_SLICES CTAs per token: each sums its slice of the hidden dimension into partial logits (the router weight
  * is a megabyte per layer: a few CTAs alone would be bound by the latency of their own loads); the CTA that arrives last on
  * the token's counter adds the partials in slice order and does softmax, top-k and the tables. */
 __global__ void __launch_bounds__(ROUTER_WARPS * 32)
-moe_router_kernel(const float *__restrict__ x, const float *__restrict__ wr, const float *__restrict__ bias, int H, int E,
-                  int topk, const void *const *__restrict__ gate_w, const void *const *__restrict__ up_w,
-                  const void *const *__restrict__ down_w, int *__restrict__ idx_out, int *__restrict__ ord_out,
-                  float *__restrict__ w_out,
-                  const void **__restrict__ gu_table, const void **__restrict__ dn_table, float *__restrict__ rpart,
-                  unsigned *__restrict__ rcount, MoeEp ep) {
+moe_router_kernel(const float *__restrict__ x, const float *__restrict__ wr, int H, int E, const RouterOut o, MoeEp ep) {
   extern __shared__ float rsm[]; // [ROUTER_WARPS][E]
   __shared__ bool is_last;
   const int t = blockIdx.x, sl = blockIdx.y, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -175,7 +317,7 @@ moe_router_kernel(const float *__restrict__ x, const float *__restrict__ wr, con
     if (i < per && lane + 32 * i < E)
       rsm[warp * E + lane + 32 * i] = acc[i];
   __syncthreads();
-  float *mine = rpart + ((size_t)t * ROUTER_SLICES + sl) * E;
+  float *mine = o.rpart + ((size_t)t * ROUTER_SLICES + sl) * E;
   for (int e = threadIdx.x; e < E; e += ROUTER_WARPS * 32) {
     float s = 0.f;
     for (int w = 0; w < ROUTER_WARPS; ++w)
@@ -185,122 +327,101 @@ moe_router_kernel(const float *__restrict__ x, const float *__restrict__ wr, con
   __threadfence();
   __syncthreads();
   if (threadIdx.x == 0) {
-    const unsigned old = atomicAdd(rcount + t, 1u);
+    const unsigned old = atomicAdd(o.rcount + t, 1u);
     is_last = old == ROUTER_SLICES - 1;
     if (is_last)
-      rcount[t] = 0; // ready for the next call
+      o.rcount[t] = 0; // ready for the next call
   }
   __syncthreads();
   if (!is_last || warp != 0)
     return;
   __threadfence();
-  // ---- warp 0: logits, softmax, top-k
-  float p[MAX_E_PER_LANE];
-  float mx = -INFINITY;
-#pragma unroll
-  for (int i = 0; i < MAX_E_PER_LANE; ++i) {
-    p[i] = -INFINITY;
-    const int e = lane + 32 * i;
-    if (i < per && e < E) {
-      float s = 0.f;
-      for (int w = 0; w < ROUTER_SLICES; ++w)
-        s += __ldcg(rpart + ((size_t)t * ROUTER_SLICES + w) * E + e);
-      p[i] = s + (bias ? bias[e] : 0.f);
-      mx = fmaxf(mx, p[i]);
-    }
+  if (E <= 128)
+    router_finish<4>(o, t, E, lane, rsm);
+  else
+    router_finish<8>(o, t, E, lane, rsm);
+}
+
+/* The same for a batch: a CTA takes TT tokens through its slice, so that the router weight crosses the L2 once per TT tokens
+ * instead of once per token, and the last arriver's warps finish a token each. Every sum is formed in the order of the kernel
+ * above (row by row inside a warp, then warp by warp, then slice by slice), so a token is routed alike by both. 256 tokens,
+ * 2048 x 128 weights: 34 us, 94 with a CTA row per token. */
+template <int TT>
+__global__ void __launch_bounds__(ROUTER_WARPS * 32)
+moe_router_rows_kernel(const float *__restrict__ x, const float *__restrict__ wr, int T, int H, int E, const RouterOut o) {
+  extern __shared__ float rsm[]; // [ROUTER_WARPS][TT][E], then the slice of the activations [TT][rows]
+  __shared__ bool is_last;
+  const int t0 = blockIdx.x * TT, sl = blockIdx.y, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  pdl_launch_dependents();
+  const int nw = ROUTER_SLICES * ROUTER_WARPS, wi = sl * ROUTER_WARPS + warp;
+  const int h0 = (int)(((long long)wi * H) / nw), h1 = (int)(((long long)(wi + 1) * H) / nw);
+  const int s0 = (int)(((long long)sl * ROUTER_WARPS * H) / nw), s1 = (int)(((long long)(sl + 1) * ROUTER_WARPS * H) / nw);
+  const int rows = s1 - s0, per = (E + 31) / 32;
+  float *xs = rsm + ROUTER_WARPS * TT * E;
+  pdl_wait();
+  for (int i = threadIdx.x; i < TT * rows; i += ROUTER_WARPS * 32) {
+    const int k = i / rows, h = i - k * rows;
+    xs[i] = t0 + k < T ? x[(size_t)(t0 + k) * H + s0 + h] : 0.f;
   }
-  for (int o = 16; o; o >>= 1)
-    mx = fmaxf(mx, __shfl_xor_sync(FULL, mx, o));
-  float sum = 0.f;
+  float acc[TT][MAX_E_PER_LANE];
 #pragma unroll
-  for (int i = 0; i < MAX_E_PER_LANE; ++i) {
-    const int e = lane + 32 * i;
-    if (i < per && e < E) {
-      p[i] = (float)exp((double)__fsub_rn(p[i], mx)); // exp_util<float>: the double exponential, rounded to float
-      sum += p[i];
-    } else {
-      p[i] = -1.f; // never selected: probabilities are >= 0
-    }
-  }
-  for (int o = 16; o; o >>= 1)
-    sum += __shfl_xor_sync(FULL, sum, o);
+  for (int k = 0; k < TT; ++k)
 #pragma unroll
-  for (int i = 0; i < MAX_E_PER_LANE; ++i)
-    if (p[i] >= 0.f)
-      p[i] = __fdiv_rn(p[i], sum);
-  // top-k in the order Tensor::topK returns it: std::partial_sort over the expert indices with the comparator
-  // "probability greater" (nntrainer/tensor/float_tensor.cpp:1155-1160). With distinct values that is plain descending
-  // order: k (+1) rounds of a warp arg-max. Among EQUAL probabilities the library's order comes from its heap moves,
-  // so when a tie touches the selection (two equal values among the k + 1 greatest) one lane reruns the selection
-  // with the library's own procedure.
-  float *pv = rsm; // the probabilities, expert-indexed (the partial sums kept here are no longer needed)
-  __syncwarp();
+    for (int i = 0; i < MAX_E_PER_LANE; ++i)
+      acc[k][i] = 0.f;
+  __syncthreads();
+  for (int h = h0; h < h1; h += 4) { // four rows in flight per lane
+    float wv[4][MAX_E_PER_LANE];
 #pragma unroll
-  for (int i = 0; i < MAX_E_PER_LANE; ++i) {
-    const int e = lane + 32 * i;
-    if (i < per && e < E)
-      pv[e] = p[i];
-  }
-  int *sel = reinterpret_cast<int *>(rsm + E); // [topk], room: ROUTER_WARPS * E floats with ROUTER_WARPS >= 2
-  float prev = -1.f;
-  bool tie = false;
-  const int rounds = topk < E ? topk + 1 : topk;
-  for (int k = 0; k < rounds; ++k) {
-    float bv = -1.f;
-    int be = 0x7fffffff;
-#pragma unroll
-    for (int i = 0; i < MAX_E_PER_LANE; ++i) {
-      const int e = lane + 32 * i;
-      if (p[i] > bv) { // ascending e within the lane: the first maximum wins
-        bv = p[i];
-        be = e;
-      }
-    }
-    for (int o = 16; o; o >>= 1) {
-      const float ov = __shfl_xor_sync(FULL, bv, o);
-      const int oe = __shfl_xor_sync(FULL, be, o);
-      if (ov > bv || (ov == bv && oe < be)) {
-        bv = ov;
-        be = oe;
-      }
-    }
-    if ((be & 31) == lane) { // the owner retires the winner
+    for (int u = 0; u < 4; ++u) {
+      const float *row = wr + (size_t)(h + u < h1 ? h + u : h1 - 1) * E;
 #pragma unroll
       for (int i = 0; i < MAX_E_PER_LANE; ++i)
-        if (i == (be >> 5))
-          p[i] = -1.f;
+        wv[u][i] = (i < per && lane + 32 * i < E) ? row[lane + 32 * i] : 0.f;
     }
-    tie = tie || (k > 0 && bv == prev);
-    prev = bv;
-    if (k < topk && lane == 0)
-      sel[k] = be;
+#pragma unroll
+    for (int u = 0; u < 4; ++u)
+      if (h + u < h1)
+#pragma unroll
+        for (int k = 0; k < TT; ++k) {
+          const float xv = xs[k * rows + h + u - s0];
+#pragma unroll
+          for (int i = 0; i < MAX_E_PER_LANE; ++i)
+            if (i < per)
+              acc[k][i] = fmaf(xv, wv[u][i], acc[k][i]);
+        }
   }
-  __syncwarp();
-  if (tie && lane == 0)
-    partial_sort_desc(pv, E, topk, sel);
-  __syncwarp();
-  float vsel = 0.f;
-  int esel = 0;
-  float ksum = 0.f;
-  for (int k = 0; k < topk; ++k)
-    ksum += pv[sel[k]]; // same sequential sum in every lane
-  if (lane < topk) {
-    esel = sel[lane];
-    vsel = pv[esel];
+#pragma unroll
+  for (int k = 0; k < TT; ++k)
+#pragma unroll
+    for (int i = 0; i < MAX_E_PER_LANE; ++i)
+      if (i < per && lane + 32 * i < E)
+        rsm[(warp * TT + k) * E + lane + 32 * i] = acc[k][i];
+  __syncthreads();
+  for (int i = threadIdx.x; i < TT * E; i += ROUTER_WARPS * 32) {
+    const int k = i / E, e = i - k * E;
+    if (t0 + k >= T)
+      break;
+    float s = 0.f;
+#pragma unroll
+    for (int w = 0; w < ROUTER_WARPS; ++w)
+      s += rsm[(w * TT + k) * E + e];
+    o.rpart[((size_t)(t0 + k) * ROUTER_SLICES + sl) * E + e] = s;
   }
-  if (lane < topk) {
-    const int pr = t * topk + lane;
-    idx_out[pr] = esel;
-    w_out[pr] = __fdiv_rn(vsel, ksum);
-    gu_table[2 * pr] = gate_w[esel];
-    gu_table[2 * pr + 1] = up_w[esel];
-    dn_table[pr] = down_w[esel];
-    // the combine adds a token's experts in ascending index: slot of the k-th smallest, for its use
-    int rank = 0;
-    for (int j = 0; j < topk; ++j)
-      rank += sel[j] < esel;
-    ord_out[t * topk + rank] = lane;
+  __threadfence();
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    const unsigned old = atomicAdd(o.rcount + t0, 1u);
+    is_last = old == ROUTER_SLICES - 1;
+    if (is_last)
+      o.rcount[t0] = 0; // ready for the next call
   }
+  __syncthreads();
+  if (!is_last)
+    return;
+  __threadfence();
+  for (int k = warp; k < TT && t0 + k < T; k += ROUTER_WARPS)
+    router_finish<TT == 8 ? 4 : 8>(o, t0 + k, E, lane, rsm + warp * (E + 32));
 }
 
 /* Sorts the (token, expert) pairs of a batch by expert: off[e] = first position of expert e's pairs in perm, tile_off[e]
@@ -438,12 +559,16 @@ __global__ void moe_combine_kernel(const float *__restrict__ dn, const int *__re
                                    long total) {
   pdl_launch_dependents();
   pdl_wait();
-  const long i = (long)blockIdx.x * blockDim.x + threadIdx.x;
+  const long i = ((long)blockIdx.x * blockDim.x + threadIdx.x) * 4; // H % 8 == 0: four outputs of one token
   if (i >= total)
     return;
   const long t = i / H;
   const int h = (int)(i - t * H);
-  y[i] = moe_combine_elem(dn, idx, ord, w, down_b, t, h, H, topk);
+  const float4 v = moe_combine_elem4(dn, idx, ord, w, down_b, t, h, H, topk);
+  if (!(reinterpret_cast<uintptr_t>(y) & 15))
+    *reinterpret_cast<float4 *>(y + i) = v;
+  else
+    y[i] = v.x, y[i + 1] = v.y, y[i + 2] = v.z, y[i + 3] = v.w;
 }
 
 /** upper bound on the polls of waits on other ranks' data (0: the default of 2^22); set from the host */
@@ -650,29 +775,39 @@ static int moe_forward(const nntr_moe_desc *d, const nntr_moe_ep *epd, unsigned 
   float *dn = reinterpret_cast<float *>(ws + s.dn);
   const unsigned P = tokens * K;
 
+  const bool grouped = !epd && tokens >= GROUPED_MIN_TOKENS;
   // the arrival counters start at zero (the workspace is zero-filled before its first use) and the last arriver of
   // every token puts its counter back, so no clearing launch is needed
   if (tokens > (unsigned)MOE_COUNTER_TOKENS)
     NNTR_CHECK_CUDA(cudaMemsetAsync(ws + s.rcount, 0, (size_t)tokens * 4, st));
   {
     cudaLaunchConfig_t cfg = {};
+    const RouterOut out = {d->router_bias, (int)K, d->gate_w, d->up_w, d->down_w, idx, ord, w, gu_tab, dn_tab,
+                           reinterpret_cast<float *>(ws + s.rpart), reinterpret_cast<unsigned *>(ws + s.rcount)};
     cfg.gridDim = dim3(tokens, ROUTER_SLICES);
     cfg.blockDim = dim3(ROUTER_WARPS * 32);
-    cfg.dynamicSmemBytes = ROUTER_WARPS * E * sizeof(float);
+    cfg.dynamicSmemBytes = (ROUTER_WARPS * E + 32) * sizeof(float);
     cfg.stream = st;
     cudaLaunchAttribute attr[1];
     attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     attr[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
-    NNTR_CHECK_CUDA(cudaLaunchKernelEx(&cfg, moe_router_kernel, x, d->router_w, d->router_bias, (int)H, (int)E, (int)K,
-                                       d->gate_w, d->up_w, d->down_w, idx, ord, w, gu_tab, dn_tab,
-                                       reinterpret_cast<float *>(ws + s.rpart),
-                                       reinterpret_cast<unsigned *>(ws + s.rcount), ep));
+    if (grouped && tokens >= ROUTER_ROWS_MIN_TOKENS && H <= 14336) { // its slices of eight tokens must fit in 48 KB beside the partial sums
+      // eight tokens per CTA row (four where the experts' partial sums would not fit)
+      const int tt = E <= 128 ? 8 : 4;
+      cfg.gridDim = dim3((tokens + tt - 1) / tt, ROUTER_SLICES);
+      cfg.dynamicSmemBytes = std::max((size_t)ROUTER_WARPS * tt * E + (size_t)tt * (H / ROUTER_SLICES + ROUTER_WARPS),
+                                      (size_t)ROUTER_WARPS * (E + 32)) * sizeof(float);
+      NNTR_CHECK_CUDA(cudaLaunchKernelEx(&cfg, tt == 8 ? moe_router_rows_kernel<8> : moe_router_rows_kernel<4>, x, d->router_w,
+                                         (int)tokens, (int)H, (int)E, out));
+    } else {
+      NNTR_CHECK_CUDA(cudaLaunchKernelEx(&cfg, moe_router_kernel, x, d->router_w, (int)H, (int)E, out, ep));
+    }
     count_launch();
   }
 
-  if (!epd && tokens >= GROUPED_MIN_TOKENS) {
+  if (grouped) {
     /* prefill: sort the pairs by expert, quantize every pair's activation into the tiles of its expert, one grouped GEMM
      * for gate and up, activation and its quantization, one grouped GEMM for down, combine. Same bits as the per-pair
      * GEMVs. */
@@ -697,7 +832,7 @@ static int moe_forward(const nntr_moe_desc *d, const nntr_moe_ep *epd, unsigned 
                                    tile_rows, P, st)))
       return rc2;
     const long n_out2 = (long)tokens * H;
-    const cudaError_t e2 = launch_pdl(moe_combine_kernel, (unsigned)((n_out2 + 255) / 256), 256, st, dn, idx, ord, w,
+    const cudaError_t e2 = launch_pdl(moe_combine_kernel, (unsigned)((n_out2 / 4 + 63) / 64), 64, st, dn, idx, ord, w,
                                       d->kind == 1 ? d->down_b : nullptr, y, (int)H, (int)K, n_out2);
     count_launch();
     return check_cuda(e2, "moe_combine launch");
@@ -738,7 +873,7 @@ static int moe_forward(const nntr_moe_desc *d, const nntr_moe_ep *epd, unsigned 
                                : launch_gemv_q4_0_batched(H, I, act, nullptr, dn, pdl, P, b2, st);
     if (rc)
       return rc;
-    const cudaError_t e = launch_pdl(moe_combine_kernel, (unsigned)((n_out + 255) / 256), 256, st, dn, idx, ord, w,
+    const cudaError_t e = launch_pdl(moe_combine_kernel, (unsigned)((n_out / 4 + 63) / 64), 64, st, dn, idx, ord, w,
                                      d->kind == 1 ? d->down_b : nullptr, y, (int)H, (int)K, n_out);
     count_launch();
     return check_cuda(e, "moe_combine launch");
@@ -817,11 +952,11 @@ extern "C" int nntr_cuda_moe_route_dev(const nntr_moe_desc *d, unsigned tokens, 
     return set_error(NNTR_CUDA_ERR_INVALID, "moe_route: workspace too small");
   uint8_t *ws = static_cast<uint8_t *>(workspace);
   NNTR_CHECK_CUDA(cudaMemsetAsync(ws + s.rcount, 0, (size_t)tokens * 4, static_cast<cudaStream_t>(stream)));
-  moe_router_kernel<<<dim3(tokens, ROUTER_SLICES), ROUTER_WARPS * 32, ROUTER_WARPS * E * sizeof(float),
-                      static_cast<cudaStream_t>(stream)>>>(
-    x, d->router_w, d->router_bias, (int)d->hidden, (int)E, (int)K, d->gate_w, d->up_w, d->down_w, idx_out, reinterpret_cast<int *>(ws + s.ord), w_out,
-    reinterpret_cast<const void **>(ws + s.gu_tab), reinterpret_cast<const void **>(ws + s.dn_tab),
-    reinterpret_cast<float *>(ws + s.rpart), reinterpret_cast<unsigned *>(ws + s.rcount), MoeEp{});
+  const RouterOut out = {d->router_bias, (int)K, d->gate_w, d->up_w, d->down_w, idx_out, reinterpret_cast<int *>(ws + s.ord),
+                         w_out, reinterpret_cast<const void **>(ws + s.gu_tab), reinterpret_cast<const void **>(ws + s.dn_tab),
+                         reinterpret_cast<float *>(ws + s.rpart), reinterpret_cast<unsigned *>(ws + s.rcount)};
+  moe_router_kernel<<<dim3(tokens, ROUTER_SLICES), ROUTER_WARPS * 32, (ROUTER_WARPS * E + 32) * sizeof(float),
+                      static_cast<cudaStream_t>(stream)>>>(x, d->router_w, (int)d->hidden, (int)E, out, MoeEp{});
   count_launch();
   return check_cuda(cudaGetLastError(), "moe_router launch");
 }

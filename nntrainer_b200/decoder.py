@@ -87,6 +87,10 @@ class Qwen3Decoder:
                       k=qkv[q_dim:q_dim + kv_dim], v=qkv[q_dim + kv_dim:], a=f(q_dim), o=f(cfg.hidden), ug=ug,
                       up=ug[:cfg.inter], gate=ug[cfg.inter:], act=f(cfg.inter), d=f(cfg.hidden), logits=f(cfg.vocab))
         self._tables()
+        import ctypes as C
+        self._calls, self._call_caches = {}, []
+        self._arg = dict(tok=C.c_void_p(), pos=C.c_uint(), pos_dev=C.c_void_p(), idx=C.c_void_p(), idx_f=C.c_void_p(),
+                         stream=C.c_void_p())
 
     class _P:  # a raw device address with the data_ptr() face the backend helpers use
         def __init__(self, p):
@@ -143,57 +147,106 @@ class Qwen3Decoder:
         ffn_up | ffn_gate (one batched launch); SwiGLU; ffn_down -- nine. With ``fuse`` the two norms run in the
         prologues of the projections behind them and the SwiGLU in the epilogue of the up | gate launch -- five (attention
         takes more launches beyond 16384 rows). Every fusion keeps the bits of the separate operators."""
-        c, b, pdl = self.cfg, self.b, self.pdl
+        torch = self.torch
+        if out_idx is None:
+            out_idx = torch.empty(1, dtype=torch.int32, device=self.dev)
+        if out_idx_f is None:
+            out_idx_f = torch.empty(1, dtype=torch.float32, device=self.dev)
+        # The launches of a step differ from the next step's in five values only: they are made into a list of calls once, whose
+        # arguments are converted already and share those five. A call then costs its launch and little else.
+        key = (self.pdl, self.fuse)
+        calls = self._calls.get(key)
+        if calls is None or any(a.kcache is not k or a.vcache is not v for a, (k, v) in zip(self.attn, self._call_caches)):
+            self._call_caches = [(a.kcache, a.vcache) for a in self.attn]
+            calls = self._calls[key] = self._make_calls()
+        v = self._arg
+        v["tok"].value, v["pos"].value = token_f.data_ptr(), pos
+        v["pos_dev"].value = pos_dev.data_ptr() if pos_dev is not None else None
+        v["idx"].value, v["idx_f"].value = out_idx.data_ptr(), out_idx_f.data_ptr()
+        v["stream"].value = be._stream()
+        for fn, args in calls:
+            rc = fn(*args)
+            if rc:
+                be.check(rc)
+        return out_idx, out_idx_f
+
+    def _make_calls(self):
+        """The C calls of a decode step in order, as (function, converted arguments)."""
+        import ctypes as C
+        from .capi import GEMV_PDL, QTYPE
+        c, b, L, v = self.cfg, self.b, be.lib(), self._arg
+        flags = GEMV_PDL if self.pdl else 0
         q_dim, kv_dim = c.n_heads * c.head_dim, c.n_kv_heads * c.head_dim
-        be.embedding(c.embedding_dtype, self._P(self.ptr["embedding0"]), token_f, c.vocab, c.hidden,
-                     out=b["x"].view(1, -1), pdl=pdl)
+        calls = []
+
+        def call(name, *args):
+            fn = getattr(L, "nntr_cuda_" + name)
+            conv = [a if isinstance(a, (C._SimpleCData, C.Structure)) or type(a).__name__ == "CArgObject" else
+                    t(a.data_ptr()) if hasattr(a, "data_ptr") else t(a) for t, a in zip(fn.argtypes, args)]
+            calls.append((fn, tuple(conv)))
+
+        w = lambda name: self._P(self.ptr[name])  # noqa: E731
+        st, eps = v["stream"], c.norm_eps
+
+        def gemv(name, x, y):
+            dtype, N, K = self._shape[name]
+            call("gemv_dev", QTYPE[dtype], N, K, x, w(name), y, flags, st)
+
+        def norm(x, name, out):
+            call("rms_norm_dev", x, w(name), out, 1, c.hidden, eps, flags, st)
+
+        def add_norm(x, r, name, total, out):
+            call("add_rms_norm_dev", x, r, total, w(name), out, 1, c.hidden, eps, flags, st)
+
+        call("embedding_dev", QTYPE[c.embedding_dtype], w("embedding0"), v["tok"], b["x"], 1, c.vocab, c.hidden, flags, st)
         x = b["x"]
-        fuse = self.fuse and self._qkv_ok
+        fuse, qt = self.fuse and self._qkv_ok, QTYPE[c.fc_dtype]
         for i in range(c.n_layers):
             p = f"layer{i}_"
-            qk_norm = (self._P(self.ptr[p + "q_norm"]), self._P(self.ptr[p + "k_norm"]), c.norm_eps)
+            at = self.attn[i]
+
+            def attention():
+                call("attention_step_dev", C.byref(at.desc), v["pos"], v["pos_dev"], at.max_seq, b["q"], b["k"], b["v"],
+                     w(p + "q_norm"), w(p + "k_norm"), eps, at.kcache, at.vcache, at.cos, at.sin, None, b["a"], at.ws,
+                     at.ws.numel(), flags, st)
+
             if fuse:
                 # 5 launches: (add +) norm + q|k|v; attention; o; add + norm + up|gate + SwiGLU; down
-                g_att, g_ffn = self._P(self.ptr[p + "attention_norm"]), self._P(self.ptr[p + "ffn_norm"])
-                if i == 0:
-                    be.gemv_add_norm(c.fc_dtype, q_dim + 2 * kv_dim, c.hidden, x, None, None, g_att, c.norm_eps,
-                                     self._qkv_packed[i], b["qkv"], pdl=pdl)
-                else:  # the previous block's output x = h + ffn_down, and its norm
-                    be.gemv_add_norm(c.fc_dtype, q_dim + 2 * kv_dim, c.hidden, b["h"], b["d"], x, g_att, c.norm_eps,
-                                     self._qkv_packed[i], b["qkv"], pdl=pdl)
-                self.attn[i].step(b["q"], b["k"], b["v"], pos, pos_dev=pos_dev, out=b["a"], pdl=pdl, qk_norm=qk_norm)
-                self._gemv(p + "attention_out", b["a"], b["o"])
-                be.gated_ffn_in(c.fc_dtype, c.inter, c.hidden, x, b["o"], b["h"], g_ffn, c.norm_eps,
-                                self._P(self.ptr[p + "ffn_up"]), self._P(self.ptr[p + "ffn_gate"]), b["act"], pdl=pdl)
-                self._gemv(p + "ffn_down", b["act"], b["d"])
+                # (behind the first layer: the previous block's output x = h + ffn_down, and its norm)
+                src = (x, None, None) if i == 0 else (b["h"], b["d"], x)
+                call("gemv_add_norm_dev", qt, q_dim + 2 * kv_dim, c.hidden, *src, w(p + "attention_norm"), eps,
+                     self._qkv_packed[i], b["qkv"], flags, st)
+                attention()
+                gemv(p + "attention_out", b["a"], b["o"])
+                call("gated_ffn_in_dev", qt, c.inter, c.hidden, x, b["o"], b["h"], w(p + "ffn_norm"), eps, w(p + "ffn_up"),
+                     w(p + "ffn_gate"), b["act"], flags, st)
+                gemv(p + "ffn_down", b["act"], b["d"])
                 continue
             if i == 0:
-                self._norm(x, p + "attention_norm", b["n"])
+                norm(x, p + "attention_norm", b["n"])
             else:  # the previous block's output x = h + ffn_down, and its norm
-                be.add_rms_norm(b["h"], b["d"], self._P(self.ptr[p + "attention_norm"]), c.norm_eps, sum_out=x, out=b["n"],
-                                pdl=pdl)
+                add_norm(b["h"], b["d"], p + "attention_norm", x, b["n"])
             if self._qkv_ok:
-                be.gemv_batched(c.fc_dtype, kv_dim, c.hidden, b["n"], self._qkv_tab[i], q_dim // kv_dim + 2, b["qkv"],
-                                pdl=pdl)
+                call("gemv_batched_dev", qt, kv_dim, c.hidden, b["n"], self._qkv_tab[i], q_dim // kv_dim + 2, b["qkv"], flags,
+                     st)
             else:
-                self._gemv(p + "wv", b["n"], b["v"])
-                self._gemv(p + "wk", b["n"], b["k"])
-                self._gemv(p + "wq", b["n"], b["q"])
-            # k_norm and q_norm (per-head RMS norms) run inside the attention launch
-            self.attn[i].step(b["q"], b["k"], b["v"], pos, pos_dev=pos_dev, out=b["a"], pdl=pdl, qk_norm=qk_norm)
-            self._gemv(p + "attention_out", b["a"], b["o"])
-            be.add_rms_norm(x, b["o"], self._P(self.ptr[p + "ffn_norm"]), c.norm_eps, sum_out=b["h"], out=b["n"], pdl=pdl)
+                gemv(p + "wv", b["n"], b["v"])
+                gemv(p + "wk", b["n"], b["k"])
+                gemv(p + "wq", b["n"], b["q"])
+            attention()  # with k_norm and q_norm (per-head RMS norms)
+            gemv(p + "attention_out", b["a"], b["o"])
+            add_norm(x, b["o"], p + "ffn_norm", b["h"], b["n"])
             if self._qkv_ok:
-                be.gemv_batched(c.fc_dtype, c.inter, c.hidden, b["n"], self._ug_tab[i], 2, b["ug"], pdl=pdl)
+                call("gemv_batched_dev", qt, c.inter, c.hidden, b["n"], self._ug_tab[i], 2, b["ug"], flags, st)
             else:
-                self._gemv(p + "ffn_up", b["n"], b["up"])
-                self._gemv(p + "ffn_gate", b["n"], b["gate"])
-            be.swiglu(b["up"], b["gate"], out=b["act"], pdl=pdl)
-            self._gemv(p + "ffn_down", b["act"], b["d"])
-        be.add_rms_norm(b["h"], b["d"], self._P(self.ptr["output_norm"]), c.norm_eps, sum_out=x, out=b["n"], pdl=pdl)
-        head = "embedding0" if c.tie_word_embeddings else "output_of_causallm"
-        self._gemv(head, b["n"], b["logits"])
-        return be.argmax(b["logits"].view(1, -1), pdl=pdl, out=(out_idx, out_idx_f))
+                gemv(p + "ffn_up", b["n"], b["up"])
+                gemv(p + "ffn_gate", b["n"], b["gate"])
+            call("swiglu_dev", b["act"], b["up"], b["gate"], c.inter, flags, st)
+            gemv(p + "ffn_down", b["act"], b["d"])
+        add_norm(b["h"], b["d"], "output_norm", x, b["n"])
+        gemv("embedding0" if c.tie_word_embeddings else "output_of_causallm", b["n"], b["logits"])
+        call("argmax_dev", b["logits"], 1, c.vocab, c.vocab, v["idx"], v["idx_f"], flags, st)
+        return calls
 
     def capture(self, start_pos: int):
         """Captures one decode step into a CUDA graph: the token id lives in ``self.tok_f`` (device float, rewritten by
