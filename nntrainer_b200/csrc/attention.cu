@@ -24,12 +24,10 @@
  * Cache layout as the reference's: [row][kv head][head_dim] fp16, one row per position.
  */
 #include <atomic>
-#include <cstring>
-
-#include <cuda.h>
 
 #include "common.cuh"
 #include "pipeline.cuh"
+#include "tma_map.cuh"
 
 namespace nntr {
 
@@ -466,11 +464,6 @@ struct AttnStep {
   int k_box, v_box; // rows a copy brings: a tile, fewer where one short tile is all there is
 };
 
-__device__ __forceinline__ void tma_tile(uint32_t dst, const CUtensorMap *map, int x, int y, uint32_t bar) {
-  asm volatile("cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];" ::"r"(dst),
-               "l"(reinterpret_cast<uint64_t>(map)), "r"(x), "r"(y), "r"(bar)
-               : "memory");
-}
 __device__ __forceinline__ uint32_t cluster_rank() {
   uint32_t r;
   asm("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
@@ -938,57 +931,6 @@ int clear_attn_status() {
 
 /* ---------------------------------------------------------------- launchers */
 
-/* Tensor map over a cache [rows][hkv * hd] fp16 with boxes of box_rows x box_dims values (swizzled: 64 values = 128
- * bytes). The driver's encoder is looked up through the runtime (the library does not link against the driver). A map depends
- * on its arguments alone; every thread keeps the last ones it made, because a decode loop comes back with the same. */
-static int encode_cache_map(CUtensorMap *map, const uint16_t *cache, unsigned rows, unsigned hkv, unsigned hd, unsigned box_dims,
-                            unsigned box_rows, bool swizzle) {
-  typedef CUresult (*EncodeTiled)(CUtensorMap *, CUtensorMapDataType, cuuint32_t, void *, const cuuint64_t *,
-                                  const cuuint64_t *, const cuuint32_t *, const cuuint32_t *, CUtensorMapInterleave,
-                                  CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
-  static std::atomic<EncodeTiled> encode{nullptr};
-  EncodeTiled enc = encode.load(std::memory_order_acquire);
-  if (!enc) {
-    void *fn = nullptr;
-    cudaDriverEntryPointQueryResult found;
-    NNTR_CHECK_CUDA(cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &fn, cudaEnableDefault, &found));
-    if (!fn || found != cudaDriverEntryPointSuccess)
-      return set_error(NNTR_CUDA_ERR_UNSUPPORTED, "attention: the driver has no cuTensorMapEncodeTiled");
-    enc = reinterpret_cast<EncodeTiled>(fn);
-    encode.store(enc, std::memory_order_release);
-  }
-  struct Key { // compared as bytes: no padding
-    const uint16_t *cache;
-    unsigned rows, hkv, hd, box_dims, box_rows, swizzle; // never all zero: an empty entry matches nothing
-  };
-  struct Entry {
-    Key key;
-    CUtensorMap map;
-  };
-  constexpr unsigned SLOTS = 64; // 12 KB per thread
-  static thread_local Entry slots[SLOTS] = {};
-  const Key key = {cache, rows, hkv, hd, box_dims, box_rows, swizzle};
-  Entry &slot = slots[((uint32_t)(reinterpret_cast<uintptr_t>(cache) >> 12) * 2654435761u >> 26) ^ (swizzle ? 1u : 0u)];
-  if (memcmp(&slot.key, &key, sizeof key) == 0) {
-    *map = slot.map;
-    return NNTR_CUDA_OK;
-  }
-  const cuuint64_t dims[2] = {(cuuint64_t)hkv * hd, rows};
-  const cuuint64_t strides[1] = {(cuuint64_t)hkv * hd * 2}; // bytes between rows: a multiple of 16 (head_dim % 8 == 0)
-  const cuuint32_t box[2] = {box_dims, box_rows};
-  const cuuint32_t estr[2] = {1, 1};
-  const CUresult r = enc(&slot.map, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, const_cast<uint16_t *>(cache), dims, strides, box, estr,
-                         CU_TENSOR_MAP_INTERLEAVE_NONE, swizzle ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_NONE,
-                         CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-  if (r != CUDA_SUCCESS) {
-    slot.key = Key{};
-    return set_error(NNTR_CUDA_ERR_CUDA, "attention: cuTensorMapEncodeTiled failed (%d)", (int)r);
-  }
-  slot.key = key;
-  *map = slot.map;
-  return NNTR_CUDA_OK;
-}
-
 static int check_attn(const nntr_attn_desc *a) {
   if (!a || a->n_heads_q == 0 || a->n_heads_kv == 0 || a->head_dim == 0)
     return set_error(NNTR_CUDA_ERR_INVALID, "attention: null or empty description");
@@ -1098,8 +1040,10 @@ static int launch_attn_cluster(AttnStep a, unsigned bound, unsigned rows, unsign
     attr_done[dev & 63].fetch_or(bit, std::memory_order_release);
   }
   CUtensorMap kmap, vmap;
-  int rc = encode_cache_map(&kmap, a.kcache, bound, (unsigned)a.hkv, (unsigned)hd, 64, (unsigned)a.k_box, true);
-  if (rc || (rc = encode_cache_map(&vmap, a.vcache, bound, (unsigned)a.hkv, (unsigned)hd, (unsigned)dims, (unsigned)a.v_box, false)))
+  // maps over the caches, [bound rows][hkv * hd] fp16; keys swizzled: 64 values = 128 bytes
+  const uint64_t width = (uint64_t)a.hkv * hd;
+  int rc = encode_map_2d(&kmap, a.kcache, 2, width, bound, width * 2, 64, (unsigned)a.k_box, true);
+  if (rc || (rc = encode_map_2d(&vmap, a.vcache, 2, width, bound, width * 2, (unsigned)dims, (unsigned)a.v_box, false)))
     return rc;
   cudaLaunchConfig_t cfg = {};
   cudaLaunchAttribute attr[2];

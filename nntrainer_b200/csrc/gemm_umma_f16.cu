@@ -28,21 +28,32 @@
  * One CTA owns two tiles of 128 activation rows (MMA M, tensor-memory lanes)
  * against the same 256 weight rows (MMA N, columns), so every expanded weight
  * stage feeds two MMAs, and walks K in stages of 64 (one pair of sub-blocks):
- *   warps 0-15  producers: two threads per weight row expand its 32 nibble bytes
- *               of the stage into 64 fp16 values. A 32-bit word yields four half2 with one
+ *   warps 0-15  producers: expand a stage's nibble bytes into 64 fp16 values per
+ *               weight row. A 32-bit word yields four half2 with one
  *               logic op each ((w >> s) & 0x000F000F | 0x64006400 is
  *               (1024 + n_lo, 1024 + n_hi)), so the K order inside a stage is
  *               the order that unpack produces; the activation tiles are written
- *               in the same order (a dot product does not care). After the
- *               last stage the same warps are the epilogue: tcgen05.ld of the
- *               tile, float4 stores of C.
+ *               in the same order (a dot product does not care). Q4_K and Q4_0:
+ *               one thread per row, eight warps take the even and eight the odd
+ *               stages. Q6_K: two threads per row, all warps every stage. After
+ *               the last stage the same warps are the epilogue: tcgen05.ld of the
+ *               tile, a turn through shared memory, stores of C by whole lines.
  *   warp 16     one thread issues 8 MMAs (128 x 256 x 16) per stage.
  *   warp 17     one thread starts the bulk copies of the activation stages, each
  *               as soon as the MMAs that read its slot have retired.
+ *   warp 18     one thread starts the tiled copies of the packed weights
+ *               (Q4_K, Q4_0) into a ring of two stages.
  * Three stages of 64 KB, both accumulators (512 columns) in tensor memory. Every wait is bounded (pipeline.cuh).
+ *
+ * What bounds it: the producers. A stage's MMAs take 1024 clocks, a stage took 1780: about 520 clocks of instruction issue,
+ * and around it two waits, a fence and the arrive at 100-270 clocks each, in all sixteen warps at the same time. In two
+ * groups, one group's latencies pass while the other expands. The tile's stores took 27 of its 142 thousand clocks while
+ * every lane wrote a row of its own. Both changes, 1024 x 24576 x 4096 Q4_K: 221 -> 192 us (1076 TFLOP/s), 256 rows
+ * 74 -> 65, Q4_0 1024 rows 201 -> 186; Q6_K 256 x 151936 x 2560 552 -> 359 (the stores).
  */
 #include "common.cuh"
 #include "pipeline.cuh"
+#include "tma_map.cuh"
 
 #include <cuda_fp16.h>
 
@@ -57,12 +68,24 @@ constexpr int F16_W_BYTES = F16_TILE_N * F16_KS * 2; // 32 KB
 constexpr int F16_A_BYTES = F16_TILE_M * F16_KS * 2; // 16 KB
 constexpr int F16_STAGE_BYTES = F16_W_BYTES + 2 * F16_A_BYTES; // weights + two activation tiles (256 rows)
 constexpr int F16_STAGES = 3;
-constexpr int F16_PRODUCERS = 512; // two per weight row
+constexpr int F16_PRODUCERS = 512;
+/* Q4_K, Q4_0: two groups of 256 threads, one thread per weight row, take alternate stages; Q6_K: two threads per row */
+__host__ __device__ constexpr int f16_stage_warps(int qt) { return qt == NNTR_Q6_K ? F16_PRODUCERS / 32 : F16_PRODUCERS / 64; }
 constexpr int F16_MMA_WARP = F16_PRODUCERS / 32;
 constexpr int F16_COPY_WARP = F16_MMA_WARP + 1;
-constexpr int F16_THREADS = (F16_COPY_WARP + 1) * 32; // 576
-constexpr int F16_OFF_BARS = F16_STAGES * F16_STAGE_BYTES;
-constexpr int F16_SMEM = F16_OFF_BARS + 128;
+constexpr int F16_RAW_WARP = F16_COPY_WARP + 1;
+constexpr int F16_THREADS = (F16_RAW_WARP + 1) * 32; // 608
+/* Packed weights of a stage on their way to the producers, 32 groups of 8 rows: Q4_K the 256 nibble bytes of a pair of
+ * sub-blocks per group, plus the 128 header bytes (d, dmin, scales) of a super-block for its four stages; Q4_0 two whole
+ * blocks per group. Q6_K rows are not 16-byte aligned: their producers load from global memory. */
+constexpr int F16_RAW = 2; // one per producer group: in an odd ring a group could take a phase of the other group for its own
+__host__ __device__ constexpr int f16_raw_bytes(int qt) { return qt == NNTR_Q4_K ? 32 * 256 : qt == NNTR_Q4_0 ? 32 * 288 : 0; }
+constexpr int F16_HDR_BYTES = 32 * 128;
+constexpr int F16_OFF_RAW = F16_STAGES * F16_STAGE_BYTES;
+__host__ __device__ constexpr int f16_off_hdr(int qt) { return F16_OFF_RAW + F16_RAW * f16_raw_bytes(qt); }
+__host__ __device__ constexpr int f16_off_bars(int qt) { return f16_off_hdr(qt) + (qt == NNTR_Q4_K ? 2 * F16_HDR_BYTES : 0); }
+__host__ __device__ constexpr int f16_smem(int qt) { return f16_off_bars(qt) + 256; }
+static_assert(f16_smem(NNTR_Q4_K) <= 227 * 1024 && f16_smem(NNTR_Q4_0) <= 227 * 1024, "shared memory of a CTA");
 constexpr uint32_t F16_POLLS = 1u << 22;
 
 __device__ int g_f16_status = 0;
@@ -127,15 +150,16 @@ __device__ __forceinline__ uint32_t expand2_q40(uint32_t nib2, __half2 d) {
  *                 32 s2 ..] as low and high nibbles); n_stages = 4 * K/256. N may end inside the last 256-row tile. */
 template <int QT>
 __global__ void __launch_bounds__(F16_THREADS, 1)
-gemm_f16_kernel(const uint8_t *__restrict__ atiles, const uint8_t *__restrict__ Wb, float *__restrict__ C, int ldc, int M,
-                int N, int n_stages, int m_tiles, int c_vec4) {
+gemm_f16_kernel(const __grid_constant__ CUtensorMap wmap, const uint8_t *__restrict__ atiles, const uint8_t *__restrict__ Wb,
+                float *__restrict__ C, int ldc, int M, int N, int n_stages, int m_tiles, int c_vec4) {
   extern __shared__ __align__(128) uint8_t smem[];
-  // bars: [0..3] full, [4..7] empty, [8] tile complete
+  // bars: [0..3] full, [4..7] empty, [8] tile complete, [9..10] packed weights here, [12..13] packed weights read,
+  // [14..15] Q4_K headers here
   const uint32_t sbase = smem_u32(smem);
-  const uint32_t bar0 = sbase + F16_OFF_BARS;
+  const uint32_t bar0 = sbase + f16_off_bars(QT);
   auto BAR = [&](int i) { return bar0 + 8u * i; };
-  uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(smem + F16_OFF_BARS + 96);
-  volatile int *abort_flag = reinterpret_cast<volatile int *>(smem + F16_OFF_BARS + 104);
+  uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(smem + f16_off_bars(QT) + 128);
+  volatile int *abort_flag = reinterpret_cast<volatile int *>(smem + f16_off_bars(QT) + 136);
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   // a CTA takes two 128-row activation tiles (2*blockIdx.x, +1) against the same 256 weight rows: the expanded
   // weights of a stage feed two MMAs, which halves the expansion work per output
@@ -144,8 +168,13 @@ gemm_f16_kernel(const uint8_t *__restrict__ atiles, const uint8_t *__restrict__ 
 
   if (tid == 0) {
     for (int s = 0; s < F16_STAGES; ++s) {
-      mbar_init(BAR(s), F16_PRODUCERS / 32 + 1); // every producer warp + the copy warp's thread that armed the activation copy
-      mbar_init(BAR(4 + s), 1);             // MMAs of the stage retired
+      mbar_init(BAR(s), f16_stage_warps(QT) + 1); // the stage's producer warps + the thread that armed the activation copy
+      mbar_init(BAR(4 + s), 1);                   // MMAs of the stage retired
+    }
+    for (int s = 0; s < F16_RAW; ++s) {
+      mbar_init(BAR(9 + s), 1);
+      mbar_init(BAR(12 + s), f16_stage_warps(QT));
+      mbar_init(BAR(14 + s), 1);
     }
     mbar_init(BAR(8), 1);
     *abort_flag = 0;
@@ -164,80 +193,82 @@ gemm_f16_kernel(const uint8_t *__restrict__ atiles, const uint8_t *__restrict__ 
   if (warp < F16_MMA_WARP) {
     /* ------------------------------ producers ------------------------------ */
     const int r = tid & (F16_TILE_N - 1); // weight row inside the tile
-    const int hsel = tid >> 8;            // which half of the stage's 32 nibble bytes: chunks 2*hsel, 2*hsel + 1
+    const int hsel = tid >> 8;            // Q4_K, Q4_0: stages of this parity; Q6_K: which half of the stage's 32 nibble bytes
     const int j = r & 7;                  // row inside its 8-row group
     bool ok = true;
-    if constexpr (QT == NNTR_Q4_K) {
-    const BlockQ4Kx8 *wrow = reinterpret_cast<const BlockQ4Kx8 *>(Wb) + (size_t)(nt * (F16_TILE_N / 8) + (r >> 3)) * (n_stages / 4);
-    // A stage's inputs in registers: this thread's 16 nibble bytes (two 8-byte chunks), the two 12-byte scale groups of
-    // the stage (sub-blocks 2p: low nibbles, 2p+1: high nibbles), d and dmin of the row. Two such sets rotate, so a
-    // stage's loads are issued two stages before they are used: one stage alone does not cover the L2 latency.
-    struct StageIn {
-      uint2 q[2];
-      uint32_t g[6];
-      float dw, dmw;
+    auto slot_wait = [&](int st) { // the MMAs that read the slot have retired
+      const int use = st / F16_STAGES;
+      const bool go = use == 0 || mbar_wait(BAR(4 + st % F16_STAGES), (use - 1) & 1, abort_flag);
+      return __all_sync(0xffffffffu, go) != 0; // the warp leaves together: its lanes meet at the arrives below
     };
-    auto fetch = [&](StageIn &in, int st) {
-      const BlockQ4Kx8 *blk = wrow + (st >> 2);
-      const uint8_t *nq = blk->qs + ((st & 3) * 32 + 16 * hsel + j) * 8;
-#pragma unroll
-      for (int c = 0; c < 2; ++c)
-        in.q[c] = ldg_stream_u2(nq + c * 64);
-#pragma unroll
-      for (int i = 0; i < 6; ++i)
-        in.g[i] = __ldg(reinterpret_cast<const uint32_t *>(blk->scales + 24 * (st & 3)) + i);
-      in.dw = half_bits_to_float(blk->d[j]);
-      in.dmw = half_bits_to_float(blk->dmin[j]);
+    auto raw_wait = [&](int st) { // the stage's packed weights are here (Q4_K: half the lanes ask for the super-block's header)
+      const bool head = QT == NNTR_Q4_K && lane >= 16;
+      return __all_sync(0xffffffffu, mbar_wait(head ? BAR(14 + ((st >> 2) & 1)) : BAR(9 + st % F16_RAW),
+                                               (head ? st >> 3 : st / F16_RAW) & 1, abort_flag)) != 0;
     };
-    auto stage = [&](StageIn &in, int st) {
-      const int s = st % F16_STAGES, use = st / F16_STAGES;
-      float sc0, mn0, sc1, mn1;
-      scale_min_row(in.g[0], in.g[1], in.g[2], j, sc0, mn0);
-      scale_min_row(in.g[3], in.g[4], in.g[5], j, sc1, mn1);
-      const __half2 d_lo = __float2half2_rn(in.dw * sc0), d_hi = __float2half2_rn(in.dw * sc1);
-      const __half2 m_lo = __float2half2_rn(-(in.dmw * mn0)), m_hi = __float2half2_rn(-(in.dmw * mn1));
-      const uint2 w[2] = {in.q[0], in.q[1]};
-      fetch(in, st + 2 < n_stages ? st + 2 : n_stages - 1); // the set is free again: the stage after next travels
-      { // weights are read once from HBM: pull the lines of five stages ahead into L2 so that the loads above hit it
-        const int fst = st + 5 < n_stages ? st + 5 : n_stages - 1;
-        const uint8_t *fq = wrow[fst >> 2].qs + ((fst & 3) * 32 + 16 * hsel + j) * 8;
-        asm volatile("prefetch.global.L2 [%0];" ::"l"(fq));
-        asm volatile("prefetch.global.L2 [%0];" ::"l"(fq + 64));
-        if ((fst & 3) == 0 && hsel == 0 && j == 0)
-          asm volatile("prefetch.global.L2 [%0];" ::"l"(wrow + (fst >> 2))); // d, dmin, scales: the block's first 128 bytes
-      }
-      if (use > 0 && !mbar_wait(BAR(4 + s), (use - 1) & 1, abort_flag))
-        ok = false;
-      ok = __all_sync(0xffffffffu, ok); // the warp leaves together: its lanes meet at the arrive below
-      if (!ok)
-        return;
-      uint8_t *wdst = smem + s * F16_STAGE_BYTES + r * 16;
-#pragma unroll
-      for (int c = 0; c < 2; ++c) {
-        // word -> 8 halves in the order [lo b0, lo b2, lo b1, lo b3, hi b0, hi b2, hi b1, hi b3]
-        const uint32_t wx = w[c].x, wy = w[c].y;
-        const uint4 o0 = make_uint4(expand2(wx & 0x000f000fu, d_lo, m_lo), expand2((wx >> 8) & 0x000f000fu, d_lo, m_lo),
-                                    expand2((wx >> 4) & 0x000f000fu, d_hi, m_hi),
-                                    expand2((wx >> 12) & 0x000f000fu, d_hi, m_hi));
-        const uint4 o1 = make_uint4(expand2(wy & 0x000f000fu, d_lo, m_lo), expand2((wy >> 8) & 0x000f000fu, d_lo, m_lo),
-                                    expand2((wy >> 4) & 0x000f000fu, d_hi, m_hi),
-                                    expand2((wy >> 12) & 0x000f000fu, d_hi, m_hi));
-        *reinterpret_cast<uint4 *>(wdst + (4 * hsel + 2 * c) * (F16_TILE_N * 16)) = o0;
-        *reinterpret_cast<uint4 *>(wdst + (4 * hsel + 2 * c + 1) * (F16_TILE_N * 16)) = o1;
-      }
+    auto stage_done = [&](int st) {
       asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
       __syncwarp(); // every lane's writes are fenced; one arrival per warp keeps the barrier word off the critical path
       if (lane == 0)
-        mbar_arrive(BAR(s));
+        mbar_arrive(BAR(st % F16_STAGES));
     };
-    StageIn in0, in1;
-    fetch(in0, 0);
-    fetch(in1, 1); // n_stages is a multiple of 4
-    for (int st = 0; st < n_stages && ok; st += 2) {
-      stage(in0, st);
-      if (ok)
-        stage(in1, st + 1);
-    }
+    // The packed words are on their way to registers and the slot may be refilled. Nothing has used them yet, and an arrive
+    // right behind the loads can overtake them (seen on Q4_0: now and then eight rows held a later stage's block), so the vote
+    // that gathers the warp, and the barrier's address with it, depends on what every lane loaded.
+    const uint32_t zero = gridDim.z - 1; // 0, but not to the compiler
+    auto raw_done = [&](int st, uint32_t loaded) {
+      const uint32_t any = __any_sync(0xffffffffu, (loaded & zero) != 0);
+      if (lane == 0)
+        mbar_arrive(BAR(12 + st % F16_RAW) + any);
+    };
+    if constexpr (QT == NNTR_Q4_K) {
+      // neighbouring groups read pairs of nibble chunks in opposite order: 128 bytes apart, they would meet in the same banks
+      const int grp = r >> 3, sw = grp & 1;
+      const uint8_t *nq = smem + F16_OFF_RAW + grp * 128 + 8 * j;
+      const uint8_t *hdr = smem + f16_off_hdr(QT) + grp * 128;
+      // the next stage's words go to registers as soon as this one's are expanded, so that its ring slot refills meanwhile
+      uint2 w[4], g0, g1, g2;
+      float dw, dmw;
+      auto fetch = [&](int st) {
+        if (!raw_wait(st))
+          return false;
+#pragma unroll
+        for (int c = 0; c < 4; ++c)
+          w[c] = *reinterpret_cast<const uint2 *>(nq + (st % F16_RAW) * f16_raw_bytes(QT) + (c >> 1) * (32 * 128) + 64 * ((c & 1) ^ sw));
+        const uint8_t *h = hdr + ((st >> 2) & 1) * F16_HDR_BYTES;
+        g0 = *reinterpret_cast<const uint2 *>(h + 32 + 24 * (st & 3));
+        g1 = *reinterpret_cast<const uint2 *>(h + 40 + 24 * (st & 3));
+        g2 = *reinterpret_cast<const uint2 *>(h + 48 + 24 * (st & 3));
+        dw = half_bits_to_float(*reinterpret_cast<const uint16_t *>(h + 2 * j));
+        dmw = half_bits_to_float(*reinterpret_cast<const uint16_t *>(h + 16 + 2 * j));
+        raw_done(st, w[0].x ^ w[1].x ^ w[2].x ^ w[3].x ^ g0.x ^ g1.x ^ g2.x ^ __float_as_uint(dw) ^ __float_as_uint(dmw));
+        return true;
+      };
+      ok = hsel >= n_stages || fetch(hsel);
+      for (int st = hsel; st < n_stages && ok; st += 2) {
+        float sc0, mn0, sc1, mn1;
+        scale_min_row(g0.x, g0.y, g1.x, j, sc0, mn0);
+        scale_min_row(g1.y, g2.x, g2.y, j, sc1, mn1);
+        const __half2 d_lo = __float2half2_rn(dw * sc0), d_hi = __float2half2_rn(dw * sc1);
+        const __half2 m_lo = __float2half2_rn(-(dmw * mn0)), m_hi = __float2half2_rn(-(dmw * mn1));
+        if (!(ok = slot_wait(st)))
+          break;
+        uint8_t *wdst = smem + (st % F16_STAGES) * F16_STAGE_BYTES + r * 16;
+#pragma unroll
+        for (int c = 0; c < 4; ++c) {
+          // word -> 8 halves in the order [lo b0, lo b2, lo b1, lo b3, hi b0, hi b2, hi b1, hi b3]
+          const uint32_t wx = w[c].x, wy = w[c].y;
+          uint8_t *d = wdst + (2 * (c ^ sw)) * (F16_TILE_N * 16);
+          *reinterpret_cast<uint4 *>(d) =
+            make_uint4(expand2(wx & 0x000f000fu, d_lo, m_lo), expand2((wx >> 8) & 0x000f000fu, d_lo, m_lo),
+                       expand2((wx >> 4) & 0x000f000fu, d_hi, m_hi), expand2((wx >> 12) & 0x000f000fu, d_hi, m_hi));
+          *reinterpret_cast<uint4 *>(d + F16_TILE_N * 16) =
+            make_uint4(expand2(wy & 0x000f000fu, d_lo, m_lo), expand2((wy >> 8) & 0x000f000fu, d_lo, m_lo),
+                       expand2((wy >> 4) & 0x000f000fu, d_hi, m_hi), expand2((wy >> 12) & 0x000f000fu, d_hi, m_hi));
+        }
+        stage_done(st);
+        ok = st + 2 >= n_stages || fetch(st + 2);
+      }
     } else if constexpr (QT == NNTR_Q6_K) {
       const int n_row = nt * F16_TILE_N + r;
       const bool have_row = n_row < N; // rows beyond N: scale 0, so zero weights (their columns are not stored either)
@@ -313,87 +344,91 @@ gemm_f16_kernel(const uint8_t *__restrict__ atiles, const uint8_t *__restrict__ 
         }
       }
     } else {
-      const BlockQ40x8 *wrow = reinterpret_cast<const BlockQ40x8 *>(Wb) + (size_t)(nt * (F16_TILE_N / 8) + (r >> 3)) * (n_stages * 2);
-      // this thread expands block 2*st + hsel of the row: 16 nibble bytes = four words = four 16-byte chunks of halves.
-      // Two register sets rotate: a stage's loads are issued two stages before they are used.
-      struct StageIn {
-        uint2 qa, qb;
-        uint16_t dbits;
-      };
-      auto fetch = [&](StageIn &in, int st) {
-        const BlockQ40x8 *blk = wrow + 2 * st + hsel;
-        in.qa = ldg_stream_u2(blk->qs + j * 8);
-        in.qb = ldg_stream_u2(blk->qs + 64 + j * 8);
-        in.dbits = __ldg(&blk->d[j]);
-      };
-      auto stage = [&](StageIn &in, int st) {
-        const int s = st % F16_STAGES, use = st / F16_STAGES;
-        const __half2 d2 = __half2half2(__ushort_as_half(in.dbits));
-        const uint32_t w[4] = {in.qa.x ^ 0x88888888u, in.qa.y ^ 0x88888888u, in.qb.x ^ 0x88888888u, in.qb.y ^ 0x88888888u};
-        fetch(in, st + 2 < n_stages ? st + 2 : n_stages - 1); // the set is free again: the stage after next travels
-        if (j == 0) { // five stages ahead goes to L2
-          const BlockQ40x8 *fblk = wrow + 2 * (st + 5 < n_stages ? st + 5 : n_stages - 1) + hsel;
-          asm volatile("prefetch.global.L2 [%0];" ::"l"(fblk));
-          asm volatile("prefetch.global.L2 [%0];" ::"l"(reinterpret_cast<const uint8_t *>(fblk) + 128));
-        }
-        if (use > 0 && !mbar_wait(BAR(4 + s), (use - 1) & 1, abort_flag))
-          ok = false;
-        ok = __all_sync(0xffffffffu, ok); // the warp leaves together: its lanes meet at the arrive below
-        if (!ok)
-          return;
-        uint8_t *wdst = smem + s * F16_STAGE_BYTES + r * 16 + (4 * hsel) * (F16_TILE_N * 16);
+      // the two blocks of a stage: 16 nibble bytes each = four words = four 16-byte chunks of halves
+      const uint8_t *blk0 = smem + F16_OFF_RAW + (r >> 3) * 144;
+      uint2 q[4];
+      uint16_t dbits[2];
+      auto fetch = [&](int st) {
+        if (!raw_wait(st))
+          return false;
+        const uint8_t *blk = blk0 + (st % F16_RAW) * f16_raw_bytes(QT);
 #pragma unroll
-        for (int wi = 0; wi < 4; ++wi) // chunk wi: elements 4wi + {0,2,1,3} then 16 + 4wi + {0,2,1,3} of the block
-          *reinterpret_cast<uint4 *>(wdst + wi * (F16_TILE_N * 16)) =
-            make_uint4(expand2_q40(w[wi] & 0x000f000fu, d2), expand2_q40((w[wi] >> 8) & 0x000f000fu, d2),
-                       expand2_q40((w[wi] >> 4) & 0x000f000fu, d2), expand2_q40((w[wi] >> 12) & 0x000f000fu, d2));
-        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-        __syncwarp(); // every lane's writes are fenced; one arrival per warp keeps the barrier word off the critical path
-        if (lane == 0)
-          mbar_arrive(BAR(s));
+        for (int k = 0; k < 2; ++k) {
+          q[2 * k] = *reinterpret_cast<const uint2 *>(blk + k * (32 * 144) + 16 + 8 * j);
+          q[2 * k + 1] = *reinterpret_cast<const uint2 *>(blk + k * (32 * 144) + 80 + 8 * j);
+          dbits[k] = *reinterpret_cast<const uint16_t *>(blk + k * (32 * 144) + 2 * j);
+        }
+        raw_done(st, q[0].x ^ q[1].x ^ q[2].x ^ q[3].x ^ dbits[0] ^ dbits[1]);
+        return true;
       };
-      StageIn in0, in1;
-      fetch(in0, 0);
-      fetch(in1, n_stages > 1 ? 1 : 0);
-      for (int st = 0; st < n_stages && ok; st += 2) { // n_stages may be odd (K = 2880)
-        stage(in0, st);
-        if (ok && st + 1 < n_stages)
-          stage(in1, st + 1);
+      ok = hsel >= n_stages || fetch(hsel); // n_stages may be odd (K = 2880)
+      for (int st = hsel; st < n_stages && ok; st += 2) {
+        if (!(ok = slot_wait(st)))
+          break;
+        uint8_t *wdst = smem + (st % F16_STAGES) * F16_STAGE_BYTES + r * 16;
+#pragma unroll
+        for (int k = 0; k < 2; ++k) {
+          const __half2 d2 = __half2half2(__ushort_as_half(dbits[k]));
+          const uint32_t w[4] = {q[2 * k].x ^ 0x88888888u, q[2 * k].y ^ 0x88888888u, q[2 * k + 1].x ^ 0x88888888u,
+                                 q[2 * k + 1].y ^ 0x88888888u};
+#pragma unroll
+          for (int wi = 0; wi < 4; ++wi) // chunk wi: elements 4wi + {0,2,1,3} then 16 + 4wi + {0,2,1,3} of the block
+            *reinterpret_cast<uint4 *>(wdst + (4 * k + wi) * (F16_TILE_N * 16)) =
+              make_uint4(expand2_q40(w[wi] & 0x000f000fu, d2), expand2_q40((w[wi] >> 8) & 0x000f000fu, d2),
+                         expand2_q40((w[wi] >> 4) & 0x000f000fu, d2), expand2_q40((w[wi] >> 12) & 0x000f000fu, d2));
+        }
+        stage_done(st);
+        ok = st + 2 >= n_stages || fetch(st + 2);
       }
     }
     /* ------------------------------ epilogue ------------------------------- */
-    if (ok && mbar_wait(BAR(8), 0, abort_flag)) {
+    if (__all_sync(0xffffffffu, ok && mbar_wait(BAR(8), 0, abort_flag))) {
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+      // A lane holds a row of the accumulator; stored as it is, a store instruction would touch 32 rows of C with 16 bytes
+      // each (27 of a tile's 142 thousand clocks). Every warp turns its 32 x 64 part round in the stages' memory, which is free
+      // now, and writes two rows of 256 bytes per instruction.
       const int quad = warp & 3, cg = warp >> 2; // lanes 32*quad.., columns 64*cg..
+      constexpr int PITCH = 68;                  // floats: 16-byte pieces of neighbouring rows fall into different banks
+      float *turn = reinterpret_cast<float *>(smem) + warp * (32 * PITCH);
+      const int col0 = nt * F16_TILE_N + cg * 64, cc = col0 + 4 * (lane & 15);
       for (int hm = 0; hm < (two ? 2 : 1); ++hm) {
-        const int row = (mt + hm) * F16_TILE_M + quad * 32 + lane;
+        const int row0 = (mt + hm) * F16_TILE_M + quad * 32;
         const uint32_t trow = tmem + ((uint32_t)(quad * 32) << 16) + hm * 256 + cg * 64;
-        float *dst = C + (size_t)row * ldc + nt * F16_TILE_N + cg * 64;
-#pragma unroll 1
-        for (int ch = 0; ch < 4; ++ch) {
-          uint32_t v[16];
-          tmem_ld16(trow + ch * 16, v);
+#pragma unroll
+        for (int half = 0; half < 2; ++half) { // two loads in flight
+          uint32_t v[2][16];
+          tmem_ld16(trow + half * 32, v[0]);
+          tmem_ld16(trow + half * 32 + 16, v[1]);
           asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-          const int col0 = nt * F16_TILE_N + cg * 64 + ch * 16;
-          if (row < M && col0 + 16 <= N) {
-            if (c_vec4) {
 #pragma unroll
-              for (int i = 0; i < 16; i += 4)
-                *reinterpret_cast<float4 *>(dst + ch * 16 + i) =
-                  make_float4(__uint_as_float(v[i]), __uint_as_float(v[i + 1]), __uint_as_float(v[i + 2]),
-                              __uint_as_float(v[i + 3]));
+          for (int k = 0; k < 2; ++k)
+#pragma unroll
+            for (int i = 0; i < 16; i += 4)
+              *reinterpret_cast<uint4 *>(turn + lane * PITCH + half * 32 + k * 16 + i) =
+                make_uint4(v[k][i], v[k][i + 1], v[k][i + 2], v[k][i + 3]);
+        }
+        __syncwarp();
+#pragma unroll 4
+        for (int i = 0; i < 16; ++i) {
+          const int rr = 2 * i + (lane >> 4), row = row0 + rr;
+          const float4 f = *reinterpret_cast<const float4 *>(turn + rr * PITCH + 4 * (lane & 15));
+          if (row < M) {
+            float *dst = C + (size_t)row * ldc + cc;
+            if (c_vec4 && cc + 4 <= N) {
+              *reinterpret_cast<float4 *>(dst) = f;
             } else {
-#pragma unroll
-              for (int i = 0; i < 16; ++i)
-                dst[ch * 16 + i] = __uint_as_float(v[i]);
+              if (cc < N)
+                dst[0] = f.x;
+              if (cc + 1 < N)
+                dst[1] = f.y;
+              if (cc + 2 < N)
+                dst[2] = f.z;
+              if (cc + 3 < N)
+                dst[3] = f.w;
             }
-          } else if (row < M) {
-#pragma unroll
-            for (int i = 0; i < 16; ++i)
-              if (col0 + i < N)
-                dst[ch * 16 + i] = __uint_as_float(v[i]);
           }
         }
+        __syncwarp(); // the area is rewritten by the second activation tile
       }
     }
   } else if (warp == F16_COPY_WARP) {
@@ -402,6 +437,7 @@ gemm_f16_kernel(const uint8_t *__restrict__ atiles, const uint8_t *__restrict__ 
     // its MMAs have retired, whatever the producers are doing.
     if (lane == 0) {
       const uint8_t *asrc = atiles + (size_t)mt * n_stages * F16_A_BYTES;
+      pdl_wait(); // the quantizer's tiles; the weights do not depend on the kernel before
       for (int st = 0; st < n_stages; ++st) {
         const int s = st % F16_STAGES, use = st / F16_STAGES;
         if (use > 0 && !mbar_wait(BAR(4 + s), (use - 1) & 1, abort_flag))
@@ -411,6 +447,34 @@ gemm_f16_kernel(const uint8_t *__restrict__ atiles, const uint8_t *__restrict__ 
         if (two)
           bulk_g2s(sbase + s * F16_STAGE_BYTES + F16_W_BYTES + F16_A_BYTES, asrc + ((size_t)n_stages + st) * F16_A_BYTES,
                    F16_A_BYTES, BAR(s));
+      }
+    }
+    __syncwarp();
+  } else if (warp == F16_RAW_WARP) {
+    /* ---------------------------- packed weights ---------------------------- */
+    // The latency of HBM and L2 is in this ring and the producers never wait for a load they issued themselves. Tiled
+    // copies, a box of 32 row groups x 128 (Q4_0: 144) bytes each: 32 untiled copies of 256 bytes per stage measured 1.6 times
+    // slower than no ring at all.
+    if (QT != NNTR_Q6_K && lane == 0) {
+      constexpr int BOX = QT == NNTR_Q4_K ? 128 : 144;
+      for (int st = 0; st < n_stages; ++st) {
+        const int rs = st % F16_RAW, use = st / F16_RAW;
+        if (use > 0 && !mbar_wait(BAR(12 + rs), (use - 1) & 1, abort_flag))
+          break;
+        mbar_expect_tx(BAR(9 + rs), f16_raw_bytes(QT));
+        const uint32_t dst = sbase + F16_OFF_RAW + rs * f16_raw_bytes(QT);
+        int x = st * 2 * (int)sizeof(BlockQ40x8);
+        if (QT == NNTR_Q4_K) {
+          x = (st >> 2) * (int)sizeof(BlockQ4Kx8);
+          if ((st & 3) == 0) { // two headers: the one replaced was last read three stages before the ones waited for so far
+            const int hb = (st >> 2) & 1;
+            mbar_expect_tx(BAR(14 + hb), F16_HDR_BYTES);
+            tma_tile(sbase + f16_off_hdr(QT) + hb * F16_HDR_BYTES, &wmap, x, nt * (F16_TILE_N / 8), BAR(14 + hb));
+          }
+          x += 128 + 256 * (st & 3);
+        }
+        tma_tile(dst, &wmap, x, nt * (F16_TILE_N / 8), BAR(9 + rs));
+        tma_tile(dst + 32 * BOX, &wmap, x + BOX, nt * (F16_TILE_N / 8), BAR(9 + rs));
       }
     }
     __syncwarp();
@@ -550,6 +614,23 @@ quantize_q8_0_f16_tiles_kernel(const float *__restrict__ x, int64_t ldx, uint8_t
   }
 }
 
+/** The GEMM behind its quantizer, started while that runs: barriers, tensor memory and the first packed weights are ready
+ *  when the activation tiles are (pdl_wait of the copy warp). */
+template <typename... P, typename... A>
+cudaError_t launch_after(void (*kernel)(P...), dim3 grid, int smem, cudaStream_t st, A... args) {
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid;
+  cfg.blockDim = F16_THREADS;
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = st;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, kernel, (P)args...);
+}
+
 } // namespace
 
 size_t umma_f16_workspace_bytes(unsigned M, unsigned K) {
@@ -572,9 +653,9 @@ int launch_gemm_f16(int qtype, unsigned M, unsigned N, unsigned K, const float *
   int dev = 0;
   NNTR_CHECK_CUDA(cudaGetDevice(&dev));
   if (dev < 64 && !attr_set[dev]) {
-    NNTR_CHECK_CUDA(cudaFuncSetAttribute(gemm_f16_kernel<NNTR_Q4_K>, cudaFuncAttributeMaxDynamicSharedMemorySize, F16_SMEM));
-    NNTR_CHECK_CUDA(cudaFuncSetAttribute(gemm_f16_kernel<NNTR_Q4_0>, cudaFuncAttributeMaxDynamicSharedMemorySize, F16_SMEM));
-    NNTR_CHECK_CUDA(cudaFuncSetAttribute(gemm_f16_kernel<NNTR_Q6_K>, cudaFuncAttributeMaxDynamicSharedMemorySize, F16_SMEM));
+    NNTR_CHECK_CUDA(cudaFuncSetAttribute(gemm_f16_kernel<NNTR_Q4_K>, cudaFuncAttributeMaxDynamicSharedMemorySize, f16_smem(NNTR_Q4_K)));
+    NNTR_CHECK_CUDA(cudaFuncSetAttribute(gemm_f16_kernel<NNTR_Q4_0>, cudaFuncAttributeMaxDynamicSharedMemorySize, f16_smem(NNTR_Q4_0)));
+    NNTR_CHECK_CUDA(cudaFuncSetAttribute(gemm_f16_kernel<NNTR_Q6_K>, cudaFuncAttributeMaxDynamicSharedMemorySize, f16_smem(NNTR_Q6_K)));
     attr_set[dev] = true;
   }
   const int mtiles = (int)((M + F16_TILE_M - 1) / F16_TILE_M), Mpad = mtiles * F16_TILE_M;
@@ -583,6 +664,16 @@ int launch_gemm_f16(int qtype, unsigned M, unsigned N, unsigned K, const float *
   const int c_vec4 = (ldc % 4 == 0) && !(reinterpret_cast<uintptr_t>(C) & 15);
   dim3 grid((mtiles + 1) / 2, (N + F16_TILE_N - 1) / F16_TILE_N);
   const int n_stages = (int)(K / F16_KS);
+  const uint8_t *tiles = static_cast<const uint8_t *>(ws), *W = static_cast<const uint8_t *>(B);
+  CUtensorMap wmap = {};
+  if (qtype != NNTR_Q6_K) { // rows of 8-row groups of packed weights
+    const uint64_t row = qtype == NNTR_Q4_K ? (uint64_t)(K / QK_K) * sizeof(BlockQ4Kx8) : (uint64_t)(K / 32) * sizeof(BlockQ40x8);
+    if (reinterpret_cast<uintptr_t>(B) & 15)
+      return set_error(NNTR_CUDA_ERR_INVALID, "gemm (fp16 tensor path): weights must be 16-byte aligned");
+    const int rc = encode_map_2d(&wmap, B, 1, row, N / 8, row, qtype == NNTR_Q4_K ? 128 : 144, 32, false);
+    if (rc)
+      return rc;
+  }
   if (qtype == NNTR_Q4_K || qtype == NNTR_Q6_K) {
     const int nb = (int)(K / QK_K);
     // Q4_K: rows below 4*floor(M/4) with the 4-row quantizer's sign rule; Q6_K: the row quantizer for every row
@@ -594,22 +685,19 @@ int launch_gemm_f16(int qtype, unsigned M, unsigned N, unsigned K, const float *
     count_launch();
     NNTR_CHECK_CUDA(cudaGetLastError());
     if (qtype == NNTR_Q4_K)
-      gemm_f16_kernel<NNTR_Q4_K><<<grid, F16_THREADS, F16_SMEM, st>>>(static_cast<const uint8_t *>(ws),
-                                                                      static_cast<const uint8_t *>(B), C, (int)ldc, (int)M,
-                                                                      (int)N, n_stages, mtiles, c_vec4);
+      NNTR_CHECK_CUDA(launch_after(gemm_f16_kernel<NNTR_Q4_K>, grid, f16_smem(NNTR_Q4_K), st, wmap, tiles, W, C, (int)ldc, (int)M, (int)N,
+                                   n_stages, mtiles, c_vec4));
     else
-      gemm_f16_kernel<NNTR_Q6_K><<<grid, F16_THREADS, F16_SMEM, st>>>(static_cast<const uint8_t *>(ws),
-                                                                      static_cast<const uint8_t *>(B), C, (int)ldc, (int)M,
-                                                                      (int)N, n_stages, mtiles, c_vec4);
+      NNTR_CHECK_CUDA(launch_after(gemm_f16_kernel<NNTR_Q6_K>, grid, f16_smem(NNTR_Q6_K), st, wmap, tiles, W, C, (int)ldc, (int)M, (int)N,
+                                   n_stages, mtiles, c_vec4));
   } else {
     const int64_t nwarps = (int64_t)Mpad * ((K + 255) / 256);
     quantize_q8_0_f16_tiles_kernel<<<(unsigned)((nwarps + 7) / 8), 256, 0, st>>>(A, K, static_cast<uint8_t *>(ws), (int)M,
                                                                                Mpad, (int)K);
     count_launch();
     NNTR_CHECK_CUDA(cudaGetLastError());
-    gemm_f16_kernel<NNTR_Q4_0><<<grid, F16_THREADS, F16_SMEM, st>>>(static_cast<const uint8_t *>(ws),
-                                                                    static_cast<const uint8_t *>(B), C, (int)ldc, (int)M,
-                                                                    (int)N, n_stages, mtiles, c_vec4);
+    NNTR_CHECK_CUDA(launch_after(gemm_f16_kernel<NNTR_Q4_0>, grid, f16_smem(NNTR_Q4_0), st, wmap, tiles, W, C, (int)ldc, (int)M, (int)N,
+                                   n_stages, mtiles, c_vec4));
   }
   count_launch();
   return check_cuda(cudaGetLastError(), "gemm fp16 tensor-path launch");

@@ -192,6 +192,31 @@ def test_fp16_tensor_gemm_q6_K_matches_checker(be, port, M, N, K):
     assert not np.array_equal(got.view(np.uint32), want.view(np.uint32)), "auto took the tensor path"
 
 
+@pytest.mark.parametrize("q,K", [("q4_0", 64), ("q4_0", 192), ("q4_0", 2880), ("q4_K", 256), ("q4_K", 2560)])
+def test_fp16_tensor_gemm_every_tile_sees_the_same_weights(be, q, K):
+    """A stage's expanded weights meet one or two tiles of 128 rows, and the stages ahead of the MMAs run differently far
+    in the two cases; a row's sum does not depend on it, so the calls agree bit for bit, repeatedly. One stage, an odd
+    count, many. An odd row stride of C takes the scalar stores."""
+    gen = {"q4_0": O.random_q4_0x8, "q4_K": O.random_q4_Kx8}[q]
+    rng = np.random.default_rng(K)
+    N = 20 * 256
+    B = torch.from_numpy(gen(rng, N, K)).cuda()
+    A = torch.from_numpy(rng.standard_normal((256, K)).astype(np.float32)).cuda()
+
+    def call(a, ldc):
+        C = torch.full((a.shape[0], ldc), float("nan"), device="cuda")
+        be.set_gemm_path("tensor_f16")
+        getattr(be, f"gemm_{q}")(a.shape[0], N, K, a, K, B, N, C, ldc)
+        be.set_gemm_path("auto")
+        assert bool(C[:, N:].isnan().all())
+        return C[:, :N].contiguous().view(torch.int32)
+
+    halves = torch.cat([call(A[:128].contiguous(), N + 1), call(A[128:].contiguous(), N)])
+    for ldc in (N, N + 1) * 5:
+        assert torch.equal(call(A, ldc), halves)
+    be.device_status()
+
+
 def test_int8_peak_measurement_is_plausible(be):
     """The int8 rate the prefill fraction is quoted against: a dense tcgen05 kind::i8 stream on every SM. A B200 is
     specified at 4.5 POP/s dense; anything outside 1.5 .. 6 POP/s means the measurement is not doing the work."""
