@@ -655,7 +655,7 @@ int launch_gemv_q4_K_batched(unsigned N, unsigned K, const float *x, const void 
   const long blocks_per_sm = ((long)n_groups * nb * n_problems * (pair ? 2 : 1) + sms - 1) / sms;
   const bool two_fit = 2u * smem_layout(nb, ngslot, pair ? 64 : 0).total <= 220u * 1024u;
   const int per_sm = env_int("NNTR_CUDA_GEMV_CTAS_PER_SM", (blocks_per_sm > STEP_BLOCKS && two_fit) ? 2 : 1);
-  int max_ctas = (sms * per_sm + (int)n_problems - 1) / (int)n_problems; // CTAs per problem
+  int max_ctas = sms * per_sm / (int)n_problems; // CTAs per problem, rounded down: the batch is one wave
   if (max_ctas < 1)
     max_ctas = 1;
   const unsigned grid = (unsigned)(n_groups < max_ctas ? n_groups : max_ctas);

@@ -46,7 +46,14 @@ struct MoeEp {
   unsigned long long parity_stride; // elements between the two alternating expert-output buffers
 };
 
-constexpr unsigned GROUPED_MIN_TOKENS = 8; // from here on the pairs are sorted by expert and run as per-expert GEMMs
+/* From where on the pairs are sorted by expert and run as per-expert GEMMs (all of a batch's rows for one read of an expert's
+ * weights, but three launches more than a GEMV per pair). Q4_0: from two tokens; 4 of 32 experts of 2880 x 2880, 2 / 4 / 6
+ * tokens: 64 / 84 / 91 us against 68 / 124 / 164. Q4_K: while three CTAs per pair still fit one wave of two per SM the pairs
+ * win: 8 of 128 experts of 2048 x 768, 8 / 12 / 14 tokens: 60 / 77 / 104 us against 71 / 88 / 92. */
+constexpr unsigned GROUPED_MIN_TOKENS = 2;
+static bool run_grouped(int qtype, unsigned tokens, unsigned pairs) {
+  return tokens >= GROUPED_MIN_TOKENS && (qtype == NNTR_Q4_0 || 3 * pairs > 2 * (unsigned)sm_count());
+}
 constexpr int MOE_COUNTER_TOKENS = 4096;   // arrival counters kept at the start of the scratch for up to this many tokens
 constexpr int ROUTER_WARPS = 8;
 constexpr int ROUTER_SLICES = 32; // CTAs per token
@@ -564,7 +571,8 @@ __global__ void moe_combine_kernel(const float *__restrict__ dn, const int *__re
     return;
   const long t = i / H;
   const int h = (int)(i - t * H);
-  const float4 v = moe_combine_elem4(dn, idx, ord, w, down_b, t, h, H, topk);
+  const float4 v = topk <= 4 ? moe_combine_elem4<4>(dn, idx, ord, w, down_b, t, h, H, topk)
+                             : moe_combine_elem4<8>(dn, idx, ord, w, down_b, t, h, H, topk);
   if (!(reinterpret_cast<uintptr_t>(y) & 15))
     *reinterpret_cast<float4 *>(y + i) = v;
   else
@@ -775,7 +783,7 @@ static int moe_forward(const nntr_moe_desc *d, const nntr_moe_ep *epd, unsigned 
   float *dn = reinterpret_cast<float *>(ws + s.dn);
   const unsigned P = tokens * K;
 
-  const bool grouped = !epd && tokens >= GROUPED_MIN_TOKENS;
+  const bool grouped = !epd && run_grouped(d->qtype, tokens, P);
   // the arrival counters start at zero (the workspace is zero-filled before its first use) and the last arriver of
   // every token puts its counter back, so no clearing launch is needed
   if (tokens > (unsigned)MOE_COUNTER_TOKENS)

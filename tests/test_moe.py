@@ -315,6 +315,32 @@ def test_selection_margin_is_far_above_what_the_summation_order_can_move(be, por
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("q,T,E,k", [("q4_0", 2, 8, 4), ("q4_0", 5, 8, 6), ("q4_K", 2, 16, 8), ("q4_K", 12, 128, 8),
+                                     ("q4_K", 13, 128, 8)])
+def test_a_batch_equals_its_tokens_one_by_one_around_the_grouping_lines(be, q, T, E, k):
+    """One token always runs a GEMV per (token, expert) pair. Two tokens of Q4_0 experts, and Q4_K batches whose pairs no
+    longer fit one wave of the GPU, are grouped by expert; either way a row keeps its float chain, so the bits agree."""
+    import torch
+    rng = np.random.default_rng(T * 10 + k)
+    H, I = (352, 320) if q == "q4_0" else (512, 256)
+    gen = O.random_q4_0x8 if q == "q4_0" else O.random_q4_Kx8
+    cu = lambda arrs: [torch.from_numpy(a).cuda() for a in arrs]
+    pool = [cu([gen(rng, n, m) for _ in range(4)]) for n, m in ((I, H), (I, H), (H, I))]
+    gate, up, down = ([p[e % 4] for e in range(E)] for p in pool)
+    kw = {}
+    if q == "q4_0":
+        kw = dict(kind=1, alpha=1.702, router_bias=torch.zeros(E, device="cuda"),
+                  **{n: [torch.randn(w, device="cuda") for _ in range(E)] for n, w in (("gate_b", I), ("up_b", I), ("down_b", H))})
+    router = torch.from_numpy((rng.standard_normal((H, E)) * 0.02).astype(np.float32)).cuda()
+    layer = be.MoeLayer(router, gate, up, down, k, qtype=q, **kw)
+    x = torch.from_numpy(rng.standard_normal((T, H)).astype(np.float32)).cuda()
+    got = layer.forward(x).clone()
+    single = torch.cat([layer.forward(x[i:i + 1].contiguous()).clone() for i in range(T)])
+    be.device_status()
+    assert torch.equal(got.view(torch.int32), single.view(torch.int32))
+
+
+@pytest.mark.gpu
 @pytest.mark.parametrize("T,H,I,E,k", [(8, 512, 256, 16, 4), (37, 512, 256, 16, 4), (256, 2048, 768, 128, 8)])
 def test_grouped_prefill_equals_the_per_pair_path_bit_for_bit(be, port, T, H, I, E, k):
     """From 8 tokens on the layer sorts the (token, expert) pairs by expert and runs per-expert grouped GEMMs with a
