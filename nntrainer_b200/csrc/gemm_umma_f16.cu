@@ -50,12 +50,18 @@
  * groups, one group's latencies pass while the other expands. The tile's stores took 27 of its 142 thousand clocks while
  * every lane wrote a row of its own. Both changes, 1024 x 24576 x 4096 Q4_K: 221 -> 192 us (1076 TFLOP/s), 256 rows
  * 74 -> 65, Q4_0 1024 rows 201 -> 186; Q6_K 256 x 151936 x 2560 552 -> 359 (the stores).
+ *
+ * Few tiles: a cluster of two, four or eight CTAs shares a tile, each walks a part of K (k_parts), and the sums are added
+ * through distributed shared memory. 512 x 1280 x 2560: Q4_0 40 -> 25 us, Q6_K 69 -> 33; 128 x 2560 x 8192: Q4_0 93 -> 25,
+ * Q6_K 268 -> 49.
  */
 #include "common.cuh"
 #include "pipeline.cuh"
 #include "tma_map.cuh"
 
 #include <cuda_fp16.h>
+
+#include <atomic>
 
 namespace nntr {
 
@@ -104,6 +110,31 @@ __device__ __forceinline__ void umma_f16(uint32_t tmem_d, uint64_t da, uint64_t 
                "l"(da), "l"(db), "r"(idesc), "r"(accumulate)
                : "memory");
 }
+__device__ __forceinline__ int cluster_size() {
+  uint32_t n;
+  asm("mov.u32 %0, %%cluster_nctaid.x;" : "=r"(n));
+  return (int)n;
+}
+__device__ __forceinline__ int cluster_rank() {
+  uint32_t n;
+  asm("mov.u32 %0, %%cluster_ctarank;" : "=r"(n));
+  return (int)n;
+}
+__device__ __forceinline__ void cluster_sync() {
+  asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+  asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+/** four floats at a shared address (of this CTA's window) in the CTA of the given rank */
+__device__ __forceinline__ float4 ld_cluster4(uint32_t addr, int rank) {
+  uint32_t remote;
+  float4 v;
+  asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(remote) : "r"(addr), "r"(rank));
+  asm volatile("ld.shared::cluster.v4.f32 {%0,%1,%2,%3}, [%4];"
+               : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w)
+               : "r"(remote)
+               : "memory");
+  return v;
+}
 __device__ __forceinline__ void umma_commit(uint32_t bar) {
   asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar) : "memory");
 }
@@ -143,15 +174,16 @@ __device__ __forceinline__ uint32_t expand2_q40(uint32_t nib2, __half2 d) {
   return *reinterpret_cast<const uint32_t *>(&w);
 }
 
-/* QT = NNTR_Q4_K: W is block_q4_Kx8, a stage is one pair of sub-blocks (n_stages = 4 * K/256).
- * QT = NNTR_Q4_0: W is block_q4_0x8, a stage is two 32-weight blocks (n_stages = K/64).
+/* QT = NNTR_Q4_K: W is block_q4_Kx8, a stage is one pair of sub-blocks (k_stages = 4 * K/256).
+ * QT = NNTR_Q4_0: W is block_q4_0x8, a stage is two 32-weight blocks (k_stages = K/64).
  * QT = NNTR_Q6_K: W is plain rows of block_q6_K (210 bytes, 2-byte aligned); stage (b, h, s2) of super-block b holds
  *                 the quarters s2 and s2 + 2 of its 128-element half h (the two quarters that share the bytes ql[64h +
- *                 32 s2 ..] as low and high nibbles); n_stages = 4 * K/256. N may end inside the last 256-row tile. */
+ *                 32 s2 ..] as low and high nibbles); k_stages = 4 * K/256. N may end inside the last 256-row tile. */
 template <int QT>
 __global__ void __launch_bounds__(F16_THREADS, 1)
 gemm_f16_kernel(const __grid_constant__ CUtensorMap wmap, const uint8_t *__restrict__ atiles, const uint8_t *__restrict__ Wb,
-                float *__restrict__ C, int ldc, int M, int N, int n_stages, int m_tiles, int c_vec4) {
+                float *__restrict__ C, int ldc, int M, int N, int k_stages, int m_tiles, int tiles_per_cta,
+                int c_vec4) {
   extern __shared__ __align__(128) uint8_t smem[];
   // bars: [0..3] full, [4..7] empty, [8] tile complete, [9..10] packed weights here, [12..13] packed weights read,
   // [14..15] Q4_K headers here
@@ -161,10 +193,15 @@ gemm_f16_kernel(const __grid_constant__ CUtensorMap wmap, const uint8_t *__restr
   uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(smem + f16_off_bars(QT) + 128);
   volatile int *abort_flag = reinterpret_cast<volatile int *>(smem + f16_off_bars(QT) + 136);
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  // a CTA takes two 128-row activation tiles (2*blockIdx.x, +1) against the same 256 weight rows: the expanded
+  // a CTA takes two 128-row activation tiles (unless there are SMs to spare) against the same 256 weight rows: the expanded
   // weights of a stage feed two MMAs, which halves the expansion work per output
-  const int mt = 2 * blockIdx.x, nt = blockIdx.y;
-  const bool two = mt + 1 < m_tiles;
+  // the CTAs of a cluster share a tile: each walks its part of K, whole super-blocks (Q6_K: halves; Q4_0: pairs of blocks)
+  const int parts = cluster_size(), part = cluster_rank();
+  const int mt = tiles_per_cta * (blockIdx.x / parts), nt = blockIdx.y;
+  const bool two = tiles_per_cta == 2 && mt + 1 < m_tiles;
+  constexpr int UNIT = QT == NNTR_Q4_K ? 4 : QT == NNTR_Q6_K ? 2 : 1;
+  const int units = k_stages / UNIT;
+  const int st0 = units * part / parts * UNIT, n_stages = units * (part + 1) / parts * UNIT - st0; // stages st0 ..
 
   if (tid == 0) {
     for (int s = 0; s < F16_STAGES; ++s) {
@@ -189,6 +226,45 @@ gemm_f16_kernel(const __grid_constant__ CUtensorMap wmap, const uint8_t *__restr
   __syncthreads();
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
   const uint32_t tmem = *tmem_slot;
+
+  // Epilogue. A lane holds a row of the accumulator; stored as it is, a store instruction would touch 32 rows of C with 16
+  // bytes each (27 of a tile's 142 thousand clocks). Every warp turns its 32 x 64 part round in the stages' memory, which is
+  // free then, and whole lines are written from there.
+  constexpr int PITCH = 68; // floats: 16-byte pieces of neighbouring rows fall into different banks
+  bool tile_done = false;   // warps 0-15: all MMAs have retired
+  auto turn_area = [&](int w) { return w * (32 * PITCH); }; // of the warp with lanes 32 * (w & 3) .., columns 64 * (w >> 2) ..
+  auto turn_round = [&](int hm) {
+    const uint32_t trow = tmem + ((uint32_t)((warp & 3) * 32) << 16) + hm * 256 + (warp >> 2) * 64;
+    float *turn = reinterpret_cast<float *>(smem) + turn_area(warp);
+#pragma unroll
+    for (int half = 0; half < 2; ++half) { // two loads in flight
+      uint32_t v[2][16];
+      tmem_ld16(trow + half * 32, v[0]);
+      tmem_ld16(trow + half * 32 + 16, v[1]);
+      asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+#pragma unroll
+      for (int k = 0; k < 2; ++k)
+#pragma unroll
+        for (int i = 0; i < 16; i += 4)
+          *reinterpret_cast<uint4 *>(turn + lane * PITCH + half * 32 + k * 16 + i) =
+            make_uint4(v[k][i], v[k][i + 1], v[k][i + 2], v[k][i + 3]);
+    }
+  };
+  auto store4 = [&](int row, int col, const float4 &f) {
+    float *dst = C + (size_t)row * ldc + col;
+    if (c_vec4 && col + 4 <= N) {
+      *reinterpret_cast<float4 *>(dst) = f;
+    } else {
+      if (col < N)
+        dst[0] = f.x;
+      if (col + 1 < N)
+        dst[1] = f.y;
+      if (col + 2 < N)
+        dst[2] = f.z;
+      if (col + 3 < N)
+        dst[3] = f.w;
+    }
+  };
 
   if (warp < F16_MMA_WARP) {
     /* ------------------------------ producers ------------------------------ */
@@ -272,14 +348,14 @@ gemm_f16_kernel(const __grid_constant__ CUtensorMap wmap, const uint8_t *__restr
     } else if constexpr (QT == NNTR_Q6_K) {
       const int n_row = nt * F16_TILE_N + r;
       const bool have_row = n_row < N; // rows beyond N: scale 0, so zero weights (their columns are not stored either)
-      const int nb = n_stages / 4, n_groups = n_stages / 2;
+      const int nb = k_stages / 4, n_groups = n_stages / 2, g0 = st0 / 2;
       const uint8_t *wrow = Wb + (size_t)(have_row ? n_row : 0) * nb * sizeof(BlockQ6K);
       // A group is the two stages of one half h of a super-block: they share the 32 qh bytes. This thread: bytes
       // 16*hsel .. +15 of each stage's 32 ql bytes and of the qh bytes, each read as five aligned words and
       // funnel-shifted (blocks are 2-byte aligned), the four scales of its 16-element slices, and d.
       uint32_t rl[2][5], rh[5], rs = 0, rd = 0;
       auto fetch = [&](int g) {
-        const int b = g >> 1, h = g & 1;
+        const int b = (g0 + g) >> 1, h = (g0 + g) & 1;
         const uint8_t *blk = wrow + (size_t)b * sizeof(BlockQ6K);
         const uint32_t *al =
           reinterpret_cast<const uint32_t *>(reinterpret_cast<uintptr_t>(blk + 64 * h + 16 * hsel) & ~(uintptr_t)3);
@@ -297,7 +373,7 @@ gemm_f16_kernel(const __grid_constant__ CUtensorMap wmap, const uint8_t *__restr
       };
       fetch(0);
       for (int g = 0; g < n_groups && ok; ++g) {
-        const uint32_t sh = (uint32_t)((reinterpret_cast<uintptr_t>(wrow) + (size_t)(g >> 1) * sizeof(BlockQ6K)) & 2) * 8;
+        const uint32_t sh = (uint32_t)((reinterpret_cast<uintptr_t>(wrow) + (size_t)((g0 + g) >> 1) * sizeof(BlockQ6K)) & 2) * 8;
         uint32_t ql[2][4], qh[4];
 #pragma unroll
         for (int k = 0; k < 4; ++k) {
@@ -382,53 +458,25 @@ gemm_f16_kernel(const __grid_constant__ CUtensorMap wmap, const uint8_t *__restr
       }
     }
     /* ------------------------------ epilogue ------------------------------- */
-    if (__all_sync(0xffffffffu, ok && mbar_wait(BAR(8), 0, abort_flag))) {
+    tile_done = __all_sync(0xffffffffu, ok && mbar_wait(BAR(8), 0, abort_flag)) != 0;
+    if (tile_done) {
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-      // A lane holds a row of the accumulator; stored as it is, a store instruction would touch 32 rows of C with 16 bytes
-      // each (27 of a tile's 142 thousand clocks). Every warp turns its 32 x 64 part round in the stages' memory, which is free
-      // now, and writes two rows of 256 bytes per instruction.
-      const int quad = warp & 3, cg = warp >> 2; // lanes 32*quad.., columns 64*cg..
-      constexpr int PITCH = 68;                  // floats: 16-byte pieces of neighbouring rows fall into different banks
-      float *turn = reinterpret_cast<float *>(smem) + warp * (32 * PITCH);
-      const int col0 = nt * F16_TILE_N + cg * 64, cc = col0 + 4 * (lane & 15);
-      for (int hm = 0; hm < (two ? 2 : 1); ++hm) {
-        const int row0 = (mt + hm) * F16_TILE_M + quad * 32;
-        const uint32_t trow = tmem + ((uint32_t)(quad * 32) << 16) + hm * 256 + cg * 64;
-#pragma unroll
-        for (int half = 0; half < 2; ++half) { // two loads in flight
-          uint32_t v[2][16];
-          tmem_ld16(trow + half * 32, v[0]);
-          tmem_ld16(trow + half * 32 + 16, v[1]);
-          asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-#pragma unroll
-          for (int k = 0; k < 2; ++k)
-#pragma unroll
-            for (int i = 0; i < 16; i += 4)
-              *reinterpret_cast<uint4 *>(turn + lane * PITCH + half * 32 + k * 16 + i) =
-                make_uint4(v[k][i], v[k][i + 1], v[k][i + 2], v[k][i + 3]);
-        }
-        __syncwarp();
+      if (parts == 1) {
+        const float *turn = reinterpret_cast<const float *>(smem) + turn_area(warp);
+        const int cc = nt * F16_TILE_N + (warp >> 2) * 64 + 4 * (lane & 15);
+        for (int hm = 0; hm < (two ? 2 : 1); ++hm) {
+          const int row0 = (mt + hm) * F16_TILE_M + (warp & 3) * 32;
+          turn_round(hm);
+          __syncwarp();
 #pragma unroll 4
-        for (int i = 0; i < 16; ++i) {
-          const int rr = 2 * i + (lane >> 4), row = row0 + rr;
-          const float4 f = *reinterpret_cast<const float4 *>(turn + rr * PITCH + 4 * (lane & 15));
-          if (row < M) {
-            float *dst = C + (size_t)row * ldc + cc;
-            if (c_vec4 && cc + 4 <= N) {
-              *reinterpret_cast<float4 *>(dst) = f;
-            } else {
-              if (cc < N)
-                dst[0] = f.x;
-              if (cc + 1 < N)
-                dst[1] = f.y;
-              if (cc + 2 < N)
-                dst[2] = f.z;
-              if (cc + 3 < N)
-                dst[3] = f.w;
-            }
+          for (int i = 0; i < 16; ++i) { // two rows of 256 bytes per instruction
+            const int rr = 2 * i + (lane >> 4);
+            const float4 f = *reinterpret_cast<const float4 *>(turn + rr * PITCH + 4 * (lane & 15));
+            if (row0 + rr < M)
+              store4(row0 + rr, cc, f);
           }
+          __syncwarp(); // the area is rewritten by the second activation tile
         }
-        __syncwarp(); // the area is rewritten by the second activation tile
       }
     }
   } else if (warp == F16_COPY_WARP) {
@@ -436,7 +484,7 @@ gemm_f16_kernel(const __grid_constant__ CUtensorMap wmap, const uint8_t *__restr
     // A warp of its own keeps the activation stages as far ahead as the ring allows: a slot's copy starts the moment
     // its MMAs have retired, whatever the producers are doing.
     if (lane == 0) {
-      const uint8_t *asrc = atiles + (size_t)mt * n_stages * F16_A_BYTES;
+      const uint8_t *asrc = atiles + ((size_t)mt * k_stages + st0) * F16_A_BYTES;
       pdl_wait(); // the quantizer's tiles; the weights do not depend on the kernel before
       for (int st = 0; st < n_stages; ++st) {
         const int s = st % F16_STAGES, use = st / F16_STAGES;
@@ -445,7 +493,7 @@ gemm_f16_kernel(const __grid_constant__ CUtensorMap wmap, const uint8_t *__restr
         mbar_expect_tx(BAR(s), (two ? 2 : 1) * F16_A_BYTES);
         bulk_g2s(sbase + s * F16_STAGE_BYTES + F16_W_BYTES, asrc + (size_t)st * F16_A_BYTES, F16_A_BYTES, BAR(s));
         if (two)
-          bulk_g2s(sbase + s * F16_STAGE_BYTES + F16_W_BYTES + F16_A_BYTES, asrc + ((size_t)n_stages + st) * F16_A_BYTES,
+          bulk_g2s(sbase + s * F16_STAGE_BYTES + F16_W_BYTES + F16_A_BYTES, asrc + ((size_t)k_stages + st) * F16_A_BYTES,
                    F16_A_BYTES, BAR(s));
       }
     }
@@ -463,9 +511,9 @@ gemm_f16_kernel(const __grid_constant__ CUtensorMap wmap, const uint8_t *__restr
           break;
         mbar_expect_tx(BAR(9 + rs), f16_raw_bytes(QT));
         const uint32_t dst = sbase + F16_OFF_RAW + rs * f16_raw_bytes(QT);
-        int x = st * 2 * (int)sizeof(BlockQ40x8);
+        int x = (st0 + st) * 2 * (int)sizeof(BlockQ40x8);
         if (QT == NNTR_Q4_K) {
-          x = (st >> 2) * (int)sizeof(BlockQ4Kx8);
+          x = ((st0 + st) >> 2) * (int)sizeof(BlockQ4Kx8);
           if ((st & 3) == 0) { // two headers: the one replaced was last read three stages before the ones waited for so far
             const int hb = (st >> 2) & 1;
             mbar_expect_tx(BAR(14 + hb), F16_HDR_BYTES);
@@ -507,6 +555,34 @@ gemm_f16_kernel(const __grid_constant__ CUtensorMap wmap, const uint8_t *__restr
         umma_commit(BAR(8));
     }
     __syncwarp();
+  }
+
+  /* ------------------------------ a shared tile ------------------------------ */
+  // Every CTA of the cluster leaves its sums in its own shared memory; the rows are dealt out, and a CTA adds its rows' parts in
+  // the order of K. All threads pass all barriers, whatever went wrong before.
+  if (parts > 1) {
+    for (int hm = 0; hm < (two ? 2 : 1); ++hm) {
+      if (tile_done)
+        turn_round(hm);
+      cluster_sync();
+      const int row0 = (mt + hm) * F16_TILE_M, rows = min(F16_TILE_M, M - row0);
+      if (tile_done)
+        for (int i = tid; part + (i >> 6) * parts < rows; i += F16_PRODUCERS) {
+          const int r = part + (i >> 6) * parts, c = 4 * (i & 63);
+          const uint32_t at = sbase + 4u * (turn_area((r >> 5) + 4 * (c >> 6)) + (r & 31) * PITCH + (c & 63));
+          float4 v[8];
+#pragma unroll
+          for (int k = 0; k < 8; ++k)
+            if (k < parts)
+              v[k] = ld_cluster4(at, k);
+#pragma unroll
+          for (int k = 1; k < 8; ++k)
+            if (k < parts)
+              v[0] = make_float4(v[0].x + v[k].x, v[0].y + v[k].y, v[0].z + v[k].z, v[0].w + v[k].w);
+          store4(row0 + r, nt * F16_TILE_N + c, v[0]);
+        }
+      cluster_sync(); // the area is rewritten by the second activation tile, and nobody leaves while it is read
+    }
   }
 
   /* common tail: on an abort give copies and MMAs in flight time to land before the memory is released */
@@ -615,20 +691,57 @@ quantize_q8_0_f16_tiles_kernel(const float *__restrict__ x, int64_t ldx, uint8_t
 }
 
 /** The GEMM behind its quantizer, started while that runs: barriers, tensor memory and the first packed weights are ready
- *  when the activation tiles are (pdl_wait of the copy warp). */
+ *  when the activation tiles are (pdl_wait of the copy warp). Clusters of `parts` CTAs. */
 template <typename... P, typename... A>
-cudaError_t launch_after(void (*kernel)(P...), dim3 grid, int smem, cudaStream_t st, A... args) {
-  cudaLaunchAttribute attr[1];
+cudaError_t launch_after(void (*kernel)(P...), dim3 grid, int parts, int smem, cudaStream_t st, A... args) {
+  cudaLaunchAttribute attr[2];
   attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   attr[0].val.programmaticStreamSerializationAllowed = 1;
+  attr[1].id = cudaLaunchAttributeClusterDimension;
+  attr[1].val.clusterDim.x = parts;
+  attr[1].val.clusterDim.y = attr[1].val.clusterDim.z = 1;
   cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = grid;
+  cfg.gridDim = dim3(grid.x * parts, grid.y);
   cfg.blockDim = F16_THREADS;
   cfg.dynamicSmemBytes = smem;
   cfg.stream = st;
   cfg.attrs = attr;
-  cfg.numAttrs = 1;
+  cfg.numAttrs = parts > 1 ? 2 : 1;
   return cudaLaunchKernelEx(&cfg, kernel, (P)args...);
+}
+
+/** Into how many parts K is cut, so that few tiles still use the machine. A CTA alone walks K at 0.9 us (Q6_K 1.5) a stage
+ *  however many SMs are idle; the parts' sums cost about 2 us at the end. As many as still run in one wave of clusters, of at
+ *  least four stages each. */
+template <int QT> int k_parts(int tiles, int k_stages) {
+  static std::atomic<int> fit[64][3];
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || dev >= 64)
+    return 1;
+  for (int i = 2; i >= 0; --i) {
+    const int parts = 2 << i;
+    int n = fit[dev][i].load(std::memory_order_relaxed);
+    if (n == 0) { // clusters of that size that run at the same time
+      cudaLaunchAttribute attr[1];
+      attr[0].id = cudaLaunchAttributeClusterDimension;
+      attr[0].val.clusterDim.x = parts;
+      attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+      cudaLaunchConfig_t cfg = {};
+      cfg.gridDim = dim3(parts);
+      cfg.blockDim = F16_THREADS;
+      cfg.dynamicSmemBytes = f16_smem(QT);
+      cfg.attrs = attr;
+      cfg.numAttrs = 1;
+      if (cudaOccupancyMaxActiveClusters(&n, gemm_f16_kernel<QT>, &cfg) != cudaSuccess || n <= 0) {
+        (void)cudaGetLastError();
+        n = -1;
+      }
+      fit[dev][i].store(n, std::memory_order_relaxed);
+    }
+    if (tiles <= n && k_stages >= 4 * parts)
+      return parts;
+  }
+  return 1;
 }
 
 } // namespace
@@ -664,6 +777,22 @@ int launch_gemm_f16(int qtype, unsigned M, unsigned N, unsigned K, const float *
   const int c_vec4 = (ldc % 4 == 0) && !(reinterpret_cast<uintptr_t>(C) & 15);
   dim3 grid((mtiles + 1) / 2, (N + F16_TILE_N - 1) / F16_TILE_N);
   const int n_stages = (int)(K / F16_KS);
+  const int pairs = (int)(grid.x * grid.y);
+  const int parts = qtype == NNTR_Q4_K   ? k_parts<NNTR_Q4_K>(pairs, n_stages)
+                    : qtype == NNTR_Q6_K ? k_parts<NNTR_Q6_K>(pairs, n_stages)
+                                         : k_parts<NNTR_Q4_0>(pairs, n_stages);
+  // tiles one by one if they run in the same wave as the pairs: 128 instead of 256 columns of MMAs per stage and one sum at the
+  // end instead of two (256 x 1280 x 2560 Q4_0: 24 -> 16 us)
+  int tiles_per_cta = 2;
+  if (parts > 1 && mtiles > 1) {
+    const int tiles = mtiles * (int)grid.y;
+    if (parts == (qtype == NNTR_Q4_K   ? k_parts<NNTR_Q4_K>(tiles, n_stages)
+                  : qtype == NNTR_Q6_K ? k_parts<NNTR_Q6_K>(tiles, n_stages)
+                                       : k_parts<NNTR_Q4_0>(tiles, n_stages))) {
+      tiles_per_cta = 1;
+      grid.x = mtiles;
+    }
+  }
   const uint8_t *tiles = static_cast<const uint8_t *>(ws), *W = static_cast<const uint8_t *>(B);
   CUtensorMap wmap = {};
   if (qtype != NNTR_Q6_K) { // rows of 8-row groups of packed weights
@@ -685,19 +814,19 @@ int launch_gemm_f16(int qtype, unsigned M, unsigned N, unsigned K, const float *
     count_launch();
     NNTR_CHECK_CUDA(cudaGetLastError());
     if (qtype == NNTR_Q4_K)
-      NNTR_CHECK_CUDA(launch_after(gemm_f16_kernel<NNTR_Q4_K>, grid, f16_smem(NNTR_Q4_K), st, wmap, tiles, W, C, (int)ldc, (int)M, (int)N,
-                                   n_stages, mtiles, c_vec4));
+      NNTR_CHECK_CUDA(launch_after(gemm_f16_kernel<NNTR_Q4_K>, grid, parts, f16_smem(NNTR_Q4_K), st, wmap, tiles, W, C, (int)ldc,
+                                   (int)M, (int)N, n_stages, mtiles, tiles_per_cta, c_vec4));
     else
-      NNTR_CHECK_CUDA(launch_after(gemm_f16_kernel<NNTR_Q6_K>, grid, f16_smem(NNTR_Q6_K), st, wmap, tiles, W, C, (int)ldc, (int)M, (int)N,
-                                   n_stages, mtiles, c_vec4));
+      NNTR_CHECK_CUDA(launch_after(gemm_f16_kernel<NNTR_Q6_K>, grid, parts, f16_smem(NNTR_Q6_K), st, wmap, tiles, W, C, (int)ldc,
+                                   (int)M, (int)N, n_stages, mtiles, tiles_per_cta, c_vec4));
   } else {
     const int64_t nwarps = (int64_t)Mpad * ((K + 255) / 256);
     quantize_q8_0_f16_tiles_kernel<<<(unsigned)((nwarps + 7) / 8), 256, 0, st>>>(A, K, static_cast<uint8_t *>(ws), (int)M,
                                                                                Mpad, (int)K);
     count_launch();
     NNTR_CHECK_CUDA(cudaGetLastError());
-    NNTR_CHECK_CUDA(launch_after(gemm_f16_kernel<NNTR_Q4_0>, grid, f16_smem(NNTR_Q4_0), st, wmap, tiles, W, C, (int)ldc, (int)M, (int)N,
-                                   n_stages, mtiles, c_vec4));
+    NNTR_CHECK_CUDA(launch_after(gemm_f16_kernel<NNTR_Q4_0>, grid, parts, f16_smem(NNTR_Q4_0), st, wmap, tiles, W, C, (int)ldc,
+                                   (int)M, (int)N, n_stages, mtiles, tiles_per_cta, c_vec4));
   }
   count_launch();
   return check_cuda(cudaGetLastError(), "gemm fp16 tensor-path launch");

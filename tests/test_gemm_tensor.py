@@ -196,7 +196,8 @@ def test_fp16_tensor_gemm_q6_K_matches_checker(be, port, M, N, K):
 def test_fp16_tensor_gemm_every_tile_sees_the_same_weights(be, q, K):
     """A stage's expanded weights meet one or two tiles of 128 rows, and the stages ahead of the MMAs run differently far
     in the two cases; a row's sum does not depend on it, so the calls agree bit for bit, repeatedly. One stage, an odd
-    count, many. An odd row stride of C takes the scalar stores."""
+    count, many (K in four parts whose sums are added across a cluster, uneven for 45 stages). An odd row stride of C takes
+    the scalar stores."""
     gen = {"q4_0": O.random_q4_0x8, "q4_K": O.random_q4_Kx8}[q]
     rng = np.random.default_rng(K)
     N = 20 * 256
