@@ -1,0 +1,95 @@
+// SPDX-License-Identifier: Apache-2.0
+/**
+ * @file  cluster.cuh
+ * @brief One-dimensional clusters of CTAs that share a tile of a GEMM: each takes a part of K, and the sums meet through
+ *        distributed shared memory.
+ */
+#ifndef NNTR_CLUSTER_CUH_
+#define NNTR_CLUSTER_CUH_
+
+#include <atomic>
+
+#include "common.cuh"
+
+namespace nntr {
+
+/* the size is 1 without the launch attribute */
+__device__ __forceinline__ int cluster_size() {
+  uint32_t n;
+  asm("mov.u32 %0, %%cluster_nctaid.x;" : "=r"(n));
+  return (int)n;
+}
+__device__ __forceinline__ int cluster_rank() {
+  uint32_t n;
+  asm("mov.u32 %0, %%cluster_ctarank;" : "=r"(n));
+  return (int)n;
+}
+__device__ __forceinline__ void cluster_sync() {
+  asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+  asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+/** four floats at a shared address (of this CTA's window) in the CTA of the given rank */
+__device__ __forceinline__ float4 ld_cluster4(uint32_t addr, int rank) {
+  uint32_t remote;
+  float4 v;
+  asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(remote) : "r"(addr), "r"(rank));
+  asm volatile("ld.shared::cluster.v4.f32 {%0,%1,%2,%3}, [%4];"
+               : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w)
+               : "r"(remote)
+               : "memory");
+  return v;
+}
+
+/** Launch of a grid of grid.x * parts by grid.y CTAs in clusters of `parts` CTAs along x. The grid may start while its
+ *  predecessor runs: the kernel calls pdl_wait() before it touches what that wrote. */
+template <typename... P, typename... A>
+cudaError_t launch_in_clusters(void (*kernel)(P...), dim3 grid, int parts, int threads, int smem, cudaStream_t st, A... args) {
+  cudaLaunchAttribute attr[2];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  attr[1].id = cudaLaunchAttributeClusterDimension;
+  attr[1].val.clusterDim.x = parts;
+  attr[1].val.clusterDim.y = attr[1].val.clusterDim.z = 1;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(grid.x * parts, grid.y);
+  cfg.blockDim = threads;
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = st;
+  cfg.attrs = attr;
+  cfg.numAttrs = parts > 1 ? 2 : 1;
+  return cudaLaunchKernelEx(&cfg, kernel, (P)args...);
+}
+
+/** Clusters of 2, 4 or 8 CTAs of one kernel that run at the same time, per device, asked for once. */
+struct ClusterFit {
+  std::atomic<int> n[64][3];
+
+  template <typename... P> int operator()(void (*kernel)(P...), int parts, int threads, int smem) {
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || dev >= 64)
+      return 0;
+    std::atomic<int> &slot = n[dev][parts == 2 ? 0 : parts == 4 ? 1 : 2];
+    int v = slot.load(std::memory_order_relaxed);
+    if (v == 0) {
+      cudaLaunchAttribute attr[1];
+      attr[0].id = cudaLaunchAttributeClusterDimension;
+      attr[0].val.clusterDim.x = parts;
+      attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+      cudaLaunchConfig_t cfg = {};
+      cfg.gridDim = dim3(parts);
+      cfg.blockDim = threads;
+      cfg.dynamicSmemBytes = smem;
+      cfg.attrs = attr;
+      cfg.numAttrs = 1;
+      if (cudaOccupancyMaxActiveClusters(&v, kernel, &cfg) != cudaSuccess || v <= 0) {
+        (void)cudaGetLastError();
+        v = -1;
+      }
+      slot.store(v, std::memory_order_relaxed);
+    }
+    return v;
+  }
+};
+
+} // namespace nntr
+#endif

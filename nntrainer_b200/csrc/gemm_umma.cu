@@ -47,8 +47,11 @@
  * Cost model per CTA and super-block: 16 MMAs of 128x128x32 = 1024 tensor
  * cycles; the drain is ~12 instructions per output = ~1500 issue cycles, so
  * the kernel is bound by the drain's instruction issue, not by the tensor
- * pipe or by HBM (weights are read once per 128 activation rows).
+ * pipe or by HBM (weights are read once per 128 activation rows). With few
+ * tiles it is bound by the walk over K of one CTA, so a cluster shares a tile:
+ * 128 x 2560 x 2560 31.5 -> 15.8 us, 32 x 512 x 8192 77 -> 17.5.
  */
+#include "cluster.cuh"
 #include "common.cuh"
 #include "pipeline.cuh"
 
@@ -137,9 +140,11 @@ __device__ __forceinline__ void row_scales_half(const uint8_t *scales, int j, ui
   }
 }
 
+/* SHARED: a cluster of CTAs per tile (the plain kernel has no register to spare for it). */
+template <bool SHARED>
 __global__ void __maxnreg__(72)
 gemm_q4_K_umma_kernel(const uint8_t *__restrict__ atiles, const BlockQ4Kx8 *__restrict__ W, float *__restrict__ C,
-                      int ldc, int M, int nb, int c_vec4) {
+                      int ldc, int M, int k_blocks, int c_vec4) {
   extern __shared__ __align__(128) uint8_t smem[];
   uint64_t *bars = reinterpret_cast<uint64_t *>(smem + OFF_BARS);
   // bars: [0,1] full, [2,3] empty, [4,5] acc_full, [6,7] acc_empty, [8..11] meta_full, [12..15] head_full
@@ -147,7 +152,10 @@ gemm_q4_K_umma_kernel(const uint8_t *__restrict__ atiles, const BlockQ4Kx8 *__re
   volatile int *abort_flag = reinterpret_cast<volatile int *>(smem + OFF_BARS + 136);
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const int mt = blockIdx.x, nt = blockIdx.y;
+  // the CTAs of a cluster share a tile: each walks its part of K (super-blocks b0 .. b0 + nb - 1)
+  const int parts = SHARED ? cluster_size() : 1, part = SHARED ? cluster_rank() : 0;
+  const int mt = blockIdx.x / parts, nt = blockIdx.y;
+  const int b0 = SHARED ? k_blocks * part / parts : 0, nb = SHARED ? k_blocks * (part + 1) / parts - b0 : k_blocks;
   const uint32_t sbase = smem_u32(smem);
   const uint32_t bar0 = smem_u32(bars);
   auto BAR = [&](int i) { return bar0 + 8u * i; };
@@ -175,14 +183,16 @@ gemm_q4_K_umma_kernel(const uint8_t *__restrict__ atiles, const BlockQ4Kx8 *__re
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem = *tmem_slot;
+  constexpr int SUM_PITCH = TILE_N + 4; // floats
+  bool tile_done = false;               // drain warps of a shared tile: all sums in shared memory
 
   if (warp < PRODUCER_THREADS / 32) {
     /* ------------------------------ producers ------------------------------ */
     const int r = tid & (TILE_N - 1); // weight row inside the tile
     const int h = tid >> 7;           // which half of the row's super-block: sub-blocks 4h .. 4h+3
     const int j = r & 7;              // row inside its 8-row group
-    const BlockQ4Kx8 *wrow = W + (size_t)(nt * (TILE_N / 8) + (r >> 3)) * nb;
-    const uint8_t *asrc = atiles + (size_t)mt * nb * UMMA_ATILE_BYTES;
+    const BlockQ4Kx8 *wrow = W + (size_t)(nt * (TILE_N / 8) + (r >> 3)) * k_blocks + b0;
+    const uint8_t *asrc = atiles + ((size_t)mt * k_blocks + b0) * UMMA_ATILE_BYTES;
     /* The first 128 bytes of every block_q4_Kx8 (d, dmin, packed scales) travel two super-blocks ahead through a
      * ring of HEAD_SLOTS slots: thread t < 128 copies 16 bytes of group t/8. Every producer thread arrives on the
      * slot's barrier once per iteration, so a slot is rewritten only after all its readers have moved on. */
@@ -201,6 +211,8 @@ gemm_q4_K_umma_kernel(const uint8_t *__restrict__ atiles, const BlockQ4Kx8 *__re
 #pragma unroll
     for (int c = 0; c < 8; ++c)
       q[c] = ldg_stream_u2(wrow->qs + ((8 * h + c) * 8 + j) * 8);
+    if (tid == 0)
+      pdl_wait(); // the quantizer's tiles; the weights do not depend on the kernel before
     for (int b = 0; b < nb; ++b) {
       const int s = b & 1, u = b >> 1;
       fetch_head(b + 2);
@@ -334,7 +346,13 @@ gemm_q4_K_umma_kernel(const uint8_t *__restrict__ atiles, const BlockQ4Kx8 *__re
         mbar_arrive(BAR(6 + s));
     }
     const int row = mt * TILE_M + m;
-    if (ok && row < M) {
+    if (SHARED) { // the operand stages are free: every MMA of this CTA has retired
+      tile_done = ok;
+      float *sums = reinterpret_cast<float *>(smem) + m * SUM_PITCH + cgrp * DRAIN_COLS;
+#pragma unroll
+      for (int i = 0; i < DRAIN_COLS; i += 4)
+        *reinterpret_cast<float4 *>(sums + i) = make_float4(acc[i], acc[i + 1], acc[i + 2], acc[i + 3]);
+    } else if (ok && row < M) {
       float *dst = C + (size_t)row * ldc + nt * TILE_N + cgrp * DRAIN_COLS;
       if (c_vec4) {
 #pragma unroll
@@ -346,6 +364,37 @@ gemm_q4_K_umma_kernel(const uint8_t *__restrict__ atiles, const BlockQ4Kx8 *__re
           dst[i] = acc[i];
       }
     }
+  }
+
+  /* A shared tile: every CTA of the cluster holds its sums in its own shared memory; the rows are dealt out, and a CTA adds its
+   * rows' parts in the order of K. All threads pass both barriers, whatever went wrong before. */
+  if (SHARED) {
+    cluster_sync();
+    if (tile_done) {
+      const int rows = min(TILE_M, M - mt * TILE_M);
+      for (int i = tid - DRAIN_WARP0 * 32; part + (i >> 5) * parts < rows; i += DRAIN_WARPS * 32) {
+        const int r = part + (i >> 5) * parts, c = 4 * (i & 31);
+        float4 v[8];
+#pragma unroll
+        for (int k = 0; k < 8; ++k)
+          if (k < parts)
+            v[k] = ld_cluster4(sbase + 4u * (r * SUM_PITCH + c), k);
+#pragma unroll
+        for (int k = 1; k < 8; ++k)
+          if (k < parts)
+            v[0] = make_float4(v[0].x + v[k].x, v[0].y + v[k].y, v[0].z + v[k].z, v[0].w + v[k].w);
+        float *dst = C + (size_t)(mt * TILE_M + r) * ldc + nt * TILE_N + c;
+        if (c_vec4) {
+          *reinterpret_cast<float4 *>(dst) = v[0];
+        } else {
+          dst[0] = v[0].x;
+          dst[1] = v[0].y;
+          dst[2] = v[0].z;
+          dst[3] = v[0].w;
+        }
+      }
+    }
+    cluster_sync(); // nobody leaves while its sums are read
   }
 
   /* common tail: on an abort give copies and MMAs in flight time to land before the memory is released */
@@ -413,7 +462,8 @@ int launch_gemm_q4_K_umma(unsigned M, unsigned N, unsigned K, const float *A, co
   int dev = 0;
   NNTR_CHECK_CUDA(cudaGetDevice(&dev));
   if (dev < 64 && !attr_set[dev]) {
-    NNTR_CHECK_CUDA(cudaFuncSetAttribute(gemm_q4_K_umma_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES));
+    NNTR_CHECK_CUDA(cudaFuncSetAttribute(gemm_q4_K_umma_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES));
+    NNTR_CHECK_CUDA(cudaFuncSetAttribute(gemm_q4_K_umma_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES));
     attr_set[dev] = true;
   }
   const int nb = (int)(K / QK_K);
@@ -428,11 +478,20 @@ int launch_gemm_q4_K_umma(unsigned M, unsigned N, unsigned K, const float *A, co
   NNTR_CHECK_CUDA(cudaGetLastError());
   const int c_vec4 = (ldc % 4 == 0) && !(reinterpret_cast<uintptr_t>(C) & 15);
   dim3 grid(mtiles, N / TILE_N);
-  gemm_q4_K_umma_kernel<<<grid, CTA_THREADS, SMEM_BYTES, st>>>(static_cast<const uint8_t *>(ws),
-                                                               static_cast<const BlockQ4Kx8 *>(B), C, (int)ldc, (int)M,
-                                                               nb, c_vec4);
+  // Few tiles: K in as many parts as run in one wave of clusters. A CTA alone walks K at 2.5 us a super-block however many SMs
+  // are idle; the parts' sums cost about 2 us at the end. Two parts only for calls of one tile of rows: beyond that, from 35
+  // tiles on, a row's sum does not depend on how many rows the call has.
+  static ClusterFit fit;
+  int parts = 8;
+  while (parts > 1 && (nb < parts || (int)(grid.x * grid.y) > fit(gemm_q4_K_umma_kernel<true>, parts, CTA_THREADS, SMEM_BYTES)))
+    parts /= 2;
+  if (parts == 2 && mtiles > 1)
+    parts = 1;
+  const cudaError_t e = launch_in_clusters(parts > 1 ? gemm_q4_K_umma_kernel<true> : gemm_q4_K_umma_kernel<false>, grid, parts, CTA_THREADS, SMEM_BYTES, st,
+                                           static_cast<const uint8_t *>(ws), static_cast<const BlockQ4Kx8 *>(B), C, (int)ldc,
+                                           (int)M, nb, c_vec4);
   count_launch();
-  return check_cuda(cudaGetLastError(), "gemm_q4_K tensor-path launch");
+  return check_cuda(e, "gemm_q4_K tensor-path launch");
 }
 
 int read_umma_status(int *out) {

@@ -55,13 +55,12 @@
  * through distributed shared memory. 512 x 1280 x 2560: Q4_0 40 -> 25 us, Q6_K 69 -> 33; 128 x 2560 x 8192: Q4_0 93 -> 25,
  * Q6_K 268 -> 49.
  */
+#include "cluster.cuh"
 #include "common.cuh"
 #include "pipeline.cuh"
 #include "tma_map.cuh"
 
 #include <cuda_fp16.h>
-
-#include <atomic>
 
 namespace nntr {
 
@@ -109,31 +108,6 @@ __device__ __forceinline__ void umma_f16(uint32_t tmem_d, uint64_t da, uint64_t 
                "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}" ::"r"(tmem_d),
                "l"(da), "l"(db), "r"(idesc), "r"(accumulate)
                : "memory");
-}
-__device__ __forceinline__ int cluster_size() {
-  uint32_t n;
-  asm("mov.u32 %0, %%cluster_nctaid.x;" : "=r"(n));
-  return (int)n;
-}
-__device__ __forceinline__ int cluster_rank() {
-  uint32_t n;
-  asm("mov.u32 %0, %%cluster_ctarank;" : "=r"(n));
-  return (int)n;
-}
-__device__ __forceinline__ void cluster_sync() {
-  asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
-  asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
-}
-/** four floats at a shared address (of this CTA's window) in the CTA of the given rank */
-__device__ __forceinline__ float4 ld_cluster4(uint32_t addr, int rank) {
-  uint32_t remote;
-  float4 v;
-  asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(remote) : "r"(addr), "r"(rank));
-  asm volatile("ld.shared::cluster.v4.f32 {%0,%1,%2,%3}, [%4];"
-               : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w)
-               : "r"(remote)
-               : "memory");
-  return v;
 }
 __device__ __forceinline__ void umma_commit(uint32_t bar) {
   asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar) : "memory");
@@ -690,57 +664,14 @@ quantize_q8_0_f16_tiles_kernel(const float *__restrict__ x, int64_t ldx, uint8_t
   }
 }
 
-/** The GEMM behind its quantizer, started while that runs: barriers, tensor memory and the first packed weights are ready
- *  when the activation tiles are (pdl_wait of the copy warp). Clusters of `parts` CTAs. */
-template <typename... P, typename... A>
-cudaError_t launch_after(void (*kernel)(P...), dim3 grid, int parts, int smem, cudaStream_t st, A... args) {
-  cudaLaunchAttribute attr[2];
-  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  attr[0].val.programmaticStreamSerializationAllowed = 1;
-  attr[1].id = cudaLaunchAttributeClusterDimension;
-  attr[1].val.clusterDim.x = parts;
-  attr[1].val.clusterDim.y = attr[1].val.clusterDim.z = 1;
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(grid.x * parts, grid.y);
-  cfg.blockDim = F16_THREADS;
-  cfg.dynamicSmemBytes = smem;
-  cfg.stream = st;
-  cfg.attrs = attr;
-  cfg.numAttrs = parts > 1 ? 2 : 1;
-  return cudaLaunchKernelEx(&cfg, kernel, (P)args...);
-}
-
 /** Into how many parts K is cut, so that few tiles still use the machine. A CTA alone walks K at 0.9 us (Q6_K 1.5) a stage
  *  however many SMs are idle; the parts' sums cost about 2 us at the end. As many as still run in one wave of clusters, of at
  *  least four stages each. */
 template <int QT> int k_parts(int tiles, int k_stages) {
-  static std::atomic<int> fit[64][3];
-  int dev = 0;
-  if (cudaGetDevice(&dev) != cudaSuccess || dev >= 64)
-    return 1;
-  for (int i = 2; i >= 0; --i) {
-    const int parts = 2 << i;
-    int n = fit[dev][i].load(std::memory_order_relaxed);
-    if (n == 0) { // clusters of that size that run at the same time
-      cudaLaunchAttribute attr[1];
-      attr[0].id = cudaLaunchAttributeClusterDimension;
-      attr[0].val.clusterDim.x = parts;
-      attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
-      cudaLaunchConfig_t cfg = {};
-      cfg.gridDim = dim3(parts);
-      cfg.blockDim = F16_THREADS;
-      cfg.dynamicSmemBytes = f16_smem(QT);
-      cfg.attrs = attr;
-      cfg.numAttrs = 1;
-      if (cudaOccupancyMaxActiveClusters(&n, gemm_f16_kernel<QT>, &cfg) != cudaSuccess || n <= 0) {
-        (void)cudaGetLastError();
-        n = -1;
-      }
-      fit[dev][i].store(n, std::memory_order_relaxed);
-    }
-    if (tiles <= n && k_stages >= 4 * parts)
+  static ClusterFit fit;
+  for (int parts = 8; parts > 1; parts /= 2)
+    if (k_stages >= 4 * parts && tiles <= fit(gemm_f16_kernel<QT>, parts, F16_THREADS, f16_smem(QT)))
       return parts;
-  }
   return 1;
 }
 
@@ -814,19 +745,19 @@ int launch_gemm_f16(int qtype, unsigned M, unsigned N, unsigned K, const float *
     count_launch();
     NNTR_CHECK_CUDA(cudaGetLastError());
     if (qtype == NNTR_Q4_K)
-      NNTR_CHECK_CUDA(launch_after(gemm_f16_kernel<NNTR_Q4_K>, grid, parts, f16_smem(NNTR_Q4_K), st, wmap, tiles, W, C, (int)ldc,
-                                   (int)M, (int)N, n_stages, mtiles, tiles_per_cta, c_vec4));
+      NNTR_CHECK_CUDA(launch_in_clusters(gemm_f16_kernel<NNTR_Q4_K>, grid, parts, F16_THREADS, f16_smem(NNTR_Q4_K), st, wmap, tiles, W,
+                                         C, (int)ldc, (int)M, (int)N, n_stages, mtiles, tiles_per_cta, c_vec4));
     else
-      NNTR_CHECK_CUDA(launch_after(gemm_f16_kernel<NNTR_Q6_K>, grid, parts, f16_smem(NNTR_Q6_K), st, wmap, tiles, W, C, (int)ldc,
-                                   (int)M, (int)N, n_stages, mtiles, tiles_per_cta, c_vec4));
+      NNTR_CHECK_CUDA(launch_in_clusters(gemm_f16_kernel<NNTR_Q6_K>, grid, parts, F16_THREADS, f16_smem(NNTR_Q6_K), st, wmap, tiles, W,
+                                         C, (int)ldc, (int)M, (int)N, n_stages, mtiles, tiles_per_cta, c_vec4));
   } else {
     const int64_t nwarps = (int64_t)Mpad * ((K + 255) / 256);
     quantize_q8_0_f16_tiles_kernel<<<(unsigned)((nwarps + 7) / 8), 256, 0, st>>>(A, K, static_cast<uint8_t *>(ws), (int)M,
                                                                                Mpad, (int)K);
     count_launch();
     NNTR_CHECK_CUDA(cudaGetLastError());
-    NNTR_CHECK_CUDA(launch_after(gemm_f16_kernel<NNTR_Q4_0>, grid, parts, f16_smem(NNTR_Q4_0), st, wmap, tiles, W, C, (int)ldc,
-                                   (int)M, (int)N, n_stages, mtiles, tiles_per_cta, c_vec4));
+    NNTR_CHECK_CUDA(launch_in_clusters(gemm_f16_kernel<NNTR_Q4_0>, grid, parts, F16_THREADS, f16_smem(NNTR_Q4_0), st, wmap, tiles, W,
+                                         C, (int)ldc, (int)M, (int)N, n_stages, mtiles, tiles_per_cta, c_vec4));
   }
   count_launch();
   return check_cuda(cudaGetLastError(), "gemm fp16 tensor-path launch");

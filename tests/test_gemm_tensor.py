@@ -61,6 +61,19 @@ def test_tensor_gemm_matches_checker_and_exact_path(be, port, M, N, K):
     assert max_rel(got, exact) <= 2e-6, "integer sums are exact on both paths: only fp32 rounding may differ"
 
 
+@pytest.mark.parametrize("M,N,K,ldc", [(32, 128, 1024, 128), (129, 256, 2560, 259), (64, 1280, 2304, 1280), (40, 5120, 768, 5120)])
+def test_tensor_gemm_with_k_in_parts(be, M, N, K, ldc):
+    """Few tiles: eight, four or two CTAs share a tile (even and uneven shares of the super-blocks, rows that do not divide by
+    the parts). The integers are exact; each fp32 chain is at most K/256 + 8 roundings of 2^-24, relative to sums no larger
+    than a few times the largest result."""
+    rng = np.random.default_rng(M + N)
+    A, B = torch.from_numpy(acts(rng, M, K)).cuda(), torch.from_numpy(O.random_q4_Kx8(rng, N, K)).cuda()
+    got = run(be, "tensor", M, N, K, A, B, ldc=ldc)
+    assert np.isnan(got[:, N:]).all()
+    assert max_rel(got[:, :N], run(be, "exact", M, N, K, A, B)) <= 2e-6
+    assert np.array_equal(got.view(np.uint32), run(be, "tensor", M, N, K, A, B, ldc=ldc).view(np.uint32))
+
+
 def test_tensor_gemm_writes_rows_with_stride_ldc_and_leaves_padding(be, port):
     rng = np.random.default_rng(5)
     M, N, K, ldc = 40, 128, 512, 160
