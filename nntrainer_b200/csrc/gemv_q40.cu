@@ -24,10 +24,20 @@
  *                dependency resolves).
  *   warps 0-15   consumers: quantize x to Q8_0 into shared memory (32 values
  *                per block 16-byte aligned, scales converted to fp32 beside
- *                them), then take whole row groups: 32 blocks at a time, lane =
- *                block, eight (I_b, scale) pairs per lane into a per-warp
- *                scratch; lanes 0-7 then run the eight rows' fma chains over
- *                those 32 blocks in order, carrying the sums to the next 32.
+ *                them), then passes of 32 blocks of a row group, dealt to the
+ *                warps one by one: lane = block, eight records (I_b, fp16 d_w;
+ *                |I_b| <= 32 * 8 * 127 fits 16 bits) per lane into the area of
+ *                the batch of row groups.
+ *   warps 17-18  chains: a batch of up to eight row groups, a thread per row,
+ *                eight blocks of the ordered fma chain at a time while the
+ *                consumers are at the next batch (two areas).
+ * A CTA's share of a layer is a few row groups: with a warp per row group most
+ * of the 16 warps had nothing to do, and every pass waited for its chain.
+ * What bounded it before that: the producer thread's divisions (stage -> slot,
+ * row group), 150 clocks each and three per 9 KB stage: 20 bytes/ns per SM.
+ * 2880 x 2880 6.0 -> 4.8 us, 23680 x 2880 19.1 -> 11.5 (3.3 TB/s), eight experts
+ * of 2880 x 2880 18 -> 8; what is left for small layers is launch, the round trip
+ * of x and the 90-block chain, for wide ones the instructions of the dots.
  * Algorithmic bytes per launch: N * K/32 * 18 (weights) + 4K (x) + 4N (y).
  */
 #include "common.cuh"
@@ -39,7 +49,10 @@ namespace {
 
 constexpr int Q40_CONSUMER_WARPS = 16;
 constexpr int Q40_PRODUCER_WARP = 16;
-constexpr int Q40_THREADS = 17 * 32;
+constexpr int Q40_CHAIN_WARP0 = 17;
+constexpr int Q40_CHAIN_WARPS = 2;
+constexpr int Q40_THREADS = (Q40_CHAIN_WARP0 + Q40_CHAIN_WARPS) * 32;
+constexpr int Q40_HANDOVER = (Q40_CONSUMER_WARPS + Q40_CHAIN_WARPS) * 32; // threads of the barriers between the two
 constexpr int Q40_MAX_STAGES = 24;
 constexpr int Q40_STAGE_UNITS = 64; // blocks of one row group per stage (9216 bytes)
 constexpr uint32_t Q40_WAIT_POLLS = 1u << 22;
@@ -70,6 +83,11 @@ __device__ __forceinline__ bool wait_armed(volatile int *armed, int t, volatile 
   return false;
 }
 
+/** row groups per batch: two areas of records of at most 48 KB, a thread of the chain warps per row */
+__host__ __device__ inline int q40_batch(int nu) {
+  const int gb = 24 * 1024 / (nu * 32), most = Q40_CHAIN_WARPS * 32 / 8;
+  return gb < 1 ? 1 : gb > most ? most : gb;
+}
 struct Q40Layout {
   uint32_t actq, actd, rec, ring, bars, total;
 };
@@ -78,11 +96,10 @@ __host__ __device__ inline Q40Layout q40_layout(int nu, int stage_bytes, int n_s
   uint32_t o = 0;
   L.actq = o; // nu x 32 quantized activations
   o += (uint32_t)nu * 32;
-  L.actd = o; // nu fp32 scales
-  o += (uint32_t)nu * 4;
-  o = (o + 15u) & ~15u;
-  L.rec = o; // per consumer warp: 32 blocks x 8 rows x (I, scale)
-  o += (uint32_t)Q40_CONSUMER_WARPS * 32 * 64;
+  L.actd = o; // nu fp32 scales (read in eights)
+  o += (uint32_t)((nu + 7) / 8) * 32;
+  L.rec = o; // two batches of row groups: nu blocks x 8 rows x (I, d_w)
+  o += 2u * (uint32_t)q40_batch(nu) * (uint32_t)nu * 32;
   o = (o + 127u) & ~127u;
   L.ring = o;
   o += (uint32_t)n_stages * stage_bytes;
@@ -90,6 +107,15 @@ __host__ __device__ inline Q40Layout q40_layout(int nu, int stage_bytes, int n_s
   o += 2 * Q40_MAX_STAGES * 8 + 16;
   L.total = o;
   return L;
+}
+
+/* the areas of the batches change hands at named barriers 2, 3 (records complete) and 4, 5 (records read) */
+__device__ __forceinline__ void handover_arrive(int bar) {
+  __threadfence_block();
+  asm volatile("bar.arrive %0, %1;" ::"r"(bar), "n"(Q40_HANDOVER) : "memory");
+}
+__device__ __forceinline__ void handover_wait(int bar) {
+  asm volatile("bar.sync %0, %1;" ::"r"(bar), "n"(Q40_HANDOVER) : "memory");
 }
 
 /** 16 * (signed nibble) dot products of one word of 8 nibbles with the activations of its low and high nibbles */
@@ -124,7 +150,7 @@ gemv_q4_0_kernel(const float *__restrict__ x, const uint8_t *__restrict__ W, flo
   const uint32_t sm0 = smem_u32(smem);
   const uint32_t bar0 = sm0 + L.bars;
   auto FULL_BAR = [&](int s) { return bar0 + 8u * s; };                    // stage bytes landed
-  auto FREE_BAR = [&](int s) { return bar0 + 8u * (Q40_MAX_STAGES + s); }; // its consumer warp is done with it
+  auto FREE_BAR = [&](int s) { return bar0 + 8u * (Q40_MAX_STAGES + s); }; // its passes are done with it
   volatile int *abort_flag = reinterpret_cast<volatile int *>(smem + L.bars + 2 * Q40_MAX_STAGES * 8);
   // Number of stages the producer has armed so far. A consumer may be more than a ring ahead of the producer; a parity
   // wait on a slot that is still two uses behind would succeed at once, so a consumer first waits (bounded) until its
@@ -135,11 +161,13 @@ gemv_q4_0_kernel(const float *__restrict__ x, const uint8_t *__restrict__ W, flo
   const int g_lo = (int)((long long)n_groups * blockIdx.x / gridDim.x);
   const int g_hi = (int)((long long)n_groups * (blockIdx.x + 1) / gridDim.x);
   const int my_groups = g_hi - g_lo, my_stages = my_groups * parts;
+  const int gb = q40_batch(nu), batches = (my_groups + gb - 1) / gb; // row groups whose records are pending at a time
+  const int ppg = (nu + 31) / 32;                                    // passes per row group
 
   if (tid == 0) {
     for (int s = 0; s < n_ring; ++s) {
       mbar_init(FULL_BAR(s), 1);
-      mbar_init(FREE_BAR(s), 1);
+      mbar_init(FREE_BAR(s), 2); // a stage is two passes (a short one arrives twice)
     }
     *abort_flag = 0;
     *armed = 0;
@@ -150,32 +178,30 @@ gemv_q4_0_kernel(const float *__restrict__ x, const uint8_t *__restrict__ W, flo
 
   if (warp == Q40_PRODUCER_WARP) {
     if (lane == 0) {
-      const uint8_t *src = W + (size_t)g_lo * group_bytes;
+      const uint8_t *src = W + (size_t)g_lo * group_bytes; // the share's stages follow one another
+      int s = 0, use = 0, p = 0;                            // ring slot, its use, stage inside the row group
       for (int t = 0; t < my_stages; ++t) {
-        const int s = t % n_ring, use = t / n_ring;
         if (use > 0 && !mbar_wait(FREE_BAR(s), (use - 1) & 1, abort_flag))
           break;
-        const int g = t / parts, p = t - g * parts;
-        const int units = nu - p * Q40_STAGE_UNITS < Q40_STAGE_UNITS ? nu - p * Q40_STAGE_UNITS : Q40_STAGE_UNITS;
-        const uint32_t bytes = (uint32_t)units * (uint32_t)sizeof(BlockQ40x8);
+        const int left = nu - p * Q40_STAGE_UNITS;
+        const uint32_t bytes = (uint32_t)(left < Q40_STAGE_UNITS ? left : Q40_STAGE_UNITS) * (uint32_t)sizeof(BlockQ40x8);
         mbar_expect_tx(FULL_BAR(s), bytes);
-        bulk_g2s(sm0 + L.ring + (uint32_t)s * (uint32_t)stage_bytes,
-                 src + (size_t)g * group_bytes + (size_t)p * stage_bytes, bytes, FULL_BAR(s));
+        bulk_g2s(sm0 + L.ring + (uint32_t)s * (uint32_t)stage_bytes, src, bytes, FULL_BAR(s));
         __threadfence_block();
         *armed = t + 1;
+        src += bytes;
+        if (++p == parts)
+          p = 0;
+        if (++s == n_ring) {
+          s = 0;
+          ++use;
+        }
       }
     }
     __syncwarp();
-  } else {
-    /* ---- consumers: quantize x (256 elements per warp pass, masked beyond K), then whole row groups ---- */
+  } else if (warp < Q40_CONSUMER_WARPS) {
+    /* ---- consumers: quantize x (256 elements per warp pass, masked beyond K), then passes of 32 blocks ---- */
     pdl_wait();
-    uint32_t tag = 0;
-    unsigned long long ex_off = 0;
-    if (PUBLISH) {
-      const unsigned long long seq = (*ex.epoch - 1) * ex.layers_per_epoch + ex.layer + 1;
-      tag = (uint32_t)seq;
-      ex_off = (unsigned long long)blockIdx.y * (unsigned long long)batch.y_stride + (seq & 1) * ex.parity_stride;
-    }
     for (int u8 = warp; u8 * 256 < K; u8 += Q40_CONSUMER_WARPS) {
       const int e0 = u8 * 256 + lane * 8;
       const bool valid = e0 < K;
@@ -193,68 +219,100 @@ gemv_q4_0_kernel(const float *__restrict__ x, const uint8_t *__restrict__ W, flo
     }
     asm volatile("bar.sync 1, %0;" ::"n"(Q40_CONSUMER_WARPS * 32) : "memory");
 
-    const uint32_t myrec = sm0 + L.rec + (uint32_t)((warp * 32 + lane) * 64);
-    const uint32_t chain_rec = sm0 + L.rec + (uint32_t)(warp * 32 * 64) + 8 * (lane & 7);
-    for (int i = warp; i < my_groups; i += Q40_CONSUMER_WARPS) { // row group i of the share: stages i*parts ..
-      float acc = 0.f; // lanes 0-7: the running sum of row `lane`
-      bool ok = true;
-      for (int p = 0; p < parts && ok; ++p) {
-        const int t = i * parts + p, s = t % n_ring, use = t / n_ring;
-        if (!wait_armed(armed, t, abort_flag) || !mbar_wait(FULL_BAR(s), use & 1, abort_flag)) {
-          ok = false;
+    const FastDiv by_ppg(ppg), by_ring(n_ring);
+    bool ok = true; // after a wait that ran out the warp only keeps the handover going
+    for (int bt = 0; bt < batches; ++bt) {
+      const int buf = bt & 1, g0 = bt * gb, ng = my_groups - g0 < gb ? my_groups - g0 : gb;
+      if (bt >= 2)
+        handover_wait(4 + buf); // the chains of batch bt - 2 have read the area
+      for (int pass = warp; pass < ng * ppg && ok; pass += Q40_CONSUMER_WARPS) {
+        const int gi = by_ppg.div(pass), c = by_ppg.mod(pass, gi); // blocks 32 c .. of row group g0 + gi
+        const int t = (g0 + gi) * parts + (c >> 1), use = by_ring.div(t), s = by_ring.mod(t, use);
+        ok = wait_armed(armed, t, abort_flag) && mbar_wait(FULL_BAR(s), use & 1, abort_flag);
+        ok = __all_sync(FULL, ok);
+        if (!ok)
           break;
-        }
-        const uint32_t stage = sm0 + L.ring + (uint32_t)s * (uint32_t)stage_bytes;
-        const int ub = p * Q40_STAGE_UNITS; // first block of the row group held by this stage
+        const int ub = (c >> 1) * Q40_STAGE_UNITS; // first block of the row group held by the stage
         const int units = nu - ub < Q40_STAGE_UNITS ? nu - ub : Q40_STAGE_UNITS;
-        for (int u0 = 0; u0 < units; u0 += 32) {
-          const int u = u0 + lane;
-          if (u < units) {
-            const uint32_t blk = stage + (uint32_t)u * 144u;
-            const uint32_t aq = sm0 + L.actq + (uint32_t)(ub + u) * 32u;
-            const uint4 dh = lds128(blk); // eight fp16 scales
-            const uint4 a0 = lds128(aq), a1 = lds128(aq + 16u);
-            const float da = __uint_as_float(lds32(sm0 + L.actd + (uint32_t)(ub + u) * 4u));
-            const uint32_t dwords[4] = {dh.x, dh.y, dh.z, dh.w};
+        const int u = (c & 1) * 32 + lane;
+        if (u < units) {
+          const uint32_t blk = sm0 + L.ring + (uint32_t)s * (uint32_t)stage_bytes + (uint32_t)u * 144u;
+          const uint32_t aq = sm0 + L.actq + (uint32_t)(ub + u) * 32u;
+          const uint4 dh = lds128(blk); // eight fp16 scales
+          const uint4 a0 = lds128(aq), a1 = lds128(aq + 16u);
+          const uint32_t dwords[4] = {dh.x, dh.y, dh.z, dh.w};
+          uint32_t rec[8];
 #pragma unroll
-            for (int rp = 0; rp < 4; ++rp) { // rows 2rp, 2rp+1 share each 16-byte load
-              const uint4 qa = lds128(blk + 16 + 16 * rp);      // elements 0-7 (low nibbles), 16-23 (high) of both rows
-              const uint4 qb = lds128(blk + 16 + 64 + 16 * rp); // elements 8-15 (low), 24-31 (high)
-              int i0 = dot8(qa.x, a0.x, a1.x, 0);
-              i0 = dot8(qa.y, a0.y, a1.y, i0);
-              i0 = dot8(qb.x, a0.z, a1.z, i0);
-              i0 = dot8(qb.y, a0.w, a1.w, i0);
-              int i1 = dot8(qa.z, a0.x, a1.x, 0);
-              i1 = dot8(qa.w, a0.y, a1.y, i1);
-              i1 = dot8(qb.z, a0.z, a1.z, i1);
-              i1 = dot8(qb.w, a0.w, a1.w, i1);
-              const float d0 = __fmul_rn(half_bits_to_float((uint16_t)(dwords[rp] & 0xffffu)), da);
-              const float d1 = __fmul_rn(half_bits_to_float((uint16_t)(dwords[rp] >> 16)), da);
-              sts64(myrec + 16 * rp, (uint32_t)(i0 >> 4), __float_as_uint(d0));
-              sts64(myrec + 16 * rp + 8, (uint32_t)(i1 >> 4), __float_as_uint(d1));
-            }
+          for (int rp = 0; rp < 4; ++rp) { // rows 2rp, 2rp+1 share each 16-byte load
+            const uint4 qa = lds128(blk + 16 + 16 * rp);      // elements 0-7 (low nibbles), 16-23 (high) of both rows
+            const uint4 qb = lds128(blk + 16 + 64 + 16 * rp); // elements 8-15 (low), 24-31 (high)
+            int i0 = dot8(qa.x, a0.x, a1.x, 0);
+            i0 = dot8(qa.y, a0.y, a1.y, i0);
+            i0 = dot8(qb.x, a0.z, a1.z, i0);
+            i0 = dot8(qb.y, a0.w, a1.w, i0);
+            int i1 = dot8(qa.z, a0.x, a1.x, 0);
+            i1 = dot8(qa.w, a0.y, a1.y, i1);
+            i1 = dot8(qb.z, a0.z, a1.z, i1);
+            i1 = dot8(qb.w, a0.w, a1.w, i1);
+            rec[2 * rp] = __byte_perm((uint32_t)(i0 >> 4), dwords[rp], 0x5410);     // I | d_w << 16
+            rec[2 * rp + 1] = __byte_perm((uint32_t)(i1 >> 4), dwords[rp], 0x7610);
           }
-          __syncwarp();
-          if (lane < 8) {
-            const int n = units - u0 < 32 ? units - u0 : 32;
-            for (int k0 = 0; k0 < n; k0 += 8) { // eight pairs fetched together, then joined to the chain in order
-              uint2 pr[8];
-#pragma unroll
-              for (int k = 0; k < 8; ++k)
-                pr[k] = lds64(chain_rec + (uint32_t)((k0 + k < n ? k0 + k : n - 1) * 64));
-#pragma unroll
-              for (int k = 0; k < 8; ++k)
-                if (k0 + k < n)
-                  acc = __fmaf_rn((float)(int)pr[k].x, __uint_as_float(pr[k].y), acc);
-            }
-          }
-          __syncwarp(); // the scratch is rewritten by the next 32 blocks
+          const uint32_t to = sm0 + L.rec + (uint32_t)((buf * gb + gi) * nu + ub + u) * 32u;
+          sts128(to, rec[0], rec[1], rec[2], rec[3]);
+          sts128(to + 16, rec[4], rec[5], rec[6], rec[7]);
         }
-        if (lane == 0)
+        __syncwarp();
+        if (lane == 0) {
           mbar_arrive(FREE_BAR(s));
+          if (units <= 32)
+            mbar_arrive(FREE_BAR(s));
+        }
       }
-      if (ok && lane < 8) {
-        const size_t o = (size_t)(g_lo + i) * 8 + lane;
+      handover_arrive(2 + buf);
+    }
+  } else {
+    /* ---- chains: a thread per row of the batch ---- */
+    pdl_wait(); // y may still be read by the previous kernel
+    uint32_t tag = 0;
+    unsigned long long ex_off = 0;
+    if (PUBLISH) {
+      const unsigned long long seq = (*ex.epoch - 1) * ex.layers_per_epoch + ex.layer + 1;
+      tag = (uint32_t)seq;
+      ex_off = (unsigned long long)blockIdx.y * (unsigned long long)batch.y_stride + (seq & 1) * ex.parity_stride;
+    }
+    const int gi = (warp - Q40_CHAIN_WARP0) * 4 + (lane >> 3), r = lane & 7;
+    for (int bt = 0; bt < batches; ++bt) {
+      const int buf = bt & 1, g0 = bt * gb, ng = my_groups - g0 < gb ? my_groups - g0 : gb;
+      handover_wait(2 + buf);
+      if (gi < ng && !*abort_flag) {
+        const uint32_t rec = sm0 + L.rec + (uint32_t)((buf * gb + gi) * nu) * 32u + 4u * r, ad = sm0 + L.actd;
+        float acc = 0.f;
+        uint32_t w[8];
+        uint4 d0, d1;
+        auto fetch = [&](int k0) { // the next eight travel while these are added (past the end: the last block again)
+#pragma unroll
+          for (int k = 0; k < 8; ++k)
+            w[k] = lds32(rec + (uint32_t)(k0 + k < nu ? k0 + k : nu - 1) * 32u);
+          d0 = lds128(ad + 4u * k0);
+          d1 = lds128(ad + 4u * k0 + 16u);
+        };
+        fetch(0);
+        for (int k0 = 0; k0 < nu; k0 += 8) {
+          const uint32_t dv[8] = {d0.x, d0.y, d0.z, d0.w, d1.x, d1.y, d1.z, d1.w};
+          float fi[8], fd[8];
+#pragma unroll
+          for (int k = 0; k < 8; ++k) {
+            fi[k] = (float)((int)(w[k] << 16) >> 16);
+            fd[k] = __fmul_rn(half_bits_to_float((uint16_t)(w[k] >> 16)), __uint_as_float(dv[k]));
+          }
+          if (k0 + 8 < nu)
+            fetch(k0 + 8);
+#pragma unroll
+          for (int k = 0; k < 8; ++k)
+            if (k0 + k < nu)
+              acc = __fmaf_rn(fi[k], fd[k], acc);
+        }
+        const size_t o = (size_t)(g_lo + g0 + gi) * 8 + r;
         if (!PUBLISH) {
           y[o] = acc;
         } else {
@@ -270,11 +328,11 @@ gemv_q4_0_kernel(const float *__restrict__ x, const uint8_t *__restrict__ W, flo
             }
         }
       }
-      if (!ok)
-        break;
+      if (bt + 2 < batches)
+        handover_arrive(4 + buf);
     }
   }
-  // Every stage armed by the producer is waited for by its consumer warp, so no bulk copy is in flight here unless
+  // Every stage armed by the producer is waited for by the consumer warps of its passes, so no bulk copy is in flight here unless
   // the CTA aborted; then give the copies time to land before the memory is released.
   if (*abort_flag)
     for (int i = 0; i < 1000; ++i)

@@ -33,7 +33,8 @@
  *                store of y.
  * Per 256 weights a lane spends ~500 instructions (6-bit unpack is ~5x the work
  * of Q4_K): on this part the kernel is bound by instruction issue and latency,
- * not by HBM. Algorithmic bytes per launch: N * nb * 210 (weights) + 4K (x) +
+ * not by HBM. Rows of 33 to 64 blocks take the same kernel in two passes per row
+ * (4096 x 12288: 17 us, 99 in the dp4a kernel they used to be left to). Algorithmic bytes per launch: N * nb * 210 (weights) + 4K (x) +
  * 4N (y). Rows beyond the last whole stage form one short stage for the last
  * CTA when their byte size is a multiple of 16; otherwise they are left to the
  * caller (the dp4a kernel of gemv_dp4a.cu takes them).
@@ -80,8 +81,9 @@ __device__ __forceinline__ bool wait_armed(volatile int *armed, int t, volatile 
   return false;
 }
 
-/** whole rows a warp takes per step: lane = block of a row; at most four rows (8 chain lanes each) */
-__host__ __device__ inline int q6_rows_per_step(int nb) { return 32 / nb < 4 ? 32 / nb : 4; }
+/** whole rows a warp takes per step: lane = block of a row; at most four rows (8 chain lanes each). A row of more than 32
+ *  blocks is a step of its own, in passes of 32 blocks. */
+__host__ __device__ inline int q6_rows_per_step(int nb) { return nb > 32 ? 1 : 32 / nb < 4 ? 32 / nb : 4; }
 
 struct Q6Layout {
   uint32_t act, rec, ring, bars, total;
@@ -103,12 +105,14 @@ __host__ __device__ inline Q6Layout q6_layout(int nb, int stage_bytes, int stage
   return L;
 }
 
+/* LONG: rows of more than 32 blocks. A kernel of its own: the passes in the loop of the short rows cost those 4%. */
+template <bool LONG>
 __global__ void __launch_bounds__(Q6_THREADS, 1)
 gemv_q6_K_kernel(const float *__restrict__ x, const uint8_t *__restrict__ W, float *__restrict__ y, int n_stages_total,
                  int rows_per_stage, int nb, int n_ring, int tail_rows) {
   extern __shared__ __align__(128) uint8_t smem[];
   const int stage_blocks = rows_per_stage * nb, stage_bytes = stage_blocks * (int)sizeof(BlockQ6K);
-  const int rows_per_step = q6_rows_per_step(nb), active = rows_per_step * nb; // lanes at work in a step
+  const int rows_per_step = q6_rows_per_step(nb), active = rows_per_step * nb; // blocks of a step
   const int steps = rows_per_stage / rows_per_step;
   const Q6Layout L = q6_layout(nb, stage_bytes, stage_blocks, n_ring);
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -189,8 +193,7 @@ gemv_q6_K_kernel(const float *__restrict__ x, const uint8_t *__restrict__ W, flo
     }
     asm volatile("bar.sync 1, %0;" ::"n"(Q6_CONSUMER_WARPS * 32) : "memory");
 
-    const int b = lane % nb;                                // super-block of the lane's row
-    const uint32_t ab = sm0 + L.act + (uint32_t)b * Q6_ACT_STRIDE;
+    const uint32_t ab0 = sm0 + L.act + (uint32_t)(LONG ? lane : lane % nb) * Q6_ACT_STRIDE; // super-block of the lane's row
     const uint32_t myrec = sm0 + L.rec + (uint32_t)((warp * 32 + lane) * Q6_REC_WORDS * 4);
     // chain role: 8 lanes per row of the step
     const int crow = lane >> 3, cl = lane & 7;
@@ -205,81 +208,103 @@ gemv_q6_K_kernel(const float *__restrict__ x, const uint8_t *__restrict__ W, flo
       // rows of this step: rows_per_step, fewer in the last step of the short stage
       const int step_rows = (i < my_stages || my_tail - st * rows_per_step >= rows_per_step) ? rows_per_step
                                                                                             : my_tail - st * rows_per_step;
-      const bool work = lane < step_rows * nb, chain = crow < step_rows;
-      if (work) {
-        const int t = st * active + lane; // block inside the stage
-        const uint32_t off = (uint32_t)t * 210u;
-        const uint32_t raw = sm0 + L.ring + (uint32_t)s * (uint32_t)(stage_bytes + 16) + (off & ~3u);
-        const uint32_t sh = (off & 2u) * 8u; // 0 or 16
-        int part[8];
+      const bool chain = crow < step_rows;
+      float acc = 0.f;
+      for (int p0 = 0; p0 < (LONG ? nb : 1); p0 += 32) {
+        const bool work = LONG ? p0 + lane < nb && step_rows > 0 : lane < step_rows * nb;
+        const uint32_t ab = ab0 + (uint32_t)p0 * Q6_ACT_STRIDE;
+        if (work) {
+          const int t = st * active + p0 + lane; // block inside the stage
+          const uint32_t off = (uint32_t)t * 210u;
+          const uint32_t raw = sm0 + L.ring + (uint32_t)s * (uint32_t)(stage_bytes + 16) + (off & ~3u);
+          const uint32_t sh = (off & 2u) * 8u; // 0 or 16
+          int part[8];
 #pragma unroll
-        for (int k = 0; k < 8; ++k)
-          part[k] = 0;
-        int sc[16];
-        {
-          uint32_t prev = lds32(raw + 192);
-#pragma unroll
-          for (int k = 0; k < 4; ++k) {
-            const uint32_t next = lds32(raw + 192 + 4 * k + 4);
-            const uint32_t w = __funnelshift_r(prev, next, sh);
-            prev = next;
-#pragma unroll
-            for (int j = 0; j < 4; ++j)
-              sc[4 * k + j] = sbyte(w, j);
-          }
-          // prev now holds the aligned word with the block's d (bytes 208, 209 of the block)
-          const float dw = half_bits_to_float((uint16_t)((prev >> sh) & 0xffffu));
-          sts32(myrec + 32, __float_as_uint(__fmul_rn(__uint_as_float(lds32(ab + 512)), dw)));
-        }
-#pragma unroll
-        for (int h = 0; h < 2; ++h) {
-          uint32_t ql[16], qh[8];
+          for (int k = 0; k < 8; ++k)
+            part[k] = 0;
+          int sc[16];
           {
-            uint32_t prev = lds32(raw + 64 * h);
+            uint32_t prev = lds32(raw + 192);
 #pragma unroll
-            for (int k = 0; k < 16; ++k) {
-              const uint32_t next = lds32(raw + 64 * h + 4 * k + 4);
-              ql[k] = __funnelshift_r(prev, next, sh);
+            for (int k = 0; k < 4; ++k) {
+              const uint32_t next = lds32(raw + 192 + 4 * k + 4);
+              const uint32_t w = __funnelshift_r(prev, next, sh);
               prev = next;
+#pragma unroll
+              for (int j = 0; j < 4; ++j)
+                sc[4 * k + j] = sbyte(w, j);
             }
-            prev = lds32(raw + 128 + 32 * h);
+            // prev now holds the aligned word with the block's d (bytes 208, 209 of the block)
+            const float dw = half_bits_to_float((uint16_t)((prev >> sh) & 0xffffu));
+            sts32(myrec + 32, __float_as_uint(__fmul_rn(__uint_as_float(lds32(ab + 512)), dw)));
+          }
+#pragma unroll
+          for (int h = 0; h < 2; ++h) {
+            uint32_t ql[16], qh[8];
+            {
+              uint32_t prev = lds32(raw + 64 * h);
+#pragma unroll
+              for (int k = 0; k < 16; ++k) {
+                const uint32_t next = lds32(raw + 64 * h + 4 * k + 4);
+                ql[k] = __funnelshift_r(prev, next, sh);
+                prev = next;
+              }
+              prev = lds32(raw + 128 + 32 * h);
+#pragma unroll
+              for (int k = 0; k < 8; ++k) {
+                const uint32_t next = lds32(raw + 128 + 32 * h + 4 * k + 4);
+                qh[k] = __funnelshift_r(prev, next, sh);
+                prev = next;
+              }
+            }
+#pragma unroll
+            for (int wi = 0; wi < 8; ++wi) {
+              const uint4 a4 = lds128(ab + ((h * 8 + wi) * 4) * 4);
+              const uint4 c4 = lds128(ab + 256 + ((h * 8 + wi) * 4) * 4);
+              const uint32_t la = ql[wi], lb = ql[8 + wi], hb = qh[wi];
+              const uint32_t v0 = (la & 0x0f0f0f0fu) | ((hb << 4) & 0x30303030u);
+              const uint32_t v1 = (lb & 0x0f0f0f0fu) | ((hb << 2) & 0x30303030u);
+              const uint32_t v2 = ((la >> 4) & 0x0f0f0f0fu) | (hb & 0x30303030u);
+              const uint32_t v3 = ((lb >> 4) & 0x0f0f0f0fu) | ((hb >> 2) & 0x30303030u);
+              // scale of quarter w, elements 0-15 / 16-31: entry 8h + 2w + (wi >> 2) of the 16
+              const int g0 = 8 * h + (wi >> 2);
+              part[wi] += sc[g0 + 0] * dp4a_us(v0, a4.x, (int)c4.x);
+              part[wi] += sc[g0 + 2] * dp4a_us(v1, a4.y, (int)c4.y);
+              part[wi] += sc[g0 + 4] * dp4a_us(v2, a4.z, (int)c4.z);
+              part[wi] += sc[g0 + 6] * dp4a_us(v3, a4.w, (int)c4.w);
+            }
+          }
+#pragma unroll
+          for (int k = 0; k < 8; ++k)
+            sts32(myrec + 4 * k, (uint32_t)part[k]);
+        }
+        __syncwarp();
+        if (lane == 0 && (!LONG || p0 + 32 >= nb))
+          mbar_arrive(FREE_BAR(s)); // the stage's bytes are no longer needed by this step
+        if (!LONG && chain) {
+          for (int bb = 0; bb < nb; ++bb) {
+            const uint32_t r = crec + (uint32_t)(bb * Q6_REC_WORDS * 4);
+            acc = __fmaf_rn(__uint_as_float(lds32(r + 32 - 4 * cl)), (float)(int)lds32(r), acc);
+          }
+        }
+        if (LONG && chain) {
+          const int n = nb - p0 < 32 ? nb - p0 : 32;
+          for (int b0 = 0; b0 < n; b0 += 8) { // eight records on their way, then joined to the chain in order
+            uint32_t iv[8], dv[8];
 #pragma unroll
             for (int k = 0; k < 8; ++k) {
-              const uint32_t next = lds32(raw + 128 + 32 * h + 4 * k + 4);
-              qh[k] = __funnelshift_r(prev, next, sh);
-              prev = next;
+              const uint32_t r = crec + (uint32_t)((b0 + k < n ? b0 + k : n - 1) * Q6_REC_WORDS * 4);
+              dv[k] = lds32(r + 32 - 4 * cl);
+              iv[k] = lds32(r);
             }
-          }
 #pragma unroll
-          for (int wi = 0; wi < 8; ++wi) {
-            const uint4 a4 = lds128(ab + ((h * 8 + wi) * 4) * 4);
-            const uint4 c4 = lds128(ab + 256 + ((h * 8 + wi) * 4) * 4);
-            const uint32_t la = ql[wi], lb = ql[8 + wi], hb = qh[wi];
-            const uint32_t v0 = (la & 0x0f0f0f0fu) | ((hb << 4) & 0x30303030u);
-            const uint32_t v1 = (lb & 0x0f0f0f0fu) | ((hb << 2) & 0x30303030u);
-            const uint32_t v2 = ((la >> 4) & 0x0f0f0f0fu) | (hb & 0x30303030u);
-            const uint32_t v3 = ((lb >> 4) & 0x0f0f0f0fu) | ((hb >> 2) & 0x30303030u);
-            // scale of quarter w, elements 0-15 / 16-31: entry 8h + 2w + (wi >> 2) of the 16
-            const int g0 = 8 * h + (wi >> 2);
-            part[wi] += sc[g0 + 0] * dp4a_us(v0, a4.x, (int)c4.x);
-            part[wi] += sc[g0 + 2] * dp4a_us(v1, a4.y, (int)c4.y);
-            part[wi] += sc[g0 + 4] * dp4a_us(v2, a4.z, (int)c4.z);
-            part[wi] += sc[g0 + 6] * dp4a_us(v3, a4.w, (int)c4.w);
+            for (int k = 0; k < 8; ++k)
+              if (b0 + k < n)
+                acc = __fmaf_rn(__uint_as_float(dv[k]), (float)(int)iv[k], acc);
           }
         }
-#pragma unroll
-        for (int k = 0; k < 8; ++k)
-          sts32(myrec + 4 * k, (uint32_t)part[k]);
-      }
-      __syncwarp();
-      if (lane == 0)
-        mbar_arrive(FREE_BAR(s)); // the stage's bytes are no longer needed by this step
-      float acc = 0.f;
-      if (chain) {
-        for (int bb = 0; bb < nb; ++bb) {
-          const uint32_t r = crec + (uint32_t)(bb * Q6_REC_WORDS * 4);
-          acc = __fmaf_rn(__uint_as_float(lds32(r + 32 - 4 * cl)), (float)(int)lds32(r), acc);
-        }
+        if (LONG)
+          __syncwarp(); // the scratch is rewritten by the next pass
       }
       // ((a4+a0)+(a6+a2)) + ((a5+a1)+(a7+a3)); IEEE addition commutes, so only the pairing matters
       float u = __fadd_rn(acc, __shfl_xor_sync(FULL, acc, 4));
@@ -303,7 +328,7 @@ gemv_q6_K_kernel(const float *__restrict__ x, const uint8_t *__restrict__ W, flo
 /** Picks rows per stage and ring depth. A step is floor(32/nb) whole rows; a stage is a whole number of steps whose
  *  byte size is a multiple of 16 (rows * nb % 8 == 0), about 24 KB. False if the shape does not fit. */
 static bool q6_plan(unsigned N, int nb, int &rows_per_stage, int &n_ring, uint32_t &smem_bytes) {
-  if (nb < 1 || nb > 32)
+  if (nb < 1 || nb > 64)
     return false;
   const int rps = q6_rows_per_step(nb);
   int rs = 0;
@@ -350,7 +375,8 @@ int launch_gemv_q6_K_stream(unsigned N, unsigned K, const float *x, const void *
   int dev = 0;
   NNTR_CHECK_CUDA(cudaGetDevice(&dev));
   if (!attr_done[dev & 63]) {
-    NNTR_CHECK_CUDA(cudaFuncSetAttribute(gemv_q6_K_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, Q6_SMEM_BUDGET));
+    NNTR_CHECK_CUDA(cudaFuncSetAttribute(gemv_q6_K_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, Q6_SMEM_BUDGET));
+    NNTR_CHECK_CUDA(cudaFuncSetAttribute(gemv_q6_K_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, Q6_SMEM_BUDGET));
     attr_done[dev & 63] = true;
   }
   const int n_stages_total = (int)(N / rs);
@@ -370,8 +396,8 @@ int launch_gemv_q6_K_stream(unsigned N, unsigned K, const float *x, const void *
   attr[0].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
   cfg.numAttrs = (flags & NNTR_CUDA_GEMV_PDL) ? 1 : 0;
-  cudaError_t e = cudaLaunchKernelEx(&cfg, gemv_q6_K_kernel, x, static_cast<const uint8_t *>(B), y, n_stages_total, rs,
-                                     nb, ring, tail_rows);
+  cudaError_t e = cudaLaunchKernelEx(&cfg, nb > 32 ? gemv_q6_K_kernel<true> : gemv_q6_K_kernel<false>, x,
+                                     static_cast<const uint8_t *>(B), y, n_stages_total, rs, nb, ring, tail_rows);
   count_launch();
   return check_cuda(e, "gemv_q6_K launch");
 }

@@ -47,12 +47,13 @@ struct MoeEp {
 };
 
 /* From where on the pairs are sorted by expert and run as per-expert GEMMs (all of a batch's rows for one read of an expert's
- * weights, but three launches more than a GEMV per pair). Q4_0: from two tokens; 4 of 32 experts of 2880 x 2880, 2 / 4 / 6
- * tokens: 64 / 84 / 91 us against 68 / 124 / 164. Q4_K: while three CTAs per pair still fit one wave of two per SM the pairs
- * win: 8 of 128 experts of 2048 x 768, 8 / 12 / 14 tokens: 60 / 77 / 104 us against 71 / 88 / 92. */
+ * weights, but three launches more than a GEMV per pair): where a GEMV per pair no longer gets enough of the GPU. Q4_0 (gate and
+ * up are two problems per pair, one CTA per SM): below four CTAs per problem; 4 of 32 experts of 2880 x 2880, 2 / 4 / 5 / 8
+ * tokens: GEMVs 45 / 73 / 90 / 128 us, grouped 60 / 81 / 85 / 101. Q4_K (one problem per pair, two CTAs per SM): below three;
+ * 8 of 128 experts of 2048 x 768, 8 / 12 / 14 tokens: 60 / 77 / 104 us against 71 / 88 / 92. */
 constexpr unsigned GROUPED_MIN_TOKENS = 2;
 static bool run_grouped(int qtype, unsigned tokens, unsigned pairs) {
-  return tokens >= GROUPED_MIN_TOKENS && (qtype == NNTR_Q4_0 || 3 * pairs > 2 * (unsigned)sm_count());
+  return tokens >= GROUPED_MIN_TOKENS && (qtype == NNTR_Q4_0 ? 8 * pairs > (unsigned)sm_count() : 3 * pairs > 2 * (unsigned)sm_count());
 }
 constexpr int MOE_COUNTER_TOKENS = 4096;   // arrival counters kept at the start of the scratch for up to this many tokens
 constexpr int ROUTER_WARPS = 8;

@@ -76,6 +76,15 @@ __device__ __forceinline__ void bulk_g2s(uint32_t dst, const void *src, uint32_t
                : "memory");
 }
 
+/** Quotients by a number known at run time only, exact while dividend * n < 2^32: a multiplication instead of the 150 clocks
+ *  (64 bits: several hundred) of a division, which a loop with one thread or warp per stage of a ring cannot hide. */
+struct FastDiv {
+  uint32_t n, m;
+  __device__ __forceinline__ explicit FastDiv(uint32_t d) : n(d), m(d > 1 ? 0xffffffffu / d + 1 : 0) {}
+  __device__ __forceinline__ int div(int t) const { return n > 1 ? (int)__umulhi((uint32_t)t, m) : t; }
+  __device__ __forceinline__ int mod(int t, int q) const { return t - q * (int)n; } // q = div(t)
+};
+
 /** 4-way dot product of unsigned bytes (a) with signed bytes (b), accumulated in c */
 __device__ __forceinline__ int dp4a_us(uint32_t a, uint32_t b, int c) {
   int d;
@@ -101,6 +110,9 @@ __device__ __forceinline__ uint4 lds128(uint32_t a) {
 }
 __device__ __forceinline__ void sts32(uint32_t a, uint32_t v) {
   asm volatile("st.shared.u32 [%0], %1;" ::"r"(a), "r"(v) : "memory");
+}
+__device__ __forceinline__ void sts128(uint32_t a, uint32_t v0, uint32_t v1, uint32_t v2, uint32_t v3) {
+  asm volatile("st.shared.v4.u32 [%0], {%1, %2, %3, %4};" ::"r"(a), "r"(v0), "r"(v1), "r"(v2), "r"(v3) : "memory");
 }
 __device__ __forceinline__ void sts64(uint32_t a, uint32_t v0, uint32_t v1) {
   asm volatile("st.shared.v2.u32 [%0], {%1, %2};" ::"r"(a), "r"(v0), "r"(v1) : "memory");

@@ -150,6 +150,18 @@ def test_gemv_q6_K_streaming_kernel_row_groupings(be, port, N, K):
     assert np.array_equal(bits(y.cpu().numpy()), bits(want))
 
 
+@pytest.mark.parametrize("N,K", [(8, 8448), (300, 9728), (16, 16384), (24, 16640)])
+def test_gemv_q6_K_rows_of_more_than_32_blocks(be, port, N, K):
+    """Two passes per row (33, 38 and 64 super-blocks) in the streaming kernel, and the first size beyond it."""
+    rng = np.random.default_rng(N + K)
+    B = O.random_q6_K(rng, N, K)
+    x = acts(rng, 1, K)
+    y = torch.full((N,), float("nan"), device="cuda")
+    be.gemm_q6_K(1, N, K, dev(x), K, dev(B), N, y, N)
+    be.device_status()
+    assert np.array_equal(bits(y.cpu().numpy()), bits(port.gemm("q6_K", x, B, N)[0]))
+
+
 @pytest.mark.parametrize("N,K", [(21312, 1024), (24576, 4096), (2880, 2880), (5760, 2880)])
 def test_gemv_q4_0_streaming_kernel_many_row_groups(be, port, N, K):
     """Q4_0 decode GEMV where every CTA owns more row groups than it has consumer warps (warps run ahead of the
