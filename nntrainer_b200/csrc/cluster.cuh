@@ -40,6 +40,13 @@ __device__ __forceinline__ float4 ld_cluster4(uint32_t addr, int rank) {
   return v;
 }
 
+/** the same for a store */
+__device__ __forceinline__ void st_cluster4(uint32_t addr, int rank, const float4 &v) {
+  uint32_t remote;
+  asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(remote) : "r"(addr), "r"(rank));
+  asm volatile("st.shared::cluster.v4.f32 [%0], {%1,%2,%3,%4};" ::"r"(remote), "f"(v.x), "f"(v.y), "f"(v.z), "f"(v.w) : "memory");
+}
+
 /** Launch of a grid of grid.x * parts by grid.y CTAs in clusters of `parts` CTAs along x. The grid may start while its
  *  predecessor runs: the kernel calls pdl_wait() before it touches what that wrote. */
 template <typename... P, typename... A>

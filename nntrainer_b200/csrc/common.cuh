@@ -298,6 +298,8 @@ int launch_gemv_q4_K_batched_publish(unsigned N, unsigned K, const float *x, uns
 int read_moe_status(int *out);
 /* resident-weights variant for small per-CTA shares (gemv_q4k_resident.cu) */
 bool gemv_q4_K_resident_supported(unsigned N, unsigned K, bool exchange = false, bool norm = false);
+bool gemv_q4_K_split_supported(unsigned N, unsigned K);
+int launch_gemv_q4_K_split(unsigned N, unsigned K, const float *x, const void *B, float *y, unsigned flags, cudaStream_t st);
 struct GemvExchange;
 int launch_gemv_q4_K_resident(unsigned N, unsigned K, const float *x, const void *B, float *y, unsigned flags,
                               cudaStream_t st, const GemvExchange *exchange = nullptr, const GemvBatch *norm = nullptr);

@@ -88,12 +88,12 @@ __global__ void embedding_kernel(int qtype, const uint8_t *__restrict__ table, c
   if (!(idf >= 0.f) || id >= in_dim) {
     if (threadIdx.x == 0)
       atomicExch(&g_embed_status, NNTR_CUDA_ERR_INVALID);
-    for (unsigned i = threadIdx.x; i < out_dim; i += blockDim.x)
+    for (unsigned i = blockIdx.y * blockDim.x + threadIdx.x; i < out_dim; i += gridDim.y * blockDim.x)
       out[i] = 0.f;
     return;
   }
   const uint8_t *row = table + id * row_bytes;
-  for (unsigned i = threadIdx.x; i < out_dim; i += blockDim.x) {
+  for (unsigned i = blockIdx.y * blockDim.x + threadIdx.x; i < out_dim; i += gridDim.y * blockDim.x) {
     float v;
     if (qtype == NNTR_Q6_K) {
       v = deq_q6_K_elem(row + (size_t)(i >> 8) * sizeof(BlockQ6K), (int)(i & 255));
@@ -136,7 +136,7 @@ int launch_embedding(int qtype, const void *table, const float *ids, float *y, u
   if (n_ids == 0)
     return NNTR_CUDA_OK;
   cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(n_ids);
+  cfg.gridDim = dim3(n_ids, std::min(64u, (out_dim + 255) / 256)); // an element per thread: the row's reads are one round trip
   cfg.blockDim = dim3(256);
   cfg.stream = st;
   cudaLaunchAttribute attr[1];

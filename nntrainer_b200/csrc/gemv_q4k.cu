@@ -542,6 +542,9 @@ int launch_gemv_q4_K(unsigned N, unsigned K, const float *x, const void *B, floa
   static const int use_resident = env_int("NNTR_CUDA_GEMV_RESIDENT", 1);
   if (use_resident && x && y && B && gemv_q4_K_resident_supported(N, K))
     return launch_gemv_q4_K_resident(N, K, x, B, y, flags, st);
+  // long rows in few row groups: the same with every row shared by a cluster
+  if (use_resident && x && y && B && gemv_q4_K_split_supported(N, K))
+    return launch_gemv_q4_K_split(N, K, x, B, y, flags, st);
   GemvBatch none = {};
   return launch_gemv_q4_K_batched(N, K, x, B, y, flags, 1, none, st);
 }
@@ -699,14 +702,25 @@ int launch_gemv_q4_K_batched(unsigned N, unsigned K, const float *x, const void 
   return check_cuda(e, "gemv_q4_K launch");
 }
 
-__global__ void epoch_bump_kernel(unsigned long long *epoch) { *epoch += 1; }
+__global__ void epoch_bump_kernel(unsigned long long *epoch) {
+  pdl_wait(); // scheduled while the kernel before it runs (a decode step ends with this launch)
+  *epoch += 1;
+}
 
 int launch_epoch_bump(unsigned long long *epoch, cudaStream_t st) {
   if (!epoch)
     return set_error(NNTR_CUDA_ERR_INVALID, "epoch_bump: null pointer");
-  epoch_bump_kernel<<<1, 1, 0, st>>>(epoch);
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = cfg.blockDim = dim3(1);
+  cfg.stream = st;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  const cudaError_t e = cudaLaunchKernelEx(&cfg, epoch_bump_kernel, epoch);
   count_launch();
-  return check_cuda(cudaGetLastError(), "epoch_bump launch");
+  return check_cuda(e, "epoch_bump launch");
 }
 
 int set_exchange_poll_limit_gemv(unsigned polls) {

@@ -23,6 +23,7 @@
  * Roofline: HBM (algorithmic bytes N*K*4.5/8 + 4K + 4N per launch), as for the streaming kernel.
  * Every wait is bounded (status word of gemv_q4k.cu's family: this file has its own).
  */
+#include "cluster.cuh"
 #include "common.cuh"
 #include "pipeline.cuh"
 #include "rms.cuh"
@@ -63,8 +64,9 @@ struct RLayout {
   uint32_t ring, act, part, bars, abort_flag, total;
 };
 /** `exchange`: the part[] region doubles as the per-warp staging area of the numbered activation (1 KB per warp, used
- * before the first barrier; part[] is written after it), so it is 16 KB instead of 8 */
-__host__ __device__ inline RLayout r_layout(int nb, bool exchange, bool norm = false) {
+ * before the first barrier; part[] is written after it), so it is 16 KB instead of 8. split_groups: row groups of a cluster
+ * that one of its CTAs adds up (nb is then still the whole row's) */
+__host__ __device__ inline RLayout r_layout(int nb, bool exchange, bool norm = false, int split_groups = 0) {
   RLayout L;
   uint32_t o = 0;
   L.ring = o;
@@ -74,7 +76,10 @@ __host__ __device__ inline RLayout r_layout(int nb, bool exchange, bool norm = f
   o = (o + 15) & ~15u;
   L.part = o;
   // (with the norm prologue the area first holds the K floats of the activation row and the scale)
-  const uint32_t part_bytes = exchange ? R_WARPS * 1024 : R_MAX_BLOCKS * 8 * 16, row_bytes = norm ? nb * QK_K * 4 + 16 : 0;
+  const uint32_t part_bytes = split_groups ? split_groups * nb * 8 * 16
+                              : exchange   ? R_WARPS * 1024
+                                           : R_MAX_BLOCKS * 8 * 16,
+                 row_bytes = norm ? nb * QK_K * 4 + 16 : 0;
   o += part_bytes > row_bytes ? part_bytes : row_bytes;
   o = (o + 15) & ~15u;
   L.bars = o;
@@ -87,18 +92,25 @@ __host__ __device__ inline RLayout r_layout(int nb, bool exchange, bool norm = f
 
 } // namespace
 
-/* NORM: the activation is rms_norm(x + nm.x2) * nm.gamma, computed by every CTA for itself after the wait (the residual
+/* SPLIT: a cluster shares its row groups, each CTA holds a part of K of all of them (blocks b_lo .. of every row group) and
+ * quantizes only that part of the activation; the units' results meet in the CTA that adds the row group up (they are dealt out)
+ * and the chain runs there over the whole row. For long rows in few row groups: with whole row groups per CTA the 2560 x 9728
+ * projection of a decoder has 24 of 296 CTAs with two, which end 2.4 us after the rest, and every CTA quantizes 38 blocks (2 us).
+ * NORM: the activation is rms_norm(x + nm.x2) * nm.gamma, computed by every CTA for itself after the wait (the residual
  * add and RMS norm in front of a projection; one CTA stores the sum to nm.sum_out); see GemvBatch::act. */
-template <bool EXCHANGE, bool NORM>
+template <bool EXCHANGE, bool NORM, bool SPLIT>
 __global__ void __maxnreg__(EXCHANGE ? 64 : 56)
 gemv_q4_K_resident_kernel(const float *__restrict__ x, const BlockQ4Kx8 *__restrict__ W, float *__restrict__ y,
-                          int n_groups, int nb, const GemvExchange ex, const GemvBatch nm) {
+                          int n_groups, int k_blocks, const GemvExchange ex, const GemvBatch nm) {
   // Every use of `ex` is guarded by the compile-time EXCHANGE, so the plain instantiation carries none of that code.
   // Its pointer arrays are only ever indexed through pick8() with constant indices: a run-time index into a kernel
   // parameter would make the compiler copy the whole description into every thread's local memory (measured: 15 MB
   // of local-memory stores per launch, more than the weights).
   extern __shared__ __align__(128) uint8_t smem[];
-  const RLayout L = r_layout(nb, EXCHANGE, NORM);
+  const int csize = SPLIT ? cluster_size() : 1, crank = SPLIT ? cluster_rank() : 0;
+  const int b_lo = SPLIT ? k_blocks * crank / csize : 0, nb = SPLIT ? k_blocks * (crank + 1) / csize - b_lo : k_blocks;
+  const int n_shares = gridDim.x / csize, share = blockIdx.x / csize;
+  const RLayout L = r_layout(k_blocks, EXCHANGE, NORM, SPLIT ? ((n_groups + n_shares - 1) / n_shares + csize - 1) / csize : 0);
   uint8_t *ring = smem + L.ring;
   uint8_t *act = smem + L.act;
   float4 *part = reinterpret_cast<float4 *>(smem + L.part);
@@ -106,8 +118,8 @@ gemv_q4_K_resident_kernel(const float *__restrict__ x, const BlockQ4Kx8 *__restr
   const uint32_t bar0 = smem_u32(smem + L.bars);
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
 
-  const int g_first = (int)(((long long)blockIdx.x * n_groups) / gridDim.x);
-  const int g_end = (int)(((long long)(blockIdx.x + 1) * n_groups) / gridDim.x);
+  const int g_first = (int)(((long long)share * n_groups) / n_shares);
+  const int g_end = (int)(((long long)(share + 1) * n_groups) / n_shares);
   const int ng = g_end - g_first;
   const int total_blocks = ng * nb; // <= R_MAX_BLOCKS (checked by the launcher)
   const int n_copies = (total_blocks + R_COPY_BLOCKS - 1) / R_COPY_BLOCKS;
@@ -119,20 +131,26 @@ gemv_q4_K_resident_kernel(const float *__restrict__ x, const BlockQ4Kx8 *__restr
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   __syncthreads();
+  if (SPLIT)
+    asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory"); // waited for before the first store to a neighbour
   // let the next kernel in the stream be scheduled now: issuing the copies below can stall on the memory system, and a
   // dependent grid is launched only after every CTA of this one has passed this point
   pdl_launch_dependents();
   if (warp == 0) {
     // the CTA's whole share, one bulk copy per block so that blocks land R_BLK_STRIDE apart
-    const uint8_t *src = reinterpret_cast<const uint8_t *>(W + (size_t)g_first * nb);
+    const uint8_t *src = reinterpret_cast<const uint8_t *>(W + (size_t)g_first * k_blocks + b_lo);
+    const FastDiv by_nb(nb);
     for (int c = 0; c < n_copies; ++c) {
       const int nblk = min(R_COPY_BLOCKS, total_blocks - c * R_COPY_BLOCKS);
       if (lane == 0)
         mbar_expect_tx(bar0 + 8 * c, nblk * R_BLK_BYTES);
       __syncwarp();
-      if (lane < nblk)
-        bulk_g2s(smem_u32(ring + (c * R_COPY_BLOCKS + lane) * R_BLK_STRIDE),
-                 src + ((size_t)c * R_COPY_BLOCKS + lane) * R_BLK_BYTES, R_BLK_BYTES, bar0 + 8 * c);
+      if (lane < nblk) {
+        const int u = c * R_COPY_BLOCKS + lane; // block of the share; whole rows follow one another in memory
+        const int gu = SPLIT ? by_nb.div(u) : 0;
+        const size_t at = SPLIT ? (size_t)gu * k_blocks + by_nb.mod(u, gu) : (size_t)u;
+        bulk_g2s(smem_u32(ring + u * R_BLK_STRIDE), src + at * R_BLK_BYTES, R_BLK_BYTES, bar0 + 8 * c);
+      }
     }
   }
 
@@ -190,7 +208,7 @@ gemv_q4_K_resident_kernel(const float *__restrict__ x, const BlockQ4Kx8 *__restr
   uint32_t m2[4];    // same for the mins
   float dw = 0.f, dmw = 0.f;
   bool ok = true;
-  if (active) {
+  auto take_unit = [&]() {
     ok = mbar_wait_bounded(bar0 + 8 * (t / R_COPY_BLOCKS), 0, abort_flag, &g_resident_status, R_WAIT_POLLS, 1024);
     if (ok) {
       const uint8_t *blk = ring + t * R_BLK_STRIDE;
@@ -219,7 +237,9 @@ gemv_q4_K_resident_kernel(const float *__restrict__ x, const BlockQ4Kx8 *__restr
       dw = half_bits_to_float(*reinterpret_cast<const uint16_t *>(blk + 2 * r));
       dmw = half_bits_to_float(*reinterpret_cast<const uint16_t *>(blk + 16 + 2 * r));
     }
-  }
+  };
+  if (!SPLIT && active)
+    take_unit();
 
   // ---- everything below depends on the previous kernel's output
   if (!chained_by_tags)
@@ -323,7 +343,7 @@ gemv_q4_K_resident_kernel(const float *__restrict__ x, const BlockQ4Kx8 *__restr
         v1 = make_float4(__fmul_rn(__fmul_rn(r1.x, act_scale), m1.x), __fmul_rn(__fmul_rn(r1.y, act_scale), m1.y),
                          __fmul_rn(__fmul_rn(r1.z, act_scale), m1.z), __fmul_rn(__fmul_rn(r1.w, act_scale), m1.w));
       } else {
-        const float *xs = x + bb * QK_K + lane * 8;
+        const float *xs = x + (b_lo + bb) * QK_K + lane * 8;
         v0 = *reinterpret_cast<const float4 *>(xs);
         v1 = *reinterpret_cast<const float4 *>(xs + 4);
       }
@@ -339,6 +359,13 @@ gemv_q4_K_resident_kernel(const float *__restrict__ x, const BlockQ4Kx8 *__restr
       *reinterpret_cast<float *>(dst + 272) = qv.d;
   }
   __syncthreads();
+  if (SPLIT) {
+    // two CTAs fill an SM, so this launch's weights are not here before its activation: they travel while that is quantized
+    if (active)
+      take_unit();
+    __syncwarp();
+    asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); // every CTA of the cluster has started
+  }
 
   if (active && ok) {
     const uint8_t *a = act + b * R_ACT_STRIDE;
@@ -375,9 +402,16 @@ gemv_q4_K_resident_kernel(const float *__restrict__ x, const BlockQ4Kx8 *__restr
       j_acc = __dp2a_lo((int)bs2[p], (int)m2[p], j_acc);
     }
     const float da = *reinterpret_cast<const float *>(a + 272);
-    part[t * 8 + r] = make_float4((float)i_acc, __fmul_rn(dw, da), (float)j_acc, __fmul_rn(dmw, da));
+    const float4 res = make_float4((float)i_acc, __fmul_rn(dw, da), (float)j_acc, __fmul_rn(dmw, da));
+    if (SPLIT)
+      st_cluster4(smem_u32(part + ((size_t)(gl / csize) * k_blocks + b_lo + b) * 8 + r), gl % csize, res);
+    else
+      part[t * 8 + r] = res;
   }
-  __syncthreads();
+  if (SPLIT)
+    cluster_sync();
+  else
+    __syncthreads();
 
   if (EXCHANGE && ex.n_ranks && threadIdx.x >= R_THREADS - 32 && (int)(threadIdx.x - (R_THREADS - 32)) < ex.n_ranks) {
     // "done reading": this CTA has consumed its input (everything was quantized into shared memory before the barriers
@@ -394,12 +428,12 @@ gemv_q4_K_resident_kernel(const float *__restrict__ x, const BlockQ4Kx8 *__restr
     __syncwarp();
   }
   // ---- ordered float chain, one thread per output (ggml's acc = fma(I, d_w*d_a, acc) per super-block, ascending)
-  if (threadIdx.x < ng * 8 && !*abort_flag) {
-    const int g = threadIdx.x >> 3, rr = threadIdx.x & 7;
-    const float4 *pp = part + (size_t)g * nb * 8 + rr;
+  if ((SPLIT ? (int)(threadIdx.x >> 3) * csize + crank < ng : threadIdx.x < ng * 8) && !*abort_flag) {
+    const int slot = threadIdx.x >> 3, rr = threadIdx.x & 7, g = SPLIT ? slot * csize + crank : slot;
+    const float4 *pp = part + (size_t)slot * k_blocks * 8 + rr;
     float a0 = 0.f, a1 = 0.f;
 #pragma unroll 8
-    for (int bb = 0; bb < nb; ++bb) {
+    for (int bb = 0; bb < k_blocks; ++bb) {
       const float4 v = pp[bb * 8];
       a0 = __fmaf_rn(v.x, v.y, a0);
       a1 = __fmaf_rn(v.z, v.w, a1);
@@ -435,6 +469,72 @@ bool gemv_q4_K_resident_supported(unsigned N, unsigned K, bool exchange, bool no
   return max_groups * nb <= R_MAX_BLOCKS && r_layout(nb, exchange, norm).total <= 112u * 1024u && !(exchange && norm);
 }
 
+/** CTAs per cluster under which a launch with long rows fits (2, 4, 8: every CTA's units at most 64 blocks, one wave of two CTAs
+ *  per SM), 0 if none. Rows of 25 blocks and more: up to there whole row groups per CTA balance as well and the streaming kernel
+ *  needs no exchange (5000 x 5120: 6.6 us, split 7.4; 2560 x 9728: 8.0 and 7.6, 4096 x 8192: 9.6 and 8.2, 1280 x 12288: 7.7 and
+ *  6.7, in chains of dependent launches). */
+static int split_plan(unsigned N, unsigned K, int &shares, int &owned) {
+  static ClusterFit fit;
+  static bool attr_done[64] = {};
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || dev >= 64)
+    return 0;
+  if (!attr_done[dev]) {
+    if (cudaFuncSetAttribute(gemv_q4_K_resident_kernel<false, false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                             200 * 1024) != cudaSuccess ||
+        cudaFuncSetAttribute(gemv_q4_K_resident_kernel<false, false, true>, cudaFuncAttributePreferredSharedMemoryCarveout,
+                             cudaSharedmemCarveoutMaxShared) != cudaSuccess) {
+      (void)cudaGetLastError();
+      return 0;
+    }
+    attr_done[dev] = true;
+  }
+  if (K == 0 || K % QK_K || N % 8 || N == 0)
+    return 0;
+  const int n_groups = (int)(N / 8), nb = (int)(K / QK_K);
+  for (int parts = 2; parts <= 8; parts *= 2) {
+    shares = fit(gemv_q4_K_resident_kernel<false, false, true>, parts, R_THREADS, 100 * 1024); // one wave, two CTAs per SM
+    if (shares <= 0)
+      continue;
+    if (shares > n_groups)
+      shares = n_groups;
+    const int per_share = (n_groups + shares - 1) / shares, per_cta = (nb + parts - 1) / parts;
+    owned = (per_share + parts - 1) / parts;
+    if (nb > 24 && per_cta <= R_WARPS && per_share * per_cta <= R_MAX_BLOCKS && r_layout(nb, false, false, owned).total <= 100u * 1024u)
+      return parts;
+  }
+  return 0;
+}
+
+bool gemv_q4_K_split_supported(unsigned N, unsigned K) {
+  int shares, owned;
+  return split_plan(N, K, shares, owned) != 0;
+}
+
+int launch_gemv_q4_K_split(unsigned N, unsigned K, const float *x, const void *B, float *y, unsigned flags, cudaStream_t st) {
+  int shares = 0, owned = 0;
+  const int parts = split_plan(N, K, shares, owned);
+  if (!x || !y || !B || !parts || (reinterpret_cast<uintptr_t>(x) & 15) || (reinterpret_cast<uintptr_t>(B) & 15))
+    return set_error(NNTR_CUDA_ERR_INVALID, "gemv_q4_K (split): bad arguments");
+  cudaLaunchAttribute attr[2];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = parts;
+  attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+  attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[1].val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((unsigned)(shares * parts));
+  cfg.blockDim = dim3(R_THREADS);
+  cfg.dynamicSmemBytes = r_layout((int)(K / QK_K), false, false, owned).total;
+  cfg.stream = st;
+  cfg.attrs = attr;
+  cfg.numAttrs = (flags & NNTR_CUDA_GEMV_PDL) ? 2 : 1;
+  const cudaError_t e = cudaLaunchKernelEx(&cfg, gemv_q4_K_resident_kernel<false, false, true>, x, static_cast<const BlockQ4Kx8 *>(B),
+                                           y, (int)(N / 8), (int)(K / QK_K), GemvExchange{}, GemvBatch{});
+  count_launch();
+  return check_cuda(e, "gemv_q4_K (split) launch");
+}
+
 int launch_gemv_q4_K_resident(unsigned N, unsigned K, const float *x, const void *B, float *y, unsigned flags,
                               cudaStream_t st, const GemvExchange *exchange, const GemvBatch *norm) {
   GemvExchange ex = {};
@@ -463,9 +563,9 @@ int launch_gemv_q4_K_resident(unsigned N, unsigned K, const float *x, const void
 #define NNTR_RESIDENT_ATTRS(KERNEL)                                                                                          \
   NNTR_CHECK_CUDA(cudaFuncSetAttribute(KERNEL, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));                   \
   NNTR_CHECK_CUDA(cudaFuncSetAttribute(KERNEL, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared));
-    NNTR_RESIDENT_ATTRS((gemv_q4_K_resident_kernel<false, false>))
-    NNTR_RESIDENT_ATTRS((gemv_q4_K_resident_kernel<true, false>))
-    NNTR_RESIDENT_ATTRS((gemv_q4_K_resident_kernel<false, true>))
+    NNTR_RESIDENT_ATTRS((gemv_q4_K_resident_kernel<false, false, false>))
+    NNTR_RESIDENT_ATTRS((gemv_q4_K_resident_kernel<true, false, false>))
+    NNTR_RESIDENT_ATTRS((gemv_q4_K_resident_kernel<false, true, false>))
 #undef NNTR_RESIDENT_ATTRS
     attr_done[dev & 63] = true;
   }
@@ -480,9 +580,9 @@ int launch_gemv_q4_K_resident(unsigned N, unsigned K, const float *x, const void
   cfg.attrs = attr;
   cfg.numAttrs = (flags & NNTR_CUDA_GEMV_PDL) ? 1 : 0;
   const BlockQ4Kx8 *Wp = static_cast<const BlockQ4Kx8 *>(B);
-  cudaError_t e = exchange ? cudaLaunchKernelEx(&cfg, gemv_q4_K_resident_kernel<true, false>, x, Wp, y, n_groups, nb, ex, nm)
-                  : norm   ? cudaLaunchKernelEx(&cfg, gemv_q4_K_resident_kernel<false, true>, x, Wp, y, n_groups, nb, ex, nm)
-                           : cudaLaunchKernelEx(&cfg, gemv_q4_K_resident_kernel<false, false>, x, Wp, y, n_groups, nb, ex, nm);
+  cudaError_t e = exchange ? cudaLaunchKernelEx(&cfg, gemv_q4_K_resident_kernel<true, false, false>, x, Wp, y, n_groups, nb, ex, nm)
+                  : norm   ? cudaLaunchKernelEx(&cfg, gemv_q4_K_resident_kernel<false, true, false>, x, Wp, y, n_groups, nb, ex, nm)
+                           : cudaLaunchKernelEx(&cfg, gemv_q4_K_resident_kernel<false, false, false>, x, Wp, y, n_groups, nb, ex, nm);
   count_launch();
   return check_cuda(e, "gemv_q4_K (resident) launch");
 }

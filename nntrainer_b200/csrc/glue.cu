@@ -256,12 +256,18 @@ __global__ void argmax_kernel(const float *__restrict__ x, long long n, long lon
   const long long lo = n * sl / ARGMAX_SPLIT, hi = n * (sl + 1) / ARGMAX_SPLIT;
   float best = -INFINITY;
   unsigned bi = 0xffffffffu;
-  for (long long i = lo + threadIdx.x; i < hi; i += ARGMAX_THREADS) {
-    const float v = xr[i];
-    if (v > best || (bi == 0xffffffffu && v == best)) {
-      best = v;
-      bi = (unsigned)i;
-    }
+  constexpr int AT = 8; // on their way at a time
+  for (long long i0 = lo + threadIdx.x; i0 < hi; i0 += AT * ARGMAX_THREADS) {
+    float v[AT];
+#pragma unroll
+    for (int k = 0; k < AT; ++k)
+      v[k] = i0 + k * ARGMAX_THREADS < hi ? xr[i0 + k * ARGMAX_THREADS] : nanf(""); // never greater, never equal
+#pragma unroll
+    for (int k = 0; k < AT; ++k)
+      if (v[k] > best || (bi == 0xffffffffu && v[k] == best)) {
+        best = v[k];
+        bi = (unsigned)(i0 + k * ARGMAX_THREADS);
+      }
   }
   argmax_block_reduce(best, bi, sv, si);
   if (threadIdx.x == 0) {

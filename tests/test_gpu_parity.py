@@ -177,6 +177,19 @@ def test_gemv_q4_0_streaming_kernel_many_row_groups(be, port, N, K):
     assert np.array_equal(bits(y.cpu().numpy()), bits(want))
 
 
+@pytest.mark.parametrize("N,K", [(8, 6656), (2560, 9728), (1280, 12288), (1600, 6400), (4096, 8192)])
+def test_gemv_q4_K_long_rows_shared_by_a_cluster(be, port, N, K):
+    """Few row groups of 25 blocks and more: K in two, four or eight parts, even and uneven, one row group for a whole cluster
+    and several per CTA."""
+    rng = np.random.default_rng(N + K)
+    B = O.random_q4_Kx8(rng, N, K)
+    x = acts(rng, 1, K)
+    y = torch.full((N,), float("nan"), device="cuda")
+    be.gemm_q4_K(1, N, K, dev(x), K, dev(B), N, y, N)
+    be.device_status()
+    assert np.array_equal(bits(y.cpu().numpy()), bits(port.gemm("q4_K", x, B, N)[0]))
+
+
 def test_gemv_q6_K_streaming_kernel_full_lm_head_rows(be, port):
     """Q6_K decode GEMV with ~68 stages per CTA (consumer warps far ahead of the producer): N = 118400, K = 2560."""
     rng = np.random.default_rng(77)
