@@ -14,13 +14,13 @@
  *        d = a.Wd[e] (+ bd[e])
  *   y[token] = sum over the token's experts in ASCENDING expert index of d * w
  *
- * Decode (fewer than 8 tokens), no clearing launch: router (32 CTAs per token, the last to arrive reduces, selects and
+ * Decode (batches below the grouping line), no clearing launch: router (32 CTAs per token, the last to arrive reduces, selects and
  * writes the device-side weight-pointer tables), batched gate+up GEMV (the expert picked per problem through those
  * tables; Qwen form with Q4_K experts: one problem per pair over both matrices with the activation in the
  * epilogue -- four launches per layer; otherwise 2 * pairs problems and an activation launch -- five), batched down
  * GEMV, combine.
  * The reference runs every expert GEMV with M = 1 even in prefill, so the batched GEMV reproduces its numerics.
- * Prefill (8 tokens or more): the pairs are sorted by expert and each projection stage is ONE grouped GEMM launch over
+ * Prefill (batches above it): the pairs are sorted by expert and each projection stage is ONE grouped GEMM launch over
  * a device-side problem table; every row keeps the M = 1 float chain, so both paths give the same bits.
  * Top-k follows std::partial_sort of the GNU library, ties included (heap order emulated when two of the k + 1 greatest
  * probabilities are equal). The exponentials are the reference's (double exp for softmax and sigmoid, its table +
