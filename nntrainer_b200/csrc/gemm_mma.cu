@@ -445,22 +445,21 @@ template <int NT, typename F> __device__ __forceinline__ void with_tiles(int n, 
 
 /* --------------------------------------------------- a warp owns its rows */
 constexpr int ROWS_WARPS = 4;
-constexpr int ROWS_STAGES = 3; // units in flight per CTA
 constexpr int ROWS_W = ROWS_WARPS * 2 * (int)sizeof(BlockQ4Kx8); // the weights of a unit: 8 row groups (Q4_0: 8 blocks of 144)
 
 __device__ int g_mma_status = 0;
 
-template <int NT> struct RowsShared {
-  alignas(16) uint8_t w[ROWS_STAGES][ROWS_W];
-  alignas(16) uint8_t act[ROWS_STAGES][NT * 8 * act_row_bytes(NNTR_Q4_K)];
-  alignas(8) unsigned long long full[ROWS_STAGES], empty[ROWS_STAGES];
+template <int NT, int STAGES> struct RowsShared { // STAGES: units in flight per CTA
+  alignas(16) uint8_t w[STAGES][ROWS_W];
+  alignas(16) uint8_t act[STAGES][NT * 8 * act_row_bytes(NNTR_Q4_K)];
+  alignas(8) unsigned long long full[STAGES], empty[STAGES];
   int abort_flag;
 };
 
-template <int QT, int NT, bool GROUPED, bool TH8>
+template <int QT, int NT, bool GROUPED, bool TH8, int STAGES>
 __global__ void __launch_bounds__(ROWS_WARPS * 32, NT == 4 ? 3 : 4) gemm_mma_rows_kernel(const MmaArgs a) {
   extern __shared__ __align__(16) uint8_t rows_smem[];
-  RowsShared<NT> &sh = *reinterpret_cast<RowsShared<NT> *>(rows_smem);
+  RowsShared<NT, STAGES> &sh = *reinterpret_cast<RowsShared<NT, STAGES> *>(rows_smem);
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, g = lane >> 2, t = lane & 3;
   const int n_groups = a.N / 8, group0 = blockIdx.y * (2 * ROWS_WARPS), groups = min(2 * ROWS_WARPS, n_groups - group0);
   // this warp's two row groups inside the CTA's (past the end of N the last group is repeated and not stored)
@@ -476,7 +475,7 @@ __global__ void __launch_bounds__(ROWS_WARPS * 32, NT == 4 ? 3 : 4) gemm_mma_row
   volatile int *abort_flag = &sh.abort_flag;
   const uint32_t full0 = smem_u32(sh.full), empty0 = smem_u32(sh.empty);
   if (tid == 0) {
-    for (int s = 0; s < ROWS_STAGES; ++s) {
+    for (int s = 0; s < STAGES; ++s) {
       mbar_init(full0 + 8 * s, 1);
       mbar_init(empty0 + 8 * s, ROWS_WARPS);
     }
@@ -488,7 +487,7 @@ __global__ void __launch_bounds__(ROWS_WARPS * 32, NT == 4 ? 3 : 4) gemm_mma_row
    * kernel that writes the activations */
   auto unit_bytes = [&](int b) { return QT == NNTR_Q4_K ? (int)sizeof(BlockQ4Kx8) : min(8, a.nblk - 8 * b) * (int)sizeof(BlockQ40x8); };
   auto fetch_w = [&](int b) {
-    const int s = b % ROWS_STAGES, bytes = unit_bytes(b);
+    const int s = b % STAGES, bytes = unit_bytes(b);
     const size_t row = QT == NNTR_Q4_K ? (size_t)nb * sizeof(BlockQ4Kx8) : (size_t)a.nblk * sizeof(BlockQ40x8);
     const uint8_t *src = static_cast<const uint8_t *>(tl.W) + (size_t)group0 * row + (size_t)b * sizeof(BlockQ4Kx8);
     mbar_expect_tx(full0 + 8 * s, groups * bytes + nt * th * act_row_bytes(QT));
@@ -496,7 +495,7 @@ __global__ void __launch_bounds__(ROWS_WARPS * 32, NT == 4 ? 3 : 4) gemm_mma_row
       bulk_g2s(smem_u32(sh.w[s]) + i * (int)sizeof(BlockQ4Kx8), src + i * row, bytes, full0 + 8 * s);
   };
   auto fetch_act = [&](int b) {
-    const int s = b % ROWS_STAGES;
+    const int s = b % STAGES;
     for (int i = 0; i < nt; ++i)
       bulk_g2s(smem_u32(sh.act[s]) + i * (8 * act_row_bytes(QT)), act_unit<QT>(a.act, tl.act_tile + i, th, nb, b),
                th * act_row_bytes(QT), full0 + 8 * s);
@@ -505,11 +504,11 @@ __global__ void __launch_bounds__(ROWS_WARPS * 32, NT == 4 ? 3 : 4) gemm_mma_row
     return mbar_wait_bounded(bar, use & 1, abort_flag, &g_mma_status, 1u << 22, 2048);
   };
   if (tid == 0) {
-    for (int b = 0; b < ROWS_STAGES - 1 && b < nb; ++b)
+    for (int b = 0; b < STAGES - 1 && b < nb; ++b)
       fetch_w(b);
     if (!GROUPED)
       pdl_wait(); // only this thread reads what the kernel before wrote
-    for (int b = 0; b < ROWS_STAGES - 1 && b < nb; ++b)
+    for (int b = 0; b < STAGES - 1 && b < nb; ++b)
       fetch_act(b);
   }
   float acc[NT][4], accm[QT == NNTR_Q4_K ? NT : 1][4];
@@ -524,16 +523,16 @@ __global__ void __launch_bounds__(ROWS_WARPS * 32, NT == 4 ? 3 : 4) gemm_mma_row
   bool ok = true;
   for (int b = 0; b < nb; ++b) {
     // refill the slot that unit b - 1 left, then wait for this unit's own data
-    if (tid == 0 && b + ROWS_STAGES - 1 < nb) {
+    if (tid == 0 && b + STAGES - 1 < nb) {
       if (b > 0)
-        ok = wait(empty0 + 8 * ((b - 1) % ROWS_STAGES), (b - 1) / ROWS_STAGES);
+        ok = wait(empty0 + 8 * ((b - 1) % STAGES), (b - 1) / STAGES);
       if (ok) {
-        fetch_w(b + ROWS_STAGES - 1);
-        fetch_act(b + ROWS_STAGES - 1);
+        fetch_w(b + STAGES - 1);
+        fetch_act(b + STAGES - 1);
       }
     }
-    const int s = b % ROWS_STAGES;
-    ok = ok && wait(full0 + 8 * s, b / ROWS_STAGES);
+    const int s = b % STAGES;
+    ok = ok && wait(full0 + 8 * s, b / STAGES);
     if (!(ok = __all_sync(FULL, ok)))
       break;
     const uint8_t *act = sh.act[s];
@@ -834,7 +833,7 @@ cudaError_t launch(void (*kernel)(KArgs...), dim3 grid, unsigned block, size_t s
 }
 
 template <int QT, int NT, bool GROUPED, bool TH8>
-int run_tiles(const MmaArgs &a, unsigned tiles, unsigned z, bool ksplit, cudaStream_t st) {
+int run_tiles(const MmaArgs &a, unsigned tiles, unsigned z, bool ksplit, bool shallow, cudaStream_t st) {
   const unsigned row_tiles = (unsigned)((a.N + 15) / 16);
   static bool attr_set[64] = {};
   int dev = 0;
@@ -842,14 +841,22 @@ int run_tiles(const MmaArgs &a, unsigned tiles, unsigned z, bool ksplit, cudaStr
   if (dev < 64 && !attr_set[dev]) {
     NNTR_CHECK_CUDA(cudaFuncSetAttribute(gemm_mma_ksplit_kernel<QT, NT, GROUPED, TH8>,
                                          cudaFuncAttributeMaxDynamicSharedMemorySize, KS_SMEM));
-    NNTR_CHECK_CUDA(cudaFuncSetAttribute(gemm_mma_rows_kernel<QT, NT, GROUPED, TH8>,
-                                         cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(RowsShared<NT>)));
+    NNTR_CHECK_CUDA(cudaFuncSetAttribute(gemm_mma_rows_kernel<QT, NT, GROUPED, TH8, 3>,
+                                         cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(RowsShared<NT, 3>)));
     attr_set[dev] = true;
   }
-  const cudaError_t e =
-    ksplit ? launch(gemm_mma_ksplit_kernel<QT, NT, GROUPED, TH8>, dim3(tiles, row_tiles, z), KS_WARPS * 32, KS_SMEM, st, a)
-           : launch(gemm_mma_rows_kernel<QT, NT, GROUPED, TH8>, dim3(tiles, (row_tiles + ROWS_WARPS - 1) / ROWS_WARPS, z),
-                    ROWS_WARPS * 32, sizeof(RowsShared<NT>), st, a);
+  const dim3 rows_grid(tiles, (row_tiles + ROWS_WARPS - 1) / ROWS_WARPS, z);
+  cudaError_t e;
+  if (ksplit) {
+    e = launch(gemm_mma_ksplit_kernel<QT, NT, GROUPED, TH8>, dim3(tiles, row_tiles, z), KS_WARPS * 32, KS_SMEM, st, a);
+  } else {
+    auto kernel = gemm_mma_rows_kernel<QT, NT, GROUPED, TH8, 3>;
+    size_t smem = sizeof(RowsShared<NT, 3>);
+    if constexpr (QT == NNTR_Q4_0 && NT == 1 && GROUPED) // 23 KB: no opt-in
+      if (shallow)
+        kernel = gemm_mma_rows_kernel<QT, NT, GROUPED, TH8, 2>, smem = sizeof(RowsShared<NT, 2>);
+    e = launch(kernel, rows_grid, ROWS_WARPS * 32, smem, st, a);
+  }
   count_launch();
   return check_cuda(e, "gemm (integer warp MMA) launch");
 }
@@ -886,11 +893,11 @@ int launch_gemm_mma(int qtype, unsigned M, unsigned M4, unsigned N, unsigned K, 
   // a warp per 16 x 8nt tile fills the machine from about 8 warps per SM up; below, the warps of a CTA share the tile
   const bool ksplit = (uint64_t)tiles * ((N + 15) / 16) < 8u * (unsigned)sm_count();
   if (a.th < 8)
-    return run_tiles<NNTR_Q4_K, 1, false, false>(a, tiles, 1, ksplit, st);
+    return run_tiles<NNTR_Q4_K, 1, false, false>(a, tiles, 1, ksplit, false, st);
 #define NNTR_MMA_RUN(QT)                                                                                               \
-  (nt == 1   ? run_tiles<QT, 1, false, true>(a, tiles, 1, ksplit, st)                                                  \
-   : nt == 2 ? run_tiles<QT, 2, false, true>(a, tiles, 1, ksplit, st)                                                  \
-             : run_tiles<QT, 4, false, true>(a, tiles, 1, ksplit, st))
+  (nt == 1   ? run_tiles<QT, 1, false, true>(a, tiles, 1, ksplit, false, st)                                                  \
+   : nt == 2 ? run_tiles<QT, 2, false, true>(a, tiles, 1, ksplit, false, st)                                                  \
+             : run_tiles<QT, 4, false, true>(a, tiles, 1, ksplit, false, st))
   return qtype == NNTR_Q4_K ? NNTR_MMA_RUN(NNTR_Q4_K) : NNTR_MMA_RUN(NNTR_Q4_0);
 #undef NNTR_MMA_RUN
 }
@@ -940,10 +947,14 @@ int launch_gemm_grouped(int qtype, unsigned N, unsigned K, const void *act, floa
   const unsigned tiles = pairs < pairs / tile_rows + n_experts ? pairs : pairs / tile_rows + n_experts;
   const unsigned z = w_table1 ? 2 : 1;
   const bool ksplit = (uint64_t)tiles * z * ((N + 15) / 16) < 8u * (unsigned)sm_count();
+  // Q4_0's small tile: 55 registers, so shared memory sets the CTAs per SM, six with three units in flight and nine with two.
+  // From a pair per expert up the grid is two and more waves of six, and nine win: 4 of 32 experts of 2880 x 2880, 8 tokens
+  // 107 -> 100 us; 5 tokens (a wave and a half) 87.7 -> 89.3, so those keep three. Q4_K's tile is held to five by registers.
+  const bool shallow = pairs >= (unsigned)n_experts;
 #define NNTR_MMA_RUN(QT)                                                                                               \
-  (tile_rows == 8    ? run_tiles<QT, 1, true, true>(a, tiles, z, ksplit, st)                                           \
-   : tile_rows == 16 ? run_tiles<QT, 2, true, true>(a, tiles, z, ksplit, st)                                           \
-                     : run_tiles<QT, 4, true, true>(a, tiles, z, ksplit, st))
+  (tile_rows == 8    ? run_tiles<QT, 1, true, true>(a, tiles, z, ksplit, shallow, st)                                           \
+   : tile_rows == 16 ? run_tiles<QT, 2, true, true>(a, tiles, z, ksplit, shallow, st)                                           \
+                     : run_tiles<QT, 4, true, true>(a, tiles, z, ksplit, shallow, st))
   if (qtype == NNTR_Q4_K)
     return NNTR_MMA_RUN(NNTR_Q4_K);
   if (qtype == NNTR_Q4_0)

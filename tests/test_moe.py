@@ -341,6 +341,27 @@ def test_a_batch_equals_its_tokens_one_by_one_around_the_grouping_lines(be, q, T
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("T", [7, 8, 48])
+def test_q4_0_experts_by_tile_per_warp_equal_one_by_one_around_a_pair_per_expert(be, T):
+    """4 of 32 experts: below 32 pairs the warp-tile kernel keeps three units in flight, from there two, up to the last batch
+    of 8-row tiles (192 pairs). 704 and 352 wide: enough tiles for that kernel, K of three and two units with short last
+    ones, a last CTA with half its row groups. Every row keeps its float chain, so the bits agree."""
+    import torch
+    rng = np.random.default_rng(T)
+    H, I, E, k = 704, 352, 32, 4
+    experts = lambda n, m: [torch.from_numpy(O.random_q4_0x8(rng, n, m)).cuda() for _ in range(4)] * (E // 4)
+    bias = lambda n: [torch.randn(n, device="cuda") for _ in range(E)]
+    router = torch.from_numpy((rng.standard_normal((H, E)) * 0.02).astype(np.float32)).cuda()
+    layer = be.MoeLayer(router, experts(I, H), experts(I, H), experts(H, I), k, qtype="q4_0", kind=1, alpha=1.702,
+                        router_bias=torch.zeros(E, device="cuda"), gate_b=bias(I), up_b=bias(I), down_b=bias(H))
+    x = torch.from_numpy(rng.standard_normal((T, H)).astype(np.float32)).cuda()
+    got = layer.forward(x).clone()
+    single = torch.cat([layer.forward(x[i:i + 1].contiguous()).clone() for i in range(T)])
+    be.device_status()
+    assert torch.equal(got.view(torch.int32), single.view(torch.int32))
+
+
+@pytest.mark.gpu
 @pytest.mark.parametrize("T,H,I,E,k", [(8, 512, 256, 16, 4), (37, 512, 256, 16, 4), (256, 2048, 768, 128, 8)])
 def test_grouped_prefill_equals_the_per_pair_path_bit_for_bit(be, port, T, H, I, E, k):
     """From 8 tokens on the layer sorts the (token, expert) pairs by expert and runs per-expert grouped GEMMs with a
