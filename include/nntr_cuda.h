@@ -317,10 +317,11 @@ int nntr_cuda_attention_step_dev(const nntr_attn_desc *a, unsigned pos, const un
 
 /** nntr_cuda_attention_step_dev for `tokens` consecutive tokens from position pos on, in two launches: token i's heads are at
  *  q, k, v + i * ld, its result goes to out + i * ld_out; q is rotated in place; all rows are appended to the caches. Same
- *  bits as that many steps. Heads of up to 128 dimensions, windows of up to 16384 rows. */
-int nntr_cuda_attention_rows_dev(const nntr_attn_desc *a, unsigned pos, unsigned tokens, float *q, const float *k,
-                                 const float *v, size_t ld, const float *q_gamma, const float *k_gamma, float eps,
-                                 void *kcache, void *vcache, const float *cos_tab, const float *sin_tab, float *out,
+ *  bits as that many steps. max_rows: rows that the caches and the rotary tables hold; tokens that would end behind them are
+ *  refused before anything is launched. Heads of up to 128 dimensions, windows of up to 16384 rows. */
+int nntr_cuda_attention_rows_dev(const nntr_attn_desc *a, unsigned pos, unsigned tokens, unsigned max_rows, float *q,
+                                 const float *k, const float *v, size_t ld, const float *q_gamma, const float *k_gamma,
+                                 float eps, void *kcache, void *vcache, const float *cos_tab, const float *sin_tab, float *out,
                                  size_t ld_out, unsigned flags, void *stream);
 
 /* ------------------------------------------------------- .bin weight files */

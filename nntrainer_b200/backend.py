@@ -558,10 +558,10 @@ class Attention:
 
     def rows(self, q, k, v, ld: int, pos: int, tokens: int, out, ld_out: int, qk_norm=None, pdl: bool = False):
         """``step`` for ``tokens`` consecutive tokens from ``pos`` on: token i's heads at element i * ld of q, k and v (q is
-        rotated in place), its result at element i * ld_out of out."""
+        rotated in place), its result at element i * ld_out of out. Tokens behind row ``max_seq`` are refused."""
         qg, kg, eps = qk_norm if qk_norm is not None else (None, None, 0.0)
         check(lib().nntr_cuda_attention_rows_dev(
-            self._C.byref(self.desc), pos, tokens, q.data_ptr(), k.data_ptr(), v.data_ptr(), ld,
+            self._C.byref(self.desc), pos, tokens, self.max_seq, q.data_ptr(), k.data_ptr(), v.data_ptr(), ld,
             qg.data_ptr() if qg is not None else None, kg.data_ptr() if kg is not None else None, eps,
             self.kcache.data_ptr(), self.vcache.data_ptr(), self.cos.data_ptr(), self.sin.data_ptr(), out.data_ptr(), ld_out,
             _flags(pdl), _stream()))

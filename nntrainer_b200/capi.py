@@ -55,7 +55,7 @@ SIGNATURES = {
     "nntr_cuda_attention_decode_dev": (_i, [_vp, _u, _vp, _u, _vp, _vp, _vp, _vp, _vp, _sz, _u, _vp]),
     "nntr_cuda_attention_step_dev": (_i, [_vp, _u, _vp, _u, _vp, _vp, _vp, _vp, _vp, C.c_float, _vp, _vp, _vp, _vp, _vp, _vp,
                                           _vp, _sz, _u, _vp]),
-    "nntr_cuda_attention_rows_dev": (_i, [_vp, _u, _u, _vp, _vp, _vp, _sz, _vp, _vp, C.c_float, _vp, _vp, _vp, _vp, _vp, _sz,
+    "nntr_cuda_attention_rows_dev": (_i, [_vp, _u, _u, _u, _vp, _vp, _vp, _sz, _vp, _vp, C.c_float, _vp, _vp, _vp, _vp, _vp, _sz,
                                           _u, _vp]),
     "nntr_cuda_bin_layout": (_i, [_vp, _sz, _vp, _vp, _vp]),
     "nntr_cuda_bin_load": (_i, [C.c_char_p, _vp, _sz, _i, _i, _vp, _vp]),

@@ -1165,8 +1165,8 @@ int launch_attention_step(const nntr_attn_desc *a, unsigned pos, const unsigned 
 
 /* Consecutive tokens of a prompt: every token's rotary work and cache rows in one launch, every token's attention -- over its own
  * row and the rows before it -- in a second one. The same kernels as a decode step's, so the same bits as that many steps. */
-int launch_attention_rows(const nntr_attn_desc *a, unsigned pos, unsigned tokens, float *q, const float *k, const float *v,
-                          size_t ld, const float *q_gamma, const float *k_gamma, float eps, uint16_t *kcache, uint16_t *vcache,
+int launch_attention_rows(const nntr_attn_desc *a, unsigned pos, unsigned tokens, unsigned max_rows, float *q, const float *k,
+                          const float *v, size_t ld, const float *q_gamma, const float *k_gamma, float eps, uint16_t *kcache, uint16_t *vcache,
                           const float *cos_tab, const float *sin_tab, float *out, size_t ld_out, unsigned flags,
                           cudaStream_t st) {
   int rc = check_attn(a);
@@ -1180,6 +1180,9 @@ int launch_attention_rows(const nntr_attn_desc *a, unsigned pos, unsigned tokens
     return set_error(NNTR_CUDA_ERR_INVALID, "attention_rows: caches must be 16-byte aligned");
   if (tokens == 0)
     return NNTR_CUDA_OK;
+  if ((unsigned long long)pos + tokens > max_rows)
+    return set_error(NNTR_CUDA_ERR_INVALID, "attention_rows: positions %u to %llu beyond the %u rows allowed", pos,
+                     (unsigned long long)pos + tokens - 1, max_rows);
   const unsigned bound = pos + tokens, rows = bound < a->window ? bound : a->window;
   if (tokens > 65535 || a->head_dim > 128 || rows > AC_MAX_ROWS)
     return set_error(NNTR_CUDA_ERR_UNSUPPORTED, "attention_rows: heads of at most 128 dimensions, windows of at most %u rows",

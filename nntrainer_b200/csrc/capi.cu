@@ -640,11 +640,11 @@ int nntr_cuda_attention_step_dev(const nntr_attn_desc *a, unsigned pos, const un
                                static_cast<cudaStream_t>(stream));
 }
 
-int nntr_cuda_attention_rows_dev(const nntr_attn_desc *a, unsigned pos, unsigned tokens, float *q, const float *k,
-                                 const float *v, size_t ld, const float *q_gamma, const float *k_gamma, float eps,
+int nntr_cuda_attention_rows_dev(const nntr_attn_desc *a, unsigned pos, unsigned tokens, unsigned max_rows, float *q,
+                                 const float *k, const float *v, size_t ld, const float *q_gamma, const float *k_gamma, float eps,
                                  void *kcache, void *vcache, const float *cos_tab, const float *sin_tab, float *out,
                                  size_t ld_out, unsigned flags, void *stream) {
-  return launch_attention_rows(a, pos, tokens, q, k, v, ld, q_gamma, k_gamma, eps, static_cast<uint16_t *>(kcache),
+  return launch_attention_rows(a, pos, tokens, max_rows, q, k, v, ld, q_gamma, k_gamma, eps, static_cast<uint16_t *>(kcache),
                                static_cast<uint16_t *>(vcache), cos_tab, sin_tab, out, ld_out, flags,
                                static_cast<cudaStream_t>(stream));
 }

@@ -386,8 +386,8 @@ int launch_attention_step(const nntr_attn_desc *a, unsigned pos, const unsigned 
                           const float *k, const float *v, const float *q_gamma, const float *k_gamma, float eps,
                           uint16_t *kcache, uint16_t *vcache, const float *cos_tab, const float *sin_tab, float *q_rot,
                           float *out, void *ws, size_t ws_bytes, unsigned flags, cudaStream_t st);
-int launch_attention_rows(const nntr_attn_desc *a, unsigned pos, unsigned tokens, float *q, const float *k, const float *v,
-                          size_t ld, const float *q_gamma, const float *k_gamma, float eps, uint16_t *kcache, uint16_t *vcache,
+int launch_attention_rows(const nntr_attn_desc *a, unsigned pos, unsigned tokens, unsigned max_rows, float *q, const float *k,
+                          const float *v, size_t ld, const float *q_gamma, const float *k_gamma, float eps, uint16_t *kcache, uint16_t *vcache,
                           const float *cos_tab, const float *sin_tab, float *out, size_t ld_out, unsigned flags,
                           cudaStream_t st);
 /* host side (model_file.cu) */

@@ -322,9 +322,11 @@ class Qwen3Decoder:
         """Feeds the prompt, then ``n_new`` greedy tokens; returns them as a Python list. All of the prompt but its last token
         goes through the layers in batched passes (where their kernels apply: heads of up to 128 dimensions, hidden rows of
         up to 11264, up to 16384 positions), with the results of feeding it token by token; the token ids stay on the device until
-        the end."""
+        the end. A prompt of more than ``max_seq`` tokens is a ValueError."""
         torch, c = self.torch, self.cfg
         prompt_ids = list(prompt_ids)
+        if len(prompt_ids) > c.max_seq:  # nothing is fed then
+            raise ValueError(f"a prompt of {len(prompt_ids)} tokens does not fit the {c.max_seq} rows of the caches")
         tok = torch.empty(1, dtype=torch.float32, device=self.dev)
         out = torch.empty(n_new + 1, dtype=torch.int32, device=self.dev)
         pos = 0
