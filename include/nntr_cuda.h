@@ -142,7 +142,10 @@ int nntr_cuda_measure_int8_peak(double *tops, double *clk_per_mma);
  *  ldc is the row stride of C. M == 1 runs the decode GEMV (activation
  *  quantized inside the kernel, no workspace needed); M > 1 quantizes A into
  *  `workspace` first. K % 256 == 0 (Q4_K, Q6_K) or K % 32 == 0 (Q4_0);
- *  N % 8 == 0 (Q4_0, Q4_K). */
+ *  N % 8 == 0 (Q4_0, Q4_K).
+ *  A, workspace: 16-byte aligned. B: 16-byte aligned for Q4_K and Q4_0 (Q6_K: 2).
+ *  B at a multiple of 8 is taken too, except by the Q4_K GEMV (M == 1), but only
+ *  by the exact kernels that need no 16-byte copies; anything less is refused. */
 int nntr_cuda_gemm_q4_K_dev(unsigned M, unsigned N, unsigned K, const float *A, unsigned lda, const void *B,
                             unsigned ldb, float *C, unsigned ldc, void *workspace, size_t workspace_bytes,
                             void *stream);
@@ -418,6 +421,7 @@ typedef struct {
   unsigned top_k;            /* experts per token */
   const float *router_w;     /* fp32 [H][E], as the reference stores the gate weight */
   const float *router_bias;  /* fp32 [E] or NULL */
+  /* the experts' weights are 16-byte aligned */
   const void *const *gate_w; /* E pointers: gate projection, quantized [I][H] */
   const void *const *up_w;   /* E pointers: up projection, quantized [I][H] */
   const void *const *down_w; /* E pointers: down projection, quantized [H][I] */

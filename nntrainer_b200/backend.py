@@ -340,6 +340,10 @@ class MoeLayer:
         first = next(w for w in gate_w if w is not None)  # experts of other ranks are None under expert parallelism
         self.I = first.numel() * _BLOCK[qtype][0] // _BLOCK[qtype][1] // self.H
         self.top_k = top_k
+        # the kernels fetch the weights by 16-byte copies: a tensor that does not start at such an address (a slice of
+        # something else) is copied to one that does
+        gate_w, up_w, down_w = ([w.clone() if w is not None and w.data_ptr() % 16 else w for w in ws]
+                                for ws in (gate_w, up_w, down_w))
         self._keep = [router_w, gate_w, up_w, down_w, router_bias, gate_b, up_b, down_b]
         dev = router_w.device
 

@@ -151,6 +151,15 @@ static int check_weight_shape(int qtype, unsigned N, unsigned K) {
   }
 }
 
+/** The exact kernels read Q4_K and Q4_0 weights in pieces of up to 8 bytes, Q6_K blocks in pieces of 2; everything that fetches
+ *  them by 16-byte copies is left to weights that are aligned for it. */
+static int check_weight_alignment(int qtype, const void *B) {
+  const unsigned align = qtype == NNTR_Q6_K ? 2 : 8;
+  if (reinterpret_cast<uintptr_t>(B) & (align - 1))
+    return set_error(NNTR_CUDA_ERR_INVALID, "weights must be %u-byte aligned", align);
+  return NNTR_CUDA_OK;
+}
+
 /* ------------------------------------------------- per-thread host staging */
 struct ThreadCtx {
   cudaStream_t stream = nullptr;
@@ -319,6 +328,8 @@ static int gemm_dev(int qtype, unsigned M, unsigned N, unsigned K, const float *
     return NNTR_CUDA_OK;
   if (!A || !B || !C)
     return set_error(NNTR_CUDA_ERR_INVALID, "gemm: null pointer");
+  if ((rc = check_weight_alignment(qtype, B)))
+    return rc;
   if (M == 1) {
     switch (qtype) {
     case NNTR_Q4_K:
@@ -339,7 +350,9 @@ static int gemm_dev(int qtype, unsigned M, unsigned N, unsigned K, const float *
   /* Rows below 4*floor(M/4) are quantized the way the reference's 4-row
    * quantizer does it, the last M%4 rows the way its row quantizer does
    * (ggml_interface_omp.cpp:433-461). */
-  switch (pick_gemm_kernel(qtype, M, N, K)) {
+  // the tensor paths bring Q4_K and Q4_0 weights in by 16-byte copies
+  const bool copies = qtype == NNTR_Q6_K || !(reinterpret_cast<uintptr_t>(B) & 15);
+  switch (copies ? pick_gemm_kernel(qtype, M, N, K) : 0) {
   case 1:
     return launch_gemm_q4_K_umma(M, N, K, A, B, C, ldc, ws, st);
   case 2:
@@ -728,6 +741,8 @@ int nntr_cuda_gemv_rows_dev(int qtype, unsigned M, unsigned N, unsigned K, const
     return NNTR_CUDA_OK;
   if (!A || !B || !C)
     return set_error(NNTR_CUDA_ERR_INVALID, "gemv_rows: null pointer");
+  if ((rc = check_weight_alignment(qtype, B)))
+    return rc;
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   if (M == 1)
     return nntr_cuda_gemv_dev(qtype, N, K, A, B, C, 0, stream);

@@ -471,6 +471,11 @@ __global__ void __launch_bounds__(ROWS_WARPS * 32, NT == 4 ? 3 : 4) gemm_mma_row
     pdl_wait(); // tables and activation tiles come from the kernels before
   if (!find_tile<NT>(tl, a, blockIdx.x, GROUPED))
     return;
+  if (GROUPED && (reinterpret_cast<uintptr_t>(tl.W) & 15)) { // from a table in device memory: not seen by the launcher
+    if (tid == 0)
+      atomicExch(&g_mma_status, NNTR_CUDA_ERR_INVALID);
+    return;
+  }
   const int nt = (tl.rows + 7) >> 3, th = TH8 ? 8 : a.th;
   volatile int *abort_flag = &sh.abort_flag;
   const uint32_t full0 = smem_u32(sh.full), empty0 = smem_u32(sh.empty);
@@ -871,6 +876,8 @@ int launch_gemm_mma(int qtype, unsigned M, unsigned M4, unsigned N, unsigned K, 
                     unsigned ldc, void *ws, size_t ws_bytes, cudaStream_t st) {
   if ((reinterpret_cast<uintptr_t>(A) & 15) || (reinterpret_cast<uintptr_t>(ws) & 15))
     return set_error(NNTR_CUDA_ERR_INVALID, "gemm: activations and workspace must be 16-byte aligned");
+  if (reinterpret_cast<uintptr_t>(B) & 7)
+    return set_error(NNTR_CUDA_ERR_INVALID, "gemm: weights must be 8-byte aligned");
   MmaArgs a = {};
   a.act = static_cast<const uint8_t *>(ws);
   a.W = B;
@@ -890,8 +897,9 @@ int launch_gemm_mma(int qtype, unsigned M, unsigned M4, unsigned N, unsigned K, 
   NNTR_CHECK_CUDA(cudaGetLastError());
   const int nt = M <= 8 ? 1 : M <= 16 ? 2 : 4;
   const unsigned tiles = (M + 8 * nt - 1) / (8 * nt);
-  // a warp per 16 x 8nt tile fills the machine from about 8 warps per SM up; below, the warps of a CTA share the tile
-  const bool ksplit = (uint64_t)tiles * ((N + 15) / 16) < 8u * (unsigned)sm_count();
+  // a warp per 16 x 8nt tile fills the machine from about 8 warps per SM up; below, the warps of a CTA share the tile. Weights
+  // that are not 16-byte aligned cannot be fetched by bulk copies: the shared tile's loads of at most 8 bytes take them all.
+  const bool ksplit = (uint64_t)tiles * ((N + 15) / 16) < 8u * (unsigned)sm_count() || (reinterpret_cast<uintptr_t>(B) & 15);
   if (a.th < 8)
     return run_tiles<NNTR_Q4_K, 1, false, false>(a, tiles, 1, ksplit, false, st);
 #define NNTR_MMA_RUN(QT)                                                                                               \

@@ -227,7 +227,7 @@ int launch_gemv_q4_0(unsigned N, unsigned K, const float *x, const void *B, floa
   }();
   if (!stream_off && x && B && y && N && !(reinterpret_cast<uintptr_t>(B) & 15) && gemv_q4_0_stream_supported(N, K))
     return launch_gemv_q4_0_stream(N, K, x, B, y, flags, st);
-  if (!x || !B || !y || (reinterpret_cast<uintptr_t>(x) & 15))
+  if (!x || !B || !y || (reinterpret_cast<uintptr_t>(x) & 15) || (reinterpret_cast<uintptr_t>(B) & 7))
     return set_error(NNTR_CUDA_ERR_INVALID, "gemv_q4_0: null or misaligned pointer");
   if (N == 0)
     return NNTR_CUDA_OK;

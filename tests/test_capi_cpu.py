@@ -59,6 +59,21 @@ def test_no_device_means_error_not_fallback(L):
         capi.check(rc)
 
 
+@pytest.mark.parametrize("q,off", [("q4_K", 4), ("q4_K", 1), ("q4_0", 4), ("q4_0", 2), ("q6_K", 1)])
+@pytest.mark.parametrize("M", [1, 2, 1024])
+def test_misaligned_weights_are_refused_before_anything_is_launched(L, q, off, M):
+    """Weights at an address that the kernels' loads cannot take (they would fault); multiples of 8 (Q6_K: 2) are taken."""
+    N, K, p = 4096, 4096, 1 << 20
+    qt = capi.QTYPE[q]
+    need = L.nntr_cuda_gemm_workspace_bytes(qt, M, N, K)
+    before = L.nntr_cuda_launch_count()
+    fn = getattr(L, f"nntr_cuda_gemm_{q}_dev")
+    assert fn(M, N, K, p, K, p + off, N, p, N, p, need, None) == capi.ERR_INVALID
+    assert L.nntr_cuda_gemv_rows_dev(qt, M, N, K, p, p + off, p, N, p, need, None) == capi.ERR_INVALID
+    assert L.nntr_cuda_gemv_dev(qt, N, K, p, p + off, p, 0, None) == capi.ERR_INVALID
+    assert L.nntr_cuda_launch_count() == before
+
+
 def test_workspace_sizes(L):
     assert L.nntr_cuda_gemm_workspace_bytes(capi.Q4_K, 1, 4096, 4096) == 0
     # N % 256 == 0: room for the fp16 tensor path's activation tiles (128 rows x K halves)

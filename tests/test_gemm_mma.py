@@ -89,3 +89,21 @@ def test_largest_sums(be, port, M):
     A[M - 1, 256:] *= -1
     want = port.gemm("q4_K", A, B, N)
     assert np.array_equal(exact(be, "q4_K", A, B, N).view(np.uint32), want.view(np.uint32))
+
+
+@pytest.mark.parametrize("path", ["exact", "auto", "tensor", "tensor_f16"])
+@pytest.mark.parametrize("M,N,K", [(7, 24, 768), (37, 19072, 768), (256, 1024, 512)])
+@pytest.mark.parametrize("q,gen", [("q4_K", O.random_q4_Kx8), ("q4_0", O.random_q4_0x8)])
+def test_weights_at_a_multiple_of_eight_bytes(be, port, q, gen, M, N, K, path):
+    """No 16-byte copy may start there: every path gives the exact kernels' bits."""
+    rng = np.random.default_rng(M + N + K)
+    A = rng.standard_normal((M, K)).astype(np.float32)
+    B = gen(rng, N, K)
+    at8 = torch.zeros(B.nbytes + 16, dtype=torch.uint8, device="cuda")[8:8 + B.nbytes]
+    at8.copy_(torch.from_numpy(B.view(np.uint8).reshape(-1)))
+    assert at8.data_ptr() % 16 == 8
+    C = torch.full((M, N), float("nan"), device="cuda")
+    be.set_gemm_path(path)
+    getattr(be, f"gemm_{q}")(M, N, K, torch.from_numpy(A).cuda(), K, at8, N, C, N)
+    be.device_status()
+    assert np.array_equal(C.cpu().numpy().view(np.uint32), port.gemm(q, A, B, N).view(np.uint32))

@@ -20,6 +20,23 @@ def make_layer(rng, H, I, E, distinct=None):
 
 
 # ------------------------------------------------------------------ CPU
+def test_expert_weights_that_start_off_a_16_byte_boundary_are_copied_to_one():
+    """The tables that the kernels read may hold 16-byte aligned addresses only."""
+    torch = pytest.importorskip("torch")
+    from nntrainer_b200 import backend
+    H = I = 256
+    n = I * H // 256 * 144
+    store = torch.arange(3 * (n + 8), dtype=torch.uint8)
+    ws = [store[i * (n + 8):i * (n + 8) + n] for i in range(3)]
+    assert [w.data_ptr() % 16 for w in ws] == [0, 8, 0]
+    L = backend.MoeLayer(torch.zeros(H, 3), ws, [ws[0], None, ws[1]], ws, 1)
+    assert L._tabs[0][0] == ws[0].data_ptr() and L._tabs[1][1] == 0
+    for tab, kept in zip(L._tabs[:3], L._keep[1:4]):
+        assert all(int(p) % 16 == 0 for p in tab)
+        assert [int(p) for p in tab] == [k.data_ptr() if k is not None else 0 for k in kept]
+    assert torch.equal(L._keep[1][1], ws[1]) and torch.equal(L._keep[2][2], ws[1])
+
+
 def test_route_restatement_properties(port):
     rng = np.random.default_rng(0)
     T, H, E, k = 7, 256, 32, 4
