@@ -438,7 +438,8 @@ size_t nntr_cuda_moe_workspace_bytes(const nntr_moe_desc *d, unsigned tokens);
  *  (qwen_moe_layer.cpp:394-503) / GptOssMoELayer (gpt_oss_moe_layer.cpp:457-572)
  *  for one batch element: router, softmax, top-k, renormalise, per-(token,
  *  expert) gate/up/down GEMVs with M == 1 as the reference runs them, combine
- *  in ascending expert order. Device pointers; workspace 256-byte aligned. */
+ *  in ascending expert order. Device pointers; x 16-byte, workspace 256-byte
+ *  aligned. */
 int nntr_cuda_moe_forward_dev(const nntr_moe_desc *d, unsigned tokens, const float *x, float *y, void *workspace,
                               size_t workspace_bytes, void *stream);
 /** Routing step alone (qwen_moe_layer.cpp:439-446): expert indices [tokens][top_k]

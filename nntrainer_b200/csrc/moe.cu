@@ -750,6 +750,8 @@ static int moe_forward(const nntr_moe_desc *d, const nntr_moe_ep *epd, unsigned 
     return set_error(NNTR_CUDA_ERR_INVALID, "moe_forward: null weight table");
   if (tokens == 0)
     return NNTR_CUDA_OK;
+  if (reinterpret_cast<uintptr_t>(x) & 15) // read by 16-byte loads on both sides of the grouping line
+    return set_error(NNTR_CUDA_ERR_INVALID, "moe_forward: x must be 16-byte aligned");
   MoeEp ep = {};
   int e_lo = 0, e_hi = (int)E;
   if (epd) {

@@ -74,6 +74,19 @@ def test_misaligned_weights_are_refused_before_anything_is_launched(L, q, off, M
     assert L.nntr_cuda_launch_count() == before
 
 
+@pytest.mark.parametrize("qtype,kind", [("q4_K", 0), ("q4_0", 1)])
+@pytest.mark.parametrize("tokens", [1, 7, 64, 400])
+def test_moe_tokens_off_a_16_byte_boundary_are_refused_before_anything_is_launched(L, qtype, kind, tokens):
+    """Few tokens go through a GEMV per pair, many through grouped GEMMs: both read x by 16-byte loads."""
+    p = 1 << 20
+    d = capi.MoeDesc(kind, capi.QTYPE[qtype], 2048, 768, 64, 8, p, None, p, p, p, p, p, p, 1.0)
+    need = L.nntr_cuda_moe_workspace_bytes(ctypes.byref(d), tokens)
+    before = L.nntr_cuda_launch_count()
+    for off in (4, 8):
+        assert L.nntr_cuda_moe_forward_dev(ctypes.byref(d), tokens, p + off, p, p, need, None) == capi.ERR_INVALID
+    assert L.nntr_cuda_launch_count() == before
+
+
 def test_workspace_sizes(L):
     assert L.nntr_cuda_gemm_workspace_bytes(capi.Q4_K, 1, 4096, 4096) == 0
     # N % 256 == 0: room for the fp16 tensor path's activation tiles (128 rows x K halves)
