@@ -185,7 +185,8 @@ __device__ __forceinline__ void router_finish(const RouterOut &o, int t, int E, 
   // "probability greater" (nntrainer/tensor/float_tensor.cpp:1155-1160). With distinct values that is plain descending
   // order: k (+1) rounds of a warp arg-max. Among EQUAL probabilities the library's order comes from its heap moves,
   // so when a tie touches the selection (two equal values among the k + 1 greatest) one lane reruns the selection
-  // with the library's own procedure.
+  // with the library's own procedure. The same where a logit was not a number: then no probability is one, none compares
+  // greater, and the library's procedure still names k experts.
   float *pv = area; // the probabilities, expert-indexed
   __syncwarp();
 #pragma unroll
@@ -223,7 +224,7 @@ __device__ __forceinline__ void router_finish(const RouterOut &o, int t, int E, 
         if (i == (be >> 5))
           p[i] = -1.f;
     }
-    tie = tie || (k > 0 && bv == prev);
+    tie = tie || (k > 0 && bv == prev) || bv < 0.f; // no winner: probabilities that are not numbers
     prev = bv;
     if (k < topk && lane == 0)
       sel[k] = be;

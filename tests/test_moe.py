@@ -332,6 +332,29 @@ def test_selection_margin_is_far_above_what_the_summation_order_can_move(be, por
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("T,E,k", [(3, 1, 1), (3, 16, 4), (3, 4, 4), (64, 16, 4), (64, 200, 8)])
+def test_a_token_that_is_not_a_number_leaves_the_others_alone(be, port, T, E, k):
+    """Its probabilities are all NaN; the library's partial_sort still selects k experts, and so does the device, which
+    indexes its tables with them. Its own output is NaN, that of every other token what it is without it."""
+    import torch
+    rng = np.random.default_rng(E)
+    H, I = 512, 256
+    x = rng.standard_normal((T, H)).astype(np.float32)
+    router, gate, up, down = make_layer(rng, H, I, E, distinct=min(E, 4))
+    layer = device_layer(be, router, gate, up, down, k)
+    want = layer.forward(torch.from_numpy(x).cuda()).clone()
+    x[1, 77] = np.nan
+    xd = torch.from_numpy(x).cuda()
+    idx, _ = layer.route(xd)
+    assert np.array_equal(idx.cpu().numpy().astype(np.uint32), port.moe_route(x, router, k)[0])
+    got = layer.forward(xd)
+    be.device_status()
+    assert torch.isnan(got[1]).all()
+    others = [t for t in range(T) if t != 1]
+    assert torch.equal(got[others].view(torch.int32), want[others].view(torch.int32))
+
+
+@pytest.mark.gpu
 @pytest.mark.parametrize("q,T,E,k", [("q4_0", 3, 8, 6), ("q4_0", 4, 8, 5), ("q4_K", 2, 16, 8), ("q4_K", 12, 128, 8),
                                      ("q4_K", 13, 128, 8)])
 def test_a_batch_equals_its_tokens_one_by_one_around_the_grouping_lines(be, q, T, E, k):
