@@ -88,7 +88,7 @@ class Qwen3Decoder:
                       up=ug[:cfg.inter], gate=ug[cfg.inter:], act=f(cfg.inter), d=f(cfg.hidden), logits=f(cfg.vocab))
         self._tables()
         import ctypes as C
-        self._calls, self._call_caches = {}, []
+        self._calls, self._addressof = {}, C.addressof
         self._arg = dict(tok=C.c_void_p(), pos=C.c_uint(), pos_dev=C.c_void_p(), idx=C.c_void_p(), idx_f=C.c_void_p(),
                          stream=C.c_void_p())
 
@@ -98,10 +98,6 @@ class Qwen3Decoder:
 
         def data_ptr(self):
             return self.p
-
-    def _gemv(self, name, x, y):
-        dtype, N, K = self._shape[name]
-        be.gemv(dtype, N, K, x, self._P(self.ptr[name]), y, pdl=self.pdl)
 
     def _norm(self, x, name, out, width=None):
         be.rms_norm(x, self._P(self.ptr[name]), self.cfg.norm_eps, width=width, out=out, pdl=self.pdl)
@@ -153,12 +149,13 @@ class Qwen3Decoder:
         if out_idx_f is None:
             out_idx_f = torch.empty(1, dtype=torch.float32, device=self.dev)
         # The launches of a step differ from the next step's in five values only: they are made into a list of calls once, whose
-        # arguments are converted already and share those five. A call then costs its launch and little else.
-        key = (self.pdl, self.fuse)
-        calls = self._calls.get(key)
-        if calls is None or any(a.kcache is not k or a.vcache is not v for a, (k, v) in zip(self.attn, self._call_caches)):
-            self._call_caches = [(a.kcache, a.vcache) for a in self.attn]
-            calls = self._calls[key] = self._make_calls()
+        # arguments are converted already and share those five. A call then costs its launch and little else. A list is made
+        # again when an address in it is no longer that of the tensor it was taken from.
+        key, held = (self.pdl, self.fuse), self._held()
+        made_for, calls = self._calls.get(key, (None, None))
+        if made_for != held:
+            calls = self._make_calls()
+            self._calls[key] = held, calls
         v = self._arg
         v["tok"].value, v["pos"].value = token_f.data_ptr(), pos
         v["pos_dev"].value = pos_dev.data_ptr() if pos_dev is not None else None
@@ -169,6 +166,15 @@ class Qwen3Decoder:
             if rc:
                 be.check(rc)
         return out_idx, out_idx_f
+
+    def _held(self):
+        """The addresses (and the sizes beside them) that a list of calls holds, as they are now."""
+        held = [t.data_ptr() for ts in (self.b.values(), self._qkv_packed, self._qkv_tab, self._ug_tab) for t in ts]
+        held += self.ptr.values()
+        for a in self.attn:
+            held += (self._addressof(a.desc), a.max_seq, a.kcache.data_ptr(), a.vcache.data_ptr(), a.cos.data_ptr(),
+                     a.sin.data_ptr(), a.ws.data_ptr(), a.ws.numel())
+        return held
 
     def _make_calls(self):
         """The C calls of a decode step in order, as (function, converted arguments)."""

@@ -81,6 +81,41 @@ def test_sliding_window_shorter_than_the_context(be):
     assert np.array_equal(gl.view(np.uint32), cl.view(np.uint32))
 
 
+def test_a_replaced_cache_is_used_by_every_launch_sequence(be):
+    """The launches of a step are prepared once per launch sequence: after a layer's caches, rotary tables or an activation
+    buffer were replaced, every one of them works on the new tensors."""
+    cfg = DecoderConfig(n_layers=2, hidden=512, n_heads=8, n_kv_heads=2, head_dim=64, inter=768, vocab=1024, max_seq=32)
+    with tempfile.TemporaryDirectory() as td:
+        path = os.path.join(td, "model.bin")
+        write_bin(path, cfg, synthetic_weights(cfg, 5))
+        dec, other = Qwen3Decoder(cfg, path), Qwen3Decoder(cfg, path)
+    tok = torch.tensor([7.0], device="cuda")
+    for pdl in (True, False):  # two lists of calls, made for the first tensors
+        dec.pdl = pdl
+        dec.step(tok, 0)
+    old = [(t, t.clone()) for a in dec.attn for t in (a.kcache, a.vcache, a.ws)] + [(dec.b["h"], dec.b["h"].clone())]
+    for a in dec.attn:
+        for name in ("kcache", "vcache"):
+            setattr(a, name, torch.zeros_like(getattr(a, name)))
+        for name in ("cos", "sin", "ws"):
+            setattr(a, name, getattr(a, name).clone())
+    dec.b["h"] = torch.empty_like(dec.b["h"])
+    for pos, pdl in enumerate((True, False, True, False)):
+        dec.pdl = pdl
+        t, tf = dec.step(tok, pos)
+        w, _ = other.step(tok, pos)
+        assert int(t) == int(w)
+        assert torch.equal(dec.b["logits"].view(torch.int32), other.b["logits"].view(torch.int32))
+        tok = tf
+    be.device_status()
+    for a, b in zip(dec.attn, other.attn):
+        assert torch.equal(a.kcache, b.kcache) and torch.equal(a.vcache, b.vcache)
+    for t, was in old:
+        assert torch.equal(t, was), "a launch still used a tensor that was replaced"
+    dec.close()
+    other.close()
+
+
 @pytest.mark.parametrize("window,fc,P", [(None, "q4_K", 2), (None, "q4_K", 9), (16, "q4_K", 40), (None, "q6_K", 33),
                                          (None, "q4_K", 300)])
 def test_batched_prompt_equals_token_by_token(be, window, fc, P):
