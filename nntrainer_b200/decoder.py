@@ -328,12 +328,16 @@ class Qwen3Decoder:
         """Feeds the prompt, then ``n_new`` greedy tokens; returns them as a Python list. All of the prompt but its last token
         goes through the layers in batched passes (where their kernels apply: heads of up to 128 dimensions, hidden rows of
         up to 11264, up to 16384 positions), with the results of feeding it token by token; the token ids stay on the device until
-        the end. A prompt of more than ``max_seq`` tokens is a ValueError."""
+        the end. An empty prompt and one of more than ``max_seq`` tokens are ValueErrors; no new tokens (0 or
+        less) only feed the prompt."""
         torch, c = self.torch, self.cfg
         prompt_ids = list(prompt_ids)
+        if not prompt_ids and n_new > 0:
+            raise ValueError("generate: an empty prompt leaves nothing to continue")
         if len(prompt_ids) > c.max_seq:  # nothing is fed then
             raise ValueError(f"a prompt of {len(prompt_ids)} tokens does not fit the {c.max_seq} rows of the caches")
         tok = torch.empty(1, dtype=torch.float32, device=self.dev)
+        n_new = max(n_new, 0)
         out = torch.empty(n_new + 1, dtype=torch.int32, device=self.dev)
         pos = 0
         if len(prompt_ids) > 3 and c.head_dim <= 128 and c.hidden <= 11264 and c.max_seq <= 16384:

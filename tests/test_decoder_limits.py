@@ -51,3 +51,19 @@ def test_a_prompt_that_fills_the_caches_is_fed():
     d = _decoder(CFG)
     d.generate([1] * 64, 0)
     assert d.fed == [("rows", 0, 63), ("step", 63, 1)]
+
+
+@pytest.mark.parametrize("n_new", [1, 5])
+def test_an_empty_prompt_is_refused(n_new):
+    """There is no token to start from: nothing may be decoded from an uninitialised one."""
+    d = _decoder(CFG)
+    with pytest.raises(ValueError):
+        d.generate([], n_new)
+    assert d.fed == []
+
+
+@pytest.mark.parametrize("prompt,n_new", [([], 0), ([], -1), ([3], 0), ([3], -1), ([3, 4], -7), ([1] * 8, -2)])
+def test_no_new_tokens_feed_the_prompt_only(prompt, n_new):
+    d = _decoder(CFG)
+    assert d.generate(prompt, n_new) == []
+    assert sum(n for _, _, n in d.fed) == len(prompt)
