@@ -595,7 +595,7 @@ __device__ __forceinline__ float ordered_sum(const float *e, unsigned cnt, float
   int stops = 0;
   while (r + 256 <= cnt && stops < AC_SUM_STOPS) {
     const uint32_t ex = __float_as_uint(s) >> 23;
-    if (ex < 32) // too small for u to be a normal number
+    if (ex < 32 || ex >= 255) // too small for u to be a normal number, or no number: the serial chain keeps it
       break;
     const float inv_u = __uint_as_float((277u - ex) << 23), u = __uint_as_float((ex - 23u) << 23); // u = 2^(k - 23), k = ex - 127
     const int S = (int)(s * inv_u);                         // in [2^23, 2^24)

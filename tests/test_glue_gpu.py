@@ -363,3 +363,31 @@ def test_attention_in_one_launch_equals_the_separate_launches(be, hq, hkv, hd, r
         be.device_status()
         for x, y in zip(*got):
             assert torch.equal(x.view(torch.uint8), y.view(torch.uint8))
+
+
+@pytest.mark.parametrize("rows", [40, 767, 800, 1500, 4096])
+def test_attention_in_one_launch_keeps_what_is_not_a_number(be, rows):
+    """A sink, a cached key and a query that are not numbers, and a key that makes a score infinite: NaN where the separate
+    launches have NaN, equal bits everywhere else -- on both sides of the rows from which the ordered sum has its fast form."""
+    hq, hkv, hd = 64, 8, 64
+    g = torch.Generator(device="cuda").manual_seed(rows)
+    r = lambda *n: torch.randn(*n, generator=g, device="cuda")  # noqa: E731
+    sink, kc, vc = r(hq), r(rows, hkv, hd).half(), r(rows, hkv, hd).half()
+    q, k, v = r(hq * hd), r(hkv * hd), r(hkv * hd)
+    sink[3], sink[20], sink[21] = float("nan"), float("inf"), -float("inf")
+    kc[rows // 2, 1, 5] = float("nan")
+    kc[5, 4] = float("inf")
+    vc[7, 5, 9] = float("nan")
+    q[50 * hd + 1] = float("nan")
+    got = []
+    for separate in (False, True):
+        a = be.Attention(hq, hkv, hd, rows, sink=sink)
+        a.kcache.copy_(kc)
+        a.vcache.copy_(vc)
+        got.append(a.step(q.clone(), k, v, rows - 1, separate=separate).view(hq, hd))
+    be.device_status()
+    one, sep = got
+    assert torch.isnan(sep[3]).all() and torch.isnan(sep[8:16]).all() and torch.isnan(sep[50]).all()
+    assert torch.isnan(sep[40:48, 9]).all() and torch.isfinite(sep[40:48, :9]).all() and torch.isfinite(sep[:3]).all()
+    assert torch.equal(torch.isnan(one), torch.isnan(sep))
+    assert torch.equal(one.nan_to_num(0.5).view(torch.int32), sep.nan_to_num(0.5).view(torch.int32))
