@@ -25,6 +25,7 @@
  */
 #include <atomic>
 
+#include "cluster.cuh"
 #include "common.cuh"
 #include "pipeline.cuh"
 #include "tma_map.cuh"
@@ -464,24 +465,12 @@ struct AttnStep {
   int k_box, v_box; // rows a copy brings: a tile, fewer where one short tile is all there is
 };
 
-__device__ __forceinline__ uint32_t cluster_rank() {
-  uint32_t r;
-  asm("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
-  return r;
-}
-__device__ __forceinline__ uint32_t cluster_size() {
-  uint32_t r;
-  asm("mov.u32 %0, %%cluster_nctarank;" : "=r"(r));
-  return r;
-}
 /** store to the same shared-memory address of another CTA of the cluster */
 __device__ __forceinline__ void st_cluster(uint32_t addr, uint32_t rank, float v) {
   uint32_t remote;
   asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(remote) : "r"(addr), "r"(rank));
   asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(remote), "f"(v) : "memory");
 }
-__device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory"); }
-__device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
 
 struct AcLayout {
   uint32_t ktile, vtile, e, q, total; // offsets; the tiles are 1024-byte aligned
@@ -649,7 +638,7 @@ attn_cluster_kernel(const __grid_constant__ CUtensorMap kmap, const __grid_const
   volatile int *abort_flag = &abort_word;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int gqa = a.hq / a.hkv / a.groups, hd = HD ? HD : a.hd, per_head = (hd + DIMS - 1) / DIMS, items = gqa * per_head;
-  const uint32_t rank = cluster_rank(), csize = cluster_size();
+  const uint32_t rank = (uint32_t)cluster_rank(), csize = (uint32_t)cluster_size();
   const int cluster = (int)(blockIdx.x / csize), n = cluster / a.groups, h0 = cluster * gqa; // kv head, first query head
   uint8_t *base = reinterpret_cast<uint8_t *>((reinterpret_cast<uintptr_t>(ac_raw) + 1023) & ~(uintptr_t)1023);
   const AcLayout L = ac_layout(gqa, hd, DIMS, a.k_bufs, a.v_bufs, a.cap_rows);
@@ -787,8 +776,12 @@ attn_cluster_kernel(const __grid_constant__ CUtensorMap kmap, const __grid_const
       kpar ^= 1;
     }
   }
+  if (!ok)
+    raise_in_cluster(smem_u32(&abort_word)); // the heads' owners lack these scores
+  __syncwarp();
   cluster_arrive();
   cluster_wait(); // every score of this CTA's head is here
+  ok = !*abort_flag;
   if (a.q_inplace && rank == 0) // every CTA of the cluster has read the raw heads
     for (int i = tid; i < gqa * hd; i += AC_THREADS)
       a.q_inplace[(size_t)h0 * hd + i] = qs[i];

@@ -24,10 +24,6 @@ __device__ __forceinline__ int cluster_rank() {
   asm("mov.u32 %0, %%cluster_ctarank;" : "=r"(n));
   return (int)n;
 }
-__device__ __forceinline__ void cluster_sync() {
-  asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
-  asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
-}
 /** four floats at a shared address (of this CTA's window) in the CTA of the given rank */
 __device__ __forceinline__ float4 ld_cluster4(uint32_t addr, int rank) {
   uint32_t remote;
@@ -45,6 +41,37 @@ __device__ __forceinline__ void st_cluster4(uint32_t addr, int rank, const float
   uint32_t remote;
   asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(remote) : "r"(addr), "r"(rank));
   asm volatile("st.shared::cluster.v4.f32 [%0], {%1,%2,%3,%4};" ::"r"(remote), "f"(v.x), "f"(v.y), "f"(v.z), "f"(v.w) : "memory");
+}
+
+__device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory"); }
+__device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
+__device__ __forceinline__ void cluster_sync() {
+  cluster_arrive();
+  cluster_wait();
+}
+
+/* A wait that ran out in one CTA of a cluster leaves its neighbours' results without its part, so they have to know before they
+ * store anything. flag: shared address of the word in which a CTA notes that it gave up, the same in every CTA. */
+/** Every thread that knows that its CTA gave up raises the neighbours' flags, before the barrier behind which the parts are used
+ *  and behind one that says that all have started. */
+__device__ __forceinline__ void raise_in_cluster(uint32_t flag) {
+  for (int r = 0; r < cluster_size(); ++r) {
+    uint32_t remote;
+    asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(remote) : "r"(flag), "r"(r));
+    asm volatile("st.shared::cluster.u32 [%0], %1;" ::"r"(remote), "r"(1) : "memory");
+  }
+}
+/** Where there is no such barrier (it would cost half a microsecond): the flag of the CTA whose rank is the lane's number, 0 in
+ *  the other lanes, for a vote of the warp. Between the barrier behind which the parts are used and the one behind which the CTAs
+ *  may leave. */
+__device__ __forceinline__ uint32_t neighbour_raised(uint32_t flag, int lane) {
+  uint32_t v = 0;
+  if (lane < cluster_size()) {
+    uint32_t remote;
+    asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(remote) : "r"(flag), "r"(lane));
+    asm volatile("ld.shared::cluster.u32 %0, [%1];" : "=r"(v) : "r"(remote) : "memory");
+  }
+  return v;
 }
 
 /** Launch of a grid of grid.x * parts by grid.y CTAs in clusters of `parts` CTAs along x. The grid may start while its

@@ -347,7 +347,7 @@ gemm_q4_K_umma_kernel(const uint8_t *__restrict__ atiles, const BlockQ4Kx8 *__re
     }
     const int row = mt * TILE_M + m;
     if (SHARED) { // the operand stages are free: every MMA of this CTA has retired
-      tile_done = ok;
+      tile_done = __all_sync(0xffffffffu, ok);
       float *sums = reinterpret_cast<float *>(smem) + m * SUM_PITCH + cgrp * DRAIN_COLS;
 #pragma unroll
       for (int i = 0; i < DRAIN_COLS; i += 4)
@@ -372,6 +372,7 @@ gemm_q4_K_umma_kernel(const uint8_t *__restrict__ atiles, const BlockQ4Kx8 *__re
     cluster_sync();
     if (tile_done) {
       const int rows = min(TILE_M, M - mt * TILE_M);
+      const uint32_t raised = neighbour_raised(smem_u32(const_cast<int *>(abort_flag)), lane);
       for (int i = tid - DRAIN_WARP0 * 32; part + (i >> 5) * parts < rows; i += DRAIN_WARPS * 32) {
         const int r = part + (i >> 5) * parts, c = 4 * (i & 31);
         float4 v[8];
@@ -383,6 +384,8 @@ gemm_q4_K_umma_kernel(const uint8_t *__restrict__ atiles, const BlockQ4Kx8 *__re
         for (int k = 1; k < 8; ++k)
           if (k < parts)
             v[0] = make_float4(v[0].x + v[k].x, v[0].y + v[k].y, v[0].z + v[k].z, v[0].w + v[k].w);
+        if (__any_sync(0xffffffffu, raised)) // a part is missing: C stays as it is
+          break;
         float *dst = C + (size_t)(mt * TILE_M + r) * ldc + nt * TILE_N + c;
         if (c_vec4) {
           *reinterpret_cast<float4 *>(dst) = v[0];

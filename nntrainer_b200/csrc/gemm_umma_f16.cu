@@ -152,8 +152,11 @@ __device__ __forceinline__ uint32_t expand2_q40(uint32_t nib2, __half2 d) {
  * QT = NNTR_Q4_0: W is block_q4_0x8, a stage is two 32-weight blocks (k_stages = K/64).
  * QT = NNTR_Q6_K: W is plain rows of block_q6_K (210 bytes, 2-byte aligned); stage (b, h, s2) of super-block b holds
  *                 the quarters s2 and s2 + 2 of its 128-element half h (the two quarters that share the bytes ql[64h +
- *                 32 s2 ..] as low and high nibbles); k_stages = 4 * K/256. N may end inside the last 256-row tile. */
-template <int QT>
+ *                 32 s2 ..] as low and high nibbles); k_stages = 4 * K/256. N may end inside the last 256-row tile.
+ * SHARED: a cluster of CTAs may share the tile. A kernel of its own: the code of a shared tile in the kernel of a lone CTA costs
+ * that one registers (80 without, 96 with) and 1024 x 24576 x 4096 Q4_K 185 us instead of 182. (It keeps the test for a cluster of
+ * one, without which the compiler spills 44 bytes instead of 8.) */
+template <int QT, bool SHARED>
 __global__ void __launch_bounds__(F16_THREADS, 1)
 gemm_f16_kernel(const __grid_constant__ CUtensorMap wmap, const uint8_t *__restrict__ atiles, const uint8_t *__restrict__ Wb,
                 float *__restrict__ C, int ldc, int M, int N, int k_stages, int m_tiles, int tiles_per_cta,
@@ -170,7 +173,7 @@ gemm_f16_kernel(const __grid_constant__ CUtensorMap wmap, const uint8_t *__restr
   // a CTA takes two 128-row activation tiles (unless there are SMs to spare) against the same 256 weight rows: the expanded
   // weights of a stage feed two MMAs, which halves the expansion work per output
   // the CTAs of a cluster share a tile: each walks its part of K, whole super-blocks (Q6_K: halves; Q4_0: pairs of blocks)
-  const int parts = cluster_size(), part = cluster_rank();
+  const int parts = SHARED ? cluster_size() : 1, part = SHARED ? cluster_rank() : 0;
   const int mt = tiles_per_cta * (blockIdx.x / parts), nt = blockIdx.y;
   const bool two = tiles_per_cta == 2 && mt + 1 < m_tiles;
   constexpr int UNIT = QT == NNTR_Q4_K ? 4 : QT == NNTR_Q6_K ? 2 : 1;
@@ -534,13 +537,14 @@ gemm_f16_kernel(const __grid_constant__ CUtensorMap wmap, const uint8_t *__restr
   /* ------------------------------ a shared tile ------------------------------ */
   // Every CTA of the cluster leaves its sums in its own shared memory; the rows are dealt out, and a CTA adds its rows' parts in
   // the order of K. All threads pass all barriers, whatever went wrong before.
-  if (parts > 1) {
+  if (SHARED && parts > 1) {
     for (int hm = 0; hm < (two ? 2 : 1); ++hm) {
       if (tile_done)
         turn_round(hm);
       cluster_sync();
       const int row0 = (mt + hm) * F16_TILE_M, rows = min(F16_TILE_M, M - row0);
-      if (tile_done)
+      if (tile_done) {
+        const uint32_t raised = neighbour_raised(smem_u32(const_cast<int *>(abort_flag)), lane);
         for (int i = tid; part + (i >> 6) * parts < rows; i += F16_PRODUCERS) {
           const int r = part + (i >> 6) * parts, c = 4 * (i & 63);
           const uint32_t at = sbase + 4u * (turn_area((r >> 5) + 4 * (c >> 6)) + (r & 31) * PITCH + (c & 63));
@@ -553,8 +557,11 @@ gemm_f16_kernel(const __grid_constant__ CUtensorMap wmap, const uint8_t *__restr
           for (int k = 1; k < 8; ++k)
             if (k < parts)
               v[0] = make_float4(v[0].x + v[k].x, v[0].y + v[k].y, v[0].z + v[k].z, v[0].w + v[k].w);
+          if (__any_sync(0xffffffffu, raised)) // a part is missing: C stays as it is
+            break;
           store4(row0 + r, nt * F16_TILE_N + c, v[0]);
         }
+      }
       cluster_sync(); // the area is rewritten by the second activation tile, and nobody leaves while it is read
     }
   }
@@ -670,7 +677,7 @@ quantize_q8_0_f16_tiles_kernel(const float *__restrict__ x, int64_t ldx, uint8_t
 template <int QT> int k_parts(int tiles, int k_stages) {
   static ClusterFit fit;
   for (int parts = 8; parts > 1; parts /= 2)
-    if (k_stages >= 4 * parts && tiles <= fit(gemm_f16_kernel<QT>, parts, F16_THREADS, f16_smem(QT)))
+    if (k_stages >= 4 * parts && tiles <= fit(gemm_f16_kernel<QT, true>, parts, F16_THREADS, f16_smem(QT)))
       return parts;
   return 1;
 }
@@ -697,9 +704,12 @@ int launch_gemm_f16(int qtype, unsigned M, unsigned N, unsigned K, const float *
   int dev = 0;
   NNTR_CHECK_CUDA(cudaGetDevice(&dev));
   if (dev < 64 && !attr_set[dev]) {
-    NNTR_CHECK_CUDA(cudaFuncSetAttribute(gemm_f16_kernel<NNTR_Q4_K>, cudaFuncAttributeMaxDynamicSharedMemorySize, f16_smem(NNTR_Q4_K)));
-    NNTR_CHECK_CUDA(cudaFuncSetAttribute(gemm_f16_kernel<NNTR_Q4_0>, cudaFuncAttributeMaxDynamicSharedMemorySize, f16_smem(NNTR_Q4_0)));
-    NNTR_CHECK_CUDA(cudaFuncSetAttribute(gemm_f16_kernel<NNTR_Q6_K>, cudaFuncAttributeMaxDynamicSharedMemorySize, f16_smem(NNTR_Q6_K)));
+    NNTR_CHECK_CUDA(cudaFuncSetAttribute(gemm_f16_kernel<NNTR_Q4_K, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, f16_smem(NNTR_Q4_K)));
+    NNTR_CHECK_CUDA(cudaFuncSetAttribute(gemm_f16_kernel<NNTR_Q4_K, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, f16_smem(NNTR_Q4_K)));
+    NNTR_CHECK_CUDA(cudaFuncSetAttribute(gemm_f16_kernel<NNTR_Q4_0, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, f16_smem(NNTR_Q4_0)));
+    NNTR_CHECK_CUDA(cudaFuncSetAttribute(gemm_f16_kernel<NNTR_Q4_0, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, f16_smem(NNTR_Q4_0)));
+    NNTR_CHECK_CUDA(cudaFuncSetAttribute(gemm_f16_kernel<NNTR_Q6_K, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, f16_smem(NNTR_Q6_K)));
+    NNTR_CHECK_CUDA(cudaFuncSetAttribute(gemm_f16_kernel<NNTR_Q6_K, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, f16_smem(NNTR_Q6_K)));
     attr_set[dev] = true;
   }
   const int mtiles = (int)((M + F16_TILE_M - 1) / F16_TILE_M), Mpad = mtiles * F16_TILE_M;
@@ -745,19 +755,22 @@ int launch_gemm_f16(int qtype, unsigned M, unsigned N, unsigned K, const float *
     count_launch();
     NNTR_CHECK_CUDA(cudaGetLastError());
     if (qtype == NNTR_Q4_K)
-      NNTR_CHECK_CUDA(launch_in_clusters(gemm_f16_kernel<NNTR_Q4_K>, grid, parts, F16_THREADS, f16_smem(NNTR_Q4_K), st, wmap, tiles, W,
-                                         C, (int)ldc, (int)M, (int)N, n_stages, mtiles, tiles_per_cta, c_vec4));
+      NNTR_CHECK_CUDA(launch_in_clusters(parts > 1 ? gemm_f16_kernel<NNTR_Q4_K, true> : gemm_f16_kernel<NNTR_Q4_K, false>, grid,
+                                         parts, F16_THREADS, f16_smem(NNTR_Q4_K), st, wmap, tiles, W, C, (int)ldc, (int)M, (int)N,
+                                         n_stages, mtiles, tiles_per_cta, c_vec4));
     else
-      NNTR_CHECK_CUDA(launch_in_clusters(gemm_f16_kernel<NNTR_Q6_K>, grid, parts, F16_THREADS, f16_smem(NNTR_Q6_K), st, wmap, tiles, W,
-                                         C, (int)ldc, (int)M, (int)N, n_stages, mtiles, tiles_per_cta, c_vec4));
+      NNTR_CHECK_CUDA(launch_in_clusters(parts > 1 ? gemm_f16_kernel<NNTR_Q6_K, true> : gemm_f16_kernel<NNTR_Q6_K, false>, grid,
+                                         parts, F16_THREADS, f16_smem(NNTR_Q6_K), st, wmap, tiles, W, C, (int)ldc, (int)M, (int)N,
+                                         n_stages, mtiles, tiles_per_cta, c_vec4));
   } else {
     const int64_t nwarps = (int64_t)Mpad * ((K + 255) / 256);
     quantize_q8_0_f16_tiles_kernel<<<(unsigned)((nwarps + 7) / 8), 256, 0, st>>>(A, K, static_cast<uint8_t *>(ws), (int)M,
                                                                                Mpad, (int)K);
     count_launch();
     NNTR_CHECK_CUDA(cudaGetLastError());
-    NNTR_CHECK_CUDA(launch_in_clusters(gemm_f16_kernel<NNTR_Q4_0>, grid, parts, F16_THREADS, f16_smem(NNTR_Q4_0), st, wmap, tiles, W,
-                                         C, (int)ldc, (int)M, (int)N, n_stages, mtiles, tiles_per_cta, c_vec4));
+    NNTR_CHECK_CUDA(launch_in_clusters(parts > 1 ? gemm_f16_kernel<NNTR_Q4_0, true> : gemm_f16_kernel<NNTR_Q4_0, false>, grid,
+                                         parts, F16_THREADS, f16_smem(NNTR_Q4_0), st, wmap, tiles, W, C, (int)ldc, (int)M, (int)N,
+                                         n_stages, mtiles, tiles_per_cta, c_vec4));
   }
   count_launch();
   return check_cuda(cudaGetLastError(), "gemm fp16 tensor-path launch");

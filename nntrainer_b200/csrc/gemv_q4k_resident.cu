@@ -132,7 +132,7 @@ gemv_q4_K_resident_kernel(const float *__restrict__ x, const BlockQ4Kx8 *__restr
   }
   __syncthreads();
   if (SPLIT)
-    asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory"); // waited for before the first store to a neighbour
+    cluster_arrive(); // waited for before the first store to a neighbour
   // let the next kernel in the stream be scheduled now: issuing the copies below can stall on the memory system, and a
   // dependent grid is launched only after every CTA of this one has passed this point
   pdl_launch_dependents();
@@ -364,7 +364,7 @@ gemv_q4_K_resident_kernel(const float *__restrict__ x, const BlockQ4Kx8 *__restr
     if (active)
       take_unit();
     __syncwarp();
-    asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); // every CTA of the cluster has started
+    cluster_wait(); // every CTA of the cluster has started
   }
 
   if (active && ok) {
@@ -408,10 +408,14 @@ gemv_q4_K_resident_kernel(const float *__restrict__ x, const BlockQ4Kx8 *__restr
     else
       part[t * 8 + r] = res;
   }
-  if (SPLIT)
+  if (SPLIT) {
+    if (!ok)
+      raise_in_cluster(smem_u32(const_cast<int *>(abort_flag))); // the others' chains lack this unit
+    __syncwarp();
     cluster_sync();
-  else
+  } else {
     __syncthreads();
+  }
 
   if (EXCHANGE && ex.n_ranks && threadIdx.x >= R_THREADS - 32 && (int)(threadIdx.x - (R_THREADS - 32)) < ex.n_ranks) {
     // "done reading": this CTA has consumed its input (everything was quantized into shared memory before the barriers
