@@ -898,7 +898,7 @@ attn_cluster_kernel(const __grid_constant__ CUtensorMap kmap, const __grid_const
           acc = __fmaf_rn(pt[j], half_bits_to_float(vt[j * DIMS]), acc);
       }
       __syncwarp();
-      if (lane == 0)
+      if (lane == 0) // the tile's last loads were issued sixteen multiply-adds ago
         mbar_arrive(vempty0 + 8 * buf);
       buf = nbuf;
       par = npar;

@@ -265,14 +265,11 @@ gemm_f16_kernel(const __grid_constant__ CUtensorMap wmap, const uint8_t *__restr
       if (lane == 0)
         mbar_arrive(BAR(st % F16_STAGES));
     };
-    // The packed words are on their way to registers and the slot may be refilled. Nothing has used them yet, and an arrive
-    // right behind the loads can overtake them (seen on Q4_0: now and then eight rows held a later stage's block), so the vote
-    // that gathers the warp, and the barrier's address with it, depends on what every lane loaded.
-    const uint32_t zero = gridDim.z - 1; // 0, but not to the compiler
-    auto raw_done = [&](int st, uint32_t loaded) {
-      const uint32_t any = __any_sync(0xffffffffu, (loaded & zero) != 0);
+    auto raw_done = [&](int st) { // the packed words are on their way to registers: the slot may be refilled when they are there
+      loads_before_refill();
+      __syncwarp();
       if (lane == 0)
-        mbar_arrive(BAR(12 + st % F16_RAW) + any);
+        mbar_arrive(BAR(12 + st % F16_RAW));
     };
     if constexpr (QT == NNTR_Q4_K) {
       // neighbouring groups read pairs of nibble chunks in opposite order: 128 bytes apart, they would meet in the same banks
@@ -294,7 +291,7 @@ gemm_f16_kernel(const __grid_constant__ CUtensorMap wmap, const uint8_t *__restr
         g2 = *reinterpret_cast<const uint2 *>(h + 48 + 24 * (st & 3));
         dw = half_bits_to_float(*reinterpret_cast<const uint16_t *>(h + 2 * j));
         dmw = half_bits_to_float(*reinterpret_cast<const uint16_t *>(h + 16 + 2 * j));
-        raw_done(st, w[0].x ^ w[1].x ^ w[2].x ^ w[3].x ^ g0.x ^ g1.x ^ g2.x ^ __float_as_uint(dw) ^ __float_as_uint(dmw));
+        raw_done(st);
         return true;
       };
       ok = hsel >= n_stages || fetch(hsel);
@@ -411,7 +408,7 @@ gemm_f16_kernel(const __grid_constant__ CUtensorMap wmap, const uint8_t *__restr
           q[2 * k + 1] = *reinterpret_cast<const uint2 *>(blk + k * (32 * 144) + 80 + 8 * j);
           dbits[k] = *reinterpret_cast<const uint16_t *>(blk + k * (32 * 144) + 2 * j);
         }
-        raw_done(st, q[0].x ^ q[1].x ^ q[2].x ^ q[3].x ^ dbits[0] ^ dbits[1]);
+        raw_done(st);
         return true;
       };
       ok = hsel >= n_stages || fetch(hsel); // n_stages may be odd (K = 2880)

@@ -76,6 +76,13 @@ __device__ __forceinline__ void bulk_g2s(uint32_t dst, const void *src, uint32_t
                : "memory");
 }
 
+/** Before a warp gives a slot of shared memory back to bulk copies: the loads of every lane have been performed then. Neither the
+ *  warp's barrier nor the arrive behind it waits for loads whose values nothing has used yet, and a copy that refills the slot
+ *  may overtake them (fp16 GEMM, Q4_0 256 x 24576 x 2880, without a fence: wrong elements in every launch; with this one or
+ *  __threadfence_block(): none in 3000). Needless where the values have gone into a store, or into a chain that the next round
+ *  continues, before the slot is given back. */
+__device__ __forceinline__ void loads_before_refill() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
+
 /** Quotients by a number known at run time only, exact while dividend * n < 2^32: a multiplication instead of the 150 clocks
  *  (64 bits: several hundred) of a division, which a loop with one thread or warp per stage of a ring cannot hide. */
 struct FastDiv {
