@@ -12,7 +12,7 @@ import pytest
 torch = pytest.importorskip("torch")
 pytestmark = pytest.mark.gpu
 
-from nntrainer_b200.decoder import DecoderConfig, Qwen3Decoder  # noqa: E402
+from nntrainer_b200.decoder import DecoderConfig, Qwen3Decoder, tensor_list  # noqa: E402
 from oracle import oracle as O  # noqa: E402
 from oracle.cpu_decoder import CpuDecoder, synthetic_weights, write_bin  # noqa: E402
 
@@ -60,7 +60,7 @@ def _run(be, cfg, prompt, n_new, seed, fuse=True):
     return got, want, gpu_logits, cpu.last_logits, margin
 
 
-@pytest.mark.parametrize("fuse", [True, False], ids=["seven_launches_per_layer", "ten_launches_per_layer"])
+@pytest.mark.parametrize("fuse", [True, False], ids=["five_launches_per_layer", "nine_launches_per_layer"])
 def test_greedy_token_stream_identical_over_64_steps(be, fuse):
     """Both launch sequences: with the residual adds and norms folded into the projections' prologues, and with every
     operator in a launch of its own."""
@@ -116,16 +116,19 @@ def test_a_replaced_cache_is_used_by_every_launch_sequence(be):
     other.close()
 
 
-@pytest.mark.parametrize("window,fc,P", [(None, "q4_K", 2), (None, "q4_K", 9), (16, "q4_K", 40), (None, "q6_K", 33),
-                                         (None, "q4_K", 300)])
-def test_batched_prompt_equals_token_by_token(be, window, fc, P):
+@pytest.mark.parametrize("window,fc,P,hd", [(None, "q4_K", 2, 64), (None, "q4_K", 9, 64), (16, "q4_K", 40, 64), (None, "q6_K", 33, 64),
+                                            (None, "q4_K", 300, 64), (None, "q4_K", 258, 64), (None, "q4_K", 258, 128),
+                                            (100, "q4_K", 131, 128), (None, "q4_K", 20, 96), (None, "q4_0", 20, 64)])
+def test_batched_prompt_equals_token_by_token(be, window, fc, P, hd):
     """The prompt's batched pass against feeding the prompt through step(): tokens, final logits and both caches of every
     layer, equal bits -- a prompt too short to be batched, ragged tiles of eight rows, a window shorter than the prompt,
-    separate q, k and v projections (Q6_K), and more tokens than one pass takes."""
-    cfg = DecoderConfig(n_layers=3, hidden=512, n_heads=8, n_kv_heads=2, head_dim=64, inter=768, vocab=1024, max_seq=P + 8,
+    separate q, k and v projections (Q6_K, Q4_0), more tokens than one pass takes, a last pass of one row, and heads of more
+    than 64 dimensions, of which a CTA owns all when many tokens are at hand."""
+    cfg = DecoderConfig(n_layers=3, hidden=512, n_heads=8, n_kv_heads=2, head_dim=hd, inter=768, vocab=1024, max_seq=P + 8,
                         sliding_window=window, fc_dtype=fc)
     w = synthetic_weights(cfg, 3)
     rng = np.random.default_rng(P)
+    w.update({name: O.random_q4_0x8(rng, N, K) for name, d, N, K in tensor_list(cfg) if d == "q4_0"})
     prompt = [int(t) for t in rng.integers(0, cfg.vocab, P)]
     with tempfile.TemporaryDirectory() as td:
         path = os.path.join(td, "model.bin")
@@ -140,6 +143,7 @@ def test_batched_prompt_equals_token_by_token(be, window, fc, P):
             ref.append(int(nxt.item()))
     be.device_status()
     assert tokens == ref
+    assert torch.isfinite(want.b["logits"]).all()
     assert torch.equal(got.b["logits"].view(torch.int32), want.b["logits"].view(torch.int32))
     for a, b in zip(got.attn, want.attn):
         assert torch.equal(a.kcache.view(torch.int16), b.kcache.view(torch.int16))

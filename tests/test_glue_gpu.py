@@ -206,7 +206,7 @@ def test_fused_qk_norm_rope_equals_the_separate_launches(be):
         o1 = a1.step(q1, k1, dev(v), 3, q_rot=r1)
         q2 = dev(q)
         o2 = a2.step(q2, dev(k), dev(v), 3, qk_norm=(dev(qg), dev(kg), 1e-6), q_rot=r2)
-        assert same_bits(q2.cpu().numpy(), q), "the two-launch sequence leaves the query untouched"
+        assert same_bits(q2.cpu().numpy(), q), "the step in one launch leaves the query untouched"
         assert same_bits(r1.cpu().numpy(), r2.cpu().numpy())
         # the rotary launch of its own rotates the query in place and gives the same heads
         a3 = be.Attention(hq, hkv, hd, 8)
