@@ -122,6 +122,9 @@ size_t nntr_cuda_gemm_workspace_bytes(int qtype, unsigned M, unsigned N, unsigne
  *   AUTO        from 32 rows up TENSOR_F16 where it applies, else TENSOR where
  *               that applies, else EXACT (the default).
  *  A path that does not apply to a call falls back to EXACT.
+ *  On the two tensor paths K is cut into parts when a call has few tiles of C, so the last bits of a row may
+ *  depend on how many rows the call has (within the figures above); on the exact path they depend on M only
+ *  through the reference's rule for the last M % 4 rows.
  *  There is no CPU counterpart: the reference picks its SIMD variant at build time. */
 #define NNTR_CUDA_GEMM_PATH_AUTO 0
 #define NNTR_CUDA_GEMM_PATH_EXACT 1

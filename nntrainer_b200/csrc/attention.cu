@@ -434,10 +434,13 @@ __global__ void attn_values_kernel(const float *__restrict__ probs, const uint16
  *            ascending row order by one warp (ordered_sum).
  *   values   a thread per dimension runs the row-ordered chain over value tiles that a producer warp keeps ahead of it
  *            (tiled TMA copies, started before the scores).
- * The chains are serial at four clocks per row; they bound the kernel for long contexts, launch and exchange latencies do
- * for short ones: 64 / 8 heads of 64 at 4096 rows 48 us (four launches before: 120), 32 / 8 heads of 128 at 512 rows 11 us (two
- * launches before: 15.7), at 128 rows of a window 7 us (10.8). Ring positions are counted, not divided: an integer division in a loop that one thread runs costs more than
- * a tile's copy. */
+ * Clock stamps of one CTA per cluster, 64 / 8 heads of 64, at 512 / 2048 / 4096 / 6000 rows, in clocks: start and first copies 3000,
+ * heads rotated 1000, score tiles 2500 / 7000 / 12500 / 20600, barrier behind them 2000 to 3300, maximum 1000, exponentials 600 /
+ * 1500 / 2900 / 4400, ordered sum 5700 / 9300 / 12800 / 15700, division 400 to 2200, value chain 6800 / 23600 / 46000 / 67100. The
+ * value chain is more than half of a long context at 11.2 clocks per row, where a dependent multiply-add alone takes four (heads
+ * of 128: the same). 64 / 8 heads of 64 at 4096 rows 47 us (four launches before: 120), 32 / 8 heads of 128 at 512 rows 11 us (two
+ * launches before: 15.7), at 128 rows of a window 7 us (10.8).
+ * Ring positions are counted, not divided: an integer division in a loop that one thread runs costs more than a tile's copy. */
 constexpr int AC_THREADS = 256;
 constexpr int AC_WARPS = AC_THREADS / 32;
 constexpr int AC_TILE = 128; // cache rows per tile of keys or values
@@ -574,8 +577,8 @@ __device__ __forceinline__ float serial_sum(const float *e, unsigned lo, unsigne
  * nearest, and only for an exact half does the choice depend on S. So the integers of 256 rows are added in any order, eight rows
  * per lane, and S + their sum is the serial result as long as it stays below 2^24 and no half occurred. Where one of the two
  * happens, the lanes in front of the first such lane are taken, that lane's eight rows are added serially, and the next 256
- * rows start behind them. That takes about 250 clocks per 256 rows or interruption against 1050 for the serial chain, and
- * interruptions are few (a power of two is passed log2(rows) times; a half has probability e / s per row, so the first rows
+ * rows start behind them. That takes about 430 clocks per 256 rows, interruptions among them, against 2800 for the serial
+ * chain (11 clocks a row), and interruptions are few (a power of two is passed log2(rows) times; a half has probability e / s per row, so the first rows
  * are added serially) -- after AC_SUM_STOPS of them the rest is added serially. */
 constexpr unsigned AC_SUM_SERIAL = 64;    // rows at the start
 constexpr unsigned AC_SUM_PARALLEL = 768; // below this many rows the serial chain is as fast
@@ -841,8 +844,8 @@ attn_cluster_kernel(const __grid_constant__ CUtensorMap kmap, const __grid_const
   } else if (warp < DIMS / 32) {
     const int d = item_d0 + tid;
     float acc = 0.f;
-    // Sixteen rows in the chain while the next sixteen -- of the next tile at a tile's end -- are on their way: 4.3 clocks per
-    // row (the chain alone: 4.1; loads issued by the compiler's own schedule: 8 to 12).
+    // Sixteen rows in the chain while the next sixteen -- of the next tile at a tile's end -- are on their way. 11.2 clocks per
+    // row all the same (the dependent multiply-add: 4); what holds it up has not been found.
     float pr[2][16];
     uint16_t vb[2][16];
     auto load = [&](const uint16_t *vt, const float *pt, float(&pp)[16], uint16_t(&vv)[16]) {

@@ -291,8 +291,11 @@ static int pick_gemm_kernel(int qtype, unsigned M, unsigned N, unsigned K) {
     return umma_f16_supported(qtype, M, N, K) ? 2 : 0;
   if (M < TENSOR_PATH_MIN_M) // auto
     return 0;
-  // auto: the fp16 path is the faster kernel per tile but cuts the problem into 256 x 256 tiles; when those would
-  // leave most SMs idle the integer path's 128 x 128 tiles win
+  // auto: the fp16 path where its 256 x 256 tiles fill half of the SMs, else the integer path, whose sums are exact (C within 1e-6
+  // of the CPU's instead of 4e-4). It is not the faster one of the two on that side of the line: with K cut into parts the fp16
+  // kernel takes 29 against 33 us at 256 x 2560 x 2560, 54 against 99 at 512 x 2560 x 9728, 47 against 88 at 1024 x 4096 x 4096; up to
+  // 128 rows of 4096 weight rows the integer path is ahead or level (128 x 4096 x 4096: 21 against 25). Set
+  // NNTR_CUDA_GEMM_PATH_TENSOR_F16 to have the fp16 kernel whatever the size.
   const bool f16_ok = umma_f16_supported(qtype, M, N, K), i8_ok = umma_supported(qtype, M, N, K);
   const unsigned mt = (M + 127) / 128;
   const unsigned tiles_f16 = ((mt + 1) / 2) * ((N + 255) / 256);

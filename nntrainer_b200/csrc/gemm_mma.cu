@@ -23,8 +23,10 @@
  * Two splits of the work:
  *   gemm_mma_rows_kernel   a warp owns 16 weight rows and up to 32 activation rows over all of K; the CTA's four warps share
  *                          the unit's activation tiles and weights, which bulk copies bring into a ring. For problems with
- *                          enough such tiles to fill the machine. Bound by instruction issue (the conversions and the chains
- *                          are about 100 of the 220 instructions per 16 x 8 x 256): 256 x 24576 x 4096 286 us, 180 TOP/s
+ *                          enough such tiles to fill the machine. Bound by too few warps in flight: at 32 rows per tile 142 (Q4_0) to
+ *                          168 registers and 55 KB hold three CTAs per SM, and Q4_0 509 x 2880 x 2880 (720 CTAs, 1.6 waves) issues
+ *                          in 54 % of the active clocks with 2.5 warps per scheduler, a third of the waiting being for memory
+ *                          (the conversions and the chains are about 100 of the 220 instructions per 16 x 8 x 256): 256 x 24576 x 4096 286 us, 180 TOP/s
  *                          (CUDA-core kernel before: 2981 us); Q4_0 509 x 2880 x 2880 58 us (551).
  *   gemm_mma_ksplit_kernel eight warps share the tile and take every eighth unit of 256 along K; the terms of the chains
  *                          go through shared memory and one thread per chain adds them in order. For the others: bound by
@@ -959,6 +961,9 @@ int launch_gemm_grouped(int qtype, unsigned N, unsigned K, const void *act, floa
   // Q4_0's small tile: 55 registers, so shared memory sets the CTAs per SM, six with three units in flight and nine with two.
   // From a pair per expert up the grid is two and more waves of six, and nine win: 4 of 32 experts of 2880 x 2880, 8 tokens
   // 107 -> 100 us; 5 tokens (a wave and a half) 87.7 -> 89.3, so those keep three. Q4_K's tile is held to five by registers.
+  // The line holds for experts of that size (7 tokens, below it: three in flight 109.8 us, two 102.6) and of half the width (8 / 12 /
+  // 16 tokens 75.9 / 82.2 / 85.3 us with three, 70.9 / 74.9 / 77.5 with two). Elsewhere two in flight cost a little: 2 of 16 experts of
+  // 4096 x 4096, 12 tokens 117.3 -> 120.0; 4 of 64 experts of 1024 x 2880, 16 / 32 tokens 85.3 / 101 -> 88.8 / 103.
   const bool shallow = pairs >= (unsigned)n_experts;
 #define NNTR_MMA_RUN(QT)                                                                                               \
   (tile_rows == 8    ? run_tiles<QT, 1, true, true>(a, tiles, z, ksplit, shallow, st)                                           \

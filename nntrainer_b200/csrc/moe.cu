@@ -50,7 +50,11 @@ struct MoeEp {
  * weights, but three launches more than a GEMV per pair): where a GEMV per pair no longer gets enough of the GPU. Q4_0 (gate and
  * up are two problems per pair, one CTA per SM): below four CTAs per problem; 4 of 32 experts of 2880 x 2880, 2 / 4 / 5 / 8
  * tokens: GEMVs 45 / 73 / 90 / 128 us, grouped 60 / 81 / 85 / 101. Q4_K (one problem per pair, two CTAs per SM): below three;
- * 8 of 128 experts of 2048 x 768, 8 / 12 / 14 tokens: 60 / 77 / 104 us against 71 / 88 / 92. */
+ * 8 of 128 experts of 2048 x 768, 8 / 12 / 14 tokens: 60 / 77 / 104 us against 71 / 88 / 92. Other experts, GEMVs against grouped on
+ * both sides of the line: Q4_0 4 of 32 of 1024 x 1440, 4 / 5 / 8 / 12 tokens 29 / 33 / 41 / 64 us against 37 / 36 / 41 / 46; 2 of 16 of
+ * 4096 x 4096, 9 / 10 tokens 106 / 130 against 115 / 121; Q4_K 4 of 64 of 1024 x 512, 24 / 25 tokens 41 / 50 against 47 / 47. Wide Q4_K
+ * experts cross earlier than the line says: 4 of 32 of 4096 x 1536, 6 / 12 / 16 / 24 tokens 74 / 133 / 186 / 244 against 77 / 119 / 124 /
+ * 128, because there a GEMV per pair reads an expert's weights again for each of its tokens. */
 constexpr unsigned GROUPED_MIN_TOKENS = 2;
 static bool run_grouped(int qtype, unsigned tokens, unsigned pairs) {
   return tokens >= GROUPED_MIN_TOKENS && (qtype == NNTR_Q4_0 ? 8 * pairs > (unsigned)sm_count() : 3 * pairs > 2 * (unsigned)sm_count());
@@ -59,7 +63,10 @@ constexpr int MOE_COUNTER_TOKENS = 4096;   // arrival counters kept at the start
 constexpr int ROUTER_WARPS = 8;
 constexpr int ROUTER_SLICES = 32; // CTAs per token
 constexpr int MAX_E_PER_LANE = 8; // up to 256 experts
-constexpr unsigned ROUTER_ROWS_MIN_TOKENS = 48; // below, a CTA row per token has the weight in L2 anyway and more CTAs
+// Tokens from which the router takes eight of them at a time. The line is a cautious one: a layer with 8 of 128 experts and H =
+// 2048, with a CTA row per token / with eight tokens per CTA row, 16 / 24 / 32 / 48 / 64 tokens: 98.7 / 114.2 / 126.3 / 136.4 /
+// 147.5 us, 97.8 / 111.7 / 121.7 / 128.1 / 134.0.
+constexpr unsigned ROUTER_ROWS_MIN_TOKENS = 48;
 constexpr int ROUTER_PRE = 8;     // rows of a warp's slice fetched before the dependency wait
 
 /* std::partial_sort(idx, idx + k, idx + n, [&](a, b) { return v[a] > v[b]; }) on idx = 0..n-1, as the GNU C++ library
