@@ -565,7 +565,9 @@ __global__ void __launch_bounds__(ROWS_WARPS * 32, NT == 4 ? 3 : 4) gemm_mma_row
                        *w1 = reinterpret_cast<const BlockQ40x8 *>(sh.w[s] + wg1 * sizeof(BlockQ4Kx8));
       with_tiles<NT>(nt, [&](auto N) { q40_unit<decltype(N)::value>(acc, w0, w1, act, n, g, t, lane); });
     }
-    loads_before_refill();
+    // every lane's loads have been performed before the slot is given back (loads_before_refill() does the same here and costs 0.4 %
+    // of the grouped products)
+    __threadfence_block();
     __syncwarp();
     if (lane == 0)
       mbar_arrive(empty0 + 8 * s);
