@@ -61,7 +61,7 @@ __device__ __forceinline__ void raise_in_cluster(uint32_t flag) {
     asm volatile("st.shared::cluster.u32 [%0], %1;" ::"r"(remote), "r"(1) : "memory");
   }
 }
-/** Where there is no such barrier (it would cost half a microsecond): the flag of the CTA whose rank is the lane's number, 0 in
+/** Where there is no such barrier (it would be one more per call): the flag of the CTA whose rank is the lane's number, 0 in
  *  the other lanes, for a vote of the warp. Between the barrier behind which the parts are used and the one behind which the CTAs
  *  may leave. */
 __device__ __forceinline__ uint32_t neighbour_raised(uint32_t flag, int lane) {
