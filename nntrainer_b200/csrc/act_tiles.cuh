@@ -11,17 +11,20 @@
 
 namespace nntr {
 
-/* Activations: tiles of 8 rows, tile-major, in the order the B fragments are read: lane 4g + t of a warp holds row g of
+/* Activations: tiles of 8 rows in the order the B fragments are read: lane 4g + t of a warp holds row g of
  * the tile. Per tile and unit of 256 of K, act_row_bytes(QT) per row (rows of a tile beyond the problem's are never written;
  * they only reach output columns that are never stored):
  *   [4 pairs of 32][32 lanes][16 bytes]  the lane's 8 values of the even and the 8 of the odd 32-block
- *   Q4_K: [8] float d, [32 lanes] words (lo, hi of the 32-block t, lo, hi of t + 4): the block's sum is lo + 64 * (hi - 64)
- *   Q4_0: [8][8] half d
+ *   Q4_K: [8] float d, [32 lanes] words (lo, hi of the 32-block t, lo, hi of t + 4): the block's sum is lo + 32 * (hi - 128)
+ *   Q4_0: [4 pairs][8 rows][even, odd 32-block] half d
  * A tile of th < 8 rows is laid out with th in the place of 8 and 4 th in the place of 32 lanes. */
 __host__ __device__ constexpr int act_row_bytes(int qtype) { return qtype == NNTR_Q4_0 ? 272 : 288; }
 
-template <int QT, typename Byte> __device__ __forceinline__ Byte *act_unit(Byte *act, size_t tile, int th, int nb, int b) {
-  return act + (tile * nb + b) * (size_t)(th * act_row_bytes(QT));
+/** Unit b of tile k of a block of n_tiles tiles (all the rows of a dense problem, or those of one expert) that starts with tile
+ *  `first` of the buffer. Units are outermost, so that neighbouring tiles of a unit are one piece of memory. */
+template <int QT, typename Byte>
+__device__ __forceinline__ Byte *act_unit(Byte *act, int first, int n_tiles, int k, int th, int nb, int b) {
+  return act + ((size_t)first * nb + (size_t)b * n_tiles + k) * (size_t)(th * act_row_bytes(QT));
 }
 
 /** The values of a warp that has quantized 256 elements (lane: 8 of them from element 8 * lane) into row i of a tile. */
@@ -32,7 +35,7 @@ __device__ __forceinline__ void put_q8K(uint8_t *unit, int th, int i, const Q8KL
   s += __shfl_xor_sync(FULL, s, 2);
   if (t == 0)
     *reinterpret_cast<uint16_t *>(unit + 260 * th + (4 * i + (j & 3)) * 4 + 2 * (j >> 2)) =
-      (uint16_t)((s & 63) | (((s >> 6) + 64) << 8)); // |s| <= 32 * 127
+      (uint16_t)((s & 31) | (((s >> 5) + 128) << 8)); // |s| <= 32 * 127
   if (lane == 0)
     *reinterpret_cast<float *>(unit + 256 * th + 4 * i) = q.d;
 }
@@ -43,7 +46,7 @@ __device__ __forceinline__ void put_q80(uint8_t *unit, int th, int i, const Q80L
   *reinterpret_cast<uint32_t *>(dst) = q.w0;
   *reinterpret_cast<uint32_t *>(dst + 16) = q.w1;
   if ((lane & 3) == 0)
-    *reinterpret_cast<uint16_t *>(unit + 256 * th + 16 * i + 2 * j) = q.d_bits;
+    *reinterpret_cast<uint16_t *>(unit + 256 * th + 32 * (j >> 1) + 4 * i + 2 * (j & 1)) = q.d_bits; // th is 8
 }
 
 } // namespace nntr

@@ -355,7 +355,7 @@ int launch_gemm_mma_q6_K(unsigned M, unsigned N, unsigned K, const float *A, con
  * order being pair perm[p]; expert e has the positions off[e] .. off[e+1], the tiles tile_off[e] .. of tile_rows rows each
  * and the activation tiles act_off[e] .. of 8 rows each (rows: perm[p] / a_div of x); output row perm[p] * c_mul (+ 1 for
  * w_table1). */
-int grouped_tile_rows(unsigned pairs, unsigned n_experts);
+int grouped_tile_rows(int qtype, unsigned pairs, unsigned n_experts);
 int launch_act_tiles_grouped(int qtype, const float *x, unsigned rows, unsigned K, void *act, const int *perm, const int *idx,
                              const int *off, const int *act_off, int a_div, cudaStream_t st);
 int launch_gemm_grouped(int qtype, unsigned N, unsigned K, const void *act, float *C, unsigned ldc,

@@ -14,24 +14,23 @@
  * its A fragment is what one 8-byte (Q4_K) or 4-byte (Q4_0) piece of the interleaved weight block holds: the low and the
  * high nibbles of 4 bytes each, one logic op per fragment register and no trip through shared memory.
  *
- * sc0 * I0 + sc1 * I1 of a pair of sub-blocks is computed in fp32: |I| <= 15 * 127 * 32 and sc <= 63, so every product
- * and the sum (below 2^23) are exact. High nibbles enter in place, as 16 times their value, and meet sc1 / 16. (Seeding
- * the MMA with the bits of 1.5 * 2^23, so that its result is a float already, was measured: the four moves that set the
- * operand up for each MMA cost more than the conversions.) The sums of the mins term come from one fp16 MMA
- * of [min, 64 min] with the sums of 32 activations split into [sum & 63, sum >> 6], all of them integers fp16 holds.
+ * A sub-block's sum and its 6-bit scale meet as integers (|I| <= 15 * 127 * 32, sc <= 63): a pair of sub-blocks stays below
+ * 2^23, which fp32 holds, a super-block below 2^25, whose one conversion rounds as the reference's does. The sums of the mins
+ * term come from one fp16 MMA of [min, 32 min] with the sums of 32 activations split into [sum & 31, sum >> 5], all of them
+ * integers fp16 holds. Float steps go two at a time (fma.rn.f32x2), each rounded as by itself.
  *
  * Two splits of the work:
  *   gemm_mma_rows_kernel   a warp owns 16 weight rows and up to 32 activation rows over all of K; the CTA's four warps share
- *                          the unit's activation tiles and weights, which bulk copies bring into a ring. For problems with
- *                          enough such tiles to fill the machine. Bound by too few warps in flight: at 32 rows per tile 142 (Q4_0) to
- *                          168 registers and 55 KB hold three CTAs per SM, and Q4_0 509 x 2880 x 2880 (720 CTAs, 1.6 waves) issues
- *                          in 54 % of the active clocks with 2.5 warps per scheduler, a third of the waiting being for memory
- *                          (the conversions and the chains are about 100 of the 220 instructions per 16 x 8 x 256): 256 x 24576 x 4096 286 us, 180 TOP/s
- *                          (CUDA-core kernel before: 2981 us); Q4_0 509 x 2880 x 2880 58 us (551).
- *   gemm_mma_ksplit_kernel eight warps share the tile and take every eighth unit of 256 along K; the terms of the chains
- *                          go through shared memory and one thread per chain adds them in order. For the others: bound by
- *                          latency. 8 x 6144 x 2560 12.2 us including the quantizer's launch (25.5), 8 x 2560 x 9728
- *                          18.9 us (77.6).
+ *                          the unit's activation tiles and weights, which a fifth warp brings into a ring by bulk copies. CTAs
+ *                          stay and go through items of 64 weight rows. Bound by instruction issue, shared memory and half-rate
+ *                          operations alike: per 16 x 8 x 32 of Q4_0 about 20 instructions, 4 wavefronts of shared memory, 8 half-rate
+ *                          operations, four to five clocks of an SM each, seven taken. Q4_0 1000 x 8000 x 4096 208 us (a
+ *                          computing thread starting the copies, 25 instructions: 303), 509 x 2880 x 2880 36.9 us (51.6); Q4_K
+ *                          255 x 9728 x 2560 55.7 us (75.4).
+ *   gemm_mma_ksplit_kernel eight warps share the tile and take every eighth unit of 256 along K; the float chains go from warp
+ *                          to warp, one unit further at each. For the others: bound by that hand-over (270 clocks a unit) when
+ *                          K is long, by launch and round trips when it is short. With the quantizer's launch: Q4_K 8 x 2560 x 2560
+ *                          6.4 us, 8 x 2560 x 9728 12.3 us (terms through shared memory to one thread per chain: 8.8 and 18.7).
  */
 #include <type_traits>
 
@@ -84,40 +83,32 @@ __device__ __forceinline__ void mma_f16_k16(float (&d)[4], uint32_t a0, uint32_t
 
 __device__ __forceinline__ uint32_t h2_bits(__half2 h) { return *reinterpret_cast<const uint32_t *>(&h); }
 __device__ __forceinline__ __half2 bits_h2(uint32_t u) { return *reinterpret_cast<const __half2 *>(&u); }
-/** (v, 64 v) of a 6-bit value as half2; 0x64vv is 1024 + v */
-__device__ __forceinline__ uint32_t min_halves(uint32_t v) {
-  return h2_bits(__hmul2(__hsub2(bits_h2(v * 0x10001u | 0x64006400u), bits_h2(0x64006400u)), __floats2half2_rn(1.f, 64.f)));
+/** two fp32 operations in one instruction, each rounded as by itself */
+__device__ __forceinline__ void fma2(float &d0, float &d1, float a0, float a1, float b0, float b1) {
+  asm("{.reg .b64 a, b, d;\n\tmov.b64 a, {%2, %3};\n\tmov.b64 b, {%4, %5};\n\tmov.b64 d, {%0, %1};\n\t"
+      "fma.rn.f32x2 d, a, b, d;\n\tmov.b64 {%0, %1}, d;}"
+      : "+f"(d0), "+f"(d1)
+      : "f"(a0), "f"(a1), "f"(b0), "f"(b1));
 }
-/** (lo, hi - 64) of one 16-bit half K of an activation row's word as half2 */
+__device__ __forceinline__ float2 mul2(float a0, float a1, float b0, float b1) {
+  float2 r;
+  asm("{.reg .b64 a, b, d;\n\tmov.b64 a, {%2, %3};\n\tmov.b64 b, {%4, %5};\n\t"
+      "mul.rn.f32x2 d, a, b;\n\tmov.b64 {%0, %1}, d;}"
+      : "=f"(r.x), "=f"(r.y)
+      : "f"(a0), "f"(a1), "f"(b0), "f"(b1));
+  return r;
+}
+/** (v, 32 v) of byte K of four 6-bit values as half2; 0x64vv is 1024 + v */
+template <int K> __device__ __forceinline__ uint32_t min_halves(uint32_t v) {
+  return h2_bits(__hfma2(bits_h2(__byte_perm(v, 0x64646464u, 0x4040 | (K * 0x101))), __floats2half2_rn(1.f, 32.f),
+                         __floats2half2_rn(-1024.f, -32768.f)));
+}
+/** (lo, hi - 128) of one 16-bit half K of an activation row's word as half2 */
 template <int K> __device__ __forceinline__ uint32_t sum_halves(uint32_t w) {
-  return h2_bits(__hsub2(bits_h2(__byte_perm(w, 0x64646464u, K ? 0x4342 : 0x4140)), __floats2half2_rn(1024.f, 1088.f)));
+  return h2_bits(__hsub2(bits_h2(__byte_perm(w, 0x64646464u, K ? 0x4342 : 0x4140)), __floats2half2_rn(1024.f, 1152.f)));
 }
 
 /* ------------------------------------------------------------------ Q4_K */
-/** The weights of 16 rows x 256 as a lane holds them: g = lane / 4 picks the rows g and g + 8, t = lane % 4 the 8-byte
- *  chunk 4p + t of pair p, i.e. elements 8t .. 8t+7 of the pair's two sub-blocks. */
-struct Q4KRaw {
-  uint2 q[4][2];       // [pair][row g / g + 8]
-  uint32_t head[2][2][3]; // [row][sub-block t / t + 4]: the 12-byte group with scales and mins of the row's 8-row group
-  uint32_t d[2];       // d | dmin << 16
-};
-__device__ __forceinline__ void q4k_load(Q4KRaw &r, const BlockQ4Kx8 *lo, const BlockQ4Kx8 *hi, int g, int t) {
-#pragma unroll
-  for (int p = 0; p < 4; ++p) {
-    r.q[p][0] = ldg_stream_u2(lo->qs + ((4 * p + t) * 8 + g) * 8);
-    r.q[p][1] = ldg_stream_u2(hi->qs + ((4 * p + t) * 8 + g) * 8);
-  }
-#pragma unroll
-  for (int row = 0; row < 2; ++row) {
-    const BlockQ4Kx8 *b = row ? hi : lo;
-#pragma unroll
-    for (int s = 0; s < 2; ++s)
-#pragma unroll
-      for (int i = 0; i < 3; ++i)
-        r.head[row][s][i] = __ldg(reinterpret_cast<const uint32_t *>(b->scales + 12 * (t + 4 * s)) + i);
-    r.d[row] = (uint32_t)__ldg(&b->d[g]) | ((uint32_t)__ldg(&b->dmin[g]) << 16);
-  }
-}
 /** What the MMAs and chains need besides the nibbles. */
 struct Q4KScales {
   uint32_t sc[4];  // gathered from the quad: word t' = scales of sub-blocks t' and t' + 4 of row g (bytes 0, 1), row g + 8 (2, 3)
@@ -125,19 +116,20 @@ struct Q4KScales {
   float dw[2], dm[2];
 };
 __device__ __forceinline__ void q4k_scales(Q4KScales &s, const uint32_t (&head)[2][2][3], const uint32_t (&d)[2], int g, int lane) {
-  const int sh = 8 * (g & 3);
-  uint32_t own = 0;
+  // the bytes of this lane's rows out of the three words of a group, four (row, sub-block) at a time: word i -> x[i]
+  uint32_t x[3];
+  const uint32_t two = (g & 3) * 0x11 + 0x40; // byte g % 4 of either operand
 #pragma unroll
-  for (int row = 0; row < 2; ++row)
-#pragma unroll
-    for (int k = 0; k < 2; ++k) {
-      const uint32_t b0 = (head[row][k][0] >> sh) & 0xff, b1 = (head[row][k][1] >> sh) & 0xff,
-                     b2 = (head[row][k][2] >> sh) & 0xff;
-      const uint32_t sc = g < 4 ? (b0 & 63) : ((b2 & 0xf) | ((b0 >> 6) << 4));
-      const uint32_t mn = g < 4 ? (b1 & 63) : ((b2 >> 4) | ((b1 >> 6) << 4));
-      own |= sc << (8 * k + 16 * row);
-      s.mn[row + 2 * k] = min_halves(mn);
-    }
+  for (int i = 0; i < 3; ++i)
+    x[i] = __byte_perm(__byte_perm(head[0][0][i], head[0][1][i], two), __byte_perm(head[1][0][i], head[1][1][i], two), 0x5410);
+  // rows 0 - 3 of a group: the low six bits of words 0 (scale) and 1 (min); rows 4 - 7: a nibble of word 2 under their top bits
+  const uint32_t low = g < 4 ? 0x3f3f3f3fu : 0u, nib = g < 4 ? 0u : 0x0f0f0f0fu, top = g < 4 ? 0u : 0x30303030u;
+  const uint32_t own = (x[0] & low) | ((x[2] & nib) | ((x[0] >> 2) & top));
+  const uint32_t mins = (x[1] & low) | (((x[2] >> 4) & nib) | ((x[1] >> 2) & top));
+  s.mn[0] = min_halves<0>(mins);
+  s.mn[1] = min_halves<2>(mins);
+  s.mn[2] = min_halves<1>(mins);
+  s.mn[3] = min_halves<3>(mins);
 #pragma unroll
   for (int i = 0; i < 4; ++i)
     s.sc[i] = __shfl_sync(FULL, own, (lane & ~3) + i);
@@ -162,28 +154,9 @@ __device__ __forceinline__ void q4k_scales(Q4KScales &s, const BlockQ4Kx8 *lo, c
   }
   q4k_scales(s, head, d, g, lane);
 }
-/** scale of sub-block J of row g + 8 * row as a float (even J: as it is; odd J: over 16, because the high nibbles enter
- *  the MMA times 16): 0x4B0000bb is 2^23 + b, 0x490000bb is 2^19 + b / 16 */
-template <int J> __device__ __forceinline__ float q4k_scale(const Q4KScales &s, int row) {
-  const uint32_t w = __byte_perm(s.sc[J & 3], (J & 1) ? 0x49000000u : 0x4B000000u, 0x7440 | ((J >> 2) + 2 * row));
-  return __uint_as_float(w) - ((J & 1) ? 524288.f : 8388608.f);
-}
-struct Q4KFactors { // per pair and row: the two scales
-  float s0[4][2], s1[4][2];
-};
-__device__ __forceinline__ void q4k_factors(Q4KFactors &f, const Q4KScales &s) {
-  auto pair = [&](auto P) {
-    constexpr int p = decltype(P)::value;
-#pragma unroll
-    for (int row = 0; row < 2; ++row) {
-      f.s0[p][row] = q4k_scale<2 * p>(s, row);
-      f.s1[p][row] = q4k_scale<2 * p + 1>(s, row);
-    }
-  };
-  pair(std::integral_constant<int, 0>{});
-  pair(std::integral_constant<int, 1>{});
-  pair(std::integral_constant<int, 2>{});
-  pair(std::integral_constant<int, 3>{});
+/** scale of sub-block J of row g + 8 * row */
+template <int J> __device__ __forceinline__ int q4k_scale_int(const Q4KScales &s, int row) {
+  return (int)__byte_perm(s.sc[J & 3], 0, 0x4440 | ((J >> 2) + 2 * row));
 }
 
 /** One lane's view of a tile's unit. TH8: the tile is laid out for 8 rows. */
@@ -213,79 +186,59 @@ template <bool TH8> __device__ __forceinline__ void act_load(ActQ4K &a, const ui
   a.d = act_d<TH8>(unit, th, lane & 3);
 }
 
-/** Pair p of a 16 x 8 tile: f[c] = sc0 * I0 + sc1 * I1 (exact). c = 0..3: row g + 8 * (c / 2), activation row 2t + c % 2. */
-__device__ __forceinline__ void q4k_pair(float (&f)[4], const uint32_t (&al)[4], const uint32_t (&ah)[4], const uint4 &b,
-                                         const float (&s0)[2], const float (&s1)[2]) {
-  int lo[4], hi[4];
-  mma_u8s8(lo, al[0], al[1], al[2], al[3], b.x, b.y);
-  mma_u8s8(hi, ah[0], ah[1], ah[2], ah[3], b.z, b.w);
-#pragma unroll
-  for (int c = 0; c < 4; ++c) {
-    const int row = c >> 1;
-    f[c] = fmaf(s1[row], (float)hi[c], s0[row] * (float)lo[c]);
-  }
-}
-
 /* ------------------------------------------------------------------ Q4_0 */
-/** 16 rows x 256: word t of every 32-block of the rows g and g + 8 (elements 4t.. as low and 16 + 4t.. as high nibbles). */
-struct Q40Raw {
-  uint32_t q[8][2];
-  uint16_t d[8][2];
-};
-__device__ __forceinline__ void q40_load(Q40Raw &r, const BlockQ40x8 *lo, const BlockQ40x8 *hi, int n, int g, int t) {
-#pragma unroll
-  for (int j = 0; j < 8; ++j)
-#pragma unroll
-    for (int row = 0; row < 2; ++row) {
-      const BlockQ40x8 *b = (row ? hi : lo) + (j < n ? j : n - 1);
-      r.q[j][row] = ldg_stream_u32(b->qs + (t >> 1) * 64 + g * 8 + (t & 1) * 4);
-      r.d[j][row] = __ldg(&b->d[g]);
-    }
-}
 struct ActQ40 {
   uint4 b[4];
-  float d[2][8]; // rows 2t, 2t + 1
+  uint2 d[4]; // scales of the 32-blocks 2p, 2p + 1 of the rows 2t and 2t + 1
 };
-/** scales of the blocks 4h .. 4h + 3 of row i */
-__device__ __forceinline__ float4 act_d4(const uint8_t *unit, int i, int h) {
-  const uint2 d = *reinterpret_cast<const uint2 *>(unit + 256 * 8 + 16 * i + 8 * h);
-  const float2 lo = __half22float2(bits_h2(d.x)), hi = __half22float2(bits_h2(d.y));
-  return make_float4(lo.x, lo.y, hi.x, hi.y);
+__device__ __forceinline__ uint2 act_d2(const uint8_t *unit, int p, int t) {
+  return *reinterpret_cast<const uint2 *>(unit + 256 * 8 + 32 * p + 8 * t);
 }
 template <bool TH8> __device__ __forceinline__ void act_load(ActQ40 &a, const uint8_t *unit, int, int lane) {
   static_assert(TH8, "only Q4_K has a call with short tiles");
 #pragma unroll
-  for (int p = 0; p < 4; ++p)
+  for (int p = 0; p < 4; ++p) {
     a.b[p] = act_frag<true>(unit, p, 8, lane);
-#pragma unroll
-  for (int c = 0; c < 2; ++c)
-#pragma unroll
-    for (int h = 0; h < 2; ++h) {
-      const float4 d = act_d4(unit, 2 * (lane & 3) + c, h);
-      a.d[c][4 * h] = d.x, a.d[c][4 * h + 1] = d.y, a.d[c][4 * h + 2] = d.z, a.d[c][4 * h + 3] = d.w;
-    }
+    a.d[p] = act_d2(unit, p, lane & 3);
+  }
 }
-/** Block of a 16 x 8 tile: x[c] = 16 * (sum of (q - 8) * a). The stored nibble (q ^ 8) is q - 8 in two's complement, so
- *  in the upper half of a byte it is that times 16. q: low nibbles of rows g, g + 8, high nibbles of them, all moved there. */
-__device__ __forceinline__ void q40_block(float (&x)[4], const uint32_t (&q)[4], uint32_t b0, uint32_t b1) {
+/** a * b of two halves, exact in fp32: the instruction that multiplies halves into a float adds -0 */
+__device__ __forceinline__ float mul_halves(uint16_t a, uint16_t b) {
+  float d;
+  asm("fma.rn.f32.f16 %0, %1, %2, %3;" : "=f"(d) : "h"(a), "h"(b), "f"(-0.f));
+  return d;
+}
+/* A block of a 16 x 8 tile. The stored nibble (q ^ 8) is q - 8 in two's complement, so in the upper half of a byte it is that
+ * times 16, and everything that follows is taken times 16 too, down to the result, which is exact: the scales are halves, so a chain's
+ * values are multiples of 2^-48 and stay below 2^60 wherever they are numbers. */
+/** x: the sums times 16, s: the products of the scales; q: low nibbles of rows g, g + 8, high nibbles of them, in the upper halves of
+ *  the bytes; dw0, dw1: scales of the two rows; da: act_d2 of the pair of blocks of which this is number J */
+template <int J>
+__device__ __forceinline__ void q40_terms(float (&x)[4], float (&s)[4], const uint32_t (&q)[4], uint32_t b0, uint32_t b1, uint16_t dw0,
+                                          uint16_t dw1, uint2 da) {
   int v[4];
   mma_s8s8(v, q[0], q[1], q[2], q[3], b0, b1);
+  const uint16_t d0 = (uint16_t)(da.x >> (16 * J)), d1 = (uint16_t)(da.y >> (16 * J));
+  s[0] = mul_halves(dw0, d0), s[1] = mul_halves(dw0, d1), s[2] = mul_halves(dw1, d0), s[3] = mul_halves(dw1, d1);
 #pragma unroll
   for (int c = 0; c < 4; ++c)
     x[c] = (float)v[c];
 }
 
 /* ------------------------------------------------------- where a tile lies */
-/** Activation rows of one warp (or CTA): `rows` of them, outputs from position `pos`, tiles from `act_tile`; weights W. */
+/** Activation rows of one CTA: `rows` of them, outputs from position `pos`, tiles from act_k on of the act_tiles that start at
+ *  act_first; weights W. */
 struct Tile {
   const void *W;
-  int pos, rows, act_tile, z;
+  int pos, rows, act_first, act_tiles, act_k, z;
 };
 template <int NT> __device__ __forceinline__ bool find_tile(Tile &tl, const MmaArgs &a, int tile, bool grouped) {
   if (!grouped) {
     tl.W = a.W;
     tl.pos = tile * 8 * NT;
-    tl.act_tile = tile * NT;
+    tl.act_first = 0;
+    tl.act_tiles = (a.M + a.th - 1) / a.th;
+    tl.act_k = tile * NT;
     tl.rows = min(8 * NT, a.M - tl.pos);
     return true;
   }
@@ -303,8 +256,11 @@ template <int NT> __device__ __forceinline__ bool find_tile(Tile &tl, const MmaA
   const int k = tile - a.tile_off[lo], first = k * 8 * NT;
   tl.W = (tl.z ? a.w_table[1] : a.w_table[0])[lo];
   tl.pos = a.off[lo] + first;
-  tl.act_tile = a.act_off[lo] + k * NT;
-  tl.rows = min(8 * NT, a.off[lo + 1] - a.off[lo] - first);
+  const int all = a.off[lo + 1] - a.off[lo];
+  tl.act_first = a.act_off[lo];
+  tl.act_tiles = (all + 7) >> 3;
+  tl.act_k = k * NT;
+  tl.rows = min(8 * NT, all - first);
   return tl.rows > 0 && tl.W; // a null weight: expert of another rank
 }
 __device__ __forceinline__ float *out_row(const MmaArgs &a, const Tile &tl, int i, bool grouped) {
@@ -314,67 +270,81 @@ __device__ __forceinline__ float *out_row(const MmaArgs &a, const Tile &tl, int 
 
 /** One unit of a warp's 16 rows against up to 8 * NT activation rows in shared memory, chains in registers. The pair of
  *  sub-blocks is the outer loop, so that its fragments and factors are unpacked once for all tiles.
- *  CHAIN_FOUR: four steps per super-block; CHAIN_ONE: one; CHAIN_MIXED: four for the rows below m4 of the tile, one behind. */
+ *  CHAIN_FOUR: four steps per super-block; CHAIN_ONE: one; CHAIN_MIXED: four for the rows below m4 of the tile, one behind.
+ *  Scales meet the sums as integers: |sc * I| summed over a super-block stays below 2^25, and its one conversion rounds as the
+ *  reference's does. */
 enum { CHAIN_FOUR, CHAIN_ONE, CHAIN_MIXED };
 template <int N_TILES, int CHAIN, bool TH8, int NT>
 __device__ __forceinline__ void q4k_unit(float (&acc)[NT][4], float (&accm)[NT][4], const Q4KScales &sc, const BlockQ4Kx8 *w0,
                                          const BlockQ4Kx8 *w1, const uint8_t *act, int th, int m4, int g, int t,
                                          int lane) {
-  float s1[N_TILES][4], s2[N_TILES][4]; // four-step rows: d * da and dmin * da; one-step rows: the sums of pairs 0 + 1 and 2 + 3 (exact)
+  int sum[N_TILES][4];                  // one-step rows: of the super-block so far
+  float2 s1[N_TILES][2], s2[N_TILES][2]; // four-step rows: d * da and dmin * da of the rows 2t, 2t + 1
   uint32_t bs[N_TILES][2];
-  auto four = [&](int i, int c) { return CHAIN == CHAIN_FOUR || (CHAIN == CHAIN_MIXED && 8 * i + 2 * t + (c & 1) < m4); };
 #pragma unroll
   for (int i = 0; i < N_TILES; ++i) {
-      const uint8_t *unit = act + i * (8 * act_row_bytes(NNTR_Q4_K));
+    const uint8_t *unit = act + i * (8 * act_row_bytes(NNTR_Q4_K));
+    if (CHAIN != CHAIN_ONE) {
       const uint32_t sums = act_sums<TH8>(unit, th, lane);
       bs[i][0] = sum_halves<0>(sums);
       bs[i][1] = sum_halves<1>(sums);
-      if (CHAIN != CHAIN_ONE) {
-        const float2 d = act_d<TH8>(unit, th, t);
+      const float2 d = act_d<TH8>(unit, th, t);
 #pragma unroll
-        for (int c = 0; c < 4; ++c) {
-          s1[i][c] = four(i, c) ? __fmul_rn(sc.dw[c >> 1], (c & 1) ? d.y : d.x) : 0.f;
-          s2[i][c] = four(i, c) ? __fmul_rn(sc.dm[c >> 1], (c & 1) ? d.y : d.x) : 0.f;
-        }
-      } else {
-#pragma unroll
-        for (int c = 0; c < 4; ++c)
-          s1[i][c] = s2[i][c] = 0.f;
+      for (int r = 0; r < 2; ++r) {
+        s1[i][r] = mul2(sc.dw[r], sc.dw[r], d.x, d.y);
+        s2[i][r] = mul2(sc.dm[r], sc.dm[r], d.x, d.y);
       }
     }
+#pragma unroll
+    for (int c = 0; c < 4; ++c)
+      sum[i][c] = 0;
+  }
   auto pair = [&](auto P) {
     constexpr int p = decltype(P)::value;
     const uint2 q0 = *reinterpret_cast<const uint2 *>(w0->qs + ((4 * p + t) * 8 + g) * 8),
                 q1 = *reinterpret_cast<const uint2 *>(w1->qs + ((4 * p + t) * 8 + g) * 8);
     const uint32_t lo[4] = {q0.x & 0x0f0f0f0fu, q1.x & 0x0f0f0f0fu, q0.y & 0x0f0f0f0fu, q1.y & 0x0f0f0f0fu};
-    const uint32_t hi[4] = {q0.x & 0xf0f0f0f0u, q1.x & 0xf0f0f0f0u, q0.y & 0xf0f0f0f0u, q1.y & 0xf0f0f0f0u};
-    float f0[2], f1[2];
-#pragma unroll
-    for (int row = 0; row < 2; ++row) {
-      f0[row] = q4k_scale<2 * p>(sc, row);
-      f1[row] = q4k_scale<2 * p + 1>(sc, row);
-    }
+    const uint32_t hi[4] = {(q0.x >> 4) & 0x0f0f0f0fu, (q1.x >> 4) & 0x0f0f0f0fu, (q0.y >> 4) & 0x0f0f0f0fu,
+                            (q1.y >> 4) & 0x0f0f0f0fu};
+    const int f0[2] = {q4k_scale_int<2 * p>(sc, 0), q4k_scale_int<2 * p>(sc, 1)},
+              f1[2] = {q4k_scale_int<2 * p + 1>(sc, 0), q4k_scale_int<2 * p + 1>(sc, 1)};
     const bool own = (t >> 1) == (p & 1); // the lanes that hold the mins of this pair
     const uint32_t m0 = own ? sc.mn[2 * (p >> 1)] : 0u, m1 = own ? sc.mn[2 * (p >> 1) + 1] : 0u;
 #pragma unroll
     for (int i = 0; i < N_TILES; ++i) {
-        const uint4 x = act_frag<TH8>(act + i * (8 * act_row_bytes(NNTR_Q4_K)), p, th, lane);
-        float v[4], j[4];
-        q4k_pair(v, lo, hi, x, f0, f1);
-        if (CHAIN != CHAIN_ONE)
-          mma_f16_k8(j, m0, m1, bs[i][p >> 1]);
+      const uint4 x = act_frag<TH8>(act + i * (8 * act_row_bytes(NNTR_Q4_K)), p, th, lane);
+      int lo_sum[4], hi_sum[4];
+      mma_u8s8(lo_sum, lo[0], lo[1], lo[2], lo[3], x.x, x.y);
+      mma_u8s8(hi_sum, hi[0], hi[1], hi[2], hi[3], x.z, x.w);
+      if (CHAIN == CHAIN_ONE) {
+#pragma unroll
+        for (int c = 0; c < 4; ++c)
+          sum[i][c] += f0[c >> 1] * lo_sum[c] + f1[c >> 1] * hi_sum[c];
+        continue;
+      }
+      int v[4];
+#pragma unroll
+      for (int c = 0; c < 4; ++c)
+        v[c] = f0[c >> 1] * lo_sum[c] + f1[c >> 1] * hi_sum[c]; // below 2^23: exact as a float
+      float j[4];
+      mma_f16_k8(j, m0, m1, bs[i][p >> 1]);
+      if (CHAIN == CHAIN_FOUR) {
+#pragma unroll
+        for (int r = 0; r < 2; ++r) {
+          fma2(acc[i][2 * r], acc[i][2 * r + 1], (float)v[2 * r], (float)v[2 * r + 1], s1[i][r].x, s1[i][r].y);
+          fma2(accm[i][2 * r], accm[i][2 * r + 1], j[2 * r], j[2 * r + 1], s2[i][r].x, s2[i][r].y);
+        }
+      } else {
 #pragma unroll
         for (int c = 0; c < 4; ++c) {
-          if (CHAIN == CHAIN_FOUR || (CHAIN == CHAIN_MIXED && four(i, c))) {
-            acc[i][c] = __fmaf_rn(v[c], s1[i][c], acc[i][c]);
-            accm[i][c] = __fmaf_rn(j[c], s2[i][c], accm[i][c]);
-          } else if (p < 2) {
-            s1[i][c] += v[c];
-          } else {
-            s2[i][c] += v[c];
+          if (8 * i + 2 * t + (c & 1) < m4) {
+            acc[i][c] = __fmaf_rn((float)v[c], (c & 1) ? s1[i][c >> 1].y : s1[i][c >> 1].x, acc[i][c]);
+            accm[i][c] = __fmaf_rn(j[c], (c & 1) ? s2[i][c >> 1].y : s2[i][c >> 1].x, accm[i][c]);
           }
+          sum[i][c] += v[c];
         }
       }
+    }
   };
   pair(std::integral_constant<int, 0>{});
   pair(std::integral_constant<int, 1>{});
@@ -383,56 +353,67 @@ __device__ __forceinline__ void q4k_unit(float (&acc)[NT][4], float (&accm)[NT][
   if (CHAIN != CHAIN_FOUR) {
 #pragma unroll
     for (int i = 0; i < N_TILES; ++i) {
-        const float2 d = act_d<TH8>(act + i * (8 * act_row_bytes(NNTR_Q4_K)), th, t);
-        float j[4];
-        mma_f16_k16(j, sc.mn[0], sc.mn[1], sc.mn[2], sc.mn[3], bs[i][0], bs[i][1]);
+      const uint8_t *unit = act + i * (8 * act_row_bytes(NNTR_Q4_K));
+      const uint32_t sums = act_sums<TH8>(unit, th, lane);
+      const float2 d = act_d<TH8>(unit, th, t);
+      float j[4];
+      mma_f16_k16(j, sc.mn[0], sc.mn[1], sc.mn[2], sc.mn[3], sum_halves<0>(sums), sum_halves<1>(sums));
 #pragma unroll
-        for (int c = 0; c < 4; ++c)
-          if (CHAIN == CHAIN_ONE || !four(i, c)) { // one rounding of the exact sum of the super-block
-            const float da = (c & 1) ? d.y : d.x;
-            acc[i][c] = __fmaf_rn(__fadd_rn(s1[i][c], s2[i][c]), __fmul_rn(sc.dw[c >> 1], da), acc[i][c]);
-            accm[i][c] = __fmaf_rn(j[c], __fmul_rn(sc.dm[c >> 1], da), accm[i][c]);
-          }
+      for (int r = 0; r < 2; ++r) {
+        const float2 e1 = mul2(sc.dw[r], sc.dw[r], d.x, d.y), e2 = mul2(sc.dm[r], sc.dm[r], d.x, d.y);
+        if (CHAIN == CHAIN_ONE) { // one rounding of the exact sum of the super-block
+          fma2(acc[i][2 * r], acc[i][2 * r + 1], __int2float_rn(sum[i][2 * r]), __int2float_rn(sum[i][2 * r + 1]), e1.x, e1.y);
+          fma2(accm[i][2 * r], accm[i][2 * r + 1], j[2 * r], j[2 * r + 1], e2.x, e2.y);
+        } else {
+#pragma unroll
+          for (int k = 0; k < 2; ++k)
+            if (8 * i + 2 * t + k >= m4) {
+              const int c = 2 * r + k;
+              acc[i][c] = __fmaf_rn(__int2float_rn(sum[i][c]), k ? e1.y : e1.x, acc[i][c]);
+              accm[i][c] = __fmaf_rn(j[c], k ? e2.y : e2.x, accm[i][c]);
+            }
+        }
       }
+    }
   }
 }
 
-/** Q4_0: the n blocks of a unit, four at a time. */
-template <int N_TILES, int NT>
+/** Q4_0: the n blocks of a unit, two at a time. FULL: n is 8, no branches between them. */
+template <int N_TILES, bool FULL, int NT>
 __device__ __forceinline__ void q40_unit(float (&acc)[NT][4], const BlockQ40x8 *w0, const BlockQ40x8 *w1, const uint8_t *act,
                                          int n, int g, int t, int lane) {
 #pragma unroll
-  for (int h = 0; h < 2; ++h) {
-    if (4 * h >= n)
+  for (int p = 0; p < 4; ++p) {
+    if (!FULL && 2 * p >= n)
       break;
-    uint32_t q[4][4];
-    float dw[4][2];
+    uint32_t q[2][4];
+    uint16_t dw[2][2];
 #pragma unroll
-    for (int j = 0; j < 4; ++j) {
+    for (int j = 0; j < 2; ++j)
 #pragma unroll
       for (int row = 0; row < 2; ++row) {
-        // blocks past the end of the row: what the shared memory holds, with scale 0
-        const BlockQ40x8 *blk = (row ? w1 : w0) + 4 * h + j;
+        // a block past the end of the row: what the shared memory holds, with scale 0
+        const BlockQ40x8 *blk = (row ? w1 : w0) + 2 * p + j;
         const uint32_t w = *reinterpret_cast<const uint32_t *>(blk->qs + (t >> 1) * 64 + g * 8 + (t & 1) * 4);
         q[j][row] = (w << 4) & 0xf0f0f0f0u;
         q[j][row + 2] = w & 0xf0f0f0f0u;
-        dw[j][row] = 4 * h + j < n ? half_bits_to_float(blk->d[g]) * 0.0625f : 0.f; // the sums come times 16
+        dw[j][row] = FULL || 2 * p + j < n ? blk->d[g] : (uint16_t)0;
       }
-    }
 #pragma unroll
     for (int i = 0; i < N_TILES; ++i) {
       const uint8_t *unit = act + i * (8 * act_row_bytes(NNTR_Q4_0));
-      const uint4 x[2] = {act_frag<true>(unit, 2 * h, 8, lane), act_frag<true>(unit, 2 * h + 1, 8, lane)};
-      const float4 d0 = act_d4(unit, 2 * t, h), d1 = act_d4(unit, 2 * t + 1, h);
-      const float da[4][2] = {{d0.x, d1.x}, {d0.y, d1.y}, {d0.z, d1.z}, {d0.w, d1.w}};
+      const uint4 x = act_frag<true>(unit, p, 8, lane);
+      const uint2 da = act_d2(unit, p, t);
+      auto block = [&](auto J) {
+        constexpr int j = decltype(J)::value;
+        float v[4], s[4];
+        q40_terms<j>(v, s, q[j], j ? x.z : x.x, j ? x.w : x.y, dw[j][0], dw[j][1], da);
 #pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        float v[4];
-        q40_block(v, q[j], (j & 1) ? x[j >> 1].z : x[j >> 1].x, (j & 1) ? x[j >> 1].w : x[j >> 1].y);
-#pragma unroll
-        for (int c = 0; c < 4; ++c)
-          acc[i][c] = __fmaf_rn(v[c], __fmul_rn(dw[j][c >> 1], da[j][c & 1]), acc[i][c]);
-      }
+        for (int r = 0; r < 2; ++r)
+          fma2(acc[i][2 * r], acc[i][2 * r + 1], v[2 * r], v[2 * r + 1], s[2 * r], s[2 * r + 1]);
+      };
+      block(std::integral_constant<int, 0>{});
+      block(std::integral_constant<int, 1>{});
     }
   }
 }
@@ -446,39 +427,41 @@ template <int NT, typename F> __device__ __forceinline__ void with_tiles(int n, 
 }
 
 /* --------------------------------------------------- a warp owns its rows */
-constexpr int ROWS_WARPS = 4;
+constexpr int ROWS_WARPS = 4;                                    // that compute; a fifth one brings the data in
 constexpr int ROWS_W = ROWS_WARPS * 2 * (int)sizeof(BlockQ4Kx8); // the weights of a unit: 8 row groups (Q4_0: 8 blocks of 144)
 
 __device__ int g_mma_status = 0;
 
-template <int NT, int STAGES> struct RowsShared { // STAGES: units in flight per CTA
+/* Units in flight per CTA and the CTAs per SM that registers and shared memory are held to. More warps hide more latency until
+ * registers spill or the ring gets too short; measured with 2 to 5 stages and 2 to 9 CTAs. Q4_0 1000 x 8000 x 4096 with 3 / 4 / 5 CTAs
+ * of 32 rows 226 / 201 / 230 us; Q4_K (12 of 16 warps' worth of registers) 31 x 24576 x 4096 with 3 / 4: 51 / 70; 16 rows, 16 x 24576
+ * x 4096 with 3 / 4: 23 / 28. Q4_0 tiles of 8 rows per expert, 8 tokens through 4 of 32 experts of 2880 x 2880 with 6 / 7 / 8 CTAs:
+ * 102 / 88 / 95 (what counts there is how the last round fills). */
+template <int QT, int NT, bool GROUPED> constexpr int rows_stages() { return QT == NNTR_Q4_0 && NT == 1 && GROUPED ? 2 : 3; }
+template <int QT, int NT, bool GROUPED> constexpr int rows_ctas() {
+  return QT == NNTR_Q4_0 ? (NT >= 2 ? 4 : GROUPED ? 7 : 5) : (NT == 4 ? 3 : NT == 2 ? 3 + GROUPED : 4);
+}
+
+/** Up to 64 weight rows, `groups` row groups from group0 on, against the rows of a Tile; with every unit of 256 of K in the ring. */
+struct RowsItem {
+  Tile tl; // rows == 0: no more units
+  int group0, groups, b;
+};
+template <int NT, int STAGES> struct RowsShared {
   alignas(16) uint8_t w[STAGES][ROWS_W];
   alignas(16) uint8_t act[STAGES][NT * 8 * act_row_bytes(NNTR_Q4_K)];
   alignas(8) unsigned long long full[STAGES], empty[STAGES];
+  RowsItem item[STAGES];
   int abort_flag;
 };
 
 template <int QT, int NT, bool GROUPED, bool TH8, int STAGES>
-__global__ void __launch_bounds__(ROWS_WARPS * 32, NT == 4 ? 3 : 4) gemm_mma_rows_kernel(const MmaArgs a) {
+__global__ void __launch_bounds__(ROWS_WARPS * 32 + 32, rows_ctas<QT, NT, GROUPED>()) gemm_mma_rows_kernel(const MmaArgs a, int n_tiles, int n_z) {
   extern __shared__ __align__(16) uint8_t rows_smem[];
   RowsShared<NT, STAGES> &sh = *reinterpret_cast<RowsShared<NT, STAGES> *>(rows_smem);
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, g = lane >> 2, t = lane & 3;
-  const int n_groups = a.N / 8, group0 = blockIdx.y * (2 * ROWS_WARPS), groups = min(2 * ROWS_WARPS, n_groups - group0);
-  // this warp's two row groups inside the CTA's (past the end of N the last group is repeated and not stored)
-  const int wg0 = min(2 * warp, groups - 1), wg1 = min(2 * warp + 1, groups - 1);
-  const int nb = a.nb;
-  Tile tl;
-  tl.z = GROUPED ? blockIdx.z : 0;
-  if (GROUPED)
-    pdl_wait(); // tables and activation tiles come from the kernels before
-  if (!find_tile<NT>(tl, a, blockIdx.x, GROUPED))
-    return;
-  if (GROUPED && (reinterpret_cast<uintptr_t>(tl.W) & 15)) { // from a table in device memory: not seen by the launcher
-    if (tid == 0)
-      atomicExch(&g_mma_status, NNTR_CUDA_ERR_INVALID);
-    return;
-  }
-  const int nt = (tl.rows + 7) >> 3, th = TH8 ? 8 : a.th;
+  const int n_groups = a.N / 8, nb = a.nb;
+  const int th = TH8 ? 8 : a.th;
   volatile int *abort_flag = &sh.abort_flag;
   const uint32_t full0 = smem_u32(sh.full), empty0 = smem_u32(sh.empty);
   if (tid == 0) {
@@ -490,301 +473,419 @@ __global__ void __launch_bounds__(ROWS_WARPS * 32, NT == 4 ? 3 : 4) gemm_mma_row
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   __syncthreads();
-  /* thread 0: the copies of unit b, weights and activations apart so that the first weights need not wait for the
-   * kernel that writes the activations */
-  auto unit_bytes = [&](int b) { return QT == NNTR_Q4_K ? (int)sizeof(BlockQ4Kx8) : min(8, a.nblk - 8 * b) * (int)sizeof(BlockQ40x8); };
-  auto fetch_w = [&](int b) {
-    const int s = b % STAGES, bytes = unit_bytes(b);
-    const size_t row = QT == NNTR_Q4_K ? (size_t)nb * sizeof(BlockQ4Kx8) : (size_t)a.nblk * sizeof(BlockQ40x8);
-    const uint8_t *src = static_cast<const uint8_t *>(tl.W) + (size_t)group0 * row + (size_t)b * sizeof(BlockQ4Kx8);
-    mbar_expect_tx(full0 + 8 * s, groups * bytes + nt * th * act_row_bytes(QT));
-    for (int i = 0; i < groups; ++i)
-      bulk_g2s(smem_u32(sh.w[s]) + i * (int)sizeof(BlockQ4Kx8), src + i * row, bytes, full0 + 8 * s);
-  };
-  auto fetch_act = [&](int b) {
-    const int s = b % STAGES;
-    for (int i = 0; i < nt; ++i)
-      bulk_g2s(smem_u32(sh.act[s]) + i * (8 * act_row_bytes(QT)), act_unit<QT>(a.act, tl.act_tile + i, th, nb, b),
-               th * act_row_bytes(QT), full0 + 8 * s);
-  };
-  auto wait = [&](uint32_t bar, int use) {
-    return mbar_wait_bounded(bar, use & 1, abort_flag, &g_mma_status, 1u << 22, 2048);
-  };
-  if (tid == 0) {
-    for (int b = 0; b < STAGES - 1 && b < nb; ++b)
-      fetch_w(b);
-    if (!GROUPED)
-      pdl_wait(); // only this thread reads what the kernel before wrote
-    for (int b = 0; b < STAGES - 1 && b < nb; ++b)
-      fetch_act(b);
-  }
-  float acc[NT][4], accm[QT == NNTR_Q4_K ? NT : 1][4];
-#pragma unroll
-  for (int i = 0; i < NT; ++i)
-#pragma unroll
-    for (int c = 0; c < 4; ++c) {
-      acc[i][c] = 0.f;
-      if constexpr (QT == NNTR_Q4_K)
-        accm[i][c] = 0.f;
-    }
+  if (GROUPED)
+    pdl_wait(); // tables and activation tiles come from the kernels before
+  int slot = 0;
+  uint32_t par = 0;
   bool ok = true;
-  for (int b = 0; b < nb; ++b) {
-    // refill the slot that unit b - 1 left, then wait for this unit's own data
-    if (tid == 0 && b + STAGES - 1 < nb) {
-      if (b > 0)
-        ok = wait(empty0 + 8 * ((b - 1) % STAGES), (b - 1) / STAGES);
-      if (ok) {
-        fetch_w(b + STAGES - 1);
-        fetch_act(b + STAGES - 1);
+  auto next_slot = [&]() {
+    if (++slot == STAGES)
+      slot = 0, par ^= 1;
+  };
+  auto wait = [&](uint32_t bar, uint32_t parity) {
+    if (!__all_sync(FULL, mbar_try_wait(bar + 8 * slot, parity)))
+      ok = __all_sync(FULL, mbar_wait_bounded(bar + 8 * slot, parity, abort_flag, &g_mma_status, 1u << 22, 2048));
+    return ok;
+  };
+  if (warp == ROWS_WARPS) {
+    /* ---- A warp brings the units of all items in, a lane per copy. A bulk copy holds its warp for 50 ns, so the nine of a unit are
+     * kept away from the warps that compute. */
+    if (GROUPED)
+      n_tiles = a.tile_off[a.n_experts];
+    const int row_blocks = (n_groups + 2 * ROWS_WARPS - 1) / (2 * ROWS_WARPS), n_items = n_tiles * row_blocks * n_z;
+    const size_t row = QT == NNTR_Q4_K ? (size_t)nb * sizeof(BlockQ4Kx8) : (size_t)a.nblk * sizeof(BlockQ40x8);
+    auto fetch_act = [&](const RowsItem &it, int s) {
+      if (lane == 31)
+        bulk_g2s(smem_u32(sh.act[s]), act_unit<QT>(a.act, it.tl.act_first, it.tl.act_tiles, it.tl.act_k, th, nb, it.b),
+                 ((it.tl.rows + 7) >> 3) * th * act_row_bytes(QT), full0 + 8 * s);
+    };
+    int u = 0; // units so far; the activations of the first STAGES wait for the kernel that writes them
+    auto first_acts = [&]() {
+      if (!GROUPED)
+        pdl_wait();
+      for (int s = 0; s < u && s < STAGES; ++s)
+        fetch_act(sh.item[s], s);
+    };
+    // Whole rounds of items first. Those that are left over are cut into 2 or 4 parts of 32 or 16 weight rows where there are
+    // CTAs enough, so that the last round is shared by all of them.
+    const int rounds = n_items / (int)gridDim.x, left = n_items - rounds * (int)gridDim.x;
+    const int cut = left * 4 <= (int)gridDim.x ? 4 : left * 2 <= (int)gridDim.x ? 2 : 1;
+    for (int k = 0; k <= rounds && ok; ++k) { // tiles fastest: neighbouring CTAs share their weights
+      const bool whole = k < rounds;
+      if (!whole && (int)blockIdx.x >= left * cut)
+        break;
+      const int item = k * (int)gridDim.x + (int)blockIdx.x / (whole ? 1 : cut);
+      const int part = whole ? 0 : (int)blockIdx.x % cut, part_groups = 2 * ROWS_WARPS / (whole ? 1 : cut);
+      RowsItem it;
+      const int rest = item / n_tiles;
+      it.tl.z = rest / row_blocks;
+      it.group0 = (rest - it.tl.z * row_blocks) * (2 * ROWS_WARPS) + part * part_groups;
+      if (it.group0 >= n_groups)
+        continue;
+      if (!find_tile<NT>(it.tl, a, item - rest * n_tiles, GROUPED))
+        continue;
+      if (GROUPED && (reinterpret_cast<uintptr_t>(it.tl.W) & 15)) { // from a table in device memory: not seen by the launcher
+        if (lane == 0)
+          atomicExch(&g_mma_status, NNTR_CUDA_ERR_INVALID);
+        continue;
+      }
+      const int groups = min(part_groups, n_groups - it.group0), tiles = (it.tl.rows + 7) >> 3;
+      it.groups = groups;
+      const uint8_t *w = static_cast<const uint8_t *>(it.tl.W) + (size_t)(it.group0 + min(lane, groups - 1)) * row;
+      for (int b = 0; b < nb; ++b, ++u) {
+        if (u >= STAGES && !wait(empty0, par ^ 1))
+          break;
+        it.b = b;
+        const int bytes = QT == NNTR_Q4_K ? (int)sizeof(BlockQ4Kx8) : min(8, a.nblk - 8 * b) * (int)sizeof(BlockQ40x8);
+        if (lane == 0) {
+          sh.item[slot] = it;
+          mbar_expect_tx(full0 + 8 * slot, groups * bytes + tiles * th * act_row_bytes(QT));
+        }
+        __syncwarp();
+        if (lane < groups)
+          bulk_g2s(smem_u32(sh.w[slot]) + lane * (int)sizeof(BlockQ4Kx8), w + (size_t)b * sizeof(BlockQ4Kx8), bytes, full0 + 8 * slot);
+        if (u >= STAGES)
+          fetch_act(it, slot);
+        else if (u == STAGES - 1) {
+          ++u;
+          first_acts();
+          --u;
+        }
+        next_slot();
       }
     }
-    const int s = b % STAGES;
-    ok = ok && wait(full0 + 8 * s, b / STAGES);
-    if (!(ok = __all_sync(FULL, ok)))
-      break;
-    const uint8_t *act = sh.act[s];
-    if constexpr (QT == NNTR_Q4_K) {
-      const BlockQ4Kx8 *w0 = reinterpret_cast<const BlockQ4Kx8 *>(sh.w[s]) + wg0,
-                       *w1 = reinterpret_cast<const BlockQ4Kx8 *>(sh.w[s]) + wg1;
-      Q4KScales sc;
-      q4k_scales(sc, w0, w1, g, t, lane);
-      with_tiles<NT>(nt, [&](auto N) {
-        constexpr int n = decltype(N)::value;
-        if constexpr (GROUPED)
-          q4k_unit<n, CHAIN_ONE, true>(acc, accm, sc, w0, w1, act, 8, 0, g, t, lane);
-        else if (TH8 && tl.pos + tl.rows <= a.M4)
-          q4k_unit<n, CHAIN_FOUR, true>(acc, accm, sc, w0, w1, act, 8, 0, g, t, lane);
-        else if (TH8 && tl.pos >= a.M4)
-          q4k_unit<n, CHAIN_ONE, true>(acc, accm, sc, w0, w1, act, 8, 0, g, t, lane);
-        else // the last tile, with up to three rows of the one-step chain
-          q4k_unit<n, CHAIN_MIXED, TH8>(acc, accm, sc, w0, w1, act, th, a.M4 - tl.pos, g, t, lane);
-      });
-    } else {
-      const int n = min(8, a.nblk - 8 * b);
-      const BlockQ40x8 *w0 = reinterpret_cast<const BlockQ40x8 *>(sh.w[s] + wg0 * sizeof(BlockQ4Kx8)),
-                       *w1 = reinterpret_cast<const BlockQ40x8 *>(sh.w[s] + wg1 * sizeof(BlockQ4Kx8));
-      with_tiles<NT>(nt, [&](auto N) { q40_unit<decltype(N)::value>(acc, w0, w1, act, n, g, t, lane); });
+    if (u < STAGES)
+      first_acts();
+    if (ok && (u < STAGES || wait(empty0, par ^ 1)) && lane == 0) {
+      sh.item[slot].tl.rows = 0;
+      mbar_arrive(full0 + 8 * slot);
     }
-    // every lane's loads have been performed before the slot is given back (loads_before_refill() does the same here and costs 0.4 %
-    // of the grouped products)
-    __threadfence_block();
-    __syncwarp();
-    if (lane == 0)
-      mbar_arrive(empty0 + 8 * s);
+  } else {
+    float acc[NT][4], accm[QT == NNTR_Q4_K ? NT : 1][4];
+    while (wait(full0, par)) {
+      const Tile tl = sh.item[slot].tl;
+      const int group0 = sh.item[slot].group0, groups = sh.item[slot].groups;
+      if (tl.rows == 0)
+        break;
+      // this warp's two row groups inside the CTA's (past the end of N the last group is repeated and not stored)
+      const int wg0 = 2 * warp, wg1 = min(2 * warp + 1, groups - 1);
+      const int nt = wg0 < groups ? (tl.rows + 7) >> 3 : 0; // 0: nothing for this warp
+#pragma unroll
+      for (int i = 0; i < NT; ++i)
+#pragma unroll
+        for (int c = 0; c < 4; ++c) {
+          acc[i][c] = 0.f;
+          if constexpr (QT == NNTR_Q4_K)
+            accm[i][c] = 0.f;
+        }
+      for (int b = 0; b < nb; ++b) {
+        if (b > 0 && !wait(full0, par))
+          break;
+        const uint8_t *act = sh.act[slot];
+        if (nt == 0) {
+        } else if constexpr (QT == NNTR_Q4_K) {
+          const BlockQ4Kx8 *w0 = reinterpret_cast<const BlockQ4Kx8 *>(sh.w[slot]) + wg0,
+                           *w1 = reinterpret_cast<const BlockQ4Kx8 *>(sh.w[slot]) + wg1;
+          Q4KScales sc;
+          q4k_scales(sc, w0, w1, g, t, lane);
+          with_tiles<NT>(nt, [&](auto N) {
+            constexpr int n = decltype(N)::value;
+            if constexpr (GROUPED)
+              q4k_unit<n, CHAIN_ONE, true>(acc, accm, sc, w0, w1, act, 8, 0, g, t, lane);
+            else if (TH8 && tl.pos + tl.rows <= a.M4)
+              q4k_unit<n, CHAIN_FOUR, true>(acc, accm, sc, w0, w1, act, 8, 0, g, t, lane);
+            else if (TH8 && tl.pos >= a.M4)
+              q4k_unit<n, CHAIN_ONE, true>(acc, accm, sc, w0, w1, act, 8, 0, g, t, lane);
+            else // the last tile, with up to three rows of the one-step chain
+              q4k_unit<n, CHAIN_MIXED, TH8>(acc, accm, sc, w0, w1, act, th, a.M4 - tl.pos, g, t, lane);
+          });
+        } else {
+          const int n = min(8, a.nblk - 8 * b);
+          const BlockQ40x8 *w0 = reinterpret_cast<const BlockQ40x8 *>(sh.w[slot] + wg0 * sizeof(BlockQ4Kx8)),
+                           *w1 = reinterpret_cast<const BlockQ40x8 *>(sh.w[slot] + wg1 * sizeof(BlockQ4Kx8));
+          with_tiles<NT>(nt, [&](auto N) {
+            if (n == 8)
+              q40_unit<decltype(N)::value, true>(acc, w0, w1, act, 8, g, t, lane);
+            else
+              q40_unit<decltype(N)::value, false>(acc, w0, w1, act, n, g, t, lane);
+          });
+        }
+        // every lane's loads have been performed before the slot is given back (loads_before_refill() does the same here and costs
+        // 0.4 % of the grouped products)
+        __threadfence_block();
+        __syncwarp();
+        if (lane == 0)
+          mbar_arrive(empty0 + 8 * slot);
+        next_slot();
+      }
+      if (!ok)
+        break;
+#pragma unroll
+      for (int i = 0; i < NT; ++i)
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+          const int m = 8 * i + 2 * t + h;
+          if (m < tl.rows) {
+            float *out = out_row(a, tl, m, GROUPED) + (size_t)(group0 + 2 * warp) * 8 + g;
+#pragma unroll
+            for (int r = 0; r < 2; ++r)
+              if (wg0 + r < groups) {
+                const int c = 2 * r + h;
+                out[8 * r] = QT == NNTR_Q4_K ? __fsub_rn(acc[i][c], accm[QT == NNTR_Q4_K ? i : 0][c]) : acc[i][c] * 0.0625f;
+              }
+          }
+        }
+    }
   }
   if (!ok) { // a wait ran out: give the copies in flight time to land in this CTA's shared memory
     for (int i = 0; i < 1000; ++i)
       __nanosleep(1000);
-    return;
   }
-#pragma unroll
-  for (int i = 0; i < NT; ++i)
-#pragma unroll
-    for (int k = 0; k < 2; ++k) {
-      const int m = 8 * i + 2 * t + k;
-      if (m < tl.rows) {
-        float *out = out_row(a, tl, m, GROUPED) + (size_t)(group0 + 2 * warp) * 8 + g;
-#pragma unroll
-        for (int row = 0; row < 2; ++row)
-          if (2 * warp + row < groups) {
-            const int c = 2 * row + k;
-            out[8 * row] = QT == NNTR_Q4_K ? __fsub_rn(acc[i][c], accm[QT == NNTR_Q4_K ? i : 0][c]) : acc[i][c];
-          }
-      }
-    }
 }
 
 /* ------------------------------------------- eight warps along K, one tile */
 constexpr int KS_WARPS = 8;
-constexpr int KS_BUF = KS_WARPS * 2 * 128 * 16;          // terms of one step: [unit][half][output] float4
-constexpr int KS_DW = KS_WARPS * 16 * 8 * 4;             // [unit][row][8] floats (Q4_K uses two of them)
-constexpr int KS_DA = KS_WARPS * 8 * 8 * 4;              // [unit][activation row][8] floats (Q4_K uses one)
-constexpr int KS_SMEM = 2 * (KS_BUF + KS_DW + KS_DA);
+constexpr int KS_RING = 3;                                    // rounds of weights in flight
+constexpr int KS_W = 2 * KS_WARPS * (int)sizeof(BlockQ4Kx8);  // the weights of a round: 2 row groups x 8 units
+
+template <int NT> struct KsShared {
+  alignas(16) uint8_t w[KS_RING][KS_W];
+  alignas(16) float4 chain[KS_WARPS][NT][2][32]; // what the warp in front has added up, a lane's outputs each
+  alignas(8) unsigned long long full[KS_RING];
+  int abort_flag;
+};
+
+/** barrier `id` of two warps: the one in front arrives, the other one waits for it */
+__device__ __forceinline__ void pair_arrive(int id) { asm volatile("barrier.cta.arrive %0, 64;" ::"r"(id) : "memory"); }
+__device__ __forceinline__ void pair_sync(int id) { asm volatile("barrier.cta.sync %0, 64;" ::"r"(id) : "memory"); }
 
 template <int QT, int NT, bool GROUPED, bool TH8>
-__global__ void __launch_bounds__(KS_WARPS * 32) gemm_mma_ksplit_kernel(const MmaArgs a) {
+__global__ void __launch_bounds__(KS_WARPS * 32, 2) gemm_mma_ksplit_kernel(const MmaArgs a) {
   extern __shared__ __align__(16) uint8_t ks_smem[];
+  KsShared<NT> &sh = *reinterpret_cast<KsShared<NT> *>(ks_smem);
+  volatile int *abort_flag = &sh.abort_flag;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, g = lane >> 2, t = lane & 3;
   const int rt = blockIdx.y, nb = a.nb;
   const bool second = rt * 16 + 8 < a.N;
   const int per = (nb + KS_WARPS - 1) / KS_WARPS; // rounds
   const int upr = (nb + per - 1) / per;           // units per round, the same in every round but the last
+  const size_t row = QT == NNTR_Q4_K ? (size_t)nb * sizeof(BlockQ4Kx8) : (size_t)a.nblk * sizeof(BlockQ40x8); // bytes of a row group
+  if (tid == 0) {
+    for (int i = 0; i < KS_RING; ++i)
+      mbar_init(smem_u32(sh.full + i), 1);
+    sh.abort_flag = 0;
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  }
   Tile tl;
   tl.z = GROUPED ? blockIdx.z : 0;
-  Q4KRaw rk;
-  Q40Raw r0;
-  auto load = [&](int b) {
-    if constexpr (QT == NNTR_Q4_K) {
-      const BlockQ4Kx8 *w0 = static_cast<const BlockQ4Kx8 *>(tl.W) + (size_t)(2 * rt) * nb;
-      q4k_load(rk, w0 + b, (second ? w0 + nb : w0) + b, g, t);
-    } else {
-      const BlockQ40x8 *w0 = static_cast<const BlockQ40x8 *>(tl.W) + (size_t)(2 * rt) * a.nblk;
-      q40_load(r0, w0 + 8 * b, (second ? w0 + a.nblk : w0) + 8 * b, min(8, a.nblk - 8 * b), g, t);
-    }
+  if (GROUPED)
+    pdl_wait();
+  if (!find_tile<NT>(tl, a, blockIdx.x, GROUPED))
+    return;
+  const uint8_t *w = static_cast<const uint8_t *>(tl.W) + (size_t)(2 * rt) * row;
+  const bool copies = !(reinterpret_cast<uintptr_t>(w) & 15);
+  auto round_bytes = [&](int rd) { return (int)min((size_t)upr * sizeof(BlockQ4Kx8), row - (size_t)rd * upr * sizeof(BlockQ4Kx8)); };
+  auto fetch = [&](int rd, int slot) { // thread 0: a row group's units of a round are one piece of memory
+    const uint32_t bar = smem_u32(sh.full + slot), dst = smem_u32(sh.w[slot]);
+    const int bytes = round_bytes(rd);
+    mbar_expect_tx(bar, bytes * (1 + second));
+    for (int h = 0; h < 1 + second; ++h)
+      bulk_g2s(dst + h * (KS_W / 2), w + h * row + (size_t)rd * upr * sizeof(BlockQ4Kx8), bytes, bar);
   };
-  if constexpr (!GROUPED) { // the weights do not depend on the quantizer's kernel: fetched while it runs
-    find_tile<NT>(tl, a, blockIdx.x, false);
-    if (warp < upr)
-      load(warp);
+  if (tid == 0 && copies) // the weights do not depend on the quantizer's kernel: fetched while it runs
+    for (int rd = 0; rd < KS_RING && rd < per; ++rd)
+      fetch(rd, rd);
+  if (!GROUPED)
     pdl_wait();
-  } else {
-    pdl_wait();
-    if (!find_tile<NT>(tl, a, blockIdx.x, true))
-      return;
-    if (warp < upr)
-      load(warp);
-  }
+  __syncthreads();
   const int nt = (tl.rows + 7) >> 3, th = TH8 ? 8 : a.th;
-  // the chain of this thread: output o of the tile (row g + 8 * (o / 64), activation row 2t + (o / 32) % 2 with g, t of
-  // lane o % 32); Q4_K: threads 128.. add the mins term
-  const int o = tid & 127, kind = tid >> 7, oq = o >> 5, og = (o & 31) >> 2, ot = o & 3;
-  const int orow = og + 8 * (oq >> 1), oact = 2 * ot + (oq & 1);
-  float acc[NT];
-#pragma unroll
-  for (int i = 0; i < NT; ++i)
-    acc[i] = 0.f;
-  int step = 0;
+  using Act = std::conditional_t<QT == NNTR_Q4_K, ActQ4K, ActQ40>;
+  Act next; // activations of the step that comes next
+  auto load_act = [&](int rd, int i) {
+    if (warp < upr && rd * upr + warp < nb)
+      act_load<TH8>(next, act_unit<QT>(a.act, tl.act_first, tl.act_tiles, tl.act_k + i, th, nb, rd * upr + warp), th, lane);
+  };
+  load_act(0, 0);
+  bool ok = true;
+  int slot = 0;
+  uint32_t par = 0;
   for (int rd = 0; rd < per; ++rd) {
     const int b = rd * upr + warp;
-    const bool have = warp < upr && b < nb;
-    const int n_units = min(upr, nb - rd * upr);
-    float *dws = reinterpret_cast<float *>(ks_smem + 2 * KS_BUF + (rd & 1) * KS_DW);
-    Q4KScales sc;
-    Q4KFactors f;
-    uint2 qk[4][2];
-    uint32_t q0[8][2];
-    int n = 0;
-    if (have) {
-      if constexpr (QT == NNTR_Q4_K) {
-        q4k_scales(sc, rk.head, rk.d, g, lane);
-        q4k_factors(f, sc);
-#pragma unroll
-        for (int p = 0; p < 4; ++p)
-          qk[p][0] = rk.q[p][0], qk[p][1] = rk.q[p][1];
-        if (t == 0) {
-#pragma unroll
-          for (int row = 0; row < 2; ++row)
-            *reinterpret_cast<float2 *>(dws + (warp * 16 + g + 8 * row) * 8) = make_float2(sc.dw[row], sc.dm[row]);
-        }
-      } else {
-        n = min(8, a.nblk - 8 * b);
-#pragma unroll
-        for (int j = 0; j < 8; ++j)
-#pragma unroll
-          for (int row = 0; row < 2; ++row) {
-            q0[j][row] = r0.q[j][row];
-            if (t == (j >> 1)) // a missing block of the last unit: scale 0, the chain adds nothing
-              dws[(warp * 16 + g + 8 * row) * 8 + j] = j < n ? half_bits_to_float(r0.d[j][row]) * 0.0625f : 0.f;
-          }
-      }
-      if (rd + 1 < per && b + upr < nb)
-        load(b + upr);
+    uint8_t *wr = sh.w[slot];
+    if (!copies) { // weights that start at a multiple of 8: plain loads, round by round
+      const int bytes = round_bytes(rd);
+      __syncthreads();
+      for (int h = 0; h < 1 + second; ++h)
+        for (int i = tid * 8; i < bytes; i += KS_WARPS * 32 * 8)
+          *reinterpret_cast<uint2 *>(wr + h * (KS_W / 2) + i) = ldg_stream_u2(w + h * row + (size_t)rd * upr * sizeof(BlockQ4Kx8) + i);
+      __syncthreads();
     }
+    if (warp < upr && b < nb) {
+      if (copies && !__all_sync(FULL, mbar_try_wait(smem_u32(sh.full + slot), par)))
+        ok = mbar_wait_bounded(smem_u32(sh.full + slot), par, abort_flag, &g_mma_status, 1u << 22, 2048) && ok;
+      __syncwarp();
+      const uint8_t *u0 = wr + warp * sizeof(BlockQ4Kx8), *u1 = u0 + (second ? KS_W / 2 : 0);
+      Q4KScales sc;
+      if constexpr (QT == NNTR_Q4_K)
+        q4k_scales(sc, reinterpret_cast<const BlockQ4Kx8 *>(u0), reinterpret_cast<const BlockQ4Kx8 *>(u1), g, t, lane);
+      const int to_warp = warp + 1 < upr ? warp + 1 : 0;
 #pragma unroll
-    for (int i = 0; i < NT; ++i) {
-      if (i >= nt)
-        break;
-      float4 *buf = reinterpret_cast<float4 *>(ks_smem + (step & 1) * KS_BUF);
-      float *das = reinterpret_cast<float *>(ks_smem + 2 * (KS_BUF + KS_DW) + (step & 1) * KS_DA);
-      ++step;
-      if (have) {
-        const uint8_t *unit = act_unit<QT>(a.act, tl.act_tile + i, th, nb, b);
-        float4 *mine = buf + warp * 256 + lane;
-        if constexpr (QT == NNTR_Q4_K) {
-          ActQ4K x;
-          act_load<TH8>(x, unit, th, lane);
-          if (g == 0)
-            das[(warp * 8 + 2 * t) * 8] = x.d.x, das[(warp * 8 + 2 * t + 1) * 8] = x.d.y;
-          const uint32_t bs0 = sum_halves<0>(x.sums), bs1 = sum_halves<1>(x.sums);
-          float v[4][4], j[4][4];
-#pragma unroll
-          for (int p = 0; p < 4; ++p) {
-            const uint32_t lo[4] = {qk[p][0].x & 0x0f0f0f0fu, qk[p][1].x & 0x0f0f0f0fu, qk[p][0].y & 0x0f0f0f0fu, qk[p][1].y & 0x0f0f0f0fu};
-            const uint32_t hi[4] = {qk[p][0].x & 0xf0f0f0f0u, qk[p][1].x & 0xf0f0f0f0u, qk[p][0].y & 0xf0f0f0f0u, qk[p][1].y & 0xf0f0f0f0u};
-            q4k_pair(v[p], lo, hi, x.b[p], f.s0[p], f.s1[p]);
-            mma_f16_k8(j[p], sc.mn[2 * (p >> 1)], sc.mn[2 * (p >> 1) + 1], (t >> 1) == (p & 1) ? (p < 2 ? bs0 : bs1) : 0u);
-          }
-#pragma unroll
-          for (int c = 0; c < 4; ++c) {
-            mine[32 * c] = make_float4(v[0][c], v[1][c], v[2][c], v[3][c]);
-            mine[128 + 32 * c] = make_float4(j[0][c], j[1][c], j[2][c], j[3][c]);
-          }
-        } else {
-          ActQ40 x;
-          act_load<TH8>(x, unit, th, lane);
-          if (g == 0) {
-#pragma unroll
-            for (int c = 0; c < 2; ++c)
-#pragma unroll
-              for (int j = 0; j < 8; ++j)
-                das[(warp * 8 + 2 * t + c) * 8 + j] = x.d[c][j];
-          }
-#pragma unroll
-          for (int h = 0; h < 2; ++h) {
-            float v[4][4];
-#pragma unroll
-            for (int j = 0; j < 4; ++j) {
-              const uint4 bb = x.b[2 * h + (j >> 1)];
-              const uint32_t w0 = q0[4 * h + j][0], w1 = q0[4 * h + j][1];
-              const uint32_t qq[4] = {(w0 << 4) & 0xf0f0f0f0u, (w1 << 4) & 0xf0f0f0f0u, w0 & 0xf0f0f0f0u, w1 & 0xf0f0f0f0u};
-              q40_block(v[j], qq, (j & 1) ? bb.z : bb.x, (j & 1) ? bb.w : bb.y);
-            }
+      for (int i = 0; i < NT; ++i) {
+        if (i >= nt)
+          break;
+        const Act x = next;
+        if (i + 1 < nt)
+          load_act(rd, i + 1);
+        else if (rd + 1 < per)
+          load_act(rd + 1, 0);
+        float acc[4], accm[4];
+        /* The chains go through the warps: this one takes them over when the units in front have been added. */
+        auto receive = [&]() {
+          if (b == 0) {
 #pragma unroll
             for (int c = 0; c < 4; ++c)
-              mine[128 * h + 32 * c] = make_float4(v[0][c], v[1][c], v[2][c], v[3][c]);
+              acc[c] = accm[c] = 0.f;
+            return;
+          }
+          pair_sync(warp * NT + i);
+          const float4 f = sh.chain[warp][i][0][lane];
+          acc[0] = f.x, acc[1] = f.y, acc[2] = f.z, acc[3] = f.w;
+          if constexpr (QT == NNTR_Q4_K) {
+            const float4 m = sh.chain[warp][i][1][lane];
+            accm[0] = m.x, accm[1] = m.y, accm[2] = m.z, accm[3] = m.w;
+          }
+        };
+        if constexpr (QT == NNTR_Q4_K) {
+          int v[4][4];
+          auto pair = [&](auto P) {
+            constexpr int p = decltype(P)::value;
+            const uint2 q0 = *reinterpret_cast<const uint2 *>(reinterpret_cast<const BlockQ4Kx8 *>(u0)->qs + ((4 * p + t) * 8 + g) * 8),
+                        q1 = *reinterpret_cast<const uint2 *>(reinterpret_cast<const BlockQ4Kx8 *>(u1)->qs + ((4 * p + t) * 8 + g) * 8);
+            int lo[4], hi[4];
+            mma_u8s8(lo, q0.x & 0x0f0f0f0fu, q1.x & 0x0f0f0f0fu, q0.y & 0x0f0f0f0fu, q1.y & 0x0f0f0f0fu, x.b[p].x, x.b[p].y);
+            mma_u8s8(hi, (q0.x >> 4) & 0x0f0f0f0fu, (q1.x >> 4) & 0x0f0f0f0fu, (q0.y >> 4) & 0x0f0f0f0fu, (q1.y >> 4) & 0x0f0f0f0fu,
+                     x.b[p].z, x.b[p].w);
+#pragma unroll
+            for (int c = 0; c < 4; ++c)
+              v[p][c] = q4k_scale_int<2 * p>(sc, c >> 1) * lo[c] + q4k_scale_int<2 * p + 1>(sc, c >> 1) * hi[c];
+          };
+          pair(std::integral_constant<int, 0>{});
+          pair(std::integral_constant<int, 1>{});
+          pair(std::integral_constant<int, 2>{});
+          pair(std::integral_constant<int, 3>{});
+          const uint32_t bs[2] = {sum_halves<0>(x.sums), sum_halves<1>(x.sums)};
+          float2 s1[2], s2[2];
+#pragma unroll
+          for (int r = 0; r < 2; ++r) {
+            s1[r] = mul2(sc.dw[r], sc.dw[r], x.d.x, x.d.y);
+            s2[r] = mul2(sc.dm[r], sc.dm[r], x.d.x, x.d.y);
+          }
+          const int m4 = GROUPED ? 0 : a.M4 - tl.pos - 8 * i; // rows of the tile below it take four steps, the others one
+          float vf[4][4], jf[4][4], v1[4], j1[4];
+          if (m4 > 0) {
+#pragma unroll
+            for (int p = 0; p < 4; ++p) {
+              mma_f16_k8(jf[p], sc.mn[2 * (p >> 1)], sc.mn[2 * (p >> 1) + 1], (t >> 1) == (p & 1) ? bs[p >> 1] : 0u);
+#pragma unroll
+              for (int c = 0; c < 4; ++c)
+                vf[p][c] = (float)v[p][c]; // below 2^23: exact
+            }
+          }
+          if (m4 < 8) {
+            mma_f16_k16(j1, sc.mn[0], sc.mn[1], sc.mn[2], sc.mn[3], bs[0], bs[1]);
+#pragma unroll
+            for (int c = 0; c < 4; ++c)
+              v1[c] = __int2float_rn((v[0][c] + v[1][c]) + (v[2][c] + v[3][c])); // one rounding of the exact sum
+          }
+          receive();
+          if (m4 >= 8) {
+#pragma unroll
+            for (int p = 0; p < 4; ++p)
+#pragma unroll
+              for (int r = 0; r < 2; ++r) {
+                fma2(acc[2 * r], acc[2 * r + 1], vf[p][2 * r], vf[p][2 * r + 1], s1[r].x, s1[r].y);
+                fma2(accm[2 * r], accm[2 * r + 1], jf[p][2 * r], jf[p][2 * r + 1], s2[r].x, s2[r].y);
+              }
+          } else if (m4 <= 0) {
+#pragma unroll
+            for (int r = 0; r < 2; ++r) {
+              fma2(acc[2 * r], acc[2 * r + 1], v1[2 * r], v1[2 * r + 1], s1[r].x, s1[r].y);
+              fma2(accm[2 * r], accm[2 * r + 1], j1[2 * r], j1[2 * r + 1], s2[r].x, s2[r].y);
+            }
+          } else {
+#pragma unroll
+            for (int c = 0; c < 4; ++c) {
+              const float e1 = (c & 1) ? s1[c >> 1].y : s1[c >> 1].x, e2 = (c & 1) ? s2[c >> 1].y : s2[c >> 1].x;
+              if (2 * t + (c & 1) < m4) {
+#pragma unroll
+                for (int p = 0; p < 4; ++p) {
+                  acc[c] = __fmaf_rn(vf[p][c], e1, acc[c]);
+                  accm[c] = __fmaf_rn(jf[p][c], e2, accm[c]);
+                }
+              } else {
+                acc[c] = __fmaf_rn(v1[c], e1, acc[c]);
+                accm[c] = __fmaf_rn(j1[c], e2, accm[c]);
+              }
+            }
+          }
+        } else {
+          const int n = min(8, a.nblk - 8 * b);
+          float v[8][4], s[8][4];
+          auto block = [&](auto J) {
+            constexpr int j = decltype(J)::value;
+            // a block past the end of the row: what the shared memory holds, with scale 0
+            const BlockQ40x8 *k0 = reinterpret_cast<const BlockQ40x8 *>(u0) + j, *k1 = reinterpret_cast<const BlockQ40x8 *>(u1) + j;
+            const uint4 bb = x.b[j >> 1];
+            const uint32_t at = (t >> 1) * 64 + g * 8 + (t & 1) * 4;
+            const uint32_t w0 = *reinterpret_cast<const uint32_t *>(k0->qs + at), w1 = *reinterpret_cast<const uint32_t *>(k1->qs + at);
+            const uint32_t qq[4] = {(w0 << 4) & 0xf0f0f0f0u, (w1 << 4) & 0xf0f0f0f0u, w0 & 0xf0f0f0f0u, w1 & 0xf0f0f0f0u};
+            q40_terms<j & 1>(v[j], s[j], qq, (j & 1) ? bb.z : bb.x, (j & 1) ? bb.w : bb.y,
+                             j < n ? k0->d[g] : (uint16_t)0, j < n ? k1->d[g] : (uint16_t)0, x.d[j >> 1]);
+          };
+          block(std::integral_constant<int, 0>{});
+          block(std::integral_constant<int, 1>{});
+          block(std::integral_constant<int, 2>{});
+          block(std::integral_constant<int, 3>{});
+          block(std::integral_constant<int, 4>{});
+          block(std::integral_constant<int, 5>{});
+          block(std::integral_constant<int, 6>{});
+          block(std::integral_constant<int, 7>{});
+          receive();
+#pragma unroll
+          for (int j = 0; j < 8; ++j)
+#pragma unroll
+            for (int r = 0; r < 2; ++r)
+              fma2(acc[2 * r], acc[2 * r + 1], v[j][2 * r], v[j][2 * r + 1], s[j][2 * r], s[j][2 * r + 1]);
+        }
+        if (b + 1 < nb) {
+          sh.chain[to_warp][i][0][lane] = make_float4(acc[0], acc[1], acc[2], acc[3]);
+          if constexpr (QT == NNTR_Q4_K)
+            sh.chain[to_warp][i][1][lane] = make_float4(accm[0], accm[1], accm[2], accm[3]);
+          pair_arrive(to_warp * NT + i);
+        } else if (ok) {
+#pragma unroll
+          for (int c = 0; c < 4; ++c) {
+            const int m = 8 * i + 2 * t + (c & 1);
+            if (m < tl.rows && (c < 2 || second))
+              out_row(a, tl, m, GROUPED)[rt * 16 + g + 8 * (c >> 1)] = QT == NNTR_Q4_K ? __fsub_rn(acc[c], accm[c]) : acc[c] * 0.0625f;
           }
         }
       }
-      __syncthreads();
-      // the chains: terms in ascending K order
-      if constexpr (QT == NNTR_Q4_K) {
-        const bool four = !GROUPED && tl.pos + 8 * i + oact < a.M4;
-        for (int u = 0; u < n_units; ++u) {
-          const float4 v = buf[u * 256 + 128 * kind + o];
-          const float s = __fmul_rn(dws[(u * 16 + orow) * 8 + kind], das[(u * 8 + oact) * 8]);
-          if (four) {
-            acc[i] = __fmaf_rn(v.x, s, acc[i]);
-            acc[i] = __fmaf_rn(v.y, s, acc[i]);
-            acc[i] = __fmaf_rn(v.z, s, acc[i]);
-            acc[i] = __fmaf_rn(v.w, s, acc[i]);
-          } else { // one rounding of the exact sum: the halves stay below 2^24
-            acc[i] = __fmaf_rn(__fadd_rn(v.x + v.y, v.z + v.w), s, acc[i]);
-          }
-        }
-      } else if (kind == 0) {
-        for (int u = 0; u < n_units; ++u) {
-          const float4 v0 = buf[u * 256 + o], v1 = buf[u * 256 + 128 + o];
-          const float4 *dw = reinterpret_cast<const float4 *>(dws + (u * 16 + orow) * 8);
-          const float4 *da = reinterpret_cast<const float4 *>(das + (u * 8 + oact) * 8);
-          const float4 w0 = dw[0], w1 = dw[1], a0 = da[0], a1 = da[1];
-          acc[i] = __fmaf_rn(v0.x, __fmul_rn(w0.x, a0.x), acc[i]);
-          acc[i] = __fmaf_rn(v0.y, __fmul_rn(w0.y, a0.y), acc[i]);
-          acc[i] = __fmaf_rn(v0.z, __fmul_rn(w0.z, a0.z), acc[i]);
-          acc[i] = __fmaf_rn(v0.w, __fmul_rn(w0.w, a0.w), acc[i]);
-          acc[i] = __fmaf_rn(v1.x, __fmul_rn(w1.x, a1.x), acc[i]);
-          acc[i] = __fmaf_rn(v1.y, __fmul_rn(w1.y, a1.y), acc[i]);
-          acc[i] = __fmaf_rn(v1.z, __fmul_rn(w1.z, a1.z), acc[i]);
-          acc[i] = __fmaf_rn(v1.w, __fmul_rn(w1.w, a1.w), acc[i]);
+      // The chains of this round's first unit have come through every unit of the round before, so nobody reads its weights any more.
+      if (warp == 0 && rd > 0 && rd - 1 + KS_RING < per && copies) {
+        __syncwarp();
+        if (lane == 0 && ok) {
+          loads_before_refill();
+          fetch(rd - 1 + KS_RING, slot ? slot - 1 : KS_RING - 1);
         }
       }
     }
+    if (++slot == KS_RING)
+      slot = 0, par ^= 1;
   }
-  float *fin = reinterpret_cast<float *>(ks_smem);
-  if constexpr (QT == NNTR_Q4_K) {
-    __syncthreads(); // the last chains have read the buffers
-    if (kind)
-#pragma unroll
-      for (int i = 0; i < NT; ++i)
-        fin[i * 128 + o] = acc[i];
-    __syncthreads();
-  }
-  if (kind == 0 && (orow < 8 || second)) {
-#pragma unroll
-    for (int i = 0; i < NT; ++i)
-      if (8 * i + oact < tl.rows) {
-        float *out = out_row(a, tl, 8 * i + oact, GROUPED) + rt * 16 + orow;
-        *out = QT == NNTR_Q4_K ? __fsub_rn(acc[i], fin[i * 128 + o]) : acc[i];
-      }
+  if (!ok) { // a wait ran out: give the copies in flight time to land in this CTA's shared memory
+    for (int i = 0; i < 1000; ++i)
+      __nanosleep(1000);
   }
 }
 
@@ -802,16 +903,18 @@ act_tiles_kernel(const float *__restrict__ x, int64_t ldx, uint8_t *__restrict__
   if (w >= (int64_t)M * nb)
     return;
   const int pos = (int)(w / nb), b = (int)(w - (int64_t)pos * nb);
-  int row = pos, tile = pos / th, i = pos - tile * th;
+  int row = pos, first = 0, n_tiles = (M + th - 1) / th, tile = pos / th, i = pos - tile * th;
   if (perm) {
     pdl_wait();
     const int pair = perm[pos], e = idx[pair];
     row = pair / a_div;
     i = pos - off[e];
-    tile = act_off[e] + (i >> 3);
+    first = act_off[e];
+    n_tiles = (off[e + 1] - off[e] + 7) >> 3;
+    tile = i >> 3;
     i &= 7;
   }
-  uint8_t *unit = act_unit<QT>(act, tile, th, nb, b);
+  uint8_t *unit = act_unit<QT>(act, first, n_tiles, tile, th, nb, b);
   const float *src = x + (int64_t)row * ldx + (int64_t)b * QK_K + lane * 8;
   if constexpr (QT == NNTR_Q4_K) {
     put_q8K(unit, th, i, q8K_quantize_warp(*reinterpret_cast<const float4 *>(src), *reinterpret_cast<const float4 *>(src + 4),
@@ -843,29 +946,30 @@ cudaError_t launch(void (*kernel)(KArgs...), dim3 grid, unsigned block, size_t s
 }
 
 template <int QT, int NT, bool GROUPED, bool TH8>
-int run_tiles(const MmaArgs &a, unsigned tiles, unsigned z, bool ksplit, bool shallow, cudaStream_t st) {
+int run_tiles(const MmaArgs &a, unsigned tiles, unsigned z, bool ksplit, cudaStream_t st) {
   const unsigned row_tiles = (unsigned)((a.N + 15) / 16);
+  constexpr int stages = rows_stages<QT, NT, GROUPED>(), ctas = rows_ctas<QT, NT, GROUPED>();
+  constexpr size_t smem = sizeof(RowsShared<NT, stages>);
   static bool attr_set[64] = {};
   int dev = 0;
   NNTR_CHECK_CUDA(cudaGetDevice(&dev));
   if (dev < 64 && !attr_set[dev]) {
-    NNTR_CHECK_CUDA(cudaFuncSetAttribute(gemm_mma_ksplit_kernel<QT, NT, GROUPED, TH8>,
-                                         cudaFuncAttributeMaxDynamicSharedMemorySize, KS_SMEM));
-    NNTR_CHECK_CUDA(cudaFuncSetAttribute(gemm_mma_rows_kernel<QT, NT, GROUPED, TH8, 3>,
-                                         cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(RowsShared<NT, 3>)));
+    if constexpr (NT <= 2)
+      NNTR_CHECK_CUDA(cudaFuncSetAttribute(gemm_mma_ksplit_kernel<QT, NT, GROUPED, TH8>,
+                                           cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(KsShared<NT>)));
+    NNTR_CHECK_CUDA(cudaFuncSetAttribute(gemm_mma_rows_kernel<QT, NT, GROUPED, TH8, stages>,
+                                         cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     attr_set[dev] = true;
   }
-  const dim3 rows_grid(tiles, (row_tiles + ROWS_WARPS - 1) / ROWS_WARPS, z);
-  cudaError_t e;
-  if (ksplit) {
-    e = launch(gemm_mma_ksplit_kernel<QT, NT, GROUPED, TH8>, dim3(tiles, row_tiles, z), KS_WARPS * 32, KS_SMEM, st, a);
+  cudaError_t e = cudaSuccess;
+  if (NT <= 2 && ksplit) {
+    if constexpr (NT <= 2)
+      e = launch(gemm_mma_ksplit_kernel<QT, NT, GROUPED, TH8>, dim3(tiles, row_tiles, z), KS_WARPS * 32, sizeof(KsShared<NT>), st, a);
   } else {
-    auto kernel = gemm_mma_rows_kernel<QT, NT, GROUPED, TH8, 3>;
-    size_t smem = sizeof(RowsShared<NT, 3>);
-    if constexpr (QT == NNTR_Q4_0 && NT == 1 && GROUPED) // 23 KB: no opt-in
-      if (shallow)
-        kernel = gemm_mma_rows_kernel<QT, NT, GROUPED, TH8, 2>, smem = sizeof(RowsShared<NT, 2>);
-    e = launch(kernel, rows_grid, ROWS_WARPS * 32, smem, st, a);
+    const uint64_t items = (uint64_t)tiles * ((row_tiles + ROWS_WARPS - 1) / ROWS_WARPS) * z;
+    const uint64_t slots = (uint64_t)ctas * (unsigned)sm_count();
+    e = launch(gemm_mma_rows_kernel<QT, NT, GROUPED, TH8, stages>, dim3((unsigned)(4 * items < slots ? 4 * items : slots)), ROWS_WARPS * 32 + 32,
+               smem, st, a, (int)tiles, (int)z);
   }
   count_launch();
   return check_cuda(e, "gemm (integer warp MMA) launch");
@@ -900,25 +1004,42 @@ int launch_gemm_mma(int qtype, unsigned M, unsigned M4, unsigned N, unsigned K, 
                                  nullptr, 1);
   count_launch();
   NNTR_CHECK_CUDA(cudaGetLastError());
-  const int nt = M <= 8 ? 1 : M <= 16 ? 2 : 4;
-  const unsigned tiles = (M + 8 * nt - 1) / (8 * nt);
-  // a warp per 16 x 8nt tile fills the machine from about 8 warps per SM up; below, the warps of a CTA share the tile. Weights
-  // that are not 16-byte aligned cannot be fetched by bulk copies: the shared tile's loads of at most 8 bytes take them all.
-  const bool ksplit = (uint64_t)tiles * ((N + 15) / 16) < 8u * (unsigned)sm_count() || (reinterpret_cast<uintptr_t>(B) & 15);
+  // Weights that are not 16-byte aligned cannot be fetched by bulk copies: the shared tile's plain loads take them all.
+  const bool misaligned = reinterpret_cast<uintptr_t>(B) & 15;
+  const unsigned row_tiles = (N + 15) / 16, row_blocks = (N + 63) / 64, sms = (unsigned)sm_count();
+  const auto tiles_of = [&](unsigned nt) { return (M + 8 * nt - 1) / (8 * nt); };
+  // One CTA per tile of 8 or 16 rows as long as all of them run at once, two per SM. Beyond that a warp per tile: of 32 rows (the
+  // weights are unpacked once for them) where CTAs of 64 weight rows still give every SM work, else of 16, else of 8. Measured on both
+  // sides: Q4_K 8 x 2560 x 2560 (160 CTAs) 6.4 us, a warp per tile 8.8; 8 x 6144 x 2560 (384) 9.5 and 9.0; 31 x 2560 x 2560 (320 of 16
+  // rows) 12.6 and 11.4. A warp per tile of 16 / 32 rows: Q4_K 31 x 12288 x 4096 (192 items of 32) 27.5 / 36.9 us, 63 x 9728 x 2560
+  // (304) 22.8 / 22.0; Q4_0 31 x 2560 x 2560 (40) 9.2 / 10.9, 64 x 2880 x 2880 (90) 12.8 / 12.7, 31 x 12288 x 4096 (192) 23.1 / 20.6;
+  // of 8 / 16 rows: Q4_K 31 x 2560 x 2560 (80 of 16) 11.4 / 11.8, 16 x 6144 x 2560 (96) 10.8 / 10.6.
+  const bool ksplit = misaligned || (uint64_t)tiles_of(2) * row_tiles <= 2u * sms;
+  unsigned nt;
+  if (ksplit)
+    nt = (uint64_t)tiles_of(1) * row_tiles <= 2u * sms ? 1 : 2;
+  else if (qtype == NNTR_Q4_K)
+    nt = M <= 8 ? 1 : M > 16 && tiles_of(4) * row_blocks >= 2 * sms ? 4 : 3 * tiles_of(2) * row_blocks >= 2 * sms ? 2 : 1;
+  else
+    nt = M <= 8 ? 1 : M > 16 && 3 * tiles_of(4) * row_blocks >= 2 * sms ? 4 : 2;
+  const unsigned tiles = tiles_of(a.th < 8 ? 1 : nt);
   if (a.th < 8)
-    return run_tiles<NNTR_Q4_K, 1, false, false>(a, tiles, 1, ksplit, false, st);
+    return run_tiles<NNTR_Q4_K, 1, false, false>(a, tiles, 1, ksplit, st);
 #define NNTR_MMA_RUN(QT)                                                                                               \
-  (nt == 1   ? run_tiles<QT, 1, false, true>(a, tiles, 1, ksplit, false, st)                                                  \
-   : nt == 2 ? run_tiles<QT, 2, false, true>(a, tiles, 1, ksplit, false, st)                                                  \
-             : run_tiles<QT, 4, false, true>(a, tiles, 1, ksplit, false, st))
+  (nt == 1   ? run_tiles<QT, 1, false, true>(a, tiles, 1, ksplit, st)                                                  \
+   : nt == 2 ? run_tiles<QT, 2, false, true>(a, tiles, 1, ksplit, st)                                                  \
+             : run_tiles<QT, 4, false, true>(a, tiles, 1, ksplit, st))
   return qtype == NNTR_Q4_K ? NNTR_MMA_RUN(NNTR_Q4_K) : NNTR_MMA_RUN(NNTR_Q4_0);
 #undef NNTR_MMA_RUN
 }
 
-int grouped_tile_rows(unsigned pairs, unsigned n_experts) {
-  // tiles of 8, 16 or 32 rows: about what an expert gets, so that few experts need a second tile (which fetches the
-  // expert's weights again) and short ones carry little padding
-  return pairs <= 6 * n_experts ? 8 : pairs <= 12 * n_experts ? 16 : 32;
+int grouped_tile_rows(int qtype, unsigned pairs, unsigned n_experts) {
+  // Tiles of about what an expert gets, so that few experts need a second tile (which fetches and unpacks the expert's weights
+  // again). A warp skips the rows that a tile lacks, so a large tile costs registers only. Q4_K, 8 of 128 experts of 2048 x 768, 32 /
+  // 100 / 200 / 256 tokens in tiles of 16 and of 32: 105 / 123 / 153 / 184 us and 119 / 138 / 160 / 178; tiles of 8 are behind or
+  // level (109 / 132 / 204 / 242). Q4_0, 4 of 32 of 2880 x 2880, 8 / 40 / 64 / 100 tokens in tiles of 8 and of 32: 89 / 133 / 147 /
+  // 203 us and 101 / 140 / 142 / 161; 16 is between them (99 / 138 / 142 / 170).
+  return qtype == NNTR_Q4_K ? (pairs <= 14 * n_experts ? 16 : 32) : (pairs <= 6 * n_experts ? 8 : 32);
 }
 
 int launch_act_tiles_grouped(int qtype, const float *x, unsigned rows, unsigned K, void *act, const int *perm, const int *idx,
@@ -959,23 +1080,13 @@ int launch_gemm_grouped(int qtype, unsigned N, unsigned K, const void *act, floa
   // sum over the experts of ceil(count / tile_rows), at most one tile per pair
   const unsigned tiles = pairs < pairs / tile_rows + n_experts ? pairs : pairs / tile_rows + n_experts;
   const unsigned z = w_table1 ? 2 : 1;
-  const bool ksplit = (uint64_t)tiles * z * ((N + 15) / 16) < 8u * (unsigned)sm_count();
-  // Q4_0's small tile: 55 registers, so shared memory sets the CTAs per SM, six with three units in flight and nine with two.
-  // From a pair per expert up the grid is two and more waves of six, and nine win: 4 of 32 experts of 2880 x 2880, 8 tokens
-  // 107 -> 100 us; 5 tokens (a wave and a half) 87.7 -> 89.3, so those keep three. Q4_K's tile is held to five by registers.
-  // The line holds for experts of that size (7 tokens, below it: three in flight 109.8 us, two 102.6) and of half the width (8 / 12 /
-  // 16 tokens 75.9 / 82.2 / 85.3 us with three, 70.9 / 74.9 / 77.5 with two). Elsewhere two in flight cost a little: 2 of 16 experts of
-  // 4096 x 4096, 12 tokens 117.3 -> 120.0; 4 of 64 experts of 1024 x 2880, 16 / 32 tokens 85.3 / 101 -> 88.8 / 103.
-  const bool shallow = pairs >= (unsigned)n_experts;
-#define NNTR_MMA_RUN(QT)                                                                                               \
-  (tile_rows == 8    ? run_tiles<QT, 1, true, true>(a, tiles, z, ksplit, shallow, st)                                           \
-   : tile_rows == 16 ? run_tiles<QT, 2, true, true>(a, tiles, z, ksplit, shallow, st)                                           \
-                     : run_tiles<QT, 4, true, true>(a, tiles, z, ksplit, shallow, st))
+  const bool ksplit = tile_rows <= 16 && (uint64_t)tiles * z * ((N + 15) / 16) <= 2u * (unsigned)sm_count();
   if (qtype == NNTR_Q4_K)
-    return NNTR_MMA_RUN(NNTR_Q4_K);
+    return tile_rows <= 16 ? run_tiles<NNTR_Q4_K, 2, true, true>(a, tiles, z, ksplit, st)
+                           : run_tiles<NNTR_Q4_K, 4, true, true>(a, tiles, z, ksplit, st);
   if (qtype == NNTR_Q4_0)
-    return NNTR_MMA_RUN(NNTR_Q4_0);
-#undef NNTR_MMA_RUN
+    return tile_rows <= 8 ? run_tiles<NNTR_Q4_0, 1, true, true>(a, tiles, z, ksplit, st)
+                          : run_tiles<NNTR_Q4_0, 4, true, true>(a, tiles, z, ksplit, st);
   return set_error(NNTR_CUDA_ERR_UNSUPPORTED, "gemm_grouped: expert weights must be Q4_K or Q4_0");
 }
 

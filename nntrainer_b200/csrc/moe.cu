@@ -533,7 +533,7 @@ moe_act_tiles_kernel(const float *__restrict__ gu, uint8_t *__restrict__ act, co
     for (int k = 0; k < 8; ++k)
       v[k] = 0.f;
   }
-  uint8_t *unit = act_unit<QT>(act, act_off[e] + (i >> 3), 8, nb, b);
+  uint8_t *unit = act_unit<QT>(act, act_off[e], (off[e + 1] - off[e] + 7) >> 3, i >> 3, 8, nb, b);
   const float4 v0 = make_float4(v[0], v[1], v[2], v[3]), v1 = make_float4(v[4], v[5], v[6], v[7]);
   if constexpr (QT == NNTR_Q4_K)
     put_q8K(unit, 8, i & 7, q8K_quantize_warp(v0, v1, lane, 0), lane);
@@ -832,7 +832,7 @@ static int moe_forward(const nntr_moe_desc *d, const nntr_moe_ep *epd, unsigned 
      * GEMVs. */
     int *off = reinterpret_cast<int *>(ws + s.off), *tile_off = reinterpret_cast<int *>(ws + s.tile_off),
         *act_off = reinterpret_cast<int *>(ws + s.act_off), *perm = reinterpret_cast<int *>(ws + s.perm);
-    const int tile_rows = grouped_tile_rows(P, E);
+    const int tile_rows = grouped_tile_rows(d->qtype, P, E);
     NNTR_CHECK_CUDA(launch_pdl(moe_permute_kernel, 1u, 1024u, st, idx, (int)P, (int)E, tile_rows, off, tile_off, act_off,
                                perm));
     count_launch();
