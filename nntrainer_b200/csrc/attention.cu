@@ -434,18 +434,24 @@ __global__ void attn_values_kernel(const float *__restrict__ probs, const uint16
  *            ascending row order by one warp (ordered_sum).
  *   values   a thread per dimension runs the row-ordered chain over value tiles that a producer warp keeps ahead of it
  *            (tiled TMA copies, started before the scores).
- * Clock stamps of one CTA per cluster, 64 / 8 heads of 64, at 512 / 2048 / 4096 / 6000 rows, in clocks: start and first copies 3000,
- * heads rotated 1000, score tiles 2500 / 7000 / 12500 / 20600, barrier behind them 2000 to 3300, maximum 1000, exponentials 600 /
- * 1500 / 2900 / 4400, ordered sum 5700 / 9300 / 12800 / 15700, division 400 to 2200, value chain 6800 / 23600 / 46000 / 67100. The
- * value chain is more than half of a long context at 11.2 clocks per row, where a dependent multiply-add alone takes four (heads
- * of 128: the same). 64 / 8 heads of 64 at 4096 rows 47 us (four launches before: 120), 32 / 8 heads of 128 at 512 rows 11 us (two
- * launches before: 15.7), at 128 rows of a window 7 us (10.8).
+ * Clock stamps of one CTA per cluster, 64 / 8 heads of 64, at 512 / 4096 rows, in clocks: start and first copies 900 / 1000, heads
+ * rotated 900, score tiles 1700 / 9100, barrier behind them 2200 / 2600, maximum 900, exponentials 600 / 2800, ordered sum 2600 /
+ * 11500, division 400 / 1450, value chain 5600 / 33000. The value chain is half of a long context at about 8 clocks per row (six
+ * inside a tile, the rest where it waits for one), where a dependent multiply-add alone takes four. 64 / 8 heads of 64 at 4096
+ * rows 37 us, 32 / 8 heads of 128 at 512 rows 11.3 us (with generic accesses to the tiles, and value tiles of 128 rows: 45 and
+ * 12.4), at 128 rows of a window 8.0 us with the copy of q (8.4). Measured and not kept: value tiles turned round by the idle warps
+ * for 16-byte loads (46 us), half of the ring waited for at a time (44), four blocks of the ordered sum at once (16900 clocks
+ * instead of 11500), two rows and two heads per thread in the scores (heads of 64: 1800 a tile instead of 1900; of 128: 2660
+ * instead of 2200).
  * Ring positions are counted, not divided: an integer division in a loop that one thread runs costs more than a tile's copy. */
 constexpr int AC_THREADS = 256;
 constexpr int AC_WARPS = AC_THREADS / 32;
-constexpr int AC_TILE = 128; // cache rows per tile of keys or values
+constexpr int AC_TILE = 128; // cache rows per tile of keys
+constexpr uint32_t AC_SMEM_ALONE = 200u * 1024u; // of which two CTAs do not fit an SM, nor one and the next kernel's
 constexpr int AC_KBUF_MAX = 4;
 constexpr int AC_VBUF_MAX = 6;
+/** cache rows per tile of values: a wait for a tile costs 350 clocks of the chain */
+template <int DIMS> constexpr int AC_VROWS = DIMS == 64 ? 256 : 128;
 constexpr unsigned AC_MAX_ROWS = 16384; // rows of one head kept as floats in shared memory
 constexpr uint32_t AC_POLLS = 1u << 22;
 __device__ int g_attn_status = 0; // raised when a bounded wait for a tile runs out
@@ -482,15 +488,15 @@ __device__ __forceinline__ void st_cluster(uint32_t addr, uint32_t rank, float v
 struct AcLayout {
   uint32_t ktile, vtile, e, q, total; // offsets; the tiles are 1024-byte aligned
 };
-__host__ __device__ inline AcLayout ac_layout(int gqa, int hd, int dims, int k_bufs, int v_bufs, unsigned cap_rows) {
+__host__ __device__ inline AcLayout ac_layout(int gqa, int hd, int dims, int k_bufs, int v_bufs, int v_box, unsigned cap_rows) {
   AcLayout L;
   uint32_t o = 0;
   L.ktile = o;
   o += (uint32_t)k_bufs * (uint32_t)((hd + 63) / 64) * AC_TILE * 128;
   L.vtile = o;
-  o += (uint32_t)v_bufs * AC_TILE * dims * 2;
+  o += (uint32_t)v_bufs * v_box * dims * 2; // one tile, or whole ones
   L.e = o; // scores, exponentials, probabilities of whole tiles; a spare block so that the sum may read ahead
-  o += (cap_rows + AC_TILE - 1) / AC_TILE * AC_TILE * 4 + 1024;
+  o += (cap_rows + 255) / 256 * 256 * 4 + 1024;
   L.q = o; // rotated query heads, then the new key head
   o += (uint32_t)(gqa + 1) * hd * 4;
   L.total = o + 1024;
@@ -510,21 +516,18 @@ __device__ __forceinline__ void dot_rows(const uint8_t *tile, int row, const flo
   for (int c = 0; c < (HD ? HD : hd) / 8; ++c) {
     const uint4 w = *reinterpret_cast<const uint4 *>(tile + (c >> 3) * (AC_TILE * 128) + row * 128 + (((c & 7) ^ (row & 7)) << 4));
     const uint32_t ws[4] = {w.x, w.y, w.z, w.w};
-    float kv[8];
+    float2 kv[4];
 #pragma unroll
-    for (int i = 0; i < 4; ++i) {
-      const float2 f = __half22float2(*reinterpret_cast<const __half2 *>(&ws[i]));
-      kv[2 * i] = f.x;
-      kv[2 * i + 1] = f.y;
-    }
+    for (int i = 0; i < 4; ++i)
+      kv[i] = __half22float2(*reinterpret_cast<const __half2 *>(&ws[i]));
 #pragma unroll
     for (int h = 0; h < H; ++h) {
       const float4 a = *reinterpret_cast<const float4 *>(qs + h * hd + 8 * c),
                    b = *reinterpret_cast<const float4 *>(qs + h * hd + 8 * c + 4);
-      const float qv[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
-#pragma unroll
-      for (int l = 0; l < 8; ++l)
-        acc[h][l] = __fmaf_rn(qv[l], kv[l], acc[h][l]);
+      fma2(acc[h][0], acc[h][1], a.x, a.y, kv[0].x, kv[0].y);
+      fma2(acc[h][2], acc[h][3], a.z, a.w, kv[1].x, kv[1].y);
+      fma2(acc[h][4], acc[h][5], b.x, b.y, kv[2].x, kv[2].y);
+      fma2(acc[h][6], acc[h][7], b.z, b.w, kv[3].x, kv[3].y);
     }
   }
 #pragma unroll
@@ -647,12 +650,12 @@ attn_cluster_kernel(const __grid_constant__ CUtensorMap kmap, const __grid_const
   const int gqa = a.hq / a.hkv / a.groups, hd = HD ? HD : a.hd, per_head = (hd + DIMS - 1) / DIMS, items = gqa * per_head;
   const uint32_t rank = (uint32_t)cluster_rank(), csize = (uint32_t)cluster_size();
   const int cluster = (int)(blockIdx.x / csize), n = cluster / a.groups, h0 = cluster * gqa; // kv head, first query head
-  uint8_t *base = reinterpret_cast<uint8_t *>((reinterpret_cast<uintptr_t>(ac_raw) + 1023) & ~(uintptr_t)1023);
-  const AcLayout L = ac_layout(gqa, hd, DIMS, a.k_bufs, a.v_bufs, a.cap_rows);
+  uint8_t *base = ac_raw + (-smem_u32(ac_raw) & 1023u); // an offset: rounding the pointer itself up makes every access a generic one
+  const AcLayout L = ac_layout(gqa, hd, DIMS, a.k_bufs, a.v_bufs, a.v_box, a.cap_rows);
   uint8_t *ktile = base + L.ktile, *vtile = base + L.vtile;
   float *e = reinterpret_cast<float *>(base + L.e), *qs = reinterpret_cast<float *>(base + L.q), *kown = qs + gqa * hd;
   const int k_halves = (hd + 63) / 64;
-  const uint32_t kbytes = (uint32_t)k_halves * AC_TILE * 128, vbytes = AC_TILE * DIMS * 2; // of a buffer
+  const uint32_t kbytes = (uint32_t)k_halves * AC_TILE * 128, vbytes = (uint32_t)a.v_box * DIMS * 2; // of a buffer
   const uint32_t ksm = smem_u32(ktile), vsm = smem_u32(vtile), esm = smem_u32(e);
   const uint32_t kbar0 = smem_u32(kbar), vfull0 = smem_u32(vfull), vempty0 = smem_u32(vempty);
   if (tid == 0) {
@@ -681,7 +684,8 @@ attn_cluster_kernel(const __grid_constant__ CUtensorMap kmap, const __grid_const
   const int item_head = (int)rank / per_head, item_d0 = ((int)rank % per_head) * DIMS;
   const bool has_item = (int)rank < items, has_own = a.rope && r_lo < cnt && r_hi == cnt;
   const bool append = has_own && cluster % a.groups == 0; // one cluster per kv head appends the token's rows
-  const unsigned k_tiles = (r_hi - r_lo + AC_TILE - 1) / AC_TILE, v_tiles = (cached + AC_TILE - 1) / AC_TILE;
+  constexpr int VROWS = AC_VROWS<DIMS>;
+  const unsigned k_tiles = (r_hi - r_lo + AC_TILE - 1) / AC_TILE, v_tiles = (cached + VROWS - 1) / VROWS;
   auto issue_k = [&](unsigned t, int buf) {
     const uint32_t bar = kbar0 + 8 * buf;
     mbar_expect_tx(bar, (uint32_t)(k_halves * a.k_box) * 128);
@@ -691,7 +695,7 @@ attn_cluster_kernel(const __grid_constant__ CUtensorMap kmap, const __grid_const
   auto issue_v = [&](unsigned t, int buf) {
     const uint32_t bar = vfull0 + 8 * buf;
     mbar_expect_tx(bar, (uint32_t)a.v_box * DIMS * 2);
-    tma_tile(vsm + buf * vbytes, &vmap, n * hd + item_d0, (int)(first + t * AC_TILE), bar);
+    tma_tile(vsm + buf * vbytes, &vmap, n * hd + item_d0, (int)(first + t * VROWS), bar);
   };
   if (tid == 0)
     for (unsigned t = 0; t < (unsigned)a.k_bufs && t < k_tiles; ++t)
@@ -866,8 +870,8 @@ attn_cluster_kernel(const __grid_constant__ CUtensorMap kmap, const __grid_const
       load(vt, e, pr[0], vb[0]); // reads past the last row stay in shared memory and are not used
     }
     for (unsigned t = 0; t < v_tiles; ++t) {
-      const float *pt = e + t * AC_TILE;
-      const unsigned rows = min(cached - t * AC_TILE, (unsigned)AC_TILE);
+      const float *pt = e + t * VROWS;
+      const unsigned rows = min(cached - t * VROWS, (unsigned)VROWS);
       int nbuf = buf + 1;
       uint32_t npar = par;
       if (nbuf == a.v_bufs) {
@@ -875,19 +879,24 @@ attn_cluster_kernel(const __grid_constant__ CUtensorMap kmap, const __grid_const
         npar ^= 1;
       }
       const uint16_t *nvt = reinterpret_cast<const uint16_t *>(vtile + nbuf * vbytes) + tid;
-      if (rows == AC_TILE) {
-#pragma unroll
-        for (int j = 0; j < AC_TILE; j += 16) {
-          const int k = (j / 16) & 1;
-          if (j + 16 < AC_TILE) {
-            load(vt + (j + 16) * DIMS, pt + j + 16, pr[k ^ 1], vb[k ^ 1]);
-          } else if (t + 1 < v_tiles) {
-            ok = mbar_wait_bounded(vfull0 + 8 * nbuf, npar, abort_flag, &g_attn_status, AC_POLLS, 1024) && ok;
-            load(nvt, pt + AC_TILE, pr[k ^ 1], vb[k ^ 1]);
-          }
+      // asked now, needed sixteen rows before this tile's end: the answer takes about a hundred clocks
+      const bool next_here = t + 1 < v_tiles && mbar_try_wait(vfull0 + 8 * nbuf, npar);
+      if (rows == VROWS) {
+        // Unrolled further, a tile of 256 rows is 14 KB of code: 1.6 us less for 4096 rows (36.8 and 35.2), but 4 % more for a decode step
+        // of a context of 512 (16 tokens over four layers 3386 us, 3252 like this), where every launch fetches its code anew. Not at all: 39.5.
+#pragma unroll(DIMS == 64 ? 2 : 4)
+        for (int j = 0; j < VROWS; j += 32) {
+          load(vt + (j + 16) * DIMS, pt + j + 16, pr[1], vb[1]);
 #pragma unroll
           for (int u = 0; u < 16; ++u)
-            acc = __fmaf_rn(pr[k][u], half_bits_to_float(vb[k][u]), acc);
+            acc = __fmaf_rn(pr[0][u], half_bits_to_float(vb[0][u]), acc);
+          const bool end = j + 32 == VROWS;
+          if (end && t + 1 < v_tiles && !next_here)
+            ok = mbar_wait_bounded(vfull0 + 8 * nbuf, npar, abort_flag, &g_attn_status, AC_POLLS, 1024) && ok;
+          load(end ? nvt : vt + (j + 32) * DIMS, pt + j + 32, pr[0], vb[0]); // behind the last tile: read and not used
+#pragma unroll
+          for (int u = 0; u < 16; ++u)
+            acc = __fmaf_rn(pr[1][u], half_bits_to_float(vb[1][u]), acc);
         }
       } else { // the last tile
         unsigned j = 0;
@@ -1018,16 +1027,17 @@ static int launch_attn_cluster(AttnStep a, unsigned bound, unsigned rows, unsign
     csize /= 2;
   // buffers for what the launch can need, no more: the next kernel's CTAs want room beside this one's
   a.cap_rows = rows;
-  const unsigned k_tiles = ((rows + csize - 1) / csize + AC_TILE - 1) / AC_TILE, v_tiles = (rows + AC_TILE - 1) / AC_TILE;
+  const unsigned k_tiles = ((rows + csize - 1) / csize + AC_TILE - 1) / AC_TILE, v_rows = dims == 64 ? 256u : 128u, v_tiles = (rows + v_rows - 1) / v_rows;
   const unsigned k_max = hd <= 64 ? 4u : 2u;
   a.k_bufs = (int)(k_tiles < k_max ? k_tiles : k_max);
-  a.v_bufs = (int)(v_tiles < (unsigned)AC_VBUF_MAX ? v_tiles : (unsigned)AC_VBUF_MAX);
+  const unsigned v_max = dims == 64 ? 3u : (unsigned)AC_VBUF_MAX;
+  a.v_bufs = (int)(v_tiles < v_max ? v_tiles : v_max);
   const auto box = [](unsigned n) { return n <= 32 ? 32 : n <= 64 ? 64 : AC_TILE; };
   a.k_box = box((rows + csize - 1) / csize);
-  a.v_box = box(rows);
-  AcLayout L = ac_layout(gqa, hd, dims, a.k_bufs, a.v_bufs, rows);
+  a.v_box = (int)((rows < v_rows ? rows : v_rows) + 31) / 32 * 32;
+  AcLayout L = ac_layout(gqa, hd, dims, a.k_bufs, a.v_bufs, a.v_box, rows);
   while (L.total > 200u * 1024u && a.v_bufs > 2)
-    L = ac_layout(gqa, hd, dims, a.k_bufs, --a.v_bufs, rows);
+    L = ac_layout(gqa, hd, dims, a.k_bufs, --a.v_bufs, a.v_box, rows);
   const auto kernel = hd == 128  ? (dims == 64 ? attn_cluster_kernel<128, 64> : attn_cluster_kernel<128, 128>)
                       : hd == 64 ? attn_cluster_kernel<64, 64>
                                  : (dims == 64 ? attn_cluster_kernel<0, 64> : attn_cluster_kernel<0, 128>);
@@ -1057,7 +1067,10 @@ static int launch_attn_cluster(AttnStep a, unsigned bound, unsigned rows, unsign
   cfg.stream = st;
   cfg.gridDim = dim3(clusters * csize, a.tokens);
   cfg.blockDim = dim3(AC_THREADS);
-  cfg.dynamicSmemBytes = L.total;
+  // A decode step's CTAs keep their SMs to themselves: a second one of them, or the next launch's, let in early, takes issue slots and
+  // the way to memory from a kernel that is bound by latency. 16 tokens over four layers at a context of 100 / 250 / 512: 3144 / 3156
+  // / 3276 us where only a second one is kept out (116 KB), 3052 / 3069 / 3243 with 200 KB.
+  cfg.dynamicSmemBytes = a.tokens == 1 && L.total < AC_SMEM_ALONE ? AC_SMEM_ALONE : L.total;
   const cudaError_t e = cudaLaunchKernelEx(&cfg, kernel, kmap, vmap, a);
   count_launch();
   *taken = true;

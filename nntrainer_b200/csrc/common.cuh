@@ -93,6 +93,30 @@ __device__ __forceinline__ void scale_min_k4(int j, const uint8_t *q, int &sc, i
   }
 }
 
+/** two fp32 operations in one instruction, each rounded as by itself */
+__device__ __forceinline__ void fma2(float &d0, float &d1, float a0, float a1, float b0, float b1) {
+  asm("{.reg .b64 a, b, d;\n\tmov.b64 a, {%2, %3};\n\tmov.b64 b, {%4, %5};\n\tmov.b64 d, {%0, %1};\n\t"
+      "fma.rn.f32x2 d, a, b, d;\n\tmov.b64 {%0, %1}, d;}"
+      : "+f"(d0), "+f"(d1)
+      : "f"(a0), "f"(a1), "f"(b0), "f"(b1));
+}
+__device__ __forceinline__ float2 add2(float a0, float a1, float b0, float b1) {
+  float2 r;
+  asm("{.reg .b64 a, b, d;\n\tmov.b64 a, {%2, %3};\n\tmov.b64 b, {%4, %5};\n\t"
+      "add.rn.f32x2 d, a, b;\n\tmov.b64 {%0, %1}, d;}"
+      : "=f"(r.x), "=f"(r.y)
+      : "f"(a0), "f"(a1), "f"(b0), "f"(b1));
+  return r;
+}
+__device__ __forceinline__ float2 mul2(float a0, float a1, float b0, float b1) {
+  float2 r;
+  asm("{.reg .b64 a, b, d;\n\tmov.b64 a, {%2, %3};\n\tmov.b64 b, {%4, %5};\n\t"
+      "mul.rn.f32x2 d, a, b;\n\tmov.b64 {%0, %1}, d;}"
+      : "=f"(r.x), "=f"(r.y)
+      : "f"(a0), "f"(a1), "f"(b0), "f"(b1));
+  return r;
+}
+
 /** Programmatic dependent launch: wait until the kernels this one depends on
  *  have finished and their writes are visible (no-op without the attribute). */
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }

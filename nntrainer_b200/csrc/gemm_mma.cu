@@ -83,21 +83,6 @@ __device__ __forceinline__ void mma_f16_k16(float (&d)[4], uint32_t a0, uint32_t
 
 __device__ __forceinline__ uint32_t h2_bits(__half2 h) { return *reinterpret_cast<const uint32_t *>(&h); }
 __device__ __forceinline__ __half2 bits_h2(uint32_t u) { return *reinterpret_cast<const __half2 *>(&u); }
-/** two fp32 operations in one instruction, each rounded as by itself */
-__device__ __forceinline__ void fma2(float &d0, float &d1, float a0, float a1, float b0, float b1) {
-  asm("{.reg .b64 a, b, d;\n\tmov.b64 a, {%2, %3};\n\tmov.b64 b, {%4, %5};\n\tmov.b64 d, {%0, %1};\n\t"
-      "fma.rn.f32x2 d, a, b, d;\n\tmov.b64 {%0, %1}, d;}"
-      : "+f"(d0), "+f"(d1)
-      : "f"(a0), "f"(a1), "f"(b0), "f"(b1));
-}
-__device__ __forceinline__ float2 mul2(float a0, float a1, float b0, float b1) {
-  float2 r;
-  asm("{.reg .b64 a, b, d;\n\tmov.b64 a, {%2, %3};\n\tmov.b64 b, {%4, %5};\n\t"
-      "mul.rn.f32x2 d, a, b;\n\tmov.b64 {%0, %1}, d;}"
-      : "=f"(r.x), "=f"(r.y)
-      : "f"(a0), "f"(a1), "f"(b0), "f"(b1));
-  return r;
-}
 /** (v, 32 v) of byte K of four 6-bit values as half2; 0x64vv is 1024 + v */
 template <int K> __device__ __forceinline__ uint32_t min_halves(uint32_t v) {
   return h2_bits(__hfma2(bits_h2(__byte_perm(v, 0x64646464u, 0x4040 | (K * 0x101))), __floats2half2_rn(1.f, 32.f),
