@@ -23,7 +23,7 @@
  *
  * A warp owns 16 weight rows and up to 16 activation rows (32 chain accumulators per 8 rows) over all of K and shares
  * nothing with other warps. Bound by the unpack (about 390 logic and 270 multiply instructions per 16 x 256 weights, at
- * half rate both): 8 x 151936 x 2560 131 us (CUDA-core kernel before: 697; the weights' bytes alone take 49), 31 rows 368 us
+ * half rate both): 8 x 151936 x 2560 129 us (CUDA-core kernel before: 697; the weights' bytes alone take 49), 31 rows 339 us
  * (2360). Bringing the rows in by 4- and 8-byte asynchronous copies or through registers measured the same or slower.
  */
 #include "common.cuh"
@@ -73,6 +73,9 @@ template <int NT>
 __global__ void __launch_bounds__(Q6M_WARPS * 32, 3)
 gemm_q6_K_mma_kernel(const uint8_t *__restrict__ act, const uint8_t *__restrict__ W, float *__restrict__ C, int ldc, int M,
                      int N, int nb) {
+  // High nibbles used where they lie, with their own factors: the same number of operations, 187 against 193 us for 16 x 151936 x
+  // 2560 and 338 against 346 for 31 rows; with one tile of rows 130 against 128 and 32.4 against 30.3 for 5 x 4096 x 4096.
+  constexpr bool IN_PLACE = NT == 2;
   __shared__ alignas(16) uint32_t stage[Q6M_WARPS][Q6M_STAGES][Q6M_STAGE_WORDS];
   __shared__ alignas(8) unsigned long long bars[Q6M_WARPS][Q6M_STAGES];
   __shared__ int aborted[Q6M_WARPS]; // one per warp: the warps of a CTA do not meet
@@ -175,10 +178,11 @@ gemm_q6_K_mma_kernel(const uint8_t *__restrict__ act, const uint8_t *__restrict_
         for (int k = 0; k < 2; ++k) {
           // the byte in both halves; its low nibble over 1024, its high nibble + 8 (sign bit flipped) over 64
           const uint32_t sc = __byte_perm(scales[r][k], 0, e ? 0x4141 : 0x4040);
-          s_lo[r][k] = __hfma2(u2h(lop3<LUT_AND_OR>(sc, 0x000f000fu, 0x64006400u)), __float2half2_rn(0.25f), __float2half2_rn(-256.f));
-          s_hi[r][k] = __hfma2(u2h(lop3<LUT_AND_XOR>(sc, 0x00f000f0u, 0x54805480u)), __float2half2_rn(4.f), __float2half2_rn(-288.f));
-          o_lo[r][k] = __hmul2(s_lo[r][k], __float2half2_rn(-1056.f));
-          o_hi[r][k] = __hmul2(s_hi[r][k], __float2half2_rn(-1056.f));
+          const float over = IN_PLACE && k ? 0.0625f : 1.f, offset = IN_PLACE && k ? -1536.f : -1056.f; // in place: values times 16
+          s_lo[r][k] = __hfma2(u2h(lop3<LUT_AND_OR>(sc, 0x000f000fu, 0x64006400u)), __float2half2_rn(0.25f * over), __float2half2_rn(-256.f * over));
+          s_hi[r][k] = __hfma2(u2h(lop3<LUT_AND_XOR>(sc, 0x00f000f0u, 0x54805480u)), __float2half2_rn(4.f * over), __float2half2_rn(-288.f * over));
+          o_lo[r][k] = __hmul2(s_lo[r][k], __float2half2_rn(offset));
+          o_hi[r][k] = __hmul2(s_hi[r][k], __float2half2_rn(offset));
         }
 #pragma unroll
       for (int l4 = 0; l4 < 4; ++l4) {
@@ -190,18 +194,29 @@ gemm_q6_K_mma_kernel(const uint8_t *__restrict__ act, const uint8_t *__restrict_
           const uint32_t lw = __funnelshift_r(ql[r], ql1, sh[r]), hw = __funnelshift_r(qh[r], qh1, sh[r]);
           ql[r] = ql1;
           qh[r] = qh1;
+          __half2 q0[2], q1[2]; // of the two quarters: bytes 0, 2 and 1, 3 as halves 1024 + q
+          if (IN_PLACE) {      // (high nibbles: 1024 + 16 q)
+            const uint32_t l8 = lw >> 8, u = hw << (4 - 2 * run), u8 = hw >> (4 + 2 * run);
+            q0[0] = u2h(lop3<LUT_AND_OR>(lw, 0x000f000fu, lop3<LUT_AND_OR>(u, 0x00300030u, 0x64006400u)));
+            q0[1] = u2h(lop3<LUT_AND_OR>(lw, 0x00f000f0u, lop3<LUT_AND_OR>(u, 0x03000300u, 0x64006400u)));
+            q1[0] = u2h(lop3<LUT_AND_OR>(l8, 0x000f000fu, lop3<LUT_AND_OR>(u8, 0x00300030u, 0x64006400u)));
+            q1[1] = u2h(lop3<LUT_AND_OR>(l8, 0x00f000f0u, lop3<LUT_AND_OR>(u8, 0x03000300u, 0x64006400u)));
+          } else {
+#pragma unroll
+            for (int k = 0; k < 2; ++k) {
+              // low nibbles of one word, above them the bits of the other (bits 6 and 7 of the bytes are masked off below)
+              const uint32_t n = k ? lw >> 4 : lw, up = k ? hw >> (2 * run) : hw << (4 - 2 * run);
+              const uint32_t q = lop3<LUT_SELECT>(n, up, 0x0f0f0f0fu);
+              q0[k] = u2h(lop3<LUT_AND_OR>(q, 0x003f003fu, 0x64006400u));
+              q1[k] = u2h(lop3<LUT_AND_OR>(q >> 8, 0x003f003fu, 0x64006400u));
+            }
+          }
 #pragma unroll
           for (int k = 0; k < 2; ++k) {
-            // low nibbles of one word, above them the bits of the other (bits 6 and 7 of the bytes are masked off below);
-            // bytes 0, 2 and 1, 3 as halves 1024 + q
-            const uint32_t n = k ? lw >> 4 : lw, up = k ? hw >> (2 * run) : hw << (4 - 2 * run);
-            const uint32_t q = lop3<LUT_SELECT>(n, up, 0x0f0f0f0fu);
-            const __half2 q0 = u2h(lop3<LUT_AND_OR>(q, 0x003f003fu, 0x64006400u)),
-                          q1 = u2h(lop3<LUT_AND_OR>(q >> 8, 0x003f003fu, 0x64006400u));
-            al[k][r] = h2u(__hfma2(q0, s_lo[r][k], o_lo[r][k]));
-            al[k][r + 2] = h2u(__hfma2(q1, s_lo[r][k], o_lo[r][k]));
-            ah[k][r] = h2u(__hfma2(q0, s_hi[r][k], o_hi[r][k]));
-            ah[k][r + 2] = h2u(__hfma2(q1, s_hi[r][k], o_hi[r][k]));
+            al[k][r] = h2u(__hfma2(q0[k], s_lo[r][k], o_lo[r][k]));
+            al[k][r + 2] = h2u(__hfma2(q1[k], s_lo[r][k], o_lo[r][k]));
+            ah[k][r] = h2u(__hfma2(q0[k], s_hi[r][k], o_hi[r][k]));
+            ah[k][r + 2] = h2u(__hfma2(q1[k], s_hi[r][k], o_hi[r][k]));
           }
         }
 #pragma unroll
@@ -216,8 +231,10 @@ gemm_q6_K_mma_kernel(const uint8_t *__restrict__ act, const uint8_t *__restrict_
             mma_f16(p, al[0], v.x, v.y);
             mma_f16(p2, al[1], v.z, v.w);
 #pragma unroll
-            for (int c = 0; c < 4; ++c)
-              acc[i][l][c] = __fmaf_rn(d[i][c], p[c] + p2[c], acc[i][l][c]);
+            for (int c = 0; c < 4; c += 2) {
+              const float2 sum = add2(p[c], p[c + 1], p2[c], p2[c + 1]);
+              fma2(acc[i][l][c], acc[i][l][c + 1], d[i][c], d[i][c + 1], sum.x, sum.y);
+            }
           }
       }
     }
