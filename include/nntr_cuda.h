@@ -71,7 +71,8 @@ uint64_t nntr_cuda_launch_count(void);
 /** Synchronizes the device, then reports whether any kernel of this library
  *  gave up on one of its bounded waits (every device-side wait has an iteration
  *  limit; on expiry the kernel raises a status word and returns instead of
- *  hanging): NNTR_CUDA_OK, or NNTR_CUDA_ERR_TIMEOUT. */
+ *  hanging): NNTR_CUDA_OK, or NNTR_CUDA_ERR_TIMEOUT. NNTR_CUDA_ERR_INVALID: a
+ *  kernel found an expert's weights that are not 16-byte aligned in a table. */
 int nntr_cuda_device_status(void);
 /** Zeroes every status word of the bound device, so that a process that has seen NNTR_CUDA_ERR_TIMEOUT (or a
  *  rejected embedding index) can go on: nntr_cuda_device_status() reports a condition once per occurrence only if

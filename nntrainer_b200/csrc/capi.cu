@@ -545,7 +545,8 @@ int nntr_cuda_device_status(void) {
   if (!v && (rc = read_q6m_status(&v)))
     return rc;
   if (v)
-    return set_error(v, "a device kernel gave up on a bounded wait (status %d)", v);
+    return set_error(v, v == NNTR_CUDA_ERR_INVALID ? "a device kernel found expert weights that are not 16-byte aligned (status %d)"
+                                                   : "a device kernel gave up on a bounded wait (status %d)", v);
   if ((rc = read_embed_status(&v, false)))
     return rc;
   if (v)

@@ -640,13 +640,19 @@ template <int NT> struct KsShared {
   int abort_flag;
 };
 
-/** barrier `id` of two warps: the one in front arrives, the other one waits for it */
+/** barrier `id` of two warps: the one in front arrives, the other one waits for it. Two tiles of rows take all sixteen barriers,
+ *  number 0 among them, so nothing between the first hand-over and the last may be a barrier of the whole CTA. */
 __device__ __forceinline__ void pair_arrive(int id) { asm volatile("barrier.cta.arrive %0, 64;" ::"r"(id) : "memory"); }
 __device__ __forceinline__ void pair_sync(int id) { asm volatile("barrier.cta.sync %0, 64;" ::"r"(id) : "memory"); }
 
-template <int QT, int NT, bool GROUPED, bool TH8>
+/** COPIES: the weights start at a multiple of 16 and bulk copies bring them in; otherwise they start at a multiple of 8 and every
+ *  warp brings its own units in by 8-byte copies. Instances of their own: as branches of one they cost Q4_K with two tiles 2 to 3 %
+ *  (16 x 4096 x 4096 9.8 -> 10.1 us). Q4_K at a multiple of 8, 8 x 2560 x 9728 13.0 us, 256 x 4096 x 4096 101 (loads into registers one
+ *  round ahead: 18.7 and 135; every warp's loads and then its products: 19.8 and 141). */
+template <int QT, int NT, bool GROUPED, bool TH8, bool COPIES>
 __global__ void __launch_bounds__(KS_WARPS * 32, 2) gemm_mma_ksplit_kernel(const MmaArgs a) {
   extern __shared__ __align__(16) uint8_t ks_smem[];
+  static_assert(KS_WARPS * NT <= 16, "a hand-over barrier per warp and tile");
   KsShared<NT> &sh = *reinterpret_cast<KsShared<NT> *>(ks_smem);
   volatile int *abort_flag = &sh.abort_flag;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, g = lane >> 2, t = lane & 3;
@@ -667,8 +673,12 @@ __global__ void __launch_bounds__(KS_WARPS * 32, 2) gemm_mma_ksplit_kernel(const
     pdl_wait();
   if (!find_tile<NT>(tl, a, blockIdx.x, GROUPED))
     return;
+  if (GROUPED && (reinterpret_cast<uintptr_t>(tl.W) & 15)) { // from a table in device memory: not seen by the launcher
+    if (tid == 0)
+      atomicExch(&g_mma_status, NNTR_CUDA_ERR_INVALID);
+    return;
+  }
   const uint8_t *w = static_cast<const uint8_t *>(tl.W) + (size_t)(2 * rt) * row;
-  const bool copies = !(reinterpret_cast<uintptr_t>(w) & 15);
   auto round_bytes = [&](int rd) { return (int)min((size_t)upr * sizeof(BlockQ4Kx8), row - (size_t)rd * upr * sizeof(BlockQ4Kx8)); };
   auto fetch = [&](int rd, int slot) { // thread 0: a row group's units of a round are one piece of memory
     const uint32_t bar = smem_u32(sh.full + slot), dst = smem_u32(sh.w[slot]);
@@ -677,7 +687,24 @@ __global__ void __launch_bounds__(KS_WARPS * 32, 2) gemm_mma_ksplit_kernel(const
     for (int h = 0; h < 1 + second; ++h)
       bulk_g2s(dst + h * (KS_W / 2), w + h * row + (size_t)rd * upr * sizeof(BlockQ4Kx8), bytes, bar);
   };
-  if (tid == 0 && copies) // the weights do not depend on the quantizer's kernel: fetched while it runs
+  auto fetch_own = [&](int rd, int slot) { // all lanes: this warp's unit of a round, one group of copies
+    const int b = rd * upr + warp;
+    if (warp < upr && b < nb) {
+      const int bytes = QT == NNTR_Q4_K ? (int)sizeof(BlockQ4Kx8) : min(8, a.nblk - 8 * b) * (int)sizeof(BlockQ40x8);
+      const uint32_t dst = smem_u32(sh.w[slot]) + warp * (int)sizeof(BlockQ4Kx8);
+      for (int h = 0; h < 1 + second; ++h)
+        for (int i = lane * 8; i < bytes; i += 32 * 8)
+          asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(dst + h * (KS_W / 2) + i),
+                       "l"(w + h * row + (size_t)b * sizeof(BlockQ4Kx8) + i)
+                       : "memory");
+    }
+    asm volatile("cp.async.commit_group;" ::: "memory");
+  };
+  // the weights do not depend on the quantizer's kernel: fetched while it runs
+  if (!COPIES)
+    for (int rd = 0; rd < KS_RING - 1; ++rd)
+      fetch_own(rd, rd);
+  else if (tid == 0)
     for (int rd = 0; rd < KS_RING && rd < per; ++rd)
       fetch(rd, rd);
   if (!GROUPED)
@@ -697,17 +724,14 @@ __global__ void __launch_bounds__(KS_WARPS * 32, 2) gemm_mma_ksplit_kernel(const
   for (int rd = 0; rd < per; ++rd) {
     const int b = rd * upr + warp;
     uint8_t *wr = sh.w[slot];
-    if (!copies) { // weights that start at a multiple of 8: plain loads, round by round
-      const int bytes = round_bytes(rd);
-      __syncthreads();
-      for (int h = 0; h < 1 + second; ++h)
-        for (int i = tid * 8; i < bytes; i += KS_WARPS * 32 * 8)
-          *reinterpret_cast<uint2 *>(wr + h * (KS_W / 2) + i) = ldg_stream_u2(w + h * row + (size_t)rd * upr * sizeof(BlockQ4Kx8) + i);
-      __syncthreads();
-    }
     if (warp < upr && b < nb) {
-      if (copies && !__all_sync(FULL, mbar_try_wait(smem_u32(sh.full + slot), par)))
+      if (!COPIES) {
+        __syncwarp(); // all lanes are done with the unit in front
+        fetch_own(rd + KS_RING - 1, slot ? slot - 1 : KS_RING - 1);
+        asm volatile("cp.async.wait_group %0;" ::"n"(KS_RING - 1) : "memory");
+      } else if (!__all_sync(FULL, mbar_try_wait(smem_u32(sh.full + slot), par))) {
         ok = mbar_wait_bounded(smem_u32(sh.full + slot), par, abort_flag, &g_mma_status, 1u << 22, 2048) && ok;
+      }
       __syncwarp();
       const uint8_t *u0 = wr + warp * sizeof(BlockQ4Kx8), *u1 = u0 + (second ? KS_W / 2 : 0);
       Q4KScales sc;
@@ -857,7 +881,7 @@ __global__ void __launch_bounds__(KS_WARPS * 32, 2) gemm_mma_ksplit_kernel(const
         }
       }
       // The chains of this round's first unit have come through every unit of the round before, so nobody reads its weights any more.
-      if (warp == 0 && rd > 0 && rd - 1 + KS_RING < per && copies) {
+      if (COPIES && warp == 0 && rd > 0 && rd - 1 + KS_RING < per) {
         __syncwarp();
         if (lane == 0 && ok) {
           loads_before_refill();
@@ -931,7 +955,7 @@ cudaError_t launch(void (*kernel)(KArgs...), dim3 grid, unsigned block, size_t s
 }
 
 template <int QT, int NT, bool GROUPED, bool TH8>
-int run_tiles(const MmaArgs &a, unsigned tiles, unsigned z, bool ksplit, cudaStream_t st) {
+int run_tiles(const MmaArgs &a, unsigned tiles, unsigned z, bool ksplit, bool misaligned, cudaStream_t st) {
   const unsigned row_tiles = (unsigned)((a.N + 15) / 16);
   constexpr int stages = rows_stages<QT, NT, GROUPED>(), ctas = rows_ctas<QT, NT, GROUPED>();
   constexpr size_t smem = sizeof(RowsShared<NT, stages>);
@@ -939,9 +963,12 @@ int run_tiles(const MmaArgs &a, unsigned tiles, unsigned z, bool ksplit, cudaStr
   int dev = 0;
   NNTR_CHECK_CUDA(cudaGetDevice(&dev));
   if (dev < 64 && !attr_set[dev]) {
-    if constexpr (NT <= 2)
-      NNTR_CHECK_CUDA(cudaFuncSetAttribute(gemm_mma_ksplit_kernel<QT, NT, GROUPED, TH8>,
+    if constexpr (NT <= 2) {
+      NNTR_CHECK_CUDA(cudaFuncSetAttribute(gemm_mma_ksplit_kernel<QT, NT, GROUPED, TH8, true>,
                                            cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(KsShared<NT>)));
+      NNTR_CHECK_CUDA(cudaFuncSetAttribute(gemm_mma_ksplit_kernel<QT, NT, GROUPED, TH8, GROUPED>,
+                                           cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(KsShared<NT>)));
+    }
     NNTR_CHECK_CUDA(cudaFuncSetAttribute(gemm_mma_rows_kernel<QT, NT, GROUPED, TH8, stages>,
                                          cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     attr_set[dev] = true;
@@ -949,7 +976,8 @@ int run_tiles(const MmaArgs &a, unsigned tiles, unsigned z, bool ksplit, cudaStr
   cudaError_t e = cudaSuccess;
   if (NT <= 2 && ksplit) {
     if constexpr (NT <= 2)
-      e = launch(gemm_mma_ksplit_kernel<QT, NT, GROUPED, TH8>, dim3(tiles, row_tiles, z), KS_WARPS * 32, sizeof(KsShared<NT>), st, a);
+      e = launch(misaligned ? gemm_mma_ksplit_kernel<QT, NT, GROUPED, TH8, GROUPED> : gemm_mma_ksplit_kernel<QT, NT, GROUPED, TH8, true>,
+                 dim3(tiles, row_tiles, z), KS_WARPS * 32, sizeof(KsShared<NT>), st, a);
   } else {
     const uint64_t items = (uint64_t)tiles * ((row_tiles + ROWS_WARPS - 1) / ROWS_WARPS) * z;
     const uint64_t slots = (uint64_t)ctas * (unsigned)sm_count();
@@ -989,7 +1017,7 @@ int launch_gemm_mma(int qtype, unsigned M, unsigned M4, unsigned N, unsigned K, 
                                  nullptr, 1);
   count_launch();
   NNTR_CHECK_CUDA(cudaGetLastError());
-  // Weights that are not 16-byte aligned cannot be fetched by bulk copies: the shared tile's plain loads take them all.
+  // Weights that are not 16-byte aligned cannot be fetched by bulk copies: the shared tile has 8-byte copies for them.
   const bool misaligned = reinterpret_cast<uintptr_t>(B) & 15;
   const unsigned row_tiles = (N + 15) / 16, row_blocks = (N + 63) / 64, sms = (unsigned)sm_count();
   const auto tiles_of = [&](unsigned nt) { return (M + 8 * nt - 1) / (8 * nt); };
@@ -1009,11 +1037,11 @@ int launch_gemm_mma(int qtype, unsigned M, unsigned M4, unsigned N, unsigned K, 
     nt = M <= 8 ? 1 : M > 16 && 3 * tiles_of(4) * row_blocks >= 2 * sms ? 4 : 2;
   const unsigned tiles = tiles_of(a.th < 8 ? 1 : nt);
   if (a.th < 8)
-    return run_tiles<NNTR_Q4_K, 1, false, false>(a, tiles, 1, ksplit, st);
+    return run_tiles<NNTR_Q4_K, 1, false, false>(a, tiles, 1, ksplit, misaligned, st);
 #define NNTR_MMA_RUN(QT)                                                                                               \
-  (nt == 1   ? run_tiles<QT, 1, false, true>(a, tiles, 1, ksplit, st)                                                  \
-   : nt == 2 ? run_tiles<QT, 2, false, true>(a, tiles, 1, ksplit, st)                                                  \
-             : run_tiles<QT, 4, false, true>(a, tiles, 1, ksplit, st))
+  (nt == 1   ? run_tiles<QT, 1, false, true>(a, tiles, 1, ksplit, misaligned, st)                                                  \
+   : nt == 2 ? run_tiles<QT, 2, false, true>(a, tiles, 1, ksplit, misaligned, st)                                                  \
+             : run_tiles<QT, 4, false, true>(a, tiles, 1, ksplit, misaligned, st))
   return qtype == NNTR_Q4_K ? NNTR_MMA_RUN(NNTR_Q4_K) : NNTR_MMA_RUN(NNTR_Q4_0);
 #undef NNTR_MMA_RUN
 }
@@ -1067,11 +1095,11 @@ int launch_gemm_grouped(int qtype, unsigned N, unsigned K, const void *act, floa
   const unsigned z = w_table1 ? 2 : 1;
   const bool ksplit = tile_rows <= 16 && (uint64_t)tiles * z * ((N + 15) / 16) <= 2u * (unsigned)sm_count();
   if (qtype == NNTR_Q4_K)
-    return tile_rows <= 16 ? run_tiles<NNTR_Q4_K, 2, true, true>(a, tiles, z, ksplit, st)
-                           : run_tiles<NNTR_Q4_K, 4, true, true>(a, tiles, z, ksplit, st);
+    return tile_rows <= 16 ? run_tiles<NNTR_Q4_K, 2, true, true>(a, tiles, z, ksplit, false, st)
+                           : run_tiles<NNTR_Q4_K, 4, true, true>(a, tiles, z, ksplit, false, st);
   if (qtype == NNTR_Q4_0)
-    return tile_rows <= 8 ? run_tiles<NNTR_Q4_0, 1, true, true>(a, tiles, z, ksplit, st)
-                          : run_tiles<NNTR_Q4_0, 4, true, true>(a, tiles, z, ksplit, st);
+    return tile_rows <= 8 ? run_tiles<NNTR_Q4_0, 1, true, true>(a, tiles, z, ksplit, false, st)
+                          : run_tiles<NNTR_Q4_0, 4, true, true>(a, tiles, z, ksplit, false, st);
   return set_error(NNTR_CUDA_ERR_UNSUPPORTED, "gemm_grouped: expert weights must be Q4_K or Q4_0");
 }
 
