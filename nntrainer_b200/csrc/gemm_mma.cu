@@ -640,11 +640,6 @@ template <int NT> struct KsShared {
   int abort_flag;
 };
 
-/** barrier `id` of two warps: the one in front arrives, the other one waits for it. Two tiles of rows take all sixteen barriers,
- *  number 0 among them, so nothing between the first hand-over and the last may be a barrier of the whole CTA. */
-__device__ __forceinline__ void pair_arrive(int id) { asm volatile("barrier.cta.arrive %0, 64;" ::"r"(id) : "memory"); }
-__device__ __forceinline__ void pair_sync(int id) { asm volatile("barrier.cta.sync %0, 64;" ::"r"(id) : "memory"); }
-
 /** COPIES: the weights start at a multiple of 16 and bulk copies bring them in; otherwise they start at a multiple of 8 and every
  *  warp brings its own units in by 8-byte copies. Instances of their own: as branches of one they cost Q4_K with two tiles 2 to 3 %
  *  (16 x 4096 x 4096 9.8 -> 10.1 us). Q4_K at a multiple of 8, 8 x 2560 x 9728 13.0 us, 256 x 4096 x 4096 101 (loads into registers one
@@ -652,7 +647,7 @@ __device__ __forceinline__ void pair_sync(int id) { asm volatile("barrier.cta.sy
 template <int QT, int NT, bool GROUPED, bool TH8, bool COPIES>
 __global__ void __launch_bounds__(KS_WARPS * 32, 2) gemm_mma_ksplit_kernel(const MmaArgs a) {
   extern __shared__ __align__(16) uint8_t ks_smem[];
-  static_assert(KS_WARPS * NT <= 16, "a hand-over barrier per warp and tile");
+  static_assert(KS_WARPS * NT <= 16, "a hand-over barrier per warp and tile"); // with 16, nothing in the loop may be a barrier of the CTA
   KsShared<NT> &sh = *reinterpret_cast<KsShared<NT> *>(ks_smem);
   volatile int *abort_flag = &sh.abort_flag;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, g = lane >> 2, t = lane & 3;
@@ -871,7 +866,7 @@ __global__ void __launch_bounds__(KS_WARPS * 32, 2) gemm_mma_ksplit_kernel(const
           if constexpr (QT == NNTR_Q4_K)
             sh.chain[to_warp][i][1][lane] = make_float4(accm[0], accm[1], accm[2], accm[3]);
           pair_arrive(to_warp * NT + i);
-        } else if (ok) {
+        } else if (nobody_gave_up(ok, abort_flag)) {
 #pragma unroll
           for (int c = 0; c < 4; ++c) {
             const int m = 8 * i + 2 * t + (c & 1);

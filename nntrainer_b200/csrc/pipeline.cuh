@@ -68,6 +68,14 @@ __device__ __forceinline__ bool mbar_wait_bounded(uint32_t bar, uint32_t parity,
   return false;
 }
 
+/** A chain that goes from warp to warp: the warp in front arrives at barrier `id`, the one behind waits for it. Number 0 is the
+ *  barrier of __syncthreads(): where it is used for a hand-over, no barrier of the whole CTA may lie between the first and the last. */
+__device__ __forceinline__ void pair_arrive(int id) { asm volatile("barrier.cta.arrive %0, 64;" ::"r"(id) : "memory"); }
+__device__ __forceinline__ void pair_sync(int id) { asm volatile("barrier.cta.sync %0, 64;" ::"r"(id) : "memory"); }
+/** For the last warp of such a chain, behind its hand-over: whether its own waits and those of every warp in front (that raise the
+ *  flag before they hand over) came to their end. Without that the sums are incomplete and must not be stored. */
+__device__ __forceinline__ bool nobody_gave_up(bool ok, const volatile int *abort_flag) { return ok && !*abort_flag; }
+
 /** Bulk copy global -> shared memory of this CTA, completion counted in bytes on an mbarrier. Both addresses 16-byte
  *  aligned, size a multiple of 16. Local memory only (no multicast). */
 __device__ __forceinline__ void bulk_g2s(uint32_t dst, const void *src, uint32_t bytes, uint32_t bar) {
