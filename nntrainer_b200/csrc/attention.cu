@@ -434,12 +434,14 @@ __global__ void attn_values_kernel(const float *__restrict__ probs, const uint16
  *            ascending row order by one warp (ordered_sum).
  *   values   a thread per dimension runs the row-ordered chain over value tiles that a producer warp keeps ahead of it
  *            (tiled TMA copies, started before the scores).
- * Clock stamps of one CTA per cluster, 64 / 8 heads of 64, at 512 / 4096 rows, in clocks: start and first copies 900 / 1000, heads
- * rotated 900, score tiles 1700 / 9100, barrier behind them 2200 / 2600, maximum 900, exponentials 600 / 2800, ordered sum 2600 /
- * 11500, division 400 / 1450, value chain 5600 / 33000. The value chain is half of a long context at about 8 clocks per row (six
- * inside a tile, the rest where it waits for one), where a dependent multiply-add alone takes four. 64 / 8 heads of 64 at 4096
- * rows 37 us, 32 / 8 heads of 128 at 512 rows 11.3 us (with generic accesses to the tiles, and value tiles of 128 rows: 45 and
- * 12.4), at 128 rows of a window 8.0 us with the copy of q (8.4). Measured and not kept: value tiles turned round by the idle warps
+ * Clock stamps of one CTA, 64 / 8 heads of 64, at 512 / 4096 rows, in clocks: up to the grid dependency 1800 / 1850, first copies and
+ * heads rotated 1350 / 1450, wait for the cluster 400, score tiles 1600 / 8800, barrier behind them 2050 / 2600, maximum and
+ * exponentials 1500 / 3800, ordered sum 2500 / 11500, division 450 / 1450, value chain 5400 / 33800. The value chain is half of a long
+ * context at about 8 clocks per row (six inside a tile, the rest where it waits for one), where a dependent multiply-add alone
+ * takes four. In a decode step, whose launches find neither code nor caches at hand, the phases up to 512 rows take half as long again
+ * (32 / 8 heads of 128 at 100 rows 14300 clocks behind the dependency, alone 8900). 64 / 8 heads of 64 at 4096 rows 36.5 us, 32 / 8 heads
+ * of 128 at 512 rows 11.2 us (with generic accesses to the tiles, and value tiles of 128 rows: 45 and 12.3), at 128 rows of a window
+ * 8.0 us with the copy of q (8.4). Measured and not kept: value tiles turned round by the idle warps
  * for 16-byte loads (46 us), half of the ring waited for at a time (44), four blocks of the ordered sum at once (16900 clocks
  * instead of 11500), two rows and two heads per thread in the scores (heads of 64: 1800 a tile instead of 1900; of 128: 2660
  * instead of 2200).
@@ -447,7 +449,7 @@ __global__ void attn_values_kernel(const float *__restrict__ probs, const uint16
 constexpr int AC_THREADS = 256;
 constexpr int AC_WARPS = AC_THREADS / 32;
 constexpr int AC_TILE = 128; // cache rows per tile of keys
-constexpr uint32_t AC_SMEM_ALONE = 200u * 1024u; // of which two CTAs do not fit an SM, nor one and the next kernel's
+constexpr uint32_t AC_SMEM_ALONE = 200u * 1024u; // beside which an SM has room for launches of up to about 26 KB only
 constexpr int AC_KBUF_MAX = 4;
 constexpr int AC_VBUF_MAX = 6;
 /** cache rows per tile of values: a wait for a tile costs 350 clocks of the chain */
@@ -580,11 +582,13 @@ __device__ __forceinline__ float serial_sum(const float *e, unsigned lo, unsigne
  * nearest, and only for an exact half does the choice depend on S. So the integers of 256 rows are added in any order, eight rows
  * per lane, and S + their sum is the serial result as long as it stays below 2^24 and no half occurred. Where one of the two
  * happens, the lanes in front of the first such lane are taken, that lane's eight rows are added serially, and the next 256
- * rows start behind them. That takes about 430 clocks per 256 rows, interruptions among them, against 2800 for the serial
- * chain (11 clocks a row), and interruptions are few (a power of two is passed log2(rows) times; a half has probability e / s per row, so the first rows
- * are added serially) -- after AC_SUM_STOPS of them the rest is added serially. */
+ * rows start behind them. That takes 700 (4096 rows) to 1000 (2048) clocks per 256 rows, interruptions among them, against 1250 for the
+ * serial chain (4.9 clocks a row). A power of two is passed log2(rows) times; a half has probability e / s per row, so the first rows
+ * are added serially. After AC_SUM_STOPS interruptions the rest is added serially. */
 constexpr unsigned AC_SUM_SERIAL = 64;    // rows at the start
-constexpr unsigned AC_SUM_PARALLEL = 768; // below this many rows the serial chain is as fast
+/* Below this many rows the serial chain. The two forms cross later, between 1400 rows (64 / 8 heads of 64: 19.6 us, with the serial chain
+ * 18.2; 800 rows 15.2 and 13.6; 32 / 8 heads of 128 within 0.6 of these) and 2048 (8300 clocks, serial about 10000). */
+constexpr unsigned AC_SUM_PARALLEL = 768;
 constexpr int AC_SUM_STOPS = 40;
 __device__ __forceinline__ float ordered_sum(const float *e, unsigned cnt, float s, int lane) {
   if (cnt < AC_SUM_PARALLEL)
@@ -848,8 +852,7 @@ attn_cluster_kernel(const __grid_constant__ CUtensorMap kmap, const __grid_const
   } else if (warp < DIMS / 32) {
     const int d = item_d0 + tid;
     float acc = 0.f;
-    // Sixteen rows in the chain while the next sixteen -- of the next tile at a tile's end -- are on their way. 11.2 clocks per
-    // row all the same (the dependent multiply-add: 4); what holds it up has not been found.
+    // Sixteen rows in the chain while the next sixteen -- of the next tile at a tile's end -- are on their way.
     float pr[2][16];
     uint16_t vb[2][16];
     auto load = [&](const uint16_t *vt, const float *pt, float(&pp)[16], uint16_t(&vv)[16]) {
@@ -879,11 +882,13 @@ attn_cluster_kernel(const __grid_constant__ CUtensorMap kmap, const __grid_const
         npar ^= 1;
       }
       const uint16_t *nvt = reinterpret_cast<const uint16_t *>(vtile + nbuf * vbytes) + tid;
-      // asked now, needed sixteen rows before this tile's end: the answer takes about a hundred clocks
+      // asked now, needed sixteen rows before this tile's end: the answer takes about a hundred clocks (a question that may not suspend
+      // the thread, test_wait, measured the same: 37.2 us for 4096 rows, replay 3225 and 3231)
       const bool next_here = t + 1 < v_tiles && mbar_try_wait(vfull0 + 8 * nbuf, npar);
       if (rows == VROWS) {
-        // Unrolled further, a tile of 256 rows is 14 KB of code: 1.6 us less for 4096 rows (36.8 and 35.2), but 4 % more for a decode step
-        // of a context of 512 (16 tokens over four layers 3386 us, 3252 like this), where every launch fetches its code anew. Not at all: 39.5.
+        // Unrolled all the way, a tile of 256 rows is 14 KB of code: 1.6 us less for 4096 rows (36.8 and 35.2), but 4 % more for a decode
+        // step at a context of 512 (16 tokens over four layers 3386 us, 3252 like this), where every launch fetches its code anew. Not
+        // unrolled at all: 39.5 us.
 #pragma unroll(DIMS == 64 ? 2 : 4)
         for (int j = 0; j < VROWS; j += 32) {
           load(vt + (j + 16) * DIMS, pt + j + 16, pr[1], vb[1]);
@@ -901,7 +906,7 @@ attn_cluster_kernel(const __grid_constant__ CUtensorMap kmap, const __grid_const
       } else { // the last tile
         // The compiler unrolls these two loops further where it is let, and a short context's launch, which has just this tile, waits for
         // the code: 16 tokens over four layers at a context of 30 / 100 / 512 2976 / 3058 / 3241 us, like this 2922 / 2939 / 3219 (value
-        // phase at 100 rows 5700 clocks, 3500; taken alone, with the code at hand, 2200 and 2050). Not unrolled at all 2911 / 2928 / 3225,
+        // phase at 100 rows 5700 clocks, 3700; taken alone, with the code at hand, 2200 and 2000). Not unrolled at all 2911 / 2928 / 3225,
         // but 0.2 us more for a launch of 128 rows alone.
         unsigned j = 0;
 #pragma unroll 2
@@ -1031,7 +1036,7 @@ static int launch_attn_cluster(AttnStep a, unsigned bound, unsigned rows, unsign
   unsigned csize = clusters > 12 && items <= 4 ? 4 : 8;
   while (csize > 1 && (many || clusters * csize > 144u) && (int)(csize / 2) >= items)
     csize /= 2;
-  // buffers for what the launch can need, no more: the next kernel's CTAs want room beside this one's
+  // buffers for what the launch can need, no more: a prompt's CTAs share an SM where they fit
   a.cap_rows = rows;
   const unsigned k_tiles = ((rows + csize - 1) / csize + AC_TILE - 1) / AC_TILE, v_rows = dims == 64 ? 256u : 128u, v_tiles = (rows + v_rows - 1) / v_rows;
   const unsigned k_max = hd <= 64 ? 4u : 2u;
@@ -1074,8 +1079,9 @@ static int launch_attn_cluster(AttnStep a, unsigned bound, unsigned rows, unsign
   cfg.gridDim = dim3(clusters * csize, a.tokens);
   cfg.blockDim = dim3(AC_THREADS);
   // A decode step's CTAs keep their SMs to themselves: a second one of them, or the next launch's, let in early, takes issue slots and
-  // the way to memory from a kernel that is bound by latency. 16 tokens over four layers at a context of 100 / 250 / 512: 3144 / 3156
-  // / 3276 us where only a second one is kept out (116 KB), 3052 / 3069 / 3243 with 200 KB.
+  // the way to memory from a kernel that is bound by latency. 16 tokens over four layers, 32 / 8 heads of 128 at a context of 30 / 100 /
+  // 250 / 512: 3028 / 3059 / 3103 / 3252 us with what the buffers need, 2935 / 2949 / 3042 / 3217 with 200 KB; 64 / 8 heads of 64 at 100 /
+  // 512 / 2000: 2977 / 3229 / 3880 and 2922 / 3140 / 3880.
   cfg.dynamicSmemBytes = a.tokens == 1 && L.total < AC_SMEM_ALONE ? AC_SMEM_ALONE : L.total;
   const cudaError_t e = cudaLaunchKernelEx(&cfg, kernel, kmap, vmap, a);
   count_launch();

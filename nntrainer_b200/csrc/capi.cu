@@ -278,7 +278,11 @@ __global__ void host_done_kernel(unsigned long long *word, unsigned long long va
 
 /* --------------------------------------------------------- GEMM dispatch */
 static std::atomic<int> g_gemm_path{NNTR_CUDA_GEMM_PATH_AUTO};
-constexpr unsigned TENSOR_PATH_MIN_M = 32; // below this the exact kernels win (a 128-row activation tile is mostly padding)
+/* Below this the exact kernels win: a 128-row activation tile is mostly padding there. Exact against automatic at 32 / 64 rows: Q4_K
+ * 6144 x 2560 12.8 / 16.0 us against 19.0 / 19.5, 4096 x 4096 17.5 / 22.5 against 17.1 / 17.7, 24576 x 4096 36.1 / 66.4 against 50.0 / 50.2;
+ * Q4_0 24576 x 4096 32.8 / 50.2 against 49.5 / 49.5; Q6_K 151936 x 2560, 32 rows, 338 against 272. For Q4_K and Q4_0 the times cross
+ * between 32 and 64 rows and later. */
+constexpr unsigned TENSOR_PATH_MIN_M = 32;
 
 /* 0: exact kernels, 1: integer tensor path (kind::i8), 2: fp16 tensor path (kind::f16) */
 static int pick_gemm_kernel(int qtype, unsigned M, unsigned N, unsigned K) {

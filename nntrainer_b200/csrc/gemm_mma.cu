@@ -26,11 +26,11 @@
  *                          operations alike: per 16 x 8 x 32 of Q4_0 about 20 instructions, 4 wavefronts of shared memory, 8 half-rate
  *                          operations, four to five clocks of an SM each, seven taken. Q4_0 1000 x 8000 x 4096 208 us (a
  *                          computing thread starting the copies, 25 instructions: 303), 509 x 2880 x 2880 36.9 us (51.6); Q4_K
- *                          255 x 9728 x 2560 55.7 us (75.4).
+ *                          255 x 9728 x 2560 77.8 us, on the one-step chain of gemv_rows 55.7 (87.8 and 75.5).
  *   gemm_mma_ksplit_kernel eight warps share the tile and take every eighth unit of 256 along K; the float chains go from warp
  *                          to warp, one unit further at each. For the others: bound by that hand-over (270 clocks a unit) when
  *                          K is long, by launch and round trips when it is short. With the quantizer's launch: Q4_K 8 x 2560 x 2560
- *                          6.4 us, 8 x 2560 x 9728 12.3 us (terms through shared memory to one thread per chain: 8.8 and 18.7).
+ *                          5.9 us, 8 x 2560 x 9728 12.0 us (terms through shared memory to one thread per chain: 8.5 and 18.6).
  */
 #include <type_traits>
 
@@ -418,10 +418,15 @@ constexpr int ROWS_W = ROWS_WARPS * 2 * (int)sizeof(BlockQ4Kx8); // the weights 
 __device__ int g_mma_status = 0;
 
 /* Units in flight per CTA and the CTAs per SM that registers and shared memory are held to. More warps hide more latency until
- * registers spill or the ring gets too short; measured with 2 to 5 stages and 2 to 9 CTAs. Q4_0 1000 x 8000 x 4096 with 3 / 4 / 5 CTAs
- * of 32 rows 226 / 201 / 230 us; Q4_K (12 of 16 warps' worth of registers) 31 x 24576 x 4096 with 3 / 4: 51 / 70; 16 rows, 16 x 24576
- * x 4096 with 3 / 4: 23 / 28. Q4_0 tiles of 8 rows per expert, 8 tokens through 4 of 32 experts of 2880 x 2880 with 6 / 7 / 8 CTAs:
- * 102 / 88 / 95 (what counts there is how the last round fills). */
+ * registers spill by much or the ring gets too short; measured with 2 to 5 stages and 2 to 9 CTAs. Q4_0 1000 x 8000 x 4096 with 3 / 4 / 5
+ * CTAs of 32 rows 226 / 201 / 230 us; Q4_K (12 of 16 warps' worth of registers) 31 x 24576 x 4096 with 3 / 4: 51 / 70; 16 rows, 16 x 24576
+ * x 4096 with 3 / 4: 23 / 28. The third CTA of Q4_K's 32 rows costs 120 bytes of spills and pays for them: with 2 CTAs and none
+ * 31 x 24576 x 4096 60.5 us instead of 48.1, 255 x 9728 x 2560 85.8 instead of 77.2.
+ * Q4_0 tiles of 8 rows per expert: as many as the kernel's 55 registers allow, seven. Which number wins at one batch size depends on
+ * how the last round fills, so over sizes: 4 of 32 experts of 2880 x 2880, 17 batches of 5 to 48 tokens, 4 of 32 of 1024 x 1440 (9), 2 of
+ * 16 of 4096 x 4096 (6), 4 of 64 of 1024 x 2880 (8 batches, 5 to 96): six take 1.008 / 1.009 / 0.995 / 0.974 times as long as seven in the
+ * geometric mean, eight 1.046 / 1.001 / 1.036 / 0.982; single batches differ by up to 15 % either way (8 tokens of the first layer
+ * with 6 / 7 / 8: 94.9 / 88.8 / 97.1 us, 16 tokens 113 / 122 / 124, 24 tokens of the third 131 / 118 / 129). */
 template <int QT, int NT, bool GROUPED> constexpr int rows_stages() { return QT == NNTR_Q4_0 && NT == 1 && GROUPED ? 2 : 3; }
 template <int QT, int NT, bool GROUPED> constexpr int rows_ctas() {
   return QT == NNTR_Q4_0 ? (NT >= 2 ? 4 : GROUPED ? 7 : 5) : (NT == 4 ? 3 : NT == 2 ? 3 + GROUPED : 4);
@@ -1018,10 +1023,11 @@ int launch_gemm_mma(int qtype, unsigned M, unsigned M4, unsigned N, unsigned K, 
   const auto tiles_of = [&](unsigned nt) { return (M + 8 * nt - 1) / (8 * nt); };
   // One CTA per tile of 8 or 16 rows as long as all of them run at once, two per SM. Beyond that a warp per tile: of 32 rows (the
   // weights are unpacked once for them) where CTAs of 64 weight rows still give every SM work, else of 16, else of 8. Measured on both
-  // sides: Q4_K 8 x 2560 x 2560 (160 CTAs) 6.4 us, a warp per tile 8.8; 8 x 6144 x 2560 (384) 9.5 and 9.0; 31 x 2560 x 2560 (320 of 16
-  // rows) 12.6 and 11.4. A warp per tile of 16 / 32 rows: Q4_K 31 x 12288 x 4096 (192 items of 32) 27.5 / 36.9 us, 63 x 9728 x 2560
-  // (304) 22.8 / 22.0; Q4_0 31 x 2560 x 2560 (40) 9.2 / 10.9, 64 x 2880 x 2880 (90) 12.8 / 12.7, 31 x 12288 x 4096 (192) 23.1 / 20.6;
-  // of 8 / 16 rows: Q4_K 31 x 2560 x 2560 (80 of 16) 11.4 / 11.8, 16 x 6144 x 2560 (96) 10.8 / 10.6.
+  // sides: Q4_K 8 x 2560 x 2560 (160 CTAs) 5.9 us, a warp per tile 8.4; 8 x 4736 x 2560 (296) 5.9 and 9.1; 8 x 6144 x 2560 (384) 9.7 and
+  // 9.2; 31 x 2560 x 2560 (320 of 16 rows) 12.3 and 11.4. A warp per tile of 16 / 32 rows: Q4_K 31 x 12288 x 4096 (192 items of 32) 27.1 /
+  // 36.9 us, 64 x 9728 x 2560 (304) 24.2 / 24.4, 63 through gemv_rows 22.7 / 21.9; Q4_0 31 x 2560 x 2560 (40) 9.3 / 11.1, 64 x 2880 x 2880
+  // (90) 12.8 / 12.5, 31 x 12288 x 4096 (192) 23.6 / 20.7; of 8 / 16 rows: Q4_K 31 x 2560 x 2560 (80 of 16) 11.4 / 11.9, 16 x 6144 x 2560
+  // (96) 10.8 / 10.6.
   const bool ksplit = misaligned || (uint64_t)tiles_of(2) * row_tiles <= 2u * sms;
   unsigned nt;
   if (ksplit)

@@ -49,12 +49,13 @@ struct MoeEp {
 /* From where on the pairs are sorted by expert and run as per-expert GEMMs (all of a batch's rows for one read of an expert's
  * weights, but three launches more than a GEMV per pair): where a GEMV per pair no longer gets enough of the GPU. Q4_0 (gate and
  * up are two problems per pair, one CTA per SM): below four CTAs per problem; 4 of 32 experts of 2880 x 2880, 2 / 4 / 5 / 8
- * tokens: GEMVs 45 / 73 / 90 / 128 us, grouped 60 / 81 / 85 / 101. Q4_K (one problem per pair, two CTAs per SM): below three;
- * 8 of 128 experts of 2048 x 768, 8 / 12 / 14 tokens: 60 / 77 / 104 us against 71 / 88 / 92. Other experts, GEMVs against grouped on
- * both sides of the line: Q4_0 4 of 32 of 1024 x 1440, 4 / 5 / 8 / 12 tokens 29 / 33 / 41 / 64 us against 37 / 36 / 41 / 46; 2 of 16 of
- * 4096 x 4096, 9 / 10 tokens 106 / 130 against 115 / 121; Q4_K 4 of 64 of 1024 x 512, 24 / 25 tokens 41 / 50 against 47 / 47. Wide Q4_K
- * experts cross earlier than the line says: 4 of 32 of 4096 x 1536, 6 / 12 / 16 / 24 tokens 74 / 133 / 186 / 244 against 77 / 119 / 124 /
- * 128, because there a GEMV per pair reads an expert's weights again for each of its tokens. */
+ * tokens: GEMVs 43 / 73 / 89 / 128 us, grouped 54 / 74 / 79 / 88. Q4_K (one problem per pair, two CTAs per SM): below three;
+ * 8 of 128 experts of 2048 x 768, 8 / 10 / 12 / 14 tokens: 60 / 75 / 76 / 104 us against 65 / 70 / 75 / 80, so the grouped products are
+ * ahead a little before the line. Other experts, GEMVs against grouped on both sides of it: Q4_0 4 of 32 of 1024 x 1440, 4 / 5 / 8 / 12
+ * tokens 28 / 32 / 40 / 62 us against 34 / 36 / 37 / 42; 2 of 16 of 4096 x 4096, 8 / 9 / 10 tokens 101 / 103 / 129 against 100 / 94 / 104;
+ * Q4_K 4 of 64 of 1024 x 512, 20 / 24 / 25 tokens 39 / 40 / 48 against 41 / 43 / 44. Wide Q4_K experts cross well before the line: 4 of 32
+ * of 4096 x 1536, 6 / 12 / 16 / 24 tokens 74 / 131 / 185 / 243 against 80 / 96 / 106 / 109, because there a GEMV per pair reads an expert's
+ * weights again for each of its tokens. */
 constexpr unsigned GROUPED_MIN_TOKENS = 2;
 static bool run_grouped(int qtype, unsigned tokens, unsigned pairs) {
   return tokens >= GROUPED_MIN_TOKENS && (qtype == NNTR_Q4_0 ? 8 * pairs > (unsigned)sm_count() : 3 * pairs > 2 * (unsigned)sm_count());
