@@ -73,8 +73,6 @@ extern "C" int nntr_cuda_gemm_q4_K_noalloc_dev(unsigned M, unsigned N, unsigned 
     return NNTR_CUDA_OK;
   if (!A || !B || !C)
     return set_error(NNTR_CUDA_ERR_INVALID, "gemm_q4_K_noalloc: null pointer");
-  if (reinterpret_cast<uintptr_t>(B) & 7) // the limit of the exact kernels' loads
-    return set_error(NNTR_CUDA_ERR_INVALID, "gemm_q4_K_noalloc: weights must be 8-byte aligned");
   if (ldc < N)
     return set_error(NNTR_CUDA_ERR_INVALID, "gemm_q4_K_noalloc: ldc (%u) < N (%u)", ldc, N);
   const size_t row_bytes = (size_t)(K / QK_K) * sizeof(BlockQ8K);

@@ -74,16 +74,6 @@ def test_misaligned_weights_are_refused_before_anything_is_launched(L, q, off, M
     assert L.nntr_cuda_launch_count() == before
 
 
-@pytest.mark.parametrize("off", [1, 2, 4])
-@pytest.mark.parametrize("M", [1, 2, 37])
-def test_misaligned_weights_are_refused_by_the_entry_that_allocates_nothing(L, off, M):
-    """The same limit as for the entry with a workspace: the loads of such weights would fault."""
-    N, K, p = 64, 1024, 1 << 20
-    before = L.nntr_cuda_launch_count()
-    assert L.nntr_cuda_gemm_q4_K_noalloc_dev(M, N, K, p, K, p + off, N, p, N, None) == capi.ERR_INVALID
-    assert b"aligned" in L.nntr_cuda_last_error() and L.nntr_cuda_launch_count() == before
-
-
 @pytest.mark.parametrize("qtype,kind", [("q4_K", 0), ("q4_0", 1)])
 @pytest.mark.parametrize("tokens", [1, 7, 64, 400])
 def test_moe_tokens_off_a_16_byte_boundary_are_refused_before_anything_is_launched(L, qtype, kind, tokens):
