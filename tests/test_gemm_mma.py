@@ -32,7 +32,7 @@ def exact(be, q, A, B, N):
     return got[:, :N]
 
 
-# the first shapes run the K split, the wide ones (from about 1200 tiles of 16 rows) the kernel in which a warp owns its rows
+# the first shapes run the K split, the wide ones (more CTAs than two per SM) the kernel in which a warp owns its rows
 SHAPES = [(2, 8, 256), (7, 24, 2304), (8, 136, 2560), (9, 16, 4352), (17, 40, 768), (33, 24, 512), (3, 19000, 512),
           (16, 19000, 256), (37, 19000, 768)]
 

@@ -20,7 +20,7 @@ def be():
     backend.set_gemm_path("auto")
 
 
-# a CTA per tile: one round of one unit, two of 7 + 6, three of 6 + 6 + 5; tiles of 8 and of 16 rows
+# a CTA per tile: one round of one unit, two of 7 + 6, a tile of 16 rows with one round of two (more rounds of those below)
 # a warp per tile, 64 weight rows an item: 592 or 444 CTAs at a time, so one item each, two rounds with a rest in halves or quarters
 SHAPES = [(5, 40, 256), (12, 48, 3328), (20, 4104, 4352), (9, 2568, 512),
           (6, 37000, 256), (13, 31000, 512), (70, 12040, 512), (37, 23000, 256), (100, 16400, 256)]
@@ -75,12 +75,33 @@ def test_several_rounds_of_weights_at_a_multiple_of_eight_bytes(be, port, q, gen
     be.gemv_rows(q, M, N, K, a, torch.from_numpy(B).cuda(), E, N, ws)
     be.device_status()
     assert torch.equal(D.view(torch.int32), E.view(torch.int32))
+    getattr(be, f"gemm_{q}")(M, N, K, a, K, torch.from_numpy(B).cuda(), N, E, N)  # the same rounds of weights at a multiple of 16
+    be.device_status()
+    assert torch.equal(E.view(torch.int32), C.view(torch.int32))
     if q == "q4_K":
         D.fill_(float("nan"))
         capi.check(capi.lib().nntr_cuda_gemm_q4_K_noalloc_dev(M, N, K, a.data_ptr(), K, at8.data_ptr(), N, D.data_ptr(), N,
                                                               torch.cuda.current_stream().cuda_stream))
         be.device_status()
         assert torch.equal(D.view(torch.int32), C.view(torch.int32))
+
+
+@pytest.mark.parametrize("off", [0, 8])
+@pytest.mark.parametrize("M", [1, 3, 7])
+def test_activation_tiles_of_fewer_than_eight_rows(be, port, M, off):
+    """The built-in scratch holds seven rows of this length, but no tile of eight: rows as many as there are, 256 rounds of units."""
+    from nntrainer_b200 import capi
+    N, K = 24, 524288
+    rng = np.random.default_rng(M)
+    A = rng.standard_normal((M, K)).astype(np.float32)
+    B = O.random_q4_Kx8(rng, N, K)
+    b = torch.zeros(B.nbytes + 16, dtype=torch.uint8, device="cuda")[off:off + B.nbytes]
+    b.copy_(torch.from_numpy(B.view(np.uint8).reshape(-1)))
+    a, C = torch.from_numpy(A).cuda(), torch.full((M, N), float("nan"), device="cuda")
+    capi.check(capi.lib().nntr_cuda_gemm_q4_K_noalloc_dev(M, N, K, a.data_ptr(), K, b.data_ptr(), N, C.data_ptr(), N,
+                                                          torch.cuda.current_stream().cuda_stream))
+    be.device_status()
+    assert np.array_equal(C.cpu().numpy().view(np.uint32), port.gemm("q4_K", A, B, N).view(np.uint32))
 
 
 # both table kernels: the down product of the first layer and gate and up of the second have few tiles and split K (9 and 10 units),
