@@ -12,7 +12,7 @@
  * Those chains leave the integer domain once per 64, 256 or 32 of K, so an accumulator that lives in tensor memory would
  * be drained that often. The warp MMA m16n8k32 leaves its sums in registers instead, one sub-block per instruction, and
  * its A fragment is what one 8-byte (Q4_K) or 4-byte (Q4_0) piece of the interleaved weight block holds: the low and the
- * high nibbles of 4 bytes each, one logic op per fragment register and no trip through shared memory.
+ * high nibbles of 4 bytes each, a mask and at most a shift per fragment register.
  *
  * A sub-block's sum and its 6-bit scale meet as integers (|I| <= 15 * 127 * 32, sc <= 63): a pair of sub-blocks stays below
  * 2^23, which fp32 holds, a super-block below 2^25, whose one conversion rounds as the reference's does. The sums of the mins
