@@ -25,31 +25,34 @@
  * 256 of K, no mins term. What is left outside the tensor pipe is the nibble
  * expansion (about two instructions per weight) and one epilogue per tile.
  *
- * One CTA owns two tiles of 128 activation rows (MMA M, tensor-memory lanes)
- * against the same 256 weight rows (MMA N, columns), so every expanded weight
- * stage feeds two MMAs, and walks K in stages of 64 (one pair of sub-blocks):
+ * Up to 256 activation rows, a CTA owns two tiles of 128 of them (MMA M, tensor-memory lanes) against the same 256 weight rows (MMA N,
+ * columns), so every expanded weight stage feeds two MMAs. With more rows a pair of CTAs owns four tiles: each CTA expands half of the
+ * weight rows, an MMA (cta_group::2) takes 128 activation rows of each and the weights of both, and an expanded stage feeds 512 rows.
+ * A CTA walks K in stages of 64 (one pair of sub-blocks):
  *   warps 0-15  producers: expand a stage's nibble bytes into 64 fp16 values per
  *               weight row. A 32-bit word yields four half2 with one
  *               logic op each ((w >> s) & 0x000F000F | 0x64006400 is
  *               (1024 + n_lo, 1024 + n_hi)), so the K order inside a stage is
  *               the order that unpack produces; the activation tiles are written
  *               in the same order (a dot product does not care). Q4_K and Q4_0:
- *               one thread per row, eight warps take the even and eight the odd
- *               stages. Q6_K: two threads per row, all warps every stage. After
+ *               one thread per row, two groups of eight warps (pair: four of four)
+ *               take the stages in turn. Q6_K: two threads per row, all warps
+ *               every stage (pair: two groups, two stages in turn). After
  *               the last stage the same warps are the epilogue: tcgen05.ld of the
  *               tile, a turn through shared memory, stores of C by whole lines.
- *   warp 16     one thread issues 8 MMAs (128 x 256 x 16) per stage.
+ *   warp 16     one thread issues 8 MMAs per stage; in a pair's second CTA it
+ *               tells the first one that a stage is ready here.
  *   warp 17     one thread starts the bulk copies of the activation stages, each
  *               as soon as the MMAs that read its slot have retired.
  *   warp 18     one thread starts the tiled copies of the packed weights
- *               (Q4_K, Q4_0) into a ring of two stages.
- * Three stages of 64 KB, both accumulators (512 columns) in tensor memory. Every wait is bounded (pipeline.cuh).
+ *               (Q4_K, Q4_0) into a ring of two (pair: four) stages.
+ * Three stages of 64 KB (pair: four of 48), both accumulators (512 columns) in tensor memory. Every wait is bounded (pipeline.cuh).
  *
- * What bounds it: the producers. A stage's MMAs take 1024 clocks, a stage took 1780: about 520 clocks of instruction issue,
- * and around it two waits, a fence and the arrive at 100-270 clocks each, in all sixteen warps at the same time. In two
- * groups, one group's latencies pass while the other expands. The tile's stores took 27 of its 142 thousand clocks while
- * every lane wrote a row of its own. Both changes, 1024 x 24576 x 4096 Q4_K: 221 -> 192 us (1076 TFLOP/s), 256 rows
- * 74 -> 65, Q4_0 1024 rows 201 -> 186; Q6_K 256 x 151936 x 2560 552 -> 359 (the stores).
+ * What bounds it. A stage's MMAs take 1024 clocks. A CTA alone takes 1310 a stage: its producers, and the shared memory, which
+ * carries 96 KB for the MMAs, 64 of stores and copies and the packed weights. A pair takes 1070, the MMAs: half of the expansion and 64 KB
+ * for the MMAs. (With no expansion and no copies at all 1050; a hand-over from CTA to CTA with release and acquire at cluster
+ * scope 1600: it is one more latency in each round of the ring.) Q4_K 24576 x 4096, 1024 rows 184.6 -> 167 us, 512
+ * rows 115.9 -> 101.6; Q4_0 512 rows of 24576 x 2880 85.2 -> 77.3; Q6_K 151936 x 2560, 300 / 512 rows 515 / 572 -> 346 / 380.
  *
  * Few tiles: a cluster of two, four or eight CTAs shares a tile, each walks a part of K (k_parts), and the sums are added
  * through distributed shared memory. 512 x 1280 x 2560: Q4_0 40 -> 25 us, Q6_K 69 -> 33; 128 x 2560 x 8192: Q4_0 93 -> 25,
@@ -66,31 +69,40 @@ namespace nntr {
 
 namespace {
 
-constexpr int F16_TILE_M = 128;  // activation rows per CTA
-constexpr int F16_TILE_N = 256;  // weight rows per CTA
+constexpr int F16_TILE_M = 128;  // rows of an activation tile
+constexpr int F16_TILE_N = 256;  // weight rows of a tile of C
 constexpr int F16_KS = 64;       // K per stage
-constexpr int F16_W_BYTES = F16_TILE_N * F16_KS * 2; // 32 KB
 constexpr int F16_A_BYTES = F16_TILE_M * F16_KS * 2; // 16 KB
-constexpr int F16_STAGE_BYTES = F16_W_BYTES + 2 * F16_A_BYTES; // weights + two activation tiles (256 rows)
-constexpr int F16_STAGES = 3;
 constexpr int F16_PRODUCERS = 512;
-/* Q4_K, Q4_0: two groups of 256 threads, one thread per weight row, take alternate stages; Q6_K: two threads per row */
-__host__ __device__ constexpr int f16_stage_warps(int qt) { return qt == NNTR_Q6_K ? F16_PRODUCERS / 32 : F16_PRODUCERS / 64; }
 constexpr int F16_MMA_WARP = F16_PRODUCERS / 32;
 constexpr int F16_COPY_WARP = F16_MMA_WARP + 1;
 constexpr int F16_RAW_WARP = F16_COPY_WARP + 1;
 constexpr int F16_THREADS = (F16_RAW_WARP + 1) * 32; // 608
-/* Packed weights of a stage on their way to the producers, 32 groups of 8 rows: Q4_K the 256 nibble bytes of a pair of
- * sub-blocks per group, plus the 128 header bytes (d, dmin, scales) of a super-block for its four stages; Q4_0 two whole
- * blocks per group. Q6_K rows are not 16-byte aligned: their producers load from global memory. */
-constexpr int F16_RAW = 2; // one per producer group: in an odd ring a group could take a phase of the other group for its own
-__host__ __device__ constexpr int f16_raw_bytes(int qt) { return qt == NNTR_Q4_K ? 32 * 256 : qt == NNTR_Q4_0 ? 32 * 288 : 0; }
-constexpr int F16_HDR_BYTES = 32 * 128;
-constexpr int F16_OFF_RAW = F16_STAGES * F16_STAGE_BYTES;
-__host__ __device__ constexpr int f16_off_hdr(int qt) { return F16_OFF_RAW + F16_RAW * f16_raw_bytes(qt); }
-__host__ __device__ constexpr int f16_off_bars(int qt) { return f16_off_hdr(qt) + (qt == NNTR_Q4_K ? 2 * F16_HDR_BYTES : 0); }
-__host__ __device__ constexpr int f16_smem(int qt) { return f16_off_bars(qt) + 256; }
-static_assert(f16_smem(NNTR_Q4_K) <= 227 * 1024 && f16_smem(NNTR_Q4_0) <= 227 * 1024, "shared memory of a CTA");
+/* How a tile of C is dealt out: a CTA of its own, a cluster whose CTAs share it along K, a pair of CTAs with one MMA over both. */
+enum F16Mode { F16_LONE, F16_SHARED, F16_PAIR };
+template <int QT, int MODE> struct F16Cfg {
+  static constexpr int W_ROWS = MODE == F16_PAIR ? F16_TILE_N / 2 : F16_TILE_N; // weight rows that a CTA expands
+  static constexpr int W_BYTES = W_ROWS * F16_KS * 2;
+  static constexpr int STAGE_BYTES = W_BYTES + 2 * F16_A_BYTES; // weights + two activation tiles
+  static constexpr int STAGES = MODE == F16_PAIR ? 4 : 3;
+  /* Groups of producers, each with the next stage in turn. Q4_K, Q4_0: a thread per weight row; Q6_K: two, and two stages in turn */
+  static constexpr int GROUPS = F16_PRODUCERS / (QT == NNTR_Q6_K ? 2 * W_ROWS : W_ROWS);
+  static constexpr int STAGE_WARPS = F16_PRODUCERS / 32 / GROUPS;
+  /* Packed weights of a stage on their way to the producers, groups of 8 rows: Q4_K the 256 nibble bytes of a pair of
+   * sub-blocks per group, plus the 128 header bytes (d, dmin, scales) of a super-block for its four stages; Q4_0 two whole
+   * blocks per group. Q6_K rows are not 16-byte aligned: their producers load from global memory. */
+  static constexpr int RAW = W_ROWS == F16_TILE_N ? 2 : 4; // one per producer group: with another number a group could take a phase of another group for its own
+  static constexpr int ROW_GROUPS = W_ROWS / 8;
+  static constexpr int RAW_BOX = QT == NNTR_Q4_K ? 128 : 144;
+  static constexpr int RAW_BYTES = QT == NNTR_Q6_K ? 0 : ROW_GROUPS * 2 * RAW_BOX;
+  static constexpr int HDR_BYTES = ROW_GROUPS * 128;
+  static constexpr int OFF_RAW = STAGES * STAGE_BYTES;
+  static constexpr int OFF_HDR = OFF_RAW + RAW * RAW_BYTES;
+  static constexpr int OFF_BARS = OFF_HDR + (QT == NNTR_Q4_K ? 2 * HDR_BYTES : 0);
+  static constexpr int SMEM = OFF_BARS + 256;
+  static_assert(SMEM <= 227 * 1024, "shared memory of a CTA");
+  static_assert(QT == NNTR_Q6_K || RAW == GROUPS, "ring of packed weights");
+};
 constexpr uint32_t F16_POLLS = 1u << 22;
 
 __device__ int g_f16_status = 0;
@@ -103,14 +115,50 @@ __device__ __forceinline__ uint64_t umma_desc(uint32_t saddr, uint32_t lbo, uint
   return (uint64_t)((saddr >> 4) & 0x3fff) | ((uint64_t)((lbo >> 4) & 0x3fff) << 16) |
          ((uint64_t)((sbo >> 4) & 0x3fff) << 32) | ((uint64_t)1 << 46);
 }
+/* PAIR: one MMA over two CTAs of a cluster, issued by the first; the descriptors hold for the shared memory of both */
+template <bool PAIR>
 __device__ __forceinline__ void umma_f16(uint32_t tmem_d, uint64_t da, uint64_t db, uint32_t idesc, uint32_t accumulate) {
-  asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.u32 p, %4, 0;\n\t"
-               "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}" ::"r"(tmem_d),
-               "l"(da), "l"(db), "r"(idesc), "r"(accumulate)
-               : "memory");
+  if constexpr (PAIR)
+    asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.u32 p, %4, 0;\n\t"
+                 "tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n\t}" ::"r"(tmem_d),
+                 "l"(da), "l"(db), "r"(idesc), "r"(accumulate)
+                 : "memory");
+  else
+    asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.u32 p, %4, 0;\n\t"
+                 "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}" ::"r"(tmem_d),
+                 "l"(da), "l"(db), "r"(idesc), "r"(accumulate)
+                 : "memory");
 }
-__device__ __forceinline__ void umma_commit(uint32_t bar) {
-  asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar) : "memory");
+/* the barrier at this address, PAIR: in both CTAs, when the MMAs issued so far have retired */
+template <bool PAIR> __device__ __forceinline__ void umma_commit(uint32_t bar) {
+  if constexpr (PAIR)
+    asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;" ::"r"(bar),
+                 "h"((uint16_t)3)
+                 : "memory");
+  else
+    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar) : "memory");
+}
+template <bool PAIR> __device__ __forceinline__ void tmem_alloc_all(uint32_t slot) {
+  if constexpr (PAIR) {
+    asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(slot), "r"(512u) : "memory");
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;");
+  } else {
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(slot), "r"(512u) : "memory");
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
+  }
+}
+template <bool PAIR> __device__ __forceinline__ void tmem_free_all(uint32_t tmem) {
+  if constexpr (PAIR)
+    asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(512u));
+  else
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(512u));
+}
+/** Arrival at the barrier at this address in another CTA of the cluster. No release at cluster scope: what the MMAs of the other CTA's
+ *  thread read here was written by this CTA's warps and copies, behind their proxy fences and this CTA's barrier, and is read by this SM. */
+__device__ __forceinline__ void mbar_arrive_remote(uint32_t bar, uint32_t rank) {
+  uint32_t remote;
+  asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(remote) : "r"(bar), "r"(rank));
+  asm volatile("mbarrier.arrive.shared::cluster.b64 _, [%0];" ::"r"(remote) : "memory");
 }
 __device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t (&r)[16]) {
   asm volatile("tcgen05.ld.sync.aligned.32x32b.x16.b32 "
@@ -153,54 +201,62 @@ __device__ __forceinline__ uint32_t expand2_q40(uint32_t nib2, __half2 d) {
  * QT = NNTR_Q6_K: W is plain rows of block_q6_K (210 bytes, 2-byte aligned); stage (b, h, s2) of super-block b holds
  *                 the quarters s2 and s2 + 2 of its 128-element half h (the two quarters that share the bytes ql[64h +
  *                 32 s2 ..] as low and high nibbles); k_stages = 4 * K/256. N may end inside the last 256-row tile.
- * SHARED: a cluster of CTAs may share the tile. A kernel of its own: the code of a shared tile in the kernel of a lone CTA costs
+ * F16_PAIR: the cluster's two CTAs expand 128 of the 256 weight rows each and hold two of four activation tiles; an MMA takes
+ * 128 activation rows of each and the weights of both, so a stage's expansion serves 512 rows instead of 256, and a CTA's MMAs read half
+ * of the weights from its own shared memory only.
+ * F16_SHARED: a cluster of CTAs may share the tile. A kernel of its own: the code of a shared tile in the kernel of a lone CTA costs
  * that one registers (80 without, 96 with) and 1024 x 24576 x 4096 Q4_K 185 us instead of 182. (It keeps the test for a cluster of
  * one, without which the compiler spills 44 bytes instead of 8.) */
-template <int QT, bool SHARED>
+template <int QT, int MODE>
 __global__ void __launch_bounds__(F16_THREADS, 1)
 gemm_f16_kernel(const __grid_constant__ CUtensorMap wmap, const uint8_t *__restrict__ atiles, const uint8_t *__restrict__ Wb,
                 float *__restrict__ C, int ldc, int M, int N, int k_stages, int m_tiles, int tiles_per_cta,
                 int c_vec4) {
   extern __shared__ __align__(128) uint8_t smem[];
-  // bars: [0..3] full, [4..7] empty, [8] tile complete, [9..10] packed weights here, [12..13] packed weights read,
-  // [14..15] Q4_K headers here
+  using Cfg = F16Cfg<QT, MODE>;
+  constexpr bool SHARED = MODE == F16_SHARED, PAIR = MODE == F16_PAIR;
+  // bars: [0..3] full, [4..7] empty, [8] tile complete, [9..12] packed weights here, [13..16] packed weights read,
+  // [17..18] Q4_K headers here
   const uint32_t sbase = smem_u32(smem);
-  const uint32_t bar0 = sbase + f16_off_bars(QT);
+  const uint32_t bar0 = sbase + Cfg::OFF_BARS;
   auto BAR = [&](int i) { return bar0 + 8u * i; };
-  uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(smem + f16_off_bars(QT) + 128);
-  volatile int *abort_flag = reinterpret_cast<volatile int *>(smem + f16_off_bars(QT) + 136);
+  uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(smem + Cfg::OFF_BARS + 192);
+  volatile int *abort_flag = reinterpret_cast<volatile int *>(smem + Cfg::OFF_BARS + 200);
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   // a CTA takes two 128-row activation tiles (unless there are SMs to spare) against the same 256 weight rows: the expanded
   // weights of a stage feed two MMAs, which halves the expansion work per output
   // the CTAs of a cluster share a tile: each walks its part of K, whole super-blocks (Q6_K: halves; Q4_0: pairs of blocks)
   const int parts = SHARED ? cluster_size() : 1, part = SHARED ? cluster_rank() : 0;
-  const int mt = tiles_per_cta * (blockIdx.x / parts), nt = blockIdx.y;
-  const bool two = tiles_per_cta == 2 && mt + 1 < m_tiles;
+  // a pair takes four activation tiles, its CTAs alternate ones
+  const int peer = PAIR ? cluster_rank() : 0, mt_step = PAIR ? 2 : 1; // place in the pair
+  const int mt = PAIR ? 4 * (blockIdx.x / 2) + peer : tiles_per_cta * (blockIdx.x / parts), nt = blockIdx.y;
+  const bool two = PAIR ? mt - peer + 2 < m_tiles : tiles_per_cta == 2 && mt + 1 < m_tiles; // the same in both CTAs of a pair
   constexpr int UNIT = QT == NNTR_Q4_K ? 4 : QT == NNTR_Q6_K ? 2 : 1;
   const int units = k_stages / UNIT;
   const int st0 = units * part / parts * UNIT, n_stages = units * (part + 1) / parts * UNIT - st0; // stages st0 ..
 
   if (tid == 0) {
-    for (int s = 0; s < F16_STAGES; ++s) {
-      mbar_init(BAR(s), f16_stage_warps(QT) + 1); // the stage's producer warps + the thread that armed the activation copy
-      mbar_init(BAR(4 + s), 1);                   // MMAs of the stage retired
+    for (int s = 0; s < Cfg::STAGES; ++s) {
+      // the stage's producer warps + the thread that armed the activation copy + in the pair's first CTA the other one
+      mbar_init(BAR(s), Cfg::STAGE_WARPS + 1 + (PAIR && peer == 0));
+      mbar_init(BAR(4 + s), 1); // MMAs of the stage retired
     }
-    for (int s = 0; s < F16_RAW; ++s) {
+    for (int s = 0; s < Cfg::RAW; ++s) {
       mbar_init(BAR(9 + s), 1);
-      mbar_init(BAR(12 + s), f16_stage_warps(QT));
-      mbar_init(BAR(14 + s), 1);
+      mbar_init(BAR(13 + s), Cfg::STAGE_WARPS);
     }
+    mbar_init(BAR(17), 1);
+    mbar_init(BAR(18), 1);
     mbar_init(BAR(8), 1);
     *abort_flag = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
-  if (warp == F16_MMA_WARP) {
-    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)),
-                 "r"(512u));
-    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
-  }
+  if (warp == F16_MMA_WARP)
+    tmem_alloc_all<PAIR>(smem_u32(tmem_slot));
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
+  if (PAIR)
+    cluster_sync(); // the other CTA's barriers and tensor memory are there
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
   const uint32_t tmem = *tmem_slot;
 
@@ -245,37 +301,37 @@ gemm_f16_kernel(const __grid_constant__ CUtensorMap wmap, const uint8_t *__restr
 
   if (warp < F16_MMA_WARP) {
     /* ------------------------------ producers ------------------------------ */
-    const int r = tid & (F16_TILE_N - 1); // weight row inside the tile
-    const int hsel = tid >> 8;            // Q4_K, Q4_0: stages of this parity; Q6_K: which half of the stage's 32 nibble bytes
+    const int r = tid % Cfg::W_ROWS;    // weight row inside the CTA's part of the tile
+    const int hsel = tid / Cfg::W_ROWS; // Q4_K, Q4_0: the thread's group; Q6_K, modulo 2: which half of the stage's 32 nibble bytes
     const int j = r & 7;                  // row inside its 8-row group
     bool ok = true;
     auto slot_wait = [&](int st) { // the MMAs that read the slot have retired
-      const int use = st / F16_STAGES;
-      const bool go = use == 0 || mbar_wait(BAR(4 + st % F16_STAGES), (use - 1) & 1, abort_flag);
+      const int use = st / Cfg::STAGES;
+      const bool go = use == 0 || mbar_wait(BAR(4 + st % Cfg::STAGES), (use - 1) & 1, abort_flag);
       return __all_sync(0xffffffffu, go) != 0; // the warp leaves together: its lanes meet at the arrives below
     };
     auto raw_wait = [&](int st) { // the stage's packed weights are here (Q4_K: half the lanes ask for the super-block's header)
       const bool head = QT == NNTR_Q4_K && lane >= 16;
-      return __all_sync(0xffffffffu, mbar_wait(head ? BAR(14 + ((st >> 2) & 1)) : BAR(9 + st % F16_RAW),
-                                               (head ? st >> 3 : st / F16_RAW) & 1, abort_flag)) != 0;
+      return __all_sync(0xffffffffu, mbar_wait(head ? BAR(17 + ((st >> 2) & 1)) : BAR(9 + st % Cfg::RAW),
+                                               (head ? st >> 3 : st / Cfg::RAW) & 1, abort_flag)) != 0;
     };
     auto stage_done = [&](int st) {
       asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
       __syncwarp(); // every lane's writes are fenced; one arrival per warp keeps the barrier word off the critical path
       if (lane == 0)
-        mbar_arrive(BAR(st % F16_STAGES));
+        mbar_arrive(BAR(st % Cfg::STAGES));
     };
     auto raw_done = [&](int st) { // the packed words are on their way to registers: the slot may be refilled when they are there
       loads_before_refill();
       __syncwarp();
       if (lane == 0)
-        mbar_arrive(BAR(12 + st % F16_RAW));
+        mbar_arrive(BAR(13 + st % Cfg::RAW));
     };
     if constexpr (QT == NNTR_Q4_K) {
       // neighbouring groups read pairs of nibble chunks in opposite order: 128 bytes apart, they would meet in the same banks
       const int grp = r >> 3, sw = grp & 1;
-      const uint8_t *nq = smem + F16_OFF_RAW + grp * 128 + 8 * j;
-      const uint8_t *hdr = smem + f16_off_hdr(QT) + grp * 128;
+      const uint8_t *nq = smem + Cfg::OFF_RAW + grp * 128 + 8 * j;
+      const uint8_t *hdr = smem + Cfg::OFF_HDR + grp * 128;
       // the next stage's words go to registers as soon as this one's are expanded, so that its ring slot refills meanwhile
       uint2 w[4], g0, g1, g2;
       float dw, dmw;
@@ -284,8 +340,8 @@ gemm_f16_kernel(const __grid_constant__ CUtensorMap wmap, const uint8_t *__restr
           return false;
 #pragma unroll
         for (int c = 0; c < 4; ++c)
-          w[c] = *reinterpret_cast<const uint2 *>(nq + (st % F16_RAW) * f16_raw_bytes(QT) + (c >> 1) * (32 * 128) + 64 * ((c & 1) ^ sw));
-        const uint8_t *h = hdr + ((st >> 2) & 1) * F16_HDR_BYTES;
+          w[c] = *reinterpret_cast<const uint2 *>(nq + (st % Cfg::RAW) * Cfg::RAW_BYTES + (c >> 1) * (Cfg::ROW_GROUPS * 128) + 64 * ((c & 1) ^ sw));
+        const uint8_t *h = hdr + ((st >> 2) & 1) * Cfg::HDR_BYTES;
         g0 = *reinterpret_cast<const uint2 *>(h + 32 + 24 * (st & 3));
         g1 = *reinterpret_cast<const uint2 *>(h + 40 + 24 * (st & 3));
         g2 = *reinterpret_cast<const uint2 *>(h + 48 + 24 * (st & 3));
@@ -295,7 +351,7 @@ gemm_f16_kernel(const __grid_constant__ CUtensorMap wmap, const uint8_t *__restr
         return true;
       };
       ok = hsel >= n_stages || fetch(hsel);
-      for (int st = hsel; st < n_stages && ok; st += 2) {
+      for (int st = hsel; st < n_stages && ok; st += Cfg::GROUPS) {
         float sc0, mn0, sc1, mn1;
         scale_min_row(g0.x, g0.y, g1.x, j, sc0, mn0);
         scale_min_row(g1.y, g2.x, g2.y, j, sc1, mn1);
@@ -303,24 +359,24 @@ gemm_f16_kernel(const __grid_constant__ CUtensorMap wmap, const uint8_t *__restr
         const __half2 m_lo = __float2half2_rn(-(dmw * mn0)), m_hi = __float2half2_rn(-(dmw * mn1));
         if (!(ok = slot_wait(st)))
           break;
-        uint8_t *wdst = smem + (st % F16_STAGES) * F16_STAGE_BYTES + r * 16;
+        uint8_t *wdst = smem + (st % Cfg::STAGES) * Cfg::STAGE_BYTES + r * 16;
 #pragma unroll
         for (int c = 0; c < 4; ++c) {
           // word -> 8 halves in the order [lo b0, lo b2, lo b1, lo b3, hi b0, hi b2, hi b1, hi b3]
           const uint32_t wx = w[c].x, wy = w[c].y;
-          uint8_t *d = wdst + (2 * (c ^ sw)) * (F16_TILE_N * 16);
+          uint8_t *d = wdst + (2 * (c ^ sw)) * (Cfg::W_ROWS * 16);
           *reinterpret_cast<uint4 *>(d) =
             make_uint4(expand2(wx & 0x000f000fu, d_lo, m_lo), expand2((wx >> 8) & 0x000f000fu, d_lo, m_lo),
                        expand2((wx >> 4) & 0x000f000fu, d_hi, m_hi), expand2((wx >> 12) & 0x000f000fu, d_hi, m_hi));
-          *reinterpret_cast<uint4 *>(d + F16_TILE_N * 16) =
+          *reinterpret_cast<uint4 *>(d + Cfg::W_ROWS * 16) =
             make_uint4(expand2(wy & 0x000f000fu, d_lo, m_lo), expand2((wy >> 8) & 0x000f000fu, d_lo, m_lo),
                        expand2((wy >> 4) & 0x000f000fu, d_hi, m_hi), expand2((wy >> 12) & 0x000f000fu, d_hi, m_hi));
         }
         stage_done(st);
-        ok = st + 2 >= n_stages || fetch(st + 2);
+        ok = st + Cfg::GROUPS >= n_stages || fetch(st + Cfg::GROUPS);
       }
     } else if constexpr (QT == NNTR_Q6_K) {
-      const int n_row = nt * F16_TILE_N + r;
+      const int n_row = nt * F16_TILE_N + peer * Cfg::W_ROWS + r, qhalf = hsel & 1;
       const bool have_row = n_row < N; // rows beyond N: scale 0, so zero weights (their columns are not stored either)
       const int nb = k_stages / 4, n_groups = n_stages / 2, g0 = st0 / 2;
       const uint8_t *wrow = Wb + (size_t)(have_row ? n_row : 0) * nb * sizeof(BlockQ6K);
@@ -332,21 +388,22 @@ gemm_f16_kernel(const __grid_constant__ CUtensorMap wmap, const uint8_t *__restr
         const int b = (g0 + g) >> 1, h = (g0 + g) & 1;
         const uint8_t *blk = wrow + (size_t)b * sizeof(BlockQ6K);
         const uint32_t *al =
-          reinterpret_cast<const uint32_t *>(reinterpret_cast<uintptr_t>(blk + 64 * h + 16 * hsel) & ~(uintptr_t)3);
+          reinterpret_cast<const uint32_t *>(reinterpret_cast<uintptr_t>(blk + 64 * h + 16 * qhalf) & ~(uintptr_t)3);
         const uint32_t *ah =
-          reinterpret_cast<const uint32_t *>(reinterpret_cast<uintptr_t>(blk + 128 + 32 * h + 16 * hsel) & ~(uintptr_t)3);
+          reinterpret_cast<const uint32_t *>(reinterpret_cast<uintptr_t>(blk + 128 + 32 * h + 16 * qhalf) & ~(uintptr_t)3);
 #pragma unroll
         for (int k = 0; k < 5; ++k) {
           rl[0][k] = __ldg(al + k);
           rl[1][k] = __ldg(al + 8 + k);
           rh[k] = __ldg(ah + k);
         }
-        const uint8_t *sc = blk + 192 + 8 * h + hsel; // scale of quarter w: sc[2 w]
+        const uint8_t *sc = blk + 192 + 8 * h + qhalf; // scale of quarter w: sc[2 w]
         rs = (uint32_t)__ldg(sc) | ((uint32_t)__ldg(sc + 2) << 8) | ((uint32_t)__ldg(sc + 4) << 16) | ((uint32_t)__ldg(sc + 6) << 24);
         rd = __ldg(reinterpret_cast<const uint16_t *>(blk + 208));
       };
-      fetch(0);
-      for (int g = 0; g < n_groups && ok; ++g) {
+      const int first = hsel / 2;
+      fetch(first < n_groups ? first : 0);
+      for (int g = first; g < n_groups && ok; g += Cfg::GROUPS) {
         const uint32_t sh = (uint32_t)((reinterpret_cast<uintptr_t>(wrow) + (size_t)((g0 + g) >> 1) * sizeof(BlockQ6K)) & 2) * 8;
         uint32_t ql[2][4], qh[4];
 #pragma unroll
@@ -357,10 +414,10 @@ gemm_f16_kernel(const __grid_constant__ CUtensorMap wmap, const uint8_t *__restr
         }
         const float d = have_row ? half_bits_to_float((uint16_t)rd) : 0.f;
         const uint32_t scs = rs;
-        fetch(g + 1 < n_groups ? g + 1 : g); // the next group travels while this one is expanded
+        fetch(g + Cfg::GROUPS < n_groups ? g + Cfg::GROUPS : g); // the next group travels while this one is expanded
 #pragma unroll
         for (int s2 = 0; s2 < 2; ++s2) {
-          const int st = 2 * g + s2, s = st % F16_STAGES, use = st / F16_STAGES;
+          const int st = 2 * g + s2, s = st % Cfg::STAGES, use = st / Cfg::STAGES;
           const __half2 d_lo = __float2half2_rn(d * (float)(int)(int8_t)(scs >> (8 * s2)));
           const __half2 d_hi = __float2half2_rn(d * (float)(int)(int8_t)(scs >> (8 * s2 + 16)));
           if (use > 0 && !mbar_wait(BAR(4 + s), (use - 1) & 1, abort_flag))
@@ -368,7 +425,7 @@ gemm_f16_kernel(const __grid_constant__ CUtensorMap wmap, const uint8_t *__restr
           ok = __all_sync(0xffffffffu, ok); // the warp leaves together: its lanes meet at the arrive below
           if (!ok)
             break;
-          uint8_t *wdst = smem + s * F16_STAGE_BYTES + r * 16 + (4 * hsel) * (F16_TILE_N * 16);
+          uint8_t *wdst = smem + s * Cfg::STAGE_BYTES + r * 16 + (4 * qhalf) * (Cfg::W_ROWS * 16);
           const __half2 off = __half2half2(__ushort_as_half(0x6420)); // 1024 + 32
 #pragma unroll
           for (int i = 0; i < 4; ++i) {
@@ -383,7 +440,7 @@ gemm_f16_kernel(const __grid_constant__ CUtensorMap wmap, const uint8_t *__restr
             const __half2 w1 = __hmul2(__hsub2(*reinterpret_cast<const __half2 *>(&t1), off), d_lo);
             const __half2 w2 = __hmul2(__hsub2(*reinterpret_cast<const __half2 *>(&t2), off), d_hi);
             const __half2 w3 = __hmul2(__hsub2(*reinterpret_cast<const __half2 *>(&t3), off), d_hi);
-            *reinterpret_cast<uint4 *>(wdst + i * (F16_TILE_N * 16)) =
+            *reinterpret_cast<uint4 *>(wdst + i * (Cfg::W_ROWS * 16)) =
               make_uint4(*reinterpret_cast<const uint32_t *>(&w0), *reinterpret_cast<const uint32_t *>(&w1),
                          *reinterpret_cast<const uint32_t *>(&w2), *reinterpret_cast<const uint32_t *>(&w3));
           }
@@ -395,27 +452,27 @@ gemm_f16_kernel(const __grid_constant__ CUtensorMap wmap, const uint8_t *__restr
       }
     } else {
       // the two blocks of a stage: 16 nibble bytes each = four words = four 16-byte chunks of halves
-      const uint8_t *blk0 = smem + F16_OFF_RAW + (r >> 3) * 144;
+      const uint8_t *blk0 = smem + Cfg::OFF_RAW + (r >> 3) * 144;
       uint2 q[4];
       uint16_t dbits[2];
       auto fetch = [&](int st) {
         if (!raw_wait(st))
           return false;
-        const uint8_t *blk = blk0 + (st % F16_RAW) * f16_raw_bytes(QT);
+        const uint8_t *blk = blk0 + (st % Cfg::RAW) * Cfg::RAW_BYTES;
 #pragma unroll
         for (int k = 0; k < 2; ++k) {
-          q[2 * k] = *reinterpret_cast<const uint2 *>(blk + k * (32 * 144) + 16 + 8 * j);
-          q[2 * k + 1] = *reinterpret_cast<const uint2 *>(blk + k * (32 * 144) + 80 + 8 * j);
-          dbits[k] = *reinterpret_cast<const uint16_t *>(blk + k * (32 * 144) + 2 * j);
+          q[2 * k] = *reinterpret_cast<const uint2 *>(blk + k * (Cfg::ROW_GROUPS * 144) + 16 + 8 * j);
+          q[2 * k + 1] = *reinterpret_cast<const uint2 *>(blk + k * (Cfg::ROW_GROUPS * 144) + 80 + 8 * j);
+          dbits[k] = *reinterpret_cast<const uint16_t *>(blk + k * (Cfg::ROW_GROUPS * 144) + 2 * j);
         }
         raw_done(st);
         return true;
       };
       ok = hsel >= n_stages || fetch(hsel); // n_stages may be odd (K = 2880)
-      for (int st = hsel; st < n_stages && ok; st += 2) {
+      for (int st = hsel; st < n_stages && ok; st += Cfg::GROUPS) {
         if (!(ok = slot_wait(st)))
           break;
-        uint8_t *wdst = smem + (st % F16_STAGES) * F16_STAGE_BYTES + r * 16;
+        uint8_t *wdst = smem + (st % Cfg::STAGES) * Cfg::STAGE_BYTES + r * 16;
 #pragma unroll
         for (int k = 0; k < 2; ++k) {
           const __half2 d2 = __half2half2(__ushort_as_half(dbits[k]));
@@ -423,12 +480,12 @@ gemm_f16_kernel(const __grid_constant__ CUtensorMap wmap, const uint8_t *__restr
                                  q[2 * k + 1].y ^ 0x88888888u};
 #pragma unroll
           for (int wi = 0; wi < 4; ++wi) // chunk wi: elements 4wi + {0,2,1,3} then 16 + 4wi + {0,2,1,3} of the block
-            *reinterpret_cast<uint4 *>(wdst + (4 * k + wi) * (F16_TILE_N * 16)) =
+            *reinterpret_cast<uint4 *>(wdst + (4 * k + wi) * (Cfg::W_ROWS * 16)) =
               make_uint4(expand2_q40(w[wi] & 0x000f000fu, d2), expand2_q40((w[wi] >> 8) & 0x000f000fu, d2),
                          expand2_q40((w[wi] >> 4) & 0x000f000fu, d2), expand2_q40((w[wi] >> 12) & 0x000f000fu, d2));
         }
         stage_done(st);
-        ok = st + 2 >= n_stages || fetch(st + 2);
+        ok = st + Cfg::GROUPS >= n_stages || fetch(st + Cfg::GROUPS);
       }
     }
     /* ------------------------------ epilogue ------------------------------- */
@@ -439,7 +496,7 @@ gemm_f16_kernel(const __grid_constant__ CUtensorMap wmap, const uint8_t *__restr
         const float *turn = reinterpret_cast<const float *>(smem) + turn_area(warp);
         const int cc = nt * F16_TILE_N + (warp >> 2) * 64 + 4 * (lane & 15);
         for (int hm = 0; hm < (two ? 2 : 1); ++hm) {
-          const int row0 = (mt + hm) * F16_TILE_M + (warp & 3) * 32;
+          const int row0 = (mt + mt_step * hm) * F16_TILE_M + (warp & 3) * 32;
           turn_round(hm);
           __syncwarp();
 #pragma unroll 4
@@ -459,16 +516,19 @@ gemm_f16_kernel(const __grid_constant__ CUtensorMap wmap, const uint8_t *__restr
     // its MMAs have retired, whatever the producers are doing.
     if (lane == 0) {
       const uint8_t *asrc = atiles + ((size_t)mt * k_stages + st0) * F16_A_BYTES;
+      // a pair's last tiles may lack partners: what the MMA makes of the memory there is not stored
+      const bool have0 = mt < m_tiles, have1 = two && mt + mt_step < m_tiles;
       pdl_wait(); // the quantizer's tiles; the weights do not depend on the kernel before
       for (int st = 0; st < n_stages; ++st) {
-        const int s = st % F16_STAGES, use = st / F16_STAGES;
+        const int s = st % Cfg::STAGES, use = st / Cfg::STAGES;
         if (use > 0 && !mbar_wait(BAR(4 + s), (use - 1) & 1, abort_flag))
           break;
-        mbar_expect_tx(BAR(s), (two ? 2 : 1) * F16_A_BYTES);
-        bulk_g2s(sbase + s * F16_STAGE_BYTES + F16_W_BYTES, asrc + (size_t)st * F16_A_BYTES, F16_A_BYTES, BAR(s));
-        if (two)
-          bulk_g2s(sbase + s * F16_STAGE_BYTES + F16_W_BYTES + F16_A_BYTES, asrc + ((size_t)k_stages + st) * F16_A_BYTES,
-                   F16_A_BYTES, BAR(s));
+        mbar_expect_tx(BAR(s), (have0 + have1) * F16_A_BYTES);
+        const uint32_t dst = sbase + s * Cfg::STAGE_BYTES + Cfg::W_BYTES;
+        if (have0)
+          bulk_g2s(dst, asrc + (size_t)st * F16_A_BYTES, F16_A_BYTES, BAR(s));
+        if (have1)
+          bulk_g2s(dst + F16_A_BYTES, asrc + ((size_t)mt_step * k_stages + st) * F16_A_BYTES, F16_A_BYTES, BAR(s));
       }
     }
     __syncwarp();
@@ -478,55 +538,62 @@ gemm_f16_kernel(const __grid_constant__ CUtensorMap wmap, const uint8_t *__restr
     // copies, a box of 32 row groups x 128 (Q4_0: 144) bytes each: 32 untiled copies of 256 bytes per stage measured 1.6 times
     // slower than no ring at all.
     if (QT != NNTR_Q6_K && lane == 0) {
-      constexpr int BOX = QT == NNTR_Q4_K ? 128 : 144;
+      const int y = (nt * F16_TILE_N + peer * Cfg::W_ROWS) / 8;
       for (int st = 0; st < n_stages; ++st) {
-        const int rs = st % F16_RAW, use = st / F16_RAW;
-        if (use > 0 && !mbar_wait(BAR(12 + rs), (use - 1) & 1, abort_flag))
+        const int rs = st % Cfg::RAW, use = st / Cfg::RAW;
+        if (use > 0 && !mbar_wait(BAR(13 + rs), (use - 1) & 1, abort_flag))
           break;
-        mbar_expect_tx(BAR(9 + rs), f16_raw_bytes(QT));
-        const uint32_t dst = sbase + F16_OFF_RAW + rs * f16_raw_bytes(QT);
+        mbar_expect_tx(BAR(9 + rs), Cfg::RAW_BYTES);
+        const uint32_t dst = sbase + Cfg::OFF_RAW + rs * Cfg::RAW_BYTES;
         int x = (st0 + st) * 2 * (int)sizeof(BlockQ40x8);
         if (QT == NNTR_Q4_K) {
           x = ((st0 + st) >> 2) * (int)sizeof(BlockQ4Kx8);
-          if ((st & 3) == 0) { // two headers: the one replaced was last read three stages before the ones waited for so far
+          if ((st & 3) == 0) { // two headers: the stages up to st - RAW have been read, the one replaced served those up to st - 5
             const int hb = (st >> 2) & 1;
-            mbar_expect_tx(BAR(14 + hb), F16_HDR_BYTES);
-            tma_tile(sbase + f16_off_hdr(QT) + hb * F16_HDR_BYTES, &wmap, x, nt * (F16_TILE_N / 8), BAR(14 + hb));
+            mbar_expect_tx(BAR(17 + hb), Cfg::HDR_BYTES);
+            tma_tile(sbase + Cfg::OFF_HDR + hb * Cfg::HDR_BYTES, &wmap, x, y, BAR(17 + hb));
           }
           x += 128 + 256 * (st & 3);
         }
-        tma_tile(dst, &wmap, x, nt * (F16_TILE_N / 8), BAR(9 + rs));
-        tma_tile(dst + 32 * BOX, &wmap, x + BOX, nt * (F16_TILE_N / 8), BAR(9 + rs));
+        tma_tile(dst, &wmap, x, y, BAR(9 + rs));
+        tma_tile(dst + Cfg::ROW_GROUPS * Cfg::RAW_BOX, &wmap, x + Cfg::RAW_BOX, y, BAR(9 + rs));
       }
     }
     __syncwarp();
   } else {
     /* ------------------------------ MMA issue ------------------------------ */
-    if (lane == 0) {
-      // D = F32; A = activations (F16, 128 rows = lanes); B = weights (F16, 256 rows = columns); both K-major
+    if (lane == 0 && peer) { // the first CTA issues the MMAs: it is told what is ready here
+      for (int st = 0; st < n_stages; ++st) {
+        const int s = st % Cfg::STAGES;
+        if (!mbar_wait(BAR(s), (st / Cfg::STAGES) & 1, abort_flag))
+          break;
+        mbar_arrive_remote(BAR(s), 0);
+      }
+    } else if (lane == 0) {
+      // D = F32; A = activations (F16, 128 rows = lanes, PAIR: of each CTA); B = weights (F16, 256 rows = columns); both K-major
       const uint32_t idesc = (1u << 4) | (0u << 7) | (0u << 10) | ((uint32_t)(F16_TILE_N >> 3) << 17) |
-                             ((uint32_t)(F16_TILE_M >> 4) << 24);
+                             ((uint32_t)((PAIR ? 2 : 1) * F16_TILE_M >> 4) << 24);
       bool ok = true;
       for (int st = 0; st < n_stages && ok; ++st) {
-        const int s = st % F16_STAGES, use = st / F16_STAGES;
+        const int s = st % Cfg::STAGES, use = st / Cfg::STAGES;
         if (!mbar_wait(BAR(s), use & 1, abort_flag)) {
           ok = false;
           break;
         }
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-        const uint32_t ws = sbase + s * F16_STAGE_BYTES, as = ws + F16_W_BYTES;
+        const uint32_t ws = sbase + s * Cfg::STAGE_BYTES, as = ws + Cfg::W_BYTES;
 #pragma unroll
         for (int ks = 0; ks < 4; ++ks) { // K = 16 per instruction: two 16-byte core-matrix columns
-          const uint64_t db = umma_desc(ws + ks * 2 * (F16_TILE_N * 16), F16_TILE_N * 16, 128);
-          umma_f16(tmem, umma_desc(as + ks * 2 * (F16_TILE_M * 16), F16_TILE_M * 16, 128), db, idesc, (st | ks) != 0);
+          const uint64_t db = umma_desc(ws + ks * 2 * (Cfg::W_ROWS * 16), Cfg::W_ROWS * 16, 128);
+          umma_f16<PAIR>(tmem, umma_desc(as + ks * 2 * (F16_TILE_M * 16), F16_TILE_M * 16, 128), db, idesc, (st | ks) != 0);
           if (two)
-            umma_f16(tmem + 256, umma_desc(as + F16_A_BYTES + ks * 2 * (F16_TILE_M * 16), F16_TILE_M * 16, 128), db,
+            umma_f16<PAIR>(tmem + 256, umma_desc(as + F16_A_BYTES + ks * 2 * (F16_TILE_M * 16), F16_TILE_M * 16, 128), db,
                      idesc, (st | ks) != 0);
         }
-        umma_commit(BAR(4 + s));
+        umma_commit<PAIR>(BAR(4 + s));
       }
       if (ok)
-        umma_commit(BAR(8));
+        umma_commit<PAIR>(BAR(8));
     }
     __syncwarp();
   }
@@ -569,8 +636,10 @@ gemm_f16_kernel(const __grid_constant__ CUtensorMap wmap, const uint8_t *__restr
       __nanosleep(1000);
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
+  if (PAIR)
+    cluster_sync(); // neither CTA leaves, or frees the tensor memory, while the other needs it
   if (warp == F16_MMA_WARP)
-    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(512u));
+    tmem_free_all<PAIR>(tmem);
 }
 
 /* Activation tiles for the fp16 path: per (128 activation rows, 64 of K) 16 KB, core-matrix layout (8 halves = one
@@ -674,7 +743,7 @@ quantize_q8_0_f16_tiles_kernel(const float *__restrict__ x, int64_t ldx, uint8_t
 template <int QT> int k_parts(int tiles, int k_stages) {
   static ClusterFit fit;
   for (int parts = 8; parts > 1; parts /= 2)
-    if (k_stages >= 4 * parts && tiles <= fit(gemm_f16_kernel<QT, true>, parts, F16_THREADS, f16_smem(QT)))
+    if (k_stages >= 4 * parts && tiles <= fit(gemm_f16_kernel<QT, F16_SHARED>, parts, F16_THREADS, F16Cfg<QT, F16_SHARED>::SMEM))
       return parts;
   return 1;
 }
@@ -695,80 +764,95 @@ bool umma_f16_supported(int qtype, unsigned M, unsigned N, unsigned K) {
   return (qtype == NNTR_Q4_K && K % QK_K == 0) || (qtype == NNTR_Q4_0 && K % F16_KS == 0);
 }
 
-int launch_gemm_f16(int qtype, unsigned M, unsigned N, unsigned K, const float *A, const void *B, float *C, unsigned ldc,
-                    void *ws, cudaStream_t st) {
-  static bool attr_set[64] = {};
+namespace {
+
+template <int QT, int MODE>
+int launch_mode(dim3 grid, int cluster, cudaStream_t st, const CUtensorMap &wmap, const uint8_t *tiles, const uint8_t *W, float *C,
+                int ldc, int M, int N, int k_stages, int m_tiles, int tiles_per_cta, int c_vec4) {
+  NNTR_CHECK_CUDA(launch_in_clusters(gemm_f16_kernel<QT, MODE>, grid, cluster, F16_THREADS, F16Cfg<QT, MODE>::SMEM, st, wmap, tiles, W,
+                                     C, ldc, M, N, k_stages, m_tiles, tiles_per_cta, c_vec4));
+  return NNTR_CUDA_OK;
+}
+
+/** allows every form of the kernel its shared memory, once per device */
+template <int QT> int allow_smem() {
+  static std::atomic<uint64_t> done{0};
   int dev = 0;
   NNTR_CHECK_CUDA(cudaGetDevice(&dev));
-  if (dev < 64 && !attr_set[dev]) {
-    NNTR_CHECK_CUDA(cudaFuncSetAttribute(gemm_f16_kernel<NNTR_Q4_K, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, f16_smem(NNTR_Q4_K)));
-    NNTR_CHECK_CUDA(cudaFuncSetAttribute(gemm_f16_kernel<NNTR_Q4_K, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, f16_smem(NNTR_Q4_K)));
-    NNTR_CHECK_CUDA(cudaFuncSetAttribute(gemm_f16_kernel<NNTR_Q4_0, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, f16_smem(NNTR_Q4_0)));
-    NNTR_CHECK_CUDA(cudaFuncSetAttribute(gemm_f16_kernel<NNTR_Q4_0, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, f16_smem(NNTR_Q4_0)));
-    NNTR_CHECK_CUDA(cudaFuncSetAttribute(gemm_f16_kernel<NNTR_Q6_K, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, f16_smem(NNTR_Q6_K)));
-    NNTR_CHECK_CUDA(cudaFuncSetAttribute(gemm_f16_kernel<NNTR_Q6_K, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, f16_smem(NNTR_Q6_K)));
-    attr_set[dev] = true;
-  }
-  const int mtiles = (int)((M + F16_TILE_M - 1) / F16_TILE_M), Mpad = mtiles * F16_TILE_M;
-  if ((reinterpret_cast<uintptr_t>(A) & 15) || (reinterpret_cast<uintptr_t>(ws) & 15))
-    return set_error(NNTR_CUDA_ERR_INVALID, "gemm (fp16 tensor path): activations and workspace must be 16-byte aligned");
-  const int c_vec4 = (ldc % 4 == 0) && !(reinterpret_cast<uintptr_t>(C) & 15);
-  dim3 grid((mtiles + 1) / 2, (N + F16_TILE_N - 1) / F16_TILE_N);
-  const int n_stages = (int)(K / F16_KS);
-  const int pairs = (int)(grid.x * grid.y);
-  const int parts = qtype == NNTR_Q4_K   ? k_parts<NNTR_Q4_K>(pairs, n_stages)
-                    : qtype == NNTR_Q6_K ? k_parts<NNTR_Q6_K>(pairs, n_stages)
-                                         : k_parts<NNTR_Q4_0>(pairs, n_stages);
+  if (dev < 64 && (done.load(std::memory_order_acquire) >> dev & 1))
+    return NNTR_CUDA_OK;
+  NNTR_CHECK_CUDA(cudaFuncSetAttribute(gemm_f16_kernel<QT, F16_LONE>, cudaFuncAttributeMaxDynamicSharedMemorySize, F16Cfg<QT, F16_LONE>::SMEM));
+  NNTR_CHECK_CUDA(cudaFuncSetAttribute(gemm_f16_kernel<QT, F16_SHARED>, cudaFuncAttributeMaxDynamicSharedMemorySize, F16Cfg<QT, F16_SHARED>::SMEM));
+  NNTR_CHECK_CUDA(cudaFuncSetAttribute(gemm_f16_kernel<QT, F16_PAIR>, cudaFuncAttributeMaxDynamicSharedMemorySize, F16Cfg<QT, F16_PAIR>::SMEM));
+  if (dev < 64)
+    done.fetch_or(1ull << dev, std::memory_order_release);
+  return NNTR_CUDA_OK;
+}
+
+template <int QT>
+int launch_typed(unsigned M, unsigned N, unsigned K, const uint8_t *tiles, const void *B, float *C, unsigned ldc, cudaStream_t st) {
+  const int mtiles = (int)((M + F16_TILE_M - 1) / F16_TILE_M), n_tiles = (int)((N + F16_TILE_N - 1) / F16_TILE_N);
+  const int k_stages = (int)(K / F16_KS), c_vec4 = (ldc % 4 == 0) && !(reinterpret_cast<uintptr_t>(C) & 15);
+  int cta_m = (mtiles + 1) / 2, tiles_per_cta = 2;
+  if (const int rc = allow_smem<QT>())
+    return rc;
+  const int parts = k_parts<QT>(cta_m * n_tiles, k_stages);
+  const bool pair = parts == 1 && mtiles > 2;
   // tiles one by one if they run in the same wave as the pairs: 128 instead of 256 columns of MMAs per stage and one sum at the
   // end instead of two (256 x 1280 x 2560 Q4_0: 24 -> 16 us)
-  int tiles_per_cta = 2;
-  if (parts > 1 && mtiles > 1) {
-    const int tiles = mtiles * (int)grid.y;
-    if (parts == (qtype == NNTR_Q4_K   ? k_parts<NNTR_Q4_K>(tiles, n_stages)
-                  : qtype == NNTR_Q6_K ? k_parts<NNTR_Q6_K>(tiles, n_stages)
-                                       : k_parts<NNTR_Q4_0>(tiles, n_stages))) {
-      tiles_per_cta = 1;
-      grid.x = mtiles;
-    }
+  if (parts > 1 && mtiles > 1 && parts == k_parts<QT>(mtiles * n_tiles, k_stages)) {
+    tiles_per_cta = 1;
+    cta_m = mtiles;
   }
-  const uint8_t *tiles = static_cast<const uint8_t *>(ws), *W = static_cast<const uint8_t *>(B);
   CUtensorMap wmap = {};
-  if (qtype != NNTR_Q6_K) { // rows of 8-row groups of packed weights
-    const uint64_t row = qtype == NNTR_Q4_K ? (uint64_t)(K / QK_K) * sizeof(BlockQ4Kx8) : (uint64_t)(K / 32) * sizeof(BlockQ40x8);
-    if (reinterpret_cast<uintptr_t>(B) & 15)
-      return set_error(NNTR_CUDA_ERR_INVALID, "gemm (fp16 tensor path): weights must be 16-byte aligned");
-    const int rc = encode_map_2d(&wmap, B, 1, row, N / 8, row, qtype == NNTR_Q4_K ? 128 : 144, 32, false);
+  if (QT != NNTR_Q6_K) { // rows of 8-row groups of packed weights
+    const uint64_t row = QT == NNTR_Q4_K ? (uint64_t)(K / QK_K) * sizeof(BlockQ4Kx8) : (uint64_t)(K / 32) * sizeof(BlockQ40x8);
+    const int rc = encode_map_2d(&wmap, B, 1, row, N / 8, row, F16Cfg<QT, F16_LONE>::RAW_BOX,
+                                 pair ? F16Cfg<QT, F16_PAIR>::ROW_GROUPS : F16Cfg<QT, F16_LONE>::ROW_GROUPS, false);
     if (rc)
       return rc;
   }
+  const uint8_t *W = static_cast<const uint8_t *>(B);
+  if (pair)
+    return launch_mode<QT, F16_PAIR>(dim3((mtiles + 3) / 4, n_tiles), 2, st, wmap, tiles, W, C, (int)ldc, (int)M, (int)N, k_stages, mtiles,
+                                     2, c_vec4);
+  if (parts > 1)
+    return launch_mode<QT, F16_SHARED>(dim3(cta_m, n_tiles), parts, st, wmap, tiles, W, C, (int)ldc, (int)M, (int)N, k_stages, mtiles,
+                                       tiles_per_cta, c_vec4);
+  return launch_mode<QT, F16_LONE>(dim3(cta_m, n_tiles), 1, st, wmap, tiles, W, C, (int)ldc, (int)M, (int)N, k_stages, mtiles, 2, c_vec4);
+}
+
+} // namespace
+
+int launch_gemm_f16(int qtype, unsigned M, unsigned N, unsigned K, const float *A, const void *B, float *C, unsigned ldc,
+                    void *ws, cudaStream_t st) {
+  const int mtiles = (int)((M + F16_TILE_M - 1) / F16_TILE_M), Mpad = mtiles * F16_TILE_M;
+  if ((reinterpret_cast<uintptr_t>(A) & 15) || (reinterpret_cast<uintptr_t>(ws) & 15))
+    return set_error(NNTR_CUDA_ERR_INVALID, "gemm (fp16 tensor path): activations and workspace must be 16-byte aligned");
+  if (qtype != NNTR_Q6_K && (reinterpret_cast<uintptr_t>(B) & 15))
+    return set_error(NNTR_CUDA_ERR_INVALID, "gemm (fp16 tensor path): weights must be 16-byte aligned");
+  uint8_t *tiles = static_cast<uint8_t *>(ws);
+  int rc;
   if (qtype == NNTR_Q4_K || qtype == NNTR_Q6_K) {
     const int nb = (int)(K / QK_K);
     // Q4_K: rows below 4*floor(M/4) with the 4-row quantizer's sign rule; Q6_K: the row quantizer for every row
     // (ggml_interface_omp.cpp:545-551)
     const unsigned M4 = qtype == NNTR_Q4_K ? (M / 4) * 4 : 0;
     const int64_t nwarps = (int64_t)Mpad * nb;
-    quantize_q8_K_f16_tiles_kernel<<<(unsigned)((nwarps + 7) / 8), 256, 0, st>>>(A, K, static_cast<uint8_t *>(ws), (int)M,
-                                                                               (int)M4, Mpad, nb, qtype == NNTR_Q6_K);
+    quantize_q8_K_f16_tiles_kernel<<<(unsigned)((nwarps + 7) / 8), 256, 0, st>>>(A, K, tiles, (int)M, (int)M4, Mpad, nb,
+                                                                               qtype == NNTR_Q6_K);
     count_launch();
     NNTR_CHECK_CUDA(cudaGetLastError());
-    if (qtype == NNTR_Q4_K)
-      NNTR_CHECK_CUDA(launch_in_clusters(parts > 1 ? gemm_f16_kernel<NNTR_Q4_K, true> : gemm_f16_kernel<NNTR_Q4_K, false>, grid,
-                                         parts, F16_THREADS, f16_smem(NNTR_Q4_K), st, wmap, tiles, W, C, (int)ldc, (int)M, (int)N,
-                                         n_stages, mtiles, tiles_per_cta, c_vec4));
-    else
-      NNTR_CHECK_CUDA(launch_in_clusters(parts > 1 ? gemm_f16_kernel<NNTR_Q6_K, true> : gemm_f16_kernel<NNTR_Q6_K, false>, grid,
-                                         parts, F16_THREADS, f16_smem(NNTR_Q6_K), st, wmap, tiles, W, C, (int)ldc, (int)M, (int)N,
-                                         n_stages, mtiles, tiles_per_cta, c_vec4));
+    rc = qtype == NNTR_Q4_K ? launch_typed<NNTR_Q4_K>(M, N, K, tiles, B, C, ldc, st) : launch_typed<NNTR_Q6_K>(M, N, K, tiles, B, C, ldc, st);
   } else {
     const int64_t nwarps = (int64_t)Mpad * ((K + 255) / 256);
-    quantize_q8_0_f16_tiles_kernel<<<(unsigned)((nwarps + 7) / 8), 256, 0, st>>>(A, K, static_cast<uint8_t *>(ws), (int)M,
-                                                                               Mpad, (int)K);
+    quantize_q8_0_f16_tiles_kernel<<<(unsigned)((nwarps + 7) / 8), 256, 0, st>>>(A, K, tiles, (int)M, Mpad, (int)K);
     count_launch();
     NNTR_CHECK_CUDA(cudaGetLastError());
-    NNTR_CHECK_CUDA(launch_in_clusters(parts > 1 ? gemm_f16_kernel<NNTR_Q4_0, true> : gemm_f16_kernel<NNTR_Q4_0, false>, grid,
-                                         parts, F16_THREADS, f16_smem(NNTR_Q4_0), st, wmap, tiles, W, C, (int)ldc, (int)M, (int)N,
-                                         n_stages, mtiles, tiles_per_cta, c_vec4));
+    rc = launch_typed<NNTR_Q4_0>(M, N, K, tiles, B, C, ldc, st);
   }
+  if (rc)
+    return rc;
   count_launch();
   return check_cuda(cudaGetLastError(), "gemm fp16 tensor-path launch");
 }

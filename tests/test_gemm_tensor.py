@@ -231,6 +231,40 @@ def test_fp16_tensor_gemm_every_tile_sees_the_same_weights(be, q, K):
     be.device_status()
 
 
+@pytest.mark.parametrize("q,M,N,K", [("q4_0", 257, 256, 64), ("q4_0", 385, 512, 448), ("q4_0", 513, 9984, 704), ("q4_K", 300, 512, 256),
+                                     ("q4_K", 641, 9984, 512), ("q4_K", 897, 10240, 2304), ("q6_K", 260, 300, 256),
+                                     ("q6_K", 513, 10001, 768)])
+def test_fp16_tensor_gemm_in_pairs_of_ctas(be, q, M, N, K):
+    """More than 256 rows and no cut along K: two CTAs share a tile of 512 rows. One stage, fewer stages than producer groups,
+    an odd count; tiles of three, five and seven times 128 rows, whose last pair has a tile in one CTA only; a ragged last row and
+    (Q6_K) a ragged last column; an odd row stride of C. Every 512 weight rows are alike, so C's columns have to be, bit for bit.
+    Against the bit-exact kernels two fp16 roundings per product: 2 * 2^-11, in random directions, of the largest result."""
+    gen = {"q4_K": O.random_q4_Kx8, "q4_0": O.random_q4_0x8, "q6_K": O.random_q6_K}[q]
+    rng = np.random.default_rng(M + K)
+    B = torch.from_numpy(gen(rng, 512, K)).cuda().view(torch.uint8).reshape(-1)
+    per_row = B.numel() // 512
+    B = B.repeat((N + 511) // 512)[:N * per_row].contiguous()
+    A = torch.from_numpy(acts(rng, M, K)).cuda() if K % 256 == 0 else torch.from_numpy(rng.standard_normal((M, K)).astype(np.float32)).cuda()
+
+    def call(path, ldc):
+        C = torch.full((M, ldc), float("nan"), device="cuda")
+        be.set_gemm_path(path)
+        getattr(be, f"gemm_{q}")(M, N, K, A, K, B, N, C, ldc)
+        be.set_gemm_path("auto")
+        be.device_status()
+        assert bool(C[:, N:].isnan().all())
+        return C[:, :N].contiguous()
+
+    got, want = call("tensor_f16", N + 1), call("exact", N)
+    assert bool(got.isfinite().all())
+    assert float((got - want).abs().max() / want.abs().max()) <= 1e-3
+    for c in range(512, N, 512):
+        n = min(512, N - c)
+        assert torch.equal(got[:, c:c + n], got[:, :n])
+    for _ in range(5):
+        assert torch.equal(call("tensor_f16", N).view(torch.int32), got.view(torch.int32))
+
+
 def test_int8_peak_measurement_is_plausible(be):
     """The int8 rate the prefill fraction is quoted against: a dense tcgen05 kind::i8 stream on every SM. A B200 is
     specified at 4.5 POP/s dense; anything outside 1.5 .. 6 POP/s means the measurement is not doing the work."""
