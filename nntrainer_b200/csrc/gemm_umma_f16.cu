@@ -52,7 +52,8 @@
  * carries 96 KB for the MMAs, 64 of stores and copies and the packed weights. A pair takes 1070, the MMAs: half of the expansion and 64 KB
  * for the MMAs. (With no expansion and no copies at all 1050; a hand-over from CTA to CTA with release and acquire at cluster
  * scope 1600: it is one more latency in each round of the ring.) Q4_K 24576 x 4096, 1024 rows 184.6 -> 167 us, 512
- * rows 115.9 -> 101.6; Q4_0 512 rows of 24576 x 2880 85.2 -> 77.3; Q6_K 151936 x 2560, 300 / 512 rows 515 / 572 -> 346 / 380.
+ * rows 115.9 -> 101.6 (98.5 with even_rows()); Q4_0 512 rows of 24576 x 2880 85.2 -> 77.3 (70.6); Q6_K 151936 x 2560, 300 / 512 rows
+ * 515 / 572 -> 346 / 380.
  *
  * Few tiles: a cluster of two, four or eight CTAs shares a tile, each walks a part of K (k_parts), and the sums are added
  * through distributed shared memory. 512 x 1280 x 2560: Q4_0 40 -> 25 us, Q6_K 69 -> 33; 128 x 2560 x 8192: Q4_0 93 -> 25,
@@ -63,6 +64,7 @@
 #include "pipeline.cuh"
 #include "tma_map.cuh"
 
+#include <algorithm>
 #include <cuda_fp16.h>
 
 namespace nntr {
@@ -70,7 +72,7 @@ namespace nntr {
 namespace {
 
 constexpr int F16_TILE_M = 128;  // rows of an activation tile
-constexpr int F16_TILE_N = 256;  // weight rows of a tile of C
+constexpr int F16_TILE_N = 256;  // weight rows of a tile of C, at most
 constexpr int F16_KS = 64;       // K per stage
 constexpr int F16_A_BYTES = F16_TILE_M * F16_KS * 2; // 16 KB
 constexpr int F16_PRODUCERS = 512;
@@ -211,10 +213,11 @@ template <int QT, int MODE>
 __global__ void __launch_bounds__(F16_THREADS, 1)
 gemm_f16_kernel(const __grid_constant__ CUtensorMap wmap, const uint8_t *__restrict__ atiles, const uint8_t *__restrict__ Wb,
                 float *__restrict__ C, int ldc, int M, int N, int k_stages, int m_tiles, int tiles_per_cta,
-                int c_vec4) {
+                int max_rows, int c_vec4) {
   extern __shared__ __align__(128) uint8_t smem[];
   using Cfg = F16Cfg<QT, MODE>;
   constexpr bool SHARED = MODE == F16_SHARED, PAIR = MODE == F16_PAIR;
+  const int tile_rows = SHARED ? F16_TILE_N : max_rows; // weight rows of the tile
   // bars: [0..3] full, [4..7] empty, [8] tile complete, [9..12] packed weights here, [13..16] packed weights read,
   // [17..18] Q4_K headers here
   const uint32_t sbase = smem_u32(smem);
@@ -230,6 +233,7 @@ gemm_f16_kernel(const __grid_constant__ CUtensorMap wmap, const uint8_t *__restr
   // a pair takes four activation tiles, its CTAs alternate ones
   const int peer = PAIR ? cluster_rank() : 0, mt_step = PAIR ? 2 : 1; // place in the pair
   const int mt = PAIR ? 4 * (blockIdx.x / 2) + peer : tiles_per_cta * (blockIdx.x / parts), nt = blockIdx.y;
+  const int n0 = nt * tile_rows, own_rows = PAIR ? tile_rows / 2 : tile_rows; // the tile's first weight row, rows that this CTA expands
   const bool two = PAIR ? mt - peer + 2 < m_tiles : tiles_per_cta == 2 && mt + 1 < m_tiles; // the same in both CTAs of a pair
   constexpr int UNIT = QT == NNTR_Q4_K ? 4 : QT == NNTR_Q6_K ? 2 : 1;
   const int units = k_stages / UNIT;
@@ -284,6 +288,8 @@ gemm_f16_kernel(const __grid_constant__ CUtensorMap wmap, const uint8_t *__restr
     }
   };
   auto store4 = [&](int row, int col, const float4 &f) {
+    if (col >= n0 + tile_rows) // a multiple of 16
+      return;
     float *dst = C + (size_t)row * ldc + col;
     if (c_vec4 && col + 4 <= N) {
       *reinterpret_cast<float4 *>(dst) = f;
@@ -360,6 +366,7 @@ gemm_f16_kernel(const __grid_constant__ CUtensorMap wmap, const uint8_t *__restr
         if (!(ok = slot_wait(st)))
           break;
         uint8_t *wdst = smem + (st % Cfg::STAGES) * Cfg::STAGE_BYTES + r * 16;
+        if (r < own_rows)
 #pragma unroll
         for (int c = 0; c < 4; ++c) {
           // word -> 8 halves in the order [lo b0, lo b2, lo b1, lo b3, hi b0, hi b2, hi b1, hi b3]
@@ -376,8 +383,8 @@ gemm_f16_kernel(const __grid_constant__ CUtensorMap wmap, const uint8_t *__restr
         ok = st + Cfg::GROUPS >= n_stages || fetch(st + Cfg::GROUPS);
       }
     } else if constexpr (QT == NNTR_Q6_K) {
-      const int n_row = nt * F16_TILE_N + peer * Cfg::W_ROWS + r, qhalf = hsel & 1;
-      const bool have_row = n_row < N; // rows beyond N: scale 0, so zero weights (their columns are not stored either)
+      const int n_row = n0 + peer * own_rows + r, qhalf = hsel & 1;
+      const bool have_row = r < own_rows && n_row < N; // rows beyond N: scale 0, so zero weights (their columns are not stored either)
       const int nb = k_stages / 4, n_groups = n_stages / 2, g0 = st0 / 2;
       const uint8_t *wrow = Wb + (size_t)(have_row ? n_row : 0) * nb * sizeof(BlockQ6K);
       // A group is the two stages of one half h of a super-block: they share the 32 qh bytes. This thread: bytes
@@ -427,6 +434,7 @@ gemm_f16_kernel(const __grid_constant__ CUtensorMap wmap, const uint8_t *__restr
             break;
           uint8_t *wdst = smem + s * Cfg::STAGE_BYTES + r * 16 + (4 * qhalf) * (Cfg::W_ROWS * 16);
           const __half2 off = __half2half2(__ushort_as_half(0x6420)); // 1024 + 32
+          if (r < own_rows)
 #pragma unroll
           for (int i = 0; i < 4; ++i) {
             const uint32_t l = ql[s2][i], hq = qh[i];
@@ -473,6 +481,7 @@ gemm_f16_kernel(const __grid_constant__ CUtensorMap wmap, const uint8_t *__restr
         if (!(ok = slot_wait(st)))
           break;
         uint8_t *wdst = smem + (st % Cfg::STAGES) * Cfg::STAGE_BYTES + r * 16;
+        if (r < own_rows)
 #pragma unroll
         for (int k = 0; k < 2; ++k) {
           const __half2 d2 = __half2half2(__ushort_as_half(dbits[k]));
@@ -494,8 +503,8 @@ gemm_f16_kernel(const __grid_constant__ CUtensorMap wmap, const uint8_t *__restr
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
       if (parts == 1) {
         const float *turn = reinterpret_cast<const float *>(smem) + turn_area(warp);
-        const int cc = nt * F16_TILE_N + (warp >> 2) * 64 + 4 * (lane & 15);
-        for (int hm = 0; hm < (two ? 2 : 1); ++hm) {
+        const int cc = n0 + (warp >> 2) * 64 + 4 * (lane & 15);
+        for (int hm = 0; hm < ((warp >> 2) * 64 >= tile_rows ? 0 : two ? 2 : 1); ++hm) {
           const int row0 = (mt + mt_step * hm) * F16_TILE_M + (warp & 3) * 32;
           turn_round(hm);
           __syncwarp();
@@ -538,19 +547,20 @@ gemm_f16_kernel(const __grid_constant__ CUtensorMap wmap, const uint8_t *__restr
     // copies, a box of 32 row groups x 128 (Q4_0: 144) bytes each: 32 untiled copies of 256 bytes per stage measured 1.6 times
     // slower than no ring at all.
     if (QT != NNTR_Q6_K && lane == 0) {
-      const int y = (nt * F16_TILE_N + peer * Cfg::W_ROWS) / 8;
+      const int y = (n0 + peer * own_rows) / 8;
+      const uint32_t box = own_rows / 8 * Cfg::RAW_BOX; // bytes of a copy
       for (int st = 0; st < n_stages; ++st) {
         const int rs = st % Cfg::RAW, use = st / Cfg::RAW;
         if (use > 0 && !mbar_wait(BAR(13 + rs), (use - 1) & 1, abort_flag))
           break;
-        mbar_expect_tx(BAR(9 + rs), Cfg::RAW_BYTES);
+        mbar_expect_tx(BAR(9 + rs), 2 * box);
         const uint32_t dst = sbase + Cfg::OFF_RAW + rs * Cfg::RAW_BYTES;
         int x = (st0 + st) * 2 * (int)sizeof(BlockQ40x8);
         if (QT == NNTR_Q4_K) {
           x = ((st0 + st) >> 2) * (int)sizeof(BlockQ4Kx8);
           if ((st & 3) == 0) { // two headers: the stages up to st - RAW have been read, the one replaced served those up to st - 5
             const int hb = (st >> 2) & 1;
-            mbar_expect_tx(BAR(17 + hb), Cfg::HDR_BYTES);
+            mbar_expect_tx(BAR(17 + hb), box);
             tma_tile(sbase + Cfg::OFF_HDR + hb * Cfg::HDR_BYTES, &wmap, x, y, BAR(17 + hb));
           }
           x += 128 + 256 * (st & 3);
@@ -570,8 +580,8 @@ gemm_f16_kernel(const __grid_constant__ CUtensorMap wmap, const uint8_t *__restr
         mbar_arrive_remote(BAR(s), 0);
       }
     } else if (lane == 0) {
-      // D = F32; A = activations (F16, 128 rows = lanes, PAIR: of each CTA); B = weights (F16, 256 rows = columns); both K-major
-      const uint32_t idesc = (1u << 4) | (0u << 7) | (0u << 10) | ((uint32_t)(F16_TILE_N >> 3) << 17) |
+      // D = F32; A = activations (F16, 128 rows = lanes, PAIR: of each CTA); B = weights (F16, tile_rows rows = columns); both K-major
+      const uint32_t idesc = (1u << 4) | (0u << 7) | (0u << 10) | ((uint32_t)(tile_rows >> 3) << 17) |
                              ((uint32_t)((PAIR ? 2 : 1) * F16_TILE_M >> 4) << 24);
       bool ok = true;
       for (int st = 0; st < n_stages && ok; ++st) {
@@ -623,7 +633,7 @@ gemm_f16_kernel(const __grid_constant__ CUtensorMap wmap, const uint8_t *__restr
               v[0] = make_float4(v[0].x + v[k].x, v[0].y + v[k].y, v[0].z + v[k].z, v[0].w + v[k].w);
           if (__any_sync(0xffffffffu, raised)) // a part is missing: C stays as it is
             break;
-          store4(row0 + r, nt * F16_TILE_N + c, v[0]);
+          store4(row0 + r, n0 + c, v[0]);
         }
       }
       cluster_sync(); // the area is rewritten by the second activation tile, and nobody leaves while it is read
@@ -768,10 +778,22 @@ namespace {
 
 template <int QT, int MODE>
 int launch_mode(dim3 grid, int cluster, cudaStream_t st, const CUtensorMap &wmap, const uint8_t *tiles, const uint8_t *W, float *C,
-                int ldc, int M, int N, int k_stages, int m_tiles, int tiles_per_cta, int c_vec4) {
+                int ldc, int M, int N, int k_stages, int m_tiles, int tiles_per_cta, int tile_rows, int c_vec4) {
   NNTR_CHECK_CUDA(launch_in_clusters(gemm_f16_kernel<QT, MODE>, grid, cluster, F16_THREADS, F16Cfg<QT, MODE>::SMEM, st, wmap, tiles, W,
-                                     C, ldc, M, N, k_stages, m_tiles, tiles_per_cta, c_vec4));
+                                     C, ldc, M, N, k_stages, m_tiles, tiles_per_cta, tile_rows, c_vec4));
   return NNTR_CUDA_OK;
+}
+
+/** Weight rows of a tile, so that the tiles of m_groups rows of them fill the waves of `slots` that they need anyway: with 256 rows a
+ *  last wave can be nearly empty. A multiple of step, at least 128 (the copies of the activations cost the same for fewer rows). Q4_K
+ *  1024 x 9728 x 2560 71.8 -> 66.7 us, 256 x 24576 x 4096 58.0 -> 54.5, Q4_0 200 x 24576 x 4096 55.3 -> 49.8, Q6_K 256 x 151936 x 2560
+ *  320 -> 282, 700 x 12288 x 4096 125 -> 109; Q4_K 1024 x 24576 x 4096, whose last wave was 60 % full, 167 and 168. */
+int even_rows(int m_groups, int N, int slots, int step) {
+  const int tiles = m_groups * ((N + F16_TILE_N - 1) / F16_TILE_N);
+  if (slots < m_groups)
+    return F16_TILE_N;
+  const int n_tiles = (tiles + slots - 1) / slots * slots / m_groups, rows = (N + n_tiles - 1) / n_tiles;
+  return std::min(F16_TILE_N, std::max(128, (rows + step - 1) / step * step));
 }
 
 /** allows every form of the kernel its shared memory, once per device */
@@ -798,28 +820,30 @@ int launch_typed(unsigned M, unsigned N, unsigned K, const uint8_t *tiles, const
     return rc;
   const int parts = k_parts<QT>(cta_m * n_tiles, k_stages);
   const bool pair = parts == 1 && mtiles > 2;
-  // tiles one by one if they run in the same wave as the pairs: 128 instead of 256 columns of MMAs per stage and one sum at the
-  // end instead of two (256 x 1280 x 2560 Q4_0: 24 -> 16 us)
-  if (parts > 1 && mtiles > 1 && parts == k_parts<QT>(mtiles * n_tiles, k_stages)) {
+  int tile_rows = F16_TILE_N;
+  if (pair) {
+    static ClusterFit fit;
+    cta_m = (mtiles + 3) / 4;
+    tile_rows = even_rows(cta_m, (int)N, fit(gemm_f16_kernel<QT, F16_PAIR>, 2, F16_THREADS, F16Cfg<QT, F16_PAIR>::SMEM), 32);
+  } else if (parts == 1) {
+    tile_rows = even_rows(cta_m, (int)N, sm_count(), 16);
+  } else if (mtiles > 1 && parts == k_parts<QT>(mtiles * n_tiles, k_stages)) {
+    // tiles one by one if they run in the same wave as the pairs: 128 instead of 256 columns of MMAs per stage and one sum at the
+    // end instead of two (256 x 1280 x 2560 Q4_0: 24 -> 16 us)
     tiles_per_cta = 1;
     cta_m = mtiles;
   }
   CUtensorMap wmap = {};
   if (QT != NNTR_Q6_K) { // rows of 8-row groups of packed weights
     const uint64_t row = QT == NNTR_Q4_K ? (uint64_t)(K / QK_K) * sizeof(BlockQ4Kx8) : (uint64_t)(K / 32) * sizeof(BlockQ40x8);
-    const int rc = encode_map_2d(&wmap, B, 1, row, N / 8, row, F16Cfg<QT, F16_LONE>::RAW_BOX,
-                                 pair ? F16Cfg<QT, F16_PAIR>::ROW_GROUPS : F16Cfg<QT, F16_LONE>::ROW_GROUPS, false);
+    const int rc = encode_map_2d(&wmap, B, 1, row, N / 8, row, F16Cfg<QT, F16_LONE>::RAW_BOX, (unsigned)(pair ? tile_rows / 2 : tile_rows) / 8, false);
     if (rc)
       return rc;
   }
   const uint8_t *W = static_cast<const uint8_t *>(B);
-  if (pair)
-    return launch_mode<QT, F16_PAIR>(dim3((mtiles + 3) / 4, n_tiles), 2, st, wmap, tiles, W, C, (int)ldc, (int)M, (int)N, k_stages, mtiles,
-                                     2, c_vec4);
-  if (parts > 1)
-    return launch_mode<QT, F16_SHARED>(dim3(cta_m, n_tiles), parts, st, wmap, tiles, W, C, (int)ldc, (int)M, (int)N, k_stages, mtiles,
-                                       tiles_per_cta, c_vec4);
-  return launch_mode<QT, F16_LONE>(dim3(cta_m, n_tiles), 1, st, wmap, tiles, W, C, (int)ldc, (int)M, (int)N, k_stages, mtiles, 2, c_vec4);
+  const dim3 grid(cta_m, ((int)N + tile_rows - 1) / tile_rows);
+  const auto launch = pair ? launch_mode<QT, F16_PAIR> : parts > 1 ? launch_mode<QT, F16_SHARED> : launch_mode<QT, F16_LONE>;
+  return launch(grid, pair ? 2 : parts, st, wmap, tiles, W, C, (int)ldc, (int)M, (int)N, k_stages, mtiles, tiles_per_cta, tile_rows, c_vec4);
 }
 
 } // namespace

@@ -233,9 +233,11 @@ def test_fp16_tensor_gemm_every_tile_sees_the_same_weights(be, q, K):
 
 @pytest.mark.parametrize("q,M,N,K", [("q4_0", 257, 256, 64), ("q4_0", 385, 512, 448), ("q4_0", 513, 9984, 704), ("q4_K", 300, 512, 256),
                                      ("q4_K", 641, 9984, 512), ("q4_K", 897, 10240, 2304), ("q6_K", 260, 300, 256),
-                                     ("q6_K", 513, 10001, 768)])
-def test_fp16_tensor_gemm_in_pairs_of_ctas(be, q, M, N, K):
-    """More than 256 rows and no cut along K: two CTAs share a tile of 512 rows. One stage, fewer stages than producer groups,
+                                     ("q6_K", 513, 10001, 768), ("q4_K", 200, 20480, 512),
+                                     ("q4_0", 130, 19200, 320), ("q6_K", 100, 20001, 256)])
+def test_fp16_tensor_gemm_in_pairs_of_ctas_and_narrow_tiles(be, q, M, N, K):
+    """More than 256 rows and no cut along K: two CTAs share a tile of 512 rows. Tiles of fewer than 256 weight rows, for pairs and for
+    single CTAs, the last one ragged. One stage, fewer stages than producer groups,
     an odd count; tiles of three, five and seven times 128 rows, whose last pair has a tile in one CTA only; a ragged last row and
     (Q6_K) a ragged last column; an odd row stride of C. Every 512 weight rows are alike, so C's columns have to be, bit for bit.
     Against the bit-exact kernels two fp16 roundings per product: 2 * 2^-11, in random directions, of the largest result."""
