@@ -68,7 +68,8 @@ constexpr int MAX_E_PER_LANE = 8; // up to 256 experts
 // 2048, with a CTA row per token / with eight tokens per CTA row, 16 / 24 / 32 / 48 / 64 tokens: 98.7 / 114.2 / 126.3 / 136.4 /
 // 147.5 us, 97.8 / 111.7 / 121.7 / 128.1 / 134.0.
 constexpr unsigned ROUTER_ROWS_MIN_TOKENS = 48;
-constexpr int ROUTER_PRE = 8;     // rows of a warp's slice fetched before the dependency wait
+/** rows of a warp's slice fetched before the dependency wait: all of them for hidden sizes up to 2048 (96 experts and fewer: 3072) */
+template <int PER> constexpr int ROUTER_PRE = PER < 4 ? 12 : 8;
 
 /* std::partial_sort(idx, idx + k, idx + n, [&](a, b) { return v[a] > v[b]; }) on idx = 0..n-1, as the GNU C++ library
  * performs it (heap selection, then heap sort): out[0..k) = the indices of the k greatest values in descending order,
@@ -131,8 +132,8 @@ struct RouterOut {
 };
 
 /* One warp: logits, softmax and top-k of token t from its partial sums. area: E + 32 floats of shared memory. PER: experts per
- * lane at most (4: up to 128 experts). */
-template <int PER>
+ * lane at most (4: up to 128 experts). SUMMED: area holds the partial sums' sums already. */
+template <int PER, bool SUMMED>
 __device__ __forceinline__ void router_finish(const RouterOut &o, int t, int E, int lane, float *area) {
   const int per = (E + 31) / 32, topk = o.topk;
   const float *rpart = o.rpart, *bias = o.bias;
@@ -144,10 +145,10 @@ __device__ __forceinline__ void router_finish(const RouterOut &o, int t, int E, 
   float mx = -INFINITY;
 #pragma unroll
   for (int i = 0; i < PER; ++i)
-    p[i] = 0.f;
-  constexpr int FLY = 64 / PER; // partial sums of that many slices are on their way at a time, added in order
+    p[i] = SUMMED ? area[min(lane + 32 * i, E - 1)] : 0.f;
+  constexpr int FLY = PER > 1 ? 64 / PER : ROUTER_SLICES; // partial sums of that many slices are on their way at a time, added in order
 #pragma unroll
-  for (int w0 = 0; w0 < ROUTER_SLICES; w0 += FLY) {
+  for (int w0 = SUMMED ? ROUTER_SLICES : 0; w0 < ROUTER_SLICES; w0 += FLY) {
     float v[FLY][PER];
 #pragma unroll
     for (int w = 0; w < FLY; ++w)
@@ -204,36 +205,35 @@ __device__ __forceinline__ void router_finish(const RouterOut &o, int t, int E, 
       pv[e] = p[i];
   }
   int *sel = reinterpret_cast<int *>(area + E); // [topk]
-  float prev = -1.f;
+  // a probability's bits + 1 compare like the probability; 0: none (not a number, or taken). Two reductions by the warp's own
+  // instruction a round, in place of five rounds of shuffles of value and index: topk + 1 such rounds are a chain
+  unsigned key[PER];
+#pragma unroll
+  for (int i = 0; i < PER; ++i)
+    key[i] = p[i] >= 0.f ? __float_as_uint(p[i]) + 1u : 0u;
+  unsigned prev = 0;
   bool tie = false;
   const int rounds = topk < E ? topk + 1 : topk;
   for (int k = 0; k < rounds; ++k) {
-    float bv = -1.f;
+    unsigned bv = 0;
     int be = 0x7fffffff;
 #pragma unroll
     for (int i = 0; i < PER; ++i) {
-      const int e = lane + 32 * i;
-      if (p[i] > bv) { // ascending e within the lane: the first maximum wins
-        bv = p[i];
-        be = e;
+      if (key[i] > bv) { // ascending e within the lane: the first maximum wins
+        bv = key[i];
+        be = lane + 32 * i;
       }
     }
-    for (int o = 16; o; o >>= 1) {
-      const float ov = __shfl_xor_sync(FULL, bv, o);
-      const int oe = __shfl_xor_sync(FULL, be, o);
-      if (ov > bv || (ov == bv && oe < be)) {
-        bv = ov;
-        be = oe;
-      }
-    }
+    const unsigned top = __reduce_max_sync(FULL, bv);
+    be = (int)__reduce_min_sync(FULL, bv == top ? (unsigned)be : 0x7fffffffu);
     if ((be & 31) == lane) { // the owner retires the winner
 #pragma unroll
       for (int i = 0; i < PER; ++i)
         if (i == (be >> 5))
-          p[i] = -1.f;
+          key[i] = 0;
     }
-    tie = tie || (k > 0 && bv == prev) || bv < 0.f; // no winner: probabilities that are not numbers
-    prev = bv;
+    tie = tie || (k > 0 && top == prev) || top == 0; // no winner: probabilities that are not numbers
+    prev = top;
     if (k < topk && lane == 0)
       sel[k] = be;
   }
@@ -267,7 +267,10 @@ __device__ __forceinline__ void router_finish(const RouterOut &o, int t, int E, 
 
 /* ROUTER_SLICES CTAs per token: each sums its slice of the hidden dimension into partial logits (the router weight
  * is a megabyte per layer: a few CTAs alone would be bound by the latency of their own loads); the CTA that arrives last on
- * the token's counter adds the partials in slice order and does softmax, top-k and the tables. */
+ * the token's counter adds the partials in slice order and does softmax, top-k and the tables. Latency from end to end; one token
+ * through 8 of 128 experts of 2048 x 768 20.1 us, 4 x larger weights of 256 experts 39.1 (with code for 256 experts whatever there
+ * are, the partial sums and the selection by one warp's loads and shuffles: 23.0 and 53.6). */
+template <int PER> // experts per lane
 __global__ void __launch_bounds__(ROUTER_WARPS * 32)
 moe_router_kernel(const float *__restrict__ x, const float *__restrict__ wr, int H, int E, const RouterOut o, MoeEp ep) {
   extern __shared__ float rsm[]; // [ROUTER_WARPS][E]
@@ -275,19 +278,18 @@ moe_router_kernel(const float *__restrict__ x, const float *__restrict__ wr, int
   const int t = blockIdx.x, sl = blockIdx.y, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   pdl_launch_dependents(); // the expert GEMVs may be scheduled now; they wait for this grid before reading its tables
   // The router weight does not depend on the previous kernel: the first ROUTER_PRE rows of this warp's slice are
-  // fetched into registers before the wait (for H = 2048 that is the whole slice), so that only the activation's
+  // fetched into registers before the wait (mostly the whole slice), so that only the activation's
   // round trip is left behind it.
-  const int per = (E + 31) / 32;
   const int nw = ROUTER_SLICES * ROUTER_WARPS, wi = sl * ROUTER_WARPS + warp;
   const int h0 = (int)(((long long)wi * H) / nw), h1 = (int)(((long long)(wi + 1) * H) / nw);
-  float wpre[ROUTER_PRE][MAX_E_PER_LANE];
+  float wpre[ROUTER_PRE<PER>][PER];
 #pragma unroll
-  for (int u = 0; u < ROUTER_PRE; ++u) {
+  for (int u = 0; u < ROUTER_PRE<PER>; ++u) {
     const int hh = h0 + u < h1 ? h0 + u : h1 - 1;
     const float *row = wr + (size_t)hh * E;
 #pragma unroll
-    for (int i = 0; i < MAX_E_PER_LANE; ++i)
-      wpre[u][i] = (i < per && lane + 32 * i < E && h1 > h0) ? row[lane + 32 * i] : 0.f;
+    for (int i = 0; i < PER; ++i)
+      wpre[u][i] = (lane + 32 * i < E && h1 > h0) ? row[lane + 32 * i] : 0.f;
   }
   pdl_wait(); // x comes from the kernel before (no-op without the launch attribute)
   if (ep.n_ranks && t == 0 && sl == 0 && threadIdx.x < ep.n_ranks) {
@@ -297,41 +299,41 @@ moe_router_kernel(const float *__restrict__ x, const float *__restrict__ wr, int
     *slot = seq;
   }
   const float *xt = x + (size_t)t * H;
-  float acc[MAX_E_PER_LANE];
+  float acc[PER];
 #pragma unroll
-  for (int i = 0; i < MAX_E_PER_LANE; ++i)
+  for (int i = 0; i < PER; ++i)
     acc[i] = 0.f;
   {
-    float xv[ROUTER_PRE];
+    float xv[ROUTER_PRE<PER>];
 #pragma unroll
-    for (int u = 0; u < ROUTER_PRE; ++u)
+    for (int u = 0; u < ROUTER_PRE<PER>; ++u)
       xv[u] = h0 + u < h1 ? xt[h0 + u] : 0.f;
 #pragma unroll
-    for (int u = 0; u < ROUTER_PRE; ++u)
+    for (int u = 0; u < ROUTER_PRE<PER>; ++u)
 #pragma unroll
-      for (int i = 0; i < MAX_E_PER_LANE; ++i)
+      for (int i = 0; i < PER; ++i)
         acc[i] = fmaf(xv[u], wpre[u][i], acc[i]); // rows past the slice: x = 0, as in the tail of the loop below
   }
-  for (int h = h0 + ROUTER_PRE; h < h1; h += 4) { // four rows in flight per lane
-    float xv[4], wv[4][MAX_E_PER_LANE];
+  for (int h = h0 + ROUTER_PRE<PER>; h < h1; h += 4) { // four rows in flight per lane
+    float xv[4], wv[4][PER];
 #pragma unroll
     for (int u = 0; u < 4; ++u) {
       const int hh = h + u < h1 ? h + u : h1 - 1;
       xv[u] = h + u < h1 ? xt[hh] : 0.f;
       const float *row = wr + (size_t)hh * E;
 #pragma unroll
-      for (int i = 0; i < MAX_E_PER_LANE; ++i)
-        wv[u][i] = (i < per && lane + 32 * i < E) ? row[lane + 32 * i] : 0.f;
+      for (int i = 0; i < PER; ++i)
+        wv[u][i] = (lane + 32 * i < E) ? row[lane + 32 * i] : 0.f;
     }
 #pragma unroll
     for (int u = 0; u < 4; ++u)
 #pragma unroll
-      for (int i = 0; i < MAX_E_PER_LANE; ++i)
+      for (int i = 0; i < PER; ++i)
         acc[i] = fmaf(xv[u], wv[u][i], acc[i]);
   }
 #pragma unroll
-  for (int i = 0; i < MAX_E_PER_LANE; ++i)
-    if (i < per && lane + 32 * i < E)
+  for (int i = 0; i < PER; ++i)
+    if (lane + 32 * i < E)
       rsm[warp * E + lane + 32 * i] = acc[i];
   __syncthreads();
   float *mine = o.rpart + ((size_t)t * ROUTER_SLICES + sl) * E;
@@ -350,20 +352,30 @@ moe_router_kernel(const float *__restrict__ x, const float *__restrict__ wr, int
       o.rcount[t] = 0; // ready for the next call
   }
   __syncthreads();
-  if (!is_last || warp != 0)
+  if (!is_last)
     return;
   __threadfence();
-  if (E <= 128)
-    router_finish<4>(o, t, E, lane, rsm);
-  else
-    router_finish<8>(o, t, E, lane, rsm);
+  // a thread per expert adds its partial sums in the order of the slices, all of them on their way at once
+  for (int e = threadIdx.x; e < E; e += ROUTER_WARPS * 32) {
+    float v[ROUTER_SLICES], sum = 0.f;
+#pragma unroll
+    for (int w = 0; w < ROUTER_SLICES; ++w)
+      v[w] = __ldcg(o.rpart + ((size_t)t * ROUTER_SLICES + w) * E + e);
+#pragma unroll
+    for (int w = 0; w < ROUTER_SLICES; ++w)
+      sum += v[w];
+    rsm[e] = sum;
+  }
+  __syncthreads();
+  if (warp == 0)
+    router_finish<PER, true>(o, t, E, lane, rsm);
 }
 
 /* The same for a batch: a CTA takes TT tokens through its slice, so that the router weight crosses the L2 once per TT tokens
  * instead of once per token, and the last arriver's warps finish a token each. Every sum is formed in the order of the kernel
  * above (row by row inside a warp, then warp by warp, then slice by slice), so a token is routed alike by both. 256 tokens,
  * 2048 x 128 weights: 34 us, 94 with a CTA row per token. */
-template <int TT>
+template <int TT, int PER> // tokens, experts per lane
 __global__ void __launch_bounds__(ROUTER_WARPS * 32)
 moe_router_rows_kernel(const float *__restrict__ x, const float *__restrict__ wr, int T, int H, int E, const RouterOut o) {
   extern __shared__ float rsm[]; // [ROUTER_WARPS][TT][E], then the slice of the activations [TT][rows]
@@ -373,28 +385,28 @@ moe_router_rows_kernel(const float *__restrict__ x, const float *__restrict__ wr
   const int nw = ROUTER_SLICES * ROUTER_WARPS, wi = sl * ROUTER_WARPS + warp;
   const int h0 = (int)(((long long)wi * H) / nw), h1 = (int)(((long long)(wi + 1) * H) / nw);
   const int s0 = (int)(((long long)sl * ROUTER_WARPS * H) / nw), s1 = (int)(((long long)(sl + 1) * ROUTER_WARPS * H) / nw);
-  const int rows = s1 - s0, per = (E + 31) / 32;
+  const int rows = s1 - s0;
   float *xs = rsm + ROUTER_WARPS * TT * E;
   pdl_wait();
   for (int i = threadIdx.x; i < TT * rows; i += ROUTER_WARPS * 32) {
     const int k = i / rows, h = i - k * rows;
     xs[i] = t0 + k < T ? x[(size_t)(t0 + k) * H + s0 + h] : 0.f;
   }
-  float acc[TT][MAX_E_PER_LANE];
+  float acc[TT][PER];
 #pragma unroll
   for (int k = 0; k < TT; ++k)
 #pragma unroll
-    for (int i = 0; i < MAX_E_PER_LANE; ++i)
+    for (int i = 0; i < PER; ++i)
       acc[k][i] = 0.f;
   __syncthreads();
   for (int h = h0; h < h1; h += 4) { // four rows in flight per lane
-    float wv[4][MAX_E_PER_LANE];
+    float wv[4][PER];
 #pragma unroll
     for (int u = 0; u < 4; ++u) {
       const float *row = wr + (size_t)(h + u < h1 ? h + u : h1 - 1) * E;
 #pragma unroll
-      for (int i = 0; i < MAX_E_PER_LANE; ++i)
-        wv[u][i] = (i < per && lane + 32 * i < E) ? row[lane + 32 * i] : 0.f;
+      for (int i = 0; i < PER; ++i)
+        wv[u][i] = (lane + 32 * i < E) ? row[lane + 32 * i] : 0.f;
     }
 #pragma unroll
     for (int u = 0; u < 4; ++u)
@@ -403,16 +415,15 @@ moe_router_rows_kernel(const float *__restrict__ x, const float *__restrict__ wr
         for (int k = 0; k < TT; ++k) {
           const float xv = xs[k * rows + h + u - s0];
 #pragma unroll
-          for (int i = 0; i < MAX_E_PER_LANE; ++i)
-            if (i < per)
-              acc[k][i] = fmaf(xv, wv[u][i], acc[k][i]);
+          for (int i = 0; i < PER; ++i)
+            acc[k][i] = fmaf(xv, wv[u][i], acc[k][i]);
         }
   }
 #pragma unroll
   for (int k = 0; k < TT; ++k)
 #pragma unroll
-    for (int i = 0; i < MAX_E_PER_LANE; ++i)
-      if (i < per && lane + 32 * i < E)
+    for (int i = 0; i < PER; ++i)
+      if (lane + 32 * i < E)
         rsm[(warp * TT + k) * E + lane + 32 * i] = acc[k][i];
   __syncthreads();
   for (int i = threadIdx.x; i < TT * E; i += ROUTER_WARPS * 32) {
@@ -438,7 +449,7 @@ moe_router_rows_kernel(const float *__restrict__ x, const float *__restrict__ wr
     return;
   __threadfence();
   for (int k = warp; k < TT && t0 + k < T; k += ROUTER_WARPS)
-    router_finish<TT == 8 ? 4 : 8>(o, t0 + k, E, lane, rsm + warp * (E + 32));
+    router_finish<PER, false>(o, t0 + k, E, lane, rsm + warp * (E + 32));
 }
 
 /* Sorts the (token, expert) pairs of a batch by expert: off[e] = first position of expert e's pairs in perm, tile_off[e]
@@ -680,6 +691,11 @@ static cudaError_t launch_pdl(void (*kernel)(KArgs...), unsigned grid, unsigned 
   return cudaLaunchKernelEx(&cfg, kernel, static_cast<KArgs>(args)...);
 }
 
+/** the router for one token per CTA row, for the experts that there are */
+static auto router_kernel(unsigned E) {
+  return E <= 32 ? moe_router_kernel<1> : E <= 64 ? moe_router_kernel<2> : E <= 128 ? moe_router_kernel<4> : moe_router_kernel<8>;
+}
+
 struct MoeWs {
   size_t idx, ord, w, gu_tab, dn_tab, rpart, rcount, gu, act, dn, off, tile_off, act_off, perm, qx, qact, total;
 };
@@ -819,10 +835,13 @@ static int moe_forward(const nntr_moe_desc *d, const nntr_moe_ep *epd, unsigned 
       cfg.gridDim = dim3((tokens + tt - 1) / tt, ROUTER_SLICES);
       cfg.dynamicSmemBytes = std::max((size_t)ROUTER_WARPS * tt * E + (size_t)tt * (H / ROUTER_SLICES + ROUTER_WARPS),
                                       (size_t)ROUTER_WARPS * (E + 32)) * sizeof(float);
-      NNTR_CHECK_CUDA(cudaLaunchKernelEx(&cfg, tt == 8 ? moe_router_rows_kernel<8> : moe_router_rows_kernel<4>, x, d->router_w,
-                                         (int)tokens, (int)H, (int)E, out));
+      const auto kernel = E <= 32   ? moe_router_rows_kernel<8, 1>
+                          : E <= 64  ? moe_router_rows_kernel<8, 2>
+                          : E <= 128 ? moe_router_rows_kernel<8, 4>
+                                     : moe_router_rows_kernel<4, 8>;
+      NNTR_CHECK_CUDA(cudaLaunchKernelEx(&cfg, kernel, x, d->router_w, (int)tokens, (int)H, (int)E, out));
     } else {
-      NNTR_CHECK_CUDA(cudaLaunchKernelEx(&cfg, moe_router_kernel, x, d->router_w, (int)H, (int)E, out, ep));
+      NNTR_CHECK_CUDA(cudaLaunchKernelEx(&cfg, router_kernel(E), x, d->router_w, (int)H, (int)E, out, ep));
     }
     count_launch();
   }
@@ -975,8 +994,8 @@ extern "C" int nntr_cuda_moe_route_dev(const nntr_moe_desc *d, unsigned tokens, 
   const RouterOut out = {d->router_bias, (int)K, d->gate_w, d->up_w, d->down_w, idx_out, reinterpret_cast<int *>(ws + s.ord),
                          w_out, reinterpret_cast<const void **>(ws + s.gu_tab), reinterpret_cast<const void **>(ws + s.dn_tab),
                          reinterpret_cast<float *>(ws + s.rpart), reinterpret_cast<unsigned *>(ws + s.rcount)};
-  moe_router_kernel<<<dim3(tokens, ROUTER_SLICES), ROUTER_WARPS * 32, (ROUTER_WARPS * E + 32) * sizeof(float),
-                      static_cast<cudaStream_t>(stream)>>>(x, d->router_w, (int)d->hidden, (int)E, out, MoeEp{});
+  router_kernel(E)<<<dim3(tokens, ROUTER_SLICES), ROUTER_WARPS * 32, (ROUTER_WARPS * E + 32) * sizeof(float),
+                     static_cast<cudaStream_t>(stream)>>>(x, d->router_w, (int)d->hidden, (int)E, out, MoeEp{});
   count_launch();
   return check_cuda(cudaGetLastError(), "moe_router launch");
 }

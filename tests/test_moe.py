@@ -355,6 +355,29 @@ def test_a_token_that_is_not_a_number_leaves_the_others_alone(be, port, T, E, k)
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("E", [1, 31, 32, 33, 64, 65, 128, 129, 256])
+def test_router_for_every_number_of_experts(be, port, E):
+    """The router has a form for 32, 64, 128 and 256 experts, one for a token per row of CTAs and one for eight (four) of them. H =
+    3328: 13 rows of the weight per warp, more than are fetched ahead. The probabilities' weights to 1e-5 (sums of 3328 products in
+    another order), the batch's output equal to that of its tokens one by one."""
+    import torch
+    rng = np.random.default_rng(E)
+    H, I, T, k = 3328, 256, 50, min(8, E)
+    router, gate, up, down = make_layer(rng, H, I, E, distinct=min(E, 4))
+    layer = device_layer(be, router, gate, up, down, k)
+    x = rng.standard_normal((T, H)).astype(np.float32)
+    xd = torch.from_numpy(x).cuda()
+    idx, w = layer.route(xd)
+    ridx, rw = port.moe_route(x, router, k)
+    assert np.array_equal(idx.cpu().numpy().astype(np.uint32), ridx)
+    np.testing.assert_allclose(w.cpu().numpy(), rw, rtol=1e-5)
+    got = layer.forward(xd).clone()
+    single = torch.cat([layer.forward(xd[i:i + 1].contiguous()).clone() for i in range(T)])
+    be.device_status()
+    assert torch.equal(got.view(torch.int32), single.view(torch.int32))
+
+
+@pytest.mark.gpu
 @pytest.mark.parametrize("q,T,E,k", [("q4_0", 3, 8, 6), ("q4_0", 4, 8, 5), ("q4_K", 2, 16, 8), ("q4_K", 12, 128, 8),
                                      ("q4_K", 13, 128, 8)])
 def test_a_batch_equals_its_tokens_one_by_one_around_the_grouping_lines(be, q, T, E, k):
