@@ -376,12 +376,12 @@ size_t gemm_mma_q6_K_workspace_bytes(unsigned M, unsigned K);
 int launch_gemm_mma_q6_K(unsigned M, unsigned N, unsigned K, const float *A, const void *B, float *C, unsigned ldc, void *ws,
                          cudaStream_t st);
 /* per-expert grouped GEMM of the MoE prefill (gemm_mma.cu): (token, expert) pairs sorted by expert, position p of the
- * order being pair perm[p]; expert e has the positions off[e] .. off[e+1], the tiles tile_off[e] .. of tile_rows rows each
- * and the activation tiles act_off[e] .. of 8 rows each (rows: perm[p] / a_div of x); output row perm[p] * c_mul (+ 1 for
+ * order being pair perm[p], pair p (of token p / topk) being position inv[p]; expert e has the positions off[e] .. off[e+1], the tiles
+ * tile_off[e] .. of tile_rows rows each and the activation tiles act_off[e] .. of 8 rows each; output row perm[p] * c_mul (+ 1 for
  * w_table1). */
 int grouped_tile_rows(int qtype, unsigned pairs, unsigned n_experts);
-int launch_act_tiles_grouped(int qtype, const float *x, unsigned rows, unsigned K, void *act, const int *perm, const int *idx,
-                             const int *off, const int *act_off, int a_div, cudaStream_t st);
+int launch_act_tiles_grouped(int qtype, const float *x, unsigned tokens, unsigned topk, unsigned K, void *act, const int *inv, const int *idx,
+                             const int *off, const int *act_off, cudaStream_t st);
 int launch_gemm_grouped(int qtype, unsigned N, unsigned K, const void *act, float *C, unsigned ldc,
                         const void *const *w_table0, const void *const *w_table1, const int *off, const int *tile_off,
                         const int *act_off, const int *perm, int n_experts, int c_mul, int tile_rows, unsigned pairs,

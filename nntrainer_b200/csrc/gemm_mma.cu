@@ -899,43 +899,66 @@ __global__ void __launch_bounds__(KS_WARPS * 32, 2) gemm_mma_ksplit_kernel(const
 }
 
 /* ----------------------------------------------------- activation tiles */
-/** fp32 rows -> activation tiles; one warp per (row, unit). perm != nullptr: position p of an expert's range is the row
- *  perm[p] / a_div of x and goes to the expert's own tiles. */
-template <int QT>
-__global__ void __launch_bounds__(256)
-act_tiles_kernel(const float *__restrict__ x, int64_t ldx, uint8_t *__restrict__ act, int M, int M4, int nb, int K, int th,
-                 const int *__restrict__ perm, const int *__restrict__ idx, const int *__restrict__ off,
-                 const int *__restrict__ act_off, int a_div) {
-  pdl_launch_dependents();
-  const int lane = threadIdx.x & 31;
-  const int64_t w = (int64_t)blockIdx.x * 8 + (threadIdx.x >> 5);
-  if (w >= (int64_t)M * nb)
-    return;
-  const int pos = (int)(w / nb), b = (int)(w - (int64_t)pos * nb);
-  int row = pos, first = 0, n_tiles = (M + th - 1) / th, tile = pos / th, i = pos - tile * th;
-  if (perm) {
-    pdl_wait();
-    const int pair = perm[pos], e = idx[pair];
-    row = pair / a_div;
-    i = pos - off[e];
-    first = act_off[e];
-    n_tiles = (off[e + 1] - off[e] + 7) >> 3;
-    tile = i >> 3;
-    i &= 7;
-  }
-  uint8_t *unit = act_unit<QT>(act, first, n_tiles, tile, th, nb, b);
-  const float *src = x + (int64_t)row * ldx + (int64_t)b * QK_K + lane * 8;
+/** The 256 elements from element 256 * b of a row, a lane's eight of them quantized (rule: the quantizer's of Q4_K). */
+template <int QT> __device__ __forceinline__ auto quantize_unit(const float *row, int b, int K, int rule, int lane) {
+  const float *src = row + (int64_t)b * QK_K + lane * 8;
   if constexpr (QT == NNTR_Q4_K) {
-    put_q8K(unit, th, i, q8K_quantize_warp(*reinterpret_cast<const float4 *>(src), *reinterpret_cast<const float4 *>(src + 4),
-                                           lane, row < M4 ? 1 : 0),
-            lane);
+    return q8K_quantize_warp(*reinterpret_cast<const float4 *>(src), *reinterpret_cast<const float4 *>(src + 4), lane, rule);
   } else {
     float4 v0 = make_float4(0.f, 0.f, 0.f, 0.f), v1 = v0;
     if (b * QK_K + lane * 8 < K) { // blocks past K are zeros
       v0 = *reinterpret_cast<const float4 *>(src);
       v1 = *reinterpret_cast<const float4 *>(src + 4);
     }
-    put_q80(unit, th, i, q80_quantize_warp(v0, v1), lane);
+    return q80_quantize_warp(v0, v1);
+  }
+}
+/** fp32 rows -> activation tiles; one warp per (row, unit). */
+template <int QT>
+__global__ void __launch_bounds__(256)
+act_tiles_kernel(const float *__restrict__ x, int64_t ldx, uint8_t *__restrict__ act, int M, int M4, int nb, int K, int th) {
+  pdl_launch_dependents();
+  const int lane = threadIdx.x & 31;
+  const int64_t w = (int64_t)blockIdx.x * 8 + (threadIdx.x >> 5);
+  if (w >= (int64_t)M * nb)
+    return;
+  const int row = (int)(w / nb), b = (int)(w - (int64_t)row * nb), tile = row / th;
+  uint8_t *unit = act_unit<QT>(act, 0, (M + th - 1) / th, tile, th, nb, b);
+  const auto q = quantize_unit<QT>(x + (int64_t)row * ldx, b, K, row < M4 ? 1 : 0, lane);
+  if constexpr (QT == NNTR_Q4_K)
+    put_q8K(unit, th, row - tile * th, q, lane);
+  else
+    put_q80(unit, th, row - tile * th, q, lane);
+}
+/** The same for the rows of every expert: a token's row goes into the tiles of its topk experts. One warp per (token, unit), so that it
+ *  is quantized once and not once per expert (2048 rows of 2048 were 10.9 us of a layer's 200, cold). Lane k looks up where the
+ *  k-th copy goes. */
+template <int QT>
+__global__ void __launch_bounds__(256)
+act_tiles_grouped_kernel(const float *__restrict__ x, uint8_t *__restrict__ act, int T, int nb, int K, int topk, const int *__restrict__ inv,
+                         const int *__restrict__ idx, const int *__restrict__ off, const int *__restrict__ act_off) {
+  pdl_launch_dependents();
+  pdl_wait();
+  const int lane = threadIdx.x & 31;
+  const int64_t w = (int64_t)blockIdx.x * 8 + (threadIdx.x >> 5);
+  if (w >= (int64_t)T * nb)
+    return;
+  const int t = (int)(w / nb), b = (int)(w - (int64_t)t * nb);
+  int i = 0, first = 0, n_tiles = 0;
+  if (lane < topk) { // topk <= 32
+    const int e = idx[t * topk + lane], o = off[e];
+    i = inv[t * topk + lane] - o;
+    first = act_off[e];
+    n_tiles = (off[e + 1] - o + 7) >> 3;
+  }
+  const auto q = quantize_unit<QT>(x + (int64_t)t * K, b, K, 0, lane);
+  for (int k = 0; k < topk; ++k) {
+    const int row = __shfl_sync(FULL, i, k);
+    uint8_t *unit = act_unit<QT>(act, __shfl_sync(FULL, first, k), __shfl_sync(FULL, n_tiles, k), row >> 3, 8, nb, b);
+    if constexpr (QT == NNTR_Q4_K)
+      put_q8K(unit, 8, row & 7, q, lane);
+    else
+      put_q80(unit, 8, row & 7, q, lane);
   }
 }
 
@@ -1013,8 +1036,7 @@ int launch_gemm_mma(int qtype, unsigned M, unsigned M4, unsigned N, unsigned K, 
   a.th = M < 8 && ws_bytes < gemm_mma_workspace_bytes(qtype, M, K) ? (int)M : 8;
   const unsigned grid = (unsigned)(((int64_t)M * a.nb + 7) / 8);
   const auto quantize = qtype == NNTR_Q4_K ? act_tiles_kernel<NNTR_Q4_K> : act_tiles_kernel<NNTR_Q4_0>;
-  quantize<<<grid, 256, 0, st>>>(A, K, static_cast<uint8_t *>(ws), a.M, a.M4, a.nb, (int)K, a.th, nullptr, nullptr, nullptr,
-                                 nullptr, 1);
+  quantize<<<grid, 256, 0, st>>>(A, K, static_cast<uint8_t *>(ws), a.M, a.M4, a.nb, (int)K, a.th);
   count_launch();
   NNTR_CHECK_CUDA(cudaGetLastError());
   // Weights that are not 16-byte aligned cannot be fetched by bulk copies: the shared tile has 8-byte copies for them.
@@ -1056,13 +1078,13 @@ int grouped_tile_rows(int qtype, unsigned pairs, unsigned n_experts) {
   return qtype == NNTR_Q4_K ? (pairs <= 14 * n_experts ? 16 : 32) : (pairs <= 6 * n_experts ? 8 : 32);
 }
 
-int launch_act_tiles_grouped(int qtype, const float *x, unsigned rows, unsigned K, void *act, const int *perm, const int *idx,
-                             const int *off, const int *act_off, int a_div, cudaStream_t st) {
+int launch_act_tiles_grouped(int qtype, const float *x, unsigned tokens, unsigned topk, unsigned K, void *act, const int *inv, const int *idx,
+                             const int *off, const int *act_off, cudaStream_t st) {
   const int nb = (int)((K + 255) / 256);
-  const dim3 grid((unsigned)(((int64_t)rows * nb + 7) / 8));
-  const auto kernel = qtype == NNTR_Q4_K ? act_tiles_kernel<NNTR_Q4_K> : act_tiles_kernel<NNTR_Q4_0>;
-  const cudaError_t e = launch(kernel, grid, 256, 0, st, x, (int64_t)K, static_cast<uint8_t *>(act), (int)rows, 0, nb, (int)K,
-                               8, perm, idx, off, act_off, a_div);
+  const dim3 grid((unsigned)(((int64_t)tokens * nb + 7) / 8));
+  const auto kernel = qtype == NNTR_Q4_K ? act_tiles_grouped_kernel<NNTR_Q4_K> : act_tiles_grouped_kernel<NNTR_Q4_0>;
+  const cudaError_t e = launch(kernel, grid, 256, 0, st, x, static_cast<uint8_t *>(act), (int)tokens, nb, (int)K, (int)topk, inv, idx, off,
+                               act_off);
   count_launch();
   return check_cuda(e, "activation tiles launch");
 }

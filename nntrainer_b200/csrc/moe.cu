@@ -388,10 +388,10 @@ moe_router_rows_kernel(const float *__restrict__ x, const float *__restrict__ wr
   const int rows = s1 - s0;
   float *xs = rsm + ROUTER_WARPS * TT * E;
   pdl_wait();
-  for (int i = threadIdx.x; i < TT * rows; i += ROUTER_WARPS * 32) {
-    const int k = i / rows, h = i - k * rows;
-    xs[i] = t0 + k < T ? x[(size_t)(t0 + k) * H + s0 + h] : 0.f;
-  }
+  constexpr int SHARE = ROUTER_WARPS / TT; // warps per token outside the products: no division by a run-time number in these loops
+  const int my = warp / SHARE, from = lane + 32 * (warp % SHARE);
+  for (int h = from; h < rows; h += 32 * SHARE)
+    xs[my * rows + h] = t0 + my < T ? x[(size_t)(t0 + my) * H + s0 + h] : 0.f;
   float acc[TT][PER];
 #pragma unroll
   for (int k = 0; k < TT; ++k)
@@ -426,16 +426,14 @@ moe_router_rows_kernel(const float *__restrict__ x, const float *__restrict__ wr
       if (lane + 32 * i < E)
         rsm[(warp * TT + k) * E + lane + 32 * i] = acc[k][i];
   __syncthreads();
-  for (int i = threadIdx.x; i < TT * E; i += ROUTER_WARPS * 32) {
-    const int k = i / E, e = i - k * E;
-    if (t0 + k >= T)
-      break;
-    float s = 0.f;
+  if (t0 + my < T)
+    for (int e = from; e < E; e += 32 * SHARE) {
+      float s = 0.f;
 #pragma unroll
-    for (int w = 0; w < ROUTER_WARPS; ++w)
-      s += rsm[(w * TT + k) * E + e];
-    o.rpart[((size_t)(t0 + k) * ROUTER_SLICES + sl) * E + e] = s;
-  }
+      for (int w = 0; w < ROUTER_WARPS; ++w)
+        s += rsm[(w * TT + my) * E + e];
+      o.rpart[((size_t)(t0 + my) * ROUTER_SLICES + sl) * E + e] = s;
+    }
   __threadfence();
   __syncthreads();
   if (threadIdx.x == 0) {
@@ -454,11 +452,11 @@ moe_router_rows_kernel(const float *__restrict__ x, const float *__restrict__ wr
 
 /* Sorts the (token, expert) pairs of a batch by expert: off[e] = first position of expert e's pairs in perm, tile_off[e]
  * = first tile of tile_rows rows of expert e, act_off[e] = its first activation tile of 8 rows, perm = pair indices grouped by expert (order inside an expert is
- * arbitrary: every row of the grouped GEMM is computed on its own). One CTA; the pair list of a prefill is a few
+ * arbitrary: every row of the grouped GEMM is computed on its own), inv[pair] = the pair's position in it. One CTA; the pair list of a prefill is a few
  * thousand entries. E <= 256 = one expert per lane of the first eight warps, so the two prefix sums are warp scans. */
 __global__ void __launch_bounds__(1024) moe_permute_kernel(const int *__restrict__ idx, int P, int E, int tile_rows,
                                                           int *__restrict__ off, int *__restrict__ tile_off,
-                                                          int *__restrict__ act_off, int *__restrict__ perm) {
+                                                          int *__restrict__ act_off, int *__restrict__ perm, int *__restrict__ inv) {
   __shared__ int cnt[256], cur[256], sums[3][8];
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   if (tid < 256)
@@ -504,8 +502,11 @@ __global__ void __launch_bounds__(1024) moe_permute_kernel(const int *__restrict
     }
   }
   __syncthreads();
-  for (int p = tid; p < P; p += blockDim.x)
-    perm[atomicAdd(&cur[idx[p]], 1)] = p;
+  for (int p = tid; p < P; p += blockDim.x) {
+    const int pos = atomicAdd(&cur[idx[p]], 1);
+    perm[pos] = p;
+    inv[p] = pos;
+  }
 }
 
 /* The activation between the grouped GEMMs, quantized for the second one: position p of the sorted pairs, unit b of 256
@@ -851,12 +852,13 @@ static int moe_forward(const nntr_moe_desc *d, const nntr_moe_ep *epd, unsigned 
      * for gate and up, activation and its quantization, one grouped GEMM for down, combine. Same bits as the per-pair
      * GEMVs. */
     int *off = reinterpret_cast<int *>(ws + s.off), *tile_off = reinterpret_cast<int *>(ws + s.tile_off),
-        *act_off = reinterpret_cast<int *>(ws + s.act_off), *perm = reinterpret_cast<int *>(ws + s.perm);
+        *act_off = reinterpret_cast<int *>(ws + s.act_off), *perm = reinterpret_cast<int *>(ws + s.perm),
+        *inv = reinterpret_cast<int *>(ws + s.gu_tab); // in the place of the per-pair launches' weight table, which nothing reads here
     const int tile_rows = grouped_tile_rows(d->qtype, P, E);
     NNTR_CHECK_CUDA(launch_pdl(moe_permute_kernel, 1u, 1024u, st, idx, (int)P, (int)E, tile_rows, off, tile_off, act_off,
-                               perm));
+                               perm, inv));
     count_launch();
-    int rc2 = launch_act_tiles_grouped(d->qtype, x, P, H, ws + s.qx, perm, idx, off, act_off, (int)K, st);
+    int rc2 = launch_act_tiles_grouped(d->qtype, x, tokens, K, H, ws + s.qx, inv, idx, off, act_off, st);
     if (rc2)
       return rc2;
     if ((rc2 = launch_gemm_grouped(d->qtype, I, H, ws + s.qx, gu, I, d->gate_w, d->up_w, off, tile_off, act_off, perm, (int)E, 2,
