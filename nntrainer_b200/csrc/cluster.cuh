@@ -75,9 +75,7 @@ __device__ __forceinline__ uint32_t neighbour_raised(uint32_t flag, int lane) {
 }
 
 /** Launch of a grid of grid.x * parts by grid.y CTAs in clusters of `parts` CTAs along x. The grid may start before its
- *  predecessor is done: the kernel calls pdl_wait() before it touches what that wrote. (A predecessor that does not release its
- *  dependents itself, as the tile quantizers in front of the tensor GEMMs, does so when its last CTA ends: what is saved then is
- *  the launch, not the prologue.) */
+ *  predecessor is done: the kernel calls pdl_wait() before it touches what that wrote. */
 template <typename... P, typename... A>
 cudaError_t launch_in_clusters(void (*kernel)(P...), dim3 grid, int parts, int threads, int smem, cudaStream_t st, A... args) {
   cudaLaunchAttribute attr[2];

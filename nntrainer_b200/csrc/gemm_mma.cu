@@ -465,6 +465,8 @@ __global__ void __launch_bounds__(ROWS_WARPS * 32 + 32, rows_ctas<QT, NT, GROUPE
   __syncthreads();
   if (GROUPED)
     pdl_wait(); // tables and activation tiles come from the kernels before
+  else // (grouped, the next launch's CTAs would be let in beside the products: 64 tokens, 8 of 128 experts 113 -> 132 us)
+    pdl_launch_dependents();
   int slot = 0;
   uint32_t par = 0;
   bool ok = true;
@@ -707,8 +709,10 @@ __global__ void __launch_bounds__(KS_WARPS * 32, 2) gemm_mma_ksplit_kernel(const
   else if (tid == 0)
     for (int rd = 0; rd < KS_RING && rd < per; ++rd)
       fetch(rd, rd);
-  if (!GROUPED)
+  if (!GROUPED) {
     pdl_wait();
+    pdl_launch_dependents();
+  }
   __syncthreads();
   const int nt = (tl.rows + 7) >> 3, th = TH8 ? 8 : a.th;
   using Act = std::conditional_t<QT == NNTR_Q4_K, ActQ4K, ActQ40>;
@@ -917,7 +921,8 @@ template <int QT> __device__ __forceinline__ auto quantize_unit(const float *row
 template <int QT>
 __global__ void __launch_bounds__(256)
 act_tiles_kernel(const float *__restrict__ x, int64_t ldx, uint8_t *__restrict__ act, int M, int M4, int nb, int K, int th) {
-  pdl_launch_dependents();
+  pdl_wait();
+  pdl_launch_dependents(); // the GEMM behind fetches weights, which a kernel in front of this one may have written, and waits for the rest
   const int lane = threadIdx.x & 31;
   const int64_t w = (int64_t)blockIdx.x * 8 + (threadIdx.x >> 5);
   if (w >= (int64_t)M * nb)
@@ -1036,9 +1041,8 @@ int launch_gemm_mma(int qtype, unsigned M, unsigned M4, unsigned N, unsigned K, 
   a.th = M < 8 && ws_bytes < gemm_mma_workspace_bytes(qtype, M, K) ? (int)M : 8;
   const unsigned grid = (unsigned)(((int64_t)M * a.nb + 7) / 8);
   const auto quantize = qtype == NNTR_Q4_K ? act_tiles_kernel<NNTR_Q4_K> : act_tiles_kernel<NNTR_Q4_0>;
-  quantize<<<grid, 256, 0, st>>>(A, K, static_cast<uint8_t *>(ws), a.M, a.M4, a.nb, (int)K, a.th);
+  NNTR_CHECK_CUDA(launch(quantize, dim3(grid), 256, 0, st, A, (int64_t)K, static_cast<uint8_t *>(ws), a.M, a.M4, a.nb, (int)K, a.th));
   count_launch();
-  NNTR_CHECK_CUDA(cudaGetLastError());
   // Weights that are not 16-byte aligned cannot be fetched by bulk copies: the shared tile has 8-byte copies for them.
   const bool misaligned = reinterpret_cast<uintptr_t>(B) & 15;
   const unsigned row_tiles = (N + 15) / 16, row_blocks = (N + 63) / 64, sms = (unsigned)sm_count();

@@ -26,6 +26,7 @@
  * half rate both): 8 x 151936 x 2560 129 us (CUDA-core kernel before: 697; the weights' bytes alone take 49), 31 rows 339 us
  * (2360). Bringing the rows in by 4- and 8-byte asynchronous copies or through registers measured the same or slower.
  */
+#include "cluster.cuh"
 #include "common.cuh"
 #include "pipeline.cuh"
 
@@ -113,6 +114,7 @@ gemm_q6_K_mma_kernel(const uint8_t *__restrict__ act, const uint8_t *__restrict_
   for (int b = 0; b < Q6M_STAGES - 1 && b < nb; ++b) // the weights do not depend on the kernel before
     fetch(b);
   pdl_wait(); // the activation tiles do
+  pdl_launch_dependents();
   float acc[NT][8][4];
 #pragma unroll
   for (int i = 0; i < NT; ++i)
@@ -262,7 +264,8 @@ gemm_q6_K_mma_kernel(const uint8_t *__restrict__ act, const uint8_t *__restrict_
 /** fp32 rows -> the activation tiles above; one warp per (row, super-block). */
 __global__ void __launch_bounds__(256)
 act_tiles_q6_kernel(const float *__restrict__ x, int64_t ldx, uint8_t *__restrict__ act, int M, int nb) {
-  pdl_launch_dependents();
+  pdl_wait();
+  pdl_launch_dependents(); // the GEMM behind fetches weights, which a kernel in front of this one may have written, and waits for the rest
   const int lane = threadIdx.x & 31;
   const int64_t w = (int64_t)blockIdx.x * 8 + (threadIdx.x >> 5);
   if (w >= (int64_t)M * nb)
@@ -294,9 +297,9 @@ int launch_gemm_mma_q6_K(unsigned M, unsigned N, unsigned K, const float *A, con
   if ((reinterpret_cast<uintptr_t>(A) & 15) || (reinterpret_cast<uintptr_t>(ws) & 15) || (reinterpret_cast<uintptr_t>(B) & 1))
     return set_error(NNTR_CUDA_ERR_INVALID, "gemm_q6_K: misaligned pointer");
   const int nb = (int)(K / QK_K);
-  act_tiles_q6_kernel<<<(unsigned)(((int64_t)M * nb + 7) / 8), 256, 0, st>>>(A, K, static_cast<uint8_t *>(ws), (int)M, nb);
+  NNTR_CHECK_CUDA(launch_in_clusters(act_tiles_q6_kernel, dim3((unsigned)(((int64_t)M * nb + 7) / 8)), 1, 256, 0, st, A, (int64_t)K,
+                                     static_cast<uint8_t *>(ws), (int)M, nb));
   count_launch();
-  NNTR_CHECK_CUDA(cudaGetLastError());
   const unsigned nt = M <= 8 ? 1 : 2;
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3((M + 8 * nt - 1) / (8 * nt), ((N + 15) / 16 + Q6M_WARPS - 1) / Q6M_WARPS);

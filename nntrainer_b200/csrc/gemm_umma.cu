@@ -182,6 +182,7 @@ gemm_q4_K_umma_kernel(const uint8_t *__restrict__ atiles, const BlockQ4Kx8 *__re
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
+  pdl_launch_dependents();
   const uint32_t tmem = *tmem_slot;
   constexpr int SUM_PITCH = TILE_N + 4; // floats
   bool tile_done = false;               // drain warps of a shared tile: all sums in shared memory
@@ -420,6 +421,8 @@ gemm_q4_K_umma_kernel(const uint8_t *__restrict__ atiles, const BlockQ4Kx8 *__re
 __global__ void __launch_bounds__(256)
 quantize_q8_K_tiles_kernel(const float *__restrict__ x, int64_t ldx, uint8_t *__restrict__ tiles, int M, int M4,
                            int Mpad, int nb) {
+  pdl_wait();
+  pdl_launch_dependents(); // the GEMM behind fetches weights, which a kernel in front of this one may have written, and waits for the rest
   const int lane = threadIdx.x & 31;
   const int64_t blk = (int64_t)blockIdx.x * 8 + (threadIdx.x >> 5);
   if (blk >= (int64_t)Mpad * nb)
@@ -475,10 +478,9 @@ int launch_gemm_q4_K_umma(unsigned M, unsigned N, unsigned K, const float *A, co
   if ((reinterpret_cast<uintptr_t>(A) & 15) || (reinterpret_cast<uintptr_t>(ws) & 15))
     return set_error(NNTR_CUDA_ERR_INVALID, "gemm (tensor path): activations and workspace must be 16-byte aligned");
   const int64_t nwarps = (int64_t)Mpad * nb;
-  quantize_q8_K_tiles_kernel<<<(unsigned)((nwarps + 7) / 8), 256, 0, st>>>(A, K, static_cast<uint8_t *>(ws), (int)M,
-                                                                         (int)M4, Mpad, nb);
+  NNTR_CHECK_CUDA(launch_in_clusters(quantize_q8_K_tiles_kernel, dim3((unsigned)((nwarps + 7) / 8)), 1, 256, 0, st, A, (int64_t)K,
+                                     static_cast<uint8_t *>(ws), (int)M, (int)M4, Mpad, nb));
   count_launch();
-  NNTR_CHECK_CUDA(cudaGetLastError());
   const int c_vec4 = (ldc % 4 == 0) && !(reinterpret_cast<uintptr_t>(C) & 15);
   dim3 grid(mtiles, N / TILE_N);
   // Few tiles: K in as many parts as run in one wave of clusters. A CTA alone walks K at 2.5 us a super-block however many SMs

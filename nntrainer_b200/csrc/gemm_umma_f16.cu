@@ -261,6 +261,8 @@ gemm_f16_kernel(const __grid_constant__ CUtensorMap wmap, const uint8_t *__restr
   __syncthreads();
   if (PAIR)
     cluster_sync(); // the other CTA's barriers and tensor memory are there
+  if (!SHARED) // (shared tiles: 1024 x 2560 x 9728 85.0 us instead of 83.6)
+    pdl_launch_dependents();
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
   const uint32_t tmem = *tmem_slot;
 
@@ -660,6 +662,8 @@ gemm_f16_kernel(const __grid_constant__ CUtensorMap wmap, const uint8_t *__restr
 __global__ void __launch_bounds__(256)
 quantize_q8_K_f16_tiles_kernel(const float *__restrict__ x, int64_t ldx, uint8_t *__restrict__ tiles, int M, int M4,
                                int Mpad, int nb, int q6_order) {
+  pdl_wait();
+  pdl_launch_dependents(); // the GEMM behind fetches weights, which a kernel in front of this one may have written, and waits for the rest
   const int lane = threadIdx.x & 31;
   const int64_t blk = (int64_t)blockIdx.x * 8 + (threadIdx.x >> 5);
   if (blk >= (int64_t)Mpad * nb)
@@ -709,6 +713,8 @@ quantize_q8_K_f16_tiles_kernel(const float *__restrict__ x, int64_t ldx, uint8_t
 __global__ void __launch_bounds__(256)
 quantize_q8_0_f16_tiles_kernel(const float *__restrict__ x, int64_t ldx, uint8_t *__restrict__ tiles, int M, int Mpad,
                                int K) {
+  pdl_wait();
+  pdl_launch_dependents(); // the GEMM behind fetches weights, which a kernel in front of this one may have written, and waits for the rest
   const int lane = threadIdx.x & 31;
   const int nu = (K + 255) / 256, n_stages = K / 64;
   const int64_t unit = (int64_t)blockIdx.x * 8 + (threadIdx.x >> 5);
@@ -863,16 +869,15 @@ int launch_gemm_f16(int qtype, unsigned M, unsigned N, unsigned K, const float *
     // (ggml_interface_omp.cpp:545-551)
     const unsigned M4 = qtype == NNTR_Q4_K ? (M / 4) * 4 : 0;
     const int64_t nwarps = (int64_t)Mpad * nb;
-    quantize_q8_K_f16_tiles_kernel<<<(unsigned)((nwarps + 7) / 8), 256, 0, st>>>(A, K, tiles, (int)M, (int)M4, Mpad, nb,
-                                                                               qtype == NNTR_Q6_K);
+    NNTR_CHECK_CUDA(launch_in_clusters(quantize_q8_K_f16_tiles_kernel, dim3((unsigned)((nwarps + 7) / 8)), 1, 256, 0, st, A, (int64_t)K, tiles,
+                                       (int)M, (int)M4, Mpad, nb, (int)(qtype == NNTR_Q6_K)));
     count_launch();
-    NNTR_CHECK_CUDA(cudaGetLastError());
     rc = qtype == NNTR_Q4_K ? launch_typed<NNTR_Q4_K>(M, N, K, tiles, B, C, ldc, st) : launch_typed<NNTR_Q6_K>(M, N, K, tiles, B, C, ldc, st);
   } else {
     const int64_t nwarps = (int64_t)Mpad * ((K + 255) / 256);
-    quantize_q8_0_f16_tiles_kernel<<<(unsigned)((nwarps + 7) / 8), 256, 0, st>>>(A, K, tiles, (int)M, Mpad, (int)K);
+    NNTR_CHECK_CUDA(launch_in_clusters(quantize_q8_0_f16_tiles_kernel, dim3((unsigned)((nwarps + 7) / 8)), 1, 256, 0, st, A, (int64_t)K, tiles,
+                                       (int)M, Mpad, (int)K));
     count_launch();
-    NNTR_CHECK_CUDA(cudaGetLastError());
     rc = launch_typed<NNTR_Q4_0>(M, N, K, tiles, B, C, ldc, st);
   }
   if (rc)
