@@ -35,7 +35,6 @@ namespace nntr {
 namespace {
 
 constexpr int Q6M_WARPS = 4;
-constexpr int Q6M_STAGES = 3;
 constexpr int Q6M_COPY = 224;     // 16-byte aligned bytes around a block
 constexpr int Q6M_ROW_WORDS = 60; // 4 more: neighbouring rows fall into different banks
 constexpr uint32_t Q6M_POLLS = 1u << 22;
@@ -70,15 +69,22 @@ constexpr int LUT_SELECT = 0xE4;  // (a & c) | (b & ~c)
 constexpr int LUT_AND_OR = 0xEA;  // (a & b) | c
 constexpr int LUT_AND_XOR = 0x6A; // (a & b) ^ c
 
-template <int NT>
-__global__ void __launch_bounds__(Q6M_WARPS * 32, 3)
+/* CTAS: CTAs per SM that registers and shared memory are held to. Four with 4 bytes of spills and two stages (which leave the L1
+ * cache room for the activations; with three stages 137 us instead of 122 for 8 x 151936 x 2560, three CTAs of three stages 128), where
+ * three per SM would need a second round. */
+template <int CTAS> constexpr int Q6M_STAGES = CTAS == 4 ? 2 : 3;
+template <int NT, int CTAS>
+__global__ void __launch_bounds__(Q6M_WARPS * 32, CTAS)
 gemm_q6_K_mma_kernel(const uint8_t *__restrict__ act, const uint8_t *__restrict__ W, float *__restrict__ C, int ldc, int M,
                      int N, int nb) {
   // High nibbles used where they lie, with their own factors: the same number of operations, 187 against 193 us for 16 x 151936 x
   // 2560 and 338 against 346 for 31 rows; with one tile of rows 130 against 128 and 32.4 against 30.3 for 5 x 4096 x 4096.
   constexpr bool IN_PLACE = NT == 2;
-  __shared__ alignas(16) uint32_t stage[Q6M_WARPS][Q6M_STAGES][Q6M_STAGE_WORDS];
-  __shared__ alignas(8) unsigned long long bars[Q6M_WARPS][Q6M_STAGES];
+  constexpr int STAGES = Q6M_STAGES<CTAS>;
+  // a shift less per word of high bits (1 % with four CTAs); with three, where a warp's own latency counts, 5 x 4096 x 4096 31.7 us instead of 30.0
+  constexpr bool DENSE = NT == 1 && CTAS == 4;
+  __shared__ alignas(16) uint32_t stage[Q6M_WARPS][STAGES][Q6M_STAGE_WORDS];
+  __shared__ alignas(8) unsigned long long bars[Q6M_WARPS][STAGES];
   __shared__ int aborted[Q6M_WARPS]; // one per warp: the warps of a CTA do not meet
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, g = lane >> 2, t = lane & 3, run = t & 1, h = t >> 1;
   const int n0 = (blockIdx.y * Q6M_WARPS + warp) * 16, m0 = blockIdx.x * 8 * NT;
@@ -91,7 +97,7 @@ gemm_q6_K_mma_kernel(const uint8_t *__restrict__ act, const uint8_t *__restrict_
   const uint32_t sm = smem_u32(stage[warp][0]), bar = smem_u32(bars[warp]);
   volatile int *abort_flag = &aborted[warp];
   if (lane == 0) {
-    for (int k = 0; k < Q6M_STAGES; ++k)
+    for (int k = 0; k < STAGES; ++k)
       mbar_init(bar + 8 * k, 1);
     *abort_flag = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -102,7 +108,7 @@ gemm_q6_K_mma_kernel(const uint8_t *__restrict__ act, const uint8_t *__restrict_
   // that holds the block's own first or last byte.
   const uint8_t *mine = W + (size_t)min(n0 + (lane & 15), N - 1) * row_bytes;
   auto fetch = [&](int b) {
-    const int k = b % Q6M_STAGES;
+    const int k = b % STAGES;
     if (lane == 0)
       mbar_expect_tx(bar + 8 * k, 16 * Q6M_COPY);
     __syncwarp();
@@ -111,7 +117,7 @@ gemm_q6_K_mma_kernel(const uint8_t *__restrict__ act, const uint8_t *__restrict_
                reinterpret_cast<const void *>(reinterpret_cast<uintptr_t>(mine + (size_t)b * sizeof(BlockQ6K)) & ~(uintptr_t)15),
                Q6M_COPY, bar + 8 * k);
   };
-  for (int b = 0; b < Q6M_STAGES - 1 && b < nb; ++b) // the weights do not depend on the kernel before
+  for (int b = 0; b < STAGES - 1 && b < nb; ++b) // the weights do not depend on the kernel before
     fetch(b);
   pdl_wait(); // the activation tiles do
   pdl_launch_dependents();
@@ -129,12 +135,12 @@ gemm_q6_K_mma_kernel(const uint8_t *__restrict__ act, const uint8_t *__restrict_
                  a1 = (uint32_t)(reinterpret_cast<uintptr_t>(W) + (size_t)min(n0 + g + 8, N - 1) * row_bytes);
   bool ok = true;
   for (int b = 0; b < nb; ++b) {
-    ok = mbar_wait_bounded(bar + 8 * (b % Q6M_STAGES), (b / Q6M_STAGES) & 1, abort_flag, &g_q6m_status, Q6M_POLLS, 2048);
+    ok = mbar_wait_bounded(bar + 8 * (b % STAGES), (b / STAGES) & 1, abort_flag, &g_q6m_status, Q6M_POLLS, 2048);
     if (!(ok = __all_sync(FULL, ok)))
       break;
-    if (b + Q6M_STAGES - 1 < nb) // into the slot that was read in the previous round
-      fetch(b + Q6M_STAGES - 1);
-    const uint32_t *st = stage[warp][b % Q6M_STAGES];
+    if (b + STAGES - 1 < nb) // into the slot that was read in the previous round
+      fetch(b + STAGES - 1);
+    const uint32_t *st = stage[warp][b % STAGES];
     uint32_t sh[2];
     const uint32_t *row[2];
     float d[NT][4];
@@ -193,7 +199,9 @@ gemm_q6_K_mma_kernel(const uint8_t *__restrict__ act, const uint8_t *__restrict_
 #pragma unroll
         for (int r = 0; r < 2; ++r) {
           const uint32_t ql1 = row[r][8 * t + l + 1], qh1 = row[r][32 + 8 * h + l + 1];
-          const uint32_t lw = __funnelshift_r(ql[r], ql1, sh[r]), hw = __funnelshift_r(qh[r], qh1, sh[r]);
+          const uint32_t lw = __funnelshift_r(ql[r], ql1, sh[r]);
+          // DENSE: bits 2 run and up of the word, so that the low quarter's lie four places lower than they are put
+          const uint32_t hw = __funnelshift_r(qh[r], qh1, DENSE ? sh[r] + 2 * run : sh[r]);
           ql[r] = ql1;
           qh[r] = qh1;
           __half2 q0[2], q1[2]; // of the two quarters: bytes 0, 2 and 1, 3 as halves 1024 + q
@@ -207,7 +215,7 @@ gemm_q6_K_mma_kernel(const uint8_t *__restrict__ act, const uint8_t *__restrict_
 #pragma unroll
             for (int k = 0; k < 2; ++k) {
               // low nibbles of one word, above them the bits of the other (bits 6 and 7 of the bytes are masked off below)
-              const uint32_t n = k ? lw >> 4 : lw, up = k ? hw >> (2 * run) : hw << (4 - 2 * run);
+              const uint32_t n = k ? lw >> 4 : lw, up = DENSE ? (k ? hw : hw << 4) : k ? hw >> (2 * run) : hw << (4 - 2 * run);
               const uint32_t q = lop3<LUT_SELECT>(n, up, 0x0f0f0f0fu);
               q0[k] = u2h(lop3<LUT_AND_OR>(q, 0x003f003fu, 0x64006400u));
               q1[k] = u2h(lop3<LUT_AND_OR>(q >> 8, 0x003f003fu, 0x64006400u));
@@ -310,7 +318,12 @@ int launch_gemm_mma_q6_K(unsigned M, unsigned N, unsigned K, const float *A, con
   attr[0].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
   cfg.numAttrs = 1;
-  const cudaError_t e = cudaLaunchKernelEx(&cfg, nt == 1 ? gemm_q6_K_mma_kernel<1> : gemm_q6_K_mma_kernel<2>,
+  // one tile of rows: four CTAs per SM where three would not hold them all (8 x 32768 x 4096 61.2 -> 50.2 us, 8 x 151936 x 2560 128.2 ->
+  // 122.5; 64 CTAs, 5 x 4096 x 4096, 36.9 instead of 30.0)
+  const bool dense = nt == 1 && cfg.gridDim.x * cfg.gridDim.y > 3u * (unsigned)sm_count();
+  const cudaError_t e = cudaLaunchKernelEx(&cfg, dense     ? gemm_q6_K_mma_kernel<1, 4>
+                                                 : nt == 1 ? gemm_q6_K_mma_kernel<1, 3>
+                                                           : gemm_q6_K_mma_kernel<2, 3>,
                                            static_cast<const uint8_t *>(ws), static_cast<const uint8_t *>(B), C, (int)ldc,
                                            (int)M, (int)N, nb);
   count_launch();
