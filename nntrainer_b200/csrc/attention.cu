@@ -23,6 +23,7 @@
  *
  * Cache layout as the reference's: [row][kv head][head_dim] fp16, one row per position.
  */
+#include <algorithm>
 #include <atomic>
 
 #include "cluster.cuh"
@@ -433,7 +434,8 @@ __global__ void attn_values_kernel(const float *__restrict__ probs, const uint16
  *   softmax  a CTA owns one head (or 64 of its dimensions): maximum, exponentials and division by all threads, the sum in
  *            ascending row order by one warp (ordered_sum).
  *   values   a thread per dimension runs the row-ordered chain over value tiles that a producer warp keeps ahead of it
- *            (tiled TMA copies, started before the scores).
+ *            (tiled TMA copies, started before the scores). CTAs of 32 dimensions (long windows): six warps turn the tiles round, and
+ *            the chain loads eight rows of its dimension at once: at 4096 rows 27700 clocks instead of 33300, the launch 33.5 us.
  * Clock stamps of one CTA, 64 / 8 heads of 64, at 512 / 4096 rows, in clocks: up to the grid dependency 1800 / 1850, first copies and
  * heads rotated 1350 / 1450, wait for the cluster 400, score tiles 1600 / 8800, barrier behind them 2050 / 2600, maximum and
  * exponentials 1500 / 3800, ordered sum 2500 / 11500, division 450 / 1450, value chain 5400 / 33800. The value chain is half of a long
@@ -441,20 +443,28 @@ __global__ void attn_values_kernel(const float *__restrict__ probs, const uint16
  * takes four. In a decode step, whose launches find neither code nor caches at hand, the phases up to 512 rows take half as long again
  * (32 / 8 heads of 128 at 100 rows 14300 clocks behind the dependency, alone 8900). 64 / 8 heads of 64 at 4096 rows 36.5 us, 32 / 8 heads
  * of 128 at 512 rows 11.2 us (with generic accesses to the tiles, and value tiles of 128 rows: 45 and 12.3), at 128 rows of a window
- * 8.0 us with the copy of q (8.4). Measured and not kept: value tiles turned round by the idle warps
- * for 16-byte loads (46 us), half of the ring waited for at a time (44), four blocks of the ordered sum at once (16900 clocks
- * instead of 11500), two rows and two heads per thread in the scores (heads of 64: 1800 a tile instead of 1900; of 128: 2660
- * instead of 2200).
+ * 8.0 us with the copy of q (8.4). Measured and not kept: eight rows at a time with twenty-four more on their way (40.7 us, sixteen and
+ * sixteen 36.6: a warp waits for its loads by few counters), half of the ring waited for at a time (44), four blocks of the ordered sum
+ * at once (16900 clocks instead of 11500), the integers of all blocks of 32 rows by all warps beforehand (2 us more at 4096 rows), two rows
+ * and two heads per thread in the scores (heads of 64: 1800 a tile instead of 1900; of 128: 2660 instead of 2200).
  * Ring positions are counted, not divided: an integer division in a loop that one thread runs costs more than a tile's copy. */
 constexpr int AC_THREADS = 256;
 constexpr int AC_WARPS = AC_THREADS / 32;
-constexpr int AC_TILE = 128; // cache rows per tile of keys
+/** cache rows per tile of keys: 32 rows and one or two heads for each warp */
+template <int DIMS> constexpr int AC_KROWS = DIMS == 32 ? 256 : 128;
 constexpr uint32_t AC_SMEM_ALONE = 200u * 1024u; // beside which an SM has room for launches of up to about 26 KB only
 constexpr int AC_KBUF_MAX = 4;
 constexpr int AC_VBUF_MAX = 6;
 /** cache rows per tile of values: a wait for a tile costs 350 clocks of the chain */
-template <int DIMS> constexpr int AC_VROWS = DIMS == 64 ? 256 : 128;
+template <int DIMS> constexpr int AC_VROWS = DIMS <= 64 ? 256 : 128;
 constexpr unsigned AC_MAX_ROWS = 16384; // rows of one head kept as floats in shared memory
+/* CTAs of 32 dimensions: the warps between the first, which runs the value chain, and the last, which starts copies, turn the value tiles
+ * round, so that the chain loads eight rows of its dimension at once. */
+constexpr int AC_TURNERS = AC_WARPS - 2;
+constexpr unsigned AC_SLICED_ROWS = 1400;
+constexpr int AC_TBUF_MAX = 4;
+constexpr int AC_TPITCH = 2 * 256 + 16; // bytes of a dimension's rows in a turned tile: 16-byte pieces of neighbours in different banks
+constexpr uint32_t AC_TBYTES = 32 * AC_TPITCH;
 constexpr uint32_t AC_POLLS = 1u << 22;
 __device__ int g_attn_status = 0; // raised when a bounded wait for a tile runs out
 
@@ -474,7 +484,7 @@ struct AttnStep {
   int hq, hkv, hd;
   int groups; // clusters per kv head: more than eight query heads per kv head are split over several
   int rope;   // 0: q is rotated already and the token's rows are in the caches
-  int k_bufs, v_bufs;
+  int k_bufs, v_bufs, t_bufs; // tiles of keys, of values, turned ones of values
   unsigned tokens;   // consecutive tokens (blockIdx.y), q_ld and out_ld elements apart; their rows are in the caches
   long long q_ld, out_ld;
   int k_box, v_box; // rows a copy brings: a tile, fewer where one short tile is all there is
@@ -488,13 +498,15 @@ __device__ __forceinline__ void st_cluster(uint32_t addr, uint32_t rank, float v
 }
 
 struct AcLayout {
-  uint32_t ktile, vtile, e, q, total; // offsets; the tiles are 1024-byte aligned
+  uint32_t ktile, vtile, e, q, total; // offsets; the tiles are 1024-byte aligned; turned values take the keys' place
 };
-__host__ __device__ inline AcLayout ac_layout(int gqa, int hd, int dims, int k_bufs, int v_bufs, int v_box, unsigned cap_rows) {
+__host__ __device__ inline AcLayout ac_layout(int gqa, int hd, int dims, int k_rows, int k_bufs, int v_bufs, int t_bufs, int v_box, unsigned cap_rows) {
   AcLayout L;
   uint32_t o = 0;
   L.ktile = o;
-  o += (uint32_t)k_bufs * (uint32_t)((hd + 63) / 64) * AC_TILE * 128;
+  o += (uint32_t)k_bufs * (uint32_t)((hd + 63) / 64) * k_rows * 128;
+  if (o < (uint32_t)t_bufs * AC_TBYTES)
+    o = ((uint32_t)t_bufs * AC_TBYTES + 1023u) & ~1023u;
   L.vtile = o;
   o += (uint32_t)v_bufs * v_box * dims * 2; // one tile, or whole ones
   L.e = o; // scores, exponentials, probabilities of whole tiles; a spare block so that the sum may read ahead
@@ -506,7 +518,7 @@ __host__ __device__ inline AcLayout ac_layout(int gqa, int hd, int dims, int k_b
 }
 
 /** Scores (not yet divided) of one thread's key row against the H query heads at qs: ascending groups of eight elements. */
-template <int H, int HD>
+template <int H, int HD, int ROWS>
 __device__ __forceinline__ void dot_rows(const uint8_t *tile, int row, const float *qs, int hd, float (&sum)[H]) {
   float acc[H][8];
 #pragma unroll
@@ -516,7 +528,7 @@ __device__ __forceinline__ void dot_rows(const uint8_t *tile, int row, const flo
       acc[h][l] = 0.f;
 #pragma unroll 8
   for (int c = 0; c < (HD ? HD : hd) / 8; ++c) {
-    const uint4 w = *reinterpret_cast<const uint4 *>(tile + (c >> 3) * (AC_TILE * 128) + row * 128 + (((c & 7) ^ (row & 7)) << 4));
+    const uint4 w = *reinterpret_cast<const uint4 *>(tile + (c >> 3) * (ROWS * 128) + row * 128 + (((c & 7) ^ (row & 7)) << 4));
     const uint32_t ws[4] = {w.x, w.y, w.z, w.w};
     float2 kv[4];
 #pragma unroll
@@ -645,30 +657,38 @@ __global__ void __launch_bounds__(AC_THREADS, 1)
 attn_cluster_kernel(const __grid_constant__ CUtensorMap kmap, const __grid_constant__ CUtensorMap vmap,
                     const __grid_constant__ AttnStep a) {
   extern __shared__ uint8_t ac_raw[];
-  __shared__ __align__(8) unsigned long long kbar[AC_KBUF_MAX], vfull[AC_VBUF_MAX], vempty[AC_VBUF_MAX];
+  __shared__ __align__(8) unsigned long long kbar[AC_KBUF_MAX], vfull[AC_VBUF_MAX], vempty[AC_VBUF_MAX],
+    tfull[AC_TBUF_MAX], tempty[AC_TBUF_MAX];
   __shared__ float red[AC_WARPS];
   __shared__ float s_bcast;
   __shared__ int abort_word;
   volatile int *abort_flag = &abort_word;
+  constexpr int KROWS = AC_KROWS<DIMS>, VROWS = AC_VROWS<DIMS>;
+  constexpr bool TURN = DIMS == 32;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int gqa = a.hq / a.hkv / a.groups, hd = HD ? HD : a.hd, per_head = (hd + DIMS - 1) / DIMS, items = gqa * per_head;
   const uint32_t rank = (uint32_t)cluster_rank(), csize = (uint32_t)cluster_size();
   const int cluster = (int)(blockIdx.x / csize), n = cluster / a.groups, h0 = cluster * gqa; // kv head, first query head
   uint8_t *base = ac_raw + (-smem_u32(ac_raw) & 1023u); // an offset: rounding the pointer itself up makes every access a generic one
-  const AcLayout L = ac_layout(gqa, hd, DIMS, a.k_bufs, a.v_bufs, a.v_box, a.cap_rows);
+  const AcLayout L = ac_layout(gqa, hd, DIMS, KROWS, a.k_bufs, a.v_bufs, a.t_bufs, a.v_box, a.cap_rows);
   uint8_t *ktile = base + L.ktile, *vtile = base + L.vtile;
   float *e = reinterpret_cast<float *>(base + L.e), *qs = reinterpret_cast<float *>(base + L.q), *kown = qs + gqa * hd;
   const int k_halves = (hd + 63) / 64;
-  const uint32_t kbytes = (uint32_t)k_halves * AC_TILE * 128, vbytes = (uint32_t)a.v_box * DIMS * 2; // of a buffer
+  const uint32_t kbytes = (uint32_t)k_halves * KROWS * 128, vbytes = (uint32_t)a.v_box * DIMS * 2; // of a buffer
   const uint32_t ksm = smem_u32(ktile), vsm = smem_u32(vtile), esm = smem_u32(e);
-  const uint32_t kbar0 = smem_u32(kbar), vfull0 = smem_u32(vfull), vempty0 = smem_u32(vempty);
+  const uint32_t kbar0 = smem_u32(kbar), vfull0 = smem_u32(vfull), vempty0 = smem_u32(vempty),
+                 tfull0 = smem_u32(tfull), tempty0 = smem_u32(tempty);
   if (tid == 0) {
     abort_word = 0;
     for (int i = 0; i < a.k_bufs; ++i)
       mbar_init(kbar0 + 8 * i, 1);
     for (int i = 0; i < a.v_bufs; ++i) {
       mbar_init(vfull0 + 8 * i, 1);
-      mbar_init(vempty0 + 8 * i, DIMS / 32);
+      mbar_init(vempty0 + 8 * i, TURN ? AC_TURNERS : DIMS / 32);
+    }
+    for (int i = 0; TURN && i < a.t_bufs; ++i) {
+      mbar_init(tfull0 + 8 * i, AC_TURNERS);
+      mbar_init(tempty0 + 8 * i, 1);
     }
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
@@ -688,13 +708,12 @@ attn_cluster_kernel(const __grid_constant__ CUtensorMap kmap, const __grid_const
   const int item_head = (int)rank / per_head, item_d0 = ((int)rank % per_head) * DIMS;
   const bool has_item = (int)rank < items, has_own = a.rope && r_lo < cnt && r_hi == cnt;
   const bool append = has_own && cluster % a.groups == 0; // one cluster per kv head appends the token's rows
-  constexpr int VROWS = AC_VROWS<DIMS>;
-  const unsigned k_tiles = (r_hi - r_lo + AC_TILE - 1) / AC_TILE, v_tiles = (cached + VROWS - 1) / VROWS;
+  const unsigned k_tiles = (r_hi - r_lo + KROWS - 1) / KROWS, v_tiles = (cached + VROWS - 1) / VROWS;
   auto issue_k = [&](unsigned t, int buf) {
     const uint32_t bar = kbar0 + 8 * buf;
     mbar_expect_tx(bar, (uint32_t)(k_halves * a.k_box) * 128);
     for (int h = 0; h < k_halves; ++h)
-      tma_tile(ksm + buf * kbytes + h * (AC_TILE * 128), &kmap, n * hd + 64 * h, (int)(first + r_lo + t * AC_TILE), bar);
+      tma_tile(ksm + buf * kbytes + h * (KROWS * 128), &kmap, n * hd + 64 * h, (int)(first + r_lo + t * KROWS), bar);
   };
   auto issue_v = [&](unsigned t, int buf) {
     const uint32_t bar = vfull0 + 8 * buf;
@@ -743,7 +762,7 @@ attn_cluster_kernel(const __grid_constant__ CUtensorMap kmap, const __grid_const
   for (unsigned t = 0; t < k_tiles; ++t) {
     ok = ok && mbar_wait_bounded(kbar0 + 8 * kbuf, kpar, abort_flag, &g_attn_status, AC_POLLS, 1024);
     uint8_t *tile = ktile + kbuf * kbytes;
-    const unsigned t0 = r_lo + t * AC_TILE, rows = min(r_hi - t0, (unsigned)AC_TILE);
+    const unsigned t0 = r_lo + t * KROWS, rows = min(r_hi - t0, (unsigned)KROWS);
     if (has_own && t + 1 == k_tiles) { // the token's own row, as the cache will hold it, over what the copy found there
       const int row = (int)rows - 1;
       for (int c = tid; c < hd / 8; c += AC_THREADS) {
@@ -753,19 +772,19 @@ attn_cluster_kernel(const __grid_constant__ CUtensorMap kmap, const __grid_const
         for (int i = 0; i < 4; ++i)
           w[i] = (uint32_t)float_to_half_bits_rn(src[2 * i]) | ((uint32_t)float_to_half_bits_rn(src[2 * i + 1]) << 16);
         const uint4 v = make_uint4(w[0], w[1], w[2], w[3]);
-        *reinterpret_cast<uint4 *>(tile + (c >> 3) * (AC_TILE * 128) + row * 128 + (((c & 7) ^ (row & 7)) << 4)) = v;
+        *reinterpret_cast<uint4 *>(tile + (c >> 3) * (KROWS * 128) + row * 128 + (((c & 7) ^ (row & 7)) << 4)) = v;
         if (append)
           *reinterpret_cast<uint4 *>(a.kcache + ((size_t)p * a.hkv + n) * hd + 8 * c) = v;
       }
       __syncthreads();
     }
     if (ok) { // a unit of work: 32 rows and one or two heads
-      const int lg = rows <= 32 ? 0 : rows <= 64 ? 1 : 2, mask = (1 << lg) - 1;
+      const int lg = rows <= 32 ? 0 : rows <= 64 ? 1 : KROWS == 128 || rows <= 128 ? 2 : 3, mask = (1 << lg) - 1;
       if (gqa % 2 == 0 && ((gqa / 2) << lg) >= AC_WARPS) { // two heads at a time: a key row is converted once for both
         for (int u = warp; u < (gqa / 2) << lg; u += AC_WARPS) {
           const int row = (u & mask) * 32 + lane, g = 2 * (u >> lg);
           float s[2];
-          dot_rows<2, HD>(tile, row, qs + g * hd, hd, s);
+          dot_rows<2, HD, KROWS>(tile, row, qs + g * hd, hd, s);
           if (row < (int)rows) {
             put(t0 + row, g, s[0]);
             put(t0 + row, g + 1, s[1]);
@@ -775,7 +794,7 @@ attn_cluster_kernel(const __grid_constant__ CUtensorMap kmap, const __grid_const
         for (int u = warp; u < gqa << lg; u += AC_WARPS) {
           const int row = (u & mask) * 32 + lane, g = u >> lg;
           float s[1];
-          dot_rows<1, HD>(tile, row, qs + g * hd, hd, s);
+          dot_rows<1, HD, KROWS>(tile, row, qs + g * hd, hd, s);
           if (row < (int)rows)
             put(t0 + row, g, s[0]);
         }
@@ -823,6 +842,42 @@ attn_cluster_kernel(const __grid_constant__ CUtensorMap kmap, const __grid_const
   for (unsigned r = tid; r < cnt32; r += AC_THREADS)
     e[r] = r < cnt ? exp256_lane(__fsub_rn(e[r], mx)) : 0.f;
   __syncthreads();
+  // A turner's share of value tile t (which lies in the ring's place vbuf) into turned tile tbuf: 32 rows of 8 dimensions at a time,
+  // transposed by the load; a lane then holds pairs of rows of one dimension.
+  int vbuf = 0, tbuf = 0;
+  uint32_t vpar = 0, tpar = 1;
+  auto turn = [&](unsigned t) {
+    if (!mbar_wait_bounded(vfull0 + 8 * vbuf, vpar, abort_flag, &g_attn_status, AC_POLLS, 1024))
+      return false;
+    const int units = (int)(min(cached - t * VROWS, (unsigned)VROWS) + 31) / 32 * 4;
+    const uint32_t src = vsm + vbuf * vbytes, dst = ksm + tbuf * AC_TBYTES;
+    for (int u = warp - 1; u < units; u += AC_TURNERS) {
+      const int row = 32 * (u >> 2) + lane, c = u & 3; // rows of 64 bytes, their 16-byte pieces swizzled
+      uint32_t w[4];
+      asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];"
+                   : "=r"(w[0]), "=r"(w[1]), "=r"(w[2]), "=r"(w[3])
+                   : "r"(src + row * 64 + ((c ^ ((row >> 1) & 3)) << 4))
+                   : "memory");
+#pragma unroll
+      for (int m = 0; m < 4; ++m)
+        sts32(dst + (8 * c + (lane >> 2)) * AC_TPITCH + (32 * (u >> 2) + 8 * m + 2 * (lane & 3)) * 2, w[m]);
+    }
+    __syncwarp();
+    if (lane == 0) {
+      mbar_arrive(tfull0 + 8 * tbuf);
+      mbar_arrive(vempty0 + 8 * vbuf);
+    }
+    if (++vbuf == a.v_bufs)
+      vbuf = 0, vpar ^= 1;
+    if (++tbuf == a.t_bufs)
+      tbuf = 0, tpar ^= 1;
+    return true;
+  };
+  unsigned turned = 0;
+  const bool turner = TURN && warp > 0 && warp <= AC_TURNERS;
+  if (turner) // the tiles that are on their way already, while the sum is formed (the keys in their place have been read)
+    while (ok && turned < (unsigned)min(a.t_bufs, a.v_bufs) && turned < v_tiles)
+      ok = turn(turned++);
   if (warp == 0) {
     const float sum = ordered_sum(e, cnt32, a.sink ? exp256_lane(__fsub_rn(a.sink[head], mx)) : 0.0f, lane);
     if (lane == 0)
@@ -849,7 +904,87 @@ attn_cluster_kernel(const __grid_constant__ CUtensorMap kmap, const __grid_const
       }
     }
     __syncwarp();
-  } else if (warp < DIMS / 32) {
+  } else if (turner) {
+    while (ok && turned < v_tiles)
+      ok = mbar_wait_bounded(tempty0 + 8 * tbuf, tpar, abort_flag, &g_attn_status, AC_POLLS, 1024) && turn(turned++);
+  } else if (TURN && warp == 0) {
+    // Thirty-two rows in the chain while the next thirty-two are on their way: twelve loads, where row by row it would be forty, whose
+    // latency the chain's four clocks a row do not hide.
+    const int d = item_d0 + lane;
+    float acc = 0.f;
+    float pr[2][32];
+    uint4 vq[2][4];
+    auto load = [&](uint32_t vt, uint32_t pt, float(&pp)[32], uint4(&vv)[4]) {
+#pragma unroll
+      for (int u = 0; u < 4; ++u)
+        vv[u] = lds128(vt + 16 * u);
+#pragma unroll
+      for (int u = 0; u < 8; ++u) {
+        const uint4 f = lds128(pt + 16 * u);
+        pp[4 * u] = __uint_as_float(f.x), pp[4 * u + 1] = __uint_as_float(f.y), pp[4 * u + 2] = __uint_as_float(f.z),
+               pp[4 * u + 3] = __uint_as_float(f.w);
+      }
+    };
+    auto chain = [&](const float(&pp)[32], const uint4(&vv)[4], int n) { // the first n rows
+#pragma unroll
+      for (int u = 0; u < 32; ++u) {
+        const uint32_t w[4] = {vv[u >> 3].x, vv[u >> 3].y, vv[u >> 3].z, vv[u >> 3].w};
+        if (u < n)
+          acc = __fmaf_rn(pp[u], half_bits_to_float((uint16_t)(w[(u >> 1) & 3] >> (16 * (u & 1)))), acc);
+      }
+    };
+    int buf = 0;
+    uint32_t par = 0, vt = ksm + lane * AC_TPITCH;
+    if (v_tiles) {
+      ok = mbar_wait_bounded(tfull0, 0, abort_flag, &g_attn_status, AC_POLLS, 1024) && ok;
+      load(vt, esm, pr[0], vq[0]); // reads past the last row stay in the tile and are not used
+    }
+    for (unsigned t = 0; t < v_tiles; ++t) {
+      const uint32_t pt = esm + 4 * t * VROWS;
+      const int rows = (int)min(cached - t * VROWS, (unsigned)VROWS);
+      const bool more = t + 1 < v_tiles; // then this tile is a whole one
+      int nbuf = buf + 1;
+      uint32_t npar = par;
+      if (nbuf == a.t_bufs)
+        nbuf = 0, npar ^= 1;
+      // asked now, needed thirty-two rows before this tile's end: the answer takes about a hundred clocks
+      const bool next_here = more && mbar_try_wait(tfull0 + 8 * nbuf, npar);
+      int j = 0;
+#pragma unroll 1
+      for (; j + 64 <= rows; j += 64) {
+        load(vt + 2 * (j + 32), pt + 4 * (j + 32), pr[1], vq[1]);
+        chain(pr[0], vq[0], 32);
+        uint32_t ahead = vt + 2 * (j + 64);
+        if (j + 64 == VROWS) {
+          if (more && !next_here)
+            ok = mbar_wait_bounded(tfull0 + 8 * nbuf, npar, abort_flag, &g_attn_status, AC_POLLS, 1024) && ok;
+          ahead = ksm + nbuf * AC_TBYTES + lane * AC_TPITCH; // behind the last tile: read and not used
+        }
+        load(ahead, pt + 4 * (j + 64), pr[0], vq[0]);
+        chain(pr[1], vq[1], 32);
+      }
+      if (j < rows) { // the last tile: up to 63 rows, the first 32 of them in registers
+        if (rows - j > 32) {
+          load(vt + 2 * (j + 32), pt + 4 * (j + 32), pr[1], vq[1]);
+          chain(pr[0], vq[0], 32);
+          chain(pr[1], vq[1], rows - j - 32);
+        } else {
+          chain(pr[0], vq[0], rows - j);
+        }
+      }
+      __syncwarp();
+      if (lane == 0)
+        mbar_arrive(tempty0 + 8 * buf);
+      buf = nbuf;
+      par = npar;
+      vt = ksm + buf * AC_TBYTES + lane * AC_TPITCH;
+    }
+    if (ok) {
+      if (a.rope)
+        acc = __fmaf_rn(e[cnt - 1], half_bits_to_float(float_to_half_bits_rn(a.v[(size_t)n * hd + d])), acc);
+      out[(size_t)head * hd + d] = acc;
+    }
+  } else if (!TURN && warp < DIMS / 32) {
     const int d = item_d0 + tid;
     float acc = 0.f;
     // Sixteen rows in the chain while the next sixteen -- of the next tile at a tile's end -- are on their way.
@@ -1021,50 +1156,70 @@ static int launch_attn_cluster(AttnStep a, unsigned bound, unsigned rows, unsign
   if ((flags & NNTR_CUDA_ATTN_SEPARATE) || hd > 128 || rows > AC_MAX_ROWS)
     return NNTR_CUDA_OK;
   int gqa = a.hq / a.hkv;
-  a.groups = 1;
+  const bool many = a.tokens > 1;
+  // Of one token with a long window, a CTA for 32 dimensions of a head where the chip has room for that, in clusters of four. Shorter
+  // windows in a decode step are slower so (16 tokens over four layers, 32 / 8 heads of 128 at a context of 100 / 512: 2959 / 3197 us, with
+  // slices 3094 / 3278), because every launch there fetches its code anew and this is more of it; 64 / 8 heads of 64 at 2000: 3906, with
+  // slices 3803. Alone 64 / 8 heads of 64 at 2000 / 4096 / 6000 rows 23.2 / 36.6 / 50.4 us, with slices 21.6 / 33.5 / 45.0; 32 / 8 of 128 at
+  // 1500 / 5000 20.3 / 44.7 and 18.7 / 40.8. Heads whose CTAs would own 128 dimensions each leave most of the chip idle without: 32 / 4 heads
+  // of 128 at 512 / 3000 rows 12.2 / 34.1, with slices 10.5 / 28.1; decode steps at 100 / 512 3012 / 3325 and 3081 / 3253, three layers at
+  // 1500 3146 and 2912.
+  const int slices = hd / 32, slice_heads = hd == 64 ? 2 : 1;
+  static std::atomic<uint32_t> attr_done[64];
+  static ClusterFit fit64, fit128;
+  int dev = 0;
+  NNTR_CHECK_CUDA(cudaGetDevice(&dev));
+  if (!attr_done[dev & 63].load(std::memory_order_acquire)) {
+    for (const auto k : {attn_cluster_kernel<128, 32>, attn_cluster_kernel<128, 64>, attn_cluster_kernel<128, 128>, attn_cluster_kernel<64, 32>,
+                         attn_cluster_kernel<64, 64>, attn_cluster_kernel<0, 64>, attn_cluster_kernel<0, 128>})
+      NNTR_CHECK_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, AC_SMEM_ALONE));
+    attr_done[dev & 63].store(1, std::memory_order_release);
+  }
+  const bool sliced = !many && rows > (hd > 64 && gqa > 4 ? 256u : AC_SLICED_ROWS) && (hd == 64 || hd == 128) && gqa % slice_heads == 0 &&
+                      a.hq * slices / 4 <= (hd == 64 ? fit64(attn_cluster_kernel<64, 32>, 4, AC_THREADS, AC_SMEM_ALONE)
+                                                     : fit128(attn_cluster_kernel<128, 32>, 4, AC_THREADS, AC_SMEM_ALONE));
+  a.groups = sliced ? gqa / slice_heads : 1;
   while (gqa % a.groups || gqa / a.groups > 8) // at most 16 query heads in all (check_attn)
     ++a.groups;
   gqa /= a.groups;
-  // a CTA owns 64 dimensions of a head where eight CTAs are enough for that, else -- and for many tokens, which fill the
+  // else a CTA owns 64 dimensions of a head where eight CTAs are enough for that, or -- and for many tokens, which fill the
   // machine anyway -- the whole head
-  const bool many = a.tokens > 1;
-  const int dims = hd <= 64 || (gqa * 2 <= 8 && !many) ? 64 : 128;
+  const int dims = sliced ? 32 : hd <= 64 || (gqa * 2 <= 8 && !many) ? 64 : 128;
   const int items = gqa * ((hd + dims - 1) / dims);
   // eight CTAs per cluster while that leaves no cluster waiting for SMs -- 16 clusters of eight run in two waves (11.1 us for a
   // window of 50 rows, clusters of four 8), because a cluster lies inside one part of the chip --, at least as many as items
   const unsigned clusters = (unsigned)(a.hkv * a.groups);
-  unsigned csize = clusters > 12 && items <= 4 ? 4 : 8;
+  unsigned csize = sliced || (clusters > 12 && items <= 4) ? 4 : 8;
   while (csize > 1 && (many || clusters * csize > 144u) && (int)(csize / 2) >= items)
     csize /= 2;
   // buffers for what the launch can need, no more: a prompt's CTAs share an SM where they fit
   a.cap_rows = rows;
-  const unsigned k_tiles = ((rows + csize - 1) / csize + AC_TILE - 1) / AC_TILE, v_rows = dims == 64 ? 256u : 128u, v_tiles = (rows + v_rows - 1) / v_rows;
-  const unsigned k_max = hd <= 64 ? 4u : 2u;
+  const unsigned k_rows = sliced ? 256u : 128u, share = (rows + csize - 1) / csize;
+  const unsigned k_tiles = (share + k_rows - 1) / k_rows, v_rows = dims <= 64 ? 256u : 128u, v_tiles = (rows + v_rows - 1) / v_rows;
+  a.t_bufs = sliced ? (int)std::min(v_tiles, (unsigned)AC_TBUF_MAX) : 0;
+  const unsigned k_max = hd > 64 ? 2u : sliced ? 3u : 4u;
   a.k_bufs = (int)(k_tiles < k_max ? k_tiles : k_max);
   const unsigned v_max = dims == 64 ? 3u : (unsigned)AC_VBUF_MAX;
   a.v_bufs = (int)(v_tiles < v_max ? v_tiles : v_max);
-  const auto box = [](unsigned n) { return n <= 32 ? 32 : n <= 64 ? 64 : AC_TILE; };
-  a.k_box = box((rows + csize - 1) / csize);
+  const auto box = [&](unsigned n) { return n <= 32 ? 32 : n <= 64 ? 64 : n <= 128 ? 128 : k_rows; };
+  a.k_box = (int)box(share);
   a.v_box = (int)((rows < v_rows ? rows : v_rows) + 31) / 32 * 32;
-  AcLayout L = ac_layout(gqa, hd, dims, a.k_bufs, a.v_bufs, a.v_box, rows);
-  while (L.total > 200u * 1024u && a.v_bufs > 2)
-    L = ac_layout(gqa, hd, dims, a.k_bufs, --a.v_bufs, a.v_box, rows);
-  const auto kernel = hd == 128  ? (dims == 64 ? attn_cluster_kernel<128, 64> : attn_cluster_kernel<128, 128>)
-                      : hd == 64 ? attn_cluster_kernel<64, 64>
-                                 : (dims == 64 ? attn_cluster_kernel<0, 64> : attn_cluster_kernel<0, 128>);
-  static std::atomic<uint32_t> attr_done[64];
-  int dev = 0;
-  NNTR_CHECK_CUDA(cudaGetDevice(&dev));
-  const uint32_t bit = 1u << (hd == 128 ? (dims == 64 ? 0 : 1) : hd == 64 ? 2 : (dims == 64 ? 3 : 4));
-  if (!(attr_done[dev & 63].load(std::memory_order_acquire) & bit)) {
-    NNTR_CHECK_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
-    attr_done[dev & 63].fetch_or(bit, std::memory_order_release);
+  const auto layout = [&] { return ac_layout(gqa, hd, dims, (int)k_rows, a.k_bufs, a.v_bufs, a.t_bufs, a.v_box, rows); };
+  AcLayout L = layout();
+  while (L.total > AC_SMEM_ALONE && (a.v_bufs > 2 || a.k_bufs > 1)) {
+    a.v_bufs > 2 ? --a.v_bufs : --a.k_bufs;
+    L = layout();
   }
+  const auto kernel = hd == 128  ? (dims == 32   ? attn_cluster_kernel<128, 32>
+                                    : dims == 64 ? attn_cluster_kernel<128, 64>
+                                                 : attn_cluster_kernel<128, 128>)
+                      : hd == 64 ? (dims == 32 ? attn_cluster_kernel<64, 32> : attn_cluster_kernel<64, 64>)
+                                 : (dims == 64 ? attn_cluster_kernel<0, 64> : attn_cluster_kernel<0, 128>);
   CUtensorMap kmap, vmap;
   // maps over the caches, [bound rows][hkv * hd] fp16; keys swizzled: 64 values = 128 bytes
   const uint64_t width = (uint64_t)a.hkv * hd;
   int rc = encode_map_2d(&kmap, a.kcache, 2, width, bound, width * 2, 64, (unsigned)a.k_box, true);
-  if (rc || (rc = encode_map_2d(&vmap, a.vcache, 2, width, bound, width * 2, (unsigned)dims, (unsigned)a.v_box, false)))
+  if (rc || (rc = encode_map_2d(&vmap, a.vcache, 2, width, bound, width * 2, (unsigned)dims, (unsigned)a.v_box, sliced)))
     return rc;
   cudaLaunchConfig_t cfg = {};
   cudaLaunchAttribute attr[2];

@@ -48,7 +48,9 @@ int encode_map_2d(CUtensorMap *map, const void *base, unsigned elem_bytes, uint6
   const cuuint32_t box[2] = {box_width, box_rows}, estr[2] = {1, 1};
   const CUresult r = enc(&slot.map, elem_bytes == 1 ? CU_TENSOR_MAP_DATA_TYPE_UINT8 : CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2,
                          const_cast<void *>(base), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
-                         swizzle ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+                         !swizzle                        ? CU_TENSOR_MAP_SWIZZLE_NONE
+                         : box_width * elem_bytes == 64 ? CU_TENSOR_MAP_SWIZZLE_64B
+                                                        : CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
                          CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   if (r != CUDA_SUCCESS) {
     slot.key = Key{};

@@ -13,7 +13,7 @@
 namespace nntr {
 
 /** Map over rows of `width` elements (1 or 2 bytes each) `stride` bytes apart; a copy takes a box of box_rows x box_width.
- *  swizzle: 128-byte rows of the box are stored swizzled. base 16-byte aligned, stride and box_width * size multiples of
+ *  swizzle: rows of the box, of 128 or 64 bytes, are stored swizzled. base 16-byte aligned, stride and box_width * size multiples of
  *  16. Maps depend on the arguments alone; every thread keeps the last ones it made, because a model's calls come back. */
 int encode_map_2d(CUtensorMap *map, const void *base, unsigned elem_bytes, uint64_t width, uint64_t rows, uint64_t stride,
                   unsigned box_width, unsigned box_rows, bool swizzle);
