@@ -72,9 +72,14 @@ constexpr int LUT_AND_XOR = 0x6A; // (a & b) ^ c
 /* CTAS: CTAs per SM that registers and shared memory are held to. Four with 4 bytes of spills and two stages (which leave the L1
  * cache room for the activations; with three stages 137 us instead of 122 for 8 x 151936 x 2560, three CTAs of three stages 128), where
  * three per SM would need a second round. */
-template <int CTAS> constexpr int Q6M_STAGES = CTAS == 4 ? 2 : 3;
-template <int NT, int CTAS>
-__global__ void __launch_bounds__(Q6M_WARPS * 32, CTAS)
+template <int CTAS> constexpr int Q6M_STAGES = CTAS == 3 ? 3 : 2;
+/* SPLIT: the CTA has eight warps, all of them on the same 16 weight rows, and each takes every eighth super-block; the chains go from warp
+ * to warp, one super-block further at each. For calls with too few rows to fill the chip, where the 3400 clocks that a warp on its own
+ * takes for a super-block, one after the other, are the call's time: 5 x 4096 x 4096 30.0 -> 11.3 us, 8 x 2560 x 9728 65 -> 21. */
+constexpr int Q6S_WARPS = 8;
+constexpr int Q6S_SMEM = Q6S_WARPS * (2 * Q6M_STAGE_WORDS * 4 + 8 * 32 * 16);
+template <int NT, int CTAS, bool SPLIT>
+__global__ void __launch_bounds__((SPLIT ? Q6S_WARPS : Q6M_WARPS) * 32, CTAS)
 gemm_q6_K_mma_kernel(const uint8_t *__restrict__ act, const uint8_t *__restrict__ W, float *__restrict__ C, int ldc, int M,
                      int N, int nb) {
   // High nibbles used where they lie, with their own factors: the same number of operations, 187 against 193 us for 16 x 151936 x
@@ -83,32 +88,43 @@ gemm_q6_K_mma_kernel(const uint8_t *__restrict__ act, const uint8_t *__restrict_
   constexpr int STAGES = Q6M_STAGES<CTAS>;
   // a shift less per word of high bits (1 % with four CTAs); with three, where a warp's own latency counts, 5 x 4096 x 4096 31.7 us instead of 30.0
   constexpr bool DENSE = NT == 1 && CTAS == 4;
-  __shared__ alignas(16) uint32_t stage[Q6M_WARPS][STAGES][Q6M_STAGE_WORDS];
-  __shared__ alignas(8) unsigned long long bars[Q6M_WARPS][STAGES];
-  __shared__ int aborted[Q6M_WARPS]; // one per warp: the warps of a CTA do not meet
+  constexpr int WARPS = SPLIT ? Q6S_WARPS : Q6M_WARPS, EVERY = SPLIT ? WARPS : 1; // a warp's super-blocks
+  static_assert(!SPLIT || NT == 1, "a hand-over per super-block and warp");
+  extern __shared__ __align__(16) uint32_t split_smem[]; // SPLIT: the stages, then the chains on their way
+  __shared__ alignas(16) uint32_t stage[SPLIT ? 1 : WARPS][SPLIT ? 1 : STAGES][SPLIT ? 1 : Q6M_STAGE_WORDS];
+  __shared__ alignas(8) unsigned long long bars[WARPS][STAGES];
+  __shared__ int aborted[SPLIT ? 1 : WARPS]; // one per warp that stores for itself: the warps of such a CTA do not meet
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, g = lane >> 2, t = lane & 3, run = t & 1, h = t >> 1;
-  const int n0 = (blockIdx.y * Q6M_WARPS + warp) * 16, m0 = blockIdx.x * 8 * NT;
+  const int n0 = (SPLIT ? blockIdx.y : blockIdx.y * WARPS + warp) * 16, m0 = blockIdx.x * 8 * NT;
   if (n0 >= N) {
     pdl_wait();
     return;
   }
   const int nt = min(NT, (M - m0 + 7) >> 3);
   const size_t row_bytes = (size_t)nb * sizeof(BlockQ6K);
-  const uint32_t sm = smem_u32(stage[warp][0]), bar = smem_u32(bars[warp]);
-  volatile int *abort_flag = &aborted[warp];
+  const uint32_t bar = smem_u32(bars[warp]);
+  auto stage_of = [&](int k) { // this warp's
+    if constexpr (SPLIT)
+      return split_smem + (warp * STAGES + k) * Q6M_STAGE_WORDS;
+    else
+      return stage[warp][k];
+  };
+  const uint32_t sm = smem_u32(stage_of(0));
+  volatile int *abort_flag = &aborted[SPLIT ? 0 : warp];
   if (lane == 0) {
     for (int k = 0; k < STAGES; ++k)
       mbar_init(bar + 8 * k, 1);
-    *abort_flag = 0;
+    if (!SPLIT || warp == 0)
+      *abort_flag = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
-  __syncwarp();
+  SPLIT ? __syncthreads() : __syncwarp();
   // Copies super-block b of the 16 rows, lane i the block of row i (rows past the end repeat the last one). A block starts 0
   // to 14 bytes into a 16-byte piece, so its 210 bytes always lie in 14 whole pieces, and the copy never leaves the piece
   // that holds the block's own first or last byte.
   const uint8_t *mine = W + (size_t)min(n0 + (lane & 15), N - 1) * row_bytes;
-  auto fetch = [&](int b) {
-    const int k = b % STAGES;
+  auto fetch = [&](int u) { // the warp's u-th
+    const int k = u % STAGES, b = SPLIT ? warp + u * EVERY : u;
     if (lane == 0)
       mbar_expect_tx(bar + 8 * k, 16 * Q6M_COPY);
     __syncwarp();
@@ -117,8 +133,9 @@ gemm_q6_K_mma_kernel(const uint8_t *__restrict__ act, const uint8_t *__restrict_
                reinterpret_cast<const void *>(reinterpret_cast<uintptr_t>(mine + (size_t)b * sizeof(BlockQ6K)) & ~(uintptr_t)15),
                Q6M_COPY, bar + 8 * k);
   };
-  for (int b = 0; b < STAGES - 1 && b < nb; ++b) // the weights do not depend on the kernel before
-    fetch(b);
+  const int units = SPLIT ? (nb - warp + EVERY - 1) / EVERY : nb; // super-blocks of this warp
+  for (int u = 0; u < STAGES - 1 && u < units; ++u) // the weights do not depend on the kernel before
+    fetch(u);
   pdl_wait(); // the activation tiles do
   pdl_launch_dependents();
   float acc[NT][8][4];
@@ -134,13 +151,20 @@ gemm_q6_K_mma_kernel(const uint8_t *__restrict__ act, const uint8_t *__restrict_
   const uint32_t a0 = (uint32_t)(reinterpret_cast<uintptr_t>(W) + (size_t)min(n0 + g, N - 1) * row_bytes),
                  a1 = (uint32_t)(reinterpret_cast<uintptr_t>(W) + (size_t)min(n0 + g + 8, N - 1) * row_bytes);
   bool ok = true;
-  for (int b = 0; b < nb; ++b) {
-    ok = mbar_wait_bounded(bar + 8 * (b % STAGES), (b / STAGES) & 1, abort_flag, &g_q6m_status, Q6M_POLLS, 2048);
-    if (!(ok = __all_sync(FULL, ok)))
-      break;
-    if (b + STAGES - 1 < nb) // into the slot that was read in the previous round
-      fetch(b + STAGES - 1);
-    const uint32_t *st = stage[warp][b % STAGES];
+  for (int un = 0; un < units; ++un) {
+    const int b = SPLIT ? warp + un * EVERY : un;
+    const bool here = mbar_wait_bounded(bar + 8 * (un % STAGES), (un / STAGES) & 1, abort_flag, &g_q6m_status, Q6M_POLLS, 2048);
+    if constexpr (SPLIT) {
+      ok = __all_sync(FULL, here) && ok; // without the data the chains have to pass all the same
+      if (ok && un + STAGES - 1 < units)
+        fetch(un + STAGES - 1);
+    } else {
+      if (!(ok = __all_sync(FULL, here)))
+        break;
+      if (un + STAGES - 1 < units) // into the slot that was read in the previous round
+        fetch(un + STAGES - 1);
+    }
+    const uint32_t *st = stage_of(un % STAGES);
     uint32_t sh[2];
     const uint32_t *row[2];
     float d[NT][4];
@@ -243,10 +267,30 @@ gemm_q6_K_mma_kernel(const uint8_t *__restrict__ act, const uint8_t *__restrict_
 #pragma unroll
             for (int c = 0; c < 4; c += 2) {
               const float2 sum = add2(p[c], p[c + 1], p2[c], p2[c + 1]);
-              fma2(acc[i][l][c], acc[i][l][c + 1], d[i][c], d[i][c + 1], sum.x, sum.y);
+              if constexpr (SPLIT)
+                acc[i][l][c] = sum.x, acc[i][l][c + 1] = sum.y;
+              else
+                fma2(acc[i][l][c], acc[i][l][c + 1], d[i][c], d[i][c + 1], sum.x, sum.y);
             }
           }
       }
+    }
+    if constexpr (SPLIT) { // take the chains over, add this super-block, pass them on
+      float4 *const chains = reinterpret_cast<float4 *>(split_smem + WARPS * STAGES * Q6M_STAGE_WORDS) + lane;
+      const int from = warp, to = warp + 1 < WARPS ? warp + 1 : 0;
+      if (b > 0)
+        pair_sync(1 + from);
+#pragma unroll
+      for (int l = 0; l < 8; ++l) {
+        float4 f = b > 0 ? chains[(from * 8 + l) * 32] : make_float4(0.f, 0.f, 0.f, 0.f);
+        fma2(f.x, f.y, d[0][0], d[0][1], acc[0][l][0], acc[0][l][1]);
+        fma2(f.z, f.w, d[0][2], d[0][3], acc[0][l][2], acc[0][l][3]);
+        if (b + 1 < nb)
+          chains[(to * 8 + l) * 32] = f;
+        acc[0][l][0] = f.x, acc[0][l][1] = f.y, acc[0][l][2] = f.z, acc[0][l][3] = f.w;
+      }
+      if (b + 1 < nb)
+        pair_arrive(1 + to);
     }
     __syncwarp(); // the slot is refilled in the next round
   }
@@ -255,6 +299,8 @@ gemm_q6_K_mma_kernel(const uint8_t *__restrict__ act, const uint8_t *__restrict_
       __nanosleep(1000);
     return;
   }
+  if (SPLIT && (warp != (nb - 1) % WARPS || !nobody_gave_up(ok, abort_flag))) // the chains end in the last super-block's warp
+    return;
 #pragma unroll
   for (int i = 0; i < NT; ++i)
 #pragma unroll
@@ -308,22 +354,33 @@ int launch_gemm_mma_q6_K(unsigned M, unsigned N, unsigned K, const float *A, con
   NNTR_CHECK_CUDA(launch_in_clusters(act_tiles_q6_kernel, dim3((unsigned)(((int64_t)M * nb + 7) / 8)), 1, 256, 0, st, A, (int64_t)K,
                                      static_cast<uint8_t *>(ws), (int)M, nb));
   count_launch();
-  const unsigned nt = M <= 8 ? 1 : 2;
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3((M + 8 * nt - 1) / (8 * nt), ((N + 15) / 16 + Q6M_WARPS - 1) / Q6M_WARPS);
-  cfg.blockDim = dim3(Q6M_WARPS * 32);
-  cfg.stream = st;
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  attr[0].val.programmaticStreamSerializationAllowed = 1;
-  cfg.attrs = attr;
-  cfg.numAttrs = 1;
+  const unsigned row_tiles = (N + 15) / 16, sms = (unsigned)sm_count();
+  // A wave of shared tiles (two CTAs per SM) takes about 3.5 us and 0.45 for each super-block of K; a warp on its own 2 us for each,
+  // however few they are, 3.2 with two tiles of rows. One tile, shared / not: 8 x 4736 x 2560 (1 wave) 9.5 / 18.5 us, 9472 rows (2) 16.8 / 20.1,
+  // 14208 (3) 23.8 / 20.1; 14208 x 8192 53.5 / 62.0, 18944 x 8192 (4) 71.6 / 74.9. More rows: 31 x 1024 x 2560 9.3 / 33.9, 31 x 4096 x 4096 (4)
+  // 38.5 / 49.7, 24 x 6144 x 2560 (4) 30.1 / 32.7, 300 x 1000 x 2560 (9) 62 / 38.
+  const uint64_t waves = ((uint64_t)row_tiles * ((M + 7) / 8) + 2 * sms - 1) / (2 * sms);
+  const bool split = nb > 1 && waves * (8 + nb) <= (M <= 8 ? 4u : 7u) * nb;
+  const unsigned nt = split || M <= 8 ? 1 : 2;
+  const dim3 grid((M + 8 * nt - 1) / (8 * nt), split ? row_tiles : (row_tiles + Q6M_WARPS - 1) / Q6M_WARPS);
   // one tile of rows: four CTAs per SM where three would not hold them all (8 x 32768 x 4096 61.2 -> 50.2 us, 8 x 151936 x 2560 128.2 ->
   // 122.5; 64 CTAs, 5 x 4096 x 4096, 36.9 instead of 30.0)
-  const bool dense = nt == 1 && cfg.gridDim.x * cfg.gridDim.y > 3u * (unsigned)sm_count();
-  const cudaError_t e = cudaLaunchKernelEx(&cfg, dense     ? gemm_q6_K_mma_kernel<1, 4>
-                                                 : nt == 1 ? gemm_q6_K_mma_kernel<1, 3>
-                                                           : gemm_q6_K_mma_kernel<2, 3>,
+  const bool dense = nt == 1 && grid.x * grid.y > 3u * sms;
+  const auto kernel = split     ? gemm_q6_K_mma_kernel<1, 2, true>
+                      : dense   ? gemm_q6_K_mma_kernel<1, 4, false>
+                      : nt == 1 ? gemm_q6_K_mma_kernel<1, 3, false>
+                                : gemm_q6_K_mma_kernel<2, 3, false>;
+  if (split) {
+    static std::atomic<uint64_t> done{0}; // a bit per device
+    int dev = 0;
+    NNTR_CHECK_CUDA(cudaGetDevice(&dev));
+    if (dev >= 64 || !(done.load(std::memory_order_acquire) >> dev & 1)) {
+      NNTR_CHECK_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, Q6S_SMEM));
+      if (dev < 64)
+        done.fetch_or(1ull << dev, std::memory_order_release);
+    }
+  }
+  const cudaError_t e = launch_in_clusters(kernel, grid, 1, (split ? Q6S_WARPS : Q6M_WARPS) * 32, split ? Q6S_SMEM : 0, st,
                                            static_cast<const uint8_t *>(ws), static_cast<const uint8_t *>(B), C, (int)ldc,
                                            (int)M, (int)N, nb);
   count_launch();

@@ -52,7 +52,7 @@ def test_tile_edges(be, port, q, gen, M, N, K):
 
 
 @pytest.mark.parametrize("M,N,K", [(2, 1, 256), (7, 17, 768), (8, 130, 2560), (9, 33, 512), (31, 4097, 2304),
-                                   (5, 28497, 512)])
+                                   (5, 28497, 512), (3, 50, 4352), (24, 16, 2048)])
 def test_tile_edges_q6_K(be, port, M, N, K):
     """Rows of 210-byte blocks at every alignment (odd and even blocks per row), N that ends inside a tile of 16."""
     rng = np.random.default_rng(M + N + K)
