@@ -46,7 +46,7 @@
  *               as soon as the MMAs that read its slot have retired.
  *   warp 18     one thread starts the tiled copies of the packed weights
  *               (Q4_K, Q4_0) into a ring of two (pair: four) stages.
- * Three stages of 64 KB (pair: four of 48), both accumulators (512 columns) in tensor memory. Every wait is bounded (pipeline.cuh).
+ * Three stages of 64 KB (pair: four of 48; Q6_K alone: two of 64), both accumulators (512 columns) in tensor memory. Every wait is bounded (pipeline.cuh).
  *
  * What bounds it. A stage's MMAs take 1024 clocks. A CTA alone takes 1310 a stage: its producers, and the shared memory, which
  * carries 96 KB for the MMAs, 64 of stores and copies and the packed weights. A pair takes 1070, the MMAs: half of the expansion and 64 KB
@@ -76,6 +76,8 @@ constexpr int F16_TILE_N = 256;  // weight rows of a tile of C, at most
 constexpr int F16_KS = 64;       // K per stage
 constexpr int F16_A_BYTES = F16_TILE_M * F16_KS * 2; // 16 KB
 constexpr int F16_PRODUCERS = 512;
+constexpr int F16_TURN_PITCH = 68; // floats of a row of the epilogue's areas: 16-byte pieces of neighbours fall into different banks
+constexpr int F16_TURN_BYTES = F16_PRODUCERS * F16_TURN_PITCH * 4; // in the stages' place
 constexpr int F16_MMA_WARP = F16_PRODUCERS / 32;
 constexpr int F16_COPY_WARP = F16_MMA_WARP + 1;
 constexpr int F16_RAW_WARP = F16_COPY_WARP + 1;
@@ -86,7 +88,9 @@ template <int QT, int MODE> struct F16Cfg {
   static constexpr int W_ROWS = MODE == F16_PAIR ? F16_TILE_N / 2 : F16_TILE_N; // weight rows that a CTA expands
   static constexpr int W_BYTES = W_ROWS * F16_KS * 2;
   static constexpr int STAGE_BYTES = W_BYTES + 2 * F16_A_BYTES; // weights + two activation tiles
-  static constexpr int STAGES = MODE == F16_PAIR ? 4 : 3;
+  /* Q6_K: two, because the producers' loads live on the L1 cache that shared memory leaves (three: 256 x 151936 x 2560 280 us, 274;
+   * 100 x 4096 x 4096 36.7, 33.8) */
+  static constexpr int STAGES = MODE == F16_PAIR ? 4 : QT == NNTR_Q6_K ? 2 : 3;
   /* Groups of producers, each with the next stage in turn. Q4_K, Q4_0: a thread per weight row; Q6_K: two, and two stages in turn */
   static constexpr int GROUPS = F16_PRODUCERS / (QT == NNTR_Q6_K ? 2 * W_ROWS : W_ROWS);
   static constexpr int STAGE_WARPS = F16_PRODUCERS / 32 / GROUPS;
@@ -98,7 +102,7 @@ template <int QT, int MODE> struct F16Cfg {
   static constexpr int RAW_BOX = QT == NNTR_Q4_K ? 128 : 144;
   static constexpr int RAW_BYTES = QT == NNTR_Q6_K ? 0 : ROW_GROUPS * 2 * RAW_BOX;
   static constexpr int HDR_BYTES = ROW_GROUPS * 128;
-  static constexpr int OFF_RAW = STAGES * STAGE_BYTES;
+  static constexpr int OFF_RAW = STAGES * STAGE_BYTES > F16_TURN_BYTES ? STAGES * STAGE_BYTES : F16_TURN_BYTES;
   static constexpr int OFF_HDR = OFF_RAW + RAW * RAW_BYTES;
   static constexpr int OFF_BARS = OFF_HDR + (QT == NNTR_Q4_K ? 2 * HDR_BYTES : 0);
   static constexpr int SMEM = OFF_BARS + 256;
@@ -269,7 +273,7 @@ gemm_f16_kernel(const __grid_constant__ CUtensorMap wmap, const uint8_t *__restr
   // Epilogue. A lane holds a row of the accumulator; stored as it is, a store instruction would touch 32 rows of C with 16
   // bytes each (27 of a tile's 142 thousand clocks). Every warp turns its 32 x 64 part round in the stages' memory, which is
   // free then, and whole lines are written from there.
-  constexpr int PITCH = 68; // floats: 16-byte pieces of neighbouring rows fall into different banks
+  constexpr int PITCH = F16_TURN_PITCH;
   bool tile_done = false;   // warps 0-15: all MMAs have retired
   auto turn_area = [&](int w) { return w * (32 * PITCH); }; // of the warp with lanes 32 * (w & 3) .., columns 64 * (w >> 2) ..
   auto turn_round = [&](int hm) {

@@ -234,7 +234,8 @@ def test_fp16_tensor_gemm_every_tile_sees_the_same_weights(be, q, K):
 @pytest.mark.parametrize("q,M,N,K", [("q4_0", 257, 256, 64), ("q4_0", 385, 512, 448), ("q4_0", 513, 9984, 704), ("q4_K", 300, 512, 256),
                                      ("q4_K", 641, 9984, 512), ("q4_K", 897, 10240, 2304), ("q6_K", 260, 300, 256),
                                      ("q6_K", 513, 10001, 768), ("q4_K", 200, 20480, 512),
-                                     ("q4_0", 130, 19200, 320), ("q6_K", 100, 20001, 256)])
+                                     ("q4_0", 130, 19200, 320), ("q6_K", 100, 20001, 256), ("q4_K", 100, 19456, 768),
+                                     ("q4_0", 40, 24320, 2880), ("q6_K", 200, 32768, 1024)])
 def test_fp16_tensor_gemm_in_pairs_of_ctas_and_narrow_tiles(be, q, M, N, K):
     """More than 256 rows and no cut along K: two CTAs share a tile of 512 rows. Tiles of fewer than 256 weight rows, for pairs and for
     single CTAs, the last one ragged. One stage, fewer stages than producer groups,
