@@ -87,11 +87,13 @@ def _gemm(qtype: str, M: int, N: int, K: int, A, lda: int, B, ldb: int, C, ldc: 
             check(rc)
         return C
     need = int(L.nntr_cuda_gemm_workspace_bytes(QTYPE[qtype], M, N, K))
-    if need and (workspace is None or workspace.numel() * workspace.element_size() < need):
-        workspace = torch.empty(need, dtype=torch.uint8, device=A.device)
-    ws_ptr = workspace.data_ptr() if workspace is not None else 0
     ws_len = workspace.numel() * workspace.element_size() if workspace is not None else 0
-    check(fn(M, N, K, A.data_ptr(), lda, B.data_ptr(), ldb, C.data_ptr(), ldc, ws_ptr, ws_len, _stream()))
+    if ws_len < need:
+        workspace, ws_len = torch.empty(need, dtype=torch.uint8, device=A.device), need
+    rc = fn(M, N, K, A.data_ptr(), lda, B.data_ptr(), ldb, C.data_ptr(), ldc,
+            workspace.data_ptr() if workspace is not None else 0, ws_len, _stream())
+    if rc:
+        check(rc)
     return C
 
 
