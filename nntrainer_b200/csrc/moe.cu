@@ -64,10 +64,10 @@ constexpr int MOE_COUNTER_TOKENS = 4096;   // arrival counters kept at the start
 constexpr int ROUTER_WARPS = 8;
 constexpr int ROUTER_SLICES = 32; // CTAs per token
 constexpr int MAX_E_PER_LANE = 8; // up to 256 experts
-// Tokens from which the router takes eight of them at a time. The line is a cautious one: a layer with 8 of 128 experts and H =
-// 2048, with a CTA row per token / with eight tokens per CTA row, 16 / 24 / 32 / 48 / 64 tokens: 98.7 / 114.2 / 126.3 / 136.4 /
-// 147.5 us, 97.8 / 111.7 / 121.7 / 128.1 / 134.0.
-constexpr unsigned ROUTER_ROWS_MIN_TOKENS = 48;
+// Tokens from which the router takes eight of them at a time. Layers of 4 of 32 experts of 2880 x 2880, a CTA row per token / eight
+// tokens per CTA row, 12 / 16 / 24 / 40 tokens: 116.8 / 118.0 / 120.3 / 123.5 us, 112.0 / 114.7 / 119.1 / 119.0; 8 of 128 of 2048 x 768, 16 / 24 /
+// 32 / 40 / 48: 82.0 / 89.6 / 103.0 / 105.6 / -, 88.1 / 91.6 / 103.7 / 104.8 / 109.4; 8 of 256 of 1024 x 512, 16 / 32: 53.7 / 74.7, 55.2 / 72.0.
+static unsigned router_rows_min_tokens(unsigned experts) { return experts <= 32 ? 12 : 40; }
 /** rows of a warp's slice fetched before the dependency wait: all of them for hidden sizes up to 2048 (96 experts and fewer: 3072) */
 template <int PER> constexpr int ROUTER_PRE = PER < 4 ? 12 : 8;
 
@@ -375,8 +375,8 @@ moe_router_kernel(const float *__restrict__ x, const float *__restrict__ wr, int
  * instead of once per token, and the last arriver's warps finish a token each. Every sum is formed in the order of the kernel
  * above (row by row inside a warp, then warp by warp, then slice by slice), so a token is routed alike by both. 256 tokens,
  * 2048 x 128 weights: 34 us, 94 with a CTA row per token. */
-template <int TT, int PER> // tokens, experts per lane
-__global__ void __launch_bounds__(ROUTER_WARPS * 32)
+template <int TT, int PER, int CTAS> // tokens, experts per lane, CTAs per SM that the registers are held to
+__global__ void __launch_bounds__(ROUTER_WARPS * 32, CTAS)
 moe_router_rows_kernel(const float *__restrict__ x, const float *__restrict__ wr, int T, int H, int E, const RouterOut o) {
   extern __shared__ float rsm[]; // [ROUTER_WARPS][TT][E], then the slice of the activations [TT][rows]
   __shared__ bool is_last;
@@ -830,16 +830,20 @@ static int moe_forward(const nntr_moe_desc *d, const nntr_moe_ep *epd, unsigned 
     attr[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
-    if (grouped && tokens >= ROUTER_ROWS_MIN_TOKENS && H <= 14336) { // its slices of eight tokens must fit in 48 KB beside the partial sums
+    if (grouped && tokens >= router_rows_min_tokens(E) && H <= 14336) { // its slices of eight tokens must fit in 48 KB beside the partial sums
       // eight tokens per CTA row (four where the experts' partial sums would not fit)
       const int tt = E <= 128 ? 8 : 4;
       cfg.gridDim = dim3((tokens + tt - 1) / tt, ROUTER_SLICES);
       cfg.dynamicSmemBytes = std::max((size_t)ROUTER_WARPS * tt * E + (size_t)tt * (H / ROUTER_SLICES + ROUTER_WARPS),
                                       (size_t)ROUTER_WARPS * (E + 32)) * sizeof(float);
-      const auto kernel = E <= 32   ? moe_router_rows_kernel<8, 1>
-                          : E <= 64  ? moe_router_rows_kernel<8, 2>
-                          : E <= 128 ? moe_router_rows_kernel<8, 4>
-                                     : moe_router_rows_kernel<4, 8>;
+      // 79 registers leave three CTAs per SM, 64 (fewer rows on their way) four: better once the three would need a third round
+      // (128 experts: 256 / 400 tokens 162.9 / 210.8 -> 160.2 / 206.7 us a layer, but 48 / 128 tokens 109.4 / 124.9 -> 111.4 / 126.1)
+      const bool many = cfg.gridDim.x * ROUTER_SLICES > 6u * (unsigned)sm_count();
+      const auto kernel = E <= 32   ? moe_router_rows_kernel<8, 1, 4>
+                          : E <= 64 ? moe_router_rows_kernel<8, 2, 4>
+                          : E > 128 ? moe_router_rows_kernel<4, 8, 2>
+                          : many    ? moe_router_rows_kernel<8, 4, 4>
+                                    : moe_router_rows_kernel<8, 4, 3>;
       NNTR_CHECK_CUDA(cudaLaunchKernelEx(&cfg, kernel, x, d->router_w, (int)tokens, (int)H, (int)E, out));
     } else {
       NNTR_CHECK_CUDA(cudaLaunchKernelEx(&cfg, router_kernel(E), x, d->router_w, (int)H, (int)E, out, ep));
