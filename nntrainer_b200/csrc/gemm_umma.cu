@@ -420,9 +420,10 @@ gemm_q4_K_umma_kernel(const uint8_t *__restrict__ atiles, const BlockQ4Kx8 *__re
  * reference's 4-row quantizer, the others that of its row quantizer. */
 __global__ void __launch_bounds__(256)
 quantize_q8_K_tiles_kernel(const float *__restrict__ x, int64_t ldx, uint8_t *__restrict__ tiles, int M, int M4,
-                           int Mpad, int nb) {
+                           int Mpad, int nb, int early) {
   pdl_wait();
-  pdl_launch_dependents(); // the GEMM behind fetches weights, which a kernel in front of this one may have written, and waits for the rest
+  if (early)
+    pdl_launch_dependents(); // the GEMM behind fetches weights, which a kernel in front of this one may have written, and waits for the rest
   const int lane = threadIdx.x & 31;
   const int64_t blk = (int64_t)blockIdx.x * 8 + (threadIdx.x >> 5);
   if (blk >= (int64_t)Mpad * nb)
@@ -462,6 +463,11 @@ bool umma_supported(int qtype, unsigned M, unsigned N, unsigned K) {
   return qtype == NNTR_Q4_K && M >= 2 && N % TILE_N == 0 && K % QK_K == 0 && K > 0;
 }
 
+/* Super-blocks of K, walked by one CTA, up to which the quantizer lets the GEMM start early. 40 x 2560 x 9728 (in parts) 30.7 -> 29.7 us, 256 x 2560 x 2560 30.7 -> 30.0 us, 100 x 8320 x 2560 20.7 -> 19.8, 64 x 4096 x
+ * 4096 17.8 -> 17.2, but 44 x 10880 x 12032 118.8 -> 120.0: CTAs that come in between the quantizer's last ones lie unevenly, and a long K
+ * pays for that longer. */
+constexpr int EARLY_BLOCKS = 32;
+
 int launch_gemm_q4_K_umma(unsigned M, unsigned N, unsigned K, const float *A, const void *B, float *C, unsigned ldc,
                           void *ws, cudaStream_t st) {
   static bool attr_set[64] = {};
@@ -477,10 +483,6 @@ int launch_gemm_q4_K_umma(unsigned M, unsigned N, unsigned K, const float *A, co
   const unsigned M4 = (M / 4) * 4;
   if ((reinterpret_cast<uintptr_t>(A) & 15) || (reinterpret_cast<uintptr_t>(ws) & 15))
     return set_error(NNTR_CUDA_ERR_INVALID, "gemm (tensor path): activations and workspace must be 16-byte aligned");
-  const int64_t nwarps = (int64_t)Mpad * nb;
-  NNTR_CHECK_CUDA(launch_in_clusters(quantize_q8_K_tiles_kernel, dim3((unsigned)((nwarps + 7) / 8)), 1, 256, 0, st, A, (int64_t)K,
-                                     static_cast<uint8_t *>(ws), (int)M, (int)M4, Mpad, nb));
-  count_launch();
   const int c_vec4 = (ldc % 4 == 0) && !(reinterpret_cast<uintptr_t>(C) & 15);
   dim3 grid(mtiles, N / TILE_N);
   // Few tiles: K in as many parts as run in one wave of clusters. A CTA alone walks K at 2.5 us a super-block however many SMs
@@ -494,6 +496,10 @@ int launch_gemm_q4_K_umma(unsigned M, unsigned N, unsigned K, const float *A, co
     parts /= 2;
   if (parts == 2 && mtiles > 1)
     parts = 1;
+  const int64_t nwarps = (int64_t)Mpad * nb;
+  NNTR_CHECK_CUDA(launch_in_clusters(quantize_q8_K_tiles_kernel, dim3((unsigned)((nwarps + 7) / 8)), 1, 256, 0, st, A, (int64_t)K,
+                                     static_cast<uint8_t *>(ws), (int)M, (int)M4, Mpad, nb, (int)(parts > 1 || nb <= EARLY_BLOCKS)));
+  count_launch();
   const cudaError_t e = launch_in_clusters(parts > 1 ? gemm_q4_K_umma_kernel<true> : gemm_q4_K_umma_kernel<false>, grid, parts, CTA_THREADS, SMEM_BYTES, st,
                                            static_cast<const uint8_t *>(ws), static_cast<const BlockQ4Kx8 *>(B), C, (int)ldc,
                                            (int)M, nb, c_vec4);
