@@ -22,9 +22,10 @@
  * shared memory by bulk copies (which leave the L1 cache to the activations), and the words read there are funnel-shifted.
  *
  * A warp owns 16 weight rows and up to 16 activation rows (32 chain accumulators per 8 rows) over all of K and shares
- * nothing with other warps. Bound by the unpack (about 390 logic and 270 multiply instructions per 16 x 256 weights, at
- * half rate both): 8 x 151936 x 2560 129 us (CUDA-core kernel before: 697; the weights' bytes alone take 49), 31 rows 339 us
- * (2360). Bringing the rows in by 4- and 8-byte asynchronous copies or through registers measured the same or slower.
+ * nothing with other warps; with few rows eight warps share them along K (SPLIT below). Bound by the unpack (about 390 logic and 270
+ * multiply instructions per 16 x 256 weights, at half rate both; issue slots 58 % full, the logic pipe 54 %): 8 x 151936 x 2560 124 us
+ * (CUDA-core kernel before: 697; the weights' bytes alone take 49), 31 rows 339 us (2360). Bringing the rows in by 4- and 8-byte
+ * asynchronous copies or through registers measured the same or slower.
  */
 #include "cluster.cuh"
 #include "common.cuh"

@@ -374,7 +374,7 @@ moe_router_kernel(const float *__restrict__ x, const float *__restrict__ wr, int
 /* The same for a batch: a CTA takes TT tokens through its slice, so that the router weight crosses the L2 once per TT tokens
  * instead of once per token, and the last arriver's warps finish a token each. Every sum is formed in the order of the kernel
  * above (row by row inside a warp, then warp by warp, then slice by slice), so a token is routed alike by both. 256 tokens,
- * 2048 x 128 weights: 34 us, 94 with a CTA row per token. */
+ * 2048 x 128 weights: 22.5 us (code for 256 experts and divisions by run-time numbers 34), 94 with a CTA row per token. */
 template <int TT, int PER, int CTAS> // tokens, experts per lane, CTAs per SM that the registers are held to
 __global__ void __launch_bounds__(ROUTER_WARPS * 32, CTAS)
 moe_router_rows_kernel(const float *__restrict__ x, const float *__restrict__ wr, int T, int H, int E, const RouterOut o) {
