@@ -847,7 +847,7 @@ attn_cluster_kernel(const __grid_constant__ CUtensorMap kmap, const __grid_const
   int vbuf = 0, tbuf = 0;
   uint32_t vpar = 0, tpar = 1;
   auto turn = [&](unsigned t) {
-    if (!mbar_wait_bounded(vfull0 + 8 * vbuf, vpar, abort_flag, &g_attn_status, AC_POLLS, 1024))
+    if (!mbar_wait_warp(vfull0 + 8 * vbuf, vpar, abort_flag, &g_attn_status, AC_POLLS, 1024))
       return false;
     const int units = (int)(min(cached - t * VROWS, (unsigned)VROWS) + 31) / 32 * 4;
     const uint32_t src = vsm + vbuf * vbytes, dst = ksm + tbuf * AC_TBYTES;
@@ -906,7 +906,7 @@ attn_cluster_kernel(const __grid_constant__ CUtensorMap kmap, const __grid_const
     __syncwarp();
   } else if (turner) {
     while (ok && turned < v_tiles)
-      ok = mbar_wait_bounded(tempty0 + 8 * tbuf, tpar, abort_flag, &g_attn_status, AC_POLLS, 1024) && turn(turned++);
+      ok = mbar_wait_warp(tempty0 + 8 * tbuf, tpar, abort_flag, &g_attn_status, AC_POLLS, 1024) && turn(turned++);
   } else if (TURN && warp == 0) {
     // Thirty-two rows in the chain while the next thirty-two are on their way: twelve loads, where row by row it would be forty, whose
     // latency the chain's four clocks a row do not hide.

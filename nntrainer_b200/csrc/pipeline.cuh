@@ -68,6 +68,13 @@ __device__ __forceinline__ bool mbar_wait_bounded(uint32_t bar, uint32_t parity,
   return false;
 }
 
+/** The same for all lanes of a warp: true in every one or in none. Two lanes may learn of the phase's end and of the abort flag in
+ *  turn; in front of an instruction that takes the whole warp (ldmatrix, __syncwarp) they have to leave together. */
+__device__ __forceinline__ bool mbar_wait_warp(uint32_t bar, uint32_t parity, volatile int *abort_flag, int *status, uint32_t polls,
+                                               uint32_t spin) {
+  return __all_sync(FULL, mbar_wait_bounded(bar, parity, abort_flag, status, polls, spin)) != 0;
+}
+
 /** A chain that goes from warp to warp: the warp in front arrives at barrier `id`, the one behind waits for it. Number 0 is the
  *  barrier of __syncthreads(): where it is used for a hand-over, no barrier of the whole CTA may lie between the first and the last. */
 __device__ __forceinline__ void pair_arrive(int id) { asm volatile("barrier.cta.arrive %0, 64;" ::"r"(id) : "memory"); }
