@@ -26,7 +26,7 @@
  * expansion (about two instructions per weight) and one epilogue per tile.
  *
  * Up to 256 activation rows, a CTA owns two tiles of 128 of them (MMA M, tensor-memory lanes) against the same 256 weight rows (MMA N,
- * columns), so every expanded weight stage feeds two MMAs. With more rows a pair of CTAs owns four tiles: each CTA expands half of the
+ * columns), so every expanded weight stage feeds two MMAs. With more rows mostly a pair of CTAs owns four tiles: each CTA expands half of the
  * weight rows, an MMA (cta_group::2) takes 128 activation rows of each and the weights of both, and an expanded stage feeds 512 rows.
  * A CTA walks K in stages of 64 (one pair of sub-blocks):
  *   warps 0-15  producers: expand a stage's nibble bytes into 64 fp16 values per
@@ -806,6 +806,12 @@ int even_rows(int m_groups, int N, int slots, int step) {
   return std::min(F16_TILE_N, std::max(128, (rows + step - 1) / step * step));
 }
 
+/** What the tiles of m_groups rows of them take, in units of a stage of a tile: rounds over the slots that run at a time, each as long as
+ *  its tiles are high. */
+int64_t rounds_cost(int m_groups, int N, int slots, int tile_rows) {
+  return ((int64_t)m_groups * ((N + tile_rows - 1) / tile_rows) + slots - 1) / slots * (224 + tile_rows);
+}
+
 /** allows every form of the kernel its shared memory, once per device */
 template <int QT> int allow_smem() {
   static std::atomic<uint64_t> done{0};
@@ -829,14 +835,25 @@ int launch_typed(unsigned M, unsigned N, unsigned K, const uint8_t *tiles, const
   if (const int rc = allow_smem<QT>())
     return rc;
   const int parts = k_parts<QT>(cta_m * n_tiles, k_stages);
-  const bool pair = parts == 1 && mtiles > 2;
+  bool pair = false;
   int tile_rows = F16_TILE_N;
-  if (pair) {
-    static ClusterFit fit;
-    cta_m = (mtiles + 3) / 4;
-    tile_rows = even_rows(cta_m, (int)N, fit(gemm_f16_kernel<QT, F16_PAIR>, 2, F16_THREADS, F16Cfg<QT, F16_PAIR>::SMEM), 32);
-  } else if (parts == 1) {
+  if (parts == 1) {
     tile_rows = even_rows(cta_m, (int)N, sm_count(), 16);
+    // Pairs where their rounds take less: a stage of a tile of r weight rows takes them about (224 + r) units and a CTA alone 1.2 (Q6_K:
+    // 1.5) times as many, but a pair that has fewer than four tiles of activations works for the missing ones too, and its rounds hold
+    // half as many tiles. Q4_K, pairs / CTAs alone: 300 x 24576 x 4096 91.4 / 103.8 us, 512 95.5 / 107, 603 140.7 / 117.8, 768 143.5 / 129.6,
+    // 859 157 / 169.6, 1024 161 / 182.6; 9728 x 2560 512 / 768 / 1024 rows 33.4 / 37.0, 61.9 / 40.2, 64.8 / 70.2; 8192 x 8192 768 rows 93.7 / 106.5;
+    // Q4_0 19456 x 2560 768 / 1280 / 1792 rows 90.5 / 73.5, 126.3 / 115.1, 161.6 / 156.3; Q6_K 9728 x 2560 768 rows 64.4 / 58.4, 1280
+    // 76.8 / 101.2. Of 315 sizes of 257 to 2048 rows the other form is by no more than 2 % the faster one.
+    if (mtiles > 2) {
+      static ClusterFit fit;
+      const int quads = (mtiles + 3) / 4, slots = fit(gemm_f16_kernel<QT, F16_PAIR>, 2, F16_THREADS, F16Cfg<QT, F16_PAIR>::SMEM);
+      const int pair_rows = even_rows(quads, (int)N, slots, 32);
+      pair = slots > 0 && 10 * rounds_cost(quads, (int)N, slots, pair_rows) <=
+                            (QT == NNTR_Q6_K ? 15 : 12) * rounds_cost(cta_m, (int)N, sm_count(), tile_rows);
+      if (pair)
+        cta_m = quads, tile_rows = pair_rows;
+    }
   } else if (mtiles > 1 && parts == k_parts<QT>(mtiles * n_tiles, k_stages)) {
     // tiles one by one if they run in the same wave as the pairs: 128 instead of 256 columns of MMAs per stage and one sum at the
     // end instead of two (256 x 1280 x 2560 Q4_0: 24 -> 16 us)

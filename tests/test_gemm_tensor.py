@@ -235,9 +235,11 @@ def test_fp16_tensor_gemm_every_tile_sees_the_same_weights(be, q, K):
                                      ("q4_K", 641, 9984, 512), ("q4_K", 897, 10240, 2304), ("q6_K", 260, 300, 256),
                                      ("q6_K", 513, 10001, 768), ("q4_K", 200, 20480, 512),
                                      ("q4_0", 130, 19200, 320), ("q6_K", 100, 20001, 256), ("q4_K", 100, 19456, 768),
-                                     ("q4_0", 40, 24320, 2880), ("q6_K", 200, 32768, 1024)])
+                                     ("q4_0", 40, 24320, 2880), ("q6_K", 200, 32768, 1024), ("q4_0", 513, 8192, 704),
+                                     ("q4_K", 641, 8192, 512), ("q4_K", 800, 10240, 2304), ("q6_K", 513, 8200, 768),
+                                     ("q6_K", 700, 9728, 512)])
 def test_fp16_tensor_gemm_in_pairs_of_ctas_and_narrow_tiles(be, q, M, N, K):
-    """More than 256 rows and no cut along K: two CTAs share a tile of 512 rows. Tiles of fewer than 256 weight rows, for pairs and for
+    """More than 256 rows and no cut along K: mostly two CTAs share a tile of 512 rows. Tiles of fewer than 256 weight rows, for pairs and for
     single CTAs, the last one ragged. One stage, fewer stages than producer groups,
     an odd count; tiles of three, five and seven times 128 rows, whose last pair has a tile in one CTA only; a ragged last row and
     (Q6_K) a ragged last column; an odd row stride of C. Every 512 weight rows are alike, so C's columns have to be, bit for bit.
@@ -266,6 +268,23 @@ def test_fp16_tensor_gemm_in_pairs_of_ctas_and_narrow_tiles(be, q, M, N, K):
         assert torch.equal(got[:, c:c + n], got[:, :n])
     for _ in range(5):
         assert torch.equal(call("tensor_f16", N).view(torch.int32), got.view(torch.int32))
+
+
+@pytest.mark.parametrize("q,M,N,K,pairs", [
+    ("q4_K", 512, 9728, 2560, True), ("q4_K", 513, 9728, 2560, False), ("q4_K", 768, 9728, 2560, False), ("q4_K", 769, 9728, 2560, True),
+    ("q4_K", 700, 24576, 4096, False), ("q4_K", 700, 8192, 8192, True), ("q4_K", 1024, 24576, 4096, True), ("q4_0", 700, 12288, 2560, False),
+    ("q4_0", 1280, 19456, 2560, False), ("q6_K", 700, 9728, 2560, False), ("q6_K", 1280, 19456, 2560, True)])
+def test_fp16_tensor_gemm_is_given_to_pairs_where_they_fill_their_rounds(be, captured, q, M, N, K, pairs):
+    """A pair of CTAs takes 512 rows at a time, 148 SMs hold 74 pairs: 513 rows of 9728 weights are two rounds of pairs, half of them
+    empty, and one round of CTAs with 256 rows each. Every size here was measured in both forms, at least 5 % apart."""
+    nbytes = {"q4_K": 144 * K // 256, "q4_0": 18 * K // 32, "q6_K": 210 * K // 256}[q]
+    A, C = torch.zeros(M, K, device="cuda"), torch.empty(M, N, device="cuda")
+    B = torch.zeros(N * nbytes, dtype=torch.uint8, device="cuda")
+    ws = torch.empty(be.gemm_workspace_bytes(q, M, N, K), dtype=torch.uint8, device="cuda")
+    be.set_gemm_path("tensor_f16")
+    launches = captured(lambda: getattr(be, f"gemm_{q}")(M, N, K, A, K, B, N, C, N, ws))
+    be.set_gemm_path("auto")
+    assert [x.cluster for x in launches] == [1, 2 if pairs else 1]
 
 
 def test_int8_peak_measurement_is_plausible(be):
