@@ -265,7 +265,10 @@ gemm_f16_kernel(const __grid_constant__ CUtensorMap wmap, const uint8_t *__restr
   __syncthreads();
   if (PAIR)
     cluster_sync(); // the other CTA's barriers and tensor memory are there
-  if (!SHARED) // (shared tiles: 1024 x 2560 x 9728 85.0 us instead of 83.6)
+  // Only pairs let the next launch in early: Q4_K 512 x 14336 x 4096 50.6 us, without 51.6. CTAs alone are slowed down by its waiting CTAs:
+  // Q4_K 256 x 24576 x 4096 55.3 us, without 53.8, 1280 x 37888 x 4096 333 and 324, 603 x 9728 x 2560 39.8 and 38.9; shared tiles, 1024 x 2560 x
+  // 9728, 85.0 and 83.6.
+  if (PAIR)
     pdl_launch_dependents();
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
   const uint32_t tmem = *tmem_slot;
