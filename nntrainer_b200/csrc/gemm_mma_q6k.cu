@@ -72,7 +72,7 @@ constexpr int LUT_AND_XOR = 0x6A; // (a & b) ^ c
 
 /* CTAS: CTAs per SM that registers and shared memory are held to. Four with 4 bytes of spills and two stages (which leave the L1
  * cache room for the activations; with three stages 137 us instead of 122 for 8 x 151936 x 2560, three CTAs of three stages 128), where
- * three per SM would need a second round. */
+ * four per SM need fewer rounds. */
 template <int CTAS> constexpr int Q6M_STAGES = CTAS == 3 ? 3 : 2;
 /* SPLIT: the CTA has eight warps, all of them on the same 16 weight rows, and each takes every eighth super-block; the chains go from warp
  * to warp, one super-block further at each. For calls with too few rows to fill the chip, where the 3400 clocks that a warp on its own
@@ -364,9 +364,12 @@ int launch_gemm_mma_q6_K(unsigned M, unsigned N, unsigned K, const float *A, con
   const bool split = nb > 1 && waves * (8 + nb) <= (M <= 8 ? 4u : 7u) * nb;
   const unsigned nt = split || M <= 8 ? 1 : 2;
   const dim3 grid((M + 8 * nt - 1) / (8 * nt), split ? row_tiles : (row_tiles + Q6M_WARPS - 1) / Q6M_WARPS);
-  // one tile of rows: four CTAs per SM where three would not hold them all (8 x 32768 x 4096 61.2 -> 50.2 us, 8 x 151936 x 2560 128.2 ->
-  // 122.5; 64 CTAs, 5 x 4096 x 4096, 36.9 instead of 30.0)
-  const bool dense = nt == 1 && grid.x * grid.y > 3u * sms;
+  // One tile of rows: four CTAs per SM where that saves a round, each of which takes them about a fifth longer. Three / four CTAs, 8 rows: 37072 x
+  // 2560 (580 CTAs, two rounds / one) 41.4 / 30.7 us, 40912 x 2560 (640: two / two) 42.2 / 44.6, 56272 x 4096 (880: two / two) 76.3 / 91.8, x
+  // 8192 150 / 195, 61392 x 2560 (960: three / two) 61.6 / 54.6, 83152 x 4096 (1300: three / three) 111.5 / 124.3, 151936 x 2560 (six / five) 128.2 /
+  // 122.5; 64 CTAs, 5 x 4096 x 4096, 30.0 / 36.9.
+  const unsigned ctas = grid.x * grid.y;
+  const bool dense = nt == 1 && (ctas + 4 * sms - 1) / (4 * sms) < (ctas + 3 * sms - 1) / (3 * sms);
   const auto kernel = split     ? gemm_q6_K_mma_kernel<1, 2, true>
                       : dense   ? gemm_q6_K_mma_kernel<1, 4, false>
                       : nt == 1 ? gemm_q6_K_mma_kernel<1, 3, false>

@@ -14,7 +14,7 @@ def pytest_configure(config):
 
 
 class CapturedLaunch:
-    """A kernel of a captured CUDA graph: its grid, the CTAs of a cluster, and its arguments by position."""
+    """A kernel of a captured CUDA graph: its grid, the CTAs of a cluster, its static shared memory, and its arguments by position."""
 
     def __init__(self, node):
         from cuda.bindings import driver
@@ -24,6 +24,8 @@ class CapturedLaunch:
         err, value = driver.cuGraphKernelNodeGetAttribute(node, driver.CUlaunchAttributeID.CU_LAUNCH_ATTRIBUTE_CLUSTER_DIMENSION)
         assert err == driver.CUresult.CUDA_SUCCESS
         self.cluster = max(1, value.clusterDim.x)
+        err, self.static_shared = driver.cuFuncGetAttribute(driver.CUfunction_attribute.CU_FUNC_ATTRIBUTE_SHARED_SIZE_BYTES, self._p.func)
+        assert err == driver.CUresult.CUDA_SUCCESS
 
     def argument(self, i, ctype):
         import ctypes

@@ -51,6 +51,20 @@ def test_tile_edges(be, port, q, gen, M, N, K):
     assert np.array_equal(exact(be, q, A, B, N).view(np.uint32), want.view(np.uint32))
 
 
+@pytest.mark.parametrize("N,dense", [(28416, False), (28432, True), (37888, True), (37904, False), (56832, False), (56848, True), (75792, False),
+                                     (85264, True), (151936, True)])
+def test_q6_K_has_four_ctas_per_sm_where_that_saves_a_round(be, captured, N, dense):
+    """64 weight rows per CTA and 148 SMs: on both sides of one, two and three rounds of three and of four CTAs per SM. The two forms
+    differ in their shared memory: a CTA's four warps have three stages of 16 x 240 bytes each, with four CTAs per SM two."""
+    M, K = 8, 512
+    B = torch.zeros(N * 2 * 210, dtype=torch.uint8, device="cuda")
+    A, C = torch.zeros(M, K, device="cuda"), torch.empty(M, N, device="cuda")
+    ws = torch.empty(be.gemm_workspace_bytes("q6_K", M, N, K), dtype=torch.uint8, device="cuda")
+    launches = captured(lambda: be.gemm_q6_K(M, N, K, A, K, B, N, C, N, ws))
+    assert len(launches) == 2 and launches[1].grid == (1, (N + 63) // 64, 1)
+    assert launches[1].static_shared // (4 * 16 * 240) == (2 if dense else 3)
+
+
 @pytest.mark.parametrize("M,N,K", [(2, 1, 256), (7, 17, 768), (8, 130, 2560), (9, 33, 512), (31, 4097, 2304),
                                    (5, 28497, 512), (3, 50, 4352), (24, 16, 2048)])
 def test_tile_edges_q6_K(be, port, M, N, K):
