@@ -144,7 +144,7 @@ __device__ __forceinline__ void row_scales_half(const uint8_t *scales, int j, ui
 template <bool SHARED>
 __global__ void __maxnreg__(72)
 gemm_q4_K_umma_kernel(const uint8_t *__restrict__ atiles, const BlockQ4Kx8 *__restrict__ W, float *__restrict__ C,
-                      int ldc, int M, int k_blocks, int c_vec4) {
+                      int ldc, int M, int k_blocks, int c_vec4, int release) {
   extern __shared__ __align__(128) uint8_t smem[];
   uint64_t *bars = reinterpret_cast<uint64_t *>(smem + OFF_BARS);
   // bars: [0,1] full, [2,3] empty, [4,5] acc_full, [6,7] acc_empty, [8..11] meta_full, [12..15] head_full
@@ -182,7 +182,8 @@ gemm_q4_K_umma_kernel(const uint8_t *__restrict__ atiles, const BlockQ4Kx8 *__re
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
-  pdl_launch_dependents();
+  if (release)
+    pdl_launch_dependents();
   const uint32_t tmem = *tmem_slot;
   constexpr int SUM_PITCH = TILE_N + 4; // floats
   bool tile_done = false;               // drain warps of a shared tile: all sums in shared memory
@@ -420,10 +421,9 @@ gemm_q4_K_umma_kernel(const uint8_t *__restrict__ atiles, const BlockQ4Kx8 *__re
  * reference's 4-row quantizer, the others that of its row quantizer. */
 __global__ void __launch_bounds__(256)
 quantize_q8_K_tiles_kernel(const float *__restrict__ x, int64_t ldx, uint8_t *__restrict__ tiles, int M, int M4,
-                           int Mpad, int nb, int early) {
+                           int Mpad, int nb) {
   pdl_wait();
-  if (early)
-    pdl_launch_dependents(); // the GEMM behind fetches weights, which a kernel in front of this one may have written, and waits for the rest
+  pdl_launch_dependents(); // the GEMM behind fetches weights, which a kernel in front of this one may have written, and waits for the rest
   const int lane = threadIdx.x & 31;
   const int64_t blk = (int64_t)blockIdx.x * 8 + (threadIdx.x >> 5);
   if (blk >= (int64_t)Mpad * nb)
@@ -463,10 +463,17 @@ bool umma_supported(int qtype, unsigned M, unsigned N, unsigned K) {
   return qtype == NNTR_Q4_K && M >= 2 && N % TILE_N == 0 && K % QK_K == 0 && K > 0;
 }
 
-/* Super-blocks of K, walked by one CTA, up to which the quantizer lets the GEMM start early. 40 x 2560 x 9728 (in parts) 30.7 -> 29.7 us, 256 x 2560 x 2560 30.7 -> 30.0 us, 100 x 8320 x 2560 20.7 -> 19.8, 64 x 4096 x
- * 4096 17.8 -> 17.2, but 44 x 10880 x 12032 118.8 -> 120.0: CTAs that come in between the quantizer's last ones lie unevenly, and a long K
- * pays for that longer. */
-constexpr int EARLY_BLOCKS = 32;
+/* Whether the GEMM lets the launch behind it start early. What that saves is a launch; that launch's waiting CTAs slow the GEMM's down as
+ * long as those run, and its own start between the quantizer's last CTAs more than that where its tiles could have had an SM each. A tile
+ * shared by CTAs: where K is short for the SMs that stay free. Released / not, us: 100 x 2560 x 1024 / 4096 / 12032 (80 CTAs) 10.0 / 10.3, 16.6
+ * / 17.1, 36.6 / 35.7, 128 x 6144 x 2560 (96) 18.8 / 19.4, 128 x 4096 x 1024 / 4096 / 8192 (128) 10.5 / 11.0, 18.9 / 17.9, 28.6 / 27.4. A CTA a tile:
+ * 300 x 6144 x 1024 (144 tiles) 18.6 / 17.2, 512 x 2560 x 2560 (80) 32.0 / 30.9, 200 x 6144 x 4096 (96) 44.9 / 43.4, 400 x 10880 x 1024 (340) 44.2
+ * / 42.8; with several tiles per SM and a quantizer of more CTAs than run at a time 640 x 4096 x 6144 118.7 / 120.4, 800 x 10880 x 4096 198.7 /
+ * 201.5. */
+static bool release_early(int tiles, int parts, int nb, int64_t quantizers) {
+  const int sms = sm_count();
+  return parts > 1 ? 6 * nb <= parts * (sms - tiles * parts) : tiles > sms && quantizers > 8 * sms;
+}
 
 int launch_gemm_q4_K_umma(unsigned M, unsigned N, unsigned K, const float *A, const void *B, float *C, unsigned ldc,
                           void *ws, cudaStream_t st) {
@@ -496,13 +503,14 @@ int launch_gemm_q4_K_umma(unsigned M, unsigned N, unsigned K, const float *A, co
     parts /= 2;
   if (parts == 2 && mtiles > 1)
     parts = 1;
-  const int64_t nwarps = (int64_t)Mpad * nb;
-  NNTR_CHECK_CUDA(launch_in_clusters(quantize_q8_K_tiles_kernel, dim3((unsigned)((nwarps + 7) / 8)), 1, 256, 0, st, A, (int64_t)K,
-                                     static_cast<uint8_t *>(ws), (int)M, (int)M4, Mpad, nb, (int)(parts > 1 || nb <= EARLY_BLOCKS)));
+  const int tiles = (int)(grid.x * grid.y);
+  const int64_t quantizers = ((int64_t)Mpad * nb + 7) / 8;
+  NNTR_CHECK_CUDA(launch_in_clusters(quantize_q8_K_tiles_kernel, dim3((unsigned)quantizers), 1, 256, 0, st, A, (int64_t)K,
+                                     static_cast<uint8_t *>(ws), (int)M, (int)M4, Mpad, nb));
   count_launch();
   const cudaError_t e = launch_in_clusters(parts > 1 ? gemm_q4_K_umma_kernel<true> : gemm_q4_K_umma_kernel<false>, grid, parts, CTA_THREADS, SMEM_BYTES, st,
                                            static_cast<const uint8_t *>(ws), static_cast<const BlockQ4Kx8 *>(B), C, (int)ldc,
-                                           (int)M, nb, c_vec4);
+                                           (int)M, nb, c_vec4, (int)release_early(tiles, parts, nb, quantizers));
   count_launch();
   return check_cuda(e, "gemm_q4_K tensor-path launch");
 }

@@ -287,6 +287,23 @@ def test_fp16_tensor_gemm_is_given_to_pairs_where_they_fill_their_rounds(be, cap
     assert [x.cluster for x in launches] == [1, 2 if pairs else 1]
 
 
+@pytest.mark.parametrize("M,N,K,parts,release", [
+    (100, 2560, 1024, 4, True), (100, 2560, 12032, 4, False), (128, 4096, 1024, 4, True), (128, 4096, 4096, 4, False),
+    (128, 6144, 2560, 2, True), (300, 6144, 1024, 1, False), (200, 6144, 4096, 1, False), (400, 10880, 1024, 1, False),
+    (640, 4096, 6144, 1, True)])
+def test_integer_tensor_gemm_lets_the_next_launch_in_early_only_where_that_pays(be, captured, M, N, K, parts, release):
+    """The last argument of the kernel. Every size here was measured both ways."""
+    import ctypes
+    A, C = torch.zeros(M, K, device="cuda"), torch.empty(M, N, device="cuda")
+    B = torch.zeros(N * K // 256 * 144, dtype=torch.uint8, device="cuda")
+    ws = torch.empty(be.gemm_workspace_bytes("q4_K", M, N, K), dtype=torch.uint8, device="cuda")
+    be.set_gemm_path("tensor")
+    launches = captured(lambda: be.gemm_q4_K(M, N, K, A, K, B, N, C, N, ws))
+    be.set_gemm_path("auto")
+    assert [x.cluster for x in launches] == [1, parts]
+    assert launches[1].argument(6, ctypes.c_int) == 1 and launches[1].argument(7, ctypes.c_int) == release
+
+
 def test_int8_peak_measurement_is_plausible(be):
     """The int8 rate the prefill fraction is quoted against: a dense tcgen05 kind::i8 stream on every SM. A B200 is
     specified at 4.5 POP/s dense; anything outside 1.5 .. 6 POP/s means the measurement is not doing the work."""
