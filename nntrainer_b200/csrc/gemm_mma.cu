@@ -465,7 +465,10 @@ __global__ void __launch_bounds__(ROWS_WARPS * 32 + 32, rows_ctas<QT, NT, GROUPE
   __syncthreads();
   if (GROUPED)
     pdl_wait(); // tables and activation tiles come from the kernels before
-  else // (grouped, the next launch's CTAs would be let in beside the products: 64 tokens, 8 of 128 experts 113 -> 132 us)
+  else if (NT > 2 || (n_groups + 2 * ROWS_WARPS - 1) / (2 * ROWS_WARPS) * n_tiles * n_z > (int)gridDim.x)
+    // The next launch's CTAs are let in beside the products. Up to 16 rows and no CTA with a second item: not, 5 x 24576 x 4096 Q4_K 24.4 us,
+    // so 20.9, 8 x 24576 x 4096 Q4_0 18.5 and 17.1; more rows: 31 x 20000 x 4096 Q4_0 26.4 us, without 31.9, 40 x 9728 x 2560 Q4_K 21.7 and 23.7.
+    // (Grouped: 64 tokens, 8 of 128 experts 113 -> 132 us.)
     pdl_launch_dependents();
   int slot = 0;
   uint32_t par = 0;
