@@ -304,7 +304,9 @@ size_t nntr_cuda_attention_workspace_bytes(const nntr_attn_desc *a, unsigned max
  *  (compute_kcaches, avx2_impl.cpp:1595), softmax over those rows per head with the optional sink
  *  (softmax_row_inplace, :1181-1307), probabilities times the value cache (compute_fp16vcache_fp32_transposed, :1512):
  *  out[n_heads_q][head_dim], equal to the reference's result bit for bit. With pos_dev the grids are sized for
- *  max_rows cache rows. One launch for windows of up to 16384 rows of heads of up to 128 dimensions; else -- or with
+ *  max_rows cache rows, and pos says where the positions are expected to start (0 if that is not known): it chooses
+ *  between a form of the launch for short contexts and one for long ones, which take every position and give the same
+ *  bits. One launch for windows of up to 16384 rows of heads of up to 128 dimensions; else -- or with
  *  NNTR_CUDA_ATTN_SEPARATE in flags -- three (scores; softmax; values); same bits either way. n_heads_q % 8 == 0,
  *  head_dim % 8 == 0. */
 #define NNTR_CUDA_ATTN_SEPARATE 2u

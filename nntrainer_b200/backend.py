@@ -547,7 +547,8 @@ class Attention:
         """q [hq*hd], k, v [hkv*hd] fp32 device tensors of the token at ``pos`` -> out [hq*hd]. ``qk_norm`` = (q_gamma,
         k_gamma, eps) applies Qwen3's per-head RMS norms to q and k. One launch for windows of up to 16384 rows (up to
         2048 rows q is left as it is; ``q_rot`` receives the rotated heads if given), else -- or with ``separate`` -- the
-        rotary launch (q rotated in place) and three attention launches."""
+        rotary launch (q rotated in place) and three attention launches. With ``pos_dev`` (a device word) the position is read
+        on the device, and ``pos`` is where the positions are expected to start: it chooses the form of the launch."""
         torch = _torch()
         C = self._C
         out = torch.empty(self.hq * self.hd, dtype=torch.float32, device=q.device) if out is None else out

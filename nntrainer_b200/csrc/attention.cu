@@ -1149,8 +1149,9 @@ size_t attention_workspace_bytes(const nntr_attn_desc *a, unsigned max_rows) {
 }
 
 /* The cluster launch, or *taken = false where it does not apply: heads of more than 128 dimensions, more rows than shared
- * memory keeps, or NNTR_CUDA_ATTN_SEPARATE. */
-static int launch_attn_cluster(AttnStep a, unsigned bound, unsigned rows, unsigned flags, cudaStream_t st, bool *taken) {
+ * memory keeps, or NNTR_CUDA_ATTN_SEPARATE. bound, rows: rows of the caches and of a window that the launch must be able to take;
+ * likely: rows of the window that it is expected to have, no more than rows. */
+static int launch_attn_cluster(AttnStep a, unsigned bound, unsigned rows, unsigned likely, unsigned flags, cudaStream_t st, bool *taken) {
   const int hd = a.hd;
   *taken = false;
   if ((flags & NNTR_CUDA_ATTN_SEPARATE) || hd > 128 || rows > AC_MAX_ROWS)
@@ -1163,7 +1164,8 @@ static int launch_attn_cluster(AttnStep a, unsigned bound, unsigned rows, unsign
   // slices 3803. Alone 64 / 8 heads of 64 at 2000 / 4096 / 6000 rows 23.2 / 36.6 / 50.4 us, with slices 21.6 / 33.5 / 45.0; 32 / 8 of 128 at
   // 1500 / 5000 20.3 / 44.7 and 18.7 / 40.8. Heads whose CTAs would own 128 dimensions each leave most of the chip idle without: 32 / 4 heads
   // of 128 at 512 / 3000 rows 12.2 / 34.1, with slices 10.5 / 28.1; decode steps at 100 / 512 3012 / 3325 and 3081 / 3253, three layers at
-  // 1500 3146 and 2912.
+  // 1500 3146 and 2912. The rows that count are those that the window is likely to have: 16 tokens over three layers at a context of 100 with
+  // caches of 8192 rows, 32 / 8 heads 2160 us, with slices 2234, 64 / 8 heads of 64 2146 and 2196; at 3000 3182 and 3260, 3065 and 3180.
   const int slices = hd / 32, slice_heads = hd == 64 ? 2 : 1;
   static std::atomic<uint32_t> attr_done[64];
   static ClusterFit fit64, fit128;
@@ -1175,7 +1177,7 @@ static int launch_attn_cluster(AttnStep a, unsigned bound, unsigned rows, unsign
       NNTR_CHECK_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, AC_SMEM_ALONE));
     attr_done[dev & 63].store(1, std::memory_order_release);
   }
-  const bool sliced = !many && rows > (hd > 64 && gqa > 4 ? 256u : AC_SLICED_ROWS) && (hd == 64 || hd == 128) && gqa % slice_heads == 0 &&
+  const bool sliced = !many && likely > (hd > 64 && gqa > 4 ? 256u : AC_SLICED_ROWS) && (hd == 64 || hd == 128) && gqa % slice_heads == 0 &&
                       a.hq * slices / 4 <= (hd == 64 ? fit64(attn_cluster_kernel<64, 32>, 4, AC_THREADS, AC_SMEM_ALONE)
                                                      : fit128(attn_cluster_kernel<128, 32>, 4, AC_THREADS, AC_SMEM_ALONE));
   a.groups = sliced ? gqa / slice_heads : 1;
@@ -1244,6 +1246,12 @@ static int launch_attn_cluster(AttnStep a, unsigned bound, unsigned rows, unsign
   return check_cuda(e, "attention launch");
 }
 
+/* Rows that the window is expected to have: with the position in device memory (a captured step) pos says where the positions start. The
+ * bound of such a launch says nothing about it: caches are as long as the longest context. */
+static unsigned likely_rows(const nntr_attn_desc *a, unsigned pos, unsigned bound) {
+  return std::min(std::min(pos, bound - 1) + 1, a->window);
+}
+
 int launch_attention_decode(const nntr_attn_desc *a, unsigned pos, const unsigned *pos_dev, unsigned max_rows,
                             const float *q, const uint16_t *kcache, const uint16_t *vcache, float *out, void *ws,
                             size_t ws_bytes, unsigned flags, cudaStream_t st) {
@@ -1271,7 +1279,7 @@ int launch_attention_decode(const nntr_attn_desc *a, unsigned pos, const unsigne
   s.out = out, s.sink = a->sink, s.pos_dev = pos_dev, s.pos = pos, s.window = a->window;
   s.hq = hq, s.hkv = hkv, s.hd = hd, s.tokens = 1;
   bool taken;
-  if ((rc = launch_attn_cluster(s, bound, rows, flags, st, &taken)) || taken)
+  if ((rc = launch_attn_cluster(s, bound, rows, likely_rows(a, pos, bound), flags, st, &taken)) || taken)
     return rc;
   cudaLaunchConfig_t cfg = {};
   cudaLaunchAttribute attr[1];
@@ -1333,7 +1341,7 @@ int launch_attention_step(const nntr_attn_desc *a, unsigned pos, const unsigned 
   s.pos_dev = pos_dev, s.pos = pos, s.window = a->window;
   s.hq = hq, s.hkv = hkv, s.hd = hd, s.rope = 1, s.tokens = 1;
   bool taken;
-  if ((rc = launch_attn_cluster(s, bound, rows, flags, st, &taken)) || taken)
+  if ((rc = launch_attn_cluster(s, bound, rows, likely_rows(a, pos, bound), flags, st, &taken)) || taken)
     return rc;
   if ((rc = launch_rope_cache_append(a, pos, pos_dev, q, k, v, q_gamma, k_gamma, eps, kcache, vcache, cos_tab, sin_tab, flags,
                                      st)))
@@ -1375,7 +1383,7 @@ int launch_attention_rows(const nntr_attn_desc *a, unsigned pos, unsigned tokens
   s.hq = (int)a->n_heads_q, s.hkv = (int)a->n_heads_kv, s.hd = (int)a->head_dim;
   s.tokens = tokens, s.q_ld = (long long)ld, s.out_ld = (long long)ld_out;
   bool taken;
-  return launch_attn_cluster(s, bound, rows, flags & ~NNTR_CUDA_ATTN_SEPARATE, st, &taken);
+  return launch_attn_cluster(s, bound, rows, rows, flags & ~NNTR_CUDA_ATTN_SEPARATE, st, &taken);
 }
 
 } // namespace nntr

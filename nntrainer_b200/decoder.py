@@ -136,7 +136,8 @@ class Qwen3Decoder:
         """One decode step: ``token_f`` is a 1-element float device tensor holding the token id (the reference keeps
         ids as floats); returns (next id as int32 tensor, as float32 tensor). Logits stay in ``self.b['logits']``.
         With ``pos_dev`` (a device word) the position is read on the device, so the launches can be captured once into
-        a CUDA graph and replayed for every later token.
+        a CUDA graph and replayed for every later token; ``pos`` is then where the positions start, which chooses the form of the
+        attention launch (same bits in both).
 
         Launches per layer without ``fuse``: (residual add +) RMS norm; q | k | v projections (one batched launch);
         attention with its per-head norms, rotary work and cache append; attention_out; residual add + RMS norm;
@@ -256,7 +257,8 @@ class Qwen3Decoder:
 
     def capture(self, start_pos: int):
         """Captures one decode step into a CUDA graph: the token id lives in ``self.tok_f`` (device float, rewritten by
-        the step's own arg-max), the position in ``self.pos_dev`` (device word, advanced by the graph). Returns the
+        the step's own arg-max), the position in ``self.pos_dev`` (device word, advanced by the graph). The attention launches
+        take the form for a context of ``start_pos`` rows; any position up to ``max_seq`` may be replayed. Returns the
         graph; every ``replay()`` decodes one more token and leaves its id in ``self.tok`` / ``self.tok_f``."""
         torch = self.torch
         self.pos_dev = torch.full((2,), 0, dtype=torch.int32, device=self.dev)  # 8 bytes: the bump kernel adds to a u64
@@ -266,12 +268,12 @@ class Qwen3Decoder:
         s = torch.cuda.Stream()
         s.wait_stream(torch.cuda.current_stream())
         with torch.cuda.stream(s):
-            self.step(self.tok_f, 0, pos_dev=self.pos_dev, out_idx=self.tok, out_idx_f=self.tok_f)  # warm-up, eager
+            self.step(self.tok_f, int(start_pos), pos_dev=self.pos_dev, out_idx=self.tok, out_idx_f=self.tok_f)  # warm-up, eager
             self.pos_dev[0] = start_pos
             torch.cuda.synchronize()
             g = torch.cuda.CUDAGraph()
             with torch.cuda.graph(g, stream=s):
-                self.step(self.tok_f, 0, pos_dev=self.pos_dev, out_idx=self.tok, out_idx_f=self.tok_f)
+                self.step(self.tok_f, int(start_pos), pos_dev=self.pos_dev, out_idx=self.tok, out_idx_f=self.tok_f)
                 be.check(be.lib().nntr_cuda_epoch_bump_dev(self.pos_dev.data_ptr(), be._stream()))
         torch.cuda.current_stream().wait_stream(s)
         return g

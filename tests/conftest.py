@@ -46,6 +46,11 @@ def launches_of(graph):
 
 
 @pytest.fixture
+def launches_in():
+    return launches_of
+
+
+@pytest.fixture
 def captured():
     """captured(call): the kernels that call() launches, seen by capturing it: which form of a kernel a size is given."""
     import torch
