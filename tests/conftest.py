@@ -17,7 +17,7 @@ class CapturedLaunch:
     """A kernel of a captured CUDA graph: its grid, the CTAs of a cluster, its static shared memory, and its arguments by position."""
 
     def __init__(self, node):
-        from cuda.bindings import driver
+        driver = pytest.importorskip("cuda.bindings.driver")
         err, self._p = driver.cuGraphKernelNodeGetParams(node)
         assert err == driver.CUresult.CUDA_SUCCESS
         self.grid = (self._p.gridDimX, self._p.gridDimY, self._p.gridDimZ)
@@ -35,7 +35,7 @@ class CapturedLaunch:
 
 def launches_of(graph):
     """The kernels of a torch.cuda.CUDAGraph(keep_graph=True) in the order of their capture. Valid as long as the graph."""
-    from cuda.bindings import driver
+    driver = pytest.importorskip("cuda.bindings.driver")
     raw = driver.CUgraph(graph.raw_cuda_graph())
     err, _, n = driver.cuGraphGetNodes(raw, 0)
     assert err == driver.CUresult.CUDA_SUCCESS

@@ -365,6 +365,36 @@ def test_attention_in_one_launch_equals_the_separate_launches(be, hq, hkv, hd, r
             assert torch.equal(x.view(torch.uint8), y.view(torch.uint8))
 
 
+@pytest.mark.parametrize("max_seq,window", [(2049, None), (4096, None), (4096, 1500), (9000, None), (16384, None)])
+@pytest.mark.parametrize("hq,hkv,hd", [(64, 8, 64), (32, 8, 128), (32, 4, 128)])
+def test_the_form_for_long_contexts_at_every_fill_of_the_caches(be, captured, hq, hkv, hd, max_seq, window):
+    """The launch for long contexts over caches of max_seq rows, the position in device memory, against the separate launches: empty
+    and partial shares, no value tile, the ends of tiles of 256 rows and of their halves of 32, a window that slides (its first
+    row is not 0), and as many rows as leave room for two buffers of values and one of keys. Equal bits, caches included."""
+    g = torch.Generator(device="cuda").manual_seed(max_seq + hq)
+    r = lambda *n: torch.randn(*n, generator=g, device="cuda")  # noqa: E731
+    sink, norm = r(hq) if hd == 64 else None, (1 + 0.1 * r(hd), 1 + 0.1 * r(hd), 1e-6)
+    one, sep = (be.Attention(hq, hkv, hd, max_seq, window=window, sink=sink) for _ in range(2))
+    pos_dev = torch.zeros(1, dtype=torch.int32, device="cuda")
+    q, k, v = r(hq * hd), r(hkv * hd), r(hkv * hd)
+    launches = captured(lambda: one.step(q, k, v, max_seq - 1, pos_dev=pos_dev, qk_norm=norm))
+    assert [x.grid[0] for x in launches] == [hq * hd // 32], "not a CTA for every 32 dimensions"
+    for a, b in ((one.kcache, sep.kcache), (one.vcache, sep.vcache)):
+        a.copy_(r(*a.shape))
+        b.copy_(a)
+    at = [0, 1, 2, 31, 32, 33, 63, 64, 65, 255, 256, 257, 288, 319, 320, 321, 1023, 1024, 1025, 1499, 1500, 1501, 1789, 2048, 3000, 4095, 4097,
+          5000, 8200, 8999, 12345, 16382, 16383]
+    for pos in (p for p in at if p < max_seq):
+        q, k, v = r(hq * hd), r(hkv * hd), r(hkv * hd)
+        pos_dev.fill_(pos)
+        x = one.step(q.clone(), k, v, max_seq - 1, pos_dev=pos_dev, qk_norm=norm)
+        y = sep.step(q.clone(), k, v, pos, qk_norm=norm, separate=True)
+        assert torch.equal(x.view(torch.int32), y.view(torch.int32)), pos
+    be.device_status()
+    assert torch.equal(one.kcache.view(torch.int16), sep.kcache.view(torch.int16))
+    assert torch.equal(one.vcache.view(torch.int16), sep.vcache.view(torch.int16))
+
+
 @pytest.mark.parametrize("rows", [40, 767, 800, 1500, 4096])
 def test_attention_in_one_launch_keeps_what_is_not_a_number(be, rows):
     """A sink, a cached key and a query that are not numbers, and a key that makes a score infinite: NaN where the separate
