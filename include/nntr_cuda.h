@@ -149,7 +149,11 @@ int nntr_cuda_measure_int8_peak(double *tops, double *clk_per_mma);
  *  N % 8 == 0 (Q4_0, Q4_K).
  *  A, workspace: 16-byte aligned. B: 16-byte aligned for Q4_K and Q4_0 (Q6_K: 2).
  *  B at a multiple of 8 is taken too, except by the Q4_K GEMV (M == 1), but only
- *  by the exact kernels that need no 16-byte copies; anything less is refused. */
+ *  by the exact kernels that need no 16-byte copies; anything less is refused.
+ *  Order is the stream's: what was launched before is seen, A, B and the
+ *  workspace are read and C is written behind it. M > 1 is launched as a
+ *  programmatic dependent, so its CTAs may be resident (and wait) while what is
+ *  in front of it in the stream ends; M == 1 is launched plainly. */
 int nntr_cuda_gemm_q4_K_dev(unsigned M, unsigned N, unsigned K, const float *A, unsigned lda, const void *B,
                             unsigned ldb, float *C, unsigned ldc, void *workspace, size_t workspace_bytes,
                             void *stream);

@@ -435,18 +435,20 @@ __global__ void attn_values_kernel(const float *__restrict__ probs, const uint16
  *            ascending row order by one warp (ordered_sum).
  *   values   a thread per dimension runs the row-ordered chain over value tiles that a producer warp keeps ahead of it
  *            (tiled TMA copies, started before the scores). CTAs of 32 dimensions (long windows): six warps turn the tiles round, and
- *            the chain loads eight rows of its dimension at once: at 4096 rows 27700 clocks instead of 33300, the launch 33.5 us.
- * Clock stamps of one CTA, 64 / 8 heads of 64, at 512 / 4096 rows, in clocks: up to the grid dependency 1800 / 1850, first copies and
- * heads rotated 1350 / 1450, wait for the cluster 400, score tiles 1600 / 8800, barrier behind them 2050 / 2600, maximum and
- * exponentials 1500 / 3800, ordered sum 2500 / 11500, division 450 / 1450, value chain 5400 / 33800. The value chain is half of a long
- * context at about 8 clocks per row (six inside a tile, the rest where it waits for one), where a dependent multiply-add alone
- * takes four. In a decode step, whose launches find neither code nor caches at hand, the phases up to 512 rows take half as long again
- * (32 / 8 heads of 128 at 100 rows 14300 clocks behind the dependency, alone 8900). 64 / 8 heads of 64 at 4096 rows 36.5 us, 32 / 8 heads
- * of 128 at 512 rows 11.2 us (with generic accesses to the tiles, and value tiles of 128 rows: 45 and 12.3), at 128 rows of a window
- * 8.0 us with the copy of q (8.4). Measured and not kept: eight rows at a time with twenty-four more on their way (40.7 us, sixteen and
- * sixteen 36.6: a warp waits for its loads by few counters), half of the ring waited for at a time (44), four blocks of the ordered sum
- * at once (16900 clocks instead of 11500), the integers of all blocks of 32 rows by all warps beforehand (2 us more at 4096 rows), two rows
- * and two heads per thread in the scores (heads of 64: 1800 a tile instead of 1900; of 128: 2660 instead of 2200).
+ *            the chain loads eight rows of its dimension at once: at 4096 rows 27700 clocks instead of 33300, the launch 33.5 us
+ *            instead of 36.5.
+ * Clock stamps of one CTA, 64 / 8 heads of 64, at 512 rows (CTAs of 64 dimensions) / at 4096 (of 32), in clocks: up to the grid dependency
+ * 1800 / 2500, first copies and heads rotated 1350 / 1600, wait for the cluster 400 / 60, score tiles 1600 / 5850, barrier behind them
+ * 2050 / 1450, maximum and exponentials 1500 / 3900, ordered sum 2500 / 12050, division 450 / 1450, value chain 5400 / 28000. The value
+ * chain is half of a long context at 6.8 clocks per row, where a dependent multiply-add alone takes four (CTAs of 64 dimensions: about 8,
+ * six inside a tile, the rest where it waits for one). In a decode step, whose launches find neither code nor caches at hand, the phases
+ * up to 512 rows take half as long again (32 / 8 heads of 128 at 100 rows 14300 clocks behind the dependency, alone 8900). 32 / 8 heads
+ * of 128 at 512 rows 11.2 us (with generic accesses to the tiles, and value tiles of 128 rows, 12.3), at 128 rows of a window
+ * 8.0 us with the copy of q (8.4). Measured with CTAs of 64 dimensions at 4096 rows, 36.5 us, and not kept: eight rows at a time with
+ * twenty-four more on their way (40.7 us, sixteen and sixteen 36.6: a warp waits for its loads by few counters), half of the ring waited for
+ * at a time (44), four blocks of the ordered sum at once (16900 clocks instead of 11500), the integers of all blocks of 32 rows by all warps
+ * beforehand (2 us more), two rows and two heads per thread in the scores (heads of 64: 1800 a tile instead of 1900; of 128: 2660 instead of
+ * 2200).
  * Ring positions are counted, not divided: an integer division in a loop that one thread runs costs more than a tile's copy. */
 constexpr int AC_THREADS = 256;
 constexpr int AC_WARPS = AC_THREADS / 32;

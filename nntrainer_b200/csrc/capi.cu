@@ -278,10 +278,11 @@ __global__ void host_done_kernel(unsigned long long *word, unsigned long long va
 
 /* --------------------------------------------------------- GEMM dispatch */
 static std::atomic<int> g_gemm_path{NNTR_CUDA_GEMM_PATH_AUTO};
-/* Below this the exact kernels win: a 128-row activation tile is mostly padding there. Exact against automatic at 32 / 64 rows: Q4_K
- * 6144 x 2560 12.8 / 16.0 us against 19.0 / 19.5, 4096 x 4096 17.5 / 22.5 against 17.1 / 17.7, 24576 x 4096 36.1 / 66.4 against 50.0 / 50.2;
- * Q4_0 24576 x 4096 32.8 / 50.2 against 49.5 / 49.5; Q6_K 151936 x 2560, 32 rows, 338 against 272. For Q4_K and Q4_0 the times cross
- * between 32 and 64 rows and later. */
+/* Below this the exact kernels win: a 128-row activation tile is mostly padding there. Exact against automatic at 32 / 40 / 64 rows: Q4_K
+ * 6144 x 2560 12.4 / 14.5 / 15.9 us against 17.7 / 18.0 / 18.1, 4096 x 4096 16.9 / 17.8 / 22.1 against 16.4 / 16.6 / 17.2, 24576 x 4096 35.0 / 59 / 66.4
+ * against 48.2 / 48.2 / 48.6; Q4_0 24576 x 4096 32.0 / 46.1 / 51.7 against 44.5 / 44.6 / 44.7, 9728 x 2560 14.0 / 16.2 / 18.2 against 20.4 / 20.8 /
+ * 21.3; Q6_K 151936 x 2560, 32 rows, 338 against 244. For Q4_K and Q4_0 the times cross between 32 and 64 rows and later; the line is the one
+ * from which the interface promises the tensor cores. */
 constexpr unsigned TENSOR_PATH_MIN_M = 32;
 
 /* 0: exact kernels, 1: integer tensor path (kind::i8), 2: fp16 tensor path (kind::f16) */

@@ -46,10 +46,11 @@
  *               as soon as the MMAs that read its slot have retired.
  *   warp 18     one thread starts the tiled copies of the packed weights
  *               (Q4_K, Q4_0) into a ring of two (pair: four) stages.
- * Three stages of 64 KB (pair: four of 48; Q6_K alone: two of 64), both accumulators (512 columns) in tensor memory. Every wait is bounded (pipeline.cuh).
+ * Three stages of 64 KB (pair: four of 48; Q6_K alone or shared: two of 64), both accumulators (512 columns) in tensor memory. Every wait is bounded (pipeline.cuh).
  *
- * What bounds it. A stage's MMAs take 1024 clocks. A CTA alone takes 1310 a stage: its producers, and the shared memory, which
- * carries 96 KB for the MMAs, 64 of stores and copies and the packed weights. A pair takes 1070, the MMAs: half of the expansion and 64 KB
+ * What bounds it. A stage's MMAs take 1024 clocks. A CTA alone takes about 1600 a stage with Q4_K and 1350 with Q4_0 (the difference of K =
+ * 4096 and 8192, 256 x 37888, at the clock meanwhile): its producers, and the shared memory, which carries 96 KB for the MMAs, 64 of
+ * stores and copies and the packed weights. A pair takes 1070 (Q4_K, stamps inside a CTA), the MMAs: half of the expansion and 64 KB
  * for the MMAs. (With no expansion and no copies at all 1050; a hand-over from CTA to CTA with release and acquire at cluster
  * scope 1600: it is one more latency in each round of the ring.) Q4_K 24576 x 4096, 1024 rows 184.6 -> 167 us, 512
  * rows 115.9 -> 101.6 (98.5 with even_rows()); Q4_0 512 rows of 24576 x 2880 85.2 -> 77.3 (70.6); Q6_K 151936 x 2560, 300 / 512 rows
@@ -211,7 +212,7 @@ __device__ __forceinline__ uint32_t expand2_q40(uint32_t nib2, __half2 d) {
  * 128 activation rows of each and the weights of both, so a stage's expansion serves 512 rows instead of 256, and a CTA's MMAs read half
  * of the weights from its own shared memory only.
  * F16_SHARED: a cluster of CTAs may share the tile. A kernel of its own: the code of a shared tile in the kernel of a lone CTA costs
- * that one registers (80 without, 96 with) and 1024 x 24576 x 4096 Q4_K 185 us instead of 182. (It keeps the test for a cluster of
+ * that one registers (81 without, 96 with) and 1024 x 24576 x 4096 Q4_K 185 us instead of 182. (It keeps the test for a cluster of
  * one, without which the compiler spills 44 bytes instead of 8.) */
 template <int QT, int MODE>
 __global__ void __launch_bounds__(F16_THREADS, 1)
@@ -375,18 +376,19 @@ gemm_f16_kernel(const __grid_constant__ CUtensorMap wmap, const uint8_t *__restr
         if (!(ok = slot_wait(st)))
           break;
         uint8_t *wdst = smem + (st % Cfg::STAGES) * Cfg::STAGE_BYTES + r * 16;
-        if (r < own_rows)
+        if (r < own_rows) {
 #pragma unroll
-        for (int c = 0; c < 4; ++c) {
-          // word -> 8 halves in the order [lo b0, lo b2, lo b1, lo b3, hi b0, hi b2, hi b1, hi b3]
-          const uint32_t wx = w[c].x, wy = w[c].y;
-          uint8_t *d = wdst + (2 * (c ^ sw)) * (Cfg::W_ROWS * 16);
-          *reinterpret_cast<uint4 *>(d) =
-            make_uint4(expand2(wx & 0x000f000fu, d_lo, m_lo), expand2((wx >> 8) & 0x000f000fu, d_lo, m_lo),
-                       expand2((wx >> 4) & 0x000f000fu, d_hi, m_hi), expand2((wx >> 12) & 0x000f000fu, d_hi, m_hi));
-          *reinterpret_cast<uint4 *>(d + Cfg::W_ROWS * 16) =
-            make_uint4(expand2(wy & 0x000f000fu, d_lo, m_lo), expand2((wy >> 8) & 0x000f000fu, d_lo, m_lo),
-                       expand2((wy >> 4) & 0x000f000fu, d_hi, m_hi), expand2((wy >> 12) & 0x000f000fu, d_hi, m_hi));
+          for (int c = 0; c < 4; ++c) {
+            // word -> 8 halves in the order [lo b0, lo b2, lo b1, lo b3, hi b0, hi b2, hi b1, hi b3]
+            const uint32_t wx = w[c].x, wy = w[c].y;
+            uint8_t *d = wdst + (2 * (c ^ sw)) * (Cfg::W_ROWS * 16);
+            *reinterpret_cast<uint4 *>(d) =
+              make_uint4(expand2(wx & 0x000f000fu, d_lo, m_lo), expand2((wx >> 8) & 0x000f000fu, d_lo, m_lo),
+                         expand2((wx >> 4) & 0x000f000fu, d_hi, m_hi), expand2((wx >> 12) & 0x000f000fu, d_hi, m_hi));
+            *reinterpret_cast<uint4 *>(d + Cfg::W_ROWS * 16) =
+              make_uint4(expand2(wy & 0x000f000fu, d_lo, m_lo), expand2((wy >> 8) & 0x000f000fu, d_lo, m_lo),
+                         expand2((wy >> 4) & 0x000f000fu, d_hi, m_hi), expand2((wy >> 12) & 0x000f000fu, d_hi, m_hi));
+          }
         }
         stage_done(st);
         ok = st + Cfg::GROUPS >= n_stages || fetch(st + Cfg::GROUPS);
@@ -443,23 +445,24 @@ gemm_f16_kernel(const __grid_constant__ CUtensorMap wmap, const uint8_t *__restr
             break;
           uint8_t *wdst = smem + s * Cfg::STAGE_BYTES + r * 16 + (4 * qhalf) * (Cfg::W_ROWS * 16);
           const __half2 off = __half2half2(__ushort_as_half(0x6420)); // 1024 + 32
-          if (r < own_rows)
+          if (r < own_rows) {
 #pragma unroll
-          for (int i = 0; i < 4; ++i) {
-            const uint32_t l = ql[s2][i], hq = qh[i];
-            // the 6-bit values as bytes: low nibbles + qh bits (2 s2, 2 s2 + 1) for quarter s2, high nibbles + qh bits
-            // (2 s2 + 4, + 5) for quarter s2 + 2; a byte permute with 0x64 makes (1024 + q) halves: elements {0, 2}, {1, 3}
-            const uint32_t qlo = (l & 0x0f0f0f0fu) | ((hq << (4 - 2 * s2)) & 0x30303030u);
-            const uint32_t qhi = ((l >> 4) & 0x0f0f0f0fu) | ((hq >> (2 * s2)) & 0x30303030u);
-            const uint32_t t0 = __byte_perm(qlo, 0x64646464u, 0x4240), t1 = __byte_perm(qlo, 0x64646464u, 0x4341);
-            const uint32_t t2 = __byte_perm(qhi, 0x64646464u, 0x4240), t3 = __byte_perm(qhi, 0x64646464u, 0x4341);
-            const __half2 w0 = __hmul2(__hsub2(*reinterpret_cast<const __half2 *>(&t0), off), d_lo);
-            const __half2 w1 = __hmul2(__hsub2(*reinterpret_cast<const __half2 *>(&t1), off), d_lo);
-            const __half2 w2 = __hmul2(__hsub2(*reinterpret_cast<const __half2 *>(&t2), off), d_hi);
-            const __half2 w3 = __hmul2(__hsub2(*reinterpret_cast<const __half2 *>(&t3), off), d_hi);
-            *reinterpret_cast<uint4 *>(wdst + i * (Cfg::W_ROWS * 16)) =
-              make_uint4(*reinterpret_cast<const uint32_t *>(&w0), *reinterpret_cast<const uint32_t *>(&w1),
-                         *reinterpret_cast<const uint32_t *>(&w2), *reinterpret_cast<const uint32_t *>(&w3));
+            for (int i = 0; i < 4; ++i) {
+              const uint32_t l = ql[s2][i], hq = qh[i];
+              // the 6-bit values as bytes: low nibbles + qh bits (2 s2, 2 s2 + 1) for quarter s2, high nibbles + qh bits
+              // (2 s2 + 4, + 5) for quarter s2 + 2; a byte permute with 0x64 makes (1024 + q) halves: elements {0, 2}, {1, 3}
+              const uint32_t qlo = (l & 0x0f0f0f0fu) | ((hq << (4 - 2 * s2)) & 0x30303030u);
+              const uint32_t qhi = ((l >> 4) & 0x0f0f0f0fu) | ((hq >> (2 * s2)) & 0x30303030u);
+              const uint32_t t0 = __byte_perm(qlo, 0x64646464u, 0x4240), t1 = __byte_perm(qlo, 0x64646464u, 0x4341);
+              const uint32_t t2 = __byte_perm(qhi, 0x64646464u, 0x4240), t3 = __byte_perm(qhi, 0x64646464u, 0x4341);
+              const __half2 w0 = __hmul2(__hsub2(*reinterpret_cast<const __half2 *>(&t0), off), d_lo);
+              const __half2 w1 = __hmul2(__hsub2(*reinterpret_cast<const __half2 *>(&t1), off), d_lo);
+              const __half2 w2 = __hmul2(__hsub2(*reinterpret_cast<const __half2 *>(&t2), off), d_hi);
+              const __half2 w3 = __hmul2(__hsub2(*reinterpret_cast<const __half2 *>(&t3), off), d_hi);
+              *reinterpret_cast<uint4 *>(wdst + i * (Cfg::W_ROWS * 16)) =
+                make_uint4(*reinterpret_cast<const uint32_t *>(&w0), *reinterpret_cast<const uint32_t *>(&w1),
+                           *reinterpret_cast<const uint32_t *>(&w2), *reinterpret_cast<const uint32_t *>(&w3));
+            }
           }
           asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
           __syncwarp(); // every lane's writes are fenced; one arrival per warp keeps the barrier word off the critical path
@@ -490,17 +493,18 @@ gemm_f16_kernel(const __grid_constant__ CUtensorMap wmap, const uint8_t *__restr
         if (!(ok = slot_wait(st)))
           break;
         uint8_t *wdst = smem + (st % Cfg::STAGES) * Cfg::STAGE_BYTES + r * 16;
-        if (r < own_rows)
+        if (r < own_rows) {
 #pragma unroll
-        for (int k = 0; k < 2; ++k) {
-          const __half2 d2 = __half2half2(__ushort_as_half(dbits[k]));
-          const uint32_t w[4] = {q[2 * k].x ^ 0x88888888u, q[2 * k].y ^ 0x88888888u, q[2 * k + 1].x ^ 0x88888888u,
-                                 q[2 * k + 1].y ^ 0x88888888u};
+          for (int k = 0; k < 2; ++k) {
+            const __half2 d2 = __half2half2(__ushort_as_half(dbits[k]));
+            const uint32_t w[4] = {q[2 * k].x ^ 0x88888888u, q[2 * k].y ^ 0x88888888u, q[2 * k + 1].x ^ 0x88888888u,
+                                   q[2 * k + 1].y ^ 0x88888888u};
 #pragma unroll
-          for (int wi = 0; wi < 4; ++wi) // chunk wi: elements 4wi + {0,2,1,3} then 16 + 4wi + {0,2,1,3} of the block
-            *reinterpret_cast<uint4 *>(wdst + (4 * k + wi) * (Cfg::W_ROWS * 16)) =
-              make_uint4(expand2_q40(w[wi] & 0x000f000fu, d2), expand2_q40((w[wi] >> 8) & 0x000f000fu, d2),
-                         expand2_q40((w[wi] >> 4) & 0x000f000fu, d2), expand2_q40((w[wi] >> 12) & 0x000f000fu, d2));
+            for (int wi = 0; wi < 4; ++wi) // chunk wi: elements 4wi + {0,2,1,3} then 16 + 4wi + {0,2,1,3} of the block
+              *reinterpret_cast<uint4 *>(wdst + (4 * k + wi) * (Cfg::W_ROWS * 16)) =
+                make_uint4(expand2_q40(w[wi] & 0x000f000fu, d2), expand2_q40((w[wi] >> 8) & 0x000f000fu, d2),
+                           expand2_q40((w[wi] >> 4) & 0x000f000fu, d2), expand2_q40((w[wi] >> 12) & 0x000f000fu, d2));
+          }
         }
         stage_done(st);
         ok = st + Cfg::GROUPS >= n_stages || fetch(st + Cfg::GROUPS);
@@ -553,7 +557,7 @@ gemm_f16_kernel(const __grid_constant__ CUtensorMap wmap, const uint8_t *__restr
   } else if (warp == F16_RAW_WARP) {
     /* ---------------------------- packed weights ---------------------------- */
     // The latency of HBM and L2 is in this ring and the producers never wait for a load they issued themselves. Tiled
-    // copies, a box of 32 row groups x 128 (Q4_0: 144) bytes each: 32 untiled copies of 256 bytes per stage measured 1.6 times
+    // copies, a box of all row groups that the CTA expands x 128 (Q4_0: 144) bytes each: 32 untiled copies of 256 bytes per stage measured 1.6 times
     // slower than no ring at all.
     if (QT != NNTR_Q6_K && lane == 0) {
       const int y = (n0 + peer * own_rows) / 8;
@@ -760,7 +764,7 @@ quantize_q8_0_f16_tiles_kernel(const float *__restrict__ x, int64_t ldx, uint8_t
   }
 }
 
-/** Into how many parts K is cut, so that few tiles still use the machine. A CTA alone walks K at 0.9 us (Q6_K 1.5) a stage
+/** Into how many parts K is cut, so that few tiles still use the machine. A CTA alone walks K at 0.8 us (Q4_0 0.7, Q6_K 1.4 and more) a stage
  *  however many SMs are idle; the parts' sums cost about 2 us at the end. As many as still run in one wave of clusters, of at
  *  least four stages each. */
 template <int QT> int k_parts(int tiles, int k_stages) {

@@ -66,9 +66,11 @@ constexpr int ROUTER_SLICES = 32; // CTAs per token
 constexpr int MAX_E_PER_LANE = 8; // up to 256 experts
 // Tokens from which the router takes eight of them at a time. Layers of 4 of 32 experts of 2880 x 2880, a CTA row per token / eight
 // tokens per CTA row, 12 / 16 / 24 / 40 tokens: 116.8 / 118.0 / 120.3 / 123.5 us, 112.0 / 114.7 / 119.1 / 119.0; 8 of 128 of 2048 x 768, 16 / 24 /
-// 32 / 40 / 48: 82.0 / 89.6 / 103.0 / 105.6 / -, 88.1 / 91.6 / 103.7 / 104.8 / 109.4; 8 of 256 of 1024 x 512, 16 / 32: 53.7 / 74.7, 55.2 / 72.0.
+// 32 / 40 / 48: 82.0 / 89.6 / 103.0 / 105.6 / -, 88.1 / 91.6 / 103.7 / 104.8 / 109.4; 8 of 256 of 1024 x 512, 16 / 32: 53.7 / 74.7, 55.2 / 72.0. 33 to 64
+// experts cross earlier, and the line is a cautious one there: 8 of 64 of 2048 x 768, 16 / 20 / 32 / 40: 66.5 / 67.1 / 73.2 / 75.6, 67.7 / 66.2 /
+// 71.1 / 71.4; 4 of 40 of 2880 x 1440, 16 / 24 / 32 / 40: 80.4 / 91.6 / 92.3 / 94.6, 84.0 / 90.8 / 91.3 / 91.1.
 static unsigned router_rows_min_tokens(unsigned experts) { return experts <= 32 ? 12 : 40; }
-/** rows of a warp's slice fetched before the dependency wait: all of them for hidden sizes up to 2048 (96 experts and fewer: 3072) */
+/** rows of a warp's slice fetched before the dependency wait: all of them for hidden sizes up to 2048 (64 experts and fewer: 3072) */
 template <int PER> constexpr int ROUTER_PRE = PER < 4 ? 12 : 8;
 
 /* std::partial_sort(idx, idx + k, idx + n, [&](a, b) { return v[a] > v[b]; }) on idx = 0..n-1, as the GNU C++ library
