@@ -255,12 +255,14 @@ class Qwen3Decoder:
         call("argmax_dev", b["logits"], 1, c.vocab, c.vocab, v["idx"], v["idx_f"], flags, st)
         return calls
 
-    def capture(self, start_pos: int):
+    def capture(self, start_pos: int, tokens: int = 0):
         """Captures one decode step into a CUDA graph: the token id lives in ``self.tok_f`` (device float, rewritten by
-        the step's own arg-max), the position in ``self.pos_dev`` (device word, advanced by the graph). The attention launches
-        take the form for a context of ``start_pos`` rows; any position up to ``max_seq`` may be replayed. Returns the
-        graph; every ``replay()`` decodes one more token and leaves its id in ``self.tok`` / ``self.tok_f``."""
+        the step's own arg-max), the position in ``self.pos_dev`` (device word, advanced by the graph). Returns the
+        graph; every ``replay()`` decodes one more token and leaves its id in ``self.tok`` / ``self.tok_f``. ``tokens``: how
+        many it is meant for, if that is known; the attention launches take the form for the middle of its positions, and any
+        position up to ``max_seq`` may be replayed."""
         torch = self.torch
+        likely_pos = int(start_pos) + int(tokens) // 2
         self.pos_dev = torch.full((2,), 0, dtype=torch.int32, device=self.dev)  # 8 bytes: the bump kernel adds to a u64
         self.pos_dev[0] = start_pos
         self.tok = torch.zeros(1, dtype=torch.int32, device=self.dev)
@@ -268,12 +270,12 @@ class Qwen3Decoder:
         s = torch.cuda.Stream()
         s.wait_stream(torch.cuda.current_stream())
         with torch.cuda.stream(s):
-            self.step(self.tok_f, int(start_pos), pos_dev=self.pos_dev, out_idx=self.tok, out_idx_f=self.tok_f)  # warm-up, eager
+            self.step(self.tok_f, likely_pos, pos_dev=self.pos_dev, out_idx=self.tok, out_idx_f=self.tok_f)  # warm-up, eager
             self.pos_dev[0] = start_pos
             torch.cuda.synchronize()
             g = torch.cuda.CUDAGraph()
             with torch.cuda.graph(g, stream=s):
-                self.step(self.tok_f, int(start_pos), pos_dev=self.pos_dev, out_idx=self.tok, out_idx_f=self.tok_f)
+                self.step(self.tok_f, likely_pos, pos_dev=self.pos_dev, out_idx=self.tok, out_idx_f=self.tok_f)
                 be.check(be.lib().nntr_cuda_epoch_bump_dev(self.pos_dev.data_ptr(), be._stream()))
         torch.cuda.current_stream().wait_stream(s)
         return g

@@ -118,18 +118,18 @@ def test_a_replaced_cache_is_used_by_every_launch_sequence(be):
 
 @pytest.mark.parametrize("hq,hkv,hd", [(32, 8, 128), (32, 4, 128), (64, 8, 64)])
 def test_a_captured_step_has_the_form_for_its_context_however_long_the_caches_are(be, launches_in, monkeypatch, hq, hkv, hd):
-    """Long contexts have an attention launch of their own, slower for short ones: a graph is given it by where its positions
-    start, not by the rows that the caches could hold."""
+    """Long contexts have an attention launch of their own, slower for short ones: a graph is given it by the positions that
+    it is meant for, not by the rows that the caches could hold."""
     make = torch.cuda.CUDAGraph
     monkeypatch.setattr(torch.cuda, "CUDAGraph", lambda: make(keep_graph=True))
 
-    def grids(start, max_seq):
+    def grids(start, max_seq, tokens=0):
         cfg = DecoderConfig(n_layers=1, hidden=256, n_heads=hq, n_kv_heads=hkv, head_dim=hd, inter=256, vocab=256, max_seq=max_seq)
         with tempfile.TemporaryDirectory() as td:
             path = os.path.join(td, "model.bin")
             write_bin(path, cfg, synthetic_weights(cfg, 3))
             dec = Qwen3Decoder(cfg, path, pdl=True)
-        g = dec.capture(start)
+        g = dec.capture(start, tokens)
         seen = [x.grid for x in launches_in(g)]
         dec.close()
         return seen
@@ -138,6 +138,7 @@ def test_a_captured_step_has_the_form_for_its_context_however_long_the_caches_ar
     assert len(short) == len(long) and short != long
     assert grids(100, 4096) == short
     assert grids(2000, 4096) == long
+    assert grids(100, 4096, 4000) == long and grids(100, 4096, 100) == short
 
 
 @pytest.mark.parametrize("window,fc,P,hd", [(None, "q4_K", 2, 64), (None, "q4_K", 9, 64), (16, "q4_K", 40, 64), (None, "q6_K", 33, 64),
