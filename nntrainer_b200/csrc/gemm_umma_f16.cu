@@ -851,7 +851,7 @@ int launch_typed(unsigned M, unsigned N, unsigned K, const uint8_t *tiles, const
     // half as many tiles. Q4_K, pairs / CTAs alone: 300 x 24576 x 4096 91.4 / 103.8 us, 512 95.5 / 107, 603 140.7 / 117.8, 768 143.5 / 129.6,
     // 859 157 / 169.6, 1024 161 / 182.6; 9728 x 2560 512 / 768 / 1024 rows 33.4 / 37.0, 61.9 / 40.2, 64.8 / 70.2; 8192 x 8192 768 rows 93.7 / 106.5;
     // Q4_0 19456 x 2560 768 / 1280 / 1792 rows 90.5 / 73.5, 126.3 / 115.1, 161.6 / 156.3; Q6_K 9728 x 2560 768 rows 64.4 / 58.4, 1280
-    // 76.8 / 101.2. Of 315 sizes of 257 to 2048 rows the other form is by no more than 2 % the faster one.
+    // 76.8 / 101.2. Of 296 sizes of 257 to 2048 rows the other form is by no more than 3 % the faster one.
     if (mtiles > 2) {
       static ClusterFit fit;
       const int quads = (mtiles + 3) / 4, slots = fit(gemm_f16_kernel<QT, F16_PAIR>, 2, F16_THREADS, F16Cfg<QT, F16_PAIR>::SMEM);
